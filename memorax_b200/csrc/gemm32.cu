@@ -1,0 +1,633 @@
+// float32 matrix products on the tensor cores (tcgen05).
+//
+// A float32 number is the exact sum of three bf16 numbers (8 + 8 + 8 mantissa bits: hi + mid + lo), so a product
+// of float32 matrices is a sum of bf16 products accumulated in float32.  The six largest of the nine are kept;
+// the dropped ones (mid*lo, lo*mid, lo*lo) are below 2^-26 of |a||b|, i.e. below the rounding of a float32 product.
+//
+// Bound: the tensor pipe at six bf16 products per float32 product (1.66 PFLOP/s / 6 = 277 TFLOP/s; a plain float32
+// FMA kernel stops at about 65 here).  At M = 128, N = 256 the pipe reads 96 bytes of shared memory per cycle and
+// the conversion below writes 48, against 128 available, so shared memory binds a little before the pipe does.
+//
+// One persistent CTA per SM, warp-specialised:
+//   8 / 4 warps  epilogue: accumulators (TMEM) -> global, one row per thread, 32-byte stores
+//   8 / 12 warps producers: global float32 -> registers (a stage ahead) -> three bf16 planes in shared memory
+//   1 warp       issues the MMAs (12 per stage of 32 k)
+// Weights are split once, by split_weights, into images of the shared-memory stage, which arrive by one bulk copy per
+// stage: with both operands converted here the producers bound the kernel (127 TFLOP/s at 65536 x 1024 x 256).  A
+// gradient of a weight contracts two activations and converts both.
+// Operand planes are in the panel format of umma.cuh, which serves contraction over columns and over rows alike, so
+// nothing is transposed.
+//
+// Precision: the tensor core truncates when it adds to a float32 accumulator (measured: the error grows linearly with
+// the number of additions, 3.3e-6 of the result's norm after 192), so the five small products go to an accumulator of
+// their own, whose truncations are 2^-8 as large, and the hi*hi accumulator is drained after at most kSegment k and
+// summed in float32 registers from there on.  Errors against float64 are then those of a float32 FMA kernel.
+#include "gemm32.cuh"
+#include "mxk_common.cuh"
+#include "tma.cuh"
+#include "umma.cuh"
+
+namespace mxk {
+namespace gemm32 {
+namespace {
+
+using namespace umma;
+
+constexpr int kBM = 128, kBK = 32;
+constexpr int kSegment = 512;   // k between two drains of the accumulators
+
+struct Params {
+  const float* a;
+  long long lda;
+  const uint8_t* image;   // kOuter: unused
+  const float* b;         // kOuter only
+  long long ldb;
+  bool a_wide, b_wide;    // 32-byte aligned rows
+  float* c;
+  long long ldc;
+  int c_vec;
+  int M, N, K;
+  int k_split;           // k per split (a multiple of kBK)
+  int splits;
+  float* partial;        // [splits][M][N] when splits > 1
+  Epilogue ep;
+  int ep_vec;
+  int* status;
+};
+
+template <int BN>
+struct Layout {
+  static constexpr int kStages = BN == 256 ? 3 : (BN == 128 ? 4 : 5);
+  static constexpr int kPlaneA = kBM * kBK * 2, kPlaneB = BN * kBK * 2;   // bytes
+  static constexpr int kStage = 3 * (kPlaneA + kPlaneB);
+  static constexpr int kBarriers = kStages * kStage;
+  static constexpr int kBytes = kBarriers + 256;
+  // two accumulators of BN columns; a second pair, where TMEM has room for it, lets a tile's epilogue run under the
+  // next tile's products
+  static constexpr int kAccs = BN == 256 ? 1 : 2;
+  static constexpr uint32_t kTmem = kAccs * 2 * BN;
+};
+
+__device__ __forceinline__ void load8(const float* p, int valid, int vec, float* x) {
+  if (valid >= 8 && vec == 8) {
+    asm volatile("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]), "=f"(x[4]), "=f"(x[5]), "=f"(x[6]), "=f"(x[7])
+                 : "l"(p));
+  } else if (valid >= 8 && vec == 4) {
+    const float4 u = __ldg(reinterpret_cast<const float4*>(p)), v = __ldg(reinterpret_cast<const float4*>(p) + 1);
+    x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w;
+    x[4] = v.x; x[5] = v.y; x[6] = v.z; x[7] = v.w;
+  } else {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) x[e] = e < valid ? __ldg(p + e) : 0.f;
+  }
+}
+
+// What this thread has stored before (not through the read-only path).
+__device__ __forceinline__ void load8_own(const float* p, int valid, int vec, float* x) {
+  if (valid >= 8 && vec == 8) {
+    asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]), "=f"(x[4]), "=f"(x[5]), "=f"(x[6]), "=f"(x[7])
+                 : "l"(p)
+                 : "memory");
+  } else {
+    const volatile float* q = p;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) x[e] = e < valid ? q[e] : 0.f;
+  }
+}
+
+// hi / mid / lo bf16 planes of eight floats
+__device__ __forceinline__ void split8(const float* x, uint4& hi, uint4& mid, uint4& lo) {
+  uint32_t h[4], m[4], l[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float a = x[2 * i], b = x[2 * i + 1];
+    h[i] = pack_bf16(a, b);
+    a -= __uint_as_float(h[i] << 16);
+    b -= __uint_as_float(h[i] & 0xFFFF0000u);
+    m[i] = pack_bf16(a, b);
+    a -= __uint_as_float(m[i] << 16);
+    b -= __uint_as_float(m[i] & 0xFFFF0000u);
+    l[i] = pack_bf16(a, b);
+  }
+  hi = make_uint4(h[0], h[1], h[2], h[3]);
+  mid = make_uint4(m[0], m[1], m[2], m[3]);
+  lo = make_uint4(l[0], l[1], l[2], l[3]);
+}
+
+// One operand tile of a stage: `ROWS` contracted over its rows ([kBK][EXT]) or its columns ([EXT][kBK]); split into
+// blocks of 8 rows x 32 columns, one block per warp and turn: a lane owns 8 consecutive columns of a row, eight
+// consecutive lanes own eight rows (conflict-free 16-byte shared stores, whole 128-byte lines of global memory).
+template <bool ROWS, int EXT, int WARPS>
+struct Tile {
+  static constexpr int kRows = ROWS ? kBK : EXT;
+  static constexpr int kBlocks = EXT * kBK / 256;
+  static constexpr int kTurns = (kBlocks + WARPS - 1) / WARPS;
+  float x[kTurns][8];
+  const float* ptr[kTurns];   // this lane's vector of the block about to be loaded
+  __device__ static __forceinline__ void coords(int block, int lane, int& r, int& c) {
+    const int rb = ROWS ? (block & 3) : block, cb = ROWS ? (block >> 2) : 0;
+    r = rb * 8 + (lane & 7);
+    c = cb * 32 + (lane >> 3) * 8;
+  }
+  // ext0: the tile's first index along EXT, k0: along the contraction
+  __device__ __forceinline__ void begin(const float* base, long long ld, int warp, int lane, int ext0, int k0) {
+#pragma unroll
+    for (int i = 0; i < kTurns; ++i) {
+      int r, c;
+      coords(warp + i * WARPS, lane, r, c);
+      ptr[i] = base + static_cast<long long>(r + (ROWS ? k0 : ext0)) * ld + (c + (ROWS ? ext0 : k0));
+    }
+  }
+  __device__ __forceinline__ void advance(long long ld) {
+#pragma unroll
+    for (int i = 0; i < kTurns; ++i) ptr[i] += ROWS ? kBK * ld : static_cast<long long>(kBK);
+  }
+  // `inner`: the whole tile lies inside the matrix and its rows are 32-byte aligned
+  __device__ __forceinline__ void load(int i, bool inner, int warp, int lane, int ext0, int ext_end, int k0, int k_end) {
+    const int block = warp + i * WARPS;
+    if (kBlocks % WARPS != 0 && block >= kBlocks) return;
+    if (inner) {
+      load8(ptr[i], 8, 8, x[i]);
+    } else {
+      int r, c;
+      coords(block, lane, r, c);
+      const int row = r + (ROWS ? k0 : ext0), col = c + (ROWS ? ext0 : k0);
+      const bool in = row < (ROWS ? k_end : ext_end);
+      load8(ptr[i], in ? (ROWS ? ext_end : k_end) - col : 0, 1, x[i]);
+    }
+  }
+  __device__ __forceinline__ void store(int i, uint8_t* plane0, int warp, int lane) {
+    constexpr int kPlane = EXT * kBK * 2;
+    const int block = warp + i * WARPS;
+    if (kBlocks % WARPS != 0 && block >= kBlocks) return;
+    int r, c;
+    coords(block, lane, r, c);
+    uint4 hi, mid, lo;
+    split8(x[i], hi, mid, lo);
+    uint8_t* const dst = plane0 + ((c >> 3) * kRows + r) * 16;
+    *reinterpret_cast<uint4*>(dst) = hi;
+    *reinterpret_cast<uint4*>(dst + kPlane) = mid;
+    *reinterpret_cast<uint4*>(dst + 2 * kPlane) = lo;
+  }
+};
+
+__device__ __forceinline__ void arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* out) {
+  uint32_t r[32];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr)
+      : "memory");
+#pragma unroll
+  for (int i = 0; i < 32; ++i) out[i] = __uint_as_float(r[i]);
+}
+
+__device__ __forceinline__ void store8(float* p, int valid, int vec, const float* x) {
+  if (valid >= 8 && vec == 8) {
+    asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "f"(x[0]), "f"(x[1]), "f"(x[2]),
+                 "f"(x[3]), "f"(x[4]), "f"(x[5]), "f"(x[6]), "f"(x[7])
+                 : "memory");
+  } else if (valid >= 8 && vec == 4) {
+    reinterpret_cast<float4*>(p)[0] = make_float4(x[0], x[1], x[2], x[3]);
+    reinterpret_cast<float4*>(p)[1] = make_float4(x[4], x[5], x[6], x[7]);
+  } else {
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+      if (e < valid) p[e] = x[e];
+  }
+}
+
+// kOuter: C = A^T B, both operands contracted over their rows and converted here; else C = A W^T, W from its image.
+template <int BN, bool kOuter>
+struct Roles {
+  // (a seventeenth warp is the last that leaves 96 registers a thread)
+  static constexpr int kProducerWarps = kOuter ? 12 : 8, kEpilogueWarps = kOuter ? 4 : 8;
+  static constexpr int kMmaWarp = kProducerWarps + kEpilogueWarps;
+  static constexpr int kThreads = 32 * (kMmaWarp + 1);
+};
+
+template <int BN, bool kOuter>
+__global__ void __launch_bounds__(Roles<BN, kOuter>::kThreads, 1) gemm32_kernel(const __grid_constant__ Params p) {
+  using L = Layout<BN>;
+  using R = Roles<BN, kOuter>;
+  constexpr int kProducerWarps = R::kProducerWarps, kEpilogueWarps = R::kEpilogueWarps, kMmaWarp = R::kMmaWarp;
+  constexpr int kColumnParts = kEpilogueWarps / 4;   // epilogue warps that share the rows, and the columns between them
+  using TileA = Tile<kOuter, kBM, kProducerWarps>;
+  using TileB = Tile<true, BN, kProducerWarps>;
+  constexpr int kStages = L::kStages;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint64_t* const bars = reinterpret_cast<uint64_t*>(smem + L::kBarriers);
+  uint64_t* const full = bars;                 // producers (and the image's bulk copy) -> MMA
+  uint64_t* const empty = bars + kStages;      // MMA -> producers
+  uint64_t* const acc_full = bars + 2 * kStages;       // MMA -> epilogue
+  uint64_t* const acc_empty = bars + 2 * kStages + 2;  // epilogue -> MMA
+  uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 4);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+
+  if (tid == 0) {
+    for (int s = 0; s < kStages; ++s) { mbar_init(&full[s], kProducerWarps + (kOuter ? 0 : 1)); mbar_init(&empty[s], 1); }
+    for (int s = 0; s < 2; ++s) { mbar_init(&acc_full[s], 1); mbar_init(&acc_empty[s], kEpilogueWarps); }
+    mbar_init_fence();
+  }
+  if (warp == kMmaWarp) tmem_alloc(tmem_slot, L::kTmem);
+  fence_before_sync();
+  __syncthreads();
+  fence_after_sync();
+  const uint32_t tmem = *tmem_slot;
+  bool timed_out = false;
+
+  const int mt = (p.M + kBM - 1) / kBM, nt = (p.N + BN - 1) / BN;
+  const int tiles = mt * nt * p.splits;
+
+  if (warp >= kEpilogueWarps && warp < kMmaWarp) {
+    // ------------------------------------------------------------ producers
+    const int pw = warp - kEpilogueWarps;
+    const int k_images = (p.K + kBK - 1) / kBK;
+    int tile = blockIdx.x;
+    int stage = 0;
+    uint32_t parity = 1;   // a fresh barrier's previous phase counts as complete
+    TileA ta;
+    TileB tb;
+    int m0 = 0, n0 = 0, k0 = 0, k_end = 0;
+    bool a_inner = false, b_inner = false;
+    auto tile_begin = [&](int t) {
+      const int mn = t % (mt * nt), sp = t / (mt * nt);
+      n0 = (mn % nt) * BN;
+      m0 = (mn / nt) * kBM;
+      k0 = sp * p.k_split;
+      k_end = min(p.K, k0 + p.k_split);
+      ta.begin(p.a, p.lda, pw, lane, m0, k0);
+      if (kOuter) tb.begin(p.b, p.ldb, pw, lane, n0, k0);
+    };
+    auto bounds = [&]() {
+      const bool k_in = k0 + kBK <= k_end;
+      a_inner = p.a_wide && k_in && m0 + kBM <= p.M;
+      b_inner = p.b_wide && k_in && n0 + BN <= p.N;
+    };
+    if (tile < tiles) {
+      tile_begin(tile);
+      bounds();
+#pragma unroll
+      for (int i = 0; i < TileA::kTurns; ++i) ta.load(i, a_inner, pw, lane, m0, p.M, k0, k_end);
+      if (kOuter) {
+#pragma unroll
+        for (int i = 0; i < TileB::kTurns; ++i) tb.load(i, b_inner, pw, lane, n0, p.N, k0, k_end);
+      }
+    }
+    while (tile < tiles) {
+      const uint8_t* const image = kOuter ? nullptr : p.image + (static_cast<size_t>(n0 / BN) * k_images + k0 / kBK) * (3 * L::kPlaneB);
+      // the block after this one, whose loads are issued as this one's registers are released
+      k0 += kBK;
+      if (k0 >= k_end) {
+        tile += gridDim.x;
+        if (tile < tiles) tile_begin(tile);
+      } else {
+        ta.advance(p.lda);
+        if (kOuter) tb.advance(p.ldb);
+      }
+      const bool more = tile < tiles;
+      bounds();
+      mbar_wait_flag(&empty[stage], parity, timed_out);
+      uint8_t* const base = smem + stage * L::kStage;
+      if (!kOuter && pw == 0 && lane == 0) {
+        tma::expect_bytes(&full[stage], 3 * L::kPlaneB);
+        tma::load_bulk(base + 3 * L::kPlaneA, image, 3 * L::kPlaneB, &full[stage]);
+      }
+#pragma unroll
+      for (int i = 0; i < TileA::kTurns; ++i) {
+        ta.store(i, base, pw, lane);
+        if (more) ta.load(i, a_inner, pw, lane, m0, p.M, k0, k_end);
+      }
+      if (kOuter) {
+#pragma unroll
+        for (int i = 0; i < TileB::kTurns; ++i) {
+          tb.store(i, base + 3 * L::kPlaneA, pw, lane);
+          if (more) tb.load(i, b_inner, pw, lane, n0, p.N, k0, k_end);
+        }
+      }
+      fence_smem_to_async();
+      __syncwarp();
+      if (lane == 0) arrive(&full[stage]);
+      if (++stage == kStages) { stage = 0; parity ^= 1; }
+    }
+  } else if (warp == kMmaWarp) {
+    // ------------------------------------------------------------ tensor core
+    const bool leader = elect_one();
+    const uint32_t idesc = idesc_bf16(kBM, BN, kOuter, kOuter);
+    int stage = 0;
+    uint32_t parity = 0;
+    int turn = 0;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+      const int sp = tile / (mt * nt);
+      const int k_len = min(p.K, (sp + 1) * p.k_split) - sp * p.k_split;
+      for (int seg = 0; seg < k_len; seg += kSegment, ++turn) {
+        const int blocks = (min(k_len - seg, kSegment) + kBK - 1) / kBK;
+        const int buf = turn % L::kAccs;
+        mbar_wait_flag(&acc_empty[buf], ((turn / L::kAccs) & 1) ^ 1, timed_out);
+        fence_after_sync();
+        const uint32_t acc = tmem + buf * 2 * BN, acc_small = acc + BN;
+        for (int kb = 0; kb < blocks; ++kb) {
+          mbar_wait_flag(&full[stage], parity, timed_out);
+          fence_after_sync();
+          const uint32_t sa = smem_u32(smem + stage * L::kStage), sb = sa + 3 * L::kPlaneA;
+          constexpr uint32_t kRowsA = kOuter ? kBK : kBM, kRowsB = kOuter ? kBK : BN;
+          const Operand a0{sa, kRowsA, kOuter}, a1{sa + L::kPlaneA, kRowsA, kOuter}, a2{sa + 2 * L::kPlaneA, kRowsA, kOuter};
+          const Operand b0{sb, kRowsB, kOuter}, b1{sb + L::kPlaneB, kRowsB, kOuter}, b2{sb + 2 * L::kPlaneB, kRowsB, kOuter};
+          gemm<kBK / 16>(acc_small, a2, b0, idesc, kb > 0, leader);
+          gemm<kBK / 16>(acc_small, a0, b2, idesc, true, leader);
+          gemm<kBK / 16>(acc_small, a1, b1, idesc, true, leader);
+          gemm<kBK / 16>(acc_small, a1, b0, idesc, true, leader);
+          gemm<kBK / 16>(acc_small, a0, b1, idesc, true, leader);
+          gemm<kBK / 16>(acc, a0, b0, idesc, kb > 0, leader);
+          if (leader) commit(&empty[stage]);
+          if (++stage == kStages) { stage = 0; parity ^= 1; }
+        }
+        if (leader) commit(&acc_full[buf]);
+      }
+    }
+    // the last commits may still be on their way to barriers in this CTA's shared memory
+    for (int s = 0; s < kStages; ++s) {
+      mbar_wait_flag(&empty[stage], parity ^ 1, timed_out);
+      if (++stage == kStages) { stage = 0; parity ^= 1; }
+    }
+  } else if (warp < kEpilogueWarps) {
+    // ------------------------------------------------------------ epilogue
+    int turn = 0;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+      const int mn = tile % (mt * nt), sp = tile / (mt * nt);
+      const int n0 = (mn % nt) * BN, m0 = (mn / nt) * kBM;
+      const int m = m0 + (warp & 3) * 32 + lane;
+      const bool in = m < p.M;
+      const bool split = p.splits > 1;
+      float* const crow = split ? p.partial + (static_cast<size_t>(sp) * p.M + (in ? m : 0)) * p.N
+                                : p.c + static_cast<long long>(in ? m : 0) * p.ldc;
+      const float* const arow = (p.ep.add && !split) ? p.ep.add + static_cast<long long>(in ? m : 0) * p.ep.ld_add : nullptr;
+      const int k_len = min(p.K, (sp + 1) * p.k_split) - sp * p.k_split;
+      for (int seg = 0; seg < k_len; seg += kSegment, ++turn) {
+        const int buf = turn % L::kAccs;
+        const bool last = seg + kSegment >= k_len;
+        mbar_wait_flag(&acc_full[buf], (turn / L::kAccs) & 1, timed_out);
+        fence_after_sync();
+        const uint32_t src = tmem + buf * 2 * BN + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+#pragma unroll 1
+        for (int c = (warp >> 2) * (BN / kColumnParts); c < ((warp >> 2) + 1) * (BN / kColumnParts); c += 32) {
+          if (n0 + c >= p.N) break;
+          float v[32], w[32];
+          __syncwarp();
+          tmem_ld32(src + c, v);
+          tmem_ld32(src + BN + c, w);
+          tmem_ld_wait();
+#pragma unroll
+          for (int e = 0; e < 32; ++e) v[e] += w[e];
+#pragma unroll
+          for (int g = 0; g < 4; ++g) {
+            const int n = n0 + c + g * 8, valid = in ? p.N - n : 0;
+            if (valid <= 0) continue;
+            float ad[8];
+            if (seg > 0) {   // this thread's own earlier segment of the contraction
+              load8_own(crow + n, valid, p.c_vec, ad);
+#pragma unroll
+              for (int e = 0; e < 8; ++e) v[g * 8 + e] += ad[e];
+            }
+            if (last && !split && p.ep.bias) {
+#pragma unroll
+              for (int e = 0; e < 8; ++e)
+                if (e < valid) v[g * 8 + e] += __ldg(p.ep.bias + n + e);
+            }
+            if (last && arow) {
+              load8(arow + n, valid, p.ep_vec, ad);
+#pragma unroll
+              for (int e = 0; e < 8; ++e)
+                v[g * 8 + e] = fmaf(ad[e], (p.ep.add_scale && e < valid) ? __ldg(p.ep.add_scale + n + e) : 1.f, v[g * 8 + e]);
+            }
+            store8(crow + n, valid, p.c_vec, v + g * 8);
+          }
+        }
+        fence_before_sync();
+        __syncwarp();
+        if (lane == 0) arrive(&acc_empty[buf]);
+      }
+    }
+  }
+
+  if (timed_out && p.status) atomicExch(p.status, 1);
+  fence_before_sync();
+  __syncthreads();
+  if (warp == kMmaWarp) tmem_dealloc(tmem, L::kTmem);
+}
+
+// C = sum over splits of the partial products (fixed order: bit-reproducible) + epilogue
+__global__ void __launch_bounds__(256) reduce_splits_kernel(const float* __restrict__ partial, int splits, int M, int N,
+                                                            float* __restrict__ c, long long ldc, Epilogue ep) {
+  const long long n_all = static_cast<long long>(M) * N;
+  const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
+  if (i >= n_all) return;
+  float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+  int s = 0;
+  for (; s + 4 <= splits; s += 4) {
+    s0 += partial[(s + 0) * n_all + i];
+    s1 += partial[(s + 1) * n_all + i];
+    s2 += partial[(s + 2) * n_all + i];
+    s3 += partial[(s + 3) * n_all + i];
+  }
+  for (; s < splits; ++s) s0 += partial[s * n_all + i];
+  float acc = (s0 + s1) + (s2 + s3);
+  const int m = static_cast<int>(i / N), n = static_cast<int>(i % N);
+  if (ep.bias) acc += ep.bias[n];
+  if (ep.add) acc = fmaf(ep.add[m * ep.ld_add + n], ep.add_scale ? ep.add_scale[n] : 1.f, acc);
+  c[m * ldc + n] = acc;
+}
+
+int vec_of(const void* p, long long ld) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+  if (a % 32 == 0 && ld % 8 == 0) return 8;
+  if (a % 16 == 0 && ld % 4 == 0) return 4;
+  return 1;
+}
+
+// Width of a tile and how often the contraction is split: a tile of 256 columns halves the shared-memory traffic per
+// product, but only where enough tiles are left to give every SM one; a contraction is split when even the narrowest
+// tiles leave SMs idle and each part still has enough steps to fill the pipeline (8 stages of 32).
+struct Plan {
+  int bn, splits, k_split;
+};
+Plan plan(int M, int N, int K) {
+  const int mt = (M + kBM - 1) / kBM;
+  Plan pl{256, 1, 0};
+  const auto tiles = [&](int bn) { return static_cast<long long>(mt) * ((N + bn - 1) / bn); };
+  const int kblocks = (K + kBK - 1) / kBK;
+  if (N <= 64) pl.bn = 64;
+  else if (N <= 128) pl.bn = 128;
+  int max_splits = max(1, kblocks / 8);
+  // without enough k to split, narrower tiles are the only way to occupy more SMs
+  while (pl.bn > 64 && tiles(pl.bn) * max_splits < kNumSMs) pl.bn /= 2;
+  const long long t = tiles(pl.bn);
+  if (t < kNumSMs && max_splits > 1) {
+    pl.splits = static_cast<int>(min(static_cast<long long>(max_splits), kNumSMs / t));
+    if (pl.splits < 1) pl.splits = 1;
+  }
+  const int per = (kblocks + pl.splits - 1) / pl.splits;
+  pl.k_split = per * kBK;
+  pl.splits = (kblocks + per - 1) / per;
+  return pl;
+}
+
+template <int BN, bool kOuter>
+int launch(const Params& p, int tiles, cudaStream_t stream) {
+  if (const int st = allow_smem<gemm32_kernel<BN, kOuter>>(Layout<BN>::kBytes); st != MXK_OK) return st;
+  gemm32_kernel<BN, kOuter><<<min(tiles, kNumSMs), Roles<BN, kOuter>::kThreads, Layout<BN>::kBytes, stream>>>(p);
+  return launch_status();
+}
+
+template <bool kOuter>
+int run(Params& p, float* ws, size_t ws_bytes, int* partials, cudaStream_t stream) {
+  const Plan pl = plan(p.M, p.N, p.K);
+  if (pl.splits > 1 && (!ws || ws_bytes < static_cast<size_t>(pl.splits) * p.M * p.N * sizeof(float))) return MXK_ERR_WORKSPACE;
+  p.k_split = pl.k_split;
+  p.splits = pl.splits;
+  p.partial = ws;
+  p.c_vec = pl.splits > 1 ? vec_of(ws, p.N) : vec_of(p.c, p.ldc);
+  p.ep_vec = p.ep.add ? vec_of(p.ep.add, p.ep.ld_add) : 1;
+  p.a_wide = vec_of(p.a, p.lda) == 8;
+  p.b_wide = kOuter && vec_of(p.b, p.ldb) == 8;
+  const int tiles = ((p.M + kBM - 1) / kBM) * ((p.N + pl.bn - 1) / pl.bn) * pl.splits;
+  const int st = pl.bn == 256   ? launch<256, kOuter>(p, tiles, stream)
+                 : pl.bn == 128 ? launch<128, kOuter>(p, tiles, stream)
+                                : launch<64, kOuter>(p, tiles, stream);
+  if (partials) *partials = pl.splits;
+  if (st != MXK_OK || pl.splits == 1 || partials) return st;
+  const long long n_all = static_cast<long long>(p.M) * p.N;
+  reduce_splits_kernel<<<static_cast<unsigned>((n_all + 255) / 256), 256, 0, stream>>>(ws, pl.splits, p.M, p.N, p.c, p.ldc, p.ep);
+  return launch_status();
+}
+
+struct SplitParams {
+  WeightJob job[4];
+  int first_block[6];   // of the four images and of lambda; past the last block for what is not asked for
+  LambdaJob lambda;
+};
+
+// One thread per eight k of a weight row: reads them (zero past the matrix), writes one vector of each plane.
+__global__ void __launch_bounds__(256) split_weights_kernel(const __grid_constant__ SplitParams sp) {
+  int j = 0;
+  while (static_cast<int>(blockIdx.x) >= sp.first_block[j + 1]) ++j;
+  if (j == 4) {
+    const int n = (blockIdx.x - sp.first_block[4]) * 256 + threadIdx.x;
+    if (n < sp.lambda.N) {
+      const float r = expf(-expf(sp.lambda.nu_log[n]));
+      float s, c;
+      sincosf(expf(sp.lambda.theta_log[n]), &s, &c);
+      reinterpret_cast<float2*>(sp.lambda.lambda)[n] = make_float2(r * c, r * s);
+    }
+    return;
+  }
+  const WeightJob& jb = sp.job[j];
+  const int bn = jb.bn, kb = (jb.K + kBK - 1) / kBK;
+  const long long id = static_cast<long long>(blockIdx.x - sp.first_block[j]) * 256 + threadIdx.x;
+  // id = ((n_tile * kb + k_block) * 4 + k_group) * bn + n: consecutive threads write consecutive vectors
+  const int n_in = static_cast<int>(id % bn);
+  const long long rest = id / bn;
+  const int kg = static_cast<int>(rest & 3), k_block = static_cast<int>((rest >> 2) % kb);
+  const int n_tile = static_cast<int>((rest >> 2) / kb);
+  if (n_tile * bn >= jb.N) return;
+  const int n = n_tile * bn + n_in, k = k_block * kBK + kg * 8;
+  const auto at = [&](int row, int col) -> float {
+    if (jb.w.form == Form::kComplexRows)
+      return jb.w.ptr[row & 1][static_cast<long long>(row >> 1) * jb.w.ld + col] * (jb.w.log_scale ? expf(jb.w.log_scale[row >> 1]) : 1.f);
+    if (jb.w.form == Form::kComplexCols) {
+      const float v = jb.w.ptr[col & 1][static_cast<long long>(row) * jb.w.ld + (col >> 1)];
+      return (col & 1) ? -v : v;
+    }
+    int start = 0, s = 0;
+    for (; s < jb.w.count - 1 && row >= jb.w.row_end[s]; ++s) start = jb.w.row_end[s];
+    return jb.w.ptr[s][static_cast<long long>(row - start) * jb.w.ld + col];
+  };
+  float x[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e)
+    x[e] = (n < jb.N && k + e < jb.K) ? (jb.transposed ? at(k + e, n) : at(n, k + e)) : 0.f;
+  uint4 hi, mid, lo;
+  split8(x, hi, mid, lo);
+  uint4* const dst = static_cast<uint4*>(jb.image) + (static_cast<size_t>(n_tile) * kb + k_block) * (3 * bn * 4) + kg * bn + n_in;
+  dst[0] = hi;
+  dst[bn * 4] = mid;
+  dst[2 * bn * 4] = lo;
+}
+
+}  // namespace
+
+int tile_width(int M, int N, int K) { return plan(M, N, K).bn; }
+
+size_t image_bytes(int M, int N, int K) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  const int bn = plan(M, N, K).bn;
+  return static_cast<size_t>((N + bn - 1) / bn) * ((K + kBK - 1) / kBK) * (3 * bn * kBK * 2);
+}
+
+int split_weights(const WeightJob* jobs, int count, const LambdaJob& lambda, cudaStream_t stream) {
+  if (count < 0 || count > 4) return MXK_ERR_DIMS;
+  SplitParams sp{};
+  for (int j = 0; j < count; ++j) {
+    const WeightJob& jb = jobs[j];
+    if (!jb.image || jb.w.count < 1) return MXK_ERR_NULL;
+    if (!aligned16(jb.image)) return MXK_ERR_ALIGN;
+    sp.job[j] = jb;
+    const long long vectors = static_cast<long long>((jb.N + jb.bn - 1) / jb.bn) * jb.bn * ((jb.K + kBK - 1) / kBK) * 4;
+    sp.first_block[j + 1] = sp.first_block[j] + static_cast<int>((vectors + 255) / 256);
+  }
+  for (int j = count; j < 4; ++j) sp.first_block[j + 1] = sp.first_block[count];
+  const int blocks = sp.first_block[4] + (lambda.N + 255) / 256;
+  sp.first_block[5] = 0x7fffffff;
+  sp.lambda = lambda;
+  if (blocks == 0) return MXK_OK;
+  split_weights_kernel<<<blocks, 256, 0, stream>>>(sp);
+  return launch_status();
+}
+
+size_t workspace_bytes(int M, int N, int K) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  const Plan pl = plan(M, N, K);
+  return pl.splits > 1 ? static_cast<size_t>(pl.splits) * M * N * sizeof(float) : 0;
+}
+
+int run_weights(const float* a, long long lda, const void* image, float* c, long long ldc, int M, int N, int K,
+                const Epilogue& ep, float* ws, size_t ws_bytes, int* status, cudaStream_t stream) {
+  if (!a || !image || !c) return MXK_ERR_NULL;
+  if (M <= 0 || N <= 0 || K <= 0) return MXK_ERR_DIMS;
+  if (!aligned16(image)) return MXK_ERR_ALIGN;
+  Params p{};
+  p.a = a; p.lda = lda;
+  p.image = static_cast<const uint8_t*>(image);
+  p.c = c; p.ldc = ldc;
+  p.M = M; p.N = N; p.K = K;
+  p.ep = ep;
+  p.status = status;
+  return run<false>(p, ws, ws_bytes, nullptr, stream);
+}
+
+int run_outer(const float* a, long long lda, const float* b, long long ldb, float* c, long long ldc, int M, int N, int K,
+              float* ws, size_t ws_bytes, int* partials, int* status, cudaStream_t stream) {
+  if (!a || !b || !c) return MXK_ERR_NULL;
+  if (M <= 0 || N <= 0 || K <= 0) return MXK_ERR_DIMS;
+  Params p{};
+  p.a = a; p.lda = lda;
+  p.b = b; p.ldb = ldb;
+  p.c = c; p.ldc = ldc;
+  p.M = M; p.N = N; p.K = K;
+  p.status = status;
+  return run<true>(p, ws, ws_bytes, partials, stream);
+}
+
+}  // namespace gemm32
+}  // namespace mxk

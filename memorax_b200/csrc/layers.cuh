@@ -1,0 +1,42 @@
+// Kernels of whole layers around the scans (host-side interface): what a cell does besides its recurrence and the
+// large matrix products.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "mxk.h"
+
+namespace mxk {
+namespace layers {
+
+// ---- complex-diagonal layer (LRU), lru.cu -------------------------------------------------------------------
+struct LruWeights {
+  const float *nu_log, *theta_log, *gamma_log;   // (N)
+  const float *b_re, *b_im;                      // (N, F)
+  const float *c_re, *c_im;                      // (F, N)
+  const float* d;                                // (F)
+};
+// One time step of `B` sequences: h (B, N) complex, y (B, F); h0 / a0 / done / a_last may be null.
+int lru_step(const LruWeights& w, const float* x, const float* h0, const float* a0, const uint8_t* done, float* h,
+             float* a_last, float* y, int B, int F, int N, cudaStream_t stream);
+
+// Sum over the rows of gy * x, (rows, F) each, left as `*blocks` partial rows of F in `partial` (lru_skip_blocks rows).
+int skip_grad_blocks(long long rows);
+int skip_grad(const float* gy, const float* x, float* partial, long long rows, int F, cudaStream_t stream);
+
+// Gradients of the parameters from those of the real projection matrices (partial products of split contractions) and
+// of lambda (torch's complex convention).
+struct LruGrads {
+  const float* in_partial;    // [in_splits][2N][F]
+  const float* out_partial;   // [out_splits][F][2N]
+  const float* skip_partial;  // [skip_blocks][F]
+  const float* lambda;        // (N) complex, and its cotangent
+  const float* g_lambda;
+  int in_splits, out_splits, skip_blocks;
+  float *g_nu, *g_theta, *g_gamma, *g_b_re, *g_b_im, *g_c_re, *g_c_im, *g_d;
+};
+int lru_param_grads(const LruWeights& w, const LruGrads& g, int F, int N, cudaStream_t stream);
+
+}  // namespace layers
+}  // namespace mxk

@@ -1,0 +1,203 @@
+// The LRU layer's own kernels: a fused single time step (acting), and the gradients of its parameters from those of the
+// real projection matrices.
+#include "layers.cuh"
+#include "mxk_common.cuh"
+#include "warp_tile.cuh"
+
+namespace mxk {
+namespace layers {
+namespace {
+
+// One time step of a few sequences is two matrix-vector-like products over weights that fit L2: launch latency and the
+// depth of the memory pipeline are what counts, so every warp computes eight sequences x four outputs with its lanes
+// across the contraction (the 12 loads of an iteration are independent), and nothing but the state makes a round trip
+// through memory between the two launches.  (16 sequences, F = 128, N = 256: 25 launches, 250 us on the host -> 2.)
+__global__ void __launch_bounds__(128) lru_step_state_kernel(LruWeights w, const float* __restrict__ x,
+                                                             const float* __restrict__ h0, const float* __restrict__ a0,
+                                                             const uint8_t* __restrict__ done, float* __restrict__ h,
+                                                             float* __restrict__ a_last, int B, int F, int N) {
+  const int lane = threadIdx.x & 31, warp = blockIdx.x * 4 + (threadIdx.x >> 5);
+  const int units = (N + 1) / 2;
+  const int n0 = (warp % units) * 2, m0 = (warp / units) * 8;
+  if (m0 >= B) return;
+  WarpTile acc;
+  const float* rows[4] = {w.b_re + static_cast<size_t>(n0) * F, w.b_im + static_cast<size_t>(n0) * F,
+                          w.b_re + static_cast<size_t>(min(n0 + 1, N - 1)) * F, w.b_im + static_cast<size_t>(min(n0 + 1, N - 1)) * F};
+  acc.accumulate(x + static_cast<size_t>(m0) * F, F, min(8, B - m0), rows, F, lane);
+  const float v = acc.reduce(lane);
+  // this lane: sequence m, component j & 1 of unit n
+  const int m = m0 + (lane >> 2), n = n0 + ((lane >> 1) & 1), im = lane & 1;
+  if (m >= B || n >= N) return;
+  const float bu = v * expf(w.gamma_log[n]);
+  const float r = expf(-expf(w.nu_log[n]));
+  float s, c;
+  sincosf(expf(w.theta_log[n]), &s, &c);
+  const float lre = r * c, lim = r * s;
+  const bool reset = done && done[m] != 0;
+  const size_t at = static_cast<size_t>(m) * N + n;
+  const float2 hp = h0 ? reinterpret_cast<const float2*>(h0)[at] : make_float2(0.f, 0.f);
+  // (the terms of a complex product in the recurrence kernels' order)
+  float out = im ? fmaf(lre, hp.y, fmaf(lim, hp.x, bu)) : fmaf(lre, hp.x, fmaf(-lim, hp.y, bu));
+  if (reset) out = bu;
+  h[2 * at + im] = out;
+  if (a_last) {
+    const float2 ap = (a0 && !reset) ? reinterpret_cast<const float2*>(a0)[at] : make_float2(1.f, 0.f);
+    a_last[2 * at + im] = im ? lre * ap.y + lim * ap.x : lre * ap.x - lim * ap.y;
+  }
+}
+
+__global__ void __launch_bounds__(128) lru_step_read_kernel(LruWeights w, const float* __restrict__ x,
+                                                            const float* __restrict__ h, float* __restrict__ y, int B,
+                                                            int F, int N) {
+  const int lane = threadIdx.x & 31, warp = blockIdx.x * 4 + (threadIdx.x >> 5);
+  const int units = (F + 3) / 4;
+  const int f0 = (warp % units) * 4, m0 = (warp / units) * 8;
+  if (m0 >= B) return;
+  const int mv = min(8, B - m0);
+  WarpTile acc;
+  for (int n = lane; n < N; n += 32) {
+    float2 hv[8];
+    float cr[4], ci[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const size_t row = static_cast<size_t>(min(f0 + j, F - 1)) * N + n;
+      cr[j] = __ldg(w.c_re + row);
+      ci[j] = __ldg(w.c_im + row);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      hv[i] = reinterpret_cast<const float2*>(h)[static_cast<size_t>(m0 + min(i, mv - 1)) * N + n];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc.v[i * 4 + j] = fmaf(hv[i].x, cr[j], fmaf(-hv[i].y, ci[j], acc.v[i * 4 + j]));
+  }
+  const float v = acc.reduce(lane);
+  const int m = m0 + (lane >> 2), f = f0 + (lane & 3);
+  if (m >= B || f >= F) return;
+  const size_t at = static_cast<size_t>(m) * F + f;
+  y[at] = fmaf(x[at], w.d[f], v);
+}
+
+constexpr int kSkipBlocks = 2 * kNumSMs;
+
+// HBM-bound: one read of both operands; a block takes every gridDim.x-th group of rows, its threads the columns.
+__global__ void __launch_bounds__(256) skip_grad_kernel(const float* __restrict__ gy, const float* __restrict__ x,
+                                                        float* __restrict__ partial, long long rows, int F) {
+  __shared__ float sums[256];
+  const int per = F < 256 ? 256 / F : 1;   // rows side by side in a block
+  const int width = min(F, 256);
+  const int ro = threadIdx.x / width, ct = threadIdx.x % width;
+  for (int c0 = 0; c0 < F; c0 += 256) {
+    const int c = c0 + ct;
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+    if (ro < per && c < F) {
+      const long long step = static_cast<long long>(gridDim.x) * per;
+      long long r = static_cast<long long>(blockIdx.x) * per + ro;
+      for (; r + 3 * step < rows; r += 4 * step) {
+        float a[4], b[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          a[u] = ld_stream(gy + (r + u * step) * F + c);
+          b[u] = ld_stream(x + (r + u * step) * F + c);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) s[u] = fmaf(a[u], b[u], s[u]);
+      }
+      for (; r < rows; r += step) s[0] = fmaf(gy[r * F + c], x[r * F + c], s[0]);
+    }
+    __syncthreads();
+    sums[threadIdx.x] = (s[0] + s[1]) + (s[2] + s[3]);
+    __syncthreads();
+    if (ro == 0 && c < F) {
+      float v = 0.f;
+      for (int i = 0; i < per; ++i) v += sums[i * width + ct];
+      partial[static_cast<size_t>(blockIdx.x) * F + c] = v;
+    }
+  }
+}
+
+// Blocks 0..N-1: hidden unit n (its rows of the input projection, and lambda); N..N+F-1: feature f (its row of the
+// read-out and its skip weight).  Sums over splits run in a fixed order.
+__global__ void __launch_bounds__(128) lru_param_grads_kernel(LruWeights w, LruGrads g, int F, int N) {
+  __shared__ float red[128];
+  const int tid = threadIdx.x;
+  const auto block_sum = [&](float v) {
+    red[tid] = v;
+    __syncthreads();
+    for (int o = 64; o > 0; o >>= 1) {
+      if (tid < o) red[tid] += red[tid + o];
+      __syncthreads();
+    }
+    return red[0];
+  };
+  if (static_cast<int>(blockIdx.x) < N) {
+    const int n = blockIdx.x;
+    const float scale = expf(w.gamma_log[n]);
+    const size_t plane = static_cast<size_t>(2) * N * F;
+    float dot = 0.f;
+    for (int f = tid; f < F; f += 128) {
+      float re = 0.f, im = 0.f;
+      const float* p = g.in_partial + static_cast<size_t>(2) * n * F + f;
+#pragma unroll 4
+      for (int s = 0; s < g.in_splits; ++s) { re += p[s * plane]; im += p[s * plane + F]; }
+      re *= scale;
+      im *= scale;
+      const size_t at = static_cast<size_t>(n) * F + f;
+      g.g_b_re[at] = re;
+      g.g_b_im[at] = im;
+      dot += re * w.b_re[at] + im * w.b_im[at];
+    }
+    dot = block_sum(dot);
+    if (tid == 0) {
+      g.g_gamma[n] = dot;
+      // lambda = exp(-e^nu + i e^theta); with cotangent G (torch's convention): dL = Re(conj(G) dlambda)
+      const float2 l = reinterpret_cast<const float2*>(g.lambda)[n], gl = reinterpret_cast<const float2*>(g.g_lambda)[n];
+      g.g_nu[n] = -expf(w.nu_log[n]) * (gl.x * l.x + gl.y * l.y);
+      g.g_theta[n] = expf(w.theta_log[n]) * (gl.y * l.x - gl.x * l.y);
+    }
+  } else {
+    const int f = blockIdx.x - N;
+    const size_t plane = static_cast<size_t>(2) * N * F;
+    for (int n = tid; n < N; n += 128) {
+      float re = 0.f, im = 0.f;
+      const float2* p = reinterpret_cast<const float2*>(g.out_partial + static_cast<size_t>(f) * 2 * N) + n;
+#pragma unroll 4
+      for (int s = 0; s < g.out_splits; ++s) { const float2 v = p[s * (plane / 2)]; re += v.x; im += v.y; }
+      const size_t at = static_cast<size_t>(f) * N + n;
+      g.g_c_re[at] = re;
+      g.g_c_im[at] = -im;
+    }
+    float s = 0.f;
+    for (int b = tid; b < g.skip_blocks; b += 128) s += g.skip_partial[static_cast<size_t>(b) * F + f];
+    s = block_sum(s);
+    if (tid == 0) g.g_d[f] = s;
+  }
+}
+
+}  // namespace
+
+int lru_step(const LruWeights& w, const float* x, const float* h0, const float* a0, const uint8_t* done, float* h,
+             float* a_last, float* y, int B, int F, int N, cudaStream_t stream) {
+  if (B <= 0 || F <= 0 || N <= 0) return MXK_ERR_DIMS;
+  const long long groups = (B + 7) / 8;
+  const long long warps_h = groups * ((N + 1) / 2), warps_y = groups * ((F + 3) / 4);
+  lru_step_state_kernel<<<static_cast<unsigned>((warps_h + 3) / 4), 128, 0, stream>>>(w, x, h0, a0, done, h, a_last, B, F, N);
+  lru_step_read_kernel<<<static_cast<unsigned>((warps_y + 3) / 4), 128, 0, stream>>>(w, x, h, y, B, F, N);
+  return launch_status();
+}
+
+int skip_grad_blocks(long long rows) { return static_cast<int>(rows < kSkipBlocks ? rows : kSkipBlocks); }
+
+int skip_grad(const float* gy, const float* x, float* partial, long long rows, int F, cudaStream_t stream) {
+  skip_grad_kernel<<<skip_grad_blocks(rows), 256, 0, stream>>>(gy, x, partial, rows, F);
+  return launch_status();
+}
+
+int lru_param_grads(const LruWeights& w, const LruGrads& g, int F, int N, cudaStream_t stream) {
+  lru_param_grads_kernel<<<N + F, 128, 0, stream>>>(w, g, F, N);
+  return launch_status();
+}
+
+}  // namespace layers
+}  // namespace mxk

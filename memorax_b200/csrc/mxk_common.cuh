@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "mxk.h"
 
 namespace mxk {
@@ -15,6 +17,21 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 inline int launch_status() {
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? MXK_OK : static_cast<int>(e);
+}
+
+// Raises a kernel's dynamic shared memory limit, once per kernel and device (the call costs as much as a launch).
+template <auto kKernel>
+inline int allow_smem(int bytes) {
+  static std::atomic<uint64_t> done{0};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return static_cast<int>(e);
+  const uint64_t bit = dev < 64 ? 1ull << dev : 0;
+  if (done.load(std::memory_order_acquire) & bit) return MXK_OK;
+  e = cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e != cudaSuccess) return static_cast<int>(e);
+  done.fetch_or(bit, std::memory_order_release);
+  return MXK_OK;
 }
 
 // 16-byte streaming accesses: data that is touched once should not displace

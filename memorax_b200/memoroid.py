@@ -28,7 +28,7 @@ import torch
 from torch import nn
 from torch.nn import functional as F
 
-from . import ops
+from . import _C, ops
 
 
 def get_input_shape(inputs):
@@ -72,6 +72,10 @@ class MemoroidCellBase(nn.Module):
         """-> (next_carry, y)"""
         raise NotImplementedError
 
+    def layer(self, inputs, done, initial_carry, **kwargs):
+        """The whole layer, -> (next_carry, y): the elements, then ``scan``.  Cells with a fused form override it."""
+        return self.scan(self(inputs, **kwargs), initial_carry, done, inputs)
+
     # ---- RTRL hooks (memoroid.py:35-54); a cell without local Jacobians returns None ----
     def local_jacobian(self, carry, z, inputs, **kwargs):
         return None
@@ -114,9 +118,7 @@ class Memoroid(SequenceModel):
     def forward(self, inputs, done, initial_carry=None, **kwargs):
         # initial_carry=None means the cell's initialize_carry() value (memoroid.py:101-103);
         # the kernels take that default as NULL pointers, so it is never materialised.
-        z = self.cell(inputs, **kwargs)
-        next_carry, y = self.cell.scan(z, initial_carry, done, inputs)
-        return next_carry, y
+        return self.cell.layer(inputs, done, initial_carry, **kwargs)
 
     def initialize_carry(self, key, input_shape):
         return self.cell.initialize_carry(key, input_shape)
@@ -197,7 +199,7 @@ def _project_to_complex(x, w):
     interleaved (re_0, im_0, re_1, ...), so the (B,T,2N) product is the complex64 result in memory."""
     n, f = w.shape
     w2 = torch.view_as_real(w).permute(0, 2, 1).reshape(2 * n, f)
-    out = F.linear(x.float(), w2)
+    out = _C.linear_f32(x.float(), w2)
     return torch.view_as_complex(out.view(*out.shape[:-1], n, 2))
 
 
@@ -207,7 +209,7 @@ def _read_real_part(h, c):
     f, n = c.shape
     w2 = torch.stack([c.real, -c.imag], dim=-1).reshape(f, 2 * n)
     hr = torch.view_as_real(h)
-    return F.linear(hr.reshape(*hr.shape[:-2], 2 * n), w2)
+    return _C.linear_f32(hr.reshape(*hr.shape[:-2], 2 * n), w2)
 
 
 class _ComplexDiagonalCell(MemoroidCellBase):
@@ -245,6 +247,9 @@ class _ComplexDiagonalCell(MemoroidCellBase):
 
 
 # ---------------------------------------------------------------------- LRU
+_LRU_PARAMS = ("nu_log", "theta_log", "gamma_log", "B_real", "B_imag", "C_real", "C_imag", "D")
+
+
 class LRUCell(_ComplexDiagonalCell):
     """Complex diagonal linear recurrence with time-invariant decay (lru.py:32-108)."""
 
@@ -261,6 +266,16 @@ class LRUCell(_ComplexDiagonalCell):
         self.C_real = nn.Parameter(torch.randn(features, hidden_dim) / math.sqrt(hidden_dim))
         self.C_imag = nn.Parameter(torch.randn(features, hidden_dim) / math.sqrt(hidden_dim))
         self.D = nn.Parameter(torch.randn(features))
+
+    def layer(self, inputs, done, initial_carry, **kwargs):
+        """Projections, scan and read-out as one native call (float32); its backward pass is one autograd node.  A
+        subclass, or a call the fused layer does not cover, is composed from its parts."""
+        if type(self) is LRUCell and not kwargs:
+            h0, a0 = (None, None) if initial_carry is None else initial_carry
+            out = _C.lru_layer(inputs, [self._parameters[name] for name in _LRU_PARAMS], h0, a0, done)
+            if out is not None:
+                return (out[0], out[1]), out[2]
+        return super().layer(inputs, done, initial_carry, **kwargs)
 
     def diag_lambda(self):
         return torch.exp(torch.complex(-torch.exp(self.nu_log), torch.exp(self.theta_log)))

@@ -12,7 +12,7 @@ import ctypes
 import torch
 from torch.nn import functional as F
 
-from . import _lib
+from . import _C, _lib
 
 
 # ------------------------------------------------------------------ helpers
@@ -54,23 +54,7 @@ def linrec_fwd(a, b, h0=None, a0=None, done=None, want_decay=True):
     """h_t = done_t ? b_t : a_t h_{t-1} + b_t over (B,T,D); ``a`` is (B,T,D) or a
     time-invariant (D,).  Returns ``(h, a_last)`` (a_last None unless wanted).
     float32 or complex64, chosen by ``b.dtype``."""
-    cplx = b.is_complex()
-    dt = torch.complex64 if cplx else torch.float32
-    b = _dev(b, dt, "b")
-    a = _dev(a, dt, "a")
-    h0, a0 = _dev(h0, dt, "h0"), _dev(a0, dt, "a0")
-    bsz, steps, dim = b.shape
-    tinv = a.dim() == 1
-    if tinv:
-        assert a.shape == (dim,)
-    else:
-        assert a.shape == b.shape
-    h = torch.empty_like(b)
-    a_last = torch.empty(bsz, dim, dtype=dt, device=b.device) if want_decay else None
-    fn = "mxk_linrec_c64_fwd" if cplx else "mxk_linrec_f32_fwd"
-    _lib.call(fn, _ptr(a), int(tinv), _ptr(b), _ptr(h0), _ptr(a0), _ptr(_done_bytes(done)), _ptr(h),
-              _ptr(a_last), bsz, steps, dim, _stream())
-    return h, a_last
+    return _C.linrec_fwd(a, b, h0, a0, done, want_decay)
 
 
 def linrec_bwd(a, h, h0, done, gh, gh_last=None, need_ga=True, need_gh0=True, conjugate=False):
@@ -276,16 +260,8 @@ class MinGRUFused(torch.autograd.Function):
 # sets it to 1 and drains.  ``check=True`` on a wrapper reads it right after the launch (one host
 # sync); the autograd Functions never sync -- call :func:`check_status` where a sync is affordable
 # (end of a training step, end of a rollout).
-_STATUS_WORDS = {}
-
-
 def _status_word(device):
-    device = torch.device(device)
-    key = device.index if device.index is not None else torch.cuda.current_device()
-    word = _STATUS_WORDS.get(key)
-    if word is None:
-        word = _STATUS_WORDS[key] = torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", key))
-    return word
+    return _C.status_word(str(torch.device(device)))
 
 
 def _check_status(word, what):

@@ -1,0 +1,61 @@
+"""float32 products on the tensor cores (three bf16 terms per operand) and the LRU layer built on them."""
+import pytest
+import torch
+
+from oracle import memoroid_oracle as mo
+
+pytestmark = pytest.mark.gpu
+
+
+# edges of the 128 x {64,128,256} tiles and of the 32-deep stages, split contractions, unaligned rows
+@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (127, 64, 31), (129, 65, 33), (257, 257, 100), (300, 776, 513), (128, 256, 4000),
+                                   (20000, 512, 96)])
+def test_linear_f32_and_its_gradients_match_float64(m, n, k):
+    from memorax_b200 import _C, ops
+    g = torch.Generator("cuda").manual_seed(m + n + k)
+    mk = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    x, w, b, gy = mk(m, k).requires_grad_(), mk(n, k).requires_grad_(), mk(n).requires_grad_(), mk(m, n)
+    y = _C.linear_f32(x, w, b)
+    gx, gw, gb = torch.autograd.grad(y, (x, w, b), gy)
+    xd, wd, gd = x.detach().double(), w.detach().double(), gy.double()
+    for got, want in ((y, xd @ wd.t() + b.detach().double()), (gx, gd @ wd), (gw, gd.t() @ xd), (gb, gd.sum(0))):
+        assert float((got.detach().double() - want).norm() / want.norm()) <= 2e-6
+    ops.check_status()
+
+
+# T = 1 is the fused acting step; odd sizes leave remainders in every tile
+@pytest.mark.parametrize("shape", [(3, 1, 5, 3), (9, 1, 33, 65), (2, 17, 8, 16), (33, 40, 96, 72)])
+@pytest.mark.parametrize("with_carry", [False, True])
+def test_lru_layer_matches_the_oracle(shape, with_carry):
+    from memorax_b200.memoroid import LRUCell, Memoroid
+    bsz, steps, feat, hid = shape
+    torch.manual_seed(0)
+    cell = LRUCell(feat, hid, r_min=0.5, r_max=0.99, max_phase=0.6).cuda()
+    x = torch.randn(bsz, steps, feat, device="cuda", requires_grad=True)
+    done = torch.rand(bsz, steps, device="cuda") < 0.1
+    cplx = lambda *s: torch.view_as_complex(torch.randn(*s, 2, device="cuda"))
+    carry = (cplx(bsz, 1, hid).requires_grad_(), cplx(bsz, 1, hid)) if with_carry else None
+    gy, gl = torch.randn_like(x), cplx(bsz, 1, hid)
+    wrt = [x, *cell.parameters()] + ([carry[0]] if with_carry else [])
+    (h, a), y = Memoroid(cell)(x, done, carry)
+    grads = torch.autograd.grad((y, h), wrt, (gy, gl))
+    with torch.no_grad():
+        (h_n, a_n), y_n = Memoroid(cell)(x, done, carry)
+
+    p = {n: v.detach().cpu().double().requires_grad_() for n, v in cell.named_parameters()}
+    xd = x.detach().cpu().double().requires_grad_()
+    h0 = carry[0].detach().cpu()[:, 0].to(torch.complex128).requires_grad_() if with_carry else None
+    lam = torch.exp(torch.complex(-torch.exp(p["nu_log"]), torch.exp(p["theta_log"])))
+    b_norm = torch.complex(p["B_real"], p["B_imag"]) * torch.exp(p["gamma_log"])[:, None]
+    bu = xd.to(torch.complex128) @ b_norm.t()
+    a0 = carry[1].cpu()[:, 0].to(torch.complex128) if with_carry else None
+    hs, a_ref = mo.linrec_seq(lam, bu, h0 if with_carry else torch.zeros(bsz, hid, dtype=torch.complex128), done.cpu().double(),
+                              *([a0] if with_carry else []))
+    y_ref = (hs @ torch.complex(p["C_real"], p["C_imag"]).t()).real + p["D"] * xd
+    wrt_ref = [xd, *p.values()] + ([h0] if with_carry else [])
+    want = torch.autograd.grad((y_ref, hs[:, -1:]), wrt_ref, (gy.cpu().double(), gl.cpu().to(torch.complex128)))
+    err = lambda got, ref: float((got.detach().cpu().reshape(ref.shape) - ref.detach()).abs().max()) / max(1e-30, float(ref.detach().abs().max()))
+    for got, ref in ((h[:, 0], hs[:, -1]), (h_n[:, 0], hs[:, -1]), (a[:, 0], a_ref), (a_n[:, 0], a_ref), (y, y_ref), (y_n, y_ref)):
+        assert err(got, ref) <= 1e-5
+    for got, ref in zip(grads, want):
+        assert err(got, ref) <= 1e-4
