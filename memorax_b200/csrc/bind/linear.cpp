@@ -34,6 +34,7 @@ struct Linear32 : torch::autograd::Function<Linear32> {
     sizes.back() = N;
     const Tensor y = empty_like_of(x, sizes, at::kFloat);
     product(x, w, false, bias ? ptr(*bias) : nullptr, y, M, N, K);
+    ctx->saved_data["bias"] = bias.has_value();
     ctx->save_for_backward({x, w});
     return y;
   }
@@ -53,7 +54,7 @@ struct Linear32 : torch::autograd::Function<Linear32> {
       const Tensor ws = scratch(x, ws_bytes);
       check("run_outer", g::run_outer(ptr(gy), N, ptr(x), K, ptr(grads[1]), K, N, K, M, ptr(ws), ws_bytes, nullptr, status_ptr(x), stream()));
     }
-    if (ctx->needs_input_grad(2)) grads[2] = gy.reshape({M, N}).sum(0);
+    if (ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(2)) grads[2] = gy.reshape({M, N}).sum(0);
     return grads;
   }
 };

@@ -42,7 +42,7 @@ struct Result {
   Tensor h, a_last, y, lambda;   // h: every state (B, T, N)
 };
 
-Result forward(const Tensor& x, const variable_list& params, const Tensor& h0, const Tensor& a0, const Tensor& done) {
+Result forward(const Tensor& x, const variable_list& params, const Tensor& h0, const Tensor& a0, const Tensor& done, bool keep_lambda = false) {
   const int B = x.size(0), T = x.size(1), F = x.size(2), N = params[0].size(0);
   const auto s = stream();
   const LruWeights w = weights_of(params);
@@ -50,14 +50,14 @@ Result forward(const Tensor& x, const variable_list& params, const Tensor& h0, c
   r.h = empty_like_of(x, {B, T, N}, at::kComplexFloat);
   r.a_last = empty_like_of(x, {B, N}, at::kComplexFloat);
   r.y = empty_like_of(x, x.sizes(), at::kFloat);
-  if (T == 1) {   // acting: two launches, no intermediate but the state
+  if (T == 1 && !keep_lambda) {   // acting: two launches, no intermediate but the state
     check("lru_step", mxk::layers::lru_step(w, ptr(x), ptr(h0), ptr(a0), bytes(done), ptr(r.h), ptr(r.a_last), ptr(r.y), B, F, N, s));
     return r;
   }
   const int M = B * T;
   namespace g = mxk::gemm32;
   Arena mem;
-  const size_t lam = mem.take(8 * N), img_in = mem.take(g::image_bytes(M, 2 * N, F)), img_out = mem.take(g::image_bytes(M, F, 2 * N));
+  const size_t img_in = mem.take(g::image_bytes(M, 2 * N, F)), img_out = mem.take(g::image_bytes(M, F, 2 * N));
   const size_t ws_bytes = std::max(g::workspace_bytes(M, 2 * N, F), g::workspace_bytes(M, F, 2 * N)), ws = mem.take(ws_bytes);
   mem.alloc(x);
   int* const status = status_ptr(x);
@@ -65,7 +65,6 @@ Result forward(const Tensor& x, const variable_list& params, const Tensor& h0, c
   jobs[0] = {input_rows(w, F), false, 2 * N, F, g::tile_width(M, 2 * N, F), mem.at<void>(img_in)};
   jobs[1] = {output_cols(w, N), false, F, 2 * N, g::tile_width(M, F, 2 * N), mem.at<void>(img_out)};
   r.lambda = empty_like_of(x, {N}, at::kComplexFloat);
-  (void)lam;
   check("split_weights", g::split_weights(jobs, 2, LambdaJob{w.nu_log, w.theta_log, ptr(r.lambda), N}, s));
   // the projected inputs become the states in place: every element is read before the scan writes it
   check("run_weights", g::run_weights(ptr(x), F, mem.at<void>(img_in), ptr(r.h), 2 * N, M, 2 * N, F, {}, mem.at(ws), ws_bytes, status, s));
@@ -165,25 +164,35 @@ struct LruLayer : torch::autograd::Function<LruLayer> {
   }
 };
 
-// -> (last state (B,1,N), decay leaf (B,1,N), y (B,T,F)), or None where the call is not one for the fused layer (another
-// dtype, tensors elsewhere, a lower precision asked for): the caller then composes it from its parts.
-pybind11::object lru_layer(const Tensor& x_in, const variable_list& params, const OptTensor& h0_in, const OptTensor& a0_in,
-                           const OptTensor& done_in) {
-  if (!x_in.is_cuda() || x_in.dim() != 3 || x_in.numel() == 0 || !x_in.is_floating_point() || x_in.scalar_type() == at::kDouble ||
-      at::globalContext().allowTF32CuBLAS() || at::autocast::is_autocast_enabled(at::kCUDA) || x_in.numel() > (1ll << 40) ||
-      x_in.size(0) * x_in.size(1) > 0x7fffffff || params[3].dim() != 2 || x_in.size(2) != params[3].size(1))
-    return pybind11::none();
+// Whether a call is one for the native layer; what is not (another dtype, tensors elsewhere, a lower precision asked for)
+// the caller composes from its parts.
+bool native(const Tensor& x, const variable_list& params) {
+  if (!x.is_cuda() || x.dim() != 3 || x.numel() == 0 || !x.is_floating_point() || x.scalar_type() == at::kDouble ||
+      at::globalContext().allowTF32CuBLAS() || at::autocast::is_autocast_enabled(at::kCUDA) ||
+      x.size(0) * x.size(1) > 0x7fffffff || params[3].dim() != 2 || x.size(2) != params[3].size(1))
+    return false;
   for (const Tensor& p : params)
-    if (p.scalar_type() != at::kFloat || p.device() != x_in.device() || !p.is_contiguous()) return pybind11::none();
-  const auto leaf = [&](const OptTensor& t, const char* name) {
-    return t && t->defined() ? dev(t->select(1, 0), at::kComplexFloat, name) : Tensor();
-  };
-  const c10::cuda::CUDAGuard guard(x_in.device());
-  const Tensor x = (x_in.scalar_type() == at::kFloat ? x_in : x_in.to(at::kFloat)).contiguous();
-  const Tensor h0 = leaf(h0_in, "h0"), a0 = leaf(a0_in, "a0"), done = done_bytes(done_in);
+    if (p.scalar_type() != at::kFloat || p.device() != x.device() || !p.is_contiguous()) return false;
+  return true;
+}
+Tensor carry_leaf(const OptTensor& t, const char* name) {
+  return t && t->defined() ? dev(t->select(1, 0), at::kComplexFloat, name) : Tensor();
+}
+bool wants_grad(const Tensor& x, const variable_list& params, const Tensor& h0) {
+  if (!at::GradMode::is_enabled()) return false;
   bool grad = x.requires_grad() || (h0.defined() && h0.requires_grad());
   for (const Tensor& p : params) grad |= p.requires_grad();
-  if (at::GradMode::is_enabled() && grad) {
+  return grad;
+}
+
+// -> (last state (B,1,N), decay leaf (B,1,N), y (B,T,F)), or None
+pybind11::object lru_layer(const Tensor& x_in, const variable_list& params, const OptTensor& h0_in, const OptTensor& a0_in,
+                           const OptTensor& done_in) {
+  if (!native(x_in, params)) return pybind11::none();
+  const c10::cuda::CUDAGuard guard(x_in.device());
+  const Tensor x = (x_in.scalar_type() == at::kFloat ? x_in : x_in.to(at::kFloat)).contiguous();
+  const Tensor h0 = carry_leaf(h0_in, "h0"), a0 = carry_leaf(a0_in, "a0"), done = done_bytes(done_in);
+  if (wants_grad(x, params, h0)) {
     const variable_list out = LruLayer::apply(x, params[0], params[1], params[2], params[3], params[4], params[5], params[6],
                                               params[7], opt(h0), opt(a0), opt(done));
     return pybind11::cast(std::make_tuple(out[0], out[1], out[2]));
@@ -192,8 +201,37 @@ pybind11::object lru_layer(const Tensor& x_in, const variable_list& params, cons
   return pybind11::cast(std::make_tuple(last_state(r.h), r.a_last.unsqueeze(1), r.y));
 }
 
+// One RTRL segment without gradients: -> (last state, decay leaf, y, sensitivities of B_imag, B_real, gamma_log, nu_log,
+// theta_log), or None
+pybind11::object lru_rtrl(const Tensor& x_in, const variable_list& params, const OptTensor& h0_in, const OptTensor& a0_in,
+                          const OptTensor& done_in, const variable_list& sens_in) {
+  if (!native(x_in, params) || sens_in.size() != 5 || x_in.size(0) > 65535) return pybind11::none();
+  const int B = x_in.size(0), T = x_in.size(1), F = x_in.size(2), N = params[0].size(0);
+  const c10::cuda::CUDAGuard guard(x_in.device());
+  const Tensor x = (x_in.scalar_type() == at::kFloat ? x_in : x_in.to(at::kFloat)).contiguous();
+  const Tensor h0 = carry_leaf(h0_in, "h0"), a0 = carry_leaf(a0_in, "a0"), done = done_bytes(done_in);
+  bool grad = wants_grad(x, params, h0);
+  variable_list sens, out;
+  for (int i = 0; i < 5; ++i) {
+    const Tensor& t = sens_in[i];
+    grad |= at::GradMode::is_enabled() && t.requires_grad();
+    if (!t.is_cuda() || (i < 2 ? t.sizes() != at::IntArrayRef({B, 1, N, F}) : t.sizes() != at::IntArrayRef({B, 1, N}))) return pybind11::none();
+    sens.push_back(dev(t, at::kComplexFloat, "sensitivity"));
+    out.push_back(at::empty_like(sens.back()));
+  }
+  if (grad) return pybind11::none();
+  const Result r = forward(x, params, h0, a0, done, true);
+  mxk::layers::LruSensitivities s{ptr(sens[3]), ptr(sens[4]), ptr(sens[2]), ptr(sens[1]), ptr(sens[0]),
+                                  ptr(out[3]), ptr(out[4]), ptr(out[2]), ptr(out[1]), ptr(out[0])};
+  check("lru_sensitivities", mxk::layers::lru_sensitivities(weights_of(params), ptr(r.lambda), ptr(r.h), ptr(h0), ptr(x), bytes(done), s, B, T, F, N, stream()));
+  return pybind11::cast(std::make_tuple(last_state(r.h), r.a_last.unsqueeze(1), r.y, out));
+}
+
 }  // namespace
 
-void bind_lru(pybind11::module_& m) { m.def("lru_layer", &lru_layer); }
+void bind_lru(pybind11::module_& m) {
+  m.def("lru_layer", &lru_layer);
+  m.def("lru_rtrl", &lru_rtrl);
+}
 
 }  // namespace mxk_host

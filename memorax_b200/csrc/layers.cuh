@@ -38,5 +38,14 @@ struct LruGrads {
 };
 int lru_param_grads(const LruWeights& w, const LruGrads& g, int F, int N, cudaStream_t stream);
 
+// RTRL: sensitivities after a segment of T steps from those before it.  h (B, T, N) holds the states, h0 (B, N) the one
+// the segment started from, u (B, T, F) the inputs; each sensitivity (B, N) or (B, N, F) complex, in and out.
+struct LruSensitivities {
+  const float *nu, *theta, *gamma, *b_re, *b_im;
+  float *nu_out, *theta_out, *gamma_out, *b_re_out, *b_im_out;
+};
+int lru_sensitivities(const LruWeights& w, const float* lambda, const float* h, const float* h0, const float* u,
+                      const uint8_t* done, const LruSensitivities& s, int B, int T, int F, int N, cudaStream_t stream);
+
 }  // namespace layers
 }  // namespace mxk

@@ -175,6 +175,151 @@ __global__ void __launch_bounds__(128) lru_param_grads_kernel(LruWeights w, LruG
   }
 }
 
+// ------------------------------------------------------------------------------------------------ sensitivities
+// Every leaf obeys S_t = done_t ? J_t : lambda S_{t-1} + J_t with local Jacobians that are never formed here:
+//   nu, theta  J = -e^nu q, i e^theta q with q_t = lambda h_{t-1} (zero where step t resets)
+//   gamma      J = B u: the recurrence of the states themselves from another start, S_T = h_T + P (S_0 - h_0)
+//   B          J = gamma_n u_f and i gamma_n u_f: S_T = P S_0 + gamma_n W, W[n][f] = sum over t >= r of lambda_n^(T-1-t) u_t[f]
+// with r the last reset of the segment and P = lambda^T without one, else 0.
+
+__device__ __forceinline__ int last_reset(const uint8_t* drow, int T) {   // -1 without one; whole block
+  __shared__ int found;
+  if (threadIdx.x == 0) found = -1;
+  __syncthreads();
+  if (drow) {
+    int r = -1;
+    for (int t = threadIdx.x; t < T; t += blockDim.x)
+      if (drow[t]) r = t;
+    if (r >= 0) atomicMax(&found, r);
+  }
+  __syncthreads();
+  return found;
+}
+
+// lambda^k of the float32 lambda, multiplied up in double
+__device__ __forceinline__ float2 power(float2 l, int k) {
+  double br = l.x, bi = l.y, r = 1.0, i = 0.0;
+  for (; k > 0; k >>= 1) {
+    if (k & 1) {
+      const double t = r * br - i * bi;
+      i = r * bi + i * br;
+      r = t;
+    }
+    const double t = br * br - bi * bi;
+    bi = 2.0 * br * bi;
+    br = t;
+  }
+  return make_float2(static_cast<float>(r), static_cast<float>(i));
+}
+__device__ __forceinline__ float2 cmul(float2 a, float2 b) { return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
+__device__ __forceinline__ float2 cmul_add(float2 a, float2 b, float2 c) {
+  return make_float2(fmaf(a.x, b.x, fmaf(-a.y, b.y, c.x)), fmaf(a.x, b.y, fmaf(a.y, b.x, c.y)));
+}
+
+// nu, theta, gamma: one thread per (sequence, unit); latency-bound, so eight states are in flight per thread.
+__global__ void __launch_bounds__(128) lru_sens_units_kernel(LruWeights w, const float* __restrict__ lambda,
+                                                             const float* __restrict__ h, const float* __restrict__ h0,
+                                                             const uint8_t* __restrict__ done, LruSensitivities s, int T, int N) {
+  const int b = blockIdx.y, n = blockIdx.x * 128 + threadIdx.x;
+  const int r = last_reset(done ? done + static_cast<size_t>(b) * T : nullptr, T);
+  if (n >= N) return;
+  const float2* hs = reinterpret_cast<const float2*>(h) + static_cast<size_t>(b) * T * N + n;
+  const size_t at = static_cast<size_t>(b) * N + n;
+  const float2 l = reinterpret_cast<const float2*>(lambda)[n];
+  const float2 start = h0 ? reinterpret_cast<const float2*>(h0)[at] : make_float2(0.f, 0.f);
+  // R_t = lambda R_{t-1} + lambda h_{t-1} from step r + 1 on (R = 0 at a reset), or from the carried state
+  float2 acc = make_float2(0.f, 0.f);
+  if (r < 0) acc = cmul(l, start);
+  constexpr int kDeep = 8;
+  for (int t0 = r < 0 ? 1 : r + 1; t0 < T; t0 += kDeep) {
+    float2 prev[kDeep];
+#pragma unroll
+    for (int u = 0; u < kDeep; ++u)
+      if (t0 + u < T) prev[u] = __ldg(hs + static_cast<size_t>(t0 + u - 1) * N);
+#pragma unroll
+    for (int u = 0; u < kDeep; ++u)
+      if (t0 + u < T) acc = cmul(l, make_float2(acc.x + prev[u].x, acc.y + prev[u].y));
+  }
+  const float2 p = r < 0 ? power(l, T) : make_float2(0.f, 0.f);
+  const float en = expf(w.nu_log[n]), et = expf(w.theta_log[n]);
+  const auto old = [&](const float* q) { return reinterpret_cast<const float2*>(q)[at]; };
+  const float2 last = hs[static_cast<size_t>(T - 1) * N], g0 = old(s.gamma);
+  reinterpret_cast<float2*>(s.nu_out)[at] = cmul_add(p, old(s.nu), make_float2(-en * acc.x, -en * acc.y));
+  reinterpret_cast<float2*>(s.theta_out)[at] = cmul_add(p, old(s.theta), make_float2(-et * acc.y, et * acc.x));
+  reinterpret_cast<float2*>(s.gamma_out)[at] = cmul_add(p, make_float2(g0.x - start.x, g0.y - start.y), last);
+}
+
+// B: a block owns one sequence, eight units and 128 features; a warp one unit, a lane four features.  The powers of
+// lambda are made once per block, so a step costs two multiply-adds per entry, and only the old and the new
+// sensitivities touch memory: HBM-bound at large N F, else bound by the multiply-adds.  (64 sequences x 64 steps, 64
+// features, 128 units: the materialised Jacobians took 490 us of kernels in 76 launches.)
+constexpr int kSensUnits = 8, kSensSteps = 64, kSensFeatures = 128;
+__global__ void __launch_bounds__(256) lru_sens_inputs_kernel(LruWeights w, const float* __restrict__ lambda,
+                                                              const float* __restrict__ u, const uint8_t* __restrict__ done,
+                                                              LruSensitivities s, int T, int F, int N) {
+  __shared__ __align__(16) float us[kSensSteps][kSensFeatures];
+  __shared__ float2 pw[kSensUnits][kSensSteps + 1];
+  const int b = blockIdx.z, n0 = blockIdx.x * kSensUnits, f0 = blockIdx.y * kSensFeatures;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n = n0 + warp, f = f0 + lane * 4;
+  const int r = last_reset(done ? done + static_cast<size_t>(b) * T : nullptr, T);
+  const int first = max(r, 0);
+  for (int i = threadIdx.x; i < kSensUnits * (kSensSteps + 1); i += 256) {
+    const int un = i / (kSensSteps + 1), k = i % (kSensSteps + 1);
+    if (n0 + un < N) pw[un][k] = power(reinterpret_cast<const float2*>(lambda)[n0 + un], k);
+  }
+  float re[4] = {0.f, 0.f, 0.f, 0.f}, im[4] = {0.f, 0.f, 0.f, 0.f};
+  const float* ub = u + static_cast<size_t>(b) * T * F;
+  for (int t0 = first; t0 < T; t0 += kSensSteps) {
+    const int len = min(kSensSteps, T - t0);
+    __syncthreads();
+    for (int i = threadIdx.x; i < len * kSensFeatures; i += 256) {
+      const int t = i / kSensFeatures, c = i % kSensFeatures;
+      us[t][c] = f0 + c < F ? ub[static_cast<size_t>(t0 + t) * F + f0 + c] : 0.f;
+    }
+    __syncthreads();
+    if (n >= N || f >= F) continue;
+    const float2 shift = pw[warp][len];   // what earlier steps have decayed by at the end of this stretch
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 v = cmul(shift, make_float2(re[e], im[e]));
+      re[e] = v.x;
+      im[e] = v.y;
+    }
+#pragma unroll 8
+    for (int t = 0; t < len; ++t) {
+      const float4 x = *reinterpret_cast<const float4*>(&us[t][lane * 4]);
+      const float2 p = pw[warp][len - 1 - t];
+      re[0] = fmaf(p.x, x.x, re[0]); im[0] = fmaf(p.y, x.x, im[0]);
+      re[1] = fmaf(p.x, x.y, re[1]); im[1] = fmaf(p.y, x.y, im[1]);
+      re[2] = fmaf(p.x, x.z, re[2]); im[2] = fmaf(p.y, x.z, im[2]);
+      re[3] = fmaf(p.x, x.w, re[3]); im[3] = fmaf(p.y, x.w, im[3]);
+    }
+  }
+  if (n >= N || f >= F) return;
+  const float gamma = expf(w.gamma_log[n]);
+  const float2 p = r < 0 ? power(reinterpret_cast<const float2*>(lambda)[n], T) : make_float2(0.f, 0.f);
+  const size_t at = (static_cast<size_t>(b) * N + n) * F + f;
+  const auto one = [&](const float2 o, float x, float y) { return cmul_add(p, o, make_float2(x, y)); };
+  if (F % 4 == 0) {   // sixteen-byte accesses: two complex entries each
+#pragma unroll
+    for (int e = 0; e < 4; e += 2) {
+      const float4 o = ld_stream(reinterpret_cast<const float4*>(s.b_re + 2 * (at + e)));
+      const float4 q = ld_stream(reinterpret_cast<const float4*>(s.b_im + 2 * (at + e)));
+      const float2 v0 = one({o.x, o.y}, gamma * re[e], gamma * im[e]), v1 = one({o.z, o.w}, gamma * re[e + 1], gamma * im[e + 1]);
+      const float2 y0 = one({q.x, q.y}, -gamma * im[e], gamma * re[e]), y1 = one({q.z, q.w}, -gamma * im[e + 1], gamma * re[e + 1]);
+      *reinterpret_cast<float4*>(s.b_re_out + 2 * (at + e)) = make_float4(v0.x, v0.y, v1.x, v1.y);
+      *reinterpret_cast<float4*>(s.b_im_out + 2 * (at + e)) = make_float4(y0.x, y0.y, y1.x, y1.y);
+    }
+  } else {
+    for (int e = 0; e < 4 && f + e < F; ++e) {
+      const float2 o = reinterpret_cast<const float2*>(s.b_re)[at + e], q = reinterpret_cast<const float2*>(s.b_im)[at + e];
+      reinterpret_cast<float2*>(s.b_re_out)[at + e] = one(o, gamma * re[e], gamma * im[e]);
+      reinterpret_cast<float2*>(s.b_im_out)[at + e] = one(q, -gamma * im[e], gamma * re[e]);
+    }
+  }
+}
+
 }  // namespace
 
 int lru_step(const LruWeights& w, const float* x, const float* h0, const float* a0, const uint8_t* done, float* h,
@@ -196,6 +341,15 @@ int skip_grad(const float* gy, const float* x, float* partial, long long rows, i
 
 int lru_param_grads(const LruWeights& w, const LruGrads& g, int F, int N, cudaStream_t stream) {
   lru_param_grads_kernel<<<N + F, 128, 0, stream>>>(w, g, F, N);
+  return launch_status();
+}
+
+int lru_sensitivities(const LruWeights& w, const float* lambda, const float* h, const float* h0, const float* u,
+                      const uint8_t* done, const LruSensitivities& s, int B, int T, int F, int N, cudaStream_t stream) {
+  if (B <= 0 || T <= 0 || F <= 0 || N <= 0 || B > 65535) return MXK_ERR_DIMS;
+  lru_sens_units_kernel<<<dim3((N + 127) / 128, B), 128, 0, stream>>>(w, lambda, h, h0, done, s, T, N);
+  const dim3 grid((N + kSensUnits - 1) / kSensUnits, (F + kSensFeatures - 1) / kSensFeatures, B);
+  lru_sens_inputs_kernel<<<grid, 256, 0, stream>>>(w, lambda, u, done, s, T, F, N);
   return launch_status();
 }
 

@@ -80,6 +80,10 @@ class MemoroidCellBase(nn.Module):
     def local_jacobian(self, carry, z, inputs, **kwargs):
         return None
 
+    def jacobian_segment(self, inputs, done, carry, sensitivity):
+        """A whole ``Memoroid.local_jacobian`` segment in fused form, or None where there is none."""
+        return None
+
     def compute_phantom(self, sensitivity):
         """sum over the leaves of S . (param - stop_gradient(param)): zero in value, its gradient with respect
         to the parameters is the sensitivity (memoroid.py:38-47).  Leaves are named by attribute path."""
@@ -172,6 +176,10 @@ class Memoroid(SequenceModel):
         parameters' gradients through the sensitivities), the scan and read-out run as in ``__call__``, and the
         cell's local Jacobians are propagated from ``sensitivity`` over the segment.  ``carry`` must be given
         (the cell's ``initialize_carry`` for a fresh start)."""
+        if sensitivity is not None and not kwargs:
+            out = self.cell.jacobian_segment(inputs, done, carry, sensitivity)
+            if out is not None:
+                return out
         z = self.cell(inputs, **kwargs)
         if sensitivity is not None:
             carry = self.cell.inject_phantom(carry, self.cell.compute_phantom(sensitivity))
@@ -247,6 +255,7 @@ class _ComplexDiagonalCell(MemoroidCellBase):
 
 
 # ---------------------------------------------------------------------- LRU
+_LRU_SENSITIVITIES = ("B_imag", "B_real", "gamma_log", "nu_log", "theta_log")
 _LRU_PARAMS = ("nu_log", "theta_log", "gamma_log", "B_real", "B_imag", "C_real", "C_imag", "D")
 
 
@@ -276,6 +285,15 @@ class LRUCell(_ComplexDiagonalCell):
             if out is not None:
                 return (out[0], out[1]), out[2]
         return super().layer(inputs, done, initial_carry, **kwargs)
+
+    def jacobian_segment(self, inputs, done, carry, sensitivity):
+        """The segment without gradients: the local Jacobians are never formed, the sensitivities are updated from the
+        states and the inputs by two kernels."""
+        if type(self) is not LRUCell or done is None or sensitivity.keys() != set(_LRU_SENSITIVITIES):
+            return None
+        out = _C.lru_rtrl(inputs, [self._parameters[name] for name in _LRU_PARAMS], carry[0], carry[1], done,
+                          [sensitivity[name] for name in _LRU_SENSITIVITIES])
+        return None if out is None else ((out[0], out[1]), out[2], dict(zip(_LRU_SENSITIVITIES, out[3])))
 
     def diag_lambda(self):
         return torch.exp(torch.complex(-torch.exp(self.nu_log), torch.exp(self.theta_log)))

@@ -59,3 +59,29 @@ def test_lru_layer_matches_the_oracle(shape, with_carry):
         assert err(got, ref) <= 1e-5
     for got, ref in zip(grads, want):
         assert err(got, ref) <= 1e-4
+
+
+# stretches of 64 steps, groups of 8 units and of 128 features; with and without a reset in a sequence
+@pytest.mark.parametrize("shape", [(2, 1, 4, 3), (3, 64, 33, 9), (2, 65, 130, 16), (4, 150, 8, 130)])
+@pytest.mark.parametrize("p_done", [0.0, 0.03])
+def test_fused_rtrl_segment_matches_the_oracle(shape, p_done):
+    from memorax_b200.memoroid import LRUCell, Memoroid
+    bsz, steps, feat, hid = shape
+    torch.manual_seed(0)
+    cell = LRUCell(feat, hid, r_min=0.5, r_max=0.999, max_phase=0.6).cuda()
+    model = Memoroid(cell)
+    x, done = torch.randn(bsz, steps, feat, device="cuda"), torch.rand(bsz, steps, device="cuda") < p_done
+    cplx = lambda s: torch.view_as_complex(torch.randn(*s, 2, device="cuda"))
+    carry = (cplx((bsz, 1, hid)), torch.ones(bsz, 1, hid, dtype=torch.complex64, device="cuda"))
+    sens = {k: cplx(v.shape) for k, v in model.initialize_sensitivity(None, (bsz, feat)).items()}
+    with torch.no_grad():
+        (h, _), y, out = model.local_jacobian(x, done, carry, sens)
+    p = {n: v.detach().cpu().double() for n, v in cell.named_parameters()}
+    h_ref, y_ref, s_ref = mo.lru_rtrl_seq(
+        x.cpu().double(), done.cpu().double(), carry[0][:, 0].cpu().to(torch.complex128), p["nu_log"], p["theta_log"], p["gamma_log"],
+        torch.complex(p["B_real"], p["B_imag"]), torch.complex(p["C_real"], p["C_imag"]), p["D"],
+        {k: v.cpu().to(torch.complex128) for k, v in sens.items()})
+    err = lambda got, ref: float((got.cpu().reshape(ref.shape) - ref).abs().max()) / float(ref.abs().max())
+    assert err(h, h_ref) <= 1e-5 and err(y, y_ref) <= 1e-5
+    for name in s_ref:
+        assert err(out[name], s_ref[name]) <= 1e-5, name
