@@ -34,4 +34,5 @@ PYBIND11_MODULE(_C, m) {
   bind_linrec(m);
   bind_linear(m);
   bind_lru(m);
+  bind_mingru(m);
 }

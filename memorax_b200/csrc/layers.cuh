@@ -47,5 +47,20 @@ struct LruSensitivities {
 int lru_sensitivities(const LruWeights& w, const float* lambda, const float* h, const float* h0, const float* u,
                       const uint8_t* done, const LruSensitivities& s, int B, int T, int F, int N, cudaStream_t stream);
 
+// ---- MinGRU, mingru.cu -----------------------------------------------------------------------------------------
+// z and h_tilde are (B, T, D) with rows of both (and of their cotangents) `ld` floats apart; the rest is dense.
+// With `h_kink` (= h_tilde, writable) elements too close to zero for their sign to be sure are replaced by the product
+// dense_in (B, T, F) dense_w (D, F)^T in plain float32 order.
+int mingru_fwd(const float* z, const float* h_tilde, float* h_kink, const float* dense_in, const float* dense_w, int F,
+               long long ld, const float* x0, const float* a0, const uint8_t* done,
+               float* x, float* y, float* a_last, int B, int T, int D, cudaStream_t stream);
+// y: the read-out exp(x), or null
+int mingru_bwd(const float* z, const float* h_tilde, long long ld, const float* x, const float* y, const float* x0, const uint8_t* done,
+               const float* gx, const float* gy, const float* gx_last, float* gz, float* gh, float* gx0, int B, int T, int D,
+               cudaStream_t stream);
+// One time step of the layer: the two Dense layers w_z, w_h (D, F), the gates and the recurrence.
+int mingru_step(const float* in, const float* w_z, const float* w_h, const float* x0, const float* a0, const uint8_t* done,
+                float* x, float* y, float* a_last, int B, int F, int D, cudaStream_t stream);
+
 }  // namespace layers
 }  // namespace mxk

@@ -10,6 +10,8 @@
 // owns a single element instead (more, narrower threads).
 #include <mutex>
 
+#include "layers.cuh"
+#include "logspace.cuh"
 #include "mxk_common.cuh"
 
 namespace mxk {
@@ -499,34 +501,6 @@ reduce_rows_kernel(const float* __restrict__ partial, float* __restrict__ out, i
 }
 
 // ------------------------------------------------------------ log-space form
-// MXK_LOGSPACE_FAST (default): exp / log through the special-function unit's approximations (ex2, lg2: relative
-// error about 2^-22) instead of the full-precision library sequences, which are most of these kernels'
-// instructions.  Measured against the fp64 oracle on the fused MinGRU path (8 x 256 x 256, inputs of a few units):
-// x 8e-8, y 3e-7, cotangents 4e-7 / 6e-7 of each tensor's max-abs, against 8e-8, 2e-7, 2e-7 / 3e-7 with the library
-// functions (-DMXK_LOGSPACE_FAST=0) -- both far inside the 1e-5 / 1e-4 the tests allow -- and 0.72 against 0.91 ms
-// for the 256 x 256 x 1024 forward + backward.
-#ifndef MXK_LOGSPACE_FAST
-#define MXK_LOGSPACE_FAST 1
-#endif
-__device__ __forceinline__ float exp_ls(float x) { return MXK_LOGSPACE_FAST ? __expf(x) : expf(x); }
-__device__ __forceinline__ float log_ls(float x) { return MXK_LOGSPACE_FAST ? __logf(x) : logf(x); }
-// log(1 + e) for e in [0, 1]
-__device__ __forceinline__ float log1p_ls(float e) { return MXK_LOGSPACE_FAST ? __logf(1.f + e) : log1pf(e); }
-
-__device__ __forceinline__ float log_add_exp(float p, float q) {
-  const float hi = fmaxf(p, q), lo = fminf(p, q);
-  if (hi == -INFINITY) return -INFINITY;
-  return hi + log1p_ls(exp_ls(lo - hi));
-}
-
-// MinGRU's gate math (min_gru.py:52-61), fused into the scan when the kernels are handed the Dense layers'
-// pre-activations instead of the elements:
-//   log_state = -softplus(-z) + log g(h~),  decay = -softplus(z),  g(h) = h >= 0 ? h + 0.5 : sigmoid(h).
-__device__ __forceinline__ float softplus_f(float x) { return fmaxf(x, 0.f) + log1p_ls(exp_ls(-fabsf(x))); }
-__device__ __forceinline__ float sigmoid_f(float x) { return 1.f / (1.f + exp_ls(-x)); }
-__device__ __forceinline__ float log_g(float h) { return h >= 0.f ? log_ls(h + 0.5f) : -softplus_f(-h); }
-__device__ __forceinline__ float dlog_g(float h) { return h >= 0.f ? 1.f / (h + 0.5f) : sigmoid_f(-h); }
-
 // GATES: `ls` / `d` hold the pre-activations z / h~ and the elements are formed on the fly.
 template <int W, bool GATES>
 __global__ void __launch_bounds__(kBlock)
@@ -702,6 +676,10 @@ inline int check_dims(int B, int T, int D) {
   if (static_cast<long long>(B) * D > (1LL << 40)) return MXK_ERR_DIMS;
   return MXK_OK;
 }
+
+// One thread per channel is the better form of the MinGRU scan from five full blocks per SM on (256 x 256 x 1024 forward +
+// backward: 0.73 ms against 0.82 split over time; 96 x 250 x 512: 0.25 ms against 0.15).
+inline bool mingru_walks(int B, int D) { return static_cast<long long>(B) * D >= 5LL * kNumSMs * kBlock; }
 
 template <bool CPLX>
 int linrec_fwd(const float* a, int a_tinv, const float* b, const float* h0, const float* a0,
@@ -952,6 +930,7 @@ int mxk_mingru_f32_fwd(const float* z, const float* h_tilde, const float* x0, co
   const long long total = static_cast<long long>(B) * D;
   const int w = pick_width(total, D, false, {z, h_tilde, x0, a0, x, y, a_last});
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (!mingru_walks(B, D)) return layers::mingru_fwd(z, h_tilde, nullptr, nullptr, nullptr, 0, D, x0, a0, done, x, y, a_last, B, T, D, s);
   if (w == 4)
     loglinrec_fwd_kernel<4, true><<<blocks_for(total / 4), kBlock, 0, s>>>(z, h_tilde, x0, a0, done, x, y, a_last, B, T, D);
   else
@@ -990,6 +969,7 @@ int mxk_mingru_f32_bwd(const float* z, const float* h_tilde, const float* x, con
   const long long total = static_cast<long long>(B) * D;
   const int w = pick_width(total, D, false, {z, h_tilde, x, x0, gx, gy, gx_last, gz, gh, gx0});
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (!mingru_walks(B, D)) return layers::mingru_bwd(z, h_tilde, D, x, nullptr, x0, done, gx, gy, gx_last, gz, gh, gx0, B, T, D, s);
   if (w == 4)
     loglinrec_bwd_kernel<4, true><<<blocks_for(total / 4), kBlock, 0, s>>>(z, h_tilde, x, x0, done, gx, gy, gx_last, gz, gh, gx0, B, T, D);
   else

@@ -1,0 +1,394 @@
+// MinGRU's scan with its gate math fused in (min_gru.py:52-78 under the reset rule of memoroid.py:60-91): the two Dense
+// pre-activations in, log-space states and read-out out, and the cotangents of the pre-activations back.
+//
+//   log_state = -softplus(-z) + log g(h~),  decay = -softplus(z),  x_t = logaddexp(decay_t + x_{t-1}, log_state_t)
+//
+// The states h = exp(x) obey h_t = sigmoid(-z) h_{t-1} + sigmoid(z) g(h~) with positive terms, so the linear form loses
+// no relative precision and needs one logarithm per element instead of a logaddexp; where a pre-activation or the carry
+// is so large that exp could leave float32's range (kSafe), the block takes the log form for that stretch of time.
+//
+// Bound: HBM (16 / 28 bytes per element; 30 / 53 us for 12.3 M elements) and about five special-function evaluations
+// per element, which have to overlap: time is split over sixteen warps of a block.  A block owns 32 channels of one
+// sequence; every thread loads its stretch of at most kSteps steps, folds it into one affine map of the incoming value
+// (forward: the state, backward: the carried cotangent; a reset cuts the map's slope), the sixteen maps are chained
+// through shared memory, and the stretch is replayed from the right incoming value.  Longer sequences take several
+// turns.  (One thread per channel walking all of T in log form: 116 / 136 us at 96 x 250 x 512.)
+#include "layers.cuh"
+#include "logspace.cuh"
+#include "mxk_common.cuh"
+#include "warp_tile.cuh"
+
+namespace mxk {
+namespace layers {
+namespace {
+
+constexpr int kSegs = 16, kSteps = 8;
+
+// d log g / dh~ jumps at h~ = 0 (from 1/2 to 2), so an element whose sign hangs on the rounding of its dot product is
+// decided by the plain float32 sum in the order of k: the branch, and with it the gradient, does not depend on how the
+// product was tiled.  (Two such sums differ by about 2e-7 at
+// unit scale and 512 terms; one element in 200 000 is looked at.)
+constexpr float kNearKink = 1.f / 262144.f;
+__device__ __noinline__ float dot_in_order(const float* __restrict__ in, const float* __restrict__ w, int F) {
+  float acc = 0.f;
+#pragma unroll 32
+  for (int k = 0; k < F; ++k) acc = fmaf(in[k], w[k], acc);
+  return acc;
+}
+
+// Largest |z|, |h~| and carried x for which the linear form stays inside float32: every state is at least e^-40, and what
+// a product of decays below e^-87 would have contributed is below 1e-11 of it.
+constexpr float kSafe = 20.f;
+
+// exp, log and reciprocal inside that range (no denormals: the .ftz forms need no scaling around the special-function
+// unit, which is most of what the general ones issue)
+__device__ __forceinline__ float exp_safe(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * 1.4426950408889634f));
+  return y;
+}
+__device__ __forceinline__ float log_safe(float x) {
+  float y;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y * 0.6931471805599453f;
+}
+__device__ __forceinline__ float rcp(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// Reset bits of `count` (at most kSteps) steps from t_begin on; the warp's lanes read one byte each.
+__device__ __forceinline__ unsigned reset_mask(const uint8_t* drow, int t_begin, int count, int lane) {
+  const bool reset = drow && lane < count && drow[t_begin + lane] != 0;
+  return __ballot_sync(0xffffffffu, reset);
+}
+
+__global__ void __launch_bounds__(32 * kSegs, 2)
+mingru_fwd_kernel(const float* __restrict__ z, const float* ht, float* ht_kink, const float* __restrict__ dense_in,
+                  const float* __restrict__ dense_w, int F, long long ld, const float* __restrict__ x0,
+                  const float* __restrict__ a0, const uint8_t* __restrict__ done, float* __restrict__ x, float* __restrict__ y,
+                  float* __restrict__ a_last, int B, int T, int D, int turn_len) {
+  __shared__ float sa[kSegs][32], sq[kSegs][32], sd[kSegs][32];
+  __shared__ unsigned sr[kSegs];   // reset bits of a stretch
+  __shared__ float carry_x[32], carry_a[32];
+  const int lane = threadIdx.x & 31, seg = threadIdx.x >> 5;
+  const int groups = (D + 31) / 32;
+  const int b = blockIdx.x / groups, d = (blockIdx.x % groups) * 32 + lane;
+  const bool in = d < D;
+  const uint8_t* drow = done ? done + static_cast<size_t>(b) * T : nullptr;
+  const int len = (turn_len + kSegs - 1) / kSegs;
+  if (seg == 0) {
+    carry_x[lane] = (in && x0) ? x0[static_cast<size_t>(b) * D + d] : -INFINITY;
+    carry_a[lane] = (in && a0) ? a0[static_cast<size_t>(b) * D + d] : 0.f;
+  }
+  for (int turn = 0; turn < T; turn += turn_len) {
+    const int t_begin = turn + seg * len, t_end = min(min(T, turn + turn_len), t_begin + len);
+    const int count = t_end - t_begin;   // steps of this warp (may be negative)
+    float lv[kSteps], dv[kSteps];
+    {
+      const long long token = static_cast<long long>(b) * T + t_begin;
+      const float *pz = z + token * ld + d, *ph = ht + token * ld + d;
+#pragma unroll
+      for (int i = 0; i < kSteps; ++i) {
+        const bool on = in && i < count;
+        lv[i] = on ? ld_stream(pz) : 0.f;
+        dv[i] = on ? ld_stream(ph) : 1.f;
+        pz += ld;
+        ph += ld;
+      }
+    }
+    const unsigned resets = reset_mask(drow, t_begin, count, lane);
+    float most = 0.f, least = 1.f;
+#pragma unroll
+    for (int i = 0; i < kSteps; ++i) {
+      most = fmaxf(most, fmaxf(fabsf(lv[i]), fabsf(dv[i])));
+      least = fminf(least, fabsf(dv[i]));
+    }
+    if (ht_kink && least < kNearKink) {
+#pragma unroll
+      for (int i = 0; i < kSteps; ++i)
+        if (fabsf(dv[i]) < kNearKink) {
+          const long long token = static_cast<long long>(b) * T + t_begin + i;
+          dv[i] = dot_in_order(dense_in + token * F, dense_w + static_cast<long long>(d) * F, F);
+          ht_kink[token * ld + d] = dv[i];
+        }
+    }
+    const bool linear = !__syncthreads_or(!(most <= kSafe) || (seg == 0 && !(carry_x[lane] <= kSafe)));
+    const size_t out0 = (static_cast<size_t>(b) * T + t_begin) * D + d;
+    if (linear) {
+      // h -> A h + Q; dec: decays since the last reset
+      float A = 1.f, Q = 0.f, dec = 0.f, prod = 1.f;
+#pragma unroll
+      for (int i = 0; i < kSteps; ++i) {
+        const float zi = lv[i], hi = dv[i];
+        const float e = exp_safe(-fabsf(zi)), r = rcp(1.f + e), er = e * r;   // sigmoid(|z|), sigmoid(-|z|)
+        const float sh = rcp(1.f + exp_safe(-hi)), g = hi >= 0.f ? hi + 0.5f : sh;
+        lv[i] = (zi >= 0.f ? r : er) * g;
+        dv[i] = zi >= 0.f ? er : r;
+        if (i < count) {
+          if (resets >> i & 1u) { A = 0.f; Q = lv[i]; dec = 0.f; prod = dv[i]; }
+          else { A *= dv[i]; Q = fmaf(dv[i], Q, lv[i]); prod *= dv[i]; }
+        }
+        if (i % 4 == 3) { dec += log_safe(prod); prod = 1.f; }   // four decays are at least e^-80
+      }
+      sa[seg][lane] = A;
+      sq[seg][lane] = Q;
+      sd[seg][lane] = dec;
+      if (lane == 0) sr[seg] = resets;
+      float cur = exp_ls(carry_x[lane]);
+      __syncthreads();
+      for (int s2 = 0; s2 < seg; ++s2) cur = fmaf(sa[s2][lane], cur, sq[s2][lane]);
+      float last = 0.f;
+      float *px = x + out0, *py = y + out0;
+#pragma unroll
+      for (int i = 0; i < kSteps; ++i) {
+        if (i < count) {
+          cur = (resets >> i & 1u) ? lv[i] : fmaf(dv[i], cur, lv[i]);
+          last = log_safe(cur);
+          if (in) {
+            st_stream(px, last);
+            if (y) st_stream(py, cur);
+          }
+          px += D;
+          py += D;
+        }
+      }
+      if (t_begin < t_end && t_end == min(T, turn + turn_len)) {
+        // the thread that holds the turn's last step: the carry of the next turn
+        float acc = carry_a[lane];
+        for (int s2 = 0; s2 < kSegs; ++s2) acc = sr[s2] ? sd[s2][lane] : acc + sd[s2][lane];
+        carry_a[lane] = acc;
+        carry_x[lane] = last;
+      }
+      __syncthreads();
+      continue;
+    }
+    // log form: x -> logaddexp(A + x, Q)
+    float A = 0.f, Q = -INFINITY, dec = 0.f;
+#pragma unroll
+    for (int i = 0; i < kSteps; ++i) {
+      if (i < count) {
+        const float zi = lv[i], hi = dv[i];
+        const float lz = log1p_ls(exp_ls(-fabsf(zi)));   // shared by softplus(z) and softplus(-z)
+        lv[i] = log_g(hi) - (fmaxf(-zi, 0.f) + lz);
+        dv[i] = -(fmaxf(zi, 0.f) + lz);
+        if (resets >> i & 1u) { A = -INFINITY; Q = lv[i]; dec = dv[i]; }
+        else { A += dv[i]; Q = log_add_exp(dv[i] + Q, lv[i]); dec += dv[i]; }
+      }
+    }
+    sa[seg][lane] = A;
+    sq[seg][lane] = Q;
+    sd[seg][lane] = dec;
+    if (lane == 0) sr[seg] = resets;
+    __syncthreads();
+    float cur = carry_x[lane];
+    for (int s2 = 0; s2 < seg; ++s2) cur = log_add_exp(sa[s2][lane] + cur, sq[s2][lane]);
+    __syncthreads();   // every segment has read the carry
+#pragma unroll
+    for (int i = 0; i < kSteps; ++i) {
+      if (i < count) {
+        cur = (resets >> i & 1u) ? lv[i] : log_add_exp(dv[i] + cur, lv[i]);
+        if (in) {
+          st_stream(x + out0 + static_cast<size_t>(i) * D, cur);
+          if (y) st_stream(y + out0 + static_cast<size_t>(i) * D, exp_ls(cur));
+        }
+      }
+    }
+    if (t_begin < t_end && t_end == min(T, turn + turn_len)) {
+      float acc = carry_a[lane];
+      for (int s2 = 0; s2 < kSegs; ++s2) acc = sr[s2] ? sd[s2][lane] : acc + sd[s2][lane];
+      carry_a[lane] = acc;
+      carry_x[lane] = cur;
+    }
+    __syncthreads();
+  }
+  if (seg == 0 && in && a_last) a_last[static_cast<size_t>(b) * D + d] = carry_a[lane];
+}
+
+// y: the states exp(x) where the caller has them (else they are formed here)
+__global__ void __launch_bounds__(32 * kSegs, 2)
+mingru_bwd_kernel(const float* __restrict__ z, const float* __restrict__ ht, long long ld, const float* __restrict__ x,
+                  const float* __restrict__ y, const float* __restrict__ x0, const uint8_t* __restrict__ done,
+                  const float* __restrict__ gx, const float* __restrict__ gy, const float* __restrict__ gx_last,
+                  float* __restrict__ gz, float* __restrict__ gh, float* __restrict__ gx0, int B, int T, int D, int turn_len) {
+  __shared__ float sp[kSegs][32], sq[kSegs][32];
+  __shared__ float carry[32];
+  const int lane = threadIdx.x & 31, seg = threadIdx.x >> 5;
+  const int groups = (D + 31) / 32;
+  const int b = blockIdx.x / groups, d = (blockIdx.x % groups) * 32 + lane;
+  const bool in = d < D;
+  const uint8_t* drow = done ? done + static_cast<size_t>(b) * T : nullptr;
+  const int len = (turn_len + kSegs - 1) / kSegs;
+  if (seg == 0) carry[lane] = (in && gx_last) ? gx_last[static_cast<size_t>(b) * D + d] : 0.f;
+  for (int turn = (T - 1) / turn_len * turn_len; turn >= 0; turn -= turn_len) {
+    const int t_begin = turn + seg * len, t_end = min(min(T, turn + turn_len), t_begin + len);
+    const int count = t_end - t_begin;   // steps of this warp (may be negative)
+    const size_t at0 = (static_cast<size_t>(b) * T + t_begin) * D + d;
+    const long long io0 = (static_cast<long long>(b) * T + t_begin) * ld + d;
+    const float* const state = y ? y : x;
+    float zv[kSteps], hv[kSteps], sv[kSteps], e[kSteps], w[kSteps], prev = 0.f;
+    {
+      const float *pz = z + io0, *ph = ht + io0, *ps = state + at0, *pg = gy + at0;
+      if (in && count > 0) prev = t_begin > 0 ? ps[-D] : (x0 ? x0[static_cast<size_t>(b) * D + d] : -INFINITY);
+#pragma unroll
+      for (int i = 0; i < kSteps; ++i) {
+        const bool on = in && i < count;
+        zv[i] = on ? ld_stream(pz) : 0.f;
+        hv[i] = on ? ld_stream(ph) : 0.f;
+        sv[i] = on ? ld_stream(ps) : 1.f;
+        e[i] = (on && gy) ? ld_stream(pg) : 0.f;
+        pz += ld;
+        ph += ld;
+        ps += D;
+        pg += D;
+      }
+    }
+    const unsigned resets = reset_mask(drow, t_begin, count, lane);
+    float most = (t_begin == 0 && x0) ? fmaxf(prev, 0.f) : 0.f;
+#pragma unroll
+    for (int i = 0; i < kSteps; ++i) most = fmaxf(most, fmaxf(fabsf(zv[i]), fabsf(hv[i])));
+    const bool linear = !__syncthreads_or(!(most <= kSafe));
+    // w_t = share of the incoming state in x_t; carry' = w (e + carry), right to left
+    float P = 1.f, Q = 0.f;
+    if (linear) {
+      if (!y) {
+#pragma unroll
+        for (int i = 0; i < kSteps; ++i) sv[i] = exp_ls(sv[i]);
+      }
+      if (!y || t_begin == 0) prev = exp_ls(prev);
+      if (gx && in) {
+#pragma unroll
+        for (int i = 0; i < kSteps; ++i) e[i] = i < count ? fmaf(e[i], sv[i], gx[at0 + static_cast<size_t>(i) * D]) : 0.f;
+      } else {
+#pragma unroll
+        for (int i = 0; i < kSteps; ++i) e[i] *= sv[i];
+      }
+#pragma unroll
+      for (int i = kSteps - 1; i >= 0; --i) {
+        const float ez = exp_safe(-fabsf(zv[i])), r = rcp(1.f + ez), er = ez * r;
+        const float share = (zv[i] >= 0.f ? er : r) * (i > 0 ? sv[i > 0 ? i - 1 : 0] : prev) * rcp(sv[i]);
+        w[i] = (resets >> i & 1u) ? 0.f : share;
+        zv[i] = zv[i] >= 0.f ? r : er;   // sigmoid(z)
+        if (i < count) {
+          Q = w[i] * (e[i] + Q);
+          P *= w[i];
+        }
+      }
+    } else {
+      // log form, from the log states
+      float xv[kSteps];
+#pragma unroll
+      for (int i = 0; i < kSteps; ++i) xv[i] = (in && t_begin + i < t_end) ? x[at0 + static_cast<size_t>(i) * D] : 0.f;
+      if (y && t_begin > 0 && in && t_begin < t_end) prev = x[at0 - D];
+#pragma unroll
+      for (int i = kSteps - 1; i >= 0; --i) {
+        w[i] = 0.f;
+        if (i < count) {
+          e[i] = e[i] != 0.f ? e[i] * exp_ls(xv[i]) : 0.f;
+          if (gx && in) e[i] += gx[at0 + static_cast<size_t>(i) * D];
+          const float ez = exp_ls(-fabsf(zv[i]));
+          if (!(resets >> i & 1u)) {
+            const float p = -(fmaxf(zv[i], 0.f) + log1p_ls(ez)) + (i > 0 ? xv[i > 0 ? i - 1 : 0] : prev);
+            w[i] = p == -INFINITY ? 0.f : exp_ls(p - xv[i]);
+          }
+          zv[i] = (zv[i] >= 0.f ? 1.f : ez) / (1.f + ez);
+          Q = w[i] * (e[i] + Q);
+          P *= w[i];
+        }
+      }
+    }
+    sp[seg][lane] = P;
+    sq[seg][lane] = Q;
+    __syncthreads();
+    float c = carry[lane];
+    for (int s2 = kSegs - 1; s2 > seg; --s2) c = fmaf(sp[s2][lane], c, sq[s2][lane]);
+    __syncthreads();   // every segment has read the carry
+    float *oz = gz + io0 + (count - 1) * ld, *oh = gh + io0 + (count - 1) * ld;
+#pragma unroll
+    for (int i = kSteps - 1; i >= 0; --i) {
+      if (i < count) {
+        const float g = e[i] + c, g_d = w[i] * g, g_ls = (1.f - w[i]) * g;
+        c = g_d;
+        // d(-softplus(-z))/dz = 1 - sigmoid(z), d(-softplus(z))/dz = -sigmoid(z)
+        const float sh = rcp(1.f + exp_safe(fminf(hv[i], 80.f))), dg = hv[i] >= 0.f ? rcp(hv[i] + 0.5f) : sh;
+        if (in) {
+          st_stream(oz, fmaf(-zv[i], g, g_ls));
+          st_stream(oh, g_ls * dg);
+        }
+        oz -= ld;
+        oh -= ld;
+      }
+    }
+    if (seg == 0) carry[lane] = c;
+  }
+  if (seg == 0 && in && gx0) gx0[static_cast<size_t>(b) * D + d] = carry[lane];
+}
+
+// Steps a block takes per turn: as evenly divided as the stretches allow (T = 250 is two turns of 125, not 128 + 122).
+int turn_length(int T) {
+  const int most = kSegs * kSteps, turns = (T + most - 1) / most;
+  return (T + turns - 1) / turns;
+}
+
+__global__ void __launch_bounds__(128)
+mingru_step_kernel(const float* __restrict__ in, const float* __restrict__ w_z, const float* __restrict__ w_h,
+                   const float* __restrict__ x0, const float* __restrict__ a0, const uint8_t* __restrict__ done,
+                   float* __restrict__ x, float* __restrict__ y, float* __restrict__ a_last, int B, int F, int D) {
+  const int lane = threadIdx.x & 31, warp = blockIdx.x * 4 + (threadIdx.x >> 5);
+  const int units = (D + 1) / 2;
+  const int d0 = (warp % units) * 2, m0 = (warp / units) * 8;
+  if (m0 >= B) return;
+  const size_t r0 = static_cast<size_t>(d0) * F, r1 = static_cast<size_t>(min(d0 + 1, D - 1)) * F;
+  const float* rows[4] = {w_z + r0, w_h + r0, w_z + r1, w_h + r1};
+  WarpTile acc;
+  acc.accumulate(in + static_cast<size_t>(m0) * F, F, min(8, B - m0), rows, F, lane);
+  const float v = acc.reduce(lane);
+  const float other = __shfl_xor_sync(0xffffffffu, v, 1);
+  const int m = m0 + (lane >> 2), d = d0 + ((lane >> 1) & 1);
+  if ((lane & 1) || m >= B || d >= D) return;   // even lanes hold z, their neighbours h~
+  const float lz = log1p_ls(exp_ls(-fabsf(v)));
+  const float ls = log_g(other) - (fmaxf(-v, 0.f) + lz), dec = -(fmaxf(v, 0.f) + lz);
+  const size_t at = static_cast<size_t>(m) * D + d;
+  const bool reset = done && done[m] != 0;
+  const float cur = reset ? ls : log_add_exp(dec + (x0 ? x0[at] : -INFINITY), ls);
+  x[at] = cur;
+  y[at] = exp_ls(cur);
+  if (a_last) a_last[at] = reset ? dec : dec + (a0 ? a0[at] : 0.f);
+}
+
+unsigned blocks_of(int B, int D) { return static_cast<unsigned>(static_cast<long long>(B) * ((D + 31) / 32)); }
+int check_dims(int B, int T, int D) {
+  return (B <= 0 || T <= 0 || D <= 0 || static_cast<long long>(B) * ((D + 31) / 32) > 0x7fffffffLL) ? MXK_ERR_DIMS : MXK_OK;
+}
+
+}  // namespace
+
+int mingru_fwd(const float* z, const float* h_tilde, float* h_kink, const float* dense_in, const float* dense_w, int F,
+               long long ld, const float* x0, const float* a0, const uint8_t* done,
+               float* x, float* y, float* a_last, int B, int T, int D, cudaStream_t stream) {
+  if (const int st = check_dims(B, T, D)) return st;
+  mingru_fwd_kernel<<<blocks_of(B, D), 32 * kSegs, 0, stream>>>(z, h_tilde, h_kink, dense_in, dense_w, F, ld, x0,
+                                                                a0, done, x, y, a_last, B, T, D, turn_length(T));
+  return launch_status();
+}
+
+int mingru_bwd(const float* z, const float* h_tilde, long long ld, const float* x, const float* y, const float* x0, const uint8_t* done,
+               const float* gx, const float* gy, const float* gx_last, float* gz, float* gh, float* gx0, int B, int T, int D,
+               cudaStream_t stream) {
+  if (const int st = check_dims(B, T, D)) return st;
+  mingru_bwd_kernel<<<blocks_of(B, D), 32 * kSegs, 0, stream>>>(z, h_tilde, ld, x, y, x0, done, gx, gy, gx_last, gz, gh, gx0,
+                                                                B, T, D, turn_length(T));
+  return launch_status();
+}
+
+int mingru_step(const float* in, const float* w_z, const float* w_h, const float* x0, const float* a0, const uint8_t* done,
+                float* x, float* y, float* a_last, int B, int F, int D, cudaStream_t stream) {
+  if (B <= 0 || F <= 0 || D <= 0) return MXK_ERR_DIMS;
+  const long long warps = static_cast<long long>((B + 7) / 8) * ((D + 1) / 2);
+  mingru_step_kernel<<<static_cast<unsigned>((warps + 3) / 4), 128, 0, stream>>>(in, w_z, w_h, x0, a0, done, x, y, a_last, B, F, D);
+  return launch_status();
+}
+
+}  // namespace layers
+}  // namespace mxk

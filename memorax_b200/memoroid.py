@@ -359,6 +359,17 @@ class MinGRUCell(MemoroidCellBase):
             return MinGRUPreactivations((self.z(x), self.h(x)))
         return self.elements(x)
 
+    def layer(self, inputs, done, initial_carry, **kwargs):
+        """Dense layers, gates, scan and read-out as one native call (float32); see ``LRUCell.layer``."""
+        z, h = self._modules["z"], self._modules["h"]
+        if (type(self) is MinGRUCell and self.fused_gates and not kwargs and type(z) is nn.Linear and type(h) is nn.Linear
+                and z.bias is None and h.bias is None):
+            x0, a0 = (None, None) if initial_carry is None else initial_carry
+            out = _C.mingru_layer(inputs, z._parameters["weight"], h._parameters["weight"], x0, a0, done)
+            if out is not None:
+                return (out[0], out[1]), out[2]
+        return super().layer(inputs, done, initial_carry, **kwargs)
+
     def elements(self, x):
         z, h_tilde = self.z(x), self.h(x)
         log_z = -torch.nn.functional.softplus(-z)
