@@ -65,6 +65,7 @@ struct Arena {
 void bind_linrec(pybind11::module_& m);
 void bind_linear(pybind11::module_& m);
 void bind_lru(pybind11::module_& m);
+void bind_mamba(pybind11::module_& m);
 void bind_mingru(pybind11::module_& m);
 
 }  // namespace mxk_host

@@ -34,5 +34,6 @@ PYBIND11_MODULE(_C, m) {
   bind_linrec(m);
   bind_linear(m);
   bind_lru(m);
+  bind_mamba(m);
   bind_mingru(m);
 }

@@ -21,7 +21,7 @@ struct LruWeights {
 int lru_step(const LruWeights& w, const float* x, const float* h0, const float* a0, const uint8_t* done, float* h,
              float* a_last, float* y, int B, int F, int N, cudaStream_t stream);
 
-// Sum over the rows of gy * x, (rows, F) each, left as `*blocks` partial rows of F in `partial` (lru_skip_blocks rows).
+// Sum over the rows of gy * x (x null: of gy), (rows, F) each, left as `*blocks` partial rows of F in `partial` (lru_skip_blocks rows).
 int skip_grad_blocks(long long rows);
 int skip_grad(const float* gy, const float* x, float* partial, long long rows, int F, cudaStream_t stream);
 
@@ -61,6 +61,41 @@ int mingru_bwd(const float* z, const float* h_tilde, long long ld, const float* 
 // One time step of the layer: the two Dense layers w_z, w_h (D, F), the gates and the recurrence.
 int mingru_step(const float* in, const float* w_z, const float* w_h, const float* x0, const float* a0, const uint8_t* done,
                 float* x, float* y, float* a_last, int B, int F, int D, cudaStream_t stream);
+
+// ---- sums over the rows of several float matrices (rows, cols) in one launch, in a fixed order ---------------------
+struct ColumnSum {
+  const float* src;
+  int rows, cols;
+  float* dst;
+};
+int column_sums(const ColumnSum* jobs, int count, cudaStream_t stream);   // at most four
+
+// ---- Mamba with heads of 16 x 16 states and four convolution taps, mamba.cu -----------------------------------------
+// `proj` (B, T, ld): what the Dense layers make of the inputs, columns hidden (16 H) | gate (16 H) | B (16 H) | C (16 H) |
+// dt (H); channels of the convolution: hidden | B | C.
+struct MambaParams {
+  const float *a_log, *d, *dt_bias;   // (H)
+  const float *conv_w, *conv_b;       // (48 H, 4), (48 H)
+  const float* norm_w;                // (16 H)
+  float eps;
+};
+// Convolution, gates, scan and C h + D x: y_pre (B, T, 16 H); h0 / a0 / done / states may be null.  states: the state each
+// stretch of 64 steps starts from, for the backward pass (mamba_state_floats).
+size_t mamba_state_floats(int B, int T, int H);
+int mamba_scan_fwd(const MambaParams& w, const float* proj, long long ld, const float* h0, const float* a0, const uint8_t* done,
+                   float* y_pre, float* h_last, float* a_last, float* states, int B, int T, int H, cudaStream_t stream);
+// z = RMSNorm(y_pre) silu(gate)
+int mamba_gate_fwd(const MambaParams& w, const float* proj, long long ld, const float* y_pre, float* z, long long tokens, int H,
+                   cudaStream_t stream);
+// gz -> gy_pre and the gate columns of gproj; norm_partial: mamba_gate_blocks rows of 16 H
+int mamba_gate_blocks(long long tokens);
+int mamba_gate_bwd(const MambaParams& w, const float* proj, long long ld, const float* y_pre, const float* gz, float* gy_pre,
+                   float* gproj, float* norm_partial, long long tokens, int H, cudaStream_t stream);
+// gy_pre -> the other columns of gproj; partial (B, mamba_partial_floats(H)): conv_w | conv_b | a_log | dt_bias | d
+int mamba_partial_floats(int H);
+int mamba_scan_bwd(const MambaParams& w, const float* proj, long long ld, const uint8_t* done, const float* states,
+                   const float* gy_pre, const float* gh_last, float* gproj, float* gh0,
+                   float* partial, int B, int T, int H, cudaStream_t stream);
 
 }  // namespace layers
 }  // namespace mxk

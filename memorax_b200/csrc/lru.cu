@@ -99,12 +99,12 @@ __global__ void __launch_bounds__(256) skip_grad_kernel(const float* __restrict_
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           a[u] = ld_stream(gy + (r + u * step) * F + c);
-          b[u] = ld_stream(x + (r + u * step) * F + c);
+          b[u] = x ? ld_stream(x + (r + u * step) * F + c) : 1.f;
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) s[u] = fmaf(a[u], b[u], s[u]);
       }
-      for (; r < rows; r += step) s[0] = fmaf(gy[r * F + c], x[r * F + c], s[0]);
+      for (; r < rows; r += step) s[0] = fmaf(gy[r * F + c], x ? x[r * F + c] : 1.f, s[0]);
     }
     __syncthreads();
     sums[threadIdx.x] = (s[0] + s[1]) + (s[2] + s[3]);
@@ -320,7 +320,45 @@ __global__ void __launch_bounds__(256) lru_sens_inputs_kernel(LruWeights w, cons
   }
 }
 
+struct ColumnSums {
+  ColumnSum job[4];
+  int first_block[5];
+};
+// 32 columns per block; eight groups of rows, added in order
+__global__ void __launch_bounds__(256) column_sums_kernel(const __grid_constant__ ColumnSums p) {
+  __shared__ float part[8][33];
+  int j = 0;
+  while (static_cast<int>(blockIdx.x) >= p.first_block[j + 1]) ++j;
+  const ColumnSum& jb = p.job[j];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int col = (blockIdx.x - p.first_block[j]) * 32 + tx;
+  float s = 0.f;
+  if (col < jb.cols)
+#pragma unroll 4
+    for (int r = ty; r < jb.rows; r += 8) s += jb.src[static_cast<size_t>(r) * jb.cols + col];
+  part[ty][tx] = s;
+  __syncthreads();
+  if (ty == 0 && col < jb.cols) {
+    float t = part[0][tx];
+#pragma unroll
+    for (int i = 1; i < 8; ++i) t += part[i][tx];
+    jb.dst[col] = t;
+  }
+}
+
 }  // namespace
+
+int column_sums(const ColumnSum* jobs, int count, cudaStream_t stream) {
+  if (count < 1 || count > 4) return MXK_ERR_DIMS;
+  ColumnSums p{};
+  for (int j = 0; j < count; ++j) {
+    p.job[j] = jobs[j];
+    p.first_block[j + 1] = p.first_block[j] + (jobs[j].cols + 31) / 32;
+  }
+  for (int j = count; j < 4; ++j) p.first_block[j + 1] = 0x7fffffff;
+  column_sums_kernel<<<p.first_block[count], 256, 0, stream>>>(p);
+  return launch_status();
+}
 
 int lru_step(const LruWeights& w, const float* x, const float* h0, const float* a0, const uint8_t* done, float* h,
              float* a_last, float* y, int B, int F, int N, cudaStream_t stream) {

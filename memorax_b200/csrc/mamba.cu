@@ -1,0 +1,536 @@
+// The Mamba layer between its Dense layers (mamba.py:100-135): causal convolution, SiLU, step sizes and decays, the
+// selective scan and its read-out, RMSNorm and gate -- forward and backward -- without the (B, T, H, 16, 16) elements or
+// states in memory.
+//
+// A block owns one (sequence, head) and walks time in stretches of 64 steps: the stretch's 48 channels are convolved into
+// shared memory, its four quarters are scanned by four warps from a zero state, the quarters' end states are chained, and
+// each warp replays its quarter from the right incoming state (a lane owns 8 of the 256 states; a step is 16 multiply-adds
+// for the update and 8 for the read-out).  Bound by issue slots at full size (about 40 instructions per warp and step) and
+// by the chain of stretches when there are few sequences; the materialised form moved 2 KB per token and head and ran
+// about thirty elementwise launches each way.
+//
+// The backward pass starts every stretch from its saved state and needs sums that are each cheap in one lane layout only,
+// so three groups of four warps run side by side: C's cotangent from the states (lane = n), x's (lane = p) and B's
+// (lane = n) from the cotangent of the states.  The first group leaves every h_{t-1} in shared memory for the third,
+// which has the decay's cotangent <dh_t, h_{t-1}> as a plain dot product (as a difference of larger sums it lost two
+// digits).
+#include "layers.cuh"
+#include "mxk_common.cuh"
+
+namespace mxk {
+namespace layers {
+namespace {
+
+constexpr int kN = 16, kP = 16, kStates = kN * kP;   // per head
+constexpr int kLen = 64, kQuarter = kLen / 4;        // steps per stretch and per warp
+constexpr int kTaps = 4, kHalo = kTaps - 1;
+constexpr int kCh = 3 * 16;                          // channels of a head: x | B | C
+
+__device__ __forceinline__ float sigmoid(float x) { return 1.f / (1.f + __expf(-x)); }
+__device__ __forceinline__ float softplus(float x) { return x > 20.f ? x : log1pf(expf(x)); }
+
+// Column of `proj` and channel of the convolution for channel c of head h.
+__device__ __forceinline__ int proj_col(int c, int h, int hid) {
+  return (c < 16 ? 0 : (c < 32 ? 2 * hid : 3 * hid)) + h * 16 + (c & 15);
+}
+__device__ __forceinline__ int conv_channel(int c, int h, int hid) { return (c >> 4) * hid + h * 16 + (c & 15); }
+
+// conv_w | conv_b | a_log | dt_bias | d of every head
+__host__ __device__ constexpr int partial_floats(int H) { return 48 * H * (kTaps + 1) + 3 * H; }
+
+struct Stretch {            // of one head
+  float raw[kLen + kHalo][kCh];   // projections, three steps of the past in front
+  float act[kLen][kCh];     // silu(conv): x | B | C
+  float dt[kLen], decay[kLen];
+  unsigned char reset[kLen];
+};
+
+__device__ __forceinline__ float convolve(const Stretch& s, const MambaParams& w, int r, int c, int ch) {
+  float v = __ldg(w.conv_b + ch);
+#pragma unroll
+  for (int k = 0; k < kTaps; ++k) v = fmaf(__ldg(w.conv_w + ch * kTaps + k), s.raw[r + k][c], v);
+  return v;
+}
+
+// Convolves and activates the stretch at t0.  Ends with a barrier.
+__device__ __forceinline__ void load_stretch(Stretch& s, const MambaParams& w, const float* __restrict__ proj, long long ld,
+                                             const uint8_t* drow, int b, int h, int H, int T, int t0, int tid, int threads) {
+  const int hid = H * 16;
+  for (int i = tid; i < (kLen + kHalo) * kCh; i += threads) {
+    const int r = i / kCh, c = i % kCh, t = t0 + r - kHalo;
+    s.raw[r][c] = (t >= 0 && t < T) ? __ldg(proj + (static_cast<long long>(b) * T + t) * ld + proj_col(c, h, hid)) : 0.f;
+  }
+  if (tid < kLen) {
+    const int t = t0 + tid;
+    float dt = 0.f, decay = 1.f;
+    if (t < T) {
+      dt = softplus(__ldg(proj + (static_cast<long long>(b) * T + t) * ld + 4 * hid + h) + w.dt_bias[h]);
+      decay = expf(dt * -expf(w.a_log[h]));
+    }
+    s.dt[tid] = dt;        // past the end: nothing enters, nothing decays
+    s.decay[tid] = decay;
+    s.reset[tid] = (t < T && drow) ? drow[t] : 0;
+  }
+  __syncthreads();
+  for (int i = tid; i < kLen * kCh; i += threads) {
+    const int r = i / kCh, c = i % kCh;
+    const float v = convolve(s, w, r, c, conv_channel(c, h, hid));
+    s.act[r][c] = v * sigmoid(v);
+  }
+  __syncthreads();
+}
+
+__device__ __forceinline__ void load8(const float* p, float* v) {   // 16-byte aligned shared memory
+  const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+  v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+
+struct FwdSmem {
+  Stretch s;
+  float end[4][8][32];      // [quarter][state of a lane][lane]
+  float prod[4], dec[4];    // product of the decays (0 with a reset), and since the last reset
+  int had[4];
+  float carry[8][32];
+  float carry_a;
+};
+
+// lane = p + 16 * (n >= 8): states n = 8 * (lane / 16) + j
+__global__ void __launch_bounds__(128) mamba_scan_fwd_kernel(MambaParams w, const float* __restrict__ proj, long long ld,
+                                                             const float* __restrict__ h0, const float* __restrict__ a0,
+                                                             const uint8_t* __restrict__ done, float* __restrict__ y_pre,
+                                                             float* __restrict__ h_last, float* __restrict__ a_last,
+                                                             float* __restrict__ states, int T, int H) {
+  __shared__ __align__(16) FwdSmem sm;
+  const int tid = threadIdx.x, lane = tid & 31, q = tid >> 5;
+  const int b = blockIdx.x / H, h = blockIdx.x % H, hid = H * 16;
+  const int p = lane & 15, n0 = (lane >> 4) * 8;
+  const uint8_t* drow = done ? done + static_cast<size_t>(b) * T : nullptr;
+  const float skip = w.d[h];
+  const int stretches = (T + kLen - 1) / kLen;
+  if (q == 0) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      sm.carry[j][lane] = h0 ? h0[static_cast<size_t>(blockIdx.x) * kStates + (n0 + j) * kP + p] : 0.f;
+    if (lane == 0) sm.carry_a = a0 ? a0[blockIdx.x] : 1.f;
+  }
+  for (int c = 0; c < stretches; ++c) {
+    const int t0 = c * kLen;
+    load_stretch(sm.s, w, proj, ld, drow, b, h, H, T, t0, tid, 128);
+    float st[8], v8[8];
+    // ---- from a zero state: where the quarter ends
+    {
+      float prod = 1.f, dec = 1.f;
+      int had = 0;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) st[j] = 0.f;
+#pragma unroll 4
+      for (int i = 0; i < kQuarter; ++i) {
+        const int t = q * kQuarter + i;
+        const bool reset = sm.s.reset[t] != 0;
+        const float d = reset ? 0.f : sm.s.decay[t];
+        const float xd = sm.s.act[t][p] * sm.s.dt[t];
+        load8(&sm.s.act[t][16 + n0], v8);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) st[j] = fmaf(d, st[j], v8[j] * xd);
+        prod *= d;
+        dec = reset ? sm.s.decay[t] : dec * sm.s.decay[t];
+        had |= reset;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) sm.end[q][j][lane] = st[j];
+      if (lane == 0) { sm.prod[q] = prod; sm.dec[q] = dec; sm.had[q] = had; }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 8; ++j) st[j] = sm.carry[j][lane];
+    if (q == 0 && states) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) states[(static_cast<size_t>(blockIdx.x) * stretches + c) * kStates + (n0 + j) * kP + p] = st[j];
+    }
+    for (int s2 = 0; s2 < q; ++s2) {
+      const float d = sm.prod[s2];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) st[j] = fmaf(d, st[j], sm.end[s2][j][lane]);
+    }
+    // ---- replay with the read-out
+#pragma unroll 4
+    for (int i = 0; i < kQuarter; ++i) {
+      const int t = q * kQuarter + i;
+      const float d = sm.s.reset[t] ? 0.f : sm.s.decay[t];
+      const float x = sm.s.act[t][p], xd = x * sm.s.dt[t];
+      load8(&sm.s.act[t][16 + n0], v8);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) st[j] = fmaf(d, st[j], v8[j] * xd);
+      load8(&sm.s.act[t][32 + n0], v8);
+      float y = 0.f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) y = fmaf(v8[j], st[j], y);
+      y += __shfl_xor_sync(0xffffffffu, y, 16);
+      if (lane < 16 && t0 + t < T) y_pre[(static_cast<size_t>(b) * T + t0 + t) * hid + h * 16 + p] = fmaf(skip, x, y);
+    }
+    __syncthreads();   // carry and summaries have been read
+    if (q == 3) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) sm.carry[j][lane] = st[j];
+      if (lane == 0) {
+        float a = sm.carry_a;
+        for (int s2 = 0; s2 < 4; ++s2) a = sm.had[s2] ? sm.dec[s2] : a * sm.dec[s2];
+        sm.carry_a = a;
+      }
+    }
+  }
+  if (q == 3) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) h_last[static_cast<size_t>(blockIdx.x) * kStates + (n0 + j) * kP + p] = sm.carry[j][lane];
+    if (lane == 0) a_last[blockIdx.x] = sm.carry_a;
+  }
+}
+
+// ------------------------------------------------------------------------------------------------------ backward
+struct BwdSmem {
+  Stretch s;
+  float g[kLen + kHalo][kCh];        // cotangents of the activations, then of the convolution's output; three steps of
+                                     // the future behind
+  float gy[kLen][16];
+  union {
+    float end[3][4][8][32];          // [task][quarter]...: where a quarter ends from nothing
+    float4 prev[kLen][2][32];        // h_{t-1}, eight states per lane
+    float red[384];
+  };
+  float prod[4];
+  float carry[2][8][32];             // decay-weighted cotangent of the state entering the stretch from the right
+  float e[kLen], u0[kLen];           // <dh_t, h_{t-1}>, <dh_t, B_t x_t>
+};
+static_assert(2 * (sizeof(BwdSmem) + 1024) <= 228 * 1024, "two blocks per SM");
+
+__global__ void __launch_bounds__(384, 2) mamba_scan_bwd_kernel(MambaParams w, const float* __restrict__ proj, long long ld,
+                                                                const uint8_t* __restrict__ done,
+                                                                const float* __restrict__ states,
+                                                                const float* __restrict__ gy_pre,
+                                                                const float* __restrict__ gh_last, float* __restrict__ gproj,
+                                                                float* __restrict__ gh0, float* __restrict__ partial, int T, int H) {
+  extern __shared__ __align__(16) uint8_t raw_smem[];
+  BwdSmem& sm = *reinterpret_cast<BwdSmem*>(raw_smem);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int task = warp >> 2, q = warp & 3;   // task 0: C (lane = n), 1: x (lane = p), 2: B (lane = n)
+  const int b = blockIdx.x / H, h = blockIdx.x % H, hid = H * 16;
+  const int l16 = lane & 15, o8 = (lane >> 4) * 8;   // own index, and the first of the eight contracted ones
+  const uint8_t* drow = done ? done + static_cast<size_t>(b) * T : nullptr;
+  const float skip = w.d[h], neg_a = -expf(w.a_log[h]);
+  const int stretches = (T + kLen - 1) / kLen;
+  const size_t base = static_cast<size_t>(blockIdx.x) * kStates;
+  // state (n, p) of slot j of this lane in this task's layout
+  const auto state_at = [&](int j) { return task == 1 ? (o8 + j) * kP + l16 : l16 * kP + o8 + j; };
+
+  if (q == 0 && task > 0) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) sm.carry[task - 1][j][lane] = gh_last ? gh_last[base + state_at(j)] : 0.f;
+  }
+  for (int i = tid; i < kHalo * kCh; i += 384) sm.g[kLen + i / kCh][i % kCh] = 0.f;
+  // gradients of the convolution: thread = channel x 8 groups of 8 steps
+  const int pc = tid % kCh, pg = tid / kCh;
+  float gw[kTaps] = {0.f, 0.f, 0.f, 0.f}, gbias = 0.f, ga = 0.f, gdtb = 0.f, gd = 0.f;
+
+  for (int c = stretches - 1; c >= 0; --c) {
+    const int t0 = c * kLen;
+    for (int i = tid; i < kLen * 16; i += 384) {
+      const int r = i >> 4, p = i & 15;
+      sm.gy[r][p] = t0 + r < T ? __ldg(gy_pre + (static_cast<size_t>(b) * T + t0 + r) * hid + h * 16 + p) : 0.f;
+    }
+    load_stretch(sm.s, w, proj, ld, drow, b, h, H, T, t0, tid, 384);
+    float st[8], a8[8];
+    // ---- each quarter from nothing: states forward in time (task 0), their cotangents backward (tasks 1, 2)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) st[j] = 0.f;
+    float prod = 1.f;
+#pragma unroll 4
+    for (int i = 0; i < kQuarter; ++i) {
+      const int t = q * kQuarter + (task == 0 ? i : kQuarter - 1 - i);
+      const float d = sm.s.reset[t] ? 0.f : sm.s.decay[t];
+      if (task == 0) {
+        const float bd = sm.s.act[t][16 + l16] * sm.s.dt[t];
+        load8(&sm.s.act[t][o8], a8);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) st[j] = fmaf(d, st[j], a8[j] * bd);
+      } else {
+        const float own = task == 1 ? sm.gy[t][l16] : sm.s.act[t][32 + l16];
+        load8(task == 1 ? &sm.s.act[t][32 + o8] : &sm.gy[t][o8], a8);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) st[j] = d * fmaf(a8[j], own, st[j]);
+      }
+      prod *= d;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) sm.end[task][q][j][lane] = st[j];
+    if (task == 0 && lane == 0) sm.prod[q] = prod;
+    __syncthreads();
+    // ---- chain
+    if (task == 0) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) st[j] = states[(static_cast<size_t>(blockIdx.x) * stretches + c) * kStates + state_at(j)];
+      for (int s2 = 0; s2 < q; ++s2) {
+        const float d = sm.prod[s2];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) st[j] = fmaf(d, st[j], sm.end[0][s2][j][lane]);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) st[j] = sm.carry[task - 1][j][lane];
+      for (int s2 = 3; s2 > q; --s2) {
+        const float d = sm.prod[s2];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) st[j] = fmaf(d, st[j], sm.end[task][s2][j][lane]);
+      }
+    }
+    __syncthreads();   // summaries and carries have been read; the summaries' memory takes the states
+    // ---- replay
+    if (task == 0) {
+#pragma unroll 4
+      for (int i = 0; i < kQuarter; ++i) {
+        const int t = q * kQuarter + i;
+        const float d = sm.s.reset[t] ? 0.f : sm.s.decay[t], bd = sm.s.act[t][16 + l16] * sm.s.dt[t];
+        sm.prev[t][0][lane] = make_float4(st[0], st[1], st[2], st[3]);
+        sm.prev[t][1][lane] = make_float4(st[4], st[5], st[6], st[7]);
+        load8(&sm.s.act[t][o8], a8);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) st[j] = fmaf(d, st[j], a8[j] * bd);
+        load8(&sm.gy[t][o8], a8);
+        float v = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v = fmaf(a8[j], st[j], v);
+        v += __shfl_xor_sync(0xffffffffu, v, 16);
+        if (lane < 16) sm.g[t][32 + l16] = v;
+      }
+      asm volatile("bar.arrive %0, 64;" ::"r"(q + 1) : "memory");   // this quarter's states are there
+    } else {
+      if (task == 2) asm volatile("bar.sync %0, 64;" ::"r"(q + 1) : "memory");
+#pragma unroll 4
+      for (int i = kQuarter - 1; i >= 0; --i) {
+        const int t = q * kQuarter + i;
+        const float d = sm.s.reset[t] ? 0.f : sm.s.decay[t], dt = sm.s.dt[t];
+        const float own = task == 1 ? sm.gy[t][l16] : sm.s.act[t][32 + l16];
+        load8(task == 1 ? &sm.s.act[t][32 + o8] : &sm.gy[t][o8], a8);
+        float x8[8], v = 0.f, e = 0.f;
+        load8(task == 1 ? &sm.s.act[t][16 + o8] : &sm.s.act[t][o8], x8);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          a8[j] = fmaf(a8[j], own, st[j]);   // dh_t
+          v = fmaf(x8[j], a8[j], v);
+          st[j] = d * a8[j];
+        }
+        v += __shfl_xor_sync(0xffffffffu, v, 16);
+        if (task == 1) {
+          if (lane < 16) sm.g[t][l16] = fmaf(dt, v, skip * own);
+        } else {
+          const float4 p0 = sm.prev[t][0][lane], p1 = sm.prev[t][1][lane];
+          e = a8[0] * p0.x + a8[1] * p0.y + a8[2] * p0.z + a8[3] * p0.w;
+          e += a8[4] * p1.x + a8[5] * p1.y + a8[6] * p1.z + a8[7] * p1.w;
+          if (lane < 16) sm.g[t][16 + l16] = dt * v;
+          // lower half: <dh, h_{t-1}>, upper half: B . (cotangent of B)
+          e += __shfl_xor_sync(0xffffffffu, e, 16);
+          if (lane >= 16) e = v * sm.s.act[t][16 + l16];
+#pragma unroll
+          for (int o = 8; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+          if (l16 == 0) (lane == 0 ? sm.e : sm.u0)[t] = e;
+        }
+      }
+      if (q == 0) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) sm.carry[task - 1][j][lane] = st[j];
+      }
+    }
+    __syncthreads();
+    // ---- step size and decay
+    if (tid < kLen && t0 + tid < T) {
+      const long long tok = static_cast<long long>(b) * T + t0 + tid;
+      const float gl = sm.s.reset[tid] ? 0.f : sm.s.decay[tid] * sm.e[tid];   // cotangent of the log decay dt * neg_a
+      const float logit = __ldg(proj + tok * ld + 4 * hid + h) + w.dt_bias[h];
+      const float gdt = (sm.u0[tid] + gl * neg_a) * sigmoid(logit);
+      gproj[tok * ld + 4 * hid + h] = gdt;
+      gdtb += gdt;
+      ga += gl * sm.s.dt[tid] * neg_a;
+    }
+    // ---- through SiLU
+    for (int i = tid; i < kLen * kCh; i += 384) {
+      const int r = i / kCh, ch = i % kCh;
+      const float u = convolve(sm.s, w, r, ch, conv_channel(ch, h, hid)), sg = sigmoid(u);
+      if (ch < 16) gd = fmaf(sm.gy[r][ch], u * sg, gd);
+      sm.g[r][ch] = t0 + r < T ? sm.g[r][ch] * sg * (1.f + u * (1.f - sg)) : 0.f;
+    }
+    __syncthreads();
+    // ---- through the convolution: inputs, weights, bias
+    for (int i = tid; i < kLen * kCh; i += 384) {
+      const int r = i / kCh, cc = i % kCh;
+      if (t0 + r < T) {
+        const int chn = conv_channel(cc, h, hid);
+        float v = 0.f;
+#pragma unroll
+        for (int k = 0; k < kTaps; ++k) v = fmaf(__ldg(w.conv_w + chn * kTaps + k), sm.g[r + kHalo - k][cc], v);
+        gproj[(static_cast<long long>(b) * T + t0 + r) * ld + proj_col(cc, h, hid)] = v;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kLen / 8; ++i) {
+      const int r = pg * (kLen / 8) + i;
+      const float g = sm.g[r][pc];
+      gbias += g;
+#pragma unroll
+      for (int k = 0; k < kTaps; ++k) gw[k] = fmaf(g, sm.s.raw[r + k][pc], gw[k]);
+    }
+    __syncthreads();
+    for (int i = tid; i < kHalo * kCh; i += 384) sm.g[kLen + i / kCh][i % kCh] = sm.g[i / kCh][i % kCh];
+    __syncthreads();
+  }
+  if (gh0 && task == 1 && q == 0) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) gh0[base + state_at(j)] = sm.carry[0][j][lane];
+  }
+  // ---- parameter gradients of this (sequence, head)
+  float* const row = partial + static_cast<size_t>(b) * partial_floats(H);
+  const int channels = 3 * hid;
+  const auto over_groups = [&](float v) {   // sum over the 8 step groups of a channel, at pg == 0
+    __syncthreads();
+    sm.red[tid] = v;
+    __syncthreads();
+    float t = 0.f;
+    if (pg == 0)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) t += sm.red[i * kCh + pc];
+    return t;
+  };
+  const int chn = conv_channel(pc, h, hid);
+#pragma unroll
+  for (int k = 0; k < kTaps; ++k) {
+    const float v = over_groups(gw[k]);
+    if (pg == 0) row[chn * kTaps + k] = v;
+  }
+  {
+    const float v = over_groups(gbias);
+    if (pg == 0) row[channels * kTaps + chn] = v;
+  }
+  const auto over_block = [&](float v) {
+    __syncthreads();
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) sm.red[warp] = v;
+    __syncthreads();
+    float t = 0.f;
+#pragma unroll
+    for (int i = 0; i < 12; ++i) t += sm.red[i];
+    return t;
+  };
+  float* const heads = row + channels * (kTaps + 1);
+  const float s_a = over_block(ga), s_b = over_block(gdtb), s_d = over_block(gd);
+  if (tid == 0) {
+    heads[h] = s_a;
+    heads[H + h] = s_b;
+    heads[2 * H + h] = s_d;
+  }
+}
+
+// ----------------------------------------------------------------------------------------------- RMSNorm and gate
+constexpr int kGateBlocks = 4 * kNumSMs;
+
+// One warp per token.
+__global__ void __launch_bounds__(256) mamba_gate_fwd_kernel(MambaParams w, const float* __restrict__ proj, long long ld,
+                                                             const float* __restrict__ y_pre, float* __restrict__ z,
+                                                             long long tokens, int hid) {
+  const int lane = threadIdx.x & 31;
+  const long long tok = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+  if (tok >= tokens) return;
+  const float *y = y_pre + tok * hid, *gate = proj + tok * ld + hid;
+  float ss = 0.f;
+  for (int c = lane; c < hid; c += 32) ss = fmaf(y[c], y[c], ss);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  const float rstd = rsqrtf(ss / hid + w.eps);
+  for (int c = lane; c < hid; c += 32) {
+    const float g = __ldg(gate + c);
+    z[tok * hid + c] = y[c] * rstd * w.norm_w[c] * (g * sigmoid(g));
+  }
+}
+
+__global__ void __launch_bounds__(256) mamba_gate_bwd_kernel(MambaParams w, const float* __restrict__ proj, long long ld,
+                                                             const float* __restrict__ y_pre, const float* __restrict__ gz,
+                                                             float* __restrict__ gy_pre, float* __restrict__ gproj,
+                                                             float* __restrict__ norm_partial, long long tokens, int hid) {
+  extern __shared__ float acc[];   // [8 warps][hid]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int i = threadIdx.x; i < 8 * hid; i += 256) acc[i] = 0.f;
+  __syncthreads();
+  for (long long tok = static_cast<long long>(blockIdx.x) * 8 + warp; tok < tokens; tok += static_cast<long long>(gridDim.x) * 8) {
+    const float *y = y_pre + tok * hid, *gate = proj + tok * ld + hid, *g = gz + tok * hid;
+    float ss = 0.f, dot = 0.f;
+    for (int c = lane; c < hid; c += 32) {
+      const float gt = __ldg(gate + c), gn = g[c] * gt * sigmoid(gt) * w.norm_w[c];
+      ss = fmaf(y[c], y[c], ss);
+      dot = fmaf(gn, y[c], dot);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      dot += __shfl_xor_sync(0xffffffffu, dot, o);
+    }
+    const float rstd = rsqrtf(ss / hid + w.eps);
+    const float mean = dot * rstd * rstd / hid;   // mean of (cotangent of the normalised row) * (normalised row), times rstd
+    for (int c = lane; c < hid; c += 32) {
+      const float gt = __ldg(gate + c), sg = sigmoid(gt), yn = y[c] * rstd;
+      const float gs = g[c] * gt * sg;             // cotangent of norm(y) * weight
+      gy_pre[tok * hid + c] = rstd * gs * w.norm_w[c] - mean * yn;
+      gproj[tok * ld + hid + c] = g[c] * yn * w.norm_w[c] * sg * (1.f + gt * (1.f - sg));
+      acc[warp * hid + c] = fmaf(gs, yn, acc[warp * hid + c]);
+    }
+  }
+  __syncthreads();
+  for (int c = threadIdx.x; c < hid; c += 256) {
+    float t = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) t += acc[i * hid + c];
+    norm_partial[static_cast<size_t>(blockIdx.x) * hid + c] = t;
+  }
+}
+
+}  // namespace
+
+size_t mamba_state_floats(int B, int T, int H) { return static_cast<size_t>(B) * H * ((T + kLen - 1) / kLen) * kStates; }
+int mamba_partial_floats(int H) { return partial_floats(H); }
+int mamba_gate_blocks(long long tokens) {
+  const long long need = (tokens + 7) / 8;
+  return static_cast<int>(need < kGateBlocks ? need : kGateBlocks);
+}
+
+int mamba_scan_fwd(const MambaParams& w, const float* proj, long long ld, const float* h0, const float* a0, const uint8_t* done,
+                   float* y_pre, float* h_last, float* a_last, float* states, int B, int T, int H, cudaStream_t stream) {
+  if (B <= 0 || T <= 0 || H <= 0) return MXK_ERR_DIMS;
+  mamba_scan_fwd_kernel<<<B * H, 128, 0, stream>>>(w, proj, ld, h0, a0, done, y_pre, h_last, a_last, states, T, H);
+  return launch_status();
+}
+
+int mamba_scan_bwd(const MambaParams& w, const float* proj, long long ld, const uint8_t* done, const float* states,
+                   const float* gy_pre, const float* gh_last, float* gproj, float* gh0,
+                   float* partial, int B, int T, int H, cudaStream_t stream) {
+  if (B <= 0 || T <= 0 || H <= 0) return MXK_ERR_DIMS;
+  if (const int st = allow_smem<mamba_scan_bwd_kernel>(sizeof(BwdSmem)); st != MXK_OK) return st;
+  mamba_scan_bwd_kernel<<<B * H, 384, sizeof(BwdSmem), stream>>>(w, proj, ld, done, states, gy_pre, gh_last, gproj, gh0, partial,
+                                                                 T, H);
+  return launch_status();
+}
+
+int mamba_gate_fwd(const MambaParams& w, const float* proj, long long ld, const float* y_pre, float* z, long long tokens, int H,
+                   cudaStream_t stream) {
+  mamba_gate_fwd_kernel<<<static_cast<unsigned>((tokens + 7) / 8), 256, 0, stream>>>(w, proj, ld, y_pre, z, tokens, 16 * H);
+  return launch_status();
+}
+
+int mamba_gate_bwd(const MambaParams& w, const float* proj, long long ld, const float* y_pre, const float* gz, float* gy_pre,
+                   float* gproj, float* norm_partial, long long tokens, int H, cudaStream_t stream) {
+  const int hid = 16 * H, bytes = 8 * hid * static_cast<int>(sizeof(float));
+  if (bytes > 48 * 1024)
+    if (const int st = allow_smem<mamba_gate_bwd_kernel>(bytes); st != MXK_OK) return st;
+  mamba_gate_bwd_kernel<<<mamba_gate_blocks(tokens), 256, bytes, stream>>>(w, proj, ld, y_pre, gz, gy_pre, gproj, norm_partial, tokens, hid);
+  return launch_status();
+}
+
+}  // namespace layers
+}  // namespace mxk

@@ -702,6 +702,20 @@ class MambaCell(MemoroidCellBase):
         self.norm = nn.RMSNorm(hidden, eps=1e-6)   # flax.linen.RMSNorm's default epsilon
         self.output_projection = nn.Linear(hidden, features)
 
+    def layer(self, inputs, done, initial_carry, **kwargs):
+        """The whole layer as one native call (float32, heads of 16 x 16 states, four taps): the (B, T, H, N, P) elements
+        and states are never formed.  Other shapes, and subclasses, are composed from their parts."""
+        if type(self) is MambaCell and not kwargs and (self.head_dim, self.state_dim, self.conv_dim) == (16, 16, 4):
+            h0, a0 = (None, None) if initial_carry is None else initial_carry
+            own, sub = self._parameters, self._modules
+            of = lambda name, kind="weight": sub[name]._parameters[kind]
+            out = _C.mamba_layer(inputs, [own["A_log"], own["D"], own["dt_bias"], of("input_projection"), of("B"), of("C"), of("dt"),
+                                          of("conv"), of("conv", "bias"), of("norm"), of("output_projection"),
+                                          of("output_projection", "bias")], h0, a0, done, self.norm.eps)
+            if out is not None:
+                return (out[0], out[1]), out[2]
+        return super().layer(inputs, done, initial_carry, **kwargs)
+
     def _project(self, x):
         bsz, steps, _ = x.shape
         hidden_dim, sproj = self.num_heads * self.head_dim, self.num_heads * self.state_dim
