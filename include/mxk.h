@@ -378,7 +378,7 @@ int mxk_adam_bf16_master(void* params, float* master, const void* grads, float* 
  *
  * LayerNorm (PreNorm, blocks/normalization.py:10-35) and RMSNorm (the norm in front of the
  * cells' output projection, linear_attention.py:114): x, y (rows, D) bf16 with D a multiple of
- * 256 and at most 1024; gamma (and beta for LayerNorm) (D) bf16; mean / rstd (rows) fp32 out
+ * 8 and at most 1024; gamma (and beta for LayerNorm) (D) bf16; mean / rstd (rows) fp32 out
  * (mean unused when rms != 0).  Backward: dx (rows, D) bf16, dgamma / dbeta (D) fp32, reduced over
  * the rows in a fixed order through `workspace` (mxk_norm_bwd_workspace_bytes).
  * Gated residual (blocks/residual.py:53-59): y = x + sigmoid(g) * o over n bf16 elements

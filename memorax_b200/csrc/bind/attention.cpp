@@ -1,0 +1,331 @@
+// The linear-attention and gated-delta-rule layers in bf16: the Dense layers on the inputs as one product, the chunked
+// kernels on slices of its result, RMSNorm and output projection; the backward pass as one autograd node.  One step of a
+// few sequences (acting) takes three launches.
+#include "common.h"
+
+#include "../attention.cuh"
+#include "../layers.cuh"
+
+namespace mxk_host {
+namespace {
+
+namespace l = mxk::layers;
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+
+constexpr int kFewRows = 256;   // up to here small_product beats the 128-row tiles of a library product (and its host cost)
+
+struct Shape {
+  int B, T, F, H, d, hid, M, out;
+  int64_t ld;                   // columns of the joint projection, padded to 16 bytes
+};
+
+l::WeightRows rows_of(const variable_list& w, size_t count) {
+  l::WeightRows r{};
+  r.count = static_cast<int>(count);
+  for (size_t i = 0; i < count; ++i) {
+    r.ptr[i] = w[i].data_ptr();
+    r.rows[i] = static_cast<int>(w[i].size(0));
+  }
+  return r;
+}
+
+// x (M, F) -> (M, ld), columns past the weights zero; `stacked` keeps the joint weight for the backward pass
+Tensor project(const Tensor& x, const variable_list& w, size_t count, const Shape& s, Tensor* stacked) {
+  const Tensor proj = empty_like_of(x, {s.M, s.ld}, at::kBFloat16);
+  if (!stacked && s.M <= kFewRows && s.F % 32 == 0) {
+    check("small_product", l::small_product(x.data_ptr(), rows_of(w, count), nullptr, proj.data_ptr(), s.ld, s.M, s.F, stream()));
+    return proj;
+  }
+  const Tensor joint = empty_like_of(x, {s.ld, s.F}, at::kBFloat16);
+  check("stack_rows", l::stack_rows(rows_of(w, count), joint.data_ptr(), s.ld, s.F, stream()));
+  // the library's tiles fit q | k | v; the few columns behind them would cost it a tile column (65536 x 3088 x 512:
+  // 198 us against 160 for 3072 and 17 for 16)
+  const Tensor rows = x.view({s.M, s.F});
+  Tensor into = proj.narrow(1, 0, 3 * s.hid);
+  at::mm_out(into, rows, joint.narrow(0, 0, 3 * s.hid).t());
+  if (s.ld > 3 * s.hid) {
+    Tensor rest = proj.narrow(1, 3 * s.hid, s.ld - 3 * s.hid);
+    at::mm_out(rest, rows, joint.narrow(0, 3 * s.hid, s.ld - 3 * s.hid).t());
+  }
+  if (stacked) *stacked = joint;
+  return proj;
+}
+
+Tensor output(const Tensor& n, const Tensor& w, const Tensor& bias, const Shape& s, bool few) {
+  if (few && s.M <= kFewRows && s.hid % 32 == 0) {
+    const Tensor y = empty_like_of(n, {s.M, s.out}, at::kBFloat16);
+    check("small_product", l::small_product(n.data_ptr(), rows_of({w}, 1), bias.data_ptr(), y.data_ptr(), s.out, s.M, s.hid, stream()));
+    return y;
+  }
+  return at::addmm(bias, n, w.t());
+}
+
+// What follows the mixer: RMSNorm and output projection, and their gradients
+struct Tail {
+  Tensor n, rstd;
+};
+Tail norm_forward(const Tensor& o, const Tensor& norm_w, double norm_eps, const Shape& s) {
+  Tail t{at::empty_like(o), empty_like_of(o, {s.M}, at::kFloat)};
+  check("mxk_norm_bf16_fwd", mxk_norm_bf16_fwd(o.data_ptr(), norm_w.data_ptr(), nullptr, t.n.data_ptr(), nullptr, ptr(t.rstd), s.M, s.hid,
+                                               norm_eps, 1, stream()));
+  return t;
+}
+struct TailGrads {
+  Tensor go, norm_w, out_w, out_b;
+};
+TailGrads tail_backward(const Tensor& gy, const Tensor& o, const Tensor& n, const Tensor& rstd, const Tensor& norm_w, const Tensor& out_w, const Shape& s) {
+  TailGrads g;
+  const Tensor gn = at::mm(gy, out_w);
+  g.out_w = at::mm(gy.t(), n);
+  g.out_b = empty_like_of(gy, {s.out}, at::kBFloat16);
+  const size_t sum_bytes = mxk_colsum_workspace_bytes(s.M, s.out), norm_bytes = mxk_norm_bwd_workspace_bytes(s.M, s.hid);
+  const Tensor ws = scratch(gy, std::max(sum_bytes, norm_bytes));
+  check("mxk_colsum_bf16", mxk_colsum_bf16(gy.data_ptr(), g.out_b.data_ptr(), ws.data_ptr(), sum_bytes, s.M, s.out, stream()));
+  g.go = at::empty_like(o);
+  const Tensor gw = empty_like_of(gy, {s.hid}, at::kFloat);
+  check("mxk_norm_bf16_bwd", mxk_norm_bf16_bwd(o.data_ptr(), norm_w.data_ptr(), nullptr, ptr(rstd), gn.data_ptr(), g.go.data_ptr(), ptr(gw), nullptr,
+                                               ws.data_ptr(), norm_bytes, s.M, s.hid, 1, stream()));
+  g.norm_w = gw.to(at::kBFloat16);
+  return g;
+}
+
+bool all_bf16(const Tensor& x, const variable_list& p) {
+  if (!x.is_cuda() || x.scalar_type() != at::kBFloat16 || x.dim() != 3 || x.numel() == 0 || x.size(0) * x.size(1) > 0x7fffffff ||
+      at::autocast::is_autocast_enabled(at::kCUDA))
+    return false;
+  for (const Tensor& t : p)
+    if (t.scalar_type() != at::kBFloat16 || t.device() != x.device() || !t.is_contiguous() || (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15)) return false;
+  return true;
+}
+bool wants_grad(const Tensor& x, const variable_list& p, std::initializer_list<Tensor> carry) {
+  if (!at::GradMode::is_enabled()) return false;
+  bool grad = x.requires_grad();
+  for (const Tensor& t : p) grad |= t.requires_grad();
+  for (const Tensor& t : carry) grad |= t.defined() && t.requires_grad();
+  return grad;
+}
+Tensor leaf(const OptTensor& t, const char* name) { return t && t->defined() ? dev(t->select(1, 0), at::kFloat, name) : Tensor(); }
+const uint8_t* cols_of(const Tensor& t, int64_t column) { return static_cast<const uint8_t*>(t.data_ptr()) + 2 * column; }
+uint8_t* cols_out(const Tensor& t, int64_t column) { return static_cast<uint8_t*>(t.data_ptr()) + 2 * column; }
+
+// ------------------------------------------------------------------------------------------------ linear attention
+enum { kQ, kK, kV, kNorm, kOutW, kOutB, kLinParams };
+
+struct LinAttnLayer : torch::autograd::Function<LinAttnLayer> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& wq, const Tensor& wk, const Tensor& wv, const Tensor& norm_w,
+                               const Tensor& out_w, const Tensor& out_b, const OptTensor& s0_in, const OptTensor& z0_in, const OptTensor& done_in,
+                               int64_t heads, double eps, double norm_eps);
+  static variable_list backward(AutogradContext* ctx, const variable_list& gout);
+};
+
+Shape shape_of(const Tensor& x, int64_t heads, int64_t hid, int64_t out, int64_t extra) {
+  Shape s;
+  s.B = x.size(0); s.T = x.size(1); s.F = x.size(2);
+  s.H = heads; s.hid = hid; s.d = hid / heads;
+  s.M = s.B * s.T;
+  s.out = out;
+  s.ld = (3 * hid + extra + 7) / 8 * 8;
+  return s;
+}
+
+struct LinResult {
+  Tensor s_last, z_last, y, proj, joint, states, o;
+  Tail tail;
+};
+LinResult linattn_forward(const Tensor& x, const variable_list& p, const Tensor& s0, const Tensor& z0, const Tensor& done, const Shape& s, double eps,
+                          double norm_eps, bool keep) {
+  LinResult r;
+  r.s_last = empty_like_of(x, {s.B, s.H, s.d, s.d}, at::kFloat);
+  r.z_last = empty_like_of(x, {s.B, s.H, s.d}, at::kFloat);
+  r.proj = project(x, p, 3, s, keep ? &r.joint : nullptr);
+  if (s.T == 1 && !keep && (s.d == 64 || s.d == 32) && s.hid <= 2048) {
+    const Tensor n = empty_like_of(x, {s.M, s.hid}, at::kBFloat16);
+    check("linattn_step", l::linattn_step(r.proj.data_ptr(), s.ld, ptr(s0), ptr(z0), bytes(done), p[kNorm].data_ptr(), norm_eps, eps, n.data_ptr(),
+                                          ptr(r.s_last), ptr(r.z_last), s.B, s.H, s.d, stream()));
+    r.y = output(n, p[kOutW], p[kOutB], s, true).view({s.B, s.T, s.out});
+    return r;
+  }
+  r.o = empty_like_of(x, {s.M, s.hid}, at::kBFloat16);
+  if (keep) r.states = scratch(x, mxk_linattn_chunk_states_bytes(s.B, s.T, s.H, s.d));
+  check("mxk_linattn_bf16_fwd", mxk::linattn::forward(cols_of(r.proj, 0), cols_of(r.proj, s.hid), cols_of(r.proj, 2 * s.hid), s.ld, ptr(s0), ptr(z0), bytes(done),
+                                                      r.o.data_ptr(), ptr(r.s_last), ptr(r.z_last), ptr<void>(r.states), status_ptr(x), s.B, s.T, s.H, s.d,
+                                                      eps, 1, stream()));
+  r.tail = norm_forward(r.o, p[kNorm], norm_eps, s);
+  r.y = output(r.tail.n, p[kOutW], p[kOutB], s, !keep).view({s.B, s.T, s.out});
+  return r;
+}
+
+variable_list LinAttnLayer::forward(AutogradContext* ctx, const Tensor& x, const Tensor& wq, const Tensor& wk, const Tensor& wv, const Tensor& norm_w,
+                                    const Tensor& out_w, const Tensor& out_b, const OptTensor& s0_in, const OptTensor& z0_in, const OptTensor& done_in,
+                                    int64_t heads, double eps, double norm_eps) {
+  const variable_list p{wq, wk, wv, norm_w, out_w, out_b};
+  const Tensor s0 = s0_in.value_or(Tensor()), z0 = z0_in.value_or(Tensor()), done = done_in.value_or(Tensor());
+  const Shape s = shape_of(x, heads, wq.size(0), out_w.size(0), 0);
+  LinResult r = linattn_forward(x, p, s0, z0, done, s, eps, norm_eps, true);
+  ctx->set_materialize_grads(false);
+  ctx->saved_data["heads"] = heads;
+  ctx->saved_data["eps"] = eps;
+  ctx->saved_data["s0"] = s0.defined();
+  ctx->saved_data["z0"] = z0.defined();
+  ctx->save_for_backward({x, norm_w, out_w, done, r.proj, r.joint, r.states, r.o, r.tail.n, r.tail.rstd});
+  return {r.s_last, r.z_last, r.y};
+}
+
+variable_list LinAttnLayer::backward(AutogradContext* ctx, const variable_list& gout) {
+  const variable_list saved = ctx->get_saved_variables();
+  const Tensor &x = saved[0], &norm_w = saved[1], &out_w = saved[2], &done = saved[3], &proj = saved[4], &joint = saved[5], &states = saved[6], &o = saved[7];
+  const c10::cuda::CUDAGuard guard(x.device());
+  const int64_t hid = out_w.size(1);
+  const Shape s = shape_of(x, ctx->saved_data["heads"].toInt(), hid, out_w.size(0), 0);
+  const Tensor gy = (gout[2].defined() ? gout[2].contiguous() : empty_like_of(x, {s.M, s.out}, at::kBFloat16).zero_()).view({s.M, s.out});
+  const Tensor gs = gout[0].defined() ? gout[0].contiguous() : Tensor(), gz = gout[1].defined() ? gout[1].contiguous() : Tensor();
+  const bool has_s = ctx->saved_data["s0"].toBool(), has_z = ctx->saved_data["z0"].toBool();
+  const bool need_s = (has_s && ctx->needs_input_grad(7)) || (has_z && ctx->needs_input_grad(has_s ? 8 : 7));
+  const TailGrads t = tail_backward(gy, o, saved[8], saved[9], norm_w, out_w, s);
+  const Tensor gproj = at::empty_like(proj);
+  const Tensor gs0 = need_s ? empty_like_of(x, {s.B, s.H, s.d, s.d}, at::kFloat) : Tensor(), gz0 = need_s ? empty_like_of(x, {s.B, s.H, s.d}, at::kFloat) : Tensor();
+  check("mxk_linattn_bf16_bwd", mxk::linattn::backward(cols_of(proj, 0), cols_of(proj, hid), cols_of(proj, 2 * hid), s.ld, t.go.data_ptr(), states.data_ptr(), bytes(done),
+                                                       ptr(gs), ptr(gz), cols_out(gproj, 0), cols_out(gproj, hid), cols_out(gproj, 2 * hid), s.ld, ptr(gs0), ptr(gz0),
+                                                       status_ptr(x), s.B, s.T, s.H, s.d, ctx->saved_data["eps"].toDouble(), 1, stream()));
+  variable_list grads(13);
+  if (ctx->needs_input_grad(0)) grads[0] = at::mm(gproj, joint).view(x.sizes());
+  const Tensor gw = at::mm(gproj.t(), x.view({s.M, s.F}));
+  for (int i = 0; i < 3; ++i) grads[1 + i] = gw.narrow(0, i * hid, hid);
+  grads[4] = t.norm_w;
+  grads[5] = t.out_w;
+  grads[6] = t.out_b;
+  if (has_s) grads[7] = gs0;
+  if (has_z) grads[8] = gz0;
+  return grads;
+}
+
+// -> (s_last (B,1,H,d,d), z_last (B,1,H,d), y (B,T,F)), or None where the caller has to compose the layer
+pybind11::object linattn_layer(const Tensor& x_in, const variable_list& p, const OptTensor& s0_in, const OptTensor& z0_in, const OptTensor& done_in,
+                               int64_t heads, double eps, double norm_eps) {
+  if (!all_bf16(x_in, p) || p.size() != kLinParams) return pybind11::none();
+  const int64_t hid = p[kQ].size(0), F = x_in.size(2), d = hid / heads;
+  if (d * heads != hid || d % 8 || d < 8 || d > 64 || hid > 1024 || F % 8 || p[kQ].size(1) != F || p[kOutW].size(1) != hid || p[kOutW].size(0) % 8 ||
+      x_in.size(0) * heads > 0x7fffffff)
+    return pybind11::none();
+  const c10::cuda::CUDAGuard guard(x_in.device());
+  const Tensor x = x_in.contiguous(), s0 = leaf(s0_in, "s0"), z0 = leaf(z0_in, "z0"), done = done_bytes(done_in);
+  if (wants_grad(x, p, {s0, z0})) {
+    const variable_list out = LinAttnLayer::apply(x, p[0], p[1], p[2], p[3], p[4], p[5], opt(s0), opt(z0), opt(done), heads, eps, norm_eps);
+    return pybind11::cast(std::make_tuple(out[0].unsqueeze(1), out[1].unsqueeze(1), out[2]));
+  }
+  const LinResult r = linattn_forward(x, p, s0, z0, done, shape_of(x, heads, hid, p[kOutW].size(0), 0), eps, norm_eps, false);
+  return pybind11::cast(std::make_tuple(r.s_last.unsqueeze(1), r.z_last.unsqueeze(1), r.y));
+}
+
+// ------------------------------------------------------------------------------------------------ gated delta rule
+enum { kDq, kDk, kDv, kGateW, kGateB, kDNorm, kDOutW, kDOutB, kDeltaParams };
+
+struct DeltaResult {
+  Tensor s_last, y, proj, joint, q, k, alpha, beta, states, ws, o;
+  Tail tail;
+};
+DeltaResult delta_forward(const Tensor& x, const variable_list& p, const Tensor& s0, const Tensor& done, const Shape& s, double norm_eps, bool keep) {
+  DeltaResult r;
+  r.s_last = empty_like_of(x, {s.B, s.H, s.d, s.d}, at::kFloat);
+  r.proj = project(x, p, 4, s, keep ? &r.joint : nullptr);
+  if (s.T == 1 && !keep && s.hid <= 2048) {
+    const Tensor n = empty_like_of(x, {s.M, s.hid}, at::kBFloat16);
+    check("gdelta_step", l::gdelta_step(r.proj.data_ptr(), s.ld, p[kGateB].data_ptr(), ptr(s0), bytes(done), p[kDNorm].data_ptr(), norm_eps, n.data_ptr(),
+                                        ptr(r.s_last), s.B, s.H, s.d, stream()));
+    r.y = output(n, p[kDOutW], p[kDOutB], s, true).view({s.B, s.T, s.out});
+    return r;
+  }
+  r.q = empty_like_of(x, {s.M, s.hid}, at::kBFloat16);
+  r.k = empty_like_of(x, {s.M, s.hid}, at::kBFloat16);
+  r.alpha = empty_like_of(x, {s.M, s.H}, at::kFloat);
+  r.beta = empty_like_of(x, {s.M, s.H}, at::kFloat);
+  r.o = empty_like_of(x, {s.M, s.hid}, at::kBFloat16);
+  if (keep) r.states = scratch(x, mxk_gdelta_chunk_states_bytes(s.B, s.T, s.H, s.d));
+  const size_t ws_bytes = mxk_gdelta_workspace_bytes(s.B, s.T, s.H, s.d);
+  r.ws = scratch(x, ws_bytes);
+  check("delta_inputs", l::delta_inputs(r.proj.data_ptr(), s.ld, p[kGateB].data_ptr(), r.q.data_ptr(), r.k.data_ptr(), ptr(r.alpha), ptr(r.beta), s.M, s.H, s.d, stream()));
+  check("mxk_gdelta_bf16_fwd", mxk::gdelta::forward(r.q.data_ptr(), r.k.data_ptr(), cols_of(r.proj, 2 * s.hid), s.ld, ptr(r.alpha), ptr(r.beta), ptr(s0), bytes(done),
+                                                    r.o.data_ptr(), ptr(r.s_last), ptr<void>(r.states), r.ws.data_ptr(), ws_bytes, status_ptr(x), s.B, s.T, s.H,
+                                                    s.d, stream()));
+  r.tail = norm_forward(r.o, p[kDNorm], norm_eps, s);
+  r.y = output(r.tail.n, p[kDOutW], p[kDOutB], s, !keep).view({s.B, s.T, s.out});
+  return r;
+}
+
+struct DeltaLayer : torch::autograd::Function<DeltaLayer> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& wq, const Tensor& wk, const Tensor& wv, const Tensor& gate_w,
+                               const Tensor& gate_b, const Tensor& norm_w, const Tensor& out_w, const Tensor& out_b, const OptTensor& s0_in,
+                               const OptTensor& done_in, int64_t heads, double norm_eps) {
+    const variable_list p{wq, wk, wv, gate_w, gate_b, norm_w, out_w, out_b};
+    const Tensor s0 = s0_in.value_or(Tensor()), done = done_in.value_or(Tensor());
+    const Shape s = shape_of(x, heads, wq.size(0), out_w.size(0), 2 * heads);
+    DeltaResult r = delta_forward(x, p, s0, done, s, norm_eps, true);
+    ctx->set_materialize_grads(false);
+    ctx->saved_data["heads"] = heads;
+    ctx->saved_data["s0"] = s0.defined();
+    ctx->save_for_backward({x, gate_b, norm_w, out_w, done, r.proj, r.joint, r.q, r.k, r.alpha, r.beta, r.states, r.ws, r.o, r.tail.n, r.tail.rstd});
+    return {r.s_last, r.y};
+  }
+
+  static variable_list backward(AutogradContext* ctx, const variable_list& gout) {
+    const variable_list saved = ctx->get_saved_variables();
+    const Tensor &x = saved[0], &gate_b = saved[1], &norm_w = saved[2], &out_w = saved[3], &done = saved[4], &proj = saved[5], &joint = saved[6];
+    const Tensor &q = saved[7], &k = saved[8], &alpha = saved[9], &beta = saved[10], &states = saved[11], &ws = saved[12], &o = saved[13];
+    const c10::cuda::CUDAGuard guard(x.device());
+    const int64_t hid = out_w.size(1);
+    const Shape s = shape_of(x, ctx->saved_data["heads"].toInt(), hid, out_w.size(0), 2 * ctx->saved_data["heads"].toInt());
+    const Tensor gy = (gout[1].defined() ? gout[1].contiguous() : empty_like_of(x, {s.M, s.out}, at::kBFloat16).zero_()).view({s.M, s.out});
+    const Tensor gs = gout[0].defined() ? gout[0].contiguous() : Tensor();
+    const bool need_s0 = ctx->saved_data["s0"].toBool() && ctx->needs_input_grad(9);
+    const TailGrads t = tail_backward(gy, o, saved[14], saved[15], norm_w, out_w, s);
+    const Tensor gproj = at::empty_like(proj), gq = at::empty_like(q), gk = at::empty_like(k);
+    const Tensor ga = at::empty_like(alpha), gb = at::empty_like(beta);
+    variable_list grads(13);
+    if (need_s0) grads[9] = empty_like_of(x, {s.B, s.H, s.d, s.d}, at::kFloat);
+    check("mxk_gdelta_bf16_bwd", mxk::gdelta::backward(q.data_ptr(), k.data_ptr(), cols_of(proj, 2 * hid), ptr(alpha), ptr(beta), t.go.data_ptr(), states.data_ptr(), ws.data_ptr(),
+                                                       bytes(done), ptr(gs), gq.data_ptr(), gk.data_ptr(), cols_out(gproj, 2 * hid), s.ld, ptr(ga), ptr(gb),
+                                                       need_s0 ? ptr(grads[9]) : nullptr, status_ptr(x), s.B, s.T, s.H, s.d, stream()));
+    const int rows = l::delta_gate_blocks(s.M);
+    const Tensor part = empty_like_of(x, {rows + 1, 2 * s.H}, at::kFloat);
+    check("delta_inputs_bwd", l::delta_inputs_bwd(proj.data_ptr(), s.ld, gate_b.data_ptr(), gq.data_ptr(), gk.data_ptr(), ptr(ga), ptr(gb), gproj.data_ptr(), ptr(part), s.M, s.H,
+                                                  s.d, stream()));
+    const l::ColumnSum sum{ptr(part), rows, 2 * s.H, ptr(part) + static_cast<size_t>(rows) * 2 * s.H};
+    check("column_sums", l::column_sums(&sum, 1, stream()));
+    if (ctx->needs_input_grad(0)) grads[0] = at::mm(gproj, joint).view(x.sizes());
+    const Tensor rows_in = x.view({s.M, s.F}), gw = at::mm(gproj.narrow(1, 0, 3 * hid).t(), rows_in);
+    for (int i = 0; i < 3; ++i) grads[1 + i] = gw.narrow(0, i * hid, hid);
+    grads[4] = at::mm(gproj.narrow(1, 3 * hid, 2 * s.H).t(), rows_in);
+    grads[5] = part[rows].to(at::kBFloat16);
+    grads[6] = t.norm_w;
+    grads[7] = t.out_w;
+    grads[8] = t.out_b;
+    return grads;
+  }
+};
+
+// -> (s_last (B,1,H,d,d), y (B,T,F)), or None
+pybind11::object deltanet_layer(const Tensor& x_in, const variable_list& p, const OptTensor& s0_in, const OptTensor& done_in, int64_t heads, double norm_eps) {
+  if (!all_bf16(x_in, p) || p.size() != kDeltaParams) return pybind11::none();
+  const int64_t hid = p[kDq].size(0), F = x_in.size(2), d = hid / heads;
+  if (d * heads != hid || (d != 64 && d != 128) || hid > 1024 || heads > 64 || F % 8 || p[kDq].size(1) != F || p[kDOutW].size(1) != hid || p[kDOutW].size(0) % 8 ||
+      p[kGateW].size(0) != 2 * heads || x_in.size(0) * heads > 0x7fffffff)
+    return pybind11::none();
+  const c10::cuda::CUDAGuard guard(x_in.device());
+  const Tensor x = x_in.contiguous(), s0 = leaf(s0_in, "s0"), done = done_bytes(done_in);
+  if (wants_grad(x, p, {s0})) {
+    const variable_list out = DeltaLayer::apply(x, p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7], opt(s0), opt(done), heads, norm_eps);
+    return pybind11::cast(std::make_tuple(out[0].unsqueeze(1), out[1]));
+  }
+  const DeltaResult r = delta_forward(x, p, s0, done, shape_of(x, heads, hid, p[kDOutW].size(0), 2 * heads), norm_eps, false);
+  return pybind11::cast(std::make_tuple(r.s_last.unsqueeze(1), r.y));
+}
+
+}  // namespace
+
+void bind_attention(pybind11::module_& m) {
+  m.def("linattn_layer", &linattn_layer);
+  m.def("deltanet_layer", &deltanet_layer);
+}
+
+}  // namespace mxk_host

@@ -62,6 +62,7 @@ struct Arena {
   template <typename T = float> T* at(size_t off) const { return reinterpret_cast<T*>(base + off); }
 };
 
+void bind_attention(pybind11::module_& m);
 void bind_linrec(pybind11::module_& m);
 void bind_linear(pybind11::module_& m);
 void bind_lru(pybind11::module_& m);

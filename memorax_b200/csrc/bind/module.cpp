@@ -31,6 +31,7 @@ void assertion(const char* text) {
 PYBIND11_MODULE(_C, m) {
   using namespace mxk_host;
   m.def("status_word", [](const std::string& device) { return status_word(c10::Device(device)); });
+  bind_attention(m);
   bind_linrec(m);
   bind_linear(m);
   bind_lru(m);

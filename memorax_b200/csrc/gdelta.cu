@@ -13,6 +13,7 @@
 //   epilogue 3: output tile (one TMA store), bf16 operand copy of the new state.
 #include <cstddef>
 
+#include "attention.cuh"
 #include "gdelta_common.cuh"
 #include "tma.cuh"
 
@@ -399,26 +400,13 @@ extern "C" int mxk_debug_gdf_phase_cycles(unsigned long long* out, int reset) {
 }
 #endif
 
-extern "C" {
+namespace mxk {
+namespace gdelta {
 
-size_t mxk_gdelta_chunk_states_bytes(int B, int T, int H, int d) {
-  if (B <= 0 || T <= 0 || H <= 0 || (d != mxk::gdelta::kD && d != 64)) return 0;
-  const size_t nchunks = (static_cast<size_t>(T) + mxk::gdelta::kC - 1) / mxk::gdelta::kC;
-  return static_cast<size_t>(B) * H * nchunks * mxk::gdelta::kResidualVecs * sizeof(uint4);
-}
-
-size_t mxk_gdelta_workspace_bytes(int B, int T, int H, int d) {
-  if (B <= 0 || T <= 0 || H <= 0 || (d != mxk::gdelta::kD && d != 64)) return 0;
-  const size_t nchunks = (static_cast<size_t>(T) + mxk::gdelta::kC - 1) / mxk::gdelta::kC;
-  return static_cast<size_t>(B) * H * nchunks * mxk::gdelta::kAinvVecs * sizeof(uint4);
-}
-
-int mxk_gdelta_bf16_fwd(const void* q, const void* k, const void* v, const float* alpha, const float* beta,
+int forward(const void* q, const void* k, const void* v, long long ld_v, const float* alpha, const float* beta,
                         const float* s0, const uint8_t* done, void* o, float* s_last, void* chunk_states,
                         void* workspace, size_t workspace_bytes, int* status, int B, int T, int H, int d,
-                        mxk_stream_t stream) {
-  using namespace mxk;
-  using namespace mxk::gdelta;
+                        cudaStream_t stream) {
   if (!q || !k || !v || !alpha || !beta || !o) return MXK_ERR_NULL;
   if (B <= 0 || T <= 0 || H <= 0 || static_cast<long long>(B) * H > 0x7fffffffLL) return MXK_ERR_DIMS;
   if (d != kD && d != 64) return MXK_ERR_UNSUPPORTED;
@@ -441,15 +429,40 @@ int mxk_gdelta_bf16_fwd(const void* q, const void* k, const void* v, const float
   prm.status = status;
   prm.B = B; prm.T = T; prm.H = H; prm.d = d;
   if (!tma::make_sw_map(&prm.map_k, k, B, T, H, kC, d) || !tma::make_sw_map(&prm.map_q, q, B, T, H, kC, d) ||
-      !tma::make_sw_map(&prm.map_v, v, B, T, H, kC, d) || !tma::make_plain_map(&prm.map_o, o, B, T, H, d, kC, kD))
+      !tma::make_sw_map(&prm.map_v, v, B, T, H, kC, d, ld_v) || !tma::make_plain_map(&prm.map_o, o, B, T, H, d, kC, kD))
     return MXK_ERR_UNSUPPORTED;
-  const int st = launch_prep(k, alpha, beta, done, workspace, status, B, T, H, d, static_cast<cudaStream_t>(stream));
+  const int st = launch_prep(k, alpha, beta, done, workspace, status, B, T, H, d, stream);
   if (st != MXK_OK) return st;
   cudaError_t e = cudaFuncSetAttribute(gdelta_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(sizeof(FwdSmem)));
   if (e != cudaSuccess) return static_cast<int>(e);
-  gdelta_fwd_kernel<<<B * H, kFwdThreads, sizeof(FwdSmem), static_cast<cudaStream_t>(stream)>>>(prm);
+  gdelta_fwd_kernel<<<B * H, kFwdThreads, sizeof(FwdSmem), stream>>>(prm);
   return launch_status();
+}
+
+}  // namespace gdelta
+}  // namespace mxk
+
+extern "C" {
+
+size_t mxk_gdelta_chunk_states_bytes(int B, int T, int H, int d) {
+  if (B <= 0 || T <= 0 || H <= 0 || (d != mxk::gdelta::kD && d != 64)) return 0;
+  const size_t nchunks = (static_cast<size_t>(T) + mxk::gdelta::kC - 1) / mxk::gdelta::kC;
+  return static_cast<size_t>(B) * H * nchunks * mxk::gdelta::kResidualVecs * sizeof(uint4);
+}
+
+size_t mxk_gdelta_workspace_bytes(int B, int T, int H, int d) {
+  if (B <= 0 || T <= 0 || H <= 0 || (d != mxk::gdelta::kD && d != 64)) return 0;
+  const size_t nchunks = (static_cast<size_t>(T) + mxk::gdelta::kC - 1) / mxk::gdelta::kC;
+  return static_cast<size_t>(B) * H * nchunks * mxk::gdelta::kAinvVecs * sizeof(uint4);
+}
+
+int mxk_gdelta_bf16_fwd(const void* q, const void* k, const void* v, const float* alpha, const float* beta,
+                        const float* s0, const uint8_t* done, void* o, float* s_last, void* chunk_states,
+                        void* workspace, size_t workspace_bytes, int* status, int B, int T, int H, int d,
+                        mxk_stream_t stream) {
+  return mxk::gdelta::forward(q, k, v, 0, alpha, beta, s0, done, o, s_last, chunk_states, workspace, workspace_bytes, status, B, T,
+                              H, d, static_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

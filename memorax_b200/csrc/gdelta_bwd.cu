@@ -19,6 +19,7 @@
 // Matrices with d_v on their rows are kept transposed ([v][t]) so that thread v
 // owns one value column, as in the forward kernel; dQ and dK are accumulated transposed too
 // ([feature][token], M = 128 products: the full tensor datapath instead of half of it).
+#include "attention.cuh"
 #include "gdelta_common.cuh"
 #include "tma.cuh"
 
@@ -635,15 +636,14 @@ extern "C" int mxk_debug_gd_phase_cycles(unsigned long long* out, int reset) {
   return (int)cudaMemcpyFromSymbol(out, mxk::g_gd_phase_cycles, 24 * sizeof(unsigned long long));
 }
 
-extern "C" {
+namespace mxk {
+namespace gdelta {
 
-int mxk_gdelta_bf16_bwd(const void* q, const void* k, const void* v, const float* alpha, const float* beta,
+int backward(const void* q, const void* k, const void* v, const float* alpha, const float* beta,
                         const void* d_o, const void* chunk_states, const void* workspace, const uint8_t* done,
                         const float* ds_last,
-                        void* dq, void* dk, void* dv, float* dalpha, float* dbeta, float* ds0, int* status,
-                        int B, int T, int H, int d, mxk_stream_t stream) {
-  using namespace mxk;
-  using namespace mxk::gdelta;
+                        void* dq, void* dk, void* dv, long long ld_dv, float* dalpha, float* dbeta, float* ds0, int* status,
+                        int B, int T, int H, int d, cudaStream_t stream) {
   if (!q || !k || !v || !alpha || !beta || !d_o || !chunk_states || !workspace || !dq || !dk || !dv || !dalpha || !dbeta)
     return MXK_ERR_NULL;
   if (B <= 0 || T <= 0 || H <= 0 || static_cast<long long>(B) * H > 0x7fffffffLL) return MXK_ERR_DIMS;
@@ -677,13 +677,27 @@ int mxk_gdelta_bf16_bwd(const void* q, const void* k, const void* v, const float
   }
   if (!tma::make_sw_map(&prm.map_k, k, B, T, H, kC, d) || !tma::make_sw_map(&prm.map_q, q, B, T, H, kC, d) ||
       !tma::make_sw_map(&prm.map_do, d_o, B, T, H, kC, d) || !tma::make_sw_map(&prm.map_dq, dq, B, T, H, kC, d) ||
-      !tma::make_sw_map(&prm.map_dk, dk, B, T, H, kC, d) || !tma::make_plain_map(&prm.map_dv, dv, B, T, H, d, kC, kD))
+      !tma::make_sw_map(&prm.map_dk, dk, B, T, H, kC, d) || !tma::make_plain_map(&prm.map_dv, dv, B, T, H, d, kC, kD, ld_dv))
     return MXK_ERR_UNSUPPORTED;
   cudaError_t e = cudaFuncSetAttribute(gdelta_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(sizeof(BwdSmem)));
   if (e != cudaSuccess) return static_cast<int>(e);
-  gdelta_bwd_kernel<<<B * H, kBwdThreads, sizeof(BwdSmem), static_cast<cudaStream_t>(stream)>>>(prm);
+  gdelta_bwd_kernel<<<B * H, kBwdThreads, sizeof(BwdSmem), stream>>>(prm);
   return launch_status();
+}
+
+}  // namespace gdelta
+}  // namespace mxk
+
+extern "C" {
+
+int mxk_gdelta_bf16_bwd(const void* q, const void* k, const void* v, const float* alpha, const float* beta,
+                        const void* d_o, const void* chunk_states, const void* workspace, const uint8_t* done,
+                        const float* ds_last,
+                        void* dq, void* dk, void* dv, float* dalpha, float* dbeta, float* ds0, int* status,
+                        int B, int T, int H, int d, mxk_stream_t stream) {
+  return mxk::gdelta::backward(q, k, v, alpha, beta, d_o, chunk_states, workspace, done, ds_last, dq, dk, dv, 0, dalpha, dbeta, ds0,
+                               status, B, T, H, d, static_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

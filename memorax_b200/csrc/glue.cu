@@ -3,8 +3,7 @@
 //     RMSNorm in front of the cells' output projection, linear_attention.py:114),
 //   - the gated residual y = x + sigmoid(g) * o and its backward (blocks/residual.py:53-59),
 //   - per-head L2 normalisation of q / k and its backward (the delta-rule cell's key / query normalisation).
-// One warp owns one row of D <= 1024 elements (D a multiple of 256): each lane holds D / 32 of them as 16-byte
-// vectors, statistics are warp reductions, nothing goes through shared memory.  The (D,) parameter gradients
+// One warp owns one row of D <= 1024 elements (D a multiple of 8): each lane holds up to 4 16-byte vectors of it, statistics are warp reductions, nothing goes through shared memory.  The (D,) parameter gradients
 // are accumulated per warp in registers over a grid-stride loop of rows, combined per block in shared memory
 // and written as one partial row per block; a second kernel adds the blocks in index order (no atomics:
 // bit-reproducible).
@@ -24,45 +23,52 @@ __device__ __forceinline__ float warp_sum(float x) {
   return x;
 }
 
-// V = D / 256 16-byte vectors per lane; lane l owns elements [v * 256 + l * 8, + 8).
+// V = ceil(D / 256) 16-byte vectors per lane; lane l owns elements [v * 256 + l * 8, + 8), those past D read as zero.
 template <int V>
-__device__ __forceinline__ void load_row(const __nv_bfloat16* row, int lane, float (*x)[8]) {
+__device__ __forceinline__ void load_row(const __nv_bfloat16* row, int lane, int D, float (*x)[8]) {
 #pragma unroll
-  for (int v = 0; v < V; ++v) umma::unpack8_bf16(*reinterpret_cast<const uint4*>(row + v * 256 + lane * 8), x[v]);
+  for (int v = 0; v < V; ++v) {
+    const int at = v * 256 + lane * 8;
+    umma::unpack8_bf16(at < D ? *reinterpret_cast<const uint4*>(row + at) : make_uint4(0, 0, 0, 0), x[v]);
+  }
 }
 template <int V>
-__device__ __forceinline__ void store_row(__nv_bfloat16* row, int lane, const float (*y)[8]) {
+__device__ __forceinline__ void store_row(__nv_bfloat16* row, int lane, int D, const float (*y)[8]) {
 #pragma unroll
-  for (int v = 0; v < V; ++v) *reinterpret_cast<uint4*>(row + v * 256 + lane * 8) = umma::pack8_bf16(y[v]);
+  for (int v = 0; v < V; ++v)
+    if (v * 256 + lane * 8 < D) *reinterpret_cast<uint4*>(row + v * 256 + lane * 8) = umma::pack8_bf16(y[v]);
 }
 
 template <int V, bool RMS>
 __global__ void __launch_bounds__(kRowWarps * 32)
 norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gamma,
                 const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* __restrict__ y, float* __restrict__ mean,
-                float* __restrict__ rstd, long long rows, float eps) {
-  constexpr int D = V * 256;
+                float* __restrict__ rstd, long long rows, int D, float eps) {
+  const float inv_d = 1.f / static_cast<float>(D);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float g[V][8], b[V][8];
-  load_row<V>(gamma, lane, g);
-  if (!RMS && beta) load_row<V>(beta, lane, b);
+  load_row<V>(gamma, lane, D, g);
+  if (!RMS && beta) load_row<V>(beta, lane, D, b);
   for (long long r = static_cast<long long>(blockIdx.x) * kRowWarps + warp; r < rows; r += static_cast<long long>(gridDim.x) * kRowWarps) {
     float xv[V][8];
-    load_row<V>(x + r * D, lane, xv);
+    load_row<V>(x + r * D, lane, D, xv);
     float s = 0.f;
     if (!RMS) {
 #pragma unroll
       for (int v = 0; v < V; ++v)
 #pragma unroll
         for (int e = 0; e < 8; ++e) s += xv[v][e];
-      s = warp_sum(s) * (1.f / D);
+      s = warp_sum(s) * inv_d;
     }
     float q = 0.f;
 #pragma unroll
     for (int v = 0; v < V; ++v)
 #pragma unroll
-      for (int e = 0; e < 8; ++e) { const float c = xv[v][e] - s; q = fmaf(c, c, q); }
-    const float rs = rsqrtf(warp_sum(q) * (1.f / D) + eps);
+      for (int e = 0; e < 8; ++e) {
+        const float c = v * 256 + lane * 8 < D ? xv[v][e] - s : 0.f;
+        q = fmaf(c, c, q);
+      }
+    const float rs = rsqrtf(warp_sum(q) * inv_d + eps);
 #pragma unroll
     for (int v = 0; v < V; ++v)
 #pragma unroll
@@ -70,7 +76,7 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
         const float h = (xv[v][e] - s) * rs * g[v][e];
         xv[v][e] = (!RMS && beta) ? h + b[v][e] : h;
       }
-    store_row<V>(y + r * D, lane, xv);
+    store_row<V>(y + r * D, lane, D, xv);
     if (lane == 0) {
       if (mean) mean[r] = s;
       rstd[r] = rs;
@@ -83,20 +89,20 @@ template <int V, bool RMS>
 __global__ void __launch_bounds__(kRowWarps * 32)
 norm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gamma, const float* __restrict__ mean,
                 const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ dy, __nv_bfloat16* __restrict__ dx,
-                float* __restrict__ part, long long rows) {
-  constexpr int D = V * 256;
-  __shared__ float red[kRowWarps][D];
+                float* __restrict__ part, long long rows, int D) {
+  const float inv_d = 1.f / static_cast<float>(D);
+  __shared__ float red[kRowWarps][V * 256];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float g[V][8], dg[V][8], db[V][8];
-  load_row<V>(gamma, lane, g);
+  load_row<V>(gamma, lane, D, g);
 #pragma unroll
   for (int v = 0; v < V; ++v)
 #pragma unroll
     for (int e = 0; e < 8; ++e) dg[v][e] = db[v][e] = 0.f;
   for (long long r = static_cast<long long>(blockIdx.x) * kRowWarps + warp; r < rows; r += static_cast<long long>(gridDim.x) * kRowWarps) {
     float xv[V][8], dv[V][8];
-    load_row<V>(x + r * D, lane, xv);
-    load_row<V>(dy + r * D, lane, dv);
+    load_row<V>(x + r * D, lane, D, xv);
+    load_row<V>(dy + r * D, lane, D, dv);
     const float mu = RMS ? 0.f : mean[r], rs = rstd[r];
     float s1 = 0.f, s2 = 0.f;
 #pragma unroll
@@ -111,13 +117,13 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
         s1 += gy;
         s2 = fmaf(gy, xh, s2);
       }
-    s1 = RMS ? 0.f : warp_sum(s1) * (1.f / D);
-    s2 = warp_sum(s2) * (1.f / D);
+    s1 = RMS ? 0.f : warp_sum(s1) * inv_d;   // (elements past D have dy = gamma = 0)
+    s2 = warp_sum(s2) * inv_d;
 #pragma unroll
     for (int v = 0; v < V; ++v)
 #pragma unroll
       for (int e = 0; e < 8; ++e) xv[v][e] = rs * (dv[v][e] - s1 - xv[v][e] * s2);
-    store_row<V>(dx + r * D, lane, xv);
+    store_row<V>(dx + r * D, lane, D, xv);
   }
   // block partials: the eight warps' sums added in warp order
   for (int pass = 0; pass < (RMS ? 1 : 2); ++pass) {
@@ -335,7 +341,7 @@ l2norm_kernel(const uint4* __restrict__ x, const uint4* __restrict__ dy, uint4* 
 int check_norm(const void* x, const void* gamma, const void* y, long long rows, int D) {
   if (!x || !gamma || !y) return MXK_ERR_NULL;
   if (rows <= 0 || D <= 0) return MXK_ERR_DIMS;
-  if (D % 256 != 0 || D > 1024) return MXK_ERR_UNSUPPORTED;
+  if (D % 8 != 0 || D > 1024) return MXK_ERR_UNSUPPORTED;
   for (const void* p : {x, gamma, y})
     if (!aligned16(p)) return MXK_ERR_ALIGN;
   return MXK_OK;
@@ -404,9 +410,9 @@ int mxk_norm_bf16_fwd(const void* x, const void* gamma, const void* beta, void* 
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int blocks = norm_blocks(rows, 8), threads = kRowWarps * 32;
 #define MXK_NORM_FWD(V)                                                                                        \
-  if (rms) norm_fwd_kernel<V, true><<<blocks, threads, 0, s>>>(xp, gp, nullptr, yp, nullptr, rstd, rows, eps); \
-  else norm_fwd_kernel<V, false><<<blocks, threads, 0, s>>>(xp, gp, bp, yp, mean, rstd, rows, eps);
-  switch (D / 256) {
+  if (rms) norm_fwd_kernel<V, true><<<blocks, threads, 0, s>>>(xp, gp, nullptr, yp, nullptr, rstd, rows, D, eps); \
+  else norm_fwd_kernel<V, false><<<blocks, threads, 0, s>>>(xp, gp, bp, yp, mean, rstd, rows, D, eps);
+  switch ((D + 255) / 256) {
     case 1: MXK_NORM_FWD(1) break;
     case 2: MXK_NORM_FWD(2) break;
     case 3: MXK_NORM_FWD(3) break;
@@ -432,9 +438,9 @@ int mxk_norm_bf16_bwd(const void* x, const void* gamma, const float* mean, const
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int blocks = norm_blocks(rows), threads = kRowWarps * 32;
 #define MXK_NORM_BWD(V)                                                                                  \
-  if (rms) norm_bwd_kernel<V, true><<<blocks, threads, 0, s>>>(xp, gp, nullptr, rstd, dyp, dxp, part, rows); \
-  else norm_bwd_kernel<V, false><<<blocks, threads, 0, s>>>(xp, gp, mean, rstd, dyp, dxp, part, rows);
-  switch (D / 256) {
+  if (rms) norm_bwd_kernel<V, true><<<blocks, threads, 0, s>>>(xp, gp, nullptr, rstd, dyp, dxp, part, rows, D); \
+  else norm_bwd_kernel<V, false><<<blocks, threads, 0, s>>>(xp, gp, mean, rstd, dyp, dxp, part, rows, D);
+  switch ((D + 255) / 256) {
     case 1: MXK_NORM_BWD(1) break;
     case 2: MXK_NORM_BWD(2) break;
     case 3: MXK_NORM_BWD(3) break;

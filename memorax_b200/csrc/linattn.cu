@@ -21,6 +21,7 @@
 #include <cstddef>
 
 #include "mxk_common.cuh"
+#include "attention.cuh"
 #include "linattn_common.cuh"
 #include "tma.cuh"
 
@@ -375,19 +376,13 @@ extern "C" int mxk_debug_phase_cycles(unsigned long long* out, int reset) {
 }
 #endif
 
-extern "C" {
+namespace mxk {
+namespace linattn {
 
-size_t mxk_linattn_chunk_states_bytes(int B, int T, int H, int d) {
-  if (B <= 0 || T <= 0 || H <= 0 || d < 8 || d > mxk::linattn::kD || d % 8) return 0;
-  const size_t nchunks = (static_cast<size_t>(T) + mxk::linattn::kC - 1) / mxk::linattn::kC;
-  return static_cast<size_t>(B) * H * nchunks * (mxk::linattn::kPanelsX * mxk::linattn::kD) * sizeof(uint4);
-}
-
-int mxk_linattn_bf16_fwd(const void* q, const void* k, const void* v, const float* s0, const float* z0,
+int forward(const void* q, const void* k, const void* v, long long ld, const float* s0, const float* z0,
                          const uint8_t* done, void* o, float* s_last, float* z_last, void* chunk_states,
                          int* status, int B, int T, int H, int d, float eps, int feature_map,
-                         mxk_stream_t stream) {
-  using namespace mxk;
+                         cudaStream_t stream) {
   if (!q || !k || !v || !o) return MXK_ERR_NULL;
   if (B <= 0 || T <= 0 || H <= 0 || static_cast<long long>(B) * H > 0x7fffffffLL) return MXK_ERR_DIMS;
   if (d < 8 || d > kD || d % 8) return MXK_ERR_UNSUPPORTED;
@@ -414,14 +409,33 @@ int mxk_linattn_bf16_fwd(const void* q, const void* k, const void* v, const floa
   prm.state_bulk = (!s0 || aligned16(s0)) && (!z0 || aligned16(z0));
   // maps over the d-column tensors with 64-column boxes: the columns past d are zero-filled on loads and
   // clipped on stores
-  if (!tma::make_sw_map(&prm.map_q, q, B, T, H, kC, d) || !tma::make_sw_map(&prm.map_k, k, B, T, H, kC, d) ||
-      !tma::make_panel_map(&prm.map_v, v, B, T, H, d, kC, kPanels) || !tma::make_sw_map(&prm.map_o, o, B, T, H, kC, d))
+  if (!tma::make_sw_map(&prm.map_q, q, B, T, H, kC, d, ld) || !tma::make_sw_map(&prm.map_k, k, B, T, H, kC, d, ld) ||
+      !tma::make_panel_map(&prm.map_v, v, B, T, H, d, kC, kPanels, ld) || !tma::make_sw_map(&prm.map_o, o, B, T, H, kC, d))
     return MXK_ERR_UNSUPPORTED;
   auto kernel = d == kD ? linattn_fwd_kernel<true> : linattn_fwd_kernel<false>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(FwdSmem)));
   if (e != cudaSuccess) return static_cast<int>(e);
-  kernel<<<B * H, kThreads, sizeof(FwdSmem), static_cast<cudaStream_t>(stream)>>>(prm);
+  kernel<<<B * H, kThreads, sizeof(FwdSmem), stream>>>(prm);
   return launch_status();
+}
+
+}  // namespace linattn
+}  // namespace mxk
+
+extern "C" {
+
+size_t mxk_linattn_chunk_states_bytes(int B, int T, int H, int d) {
+  if (B <= 0 || T <= 0 || H <= 0 || d < 8 || d > mxk::linattn::kD || d % 8) return 0;
+  const size_t nchunks = (static_cast<size_t>(T) + mxk::linattn::kC - 1) / mxk::linattn::kC;
+  return static_cast<size_t>(B) * H * nchunks * (mxk::linattn::kPanelsX * mxk::linattn::kD) * sizeof(uint4);
+}
+
+int mxk_linattn_bf16_fwd(const void* q, const void* k, const void* v, const float* s0, const float* z0,
+                         const uint8_t* done, void* o, float* s_last, float* z_last, void* chunk_states,
+                         int* status, int B, int T, int H, int d, float eps, int feature_map,
+                         mxk_stream_t stream) {
+  return mxk::linattn::forward(q, k, v, 0, s0, z0, done, o, s_last, z_last, chunk_states, status, B, T, H, d, eps, feature_map,
+                               static_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

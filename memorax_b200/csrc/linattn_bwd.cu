@@ -20,6 +20,7 @@
 //   bf16 operand copy of G.
 #include <cuda_bf16.h>
 
+#include "attention.cuh"
 #include "linattn_common.cuh"
 #include "mxk_common.cuh"
 #include "tma.cuh"
@@ -509,14 +510,13 @@ extern "C" int mxk_debug_bwd_phase_cycles(unsigned long long* out, int reset) {
 }
 #endif
 
-extern "C" {
+namespace mxk {
+namespace linattn {
 
-int mxk_linattn_bf16_bwd(const void* q, const void* k, const void* v, const void* d_o, const void* chunk_states,
+int backward(const void* q, const void* k, const void* v, long long ld, const void* d_o, const void* chunk_states,
                          const uint8_t* done, const float* ds_last, const float* dz_last, void* dq, void* dk,
-                         void* dv, float* ds0, float* dz0, int* status, int B, int T, int H, int d, float eps,
-                         int feature_map, mxk_stream_t stream) {
-  using namespace mxk;
-  using namespace mxk::linattn;
+                         void* dv, long long ld_grad, float* ds0, float* dz0, int* status, int B, int T, int H, int d, float eps,
+                         int feature_map, cudaStream_t stream) {
   if (!q || !k || !v || !d_o || !chunk_states || !dq || !dk || !dv) return MXK_ERR_NULL;
   if (B <= 0 || T <= 0 || H <= 0 || static_cast<long long>(B) * H > 0x7fffffffLL) return MXK_ERR_DIMS;
   if (d < 8 || d > kD || d % 8) return MXK_ERR_UNSUPPORTED;
@@ -545,17 +545,30 @@ int mxk_linattn_bf16_bwd(const void* q, const void* k, const void* v, const void
   prm.d = d;
   // maps over the d-column tensors with 64-column boxes: the columns past d are zero-filled on loads and
   // clipped on stores
-  if (!tma::make_sw_map(&prm.map_q, q, B, T, H, kC, d) || !tma::make_sw_map(&prm.map_k, k, B, T, H, kC, d) ||
-      !tma::make_sw_map(&prm.map_v, v, B, T, H, kC, d) || !tma::make_sw_map(&prm.map_do, d_o, B, T, H, kC, d))
+  if (!tma::make_sw_map(&prm.map_q, q, B, T, H, kC, d, ld) || !tma::make_sw_map(&prm.map_k, k, B, T, H, kC, d, ld) ||
+      !tma::make_sw_map(&prm.map_v, v, B, T, H, kC, d, ld) || !tma::make_sw_map(&prm.map_do, d_o, B, T, H, kC, d))
     return MXK_ERR_UNSUPPORTED;
-  if (!tma::make_sw_map(&prm.map_dq, dq, B, T, H, kC, d) || !tma::make_sw_map(&prm.map_dk, dk, B, T, H, kC, d) ||
-      !tma::make_sw_map(&prm.map_dv, dv, B, T, H, kC, d))
+  if (!tma::make_sw_map(&prm.map_dq, dq, B, T, H, kC, d, ld_grad) || !tma::make_sw_map(&prm.map_dk, dk, B, T, H, kC, d, ld_grad) ||
+      !tma::make_sw_map(&prm.map_dv, dv, B, T, H, kC, d, ld_grad))
     return MXK_ERR_UNSUPPORTED;
   auto kernel = d == kD ? linattn_bwd_kernel<true> : linattn_bwd_kernel<false>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(BwdSmem)));
   if (e != cudaSuccess) return static_cast<int>(e);
-  kernel<<<B * H, kBwdThreads, sizeof(BwdSmem), static_cast<cudaStream_t>(stream)>>>(prm);
+  kernel<<<B * H, kBwdThreads, sizeof(BwdSmem), stream>>>(prm);
   return launch_status();
+}
+
+}  // namespace linattn
+}  // namespace mxk
+
+extern "C" {
+
+int mxk_linattn_bf16_bwd(const void* q, const void* k, const void* v, const void* d_o, const void* chunk_states,
+                         const uint8_t* done, const float* ds_last, const float* dz_last, void* dq, void* dk,
+                         void* dv, float* ds0, float* dz0, int* status, int B, int T, int H, int d, float eps,
+                         int feature_map, mxk_stream_t stream) {
+  return mxk::linattn::backward(q, k, v, 0, d_o, chunk_states, done, ds_last, dz_last, dq, dk, dv, 0, ds0, dz0, status, B, T, H, d,
+                                eps, feature_map, static_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

@@ -31,6 +31,19 @@ from torch.nn import functional as F
 from . import _C, ops
 
 
+def _weights_of(module, names):
+    """Parameters by ``submodule.kind`` out of the module dictionaries (an attribute lookup through ``nn.Module`` per
+    parameter costs more than a launch), or None where a submodule is not the plain kind the native layers know."""
+    out = []
+    for name in names:
+        sub, kind = name.split(".")
+        sub = module._modules[sub]
+        if type(sub) not in (nn.Linear, nn.RMSNorm):
+            return None
+        out.append(sub._parameters[kind])
+    return None if any(t is None for t in out) else out
+
+
 def get_input_shape(inputs):
     """(B, T, F) -> (B, F)   (utils/axes.py:46-49)."""
     return inputs.shape[:1] + inputs.shape[2:]
@@ -406,6 +419,10 @@ class MinGRUCell(MemoroidCellBase):
 
 
 # --------------------------------------------------------- linear attention
+_LINATTN_PARAMS = ("query.weight", "key.weight", "value.weight", "norm.weight", "output_projection.weight",
+                   "output_projection.bias")
+
+
 class LinearAttentionCell(MemoroidCellBase):
     """ELU+1 linear attention (linear_attention.py:14-124).  ``head_dim``: a multiple of 8, at most 64."""
 
@@ -419,6 +436,16 @@ class LinearAttentionCell(MemoroidCellBase):
         self.query = nn.Linear(in_features, hidden, bias=False)
         self.norm = nn.RMSNorm(hidden, eps=1e-6)   # flax.linen.RMSNorm's default epsilon
         self.output_projection = nn.Linear(hidden, features)
+
+    def layer(self, inputs, done, initial_carry, **kwargs):
+        """The whole layer as one native call (bf16); other dtypes, and subclasses, are composed from their parts."""
+        weights = _weights_of(self, _LINATTN_PARAMS) if type(self) is LinearAttentionCell and not kwargs else None
+        if weights is not None:
+            s0, z0 = (None, None) if initial_carry is None else initial_carry
+            out = _C.linattn_layer(inputs, weights, s0, z0, done, self.num_heads, self.eps, self._modules["norm"].eps)
+            if out is not None:
+                return (out[0], out[1]), out[2]
+        return super().layer(inputs, done, initial_carry, **kwargs)
 
     def _heads(self, t):
         return t.view(*t.shape[:2], self.num_heads, self.head_dim)
@@ -447,11 +474,15 @@ class LinearAttentionCell(MemoroidCellBase):
         bf = torch.bfloat16
         o, s_last, z_last = ops.LinAttn.apply(q.to(bf), k.to(bf), v.to(bf), s0, z0, done, self.eps, True)
         o = o.reshape(*o.shape[:2], -1).to(inputs.dtype)
-        y = ops.dense(self.norm(o), self.output_projection.weight, self.output_projection.bias)
+        y = ops.dense(ops.rms_norm(o, self.norm.weight, self.norm.eps), self.output_projection.weight, self.output_projection.bias)
         return (s_last[:, None], z_last[:, None]), y
 
 
 # ------------------------------------------------------- gated delta rule
+_DELTANET_PARAMS = ("query.weight", "key.weight", "value.weight", "gate.weight", "gate.bias", "norm.weight",
+                    "output_projection.weight", "output_projection.bias")
+
+
 class DeltaNetCell(MemoroidCellBase):
     """Gated delta-rule mixer.  The reference has no such cell; this one follows
     its cell protocol.  As a monoid the element is
@@ -475,6 +506,16 @@ class DeltaNetCell(MemoroidCellBase):
 
     def _heads(self, t):
         return t.view(*t.shape[:2], self.num_heads, self.head_dim)
+
+    def layer(self, inputs, done, initial_carry, **kwargs):
+        """The whole layer as one native call (bf16); see ``LinearAttentionCell.layer``."""
+        weights = _weights_of(self, _DELTANET_PARAMS) if type(self) is DeltaNetCell and not kwargs else None
+        if weights is not None:
+            out = _C.deltanet_layer(inputs, weights, None if initial_carry is None else initial_carry[0], done, self.num_heads,
+                                    self._modules["norm"].eps)
+            if out is not None:
+                return (out[0],), out[1]
+        return super().layer(inputs, done, initial_carry, **kwargs)
 
     def forward(self, x, **kwargs):
         """-> factored elements (k, v, alpha, beta); k is L2-normalised per head."""

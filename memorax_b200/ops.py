@@ -574,8 +574,13 @@ class MLSTMTensorCore(torch.autograd.Function):
 
 
 # ------------------------------------------------------ fused row-wise glue
+def _aligned(*tensors):
+    """Parameters cut out of a flat buffer may start anywhere; the kernels read them in 16-byte vectors."""
+    return all(t.data_ptr() % 16 == 0 for t in tensors)
+
+
 def _glue_ok(x, dim):
-    return x.is_cuda and x.dtype == torch.bfloat16 and dim % 256 == 0 and dim <= 1024
+    return x.is_cuda and x.dtype == torch.bfloat16 and dim % 8 == 0 and 0 < dim <= 1024 and x.numel() > 0
 
 
 class FusedNorm(torch.autograd.Function):
@@ -613,14 +618,14 @@ class FusedNorm(torch.autograd.Function):
 
 
 def layer_norm(x, weight, bias, eps=1e-5):
-    """nn.LayerNorm over the last dimension; the fused kernels for bf16 CUDA rows of 256..1024 elements."""
-    if _glue_ok(x, x.shape[-1]) and weight.dtype == torch.bfloat16 and bias is not None:
+    """nn.LayerNorm over the last dimension; the fused kernels for bf16 CUDA rows of up to 1024 elements."""
+    if _glue_ok(x, x.shape[-1]) and weight.dtype == torch.bfloat16 and bias is not None and _aligned(x, weight, bias):
         return FusedNorm.apply(x, weight, bias, eps, False)
     return torch.nn.functional.layer_norm(x, x.shape[-1:], weight, bias, eps)
 
 
 def rms_norm(x, weight, eps=1e-6):
-    if _glue_ok(x, x.shape[-1]) and weight.dtype == torch.bfloat16:
+    if _glue_ok(x, x.shape[-1]) and weight.dtype == torch.bfloat16 and _aligned(x, weight):
         return FusedNorm.apply(x, weight, None, eps, True)
     return torch.nn.functional.rms_norm(x, x.shape[-1:], weight, eps)
 
