@@ -25,4 +25,16 @@ int backward(const void* q, const void* k, const void* v, const float* alpha, co
              void* dv, long long ld_dv, float* dalpha, float* dbeta, float* ds0, int* status, int B, int T, int H, int d,
              cudaStream_t stream);
 }  // namespace gdelta
+namespace mlstm_tc {
+// ld_qv, hp_qv / ld_grad, hp_grad: pitch of the steps and of the heads of q and v (of dq and dv); k and dk are dense
+int forward(const void* q, const void* k, const void* v, long long ld_qv, long long hp_qv, const float* log_i, const float* log_f, const float* c0,
+            const float* n0, const float* m0, const float* f0, const uint8_t* done, void* h, float* c_last, float* n_last,
+            float* m_last, float* f_last, float* m_steps, void* chunk_states, int* status, int B, int T, int H, int d, float eps,
+            cudaStream_t stream);
+int backward(const void* q, const void* k, const void* v, long long ld_qv, long long hp_qv, const float* log_i, const float* log_f, const float* c0,
+             const float* n0, const float* m0, const uint8_t* done, const void* dh, const float* c_last, const float* n_last,
+             const float* m_steps, const void* chunk_states, const float* dc_last, const float* dn_last, const float* dm_last,
+             void* dq, void* dk, void* dv, long long ld_grad, long long hp_grad, float* dlog_i, float* dlog_f, float* dc0, float* dn0, float* dm0,
+             int* status, int B, int T, int H, int d, float eps, cudaStream_t stream);
+}  // namespace mlstm_tc
 }  // namespace mxk

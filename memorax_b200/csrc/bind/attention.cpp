@@ -1,7 +1,7 @@
 // The linear-attention and gated-delta-rule layers in bf16: the Dense layers on the inputs as one product, the chunked
 // kernels on slices of its result, RMSNorm and output projection; the backward pass as one autograd node.  One step of a
 // few sequences (acting) takes three launches.
-#include "common.h"
+#include "product.h"
 
 #include "../attention.cuh"
 #include "../layers.cuh"
@@ -39,15 +39,11 @@ Tensor project(const Tensor& x, const variable_list& w, size_t count, const Shap
   }
   const Tensor joint = empty_like_of(x, {s.ld, s.F}, at::kBFloat16);
   check("stack_rows", l::stack_rows(rows_of(w, count), joint.data_ptr(), s.ld, s.F, stream()));
-  // the library's tiles fit q | k | v; the few columns behind them would cost it a tile column (65536 x 3088 x 512:
-  // 198 us against 160 for 3072 and 17 for 16)
+  // tiles fit q | k | v; the few columns behind them would cost a tile column (65536 x 3088 x 512 in the library: 198 us
+  // against 160 for 3072 and 17 for 16)
   const Tensor rows = x.view({s.M, s.F});
-  Tensor into = proj.narrow(1, 0, 3 * s.hid);
-  at::mm_out(into, rows, joint.narrow(0, 0, 3 * s.hid).t());
-  if (s.ld > 3 * s.hid) {
-    Tensor rest = proj.narrow(1, 3 * s.hid, s.ld - 3 * s.hid);
-    at::mm_out(rest, rows, joint.narrow(0, 3 * s.hid, s.ld - 3 * s.hid).t());
-  }
+  product_into(rows, joint.narrow(0, 0, 3 * s.hid).t(), proj.narrow(1, 0, 3 * s.hid));
+  if (s.ld > 3 * s.hid) product_into(rows, joint.narrow(0, 3 * s.hid, s.ld - 3 * s.hid).t(), proj.narrow(1, 3 * s.hid, s.ld - 3 * s.hid));
   if (stacked) *stacked = joint;
   return proj;
 }
@@ -58,7 +54,7 @@ Tensor output(const Tensor& n, const Tensor& w, const Tensor& bias, const Shape&
     check("small_product", l::small_product(n.data_ptr(), rows_of({w}, 1), bias.data_ptr(), y.data_ptr(), s.out, s.M, s.hid, stream()));
     return y;
   }
-  return at::addmm(bias, n, w.t());
+  return product(n, w.t(), bias);
 }
 
 // What follows the mixer: RMSNorm and output projection, and their gradients
@@ -76,8 +72,8 @@ struct TailGrads {
 };
 TailGrads tail_backward(const Tensor& gy, const Tensor& o, const Tensor& n, const Tensor& rstd, const Tensor& norm_w, const Tensor& out_w, const Shape& s) {
   TailGrads g;
-  const Tensor gn = at::mm(gy, out_w);
-  g.out_w = at::mm(gy.t(), n);
+  const Tensor gn = product(gy, out_w);
+  g.out_w = product(gy.t(), n);
   g.out_b = empty_like_of(gy, {s.out}, at::kBFloat16);
   const size_t sum_bytes = mxk_colsum_workspace_bytes(s.M, s.out), norm_bytes = mxk_norm_bwd_workspace_bytes(s.M, s.hid);
   const Tensor ws = scratch(gy, std::max(sum_bytes, norm_bytes));
@@ -189,8 +185,8 @@ variable_list LinAttnLayer::backward(AutogradContext* ctx, const variable_list& 
                                                        ptr(gs), ptr(gz), cols_out(gproj, 0), cols_out(gproj, hid), cols_out(gproj, 2 * hid), s.ld, ptr(gs0), ptr(gz0),
                                                        status_ptr(x), s.B, s.T, s.H, s.d, ctx->saved_data["eps"].toDouble(), 1, stream()));
   variable_list grads(13);
-  if (ctx->needs_input_grad(0)) grads[0] = at::mm(gproj, joint).view(x.sizes());
-  const Tensor gw = at::mm(gproj.t(), x.view({s.M, s.F}));
+  if (ctx->needs_input_grad(0)) grads[0] = product(gproj, joint).view(x.sizes());
+  const Tensor gw = product(gproj.t(), x.view({s.M, s.F}));
   for (int i = 0; i < 3; ++i) grads[1 + i] = gw.narrow(0, i * hid, hid);
   grads[4] = t.norm_w;
   grads[5] = t.out_w;
@@ -292,10 +288,10 @@ struct DeltaLayer : torch::autograd::Function<DeltaLayer> {
                                                   s.d, stream()));
     const l::ColumnSum sum{ptr(part), rows, 2 * s.H, ptr(part) + static_cast<size_t>(rows) * 2 * s.H};
     check("column_sums", l::column_sums(&sum, 1, stream()));
-    if (ctx->needs_input_grad(0)) grads[0] = at::mm(gproj, joint).view(x.sizes());
-    const Tensor rows_in = x.view({s.M, s.F}), gw = at::mm(gproj.narrow(1, 0, 3 * hid).t(), rows_in);
+    if (ctx->needs_input_grad(0)) grads[0] = product(gproj, joint).view(x.sizes());
+    const Tensor rows_in = x.view({s.M, s.F}), gw = product(gproj.narrow(1, 0, 3 * hid).t(), rows_in);
     for (int i = 0; i < 3; ++i) grads[1 + i] = gw.narrow(0, i * hid, hid);
-    grads[4] = at::mm(gproj.narrow(1, 3 * hid, 2 * s.H).t(), rows_in);
+    grads[4] = product(gproj.narrow(1, 3 * hid, 2 * s.H).t(), rows_in);
     grads[5] = part[rows].to(at::kBFloat16);
     grads[6] = t.norm_w;
     grads[7] = t.out_w;

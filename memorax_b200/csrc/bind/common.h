@@ -68,5 +68,6 @@ void bind_linear(pybind11::module_& m);
 void bind_lru(pybind11::module_& m);
 void bind_mamba(pybind11::module_& m);
 void bind_mingru(pybind11::module_& m);
+void bind_mlstm(pybind11::module_& m);
 
 }  // namespace mxk_host

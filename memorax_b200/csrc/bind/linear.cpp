@@ -1,5 +1,5 @@
 // Dense layers in float32 on the tensor cores (gemm32.cuh), with their gradients.
-#include "common.h"
+#include "product.h"
 
 #include "../gemm32.cuh"
 
@@ -11,7 +11,7 @@ using torch::autograd::AutogradContext;
 using torch::autograd::variable_list;
 
 // c (M, N) = a (M, K) w^T, w stored (N, K) or, transposed, (K, N)
-void product(const Tensor& a, const Tensor& w, bool transposed, const float* bias, const Tensor& c, int M, int N, int K) {
+void product32(const Tensor& a, const Tensor& w, bool transposed, const float* bias, const Tensor& c, int M, int N, int K) {
   Arena mem;
   const size_t image = mem.take(g::image_bytes(M, N, K)), ws_bytes = g::workspace_bytes(M, N, K), ws = mem.take(ws_bytes);
   mem.alloc(a);
@@ -33,7 +33,7 @@ struct Linear32 : torch::autograd::Function<Linear32> {
     auto sizes = x.sizes().vec();
     sizes.back() = N;
     const Tensor y = empty_like_of(x, sizes, at::kFloat);
-    product(x, w, false, bias ? ptr(*bias) : nullptr, y, M, N, K);
+    product32(x, w, false, bias ? ptr(*bias) : nullptr, y, M, N, K);
     ctx->saved_data["bias"] = bias.has_value();
     ctx->save_for_backward({x, w});
     return y;
@@ -46,7 +46,7 @@ struct Linear32 : torch::autograd::Function<Linear32> {
     variable_list grads(3);
     if (ctx->needs_input_grad(0)) {
       grads[0] = empty_like_of(x, x.sizes(), at::kFloat);
-      product(gy, w, true, nullptr, grads[0], M, K, N);
+      product32(gy, w, true, nullptr, grads[0], M, K, N);
     }
     if (ctx->needs_input_grad(1)) {
       grads[1] = empty_like_of(w, w.sizes(), at::kFloat);
@@ -68,8 +68,18 @@ Tensor linear_f32(const Tensor& x, const Tensor& w, const OptTensor& bias) {
   return Linear32::apply(x.contiguous(), w.contiguous(), bias ? OptTensor(bias->contiguous()) : std::nullopt);
 }
 
+// a (.., M, K) b (.., K, N) (+ bias) (+ c) in bf16 through this repository's kernel
+Tensor product_bf16(const Tensor& a, const Tensor& b, const OptTensor& bias, const OptTensor& c) {
+  const c10::cuda::CUDAGuard guard(a.device());
+  if (!c) return product(a, b, bias.value_or(Tensor()));
+  product_into(a, b, *c, bias.value_or(Tensor()), true);
+  return *c;
+}
+
 }  // namespace
 
-void bind_linear(pybind11::module_& m) { m.def("linear_f32", &linear_f32, pybind11::arg("x"), pybind11::arg("w"), pybind11::arg("bias") = pybind11::none()); }
+void bind_linear(pybind11::module_& m) {
+  m.def("product_bf16", &product_bf16, pybind11::arg("a"), pybind11::arg("b"), pybind11::arg("bias") = pybind11::none(), pybind11::arg("c") = pybind11::none());
+  m.def("linear_f32", &linear_f32, pybind11::arg("x"), pybind11::arg("w"), pybind11::arg("bias") = pybind11::none()); }
 
 }  // namespace mxk_host

@@ -1,0 +1,225 @@
+// The mLSTM layer on the tensor cores (bf16): its products on slices of joint buffers, everything else fused; the backward pass as one autograd node.
+#include "product.h"
+
+#include <cmath>
+
+#include "../attention.cuh"
+#include "../layers.cuh"
+
+namespace mxk_host {
+namespace {
+
+namespace l = mxk::layers;
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+
+enum { kUp, kConvW, kConvB, kQ, kK, kV, kIW, kIB, kFW, kFB, kSkip, kNorm, kOut, kParams };
+
+struct Shape {
+  int B, T, F, H, d, hid, M;
+  float scale() const { return 1.f / std::sqrt(static_cast<float>(d)); }
+};
+Shape shape_of(const Tensor& x, const variable_list& p) {
+  Shape s;
+  s.B = x.size(0); s.T = x.size(1); s.F = x.size(2);
+  s.H = p[kQ].size(0); s.d = p[kQ].size(1);
+  s.hid = s.H * s.d;
+  s.M = s.B * s.T;
+  return s;
+}
+// columns [at, at + hid) of a (M, n) buffer as per-head matrices (H, M, d)
+Tensor heads(const Tensor& t, int at, const Shape& s) { return t.narrow(1, at, s.hid).view({s.M, s.H, s.d}).permute({1, 0, 2}); }
+// parts [first, first + count) of q | k | v of every head, out of a buffer (M, H, 3, d): (H, M, count d).  With the head
+// outermost this is the order the gates' weights are in, and q and k are one product.
+Tensor parts(const Tensor& t, int first, int count, const Shape& s) {
+  return t.view({s.M, s.H, 3 * s.d}).narrow(2, first * s.d, count * s.d).permute({1, 0, 2});
+}
+void* column(const Tensor& t, int c) { return static_cast<uint8_t*>(t.data_ptr()) + 2 * c; }
+
+struct Result {
+  Tensor y, c_last, n_last, m_last, f_last;
+  Tensor up, u, qk_w, qkv, ks, gate_w, logits, log_i, log_f, h, g, m_steps, states;
+};
+
+Result forward(const Tensor& x, const variable_list& p, const Tensor& c0, const Tensor& n0, const Tensor& m0, const Tensor& f0, const Tensor& done,
+               const Shape& s, double eps, bool keep) {
+  Result r;
+  const auto bf = at::kBFloat16;
+  const auto st = stream();
+  r.c_last = empty_like_of(x, {s.B, s.H, s.d, s.d}, at::kFloat);
+  r.n_last = empty_like_of(x, {s.B, s.H, s.d}, at::kFloat);
+  r.m_last = empty_like_of(x, {s.B, s.H}, at::kFloat);
+  r.f_last = empty_like_of(x, {s.B, s.H}, at::kFloat);
+  r.up = product(x.view({s.M, s.F}), p[kUp].t());
+  r.u = empty_like_of(x, {s.M, s.hid}, bf);
+  check("mlstm_conv_fwd", l::mlstm_conv_fwd(r.up.data_ptr(), 2 * s.hid, p[kConvW].data_ptr(), p[kConvB].data_ptr(), r.u.data_ptr(), s.B, s.T, s.hid, st));
+  r.qkv = empty_like_of(x, {s.M, 3 * s.hid}, bf);
+  r.qk_w = at::cat({p[kQ], p[kK]}, 1);   // (H, 2d, d)
+  product_into(heads(r.u, 0, s), r.qk_w.transpose(1, 2), parts(r.qkv, 0, 2, s));
+  product_into(heads(r.up, 0, s), p[kV].transpose(1, 2), parts(r.qkv, 2, 1, s));
+  r.gate_w = empty_like_of(x, {2 * s.H, 3 * s.hid}, bf);
+  l::WeightRows rows{};
+  rows.count = 2;
+  rows.ptr[0] = p[kIW].data_ptr(); rows.ptr[1] = p[kFW].data_ptr();
+  rows.rows[0] = rows.rows[1] = s.H;
+  check("stack_rows", l::stack_rows(rows, r.gate_w.data_ptr(), 2 * s.H, 3 * s.hid, st));
+  r.logits = product(r.qkv, r.gate_w.t(), at::cat({p[kIB], p[kFB]}));
+  r.log_i = empty_like_of(x, {s.M, s.H}, at::kFloat);
+  r.log_f = empty_like_of(x, {s.M, s.H}, at::kFloat);
+  r.ks = empty_like_of(x, {s.M, s.hid}, bf);
+  check("mlstm_gates_fwd", l::mlstm_gates_fwd(r.logits.data_ptr(), column(r.qkv, s.d), 3 * s.hid, 3 * s.d, s.scale(), ptr(r.log_i),
+                                              ptr(r.log_f), r.ks.data_ptr(), s.M, s.H, s.d, st));
+  r.h = empty_like_of(x, {s.M, s.hid}, bf);
+  if (keep) {
+    r.m_steps = empty_like_of(x, {s.M, s.H}, at::kFloat);
+    r.states = scratch(x, mxk_mlstm_bf16_chunk_states_bytes(s.B, s.T, s.H, s.d));
+  }
+  check("mxk_mlstm_bf16_fwd", mxk::mlstm_tc::forward(r.qkv.data_ptr(), r.ks.data_ptr(), column(r.qkv, 2 * s.d), 3 * s.hid, 3 * s.d, ptr(r.log_i), ptr(r.log_f), ptr(c0), ptr(n0),
+                                                     ptr(m0), ptr(f0), bytes(done), r.h.data_ptr(), ptr(r.c_last), ptr(r.n_last), ptr(r.m_last), ptr(r.f_last),
+                                                     ptr(r.m_steps), ptr<void>(r.states), status_ptr(x), s.B, s.T, s.H, s.d, eps, st));
+  r.g = empty_like_of(x, {s.M, s.hid}, bf);
+  check("mlstm_out_fwd", l::mlstm_out_fwd(r.h.data_ptr(), r.u.data_ptr(), column(r.up, s.hid), 2 * s.hid, p[kNorm].data_ptr(), p[kSkip].data_ptr(), r.g.data_ptr(), s.M,
+                                          s.H, s.d, st));
+  r.y = product(r.g, p[kOut].t()).view({s.B, s.T, p[kOut].size(0)});
+  return r;
+}
+
+struct MlstmLayer : torch::autograd::Function<MlstmLayer> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, at::TensorList params, const OptTensor& c0_in, const OptTensor& n0_in, const OptTensor& m0_in,
+                               const OptTensor& f0_in, const OptTensor& done_in, double eps) {
+    const variable_list p(params.begin(), params.end());
+    const Tensor c0 = c0_in.value_or(Tensor()), n0 = n0_in.value_or(Tensor()), m0 = m0_in.value_or(Tensor()), done = done_in.value_or(Tensor());
+    const Shape s = shape_of(x, p);
+    Result r = mxk_host::forward(x, p, c0, n0, m0, f0_in.value_or(Tensor()), done, s, eps, true);
+    ctx->set_materialize_grads(false);
+    ctx->saved_data["eps"] = eps;
+    variable_list saved{x};
+    saved.insert(saved.end(), p.begin(), p.end());
+    for (const Tensor& t : {c0, n0, m0, done, r.up, r.u, r.qkv, r.ks, r.gate_w, r.logits, r.log_i, r.log_f, r.h, r.g, r.m_steps, r.states, r.c_last, r.n_last, r.qk_w})
+      saved.push_back(t);
+    ctx->save_for_backward(std::move(saved));
+    ctx->mark_non_differentiable({r.f_last});
+    return {r.c_last, r.n_last, r.m_last, r.f_last, r.y};
+  }
+
+  static variable_list backward(AutogradContext* ctx, const variable_list& gout) {
+    const variable_list v = ctx->get_saved_variables();
+    const Tensor& x = v[0];
+    const variable_list p(v.begin() + 1, v.begin() + 1 + kParams);
+    const Tensor *t = &v[1 + kParams];
+    const Tensor &c0 = t[0], &n0 = t[1], &m0 = t[2], &done = t[3], &up = t[4], &u = t[5], &qkv = t[6], &ks = t[7], &gate_w = t[8], &logits = t[9], &log_i = t[10],
+                 &log_f = t[11], &h = t[12], &g = t[13], &m_steps = t[14], &states = t[15], &c_last = t[16], &n_last = t[17], &qk_w = t[18];
+    const c10::cuda::CUDAGuard guard(x.device());
+    const Shape s = shape_of(x, p);
+    const auto bf = at::kBFloat16;
+    const auto st = stream();
+    const int64_t out = p[kOut].size(0);
+    const auto given = [&](int i) { return gout[i].defined() ? gout[i].contiguous() : Tensor(); };
+    const Tensor gc = given(0), gn = given(1), gm = given(2);
+    const Tensor gy = (gout[4].defined() ? gout[4].contiguous() : empty_like_of(x, {s.M, out}, bf).zero_()).view({s.M, out});
+    // inputs of the node: x, the parameters, then what there is of the carry
+    variable_list grads(1 + kParams + 6);
+    const int first = 1 + kParams;
+    const bool need_state = c0.defined() || n0.defined() || m0.defined();
+    Tensor gc0, gn0, gm0;
+    if (need_state) {
+      gc0 = empty_like_of(x, {s.B, s.H, s.d, s.d}, at::kFloat);
+      gn0 = empty_like_of(x, {s.B, s.H, s.d}, at::kFloat);
+      gm0 = empty_like_of(x, {s.B, s.H}, at::kFloat);
+    }
+    const Tensor gg = product(gy, p[kOut]);
+    grads[1 + kOut] = product(gy.t(), g);
+    const Tensor gh = empty_like_of(x, {s.M, s.hid}, bf), gu = empty_like_of(x, {s.M, s.hid}, bf), gks = empty_like_of(x, {s.M, s.hid}, bf), gx = empty_like_of(x, {s.M, s.hid}, bf);
+    const Tensor gup = empty_like_of(x, {s.M, 2 * s.hid}, bf), gqkv = empty_like_of(x, {s.M, 3 * s.hid}, bf), glogits = empty_like_of(x, {s.M, 2 * s.H}, bf);
+    const Tensor gli = empty_like_of(x, {s.M, s.H}, at::kFloat), glf = empty_like_of(x, {s.M, s.H}, at::kFloat);
+    const int out_rows = l::mlstm_out_blocks(s.M, s.hid), gate_rows = l::mlstm_gate_blocks(s.M), conv_rows = l::mlstm_conv_blocks(s.B, s.T, s.hid);
+    const int cols[3] = {2 * s.hid, 2 * s.H, 5 * s.hid};
+    const Tensor part = empty_like_of(x, {static_cast<int64_t>(out_rows) * cols[0] + gate_rows * cols[1] + static_cast<int64_t>(conv_rows) * cols[2]}, at::kFloat);
+    float* const part_out = ptr(part);
+    float* const part_gate = part_out + static_cast<size_t>(out_rows) * cols[0];
+    float* const part_conv = part_gate + static_cast<size_t>(gate_rows) * cols[1];
+    check("mlstm_out_bwd", l::mlstm_out_bwd(gg.data_ptr(), h.data_ptr(), u.data_ptr(), column(up, s.hid), 2 * s.hid, p[kNorm].data_ptr(), p[kSkip].data_ptr(), gh.data_ptr(),
+                                            column(gup, s.hid), 2 * s.hid, gu.data_ptr(), part_out, s.M, s.H, s.d, st));
+    check("mxk_mlstm_bf16_bwd", mxk::mlstm_tc::backward(qkv.data_ptr(), ks.data_ptr(), column(qkv, 2 * s.d), 3 * s.hid, 3 * s.d, ptr(log_i), ptr(log_f), ptr(c0), ptr(n0), ptr(m0),
+                                                        bytes(done), gh.data_ptr(), ptr(c_last), ptr(n_last), ptr(m_steps), states.data_ptr(), ptr(gc), ptr(gn), ptr(gm),
+                                                        gqkv.data_ptr(), gks.data_ptr(), column(gqkv, 2 * s.d), 3 * s.hid, 3 * s.d, ptr(gli), ptr(glf), ptr(gc0), ptr(gn0), ptr(gm0),
+                                                        status_ptr(x), s.B, s.T, s.H, s.d, ctx->saved_data["eps"].toDouble(), st));
+    check("mlstm_gates_bwd", l::mlstm_gates_bwd(logits.data_ptr(), ptr(gli), ptr(glf), gks.data_ptr(), s.scale(), column(gqkv, s.d), 3 * s.hid, 3 * s.d,
+                                                glogits.data_ptr(), part_gate, s.M, s.H, s.d, st));
+    product_into(glogits, gate_w, gqkv, Tensor(), true);
+    const Tensor ggate = product(glogits.t(), qkv);
+    grads[1 + kIW] = ggate.narrow(0, 0, s.H);
+    grads[1 + kFW] = ggate.narrow(0, s.H, s.H);
+    const Tensor gqk = parts(gqkv, 0, 2, s), gvalue = parts(gqkv, 2, 1, s);
+    const Tensor gqk_w = product(gqk.transpose(1, 2), heads(u, 0, s));
+    grads[1 + kQ] = gqk_w.narrow(1, 0, s.d);
+    grads[1 + kK] = gqk_w.narrow(1, s.d, s.d);
+    grads[1 + kV] = product(gvalue.transpose(1, 2), heads(up, 0, s));
+    product_into(gqk, qk_w, heads(gu, 0, s), Tensor(), true);
+    product_into(gvalue, p[kV], heads(gx, 0, s));
+    check("mlstm_conv_bwd", l::mlstm_conv_bwd(up.data_ptr(), 2 * s.hid, p[kConvW].data_ptr(), p[kConvB].data_ptr(), gu.data_ptr(), gx.data_ptr(), gup.data_ptr(), part_conv, s.B,
+                                              s.T, s.hid, st));
+    const Tensor sums = empty_like_of(x, {cols[0] + cols[1] + cols[2]}, at::kFloat);
+    const l::ColumnSum jobs[3] = {{part_out, out_rows, cols[0], ptr(sums)}, {part_gate, gate_rows, cols[1], ptr(sums) + cols[0]}, {part_conv, conv_rows, cols[2], ptr(sums) + cols[0] + cols[1]}};
+    check("column_sums", l::column_sums(jobs, 3, st));
+    const Tensor small = sums.to(bf);
+    int64_t at = 0;
+    const auto piece = [&](int i, int64_t n) {
+      grads[1 + i] = small.narrow(0, at, n).view(p[i].sizes());
+      at += n;
+    };
+    piece(kNorm, s.hid);
+    piece(kSkip, s.hid);
+    piece(kIB, s.H);
+    piece(kFB, s.H);
+    piece(kConvW, 4 * s.hid);
+    piece(kConvB, s.hid);
+    grads[1 + kUp] = product(gup.t(), x.view({s.M, s.F}));
+    if (ctx->needs_input_grad(0)) grads[0] = product(gup, p[kUp]).view(x.sizes());
+    if (c0.defined()) grads[first] = gc0;
+    if (n0.defined()) grads[first + 1] = gn0;
+    if (m0.defined()) grads[first + 2] = gm0;
+    return grads;
+  }
+};
+
+// -> (c (B,1,H,d,d), f (B,1,H,1,1), n (B,1,H,d,1), m (B,1,H,1,1), y (B,T,F)), or None where the caller has to compose the layer
+pybind11::object mlstm_layer(const Tensor& x_in, const variable_list& p, const OptTensor& c_in, const OptTensor& f_in, const OptTensor& n_in, const OptTensor& m_in,
+                             const OptTensor& done_in, double eps) {
+  if (!x_in.is_cuda() || x_in.scalar_type() != at::kBFloat16 || x_in.dim() != 3 || x_in.numel() == 0 || p.size() != kParams ||
+      x_in.size(0) * x_in.size(1) > 0x7fffffff || at::autocast::is_autocast_enabled(at::kCUDA))
+    return pybind11::none();
+  for (const Tensor& t : p)
+    if (t.scalar_type() != at::kBFloat16 || t.device() != x_in.device() || !t.is_contiguous() || (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15)) return pybind11::none();
+  const int64_t H = p[kQ].size(0), d = p[kQ].size(1), hid = H * d, F = x_in.size(2);
+  if ((d != 16 && d != 32 && d != 64) || H > 64 || hid > 2048 || 256 % (hid / 8 > 0 ? hid / 8 : 1) || p[kUp].sizes() != at::IntArrayRef({2 * hid, F}) ||
+      p[kConvW].sizes() != at::IntArrayRef({hid, 1, 4}) || p[kOut].size(1) != hid || x_in.size(0) * H > 0x7fffffff)
+    return pybind11::none();
+  const c10::cuda::CUDAGuard guard(x_in.device());
+  const auto leaf = [&](const OptTensor& t, at::IntArrayRef sizes, const char* name) {
+    return t && t->defined() ? dev(t->reshape(sizes), at::kFloat, name) : Tensor();
+  };
+  const int64_t B = x_in.size(0);
+  const Tensor x = x_in.contiguous(), done = done_bytes(done_in);
+  const Tensor c0 = leaf(c_in, {B, H, d, d}, "c0"), f0 = leaf(f_in, {B, H}, "f0"), n0 = leaf(n_in, {B, H, d}, "n0"), m0 = leaf(m_in, {B, H}, "m0");
+  bool grad = x.requires_grad();
+  for (const Tensor& t : p) grad |= t.requires_grad();
+  for (const Tensor& t : {c0, n0, m0}) grad |= t.defined() && t.requires_grad();
+  Tensor c, f, n, m, y;
+  if (at::GradMode::is_enabled() && grad) {
+    const bool all = c0.defined() && n0.defined() && m0.defined(), none = !c0.defined() && !n0.defined() && !m0.defined();
+    if (!all && !none) return pybind11::none();
+    const variable_list out = MlstmLayer::apply(x, at::TensorList(p), opt(c0), opt(n0), opt(m0), opt(f0), opt(done), eps);
+    c = out[0]; n = out[1]; m = out[2]; f = out[3]; y = out[4];
+  } else {
+    const Result r = forward(x, p, c0, n0, m0, f0, done, shape_of(x, p), eps, false);
+    c = r.c_last; n = r.n_last; m = r.m_last; f = r.f_last; y = r.y;
+  }
+  return pybind11::cast(std::make_tuple(c.unsqueeze(1), f.view({B, 1, H, 1, 1}), n.view({B, 1, H, d, 1}), m.view({B, 1, H, 1, 1}), y));
+}
+
+}  // namespace
+
+void bind_mlstm(pybind11::module_& m) { m.def("mlstm_layer", &mlstm_layer); }
+
+}  // namespace mxk_host

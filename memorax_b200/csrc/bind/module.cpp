@@ -37,4 +37,5 @@ PYBIND11_MODULE(_C, m) {
   bind_lru(m);
   bind_mamba(m);
   bind_mingru(m);
+  bind_mlstm(m);
 }

@@ -1,0 +1,58 @@
+// bf16 products of the native layers: this repository's kernel (gemm16.cuh) where a library call's host time counts, the
+// library where the product is large.
+#pragma once
+
+#include "common.h"
+
+#include "../gemm16.cuh"
+
+namespace mxk_host {
+
+// 2 M N K above which the library's two-SM tiles are the faster form.
+constexpr double kLibraryFlops = 2e10;
+
+// c = a b (+ bias) (+ c when `accumulate`) over the last two dimensions; a (M, K), b (K, N), c (M, N), or the same with a
+// leading batch dimension: any views whose rows or columns are contiguous.
+inline void product_into(const Tensor& a, const Tensor& b, const Tensor& c, const Tensor& bias = Tensor(), bool accumulate = false) {
+  namespace g = mxk::gemm16;
+  const int n = static_cast<int>(c.dim()), r = n - 2, q = n - 1;
+  const int64_t batch = n == 3 ? c.size(0) : 1, M = c.size(r), N = c.size(q), K = a.size(q);
+  const auto rows_of = [&](const Tensor& t, bool& by_rows, bool k_is_col) {
+    // stored row-major along whichever index is contiguous
+    const bool row_major = t.stride(q) == 1;
+    by_rows = row_major != k_is_col;
+    return g::Matrix{t.data_ptr(), row_major ? t.stride(r) : t.stride(q), n == 3 ? t.stride(0) : 0};
+  };
+  bool a_rows, b_rows;
+  const g::Matrix ma = rows_of(a, a_rows, true), mb = rows_of(b, b_rows, false);
+  const auto fits = [&](const Tensor& t, const g::Matrix& m) {
+    return (t.stride(r) == 1 || t.stride(q) == 1) && m.ld % 8 == 0 && m.batch_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(m.ptr) & 15) == 0;
+  };
+  if (2.0 * batch * M * N * K <= kLibraryFlops && fits(a, ma) && fits(b, mb) && c.stride(q) == 1) {
+    const size_t bytes = g::workspace_bytes(batch, M, N, K);
+    const Tensor ws = bytes ? scratch(c, bytes) : Tensor();
+    check("gemm16", g::run(ma, a_rows, mb, b_rows, bias.defined() ? bias.data_ptr() : nullptr, c.data_ptr(), c.stride(r), n == 3 ? c.stride(0) : 0, accumulate, batch, M, N, K,
+                           ptr<void>(ws), bytes, status_ptr(c), stream()));
+    return;
+  }
+  Tensor out = c;
+  if (n == 3) {
+    if (accumulate) at::baddbmm_out(out, c, a, b);
+    else at::bmm_out(out, a, b);
+  } else if (accumulate) {
+    at::addmm_out(out, c, a, b);
+  } else if (bias.defined()) {
+    at::addmm_out(out, bias, a, b);
+  } else {
+    at::mm_out(out, a, b);
+  }
+}
+inline Tensor product(const Tensor& a, const Tensor& b, const Tensor& bias = Tensor()) {
+  auto sizes = a.sizes().vec();
+  sizes.back() = b.size(-1);
+  const Tensor c = empty_like_of(a, sizes, at::kBFloat16);
+  product_into(a, b, c, bias);
+  return c;
+}
+
+}  // namespace mxk_host

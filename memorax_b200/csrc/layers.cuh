@@ -124,5 +124,31 @@ int delta_gate_blocks(long long tokens);
 int delta_inputs_bwd(const void* qkvg, long long ld, const void* gate_bias, const void* dq, const void* dk, const float* dalpha,
                      const float* dbeta, void* g, float* partial, long long tokens, int H, int d, cudaStream_t stream);
 
+// ---- mLSTM in bf16, mlstm_layer.cu: what is elementwise around its products and its chunk kernels ------------------
+// u (tokens, hid) = silu(conv(x)), x the first `hid` columns of up (tokens, ld); weights (hid, 4), bias (hid)
+int mlstm_conv_fwd(const void* up, long long ld, const void* conv_w, const void* conv_b, void* u, int B, int T, int hid,
+                   cudaStream_t stream);
+// logits (tokens, 2H) -> log_i, log_f = log sigmoid (tokens, H); k_scaled = k scale, k a slice with pitch ld
+// between steps and hp between heads
+int mlstm_gates_fwd(const void* logits, const void* k, long long ld, int hp, float scale,
+                    float* log_i, float* log_f, void* k_scaled, long long tokens, int H, int d, cudaStream_t stream);
+// g = (LayerNorm_head(h) (1 + norm_w) + skip u) silu(z), z a slice with pitch ld
+int mlstm_out_fwd(const void* h, const void* u, const void* z, long long ld, const void* norm_w, const void* skip, void* g,
+                  long long tokens, int H, int d, cudaStream_t stream);
+// gg -> gh, gz (slice with pitch ld_gz), gu (the skip's share); partial: mlstm_out_blocks rows of norm_w | skip (2 hid)
+int mlstm_out_blocks(long long tokens, int hid);
+int mlstm_out_bwd(const void* gg, const void* h, const void* u, const void* z, long long ld, const void* norm_w, const void* skip,
+                  void* gh, void* gz, long long ld_gz, void* gu, float* partial, long long tokens, int H, int d, cudaStream_t stream);
+// gk (slice with pitches ld, hp) = gk_scaled scale; glogits (tokens, 2H); partial: mlstm_gate_blocks rows of 2 H (bias gradients)
+int mlstm_gate_blocks(long long tokens);
+int mlstm_gates_bwd(const void* logits, const float* glog_i, const float* glog_f, const void* gk_scaled,
+                    float scale, void* gk, long long ld, int hp, void* glogits, float* partial, long long tokens, int H, int d,
+                    cudaStream_t stream);
+// gu -> the first `hid` columns of gup (through SiLU and the convolution, + gx); partial: mlstm_conv_blocks rows of
+// conv_w (hid, 4) | conv_b (hid)
+int mlstm_conv_blocks(int B, int T, int hid);
+int mlstm_conv_bwd(const void* up, long long ld, const void* conv_w, const void* conv_b, const void* gu, const void* gx, void* gup,
+                   float* partial, int B, int T, int hid, cudaStream_t stream);
+
 }  // namespace layers
 }  // namespace mxk

@@ -324,9 +324,9 @@ struct ColumnSums {
   ColumnSum job[4];
   int first_block[5];
 };
-// 32 columns per block; eight groups of rows, added in order
-__global__ void __launch_bounds__(256) column_sums_kernel(const __grid_constant__ ColumnSums p) {
-  __shared__ float part[8][33];
+// 32 columns per block; 32 groups of rows (few rows per thread: latency-bound), added in order
+__global__ void __launch_bounds__(1024) column_sums_kernel(const __grid_constant__ ColumnSums p) {
+  __shared__ float part[32][33];
   int j = 0;
   while (static_cast<int>(blockIdx.x) >= p.first_block[j + 1]) ++j;
   const ColumnSum& jb = p.job[j];
@@ -335,13 +335,13 @@ __global__ void __launch_bounds__(256) column_sums_kernel(const __grid_constant_
   float s = 0.f;
   if (col < jb.cols)
 #pragma unroll 4
-    for (int r = ty; r < jb.rows; r += 8) s += jb.src[static_cast<size_t>(r) * jb.cols + col];
+    for (int r = ty; r < jb.rows; r += 32) s += jb.src[static_cast<size_t>(r) * jb.cols + col];
   part[ty][tx] = s;
   __syncthreads();
   if (ty == 0 && col < jb.cols) {
     float t = part[0][tx];
 #pragma unroll
-    for (int i = 1; i < 8; ++i) t += part[i][tx];
+    for (int i = 1; i < 32; ++i) t += part[i][tx];
     jb.dst[col] = t;
   }
 }
@@ -356,7 +356,7 @@ int column_sums(const ColumnSum* jobs, int count, cudaStream_t stream) {
     p.first_block[j + 1] = p.first_block[j] + (jobs[j].cols + 31) / 32;
   }
   for (int j = count; j < 4; ++j) p.first_block[j + 1] = 0x7fffffff;
-  column_sums_kernel<<<p.first_block[count], 256, 0, stream>>>(p);
+  column_sums_kernel<<<p.first_block[count], 1024, 0, stream>>>(p);
   return launch_status();
 }
 

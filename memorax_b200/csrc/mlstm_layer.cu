@@ -1,0 +1,485 @@
+// The elementwise work around the mLSTM layer's products and chunk kernels (mlstm.py:129-229), bf16 in and out, float32
+// arithmetic: causal convolution + SiLU, gates and key scaling, head-wise LayerNorm + skip + output gate, and their
+// gradients.  All HBM-bound, one read and one write of each operand; a thread owns eight channels (16 bytes) and walks
+// tokens, so that the convolution's window and the parameter gradients stay in registers.  (As separate torch calls they
+// were about sixty launches of a layer step.)
+#include <cuda_bf16.h>
+
+#include "layers.cuh"
+#include "mxk_common.cuh"
+#include "umma.cuh"
+
+namespace mxk {
+namespace layers {
+namespace {
+
+using umma::pack8_bf16;
+using umma::unpack8_bf16;
+using bf16 = __nv_bfloat16;
+
+constexpr int kTaps = 4;
+
+__device__ __forceinline__ float sigmoid(float x) { return 1.f / (1.f + __expf(-x)); }
+__device__ __forceinline__ float softplus(float x) { return x > 20.f ? x : log1pf(__expf(x)); }
+// a value that the bf16 layer holds in memory
+__device__ __forceinline__ float held(float x) { return __bfloat162float(__float2bfloat16(x)); }
+__device__ __forceinline__ void load8(const bf16* p, float* x) { unpack8_bf16(*reinterpret_cast<const uint4*>(p), x); }
+__device__ __forceinline__ void store8(bf16* p, const float* x) { *reinterpret_cast<uint4*>(p) = pack8_bf16(x); }
+
+struct Taps {
+  float w[kTaps][8], b[8];
+  __device__ __forceinline__ Taps(const bf16* conv_w, const bf16* conv_b, int c) {
+    float raw[8 * kTaps];
+#pragma unroll
+    for (int i = 0; i < kTaps; ++i) load8(conv_w + c * kTaps + i * 8, raw + i * 8);
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+#pragma unroll
+      for (int k = 0; k < kTaps; ++k) w[k][e] = raw[e * kTaps + k];
+    load8(conv_b + c, b);
+  }
+};
+
+template <int kRun>   // tokens per thread
+__global__ void __launch_bounds__(256) conv_fwd_kernel(const bf16* __restrict__ up, long long ld, const bf16* __restrict__ conv_w,
+                                                       const bf16* __restrict__ conv_b, bf16* __restrict__ u, int B, int T, int hid,
+                                                       int runs) {
+  const int groups = hid / 8;
+  const long long id = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
+  const int c = static_cast<int>(id % groups) * 8;
+  const long long seq_run = id / groups;
+  const int b = static_cast<int>(seq_run / runs), t0 = static_cast<int>(seq_run % runs) * kRun;
+  if (b >= B) return;
+  const Taps taps(conv_w, conv_b, c);
+  float win[kTaps][8];
+#pragma unroll
+  for (int k = 0; k < kTaps - 1; ++k) {
+    const int t = t0 - (kTaps - 1) + k;
+    if (t >= 0) load8(up + (static_cast<long long>(b) * T + t) * ld + c, win[k]);
+    else
+#pragma unroll
+      for (int e = 0; e < 8; ++e) win[k][e] = 0.f;
+  }
+  const bf16* src = up + (static_cast<long long>(b) * T + t0) * ld + c;
+  uint4 next[4];   // four steps ahead: the loop waits for no load it has just issued
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    if (t0 + i < T) next[i] = *reinterpret_cast<const uint4*>(src + i * ld);
+#pragma unroll 4
+  for (int i = 0; i < kRun; ++i) {
+    const int t = t0 + i;
+    if (t >= T) break;
+    const long long tok = static_cast<long long>(b) * T + t;
+    unpack8_bf16(next[i % 4], win[kTaps - 1]);
+    if (i + 4 < kRun && t + 4 < T) next[i % 4] = *reinterpret_cast<const uint4*>(src + (i + 4) * ld);
+    float v[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      float a = taps.b[e];
+#pragma unroll
+      for (int k = 0; k < kTaps; ++k) a = fmaf(taps.w[k][e], win[k][e], a);
+      a = held(a);
+      v[e] = a * sigmoid(a);
+    }
+    store8(u + tok * hid + c, v);
+#pragma unroll
+    for (int k = 0; k < kTaps - 1; ++k)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) win[k][e] = win[k + 1][e];
+  }
+}
+
+// A thread walks its run and the three steps after it: the convolution's output is recomputed, its cotangent
+// g_t = gu_t silu'(.) meets the four inputs it came from.
+template <int kRun>
+__global__ void __launch_bounds__(256) conv_bwd_kernel(const bf16* __restrict__ up, long long ld, const bf16* __restrict__ conv_w,
+                                                       const bf16* __restrict__ conv_b, const bf16* __restrict__ gu,
+                                                       const bf16* __restrict__ gx, bf16* __restrict__ gup,
+                                                       float* __restrict__ partial, int B, int T, int hid, int runs, int lanes) {
+  extern __shared__ float red[];   // [channel][taps + bias] sums of the block's runs, one run group at a time
+  const int groups = hid / 8;
+  // a block: `lanes` channel groups (a divisor of both 256 and groups) x 256 / lanes runs
+  const int cg = blockIdx.y * lanes + threadIdx.x % lanes, c = cg * 8;
+  const long long seq_run = static_cast<long long>(blockIdx.x) * (256 / lanes) + threadIdx.x / lanes;
+  const int b = static_cast<int>(seq_run / runs), t0 = static_cast<int>(seq_run % runs) * kRun;
+  float gw[kTaps][8], gb[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    gb[e] = 0.f;
+#pragma unroll
+    for (int k = 0; k < kTaps; ++k) gw[k][e] = 0.f;
+  }
+  if (b < B) {
+    const Taps taps(conv_w, conv_b, c);
+    float win[kTaps][8], acc[kTaps][8];   // inputs t-3..t; cotangents of inputs t-3..t
+#pragma unroll
+    for (int k = 0; k < kTaps; ++k)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) win[k][e] = acc[k][e] = 0.f;
+#pragma unroll
+    for (int k = 0; k < kTaps - 1; ++k) {
+      const int t = t0 - (kTaps - 1) + k;
+      if (t >= 0) load8(up + (static_cast<long long>(b) * T + t) * ld + c, win[k]);
+    }
+    const bf16* pu = up + (static_cast<long long>(b) * T + t0) * ld + c;
+    const bf16* pg = gu + (static_cast<long long>(b) * T + t0) * hid + c;
+    const bf16* px = gx + (static_cast<long long>(b) * T + t0) * hid + c;
+    constexpr int kAhead = 2;
+    uint4 nu[kAhead], ng[kAhead], nx[kAhead];   // the steps after this one, already on their way
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i) {
+      if (t0 + i < T) {
+        nu[i] = *reinterpret_cast<const uint4*>(pu + i * ld);
+        ng[i] = *reinterpret_cast<const uint4*>(pg + i * hid);
+        nx[i] = *reinterpret_cast<const uint4*>(px + i * hid);
+      }
+    }
+#pragma unroll kAhead
+    for (int i = 0; i < kRun + kTaps - 1; ++i) {
+      const int t = t0 + i;
+      const bool own = i < kRun;
+      const uint4 x_done = nx[(i + 1) % kAhead];   // of step t - 3 (the same slot: kAhead divides 4)
+      if (t < T) {
+        float g[8];
+        unpack8_bf16(nu[i % kAhead], win[kTaps - 1]);
+        unpack8_bf16(ng[i % kAhead], g);
+        if (t + kAhead < T && i + kAhead < kRun + kTaps - 1) {
+          nu[i % kAhead] = *reinterpret_cast<const uint4*>(pu + (i + kAhead) * ld);
+          ng[i % kAhead] = *reinterpret_cast<const uint4*>(pg + (i + kAhead) * hid);
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          float a = taps.b[e];
+#pragma unroll
+          for (int k = 0; k < kTaps; ++k) a = fmaf(taps.w[k][e], win[k][e], a);
+          a = held(a);
+          const float s = sigmoid(a);
+          g[e] *= s * (1.f + a * (1.f - s));
+          if (own) gb[e] += g[e];
+#pragma unroll
+          for (int k = 0; k < kTaps; ++k) {
+            acc[k][e] = fmaf(taps.w[k][e], g[e], acc[k][e]);
+            if (own) gw[k][e] = fmaf(g[e], win[k][e], gw[k][e]);
+          }
+        }
+      }
+      // input t - 3 has met every output it reaches
+      const int done = t - (kTaps - 1);
+      if (done >= t0 && done < T) {
+        const long long dt = static_cast<long long>(b) * T + done;
+        float x[8];
+        unpack8_bf16(x_done, x);
+        if (done + kAhead < T && done + kAhead < t0 + kRun)
+          nx[(i + 1) % kAhead] = *reinterpret_cast<const uint4*>(px + (i - (kTaps - 1) + kAhead) * hid);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[e] += acc[0][e];
+        store8(gup + dt * ld + c, x);
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+#pragma unroll
+        for (int k = 0; k < kTaps - 1; ++k) { win[k][e] = win[k + 1][e]; acc[k][e] = acc[k + 1][e]; }
+        acc[kTaps - 1][e] = 0.f;
+      }
+    }
+  }
+  // block sums, run groups added in order
+  const int l = threadIdx.x % lanes, rg = threadIdx.x / lanes;
+  for (int r = 0; r < 256 / lanes; ++r) {
+    __syncthreads();
+    if (rg == r) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        float* row = red + (l * 8 + e) * (kTaps + 1);
+#pragma unroll
+        for (int k = 0; k < kTaps; ++k) row[k] = (r ? row[k] : 0.f) + gw[k][e];
+        row[kTaps] = (r ? row[kTaps] : 0.f) + gb[e];
+      }
+    }
+  }
+  __syncthreads();
+  float* const out = partial + static_cast<size_t>(blockIdx.x) * hid * (kTaps + 1);
+  for (int i = threadIdx.x; i < lanes * 8 * (kTaps + 1); i += 256) {
+    const int ch = blockIdx.y * lanes * 8 + i / (kTaps + 1), k = i % (kTaps + 1);
+    out[k < kTaps ? ch * kTaps + k : hid * kTaps + ch] = red[i];
+  }
+}
+
+__global__ void __launch_bounds__(256) gates_fwd_kernel(const bf16* __restrict__ logits, const bf16* __restrict__ k, long long ld,
+                                                        float scale, float* __restrict__ log_i, float* __restrict__ log_f,
+                                                        bf16* __restrict__ ks, long long tokens, int H, int hid8, int hp, unsigned vec_blocks) {
+  if (blockIdx.x < vec_blocks) {
+    const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
+    const long long tok = i / hid8;
+    const int c = static_cast<int>(i % hid8) * 8;
+    if (tok >= tokens) return;
+    const int d = hid8 * 8 / H;
+    float x[8];
+    load8(k + tok * ld + c / d * hp + c % d, x);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) x[e] *= scale;
+    store8(ks + tok * hid8 * 8 + c, x);
+    return;
+  }
+  const long long i = static_cast<long long>(blockIdx.x - vec_blocks) * 256 + threadIdx.x;
+  if (i >= tokens * H) return;
+  const long long tok = i / H;
+  const int h = static_cast<int>(i % H);
+  log_i[i] = __bfloat162float(logits[tok * 2 * H + h]);
+  log_f[i] = -held(softplus(-__bfloat162float(logits[tok * 2 * H + H + h])));
+}
+
+constexpr int kGateBlocks = 2 * kNumSMs;
+
+__global__ void __launch_bounds__(256) gates_bwd_kernel(const bf16* __restrict__ logits, const float* __restrict__ glog_i,
+                                                        const float* __restrict__ glog_f,
+                                                        const bf16* __restrict__ gks, float scale, bf16* __restrict__ gk, long long ld,
+                                                        bf16* __restrict__ glogits, float* __restrict__ partial, long long tokens,
+                                                        int H, int hid8, int hp, unsigned vec_blocks) {
+  __shared__ float red[256];
+  if (blockIdx.x < vec_blocks) {
+    const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
+    const long long tok = i / hid8;
+    const int c = static_cast<int>(i % hid8) * 8;
+    if (tok >= tokens) return;
+    float x[8];
+    load8(gks + tok * hid8 * 8 + c, x);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) x[e] *= scale;
+    const int d = hid8 * 8 / H;
+    store8(gk + tok * ld + c / d * hp + c % d, x);
+    return;
+  }
+  const int cols = 2 * H, per = 256 / cols;
+  const int c = threadIdx.x % cols, ro = threadIdx.x / cols;
+  const unsigned blocks = gridDim.x - vec_blocks, blk = blockIdx.x - vec_blocks;
+  float sum = 0.f;
+  if (ro < per)
+    for (long long tok = static_cast<long long>(blk) * per + ro; tok < tokens; tok += static_cast<long long>(blocks) * per) {
+      float v;
+      if (c < H) v = held(glog_i[tok * H + c]);
+      else v = held(held(glog_f[tok * H + c - H]) * sigmoid(-__bfloat162float(logits[tok * cols + c])));
+      glogits[tok * cols + c] = __float2bfloat16(v);
+      sum += v;
+    }
+  red[threadIdx.x] = sum;
+  __syncthreads();
+  if (threadIdx.x < cols) {
+    float v = 0.f;
+    for (int i = 0; i < per; ++i) v += red[i * cols + threadIdx.x];
+    partial[blk * cols + threadIdx.x] = v;
+  }
+}
+
+// Statistics of a head vector held by d / 8 neighbouring lanes (a power of two, or the loop below takes shared turns).
+template <int LPH>
+__device__ __forceinline__ float head_sum(float v) {
+#pragma unroll
+  for (int o = 1; o < LPH; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+template <int LPH>
+__global__ void __launch_bounds__(256) out_fwd_kernel(const bf16* __restrict__ h, const bf16* __restrict__ u, const bf16* __restrict__ z,
+                                                      long long ld, const bf16* __restrict__ norm_w, const bf16* __restrict__ skip,
+                                                      bf16* __restrict__ g, long long tokens, int hid8) {
+  const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
+  const long long tok = i / hid8;
+  const int c = static_cast<int>(i % hid8) * 8;
+  const bool in = tok < tokens;
+  float x[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (in) load8(h + tok * hid8 * 8 + c, x);
+  float s = 0.f, q = 0.f;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) s += x[e];
+  const float mean = head_sum<LPH>(s) * (1.f / (8 * LPH));
+#pragma unroll
+  for (int e = 0; e < 8; ++e) q = fmaf(x[e] - mean, x[e] - mean, q);
+  const float rstd = rsqrtf(head_sum<LPH>(q) * (1.f / (8 * LPH)) + 1e-5f);
+  if (!in) return;
+  float w[8], sk[8], uu[8], zz[8];
+  load8(norm_w + c, w);
+  load8(skip + c, sk);
+  load8(u + tok * hid8 * 8 + c, uu);
+  load8(z + tok * ld + c, zz);
+#pragma unroll
+  for (int e = 0; e < 8; ++e) x[e] = held(held(held((x[e] - mean) * rstd) * held(1.f + w[e])) + held(sk[e] * uu[e])) * held(zz[e] * sigmoid(zz[e]));
+  store8(g + tok * hid8 * 8 + c, x);
+}
+
+// A thread keeps its eight channels over all its tokens (256 / hid8 tokens side by side in a block).
+template <int LPH>
+__global__ void __launch_bounds__(256) out_bwd_kernel(const bf16* __restrict__ gg, const bf16* __restrict__ h, const bf16* __restrict__ u,
+                                                      const bf16* __restrict__ z, long long ld, const bf16* __restrict__ norm_w,
+                                                      const bf16* __restrict__ skip, bf16* __restrict__ gh, bf16* __restrict__ gz,
+                                                      long long ld_gz, bf16* __restrict__ gu, float* __restrict__ partial,
+                                                      long long tokens, int hid8) {
+  __shared__ float red[256 * 16];
+  const int per = 256 / hid8;
+  const int c = (threadIdx.x % hid8) * 8, ro = threadIdx.x / hid8;
+  float w[8], sk[8], gw[8], gs[8];
+  load8(norm_w + c, w);
+  load8(skip + c, sk);
+#pragma unroll
+  for (int e = 0; e < 8; ++e) gw[e] = gs[e] = 0.f;
+  const long long step = static_cast<long long>(gridDim.x) * per;
+  for (long long t0 = static_cast<long long>(blockIdx.x) * per; t0 < tokens; t0 += step) {   // all lanes stay for the shuffles
+    const long long tok = t0 + ro;
+    const bool in = tok < tokens;
+    float x[8], g[8], uu[8], zz[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) x[e] = g[e] = uu[e] = zz[e] = 0.f;
+    if (in) {
+      load8(h + tok * hid8 * 8 + c, x);
+      load8(gg + tok * hid8 * 8 + c, g);
+      load8(u + tok * hid8 * 8 + c, uu);
+      load8(z + tok * ld + c, zz);
+    }
+    float s = 0.f, q = 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) s += x[e];
+    const float mean = head_sum<LPH>(s) * (1.f / (8 * LPH));
+#pragma unroll
+    for (int e = 0; e < 8; ++e) q = fmaf(x[e] - mean, x[e] - mean, q);
+    const float rstd = rsqrtf(head_sum<LPH>(q) * (1.f / (8 * LPH)) + 1e-5f);
+    float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const float sg = sigmoid(zz[e]), silu = held(zz[e] * sg), xh = (x[e] - mean) * rstd;
+      const float y = held(held(held(xh) * held(1.f + w[e])) + held(sk[e] * uu[e]));   // before the output gate
+      zz[e] = held(g[e] * y) * sg * (1.f + zz[e] * (1.f - sg));
+      g[e] = held(g[e] * silu);                               // cotangent of y
+      gw[e] += held(g[e] * held(xh));
+      gs[e] += held(g[e] * uu[e]);
+      uu[e] = g[e] * sk[e];
+      g[e] = held(g[e] * held(1.f + w[e]));
+      x[e] = xh;
+      s1 += g[e];
+      s2 = fmaf(g[e], xh, s2);
+    }
+    s1 = head_sum<LPH>(s1) * (1.f / (8 * LPH));
+    s2 = head_sum<LPH>(s2) * (1.f / (8 * LPH));
+#pragma unroll
+    for (int e = 0; e < 8; ++e) x[e] = rstd * (g[e] - s1 - x[e] * s2);
+    if (in) {
+      store8(gh + tok * hid8 * 8 + c, x);
+      store8(gz + tok * ld_gz + c, zz);
+      store8(gu + tok * hid8 * 8 + c, uu);
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    red[threadIdx.x * 16 + e] = gw[e];
+    red[threadIdx.x * 16 + 8 + e] = gs[e];
+  }
+  __syncthreads();
+  const int hid = hid8 * 8;
+  for (int i = threadIdx.x; i < 2 * hid; i += 256) {
+    const int ch = i % hid, at = (ch / 8) * 16 + (i < hid ? 0 : 8) + ch % 8;
+    float v = 0.f;
+    for (int r = 0; r < per; ++r) v += red[r * hid8 * 16 + at];
+    partial[static_cast<size_t>(blockIdx.x) * 2 * hid + i] = v;
+  }
+}
+
+// Tokens per thread of the convolution: sixteen reuse the window best; four where the machine would not be full (a thread
+// walks them one after the other)
+int run_of(int B, int T, int hid) { return static_cast<long long>(B) * T * (hid / 8) >= 16LL * 512 * kNumSMs ? 16 : 4; }
+int runs_of(int T, int run) { return (T + run - 1) / run; }
+// channel groups side by side in a block of the convolution's backward pass: 16 (128 channels) or what divides
+int conv_lanes(int hid) {
+  int l = 16;
+  while ((hid / 8) % l) l /= 2;
+  return l;
+}
+
+}  // namespace
+
+int mlstm_conv_fwd(const void* up, long long ld, const void* conv_w, const void* conv_b, void* u, int B, int T, int hid,
+                   cudaStream_t stream) {
+  const int run = run_of(B, T, hid), runs = runs_of(T, run);
+  const long long threads = static_cast<long long>(B) * runs * (hid / 8);
+  const auto go = [&](auto kernel) {
+    kernel<<<static_cast<unsigned>((threads + 255) / 256), 256, 0, stream>>>(
+        static_cast<const bf16*>(up), ld, static_cast<const bf16*>(conv_w), static_cast<const bf16*>(conv_b), static_cast<bf16*>(u), B, T, hid, runs);
+    return launch_status();
+  };
+  return run == 16 ? go(conv_fwd_kernel<16>) : go(conv_fwd_kernel<4>);
+}
+
+int mlstm_conv_blocks(int B, int T, int hid) {
+  const int per = 256 / conv_lanes(hid);
+  return static_cast<int>((static_cast<long long>(B) * runs_of(T, run_of(B, T, hid)) + per - 1) / per);
+}
+
+int mlstm_conv_bwd(const void* up, long long ld, const void* conv_w, const void* conv_b, const void* gu, const void* gx, void* gup,
+                   float* partial, int B, int T, int hid, cudaStream_t stream) {
+  const int lanes = conv_lanes(hid), bytes = lanes * 8 * (kTaps + 1) * static_cast<int>(sizeof(float));
+  const int run = run_of(B, T, hid), runs = runs_of(T, run);
+  const auto go = [&](auto kernel) {
+    kernel<<<dim3(mlstm_conv_blocks(B, T, hid), hid / 8 / lanes), 256, bytes, stream>>>(
+        static_cast<const bf16*>(up), ld, static_cast<const bf16*>(conv_w), static_cast<const bf16*>(conv_b), static_cast<const bf16*>(gu),
+        static_cast<const bf16*>(gx), static_cast<bf16*>(gup), partial, B, T, hid, runs, lanes);
+    return launch_status();
+  };
+  return run == 16 ? go(conv_bwd_kernel<16>) : go(conv_bwd_kernel<4>);
+}
+
+int mlstm_gates_fwd(const void* logits, const void* k, long long ld, int hp, float scale,
+                    float* log_i, float* log_f, void* k_scaled, long long tokens, int H, int d, cudaStream_t stream) {
+  const int hid8 = H * d / 8;
+  const unsigned vb = static_cast<unsigned>((tokens * hid8 + 255) / 256), gb = static_cast<unsigned>((tokens * H + 255) / 256);
+  gates_fwd_kernel<<<vb + gb, 256, 0, stream>>>(static_cast<const bf16*>(logits), static_cast<const bf16*>(k), ld, scale, log_i, log_f, static_cast<bf16*>(k_scaled), tokens, H, hid8, hp, vb);
+  return launch_status();
+}
+
+int mlstm_gate_blocks(long long tokens) {
+  const long long need = (tokens + 63) / 64;
+  return static_cast<int>(need < kGateBlocks ? need : kGateBlocks);
+}
+
+int mlstm_gates_bwd(const void* logits, const float* glog_i, const float* glog_f, const void* gk_scaled,
+                    float scale, void* gk, long long ld, int hp, void* glogits, float* partial, long long tokens, int H, int d,
+                    cudaStream_t stream) {
+  if (H > 128) return MXK_ERR_UNSUPPORTED;
+  const int hid8 = H * d / 8;
+  const unsigned vb = static_cast<unsigned>((tokens * hid8 + 255) / 256), gb = static_cast<unsigned>(mlstm_gate_blocks(tokens));
+  gates_bwd_kernel<<<vb + gb, 256, 0, stream>>>(static_cast<const bf16*>(logits), glog_i, glog_f,
+                                                static_cast<const bf16*>(gk_scaled), scale, static_cast<bf16*>(gk), ld, static_cast<bf16*>(glogits),
+                                                partial, tokens, H, hid8, hp, vb);
+  return launch_status();
+}
+
+int mlstm_out_fwd(const void* h, const void* u, const void* z, long long ld, const void* norm_w, const void* skip, void* g,
+                  long long tokens, int H, int d, cudaStream_t stream) {
+  const int hid8 = H * d / 8;
+  const unsigned blocks = static_cast<unsigned>((tokens * hid8 + 255) / 256);
+  const auto go = [&](auto kernel) {
+    kernel<<<blocks, 256, 0, stream>>>(static_cast<const bf16*>(h), static_cast<const bf16*>(u), static_cast<const bf16*>(z), ld,
+                                       static_cast<const bf16*>(norm_w), static_cast<const bf16*>(skip), static_cast<bf16*>(g), tokens, hid8);
+    return launch_status();
+  };
+  return d == 64 ? go(out_fwd_kernel<8>) : d == 32 ? go(out_fwd_kernel<4>) : d == 16 ? go(out_fwd_kernel<2>) : MXK_ERR_UNSUPPORTED;
+}
+
+int mlstm_out_blocks(long long tokens, int hid) {
+  const long long per = 256 / (hid / 8), need = (tokens + per - 1) / per, most = 4 * kNumSMs;
+  return static_cast<int>(need < most ? need : most);
+}
+
+int mlstm_out_bwd(const void* gg, const void* h, const void* u, const void* z, long long ld, const void* norm_w, const void* skip,
+                  void* gh, void* gz, long long ld_gz, void* gu, float* partial, long long tokens, int H, int d, cudaStream_t stream) {
+  const int hid8 = H * d / 8;
+  if (hid8 > 256 || 256 % hid8) return MXK_ERR_UNSUPPORTED;
+  const auto go = [&](auto kernel) {
+    kernel<<<mlstm_out_blocks(tokens, hid8 * 8), 256, 0, stream>>>(
+        static_cast<const bf16*>(gg), static_cast<const bf16*>(h), static_cast<const bf16*>(u), static_cast<const bf16*>(z), ld,
+        static_cast<const bf16*>(norm_w), static_cast<const bf16*>(skip), static_cast<bf16*>(gh), static_cast<bf16*>(gz), ld_gz,
+        static_cast<bf16*>(gu), partial, tokens, hid8);
+    return launch_status();
+  };
+  return d == 64 ? go(out_bwd_kernel<8>) : d == 32 ? go(out_bwd_kernel<4>) : d == 16 ? go(out_bwd_kernel<2>) : MXK_ERR_UNSUPPORTED;
+}
+
+}  // namespace layers
+}  // namespace mxk

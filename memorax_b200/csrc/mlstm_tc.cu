@@ -25,6 +25,7 @@
 
 #include <cstddef>
 
+#include "attention.cuh"
 #include "mxk_common.cuh"
 #include "linattn_common.cuh"
 #include "mlstm_tc_common.cuh"
@@ -337,22 +338,16 @@ extern "C" int mxk_debug_mtc_phase_cycles(unsigned long long* out, int reset) {
 }
 #endif
 
-extern "C" {
+namespace mxk {
+namespace mlstm_tc {
 
-size_t mxk_mlstm_bf16_chunk_states_bytes(int B, int T, int H, int d) {
-  if (B <= 0 || T <= 0 || H <= 0 || d < 8 || d > mxk::linattn::kD || d % 8) return 0;
-  const size_t nchunks = (static_cast<size_t>(T) + mxk::linattn::kC - 1) / mxk::linattn::kC;
-  return static_cast<size_t>(B) * H * nchunks * (mxk::linattn::kPanelsX * mxk::linattn::kD) * sizeof(uint4);
-}
-
-int mxk_mlstm_bf16_fwd(const void* q, const void* k, const void* v, const float* log_i, const float* log_f,
+int forward(const void* q, const void* k, const void* v, long long ld_qv, long long hp_qv, const float* log_i, const float* log_f,
                        const float* c0, const float* n0, const float* m0, const float* f0, const uint8_t* done,
                        void* h, float* c_last, float* n_last, float* m_last, float* f_last, float* m_steps,
-                       void* chunk_states, int* status, int B, int T, int H, int d, float eps, mxk_stream_t stream) {
-  using namespace mxk;
+                       void* chunk_states, int* status, int B, int T, int H, int d, float eps, cudaStream_t stream) {
   if (!q || !k || !v || !log_i || !log_f || !h) return MXK_ERR_NULL;
   if (B <= 0 || T <= 0 || H <= 0 || static_cast<long long>(B) * H > 0x7fffffffLL) return MXK_ERR_DIMS;
-  if (d < 8 || d > kD || d % 8) return MXK_ERR_UNSUPPORTED;
+  if (d < 8 || d > linattn::kD || d % 8) return MXK_ERR_UNSUPPORTED;
   for (const void* ptr : {q, k, v, (const void*)h, (const void*)chunk_states})
     if (ptr && !aligned16(ptr)) return MXK_ERR_ALIGN;
   for (const void* ptr : {(const void*)log_i, (const void*)log_f, (const void*)c0, (const void*)n0, (const void*)m0, (const void*)f0,
@@ -368,14 +363,33 @@ int mxk_mlstm_bf16_fwd(const void* q, const void* k, const void* v, const float*
   prm.status = status;
   prm.B = B; prm.T = T; prm.H = H; prm.d = d;
   prm.eps = eps;
-  if (!tma::make_sw_map(&prm.map_q, q, B, T, H, kC, d) || !tma::make_sw_map(&prm.map_k, k, B, T, H, kC, d) ||
-      !tma::make_panel_map(&prm.map_v, v, B, T, H, d, kC, kPanels) || !tma::make_sw_map(&prm.map_o, h, B, T, H, kC, d))
+  if (!tma::make_sw_map(&prm.map_q, q, B, T, H, kC, d, ld_qv, hp_qv) || !tma::make_sw_map(&prm.map_k, k, B, T, H, kC, d) ||
+      !tma::make_panel_map(&prm.map_v, v, B, T, H, d, kC, kPanels, ld_qv, hp_qv) || !tma::make_sw_map(&prm.map_o, h, B, T, H, kC, d))
     return MXK_ERR_UNSUPPORTED;
   cudaError_t e = cudaFuncSetAttribute(mlstm_tc_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(sizeof(FwdSmem)));
   if (e != cudaSuccess) return static_cast<int>(e);
-  mlstm_tc_fwd_kernel<<<B * H, kThreads, sizeof(FwdSmem), static_cast<cudaStream_t>(stream)>>>(prm);
+  mlstm_tc_fwd_kernel<<<B * H, kThreads, sizeof(FwdSmem), stream>>>(prm);
   return launch_status();
+}
+
+}  // namespace mlstm_tc
+}  // namespace mxk
+
+extern "C" {
+
+size_t mxk_mlstm_bf16_chunk_states_bytes(int B, int T, int H, int d) {
+  if (B <= 0 || T <= 0 || H <= 0 || d < 8 || d > mxk::linattn::kD || d % 8) return 0;
+  const size_t nchunks = (static_cast<size_t>(T) + mxk::linattn::kC - 1) / mxk::linattn::kC;
+  return static_cast<size_t>(B) * H * nchunks * (mxk::linattn::kPanelsX * mxk::linattn::kD) * sizeof(uint4);
+}
+
+int mxk_mlstm_bf16_fwd(const void* q, const void* k, const void* v, const float* log_i, const float* log_f,
+                       const float* c0, const float* n0, const float* m0, const float* f0, const uint8_t* done,
+                       void* h, float* c_last, float* n_last, float* m_last, float* f_last, float* m_steps,
+                       void* chunk_states, int* status, int B, int T, int H, int d, float eps, mxk_stream_t stream) {
+  return mxk::mlstm_tc::forward(q, k, v, 0, 0, log_i, log_f, c0, n0, m0, f0, done, h, c_last, n_last, m_last, f_last, m_steps, chunk_states,
+                                status, B, T, H, d, eps, static_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

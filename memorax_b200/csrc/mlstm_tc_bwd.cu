@@ -27,6 +27,7 @@
 
 #include "linattn_common.cuh"
 #include "mlstm_tc_common.cuh"
+#include "attention.cuh"
 #include "mxk_common.cuh"
 #include "tma.cuh"
 
@@ -668,21 +669,20 @@ extern "C" int mxk_debug_mtcb_phase_cycles(unsigned long long* out, int reset) {
 }
 #endif
 
-extern "C" {
+namespace mxk {
+namespace mlstm_tc {
 
-int mxk_mlstm_bf16_bwd(const void* q, const void* k, const void* v, const float* log_i, const float* log_f,
+int backward(const void* q, const void* k, const void* v, long long ld_qv, long long hp_qv, const float* log_i, const float* log_f,
                        const float* c0, const float* n0, const float* m0, const uint8_t* done, const void* dh,
                        const float* c_last, const float* n_last, const float* m_steps, const void* chunk_states,
-                       const float* dc_last, const float* dn_last, const float* dm_last, void* dq, void* dk, void* dv,
+                       const float* dc_last, const float* dn_last, const float* dm_last, void* dq, void* dk, void* dv, long long ld_grad, long long hp_grad,
                        float* dlog_i, float* dlog_f, float* dc0, float* dn0, float* dm0, int* status, int B, int T,
-                       int H, int d, float eps, mxk_stream_t stream) {
-  using namespace mxk;
-  using namespace mxk::linattn;
+                       int H, int d, float eps, cudaStream_t stream) {
   if (!q || !k || !v || !log_i || !log_f || !dh || !m_steps || !chunk_states || !dq || !dk || !dv || !dlog_i || !dlog_f)
     return MXK_ERR_NULL;
   if ((dc_last && !c_last) || (dn_last && !n_last)) return MXK_ERR_NULL;   // the gauge term needs the forward call's next carry
   if (B <= 0 || T <= 0 || H <= 0 || static_cast<long long>(B) * H > 0x7fffffffLL) return MXK_ERR_DIMS;
-  if (d < 8 || d > kD || d % 8) return MXK_ERR_UNSUPPORTED;
+  if (d < 8 || d > linattn::kD || d % 8) return MXK_ERR_UNSUPPORTED;
   for (const void* ptr : {q, k, v, dh, chunk_states, (const void*)dq, (const void*)dk, (const void*)dv})
     if (!aligned16(ptr)) return MXK_ERR_ALIGN;
   for (const void* ptr : {(const void*)log_i, (const void*)log_f, (const void*)c0, (const void*)n0, (const void*)m0, (const void*)c_last,
@@ -700,17 +700,33 @@ int mxk_mlstm_bf16_bwd(const void* q, const void* k, const void* v, const float*
   prm.B = B; prm.T = T; prm.H = H;
   prm.eps = eps;
   prm.d = d;
-  if (!tma::make_sw_map(&prm.map_q, q, B, T, H, kC, d) || !tma::make_sw_map(&prm.map_k, k, B, T, H, kC, d) ||
-      !tma::make_sw_map(&prm.map_v, v, B, T, H, kC, d) || !tma::make_sw_map(&prm.map_do, dh, B, T, H, kC, d))
+  if (!tma::make_sw_map(&prm.map_q, q, B, T, H, linattn::kC, d, ld_qv, hp_qv) || !tma::make_sw_map(&prm.map_k, k, B, T, H, linattn::kC, d) ||
+      !tma::make_sw_map(&prm.map_v, v, B, T, H, linattn::kC, d, ld_qv, hp_qv) || !tma::make_sw_map(&prm.map_do, dh, B, T, H, linattn::kC, d))
     return MXK_ERR_UNSUPPORTED;
-  if (!tma::make_sw_map(&prm.map_dq, dq, B, T, H, kC, d) || !tma::make_sw_map(&prm.map_dk, dk, B, T, H, kC, d) ||
-      !tma::make_sw_map(&prm.map_dv, dv, B, T, H, kC, d))
+  if (!tma::make_sw_map(&prm.map_dq, dq, B, T, H, linattn::kC, d, ld_grad, hp_grad) || !tma::make_sw_map(&prm.map_dk, dk, B, T, H, linattn::kC, d) ||
+      !tma::make_sw_map(&prm.map_dv, dv, B, T, H, linattn::kC, d, ld_grad, hp_grad))
     return MXK_ERR_UNSUPPORTED;
   cudaError_t e = cudaFuncSetAttribute(mlstm_tc_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(sizeof(BwdSmem)));
   if (e != cudaSuccess) return static_cast<int>(e);
-  mlstm_tc_bwd_kernel<<<B * H, kBwdThreads, sizeof(BwdSmem), static_cast<cudaStream_t>(stream)>>>(prm);
+  mlstm_tc_bwd_kernel<<<B * H, kBwdThreads, sizeof(BwdSmem), stream>>>(prm);
   return launch_status();
+}
+
+}  // namespace mlstm_tc
+}  // namespace mxk
+
+extern "C" {
+
+int mxk_mlstm_bf16_bwd(const void* q, const void* k, const void* v, const float* log_i, const float* log_f,
+                       const float* c0, const float* n0, const float* m0, const uint8_t* done, const void* dh,
+                       const float* c_last, const float* n_last, const float* m_steps, const void* chunk_states,
+                       const float* dc_last, const float* dn_last, const float* dm_last, void* dq, void* dk, void* dv,
+                       float* dlog_i, float* dlog_f, float* dc0, float* dn0, float* dm0, int* status, int B, int T,
+                       int H, int d, float eps, mxk_stream_t stream) {
+  return mxk::mlstm_tc::backward(q, k, v, 0, 0, log_i, log_f, c0, n0, m0, done, dh, c_last, n_last, m_steps, chunk_states, dc_last, dn_last,
+                                 dm_last, dq, dk, dv, 0, 0, dlog_i, dlog_f, dc0, dn0, dm0, status, B, T, H, d, eps,
+                                 static_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

@@ -34,20 +34,27 @@ inline EncodeTiledFn encode_tiled_fn() {
       ptr = nullptr;
     return reinterpret_cast<EncodeTiledFn>(ptr);
   }();
+  // The encoder needs the device's context on the calling thread; one that has only launched through a framework's
+  // guards (autograd's workers) may not have it yet.
+  thread_local bool ready = [] {
+    int dev = 0;
+    return cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess;
+  }();
+  (void)ready;
   return fn;
 }
 
 // Map whose loads write `rows` x D tiles of one (b, h) sequence in panel order [c/8][t][8].
-// Coordinates of a load: {0, t0, 0, h, b}.  `ld` (all maps): elements from one step to the next (default H * D), a multiple
-// of 8 -- the tensor may be a slice of a wider one.
+// Coordinates of a load: {0, t0, 0, h, b}.  `ld` (all maps): elements from one step to the next (default H * D), `hp` from
+// one head to the next (default D), multiples of 8 -- the tensor may be a slice of a wider one.
 inline bool make_panel_map(CUtensorMap* map, const void* base, int B, int T, int H, int D, int rows, int box_panels = 0,
-                           long long ld = 0) {
+                           long long ld = 0, long long hp = 0) {
   EncodeTiledFn enc = encode_tiled_fn();
   if (!enc) return false;
   const cuuint64_t row_bytes = static_cast<cuuint64_t>(ld > 0 ? ld : static_cast<long long>(H) * D) * 2;
   const cuuint64_t dims[5] = {8, static_cast<cuuint64_t>(T), static_cast<cuuint64_t>(D / 8), static_cast<cuuint64_t>(H),
                               static_cast<cuuint64_t>(B)};
-  const cuuint64_t strides[4] = {row_bytes, 16, static_cast<cuuint64_t>(D) * 2, row_bytes * T};
+  const cuuint64_t strides[4] = {row_bytes, 16, static_cast<cuuint64_t>(hp > 0 ? hp : D) * 2, row_bytes * T};
   // box_panels (default D / 8) may exceed D / 8: the panels past the tensor are zero-filled
   const cuuint32_t box[5] = {8, static_cast<cuuint32_t>(rows), static_cast<cuuint32_t>(box_panels > 0 ? box_panels : D / 8), 1, 1};
   const cuuint32_t elem[5] = {1, 1, 1, 1, 1};
@@ -60,14 +67,14 @@ inline bool make_panel_map(CUtensorMap* map, const void* base, int B, int T, int
 // box_cols (default D) may exceed D: the columns past D are zero-filled on loads and clipped on stores,
 // which is how a head of 64 columns is served by a kernel built for 128.
 inline bool make_plain_map(CUtensorMap* map, const void* base, int B, int T, int H, int D, int rows, int box_cols = 0,
-                           long long ld = 0) {
+                           long long ld = 0, long long hp = 0) {
   EncodeTiledFn enc = encode_tiled_fn();
   if (!enc) return false;
   if (box_cols <= 0) box_cols = D;
   const cuuint64_t row_bytes = static_cast<cuuint64_t>(ld > 0 ? ld : static_cast<long long>(H) * D) * 2;
   const cuuint64_t dims[4] = {static_cast<cuuint64_t>(D), static_cast<cuuint64_t>(H), static_cast<cuuint64_t>(T),
                               static_cast<cuuint64_t>(B)};
-  const cuuint64_t strides[3] = {static_cast<cuuint64_t>(D) * 2, row_bytes, row_bytes * T};
+  const cuuint64_t strides[3] = {static_cast<cuuint64_t>(hp > 0 ? hp : D) * 2, row_bytes, row_bytes * T};
   const cuuint32_t box[4] = {static_cast<cuuint32_t>(box_cols), 1, static_cast<cuuint32_t>(rows), 1};
   const cuuint32_t elem[4] = {1, 1, 1, 1};
   return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, elem,
@@ -79,13 +86,13 @@ inline bool make_plain_map(CUtensorMap* map, const void* base, int B, int T, int
 // lines (umma.cuh "SW tiles"): 128-byte pieces, about five times faster per byte than the panel map.
 // Coordinates {c0, h, t0, b} with c0 the first column of the block (a multiple of 64); the destination
 // must be 1024-byte aligned.
-inline bool make_sw_map(CUtensorMap* map, const void* base, int B, int T, int H, int rows, int D = 64, long long ld = 0) {
+inline bool make_sw_map(CUtensorMap* map, const void* base, int B, int T, int H, int rows, int D = 64, long long ld = 0, long long hp = 0) {
   EncodeTiledFn enc = encode_tiled_fn();
   if (!enc) return false;
   const cuuint64_t row_bytes = static_cast<cuuint64_t>(ld > 0 ? ld : static_cast<long long>(H) * D) * 2;
   const cuuint64_t dims[4] = {static_cast<cuuint64_t>(D), static_cast<cuuint64_t>(H), static_cast<cuuint64_t>(T),
                               static_cast<cuuint64_t>(B)};
-  const cuuint64_t strides[3] = {static_cast<cuuint64_t>(D) * 2, row_bytes, row_bytes * T};
+  const cuuint64_t strides[3] = {static_cast<cuuint64_t>(hp > 0 ? hp : D) * 2, row_bytes, row_bytes * T};
   const cuuint32_t box[4] = {64, 1, static_cast<cuuint32_t>(rows), 1};
   const cuuint32_t elem[4] = {1, 1, 1, 1};
   return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, elem,

@@ -584,6 +584,20 @@ class mLSTMCell(MemoroidCellBase):
         self.norm_weight = nn.Parameter(torch.zeros(num_heads, self.head_dim))   # MultiHeadLayerNorm: scale = 1 + weight
         self.output_projection = nn.Linear(hidden_dim, features, bias=False)
 
+    def layer(self, inputs, done, initial_carry, **kwargs):
+        """On the tensor cores in bf16 the whole layer is one native call; everything else is composed from its parts."""
+        if type(self) is mLSTMCell and self.tensor_cores and not kwargs:
+            c0, f0, n0, m0 = (None,) * 4 if initial_carry is None else initial_carry
+            own, sub = self._parameters, self._modules
+            of = lambda name, kind="weight": sub[name]._parameters[kind]
+            out = _C.mlstm_layer(inputs, [of("up_projection"), of("causal_conv"), of("causal_conv", "bias"), own["query"], own["key"],
+                                          own["value"], of("i_gate"), of("i_gate", "bias"), of("f_gate"), of("f_gate", "bias"),
+                                          own["learnable_skip"], own["norm_weight"], of("output_projection")], c0, f0, n0, m0, done,
+                                 self.eps)
+            if out is not None:
+                return out[:4], out[4]
+        return super().layer(inputs, done, initial_carry, **kwargs)
+
     def _block(self, x, kernel):
         bsz, steps, _ = x.shape
         return torch.einsum("bthd,hod->btho", x.view(bsz, steps, self.num_heads, self.head_dim), kernel)

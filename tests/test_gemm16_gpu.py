@@ -1,0 +1,39 @@
+"""bf16 products on the tensor cores against float64: tile edges, both contraction indices of either operand, batches in
+strided views, split contractions, bias and accumulation."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m,n,k", [(8, 8, 8), (127, 65, 64), (129, 136, 72), (260, 16, 200), (16, 768, 1000), (3000, 256, 96), (512, 256, 6000)])
+@pytest.mark.parametrize("a_t", [False, True])
+@pytest.mark.parametrize("b_t", [False, True])
+def test_product_matches_float64(m, n, k, a_t, b_t):
+    from memorax_b200 import _C, ops
+    pad = lambda v: -(-v // 8) * 8
+    g = torch.Generator("cuda").manual_seed(m + n + k)
+    mk = lambda r, c: torch.randn(r, pad(c), generator=g, device="cuda").bfloat16()[:, :c]
+    a, b = (mk(k, m).t() if a_t else mk(m, k)), (mk(n, k).t() if b_t else mk(k, n))
+    bias, c0 = mk(1, n)[0].contiguous(), mk(m, n).contiguous()
+    ref = a.double() @ b.double()
+    for got, want in ((_C.product_bf16(a, b), ref), (_C.product_bf16(a, b, bias), ref + bias.double()),
+                      (_C.product_bf16(a, b, None, c0.clone()), ref + c0.double())):
+        assert float((got.double() - want).norm() / want.norm()) <= 4e-3
+    ops.check_status()
+
+
+@pytest.mark.parametrize("tokens,heads,dim", [(5, 1, 16), (200, 4, 64), (130, 2, 32)])
+def test_batched_product_on_strided_heads(tokens, heads, dim):
+    from memorax_b200 import _C
+    g = torch.Generator("cuda").manual_seed(1)
+    mk = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    u, w, out = mk(tokens, heads, dim).permute(1, 0, 2), mk(heads, 2 * dim, dim), mk(tokens, heads, 3 * dim)
+    part = out[..., : 2 * dim].permute(1, 0, 2)
+    want = u.double() @ w.double().transpose(1, 2) + part.double()
+    rest = out[..., 2 * dim:].clone()
+    _C.product_bf16(u, w.transpose(1, 2), None, part)
+    assert float((part.double() - want).norm() / want.norm()) <= 4e-3 and torch.equal(out[..., 2 * dim:], rest)
+    gw = _C.product_bf16(part.transpose(1, 2), u)
+    want = part.double().transpose(1, 2) @ u.double()
+    assert float((gw.double() - want).norm() / want.norm()) <= 4e-3
