@@ -20,6 +20,7 @@ __global__ void __launch_bounds__(256)
 adam_bf16_kernel(uint4* __restrict__ p, float4* __restrict__ master, const uint4* __restrict__ g,
                  float4* __restrict__ m, float4* __restrict__ v, long long n8, float lr, float b1, float b2, float eps,
                  float c1, float c2, float gscale) {
+  enter_kernel();
   const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n8) return;
   float pf[8], gf[8];
@@ -64,8 +65,7 @@ extern "C" int mxk_adam_bf16_master(void* params, float* master, const void* gra
   const float c1 = 1.f / (1.f - powf(beta1, static_cast<float>(step)));
   const float c2 = 1.f / (1.f - powf(beta2, static_cast<float>(step)));
   const long long n8 = n / 8;
-  adam_bf16_kernel<<<static_cast<unsigned>((n8 + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<uint4*>(params), reinterpret_cast<float4*>(master), static_cast<const uint4*>(grads), reinterpret_cast<float4*>(m),
+  mxk::launch_kernel(adam_bf16_kernel, static_cast<unsigned>((n8 + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream), static_cast<uint4*>(params), reinterpret_cast<float4*>(master), static_cast<const uint4*>(grads), reinterpret_cast<float4*>(m),
       reinterpret_cast<float4*>(v), n8, lr, beta1, beta2, eps, c1, c2, grad_scale);
   return launch_status();
 }

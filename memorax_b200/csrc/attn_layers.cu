@@ -20,6 +20,7 @@ __device__ __forceinline__ float sigmoid(float x) { return 1.f / (1.f + __expf(-
 __device__ __forceinline__ float softplus(float x) { return x > 20.f ? x : log1pf(__expf(x)); }
 
 __global__ void __launch_bounds__(256) stack_rows_kernel(WeightRows w, uint4* __restrict__ dst, int padded, int k8) {
+  enter_kernel();
   const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
   if (i >= static_cast<long long>(padded) * k8) return;
   int row = static_cast<int>(i / k8);
@@ -44,6 +45,7 @@ __global__ void __launch_bounds__(256) stack_rows_kernel(WeightRows w, uint4* __
 __global__ void __launch_bounds__(128) small_product_kernel(const __nv_bfloat16* __restrict__ x, WeightRows w,
                                                             const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ c,
                                                             long long ldc, int M, int N, int K) {
+  enter_kernel();
   __shared__ float part[4][16][33];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, t = lane & 3;
@@ -129,6 +131,7 @@ __global__ void __launch_bounds__(kStepThreads) linattn_step_kernel(const __nv_b
                                                                     const __nv_bfloat16* __restrict__ norm_w, float norm_eps,
                                                                     float eps, __nv_bfloat16* __restrict__ y,
                                                                     float* __restrict__ s_last, float* __restrict__ z_last, int H) {
+  enter_kernel();
   extern __shared__ __align__(16) float sm[];   // q | k | v | o of all heads, then the denominators
   constexpr int kVecs = D / 32, kLanes = 8;     // 16-byte vectors per lane; lanes per row
   __shared__ float red[kStepThreads / 32];
@@ -188,6 +191,7 @@ __global__ void __launch_bounds__(kStepThreads) gdelta_step_kernel(const __nv_bf
                                                                    const float* __restrict__ s0, const uint8_t* __restrict__ done,
                                                                    const __nv_bfloat16* __restrict__ norm_w, float norm_eps,
                                                                    __nv_bfloat16* __restrict__ y, float* __restrict__ s_last, int H) {
+  enter_kernel();
   extern __shared__ __align__(16) float sm[];   // q | k | v | o, then alpha | beta
   constexpr int kLanes = 16, kVecs = D / 64;
   __shared__ float red[kStepThreads / 32];
@@ -257,6 +261,7 @@ __global__ void __launch_bounds__(256) delta_inputs_kernel(const __nv_bfloat16* 
                                                            const __nv_bfloat16* __restrict__ gate_bias, uint4* __restrict__ q,
                                                            uint4* __restrict__ k, float* __restrict__ alpha,
                                                            float* __restrict__ beta, long long tokens, int H, unsigned vec_blocks) {
+  enter_kernel();
   const int hid8 = H * LPH;
   if (blockIdx.x < vec_blocks) {
     const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
@@ -291,6 +296,7 @@ __global__ void __launch_bounds__(256) delta_inputs_bwd_kernel(const __nv_bfloat
                                                                const float* __restrict__ dalpha, const float* __restrict__ dbeta,
                                                                __nv_bfloat16* __restrict__ g, float* __restrict__ partial,
                                                                long long tokens, int H, unsigned vec_blocks) {
+  enter_kernel();
   __shared__ float red[256];
   const int hid8 = H * LPH, hid = hid8 * 8;
   if (blockIdx.x < vec_blocks) {
@@ -347,7 +353,7 @@ constexpr int kGateBlocks = 2 * kNumSMs;
 int stack_rows(const WeightRows& w, void* dst, int padded, int K, cudaStream_t stream) {
   if (K % 8 || w.count < 1 || w.count > kMaxWeights) return MXK_ERR_UNSUPPORTED;
   const long long vecs = static_cast<long long>(padded) * (K / 8);
-  stack_rows_kernel<<<static_cast<unsigned>((vecs + 255) / 256), 256, 0, stream>>>(w, static_cast<uint4*>(dst), padded, K / 8);
+  mxk::launch_kernel(stack_rows_kernel, static_cast<unsigned>((vecs + 255) / 256), 256, 0, stream, w, static_cast<uint4*>(dst), padded, K / 8);
   return launch_status();
 }
 
@@ -355,8 +361,7 @@ int small_product(const void* x, const WeightRows& w, const void* bias, void* c,
   if (K % 32 || M <= 0 || w.count < 1 || w.count > kMaxWeights) return MXK_ERR_UNSUPPORTED;
   int N = 0;
   for (int i = 0; i < w.count; ++i) N += w.rows[i];
-  small_product_kernel<<<dim3((N + 31) / 32, (M + 15) / 16), 128, 0, stream>>>(
-      static_cast<const __nv_bfloat16*>(x), w, static_cast<const __nv_bfloat16*>(bias), static_cast<__nv_bfloat16*>(c), ldc, M, N, K);
+  mxk::launch_kernel(small_product_kernel, dim3((N + 31) / 32, (M + 15) / 16), 128, 0, stream, static_cast<const __nv_bfloat16*>(x), w, static_cast<const __nv_bfloat16*>(bias), static_cast<__nv_bfloat16*>(c), ldc, M, N, K);
   return launch_status();
 }
 
@@ -367,8 +372,8 @@ int linattn_step(const void* qkv, long long ld, const float* s0, const float* z0
   const auto* nw = static_cast<const __nv_bfloat16*>(norm_w);
   auto* out = static_cast<__nv_bfloat16*>(y);
   if (bytes > 48 * 1024) return MXK_ERR_UNSUPPORTED;
-  if (d == 64) linattn_step_kernel<64><<<B, kStepThreads, bytes, stream>>>(x, ld, s0, z0, done, nw, norm_eps, eps, out, s_last, z_last, H);
-  else if (d == 32) linattn_step_kernel<32><<<B, kStepThreads, bytes, stream>>>(x, ld, s0, z0, done, nw, norm_eps, eps, out, s_last, z_last, H);
+  if (d == 64) mxk::launch_kernel(linattn_step_kernel<64>, B, kStepThreads, bytes, stream, x, ld, s0, z0, done, nw, norm_eps, eps, out, s_last, z_last, H);
+  else if (d == 32) mxk::launch_kernel(linattn_step_kernel<32>, B, kStepThreads, bytes, stream, x, ld, s0, z0, done, nw, norm_eps, eps, out, s_last, z_last, H);
   else return MXK_ERR_UNSUPPORTED;
   return launch_status();
 }
@@ -381,8 +386,8 @@ int gdelta_step(const void* qkvg, long long ld, const void* gate_bias, const flo
   const auto* nw = static_cast<const __nv_bfloat16*>(norm_w);
   auto* out = static_cast<__nv_bfloat16*>(y);
   if (bytes > 48 * 1024) return MXK_ERR_UNSUPPORTED;
-  if (d == 128) gdelta_step_kernel<128><<<B, kStepThreads, bytes, stream>>>(x, ld, gb, s0, done, nw, norm_eps, out, s_last, H);
-  else if (d == 64) gdelta_step_kernel<64><<<B, kStepThreads, bytes, stream>>>(x, ld, gb, s0, done, nw, norm_eps, out, s_last, H);
+  if (d == 128) mxk::launch_kernel(gdelta_step_kernel<128>, B, kStepThreads, bytes, stream, x, ld, gb, s0, done, nw, norm_eps, out, s_last, H);
+  else if (d == 64) mxk::launch_kernel(gdelta_step_kernel<64>, B, kStepThreads, bytes, stream, x, ld, gb, s0, done, nw, norm_eps, out, s_last, H);
   else return MXK_ERR_UNSUPPORTED;
   return launch_status();
 }
@@ -393,8 +398,8 @@ int delta_inputs(const void* qkvg, long long ld, const void* gate_bias, void* q,
   const unsigned vb = static_cast<unsigned>((vecs + 255) / 256), gb = static_cast<unsigned>((tokens * H + 255) / 256);
   const auto* x = static_cast<const __nv_bfloat16*>(qkvg);
   const auto* bias = static_cast<const __nv_bfloat16*>(gate_bias);
-  if (d == 64) delta_inputs_kernel<8><<<vb + gb, 256, 0, stream>>>(x, ld, bias, static_cast<uint4*>(q), static_cast<uint4*>(k), alpha, beta, tokens, H, vb);
-  else if (d == 128) delta_inputs_kernel<16><<<vb + gb, 256, 0, stream>>>(x, ld, bias, static_cast<uint4*>(q), static_cast<uint4*>(k), alpha, beta, tokens, H, vb);
+  if (d == 64) mxk::launch_kernel(delta_inputs_kernel<8>, vb + gb, 256, 0, stream, x, ld, bias, static_cast<uint4*>(q), static_cast<uint4*>(k), alpha, beta, tokens, H, vb);
+  else if (d == 128) mxk::launch_kernel(delta_inputs_kernel<16>, vb + gb, 256, 0, stream, x, ld, bias, static_cast<uint4*>(q), static_cast<uint4*>(k), alpha, beta, tokens, H, vb);
   else return MXK_ERR_UNSUPPORTED;
   return launch_status();
 }
@@ -412,8 +417,8 @@ int delta_inputs_bwd(const void* qkvg, long long ld, const void* gate_bias, cons
   const auto* x = static_cast<const __nv_bfloat16*>(qkvg);
   const auto* bias = static_cast<const __nv_bfloat16*>(gate_bias);
   auto* out = static_cast<__nv_bfloat16*>(g);
-  if (d == 64) delta_inputs_bwd_kernel<8><<<vb + gb, 256, 0, stream>>>(x, ld, bias, static_cast<const uint4*>(dq), static_cast<const uint4*>(dk), dalpha, dbeta, out, partial, tokens, H, vb);
-  else if (d == 128) delta_inputs_bwd_kernel<16><<<vb + gb, 256, 0, stream>>>(x, ld, bias, static_cast<const uint4*>(dq), static_cast<const uint4*>(dk), dalpha, dbeta, out, partial, tokens, H, vb);
+  if (d == 64) mxk::launch_kernel(delta_inputs_bwd_kernel<8>, vb + gb, 256, 0, stream, x, ld, bias, static_cast<const uint4*>(dq), static_cast<const uint4*>(dk), dalpha, dbeta, out, partial, tokens, H, vb);
+  else if (d == 128) mxk::launch_kernel(delta_inputs_bwd_kernel<16>, vb + gb, 256, 0, stream, x, ld, bias, static_cast<const uint4*>(dq), static_cast<const uint4*>(dk), dalpha, dbeta, out, partial, tokens, H, vb);
   else return MXK_ERR_UNSUPPORTED;
   return launch_status();
 }

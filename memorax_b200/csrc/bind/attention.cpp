@@ -41,20 +41,23 @@ Tensor project(const Tensor& x, const variable_list& w, size_t count, const Shap
   check("stack_rows", l::stack_rows(rows_of(w, count), joint.data_ptr(), s.ld, s.F, stream()));
   // tiles fit q | k | v; the few columns behind them would cost a tile column (65536 x 3088 x 512 in the library: 198 us
   // against 160 for 3072 and 17 for 16)
-  const Tensor rows = x.view({s.M, s.F});
-  product_into(rows, joint.narrow(0, 0, 3 * s.hid).t(), proj.narrow(1, 0, 3 * s.hid));
-  if (s.ld > 3 * s.hid) product_into(rows, joint.narrow(0, 3 * s.hid, s.ld - 3 * s.hid).t(), proj.narrow(1, 3 * s.hid, s.ld - 3 * s.hid));
+  const Tensor rows = matrix(x, s.M, s.F);
+  const int64_t main = 3 * s.hid, rest = s.ld - main;
+  product_into(rows, transposed(matrix(joint, main, s.F)), matrix(proj, s.M, main, s.ld));
+  if (rest) product_into(rows, transposed(matrix(joint, rest, s.F, 0, main * s.F)), matrix(proj, s.M, rest, s.ld, main));
   if (stacked) *stacked = joint;
   return proj;
 }
 
 Tensor output(const Tensor& n, const Tensor& w, const Tensor& bias, const Shape& s, bool few) {
   if (few && s.M <= kFewRows && s.hid % 32 == 0) {
-    const Tensor y = empty_like_of(n, {s.M, s.out}, at::kBFloat16);
+    const Tensor y = empty_like_of(n, {s.B, s.T, s.out}, at::kBFloat16);
     check("small_product", l::small_product(n.data_ptr(), rows_of({w}, 1), bias.data_ptr(), y.data_ptr(), s.out, s.M, s.hid, stream()));
     return y;
   }
-  return product(n, w.t(), bias);
+  const Tensor y = empty_like_of(n, {s.B, s.T, s.out}, at::kBFloat16);
+  product_into(n, transposed(w), matrix(y, s.M, s.out), bias);
+  return y;
 }
 
 // What follows the mixer: RMSNorm and output projection, and their gradients
@@ -62,7 +65,7 @@ struct Tail {
   Tensor n, rstd;
 };
 Tail norm_forward(const Tensor& o, const Tensor& norm_w, double norm_eps, const Shape& s) {
-  Tail t{at::empty_like(o), empty_like_of(o, {s.M}, at::kFloat)};
+  Tail t{empty_like_of(o, o.sizes(), at::kBFloat16), empty_like_of(o, {s.M}, at::kFloat)};
   check("mxk_norm_bf16_fwd", mxk_norm_bf16_fwd(o.data_ptr(), norm_w.data_ptr(), nullptr, t.n.data_ptr(), nullptr, ptr(t.rstd), s.M, s.hid,
                                                norm_eps, 1, stream()));
   return t;
@@ -73,12 +76,12 @@ struct TailGrads {
 TailGrads tail_backward(const Tensor& gy, const Tensor& o, const Tensor& n, const Tensor& rstd, const Tensor& norm_w, const Tensor& out_w, const Shape& s) {
   TailGrads g;
   const Tensor gn = product(gy, out_w);
-  g.out_w = product(gy.t(), n);
+  g.out_w = product(transposed(gy), n);
   g.out_b = empty_like_of(gy, {s.out}, at::kBFloat16);
   const size_t sum_bytes = mxk_colsum_workspace_bytes(s.M, s.out), norm_bytes = mxk_norm_bwd_workspace_bytes(s.M, s.hid);
   const Tensor ws = scratch(gy, std::max(sum_bytes, norm_bytes));
   check("mxk_colsum_bf16", mxk_colsum_bf16(gy.data_ptr(), g.out_b.data_ptr(), ws.data_ptr(), sum_bytes, s.M, s.out, stream()));
-  g.go = at::empty_like(o);
+  g.go = empty_like_of(o, o.sizes(), at::kBFloat16);
   const Tensor gw = empty_like_of(gy, {s.hid}, at::kFloat);
   check("mxk_norm_bf16_bwd", mxk_norm_bf16_bwd(o.data_ptr(), norm_w.data_ptr(), nullptr, ptr(rstd), gn.data_ptr(), g.go.data_ptr(), ptr(gw), nullptr,
                                                ws.data_ptr(), norm_bytes, s.M, s.hid, 1, stream()));
@@ -101,7 +104,6 @@ bool wants_grad(const Tensor& x, const variable_list& p, std::initializer_list<T
   for (const Tensor& t : carry) grad |= t.defined() && t.requires_grad();
   return grad;
 }
-Tensor leaf(const OptTensor& t, const char* name) { return t && t->defined() ? dev(t->select(1, 0), at::kFloat, name) : Tensor(); }
 const uint8_t* cols_of(const Tensor& t, int64_t column) { return static_cast<const uint8_t*>(t.data_ptr()) + 2 * column; }
 uint8_t* cols_out(const Tensor& t, int64_t column) { return static_cast<uint8_t*>(t.data_ptr()) + 2 * column; }
 
@@ -132,14 +134,14 @@ struct LinResult {
 LinResult linattn_forward(const Tensor& x, const variable_list& p, const Tensor& s0, const Tensor& z0, const Tensor& done, const Shape& s, double eps,
                           double norm_eps, bool keep) {
   LinResult r;
-  r.s_last = empty_like_of(x, {s.B, s.H, s.d, s.d}, at::kFloat);
-  r.z_last = empty_like_of(x, {s.B, s.H, s.d}, at::kFloat);
+  r.s_last = empty_like_of(x, {s.B, 1, s.H, s.d, s.d}, at::kFloat);
+  r.z_last = empty_like_of(x, {s.B, 1, s.H, s.d}, at::kFloat);
   r.proj = project(x, p, 3, s, keep ? &r.joint : nullptr);
   if (s.T == 1 && !keep && (s.d == 64 || s.d == 32) && s.hid <= 2048) {
     const Tensor n = empty_like_of(x, {s.M, s.hid}, at::kBFloat16);
     check("linattn_step", l::linattn_step(r.proj.data_ptr(), s.ld, ptr(s0), ptr(z0), bytes(done), p[kNorm].data_ptr(), norm_eps, eps, n.data_ptr(),
                                           ptr(r.s_last), ptr(r.z_last), s.B, s.H, s.d, stream()));
-    r.y = output(n, p[kOutW], p[kOutB], s, true).view({s.B, s.T, s.out});
+    r.y = output(n, p[kOutW], p[kOutB], s, true);
     return r;
   }
   r.o = empty_like_of(x, {s.M, s.hid}, at::kBFloat16);
@@ -148,7 +150,7 @@ LinResult linattn_forward(const Tensor& x, const variable_list& p, const Tensor&
                                                       r.o.data_ptr(), ptr(r.s_last), ptr(r.z_last), ptr<void>(r.states), status_ptr(x), s.B, s.T, s.H, s.d,
                                                       eps, 1, stream()));
   r.tail = norm_forward(r.o, p[kNorm], norm_eps, s);
-  r.y = output(r.tail.n, p[kOutW], p[kOutB], s, !keep).view({s.B, s.T, s.out});
+  r.y = output(r.tail.n, p[kOutW], p[kOutB], s, !keep);
   return r;
 }
 
@@ -174,20 +176,23 @@ variable_list LinAttnLayer::backward(AutogradContext* ctx, const variable_list& 
   const c10::cuda::CUDAGuard guard(x.device());
   const int64_t hid = out_w.size(1);
   const Shape s = shape_of(x, ctx->saved_data["heads"].toInt(), hid, out_w.size(0), 0);
-  const Tensor gy = (gout[2].defined() ? gout[2].contiguous() : empty_like_of(x, {s.M, s.out}, at::kBFloat16).zero_()).view({s.M, s.out});
+  const Tensor gy = matrix(gout[2].defined() ? gout[2].contiguous() : empty_like_of(x, {s.M, s.out}, at::kBFloat16).zero_(), s.M, s.out);
   const Tensor gs = gout[0].defined() ? gout[0].contiguous() : Tensor(), gz = gout[1].defined() ? gout[1].contiguous() : Tensor();
   const bool has_s = ctx->saved_data["s0"].toBool(), has_z = ctx->saved_data["z0"].toBool();
   const bool need_s = (has_s && ctx->needs_input_grad(7)) || (has_z && ctx->needs_input_grad(has_s ? 8 : 7));
   const TailGrads t = tail_backward(gy, o, saved[8], saved[9], norm_w, out_w, s);
-  const Tensor gproj = at::empty_like(proj);
-  const Tensor gs0 = need_s ? empty_like_of(x, {s.B, s.H, s.d, s.d}, at::kFloat) : Tensor(), gz0 = need_s ? empty_like_of(x, {s.B, s.H, s.d}, at::kFloat) : Tensor();
+  const Tensor gproj = empty_like_of(x, proj.sizes(), at::kBFloat16);
+  const Tensor gs0 = need_s ? empty_like_of(x, {s.B, 1, s.H, s.d, s.d}, at::kFloat) : Tensor(), gz0 = need_s ? empty_like_of(x, {s.B, 1, s.H, s.d}, at::kFloat) : Tensor();
   check("mxk_linattn_bf16_bwd", mxk::linattn::backward(cols_of(proj, 0), cols_of(proj, hid), cols_of(proj, 2 * hid), s.ld, t.go.data_ptr(), states.data_ptr(), bytes(done),
                                                        ptr(gs), ptr(gz), cols_out(gproj, 0), cols_out(gproj, hid), cols_out(gproj, 2 * hid), s.ld, ptr(gs0), ptr(gz0),
                                                        status_ptr(x), s.B, s.T, s.H, s.d, ctx->saved_data["eps"].toDouble(), 1, stream()));
   variable_list grads(13);
-  if (ctx->needs_input_grad(0)) grads[0] = product(gproj, joint).view(x.sizes());
-  const Tensor gw = product(gproj.t(), x.view({s.M, s.F}));
-  for (int i = 0; i < 3; ++i) grads[1 + i] = gw.narrow(0, i * hid, hid);
+  if (ctx->needs_input_grad(0)) {
+    grads[0] = empty_like_of(x, x.sizes(), at::kBFloat16);
+    product_into(gproj, joint, matrix(grads[0], s.M, s.F));
+  }
+  const Tensor gw = product(transposed(gproj), matrix(x, s.M, s.F));
+  for (int i = 0; i < 3; ++i) grads[1 + i] = piece(gw, i * hid * s.F, {hid, s.F});
   grads[4] = t.norm_w;
   grads[5] = t.out_w;
   grads[6] = t.out_b;
@@ -205,13 +210,13 @@ pybind11::object linattn_layer(const Tensor& x_in, const variable_list& p, const
       x_in.size(0) * heads > 0x7fffffff)
     return pybind11::none();
   const c10::cuda::CUDAGuard guard(x_in.device());
-  const Tensor x = x_in.contiguous(), s0 = leaf(s0_in, "s0"), z0 = leaf(z0_in, "z0"), done = done_bytes(done_in);
+  const Tensor x = x_in.contiguous(), s0 = carry_leaf(s0_in, x.size(0) * hid * d, at::kFloat, "s0"), z0 = carry_leaf(z0_in, x.size(0) * hid, at::kFloat, "z0"), done = done_bytes(done_in, x.size(0) * x.size(1));
   if (wants_grad(x, p, {s0, z0})) {
     const variable_list out = LinAttnLayer::apply(x, p[0], p[1], p[2], p[3], p[4], p[5], opt(s0), opt(z0), opt(done), heads, eps, norm_eps);
-    return pybind11::cast(std::make_tuple(out[0].unsqueeze(1), out[1].unsqueeze(1), out[2]));
+    return pybind11::cast(std::make_tuple(out[0], out[1], out[2]));
   }
   const LinResult r = linattn_forward(x, p, s0, z0, done, shape_of(x, heads, hid, p[kOutW].size(0), 0), eps, norm_eps, false);
-  return pybind11::cast(std::make_tuple(r.s_last.unsqueeze(1), r.z_last.unsqueeze(1), r.y));
+  return pybind11::cast(std::make_tuple(r.s_last, r.z_last, r.y));
 }
 
 // ------------------------------------------------------------------------------------------------ gated delta rule
@@ -223,13 +228,13 @@ struct DeltaResult {
 };
 DeltaResult delta_forward(const Tensor& x, const variable_list& p, const Tensor& s0, const Tensor& done, const Shape& s, double norm_eps, bool keep) {
   DeltaResult r;
-  r.s_last = empty_like_of(x, {s.B, s.H, s.d, s.d}, at::kFloat);
+  r.s_last = empty_like_of(x, {s.B, 1, s.H, s.d, s.d}, at::kFloat);
   r.proj = project(x, p, 4, s, keep ? &r.joint : nullptr);
   if (s.T == 1 && !keep && s.hid <= 2048) {
     const Tensor n = empty_like_of(x, {s.M, s.hid}, at::kBFloat16);
     check("gdelta_step", l::gdelta_step(r.proj.data_ptr(), s.ld, p[kGateB].data_ptr(), ptr(s0), bytes(done), p[kDNorm].data_ptr(), norm_eps, n.data_ptr(),
                                         ptr(r.s_last), s.B, s.H, s.d, stream()));
-    r.y = output(n, p[kDOutW], p[kDOutB], s, true).view({s.B, s.T, s.out});
+    r.y = output(n, p[kDOutW], p[kDOutB], s, true);
     return r;
   }
   r.q = empty_like_of(x, {s.M, s.hid}, at::kBFloat16);
@@ -245,7 +250,7 @@ DeltaResult delta_forward(const Tensor& x, const variable_list& p, const Tensor&
                                                     r.o.data_ptr(), ptr(r.s_last), ptr<void>(r.states), r.ws.data_ptr(), ws_bytes, status_ptr(x), s.B, s.T, s.H,
                                                     s.d, stream()));
   r.tail = norm_forward(r.o, p[kDNorm], norm_eps, s);
-  r.y = output(r.tail.n, p[kDOutW], p[kDOutB], s, !keep).view({s.B, s.T, s.out});
+  r.y = output(r.tail.n, p[kDOutW], p[kDOutB], s, !keep);
   return r;
 }
 
@@ -271,14 +276,14 @@ struct DeltaLayer : torch::autograd::Function<DeltaLayer> {
     const c10::cuda::CUDAGuard guard(x.device());
     const int64_t hid = out_w.size(1);
     const Shape s = shape_of(x, ctx->saved_data["heads"].toInt(), hid, out_w.size(0), 2 * ctx->saved_data["heads"].toInt());
-    const Tensor gy = (gout[1].defined() ? gout[1].contiguous() : empty_like_of(x, {s.M, s.out}, at::kBFloat16).zero_()).view({s.M, s.out});
+    const Tensor gy = matrix(gout[1].defined() ? gout[1].contiguous() : empty_like_of(x, {s.M, s.out}, at::kBFloat16).zero_(), s.M, s.out);
     const Tensor gs = gout[0].defined() ? gout[0].contiguous() : Tensor();
     const bool need_s0 = ctx->saved_data["s0"].toBool() && ctx->needs_input_grad(9);
     const TailGrads t = tail_backward(gy, o, saved[14], saved[15], norm_w, out_w, s);
-    const Tensor gproj = at::empty_like(proj), gq = at::empty_like(q), gk = at::empty_like(k);
-    const Tensor ga = at::empty_like(alpha), gb = at::empty_like(beta);
+    const Tensor gproj = empty_like_of(x, proj.sizes(), at::kBFloat16), gq = empty_like_of(x, q.sizes(), at::kBFloat16), gk = empty_like_of(x, k.sizes(), at::kBFloat16);
+    const Tensor ga = empty_like_of(x, alpha.sizes(), at::kFloat), gb = empty_like_of(x, beta.sizes(), at::kFloat);
     variable_list grads(13);
-    if (need_s0) grads[9] = empty_like_of(x, {s.B, s.H, s.d, s.d}, at::kFloat);
+    if (need_s0) grads[9] = empty_like_of(x, {s.B, 1, s.H, s.d, s.d}, at::kFloat);
     check("mxk_gdelta_bf16_bwd", mxk::gdelta::backward(q.data_ptr(), k.data_ptr(), cols_of(proj, 2 * hid), ptr(alpha), ptr(beta), t.go.data_ptr(), states.data_ptr(), ws.data_ptr(),
                                                        bytes(done), ptr(gs), gq.data_ptr(), gk.data_ptr(), cols_out(gproj, 2 * hid), s.ld, ptr(ga), ptr(gb),
                                                        need_s0 ? ptr(grads[9]) : nullptr, status_ptr(x), s.B, s.T, s.H, s.d, stream()));
@@ -288,10 +293,13 @@ struct DeltaLayer : torch::autograd::Function<DeltaLayer> {
                                                   s.d, stream()));
     const l::ColumnSum sum{ptr(part), rows, 2 * s.H, ptr(part) + static_cast<size_t>(rows) * 2 * s.H};
     check("column_sums", l::column_sums(&sum, 1, stream()));
-    if (ctx->needs_input_grad(0)) grads[0] = product(gproj, joint).view(x.sizes());
-    const Tensor rows_in = x.view({s.M, s.F}), gw = product(gproj.narrow(1, 0, 3 * hid).t(), rows_in);
-    for (int i = 0; i < 3; ++i) grads[1 + i] = gw.narrow(0, i * hid, hid);
-    grads[4] = product(gproj.narrow(1, 3 * hid, 2 * s.H).t(), rows_in);
+    if (ctx->needs_input_grad(0)) {
+      grads[0] = empty_like_of(x, x.sizes(), at::kBFloat16);
+      product_into(gproj, joint, matrix(grads[0], s.M, s.F));
+    }
+    const Tensor rows_in = matrix(x, s.M, s.F), gw = product(transposed(matrix(gproj, s.M, 3 * hid, s.ld)), rows_in);
+    for (int i = 0; i < 3; ++i) grads[1 + i] = piece(gw, i * hid * s.F, {hid, s.F});
+    grads[4] = product(transposed(matrix(gproj, s.M, 2 * s.H, s.ld, 3 * hid)), rows_in);
     grads[5] = part[rows].to(at::kBFloat16);
     grads[6] = t.norm_w;
     grads[7] = t.out_w;
@@ -308,13 +316,13 @@ pybind11::object deltanet_layer(const Tensor& x_in, const variable_list& p, cons
       p[kGateW].size(0) != 2 * heads || x_in.size(0) * heads > 0x7fffffff)
     return pybind11::none();
   const c10::cuda::CUDAGuard guard(x_in.device());
-  const Tensor x = x_in.contiguous(), s0 = leaf(s0_in, "s0"), done = done_bytes(done_in);
+  const Tensor x = x_in.contiguous(), s0 = carry_leaf(s0_in, x.size(0) * hid * d, at::kFloat, "s0"), done = done_bytes(done_in, x.size(0) * x.size(1));
   if (wants_grad(x, p, {s0})) {
     const variable_list out = DeltaLayer::apply(x, p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7], opt(s0), opt(done), heads, norm_eps);
-    return pybind11::cast(std::make_tuple(out[0].unsqueeze(1), out[1]));
+    return pybind11::cast(std::make_tuple(out[0], out[1]));
   }
   const DeltaResult r = delta_forward(x, p, s0, done, shape_of(x, heads, hid, p[kDOutW].size(0), 2 * heads), norm_eps, false);
-  return pybind11::cast(std::make_tuple(r.s_last.unsqueeze(1), r.y));
+  return pybind11::cast(std::make_tuple(r.s_last, r.y));
 }
 
 }  // namespace

@@ -3,6 +3,7 @@
 
 #include <ATen/autocast_mode.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
@@ -38,17 +39,47 @@ inline Tensor dev(const OptTensor& t, at::ScalarType dtype, const char* name) {
   return (t->scalar_type() == dtype ? *t : t->to(dtype)).contiguous();
 }
 // (B,T) flags of any dtype -> bytes
-inline Tensor done_bytes(const OptTensor& done) {
+inline Tensor done_bytes(const OptTensor& done, int64_t steps) {
   if (!done || !done->defined()) return Tensor();
   TORCH_CHECK_VALUE(done->is_cuda(), "done must be a CUDA tensor");
+  TORCH_CHECK_VALUE(done->numel() == steps, "done has ", done->numel(), " flags for ", steps, " steps");
   if (done->scalar_type() == at::kBool || done->scalar_type() == at::kByte) return done->contiguous();
   return done->ne(0).contiguous();
 }
+// Allocations and views of buffers that no graph tracks, without a trip through the dispatcher (1-2 us each, and a layer
+// has tens of them).
 inline Tensor empty_like_of(const Tensor& t, at::IntArrayRef sizes, at::ScalarType dtype) {
-  return at::empty(sizes, t.options().dtype(dtype).requires_grad(false));
+  return Tensor(at::detail::empty_cuda(sizes, dtype, t.device(), std::nullopt));
 }
-inline Tensor scratch(const Tensor& t, size_t n) {
-  return at::empty({static_cast<int64_t>(n ? n : 1)}, t.options().dtype(at::kByte).requires_grad(false));
+inline Tensor scratch(const Tensor& t, size_t n) { return empty_like_of(t, {static_cast<int64_t>(n ? n : 1)}, at::kByte); }
+inline Tensor view_of(const Tensor& t, int64_t offset, at::IntArrayRef sizes, at::IntArrayRef strides) {
+  Tensor v = at::detail::make_tensor<c10::TensorImpl>(c10::TensorImpl::VIEW, c10::Storage(t.storage()), t.key_set(), t.dtype());
+  v.unsafeGetTensorImpl()->set_storage_offset(t.storage_offset() + offset);
+  v.unsafeGetTensorImpl()->set_sizes_and_strides(sizes, strides);
+  return v;
+}
+// (rows, cols) at an element offset, and the same transposed
+inline Tensor matrix(const Tensor& t, int64_t rows, int64_t cols, int64_t ld = 0, int64_t offset = 0) {
+  return view_of(t, offset, {rows, cols}, {ld ? ld : cols, 1});
+}
+inline Tensor transposed(const Tensor& t) { return view_of(t, 0, {t.size(1), t.size(0)}, {t.stride(1), t.stride(0)}); }
+// contiguous, `sizes` at an element offset
+inline Tensor piece(const Tensor& t, int64_t offset, at::IntArrayRef sizes) {
+  c10::SmallVector<int64_t, 6> strides(sizes.size(), 1);
+  for (int i = static_cast<int>(sizes.size()) - 2; i >= 0; --i) strides[i] = strides[i + 1] * sizes[i + 1];
+  return view_of(t, offset, sizes, strides);
+}
+// A leaf of the carry with its singleton time axis kept: (B, 1, ...) and (B, ...) are the same memory.
+inline Tensor carry_leaf(const OptTensor& t, int64_t numel, at::ScalarType dtype, const char* name) {
+  if (!t || !t->defined()) return Tensor();
+  const Tensor leaf = dev(t->dim() > 1 && t->size(1) != 1 ? t->narrow(1, 0, 1) : *t, dtype, name);
+  TORCH_CHECK_VALUE(leaf.numel() == numel, name, " of the carry has ", leaf.numel(), " elements, expected ", numel);
+  return leaf;
+}
+// the last step of contiguous states (B, T, N)
+inline Tensor last_state(const Tensor& h) {
+  const int64_t B = h.size(0), T = h.size(1), N = h.size(2);
+  return view_of(h, (T - 1) * N, {B, 1, N}, {T * N, N, 1});
 }
 inline size_t align_up(size_t n) { return (n + 255) & ~static_cast<size_t>(255); }
 

@@ -9,9 +9,9 @@ std::tuple<Tensor, OptTensor> linrec_fwd(const Tensor& a_in, const Tensor& b_in,
   const bool cplx = b_in.is_complex();
   const auto dt = cplx ? at::kComplexFloat : at::kFloat;
   const Tensor b = dev(b_in, dt, "b"), a = dev(a_in, dt, "a"), h0 = dev(h0_in, dt, "h0"), a0 = dev(a0_in, dt, "a0");
-  const Tensor done = done_bytes(done_in);
   const c10::cuda::CUDAGuard guard(b.device());
   TORCH_CHECK_VALUE(b.dim() == 3, "b must be (B, T, D)");
+  const Tensor done = done_bytes(done_in, b.size(0) * b.size(1));
   const int64_t bsz = b.size(0), steps = b.size(1), dim = b.size(2);
   const bool tinv = a.dim() == 1;
   if (tinv ? a.size(0) != dim : a.sizes() != b.sizes()) assertion("a must be (D,) or of b's shape");

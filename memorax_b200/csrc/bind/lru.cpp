@@ -48,7 +48,7 @@ Result forward(const Tensor& x, const variable_list& params, const Tensor& h0, c
   const LruWeights w = weights_of(params);
   Result r;
   r.h = empty_like_of(x, {B, T, N}, at::kComplexFloat);
-  r.a_last = empty_like_of(x, {B, N}, at::kComplexFloat);
+  r.a_last = empty_like_of(x, {B, 1, N}, at::kComplexFloat);
   r.y = empty_like_of(x, x.sizes(), at::kFloat);
   if (T == 1 && !keep_lambda) {   // acting: two launches, no intermediate but the state
     check("lru_step", mxk::layers::lru_step(w, ptr(x), ptr(h0), ptr(a0), bytes(done), ptr(r.h), ptr(r.a_last), ptr(r.y), B, F, N, s));
@@ -77,8 +77,6 @@ Result forward(const Tensor& x, const variable_list& params, const Tensor& h0, c
   return r;
 }
 
-Tensor last_state(const Tensor& h) { return h.narrow(1, h.size(1) - 1, 1); }
-
 struct LruLayer : torch::autograd::Function<LruLayer> {
   static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& nu, const Tensor& theta, const Tensor& gamma,
                                const Tensor& b_re, const Tensor& b_im, const Tensor& c_re, const Tensor& c_im, const Tensor& d,
@@ -90,9 +88,8 @@ struct LruLayer : torch::autograd::Function<LruLayer> {
     variable_list saved{x, nu, theta, gamma, b_re, b_im, c_re, c_im, d, h0, done, r.h, r.lambda};
     ctx->save_for_backward(std::move(saved));
     Tensor last = last_state(r.h).clone();   // (an output may not share memory with what the backward pass reads)
-    Tensor a_last = r.a_last.unsqueeze(1);
-    ctx->mark_non_differentiable({a_last});
-    return {last, a_last, r.y};
+    ctx->mark_non_differentiable({r.a_last});
+    return {last, r.a_last, r.y};
   }
 
   static variable_list backward(AutogradContext* ctx, const variable_list& gout) {
@@ -112,7 +109,7 @@ struct LruLayer : torch::autograd::Function<LruLayer> {
     const Tensor gy = gout[2].defined() ? gout[2].contiguous() : at::zeros_like(x);
 
     Tensor gx = empty_like_of(x, x.sizes(), at::kFloat);
-    Tensor gh0 = need_h0 ? empty_like_of(x, {B, N}, at::kComplexFloat) : Tensor();
+    Tensor gh0 = need_h0 ? empty_like_of(x, {B, 1, N}, at::kComplexFloat) : Tensor();
     Tensor gz = empty_like_of(x, {B, T, N}, at::kComplexFloat);   // cotangent of the states, then of the projected inputs
     Arena mem;
     const size_t img_out = mem.take(g::image_bytes(M, 2 * N, F)), img_in = mem.take(g::image_bytes(M, F, 2 * N));
@@ -168,15 +165,12 @@ struct LruLayer : torch::autograd::Function<LruLayer> {
 // the caller composes from its parts.
 bool native(const Tensor& x, const variable_list& params) {
   if (!x.is_cuda() || x.dim() != 3 || x.numel() == 0 || !x.is_floating_point() || x.scalar_type() == at::kDouble ||
-      at::globalContext().allowTF32CuBLAS() || at::autocast::is_autocast_enabled(at::kCUDA) ||
+      (x.size(1) > 1 && at::globalContext().allowTF32CuBLAS()) || at::autocast::is_autocast_enabled(at::kCUDA) ||
       x.size(0) * x.size(1) > 0x7fffffff || params[3].dim() != 2 || x.size(2) != params[3].size(1))
     return false;
   for (const Tensor& p : params)
     if (p.scalar_type() != at::kFloat || p.device() != x.device() || !p.is_contiguous()) return false;
   return true;
-}
-Tensor carry_leaf(const OptTensor& t, const char* name) {
-  return t && t->defined() ? dev(t->select(1, 0), at::kComplexFloat, name) : Tensor();
 }
 bool wants_grad(const Tensor& x, const variable_list& params, const Tensor& h0) {
   if (!at::GradMode::is_enabled()) return false;
@@ -191,14 +185,14 @@ pybind11::object lru_layer(const Tensor& x_in, const variable_list& params, cons
   if (!native(x_in, params)) return pybind11::none();
   const c10::cuda::CUDAGuard guard(x_in.device());
   const Tensor x = (x_in.scalar_type() == at::kFloat ? x_in : x_in.to(at::kFloat)).contiguous();
-  const Tensor h0 = carry_leaf(h0_in, "h0"), a0 = carry_leaf(a0_in, "a0"), done = done_bytes(done_in);
+  const Tensor h0 = carry_leaf(h0_in, x.size(0) * params[0].size(0), at::kComplexFloat, "h0"), a0 = carry_leaf(a0_in, x.size(0) * params[0].size(0), at::kComplexFloat, "a0"), done = done_bytes(done_in, x.size(0) * x.size(1));
   if (wants_grad(x, params, h0)) {
     const variable_list out = LruLayer::apply(x, params[0], params[1], params[2], params[3], params[4], params[5], params[6],
                                               params[7], opt(h0), opt(a0), opt(done));
     return pybind11::cast(std::make_tuple(out[0], out[1], out[2]));
   }
   const Result r = forward(x, params, h0, a0, done);
-  return pybind11::cast(std::make_tuple(last_state(r.h), r.a_last.unsqueeze(1), r.y));
+  return pybind11::cast(std::make_tuple(last_state(r.h), r.a_last, r.y));
 }
 
 // One RTRL segment without gradients: -> (last state, decay leaf, y, sensitivities of B_imag, B_real, gamma_log, nu_log,
@@ -209,7 +203,7 @@ pybind11::object lru_rtrl(const Tensor& x_in, const variable_list& params, const
   const int B = x_in.size(0), T = x_in.size(1), F = x_in.size(2), N = params[0].size(0);
   const c10::cuda::CUDAGuard guard(x_in.device());
   const Tensor x = (x_in.scalar_type() == at::kFloat ? x_in : x_in.to(at::kFloat)).contiguous();
-  const Tensor h0 = carry_leaf(h0_in, "h0"), a0 = carry_leaf(a0_in, "a0"), done = done_bytes(done_in);
+  const Tensor h0 = carry_leaf(h0_in, x.size(0) * params[0].size(0), at::kComplexFloat, "h0"), a0 = carry_leaf(a0_in, x.size(0) * params[0].size(0), at::kComplexFloat, "a0"), done = done_bytes(done_in, x.size(0) * x.size(1));
   bool grad = wants_grad(x, params, h0);
   variable_list sens, out;
   for (int i = 0; i < 5; ++i) {
@@ -224,7 +218,7 @@ pybind11::object lru_rtrl(const Tensor& x_in, const variable_list& params, const
   mxk::layers::LruSensitivities s{ptr(sens[3]), ptr(sens[4]), ptr(sens[2]), ptr(sens[1]), ptr(sens[0]),
                                   ptr(out[3]), ptr(out[4]), ptr(out[2]), ptr(out[1]), ptr(out[0])};
   check("lru_sensitivities", mxk::layers::lru_sensitivities(weights_of(params), ptr(r.lambda), ptr(r.h), ptr(h0), ptr(x), bytes(done), s, B, T, F, N, stream()));
-  return pybind11::cast(std::make_tuple(last_state(r.h), r.a_last.unsqueeze(1), r.y, out));
+  return pybind11::cast(std::make_tuple(last_state(r.h), r.a_last, r.y, out));
 }
 
 }  // namespace

@@ -100,7 +100,7 @@ struct MambaLayer : torch::autograd::Function<MambaLayer> {
     const Tensor gy = gout[2].defined() ? gout[2].contiguous() : empty_like_of(x, {B, T, out}, at::kFloat).zero_();
     variable_list grads(17);
     if (need_x) grads[0] = empty_like_of(x, x.sizes(), at::kFloat);
-    if (need_h0) grads[13] = empty_like_of(x, {B, H, 16, 16}, at::kFloat);
+    if (need_h0) grads[13] = empty_like_of(x, {B, 1, H, 16, 16}, at::kFloat);
     const Tensor gw_in = empty_like_of(x, {65 * H, F}, at::kFloat), gw_out = empty_like_of(x, {out, hid}, at::kFloat);
     const int scan_cols = l::mamba_partial_floats(H), gate_rows = l::mamba_gate_blocks(M), bias_rows = l::skip_grad_blocks(M);
     const Tensor small = empty_like_of(x, {scan_cols + hid + out}, at::kFloat);
@@ -128,19 +128,18 @@ struct MambaLayer : torch::autograd::Function<MambaLayer> {
     if (need_x) check("run_weights", g::run_weights(mem.at(gproj), ld, mem.at<void>(img_in), ptr(grads[0]), F, M, F, 65 * H, {}, mem.at(ws), ws_bytes, status, s));
     check("run_outer", g::run_outer(mem.at(gproj), ld, ptr(x), F, ptr(gw_in), F, 65 * H, F, M, mem.at(ws), ws_bytes, nullptr, status, s));
     const int channels = 48 * H;
-    const auto piece = [&](int at, at::IntArrayRef sizes) { return small.narrow(0, at, c10::multiply_integers(sizes)).view(sizes); };
-    grads[1 + kConvW] = piece(0, {channels, 1, 4});
-    grads[1 + kConvB] = piece(4 * channels, {channels});
-    grads[1 + kALog] = piece(5 * channels, {H});
-    grads[1 + kDtBias] = piece(5 * channels + H, {H});
-    grads[1 + kD] = piece(5 * channels + 2 * H, {H});
-    grads[1 + kNormW] = piece(scan_cols, {hid});
-    grads[1 + kOutB] = piece(scan_cols + hid, {out});
+    grads[1 + kConvW] = piece(small, 0, {channels, 1, 4});
+    grads[1 + kConvB] = piece(small, 4 * channels, {channels});
+    grads[1 + kALog] = piece(small, 5 * channels, {H});
+    grads[1 + kDtBias] = piece(small, 5 * channels + H, {H});
+    grads[1 + kD] = piece(small, 5 * channels + 2 * H, {H});
+    grads[1 + kNormW] = piece(small, scan_cols, {hid});
+    grads[1 + kOutB] = piece(small, scan_cols + hid, {out});
     grads[1 + kOutW] = gw_out;
-    grads[1 + kIn] = gw_in.narrow(0, 0, 2 * hid);
-    grads[1 + kB] = gw_in.narrow(0, 2 * hid, hid);
-    grads[1 + kC] = gw_in.narrow(0, 3 * hid, hid);
-    grads[1 + kDt] = gw_in.narrow(0, 4 * hid, H);
+    grads[1 + kIn] = piece(gw_in, 0, {2 * hid, F});
+    grads[1 + kB] = piece(gw_in, 2ll * hid * F, {hid, F});
+    grads[1 + kC] = piece(gw_in, 3ll * hid * F, {hid, F});
+    grads[1 + kDt] = piece(gw_in, 4ll * hid * F, {H, F});
     return grads;
   }
 };
@@ -156,9 +155,8 @@ pybind11::object mamba_layer(const Tensor& x_in, const variable_list& p, const O
   if (p[kIn].sizes() != at::IntArrayRef({32 * H, F}) || p[kB].sizes() != at::IntArrayRef({16 * H, F}) || p[kC].sizes() != at::IntArrayRef({16 * H, F}) ||
       p[kDt].sizes() != at::IntArrayRef({H, F}) || p[kConvW].sizes() != at::IntArrayRef({48 * H, 1, 4}) || p[kOutW].size(1) != 16 * H || x_in.size(0) * H > 0x7fffffff)
     return pybind11::none();
-  const auto leaf = [&](const OptTensor& t, const char* name) { return t && t->defined() ? dev(t->select(1, 0), at::kFloat, name) : Tensor(); };
   const c10::cuda::CUDAGuard guard(x_in.device());
-  const Tensor x = x_in.contiguous(), h0 = leaf(h0_in, "h0"), a0 = leaf(a0_in, "a0"), done = done_bytes(done_in);
+  const Tensor x = x_in.contiguous(), h0 = carry_leaf(h0_in, x.size(0) * H * 256, at::kFloat, "h0"), a0 = carry_leaf(a0_in, x.size(0) * H, at::kFloat, "a0"), done = done_bytes(done_in, x.size(0) * x.size(1));
   bool grad = x.requires_grad() || (h0.defined() && h0.requires_grad());
   for (const Tensor& t : p) grad |= t.requires_grad();
   if (at::GradMode::is_enabled() && grad) {

@@ -32,7 +32,7 @@ Result forward(const Tensor& in, const Tensor& w_z, const Tensor& w_h, const Ten
   Result r;
   r.x = empty_like_of(in, {B, T, D}, at::kFloat);
   r.y = empty_like_of(in, {B, T, D}, at::kFloat);
-  r.a_last = empty_like_of(in, {B, D}, at::kFloat);
+  r.a_last = empty_like_of(in, {B, 1, D}, at::kFloat);
   if (T == 1 && !keep) {
     check("mingru_step", mxk::layers::mingru_step(ptr(in), ptr(w_z), ptr(w_h), ptr(x0), ptr(a0), bytes(done), ptr(r.x), ptr(r.y), ptr(r.a_last), B, F, D, stream()));
     return r;
@@ -48,8 +48,6 @@ Result forward(const Tensor& in, const Tensor& w_z, const Tensor& w_h, const Ten
   return r;
 }
 
-Tensor last_state(const Tensor& x) { return x.narrow(1, x.size(1) - 1, 1); }
-
 struct MinGruLayer : torch::autograd::Function<MinGruLayer> {
   static variable_list forward(AutogradContext* ctx, const Tensor& in, const Tensor& w_z, const Tensor& w_h, const OptTensor& x0_in,
                                const OptTensor& a0_in, const OptTensor& done_in) {
@@ -57,9 +55,8 @@ struct MinGruLayer : torch::autograd::Function<MinGruLayer> {
     Result r = mxk_host::forward(in, w_z, w_h, x0, a0, done, true);
     ctx->set_materialize_grads(false);
     ctx->save_for_backward({in, w_z, w_h, x0, done, r.x, r.zh, r.y});
-    const Tensor a_last = r.a_last.unsqueeze(1);
-    ctx->mark_non_differentiable({a_last});
-    return {last_state(r.x).clone(), a_last, r.y};
+    ctx->mark_non_differentiable({r.a_last});
+    return {last_state(r.x).clone(), r.a_last, r.y};
   }
 
   static variable_list backward(AutogradContext* ctx, const variable_list& gout) {
@@ -72,7 +69,7 @@ struct MinGruLayer : torch::autograd::Function<MinGruLayer> {
     const Tensor gx_last = gout[0].defined() ? gout[0].contiguous() : Tensor();
     const Tensor gy = gout[2].defined() ? gout[2].contiguous() : at::zeros_like(x);
     variable_list grads(6);
-    if (need_x0) grads[3] = empty_like_of(in, {B, D}, at::kFloat);
+    if (need_x0) grads[3] = empty_like_of(in, {B, 1, D}, at::kFloat);
     if (need_in) grads[0] = empty_like_of(in, in.sizes(), at::kFloat);
     const Tensor gw = need_w ? empty_like_of(in, {2 * D, F}, at::kFloat) : Tensor();
     Arena mem;
@@ -88,8 +85,8 @@ struct MinGruLayer : torch::autograd::Function<MinGruLayer> {
     }
     if (need_w) {
       check("run_outer", g::run_outer(mem.at(gzh), 2 * D, ptr(in), F, ptr(gw), F, 2 * D, F, M, mem.at(ws), ws_bytes, nullptr, status_ptr(in), stream()));
-      grads[1] = gw.narrow(0, 0, D);
-      grads[2] = gw.narrow(0, D, D);
+      grads[1] = piece(gw, 0, {D, F});
+      grads[2] = piece(gw, static_cast<int64_t>(D) * F, {D, F});
     }
     return grads;
   }
@@ -101,17 +98,16 @@ pybind11::object mingru_layer(const Tensor& in_, const Tensor& w_z, const Tensor
   const auto fits = [&](const Tensor& t) { return t.is_cuda() && t.scalar_type() == at::kFloat && t.device() == in_.device(); };
   if (!fits(in_) || !fits(w_z) || !fits(w_h) || in_.dim() != 3 || in_.numel() == 0 || w_z.dim() != 2 || w_z.sizes() != w_h.sizes() ||
       !w_z.is_contiguous() || !w_h.is_contiguous() || in_.size(2) != w_z.size(1) || in_.size(0) * in_.size(1) > 0x7fffffff ||
-      at::globalContext().allowTF32CuBLAS() || at::autocast::is_autocast_enabled(at::kCUDA))
+      (in_.size(1) > 1 && at::globalContext().allowTF32CuBLAS()) || at::autocast::is_autocast_enabled(at::kCUDA))
     return pybind11::none();
-  const auto leaf = [&](const OptTensor& t, const char* name) { return t && t->defined() ? dev(t->select(1, 0), at::kFloat, name) : Tensor(); };
   const c10::cuda::CUDAGuard guard(in_.device());
-  const Tensor in = in_.contiguous(), x0 = leaf(x0_in, "x0"), a0 = leaf(a0_in, "a0"), done = done_bytes(done_in);
+  const Tensor in = in_.contiguous(), x0 = carry_leaf(x0_in, in.size(0) * w_z.size(0), at::kFloat, "x0"), a0 = carry_leaf(a0_in, in.size(0) * w_z.size(0), at::kFloat, "a0"), done = done_bytes(done_in, in.size(0) * in.size(1));
   if (at::GradMode::is_enabled() && (in.requires_grad() || w_z.requires_grad() || w_h.requires_grad() || (x0.defined() && x0.requires_grad()))) {
     const variable_list out = MinGruLayer::apply(in, w_z, w_h, opt(x0), opt(a0), opt(done));
     return pybind11::cast(std::make_tuple(out[0], out[1], out[2]));
   }
   const Result r = forward(in, w_z, w_h, x0, a0, done, false);
-  return pybind11::cast(std::make_tuple(last_state(r.x), r.a_last.unsqueeze(1), r.y));
+  return pybind11::cast(std::make_tuple(last_state(r.x), r.a_last, r.y));
 }
 
 }  // namespace

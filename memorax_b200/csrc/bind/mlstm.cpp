@@ -27,12 +27,14 @@ Shape shape_of(const Tensor& x, const variable_list& p) {
   s.M = s.B * s.T;
   return s;
 }
+// (H, a, b) -> (H, b, a)
+Tensor swapped(const Tensor& t) { return view_of(t, 0, {t.size(0), t.size(2), t.size(1)}, {t.stride(0), t.stride(2), t.stride(1)}); }
 // columns [at, at + hid) of a (M, n) buffer as per-head matrices (H, M, d)
-Tensor heads(const Tensor& t, int at, const Shape& s) { return t.narrow(1, at, s.hid).view({s.M, s.H, s.d}).permute({1, 0, 2}); }
+Tensor heads(const Tensor& t, int at, const Shape& s) { return view_of(t, at, {s.H, s.M, s.d}, {s.d, t.size(1), 1}); }
 // parts [first, first + count) of q | k | v of every head, out of a buffer (M, H, 3, d): (H, M, count d).  With the head
 // outermost this is the order the gates' weights are in, and q and k are one product.
 Tensor parts(const Tensor& t, int first, int count, const Shape& s) {
-  return t.view({s.M, s.H, 3 * s.d}).narrow(2, first * s.d, count * s.d).permute({1, 0, 2});
+  return view_of(t, first * s.d, {s.H, s.M, count * s.d}, {3 * s.d, t.size(1), 1});
 }
 void* column(const Tensor& t, int c) { return static_cast<uint8_t*>(t.data_ptr()) + 2 * c; }
 
@@ -46,24 +48,24 @@ Result forward(const Tensor& x, const variable_list& p, const Tensor& c0, const 
   Result r;
   const auto bf = at::kBFloat16;
   const auto st = stream();
-  r.c_last = empty_like_of(x, {s.B, s.H, s.d, s.d}, at::kFloat);
-  r.n_last = empty_like_of(x, {s.B, s.H, s.d}, at::kFloat);
-  r.m_last = empty_like_of(x, {s.B, s.H}, at::kFloat);
-  r.f_last = empty_like_of(x, {s.B, s.H}, at::kFloat);
-  r.up = product(x.view({s.M, s.F}), p[kUp].t());
+  r.c_last = empty_like_of(x, {s.B, 1, s.H, s.d, s.d}, at::kFloat);
+  r.n_last = empty_like_of(x, {s.B, 1, s.H, s.d, 1}, at::kFloat);
+  r.m_last = empty_like_of(x, {s.B, 1, s.H, 1, 1}, at::kFloat);
+  r.f_last = empty_like_of(x, {s.B, 1, s.H, 1, 1}, at::kFloat);
+  r.up = product(matrix(x, s.M, s.F), transposed(p[kUp]));
   r.u = empty_like_of(x, {s.M, s.hid}, bf);
   check("mlstm_conv_fwd", l::mlstm_conv_fwd(r.up.data_ptr(), 2 * s.hid, p[kConvW].data_ptr(), p[kConvB].data_ptr(), r.u.data_ptr(), s.B, s.T, s.hid, st));
   r.qkv = empty_like_of(x, {s.M, 3 * s.hid}, bf);
   r.qk_w = at::cat({p[kQ], p[kK]}, 1);   // (H, 2d, d)
-  product_into(heads(r.u, 0, s), r.qk_w.transpose(1, 2), parts(r.qkv, 0, 2, s));
-  product_into(heads(r.up, 0, s), p[kV].transpose(1, 2), parts(r.qkv, 2, 1, s));
+  product_into(heads(r.u, 0, s), swapped(r.qk_w), parts(r.qkv, 0, 2, s));
+  product_into(heads(r.up, 0, s), swapped(p[kV]), parts(r.qkv, 2, 1, s));
   r.gate_w = empty_like_of(x, {2 * s.H, 3 * s.hid}, bf);
   l::WeightRows rows{};
   rows.count = 2;
   rows.ptr[0] = p[kIW].data_ptr(); rows.ptr[1] = p[kFW].data_ptr();
   rows.rows[0] = rows.rows[1] = s.H;
   check("stack_rows", l::stack_rows(rows, r.gate_w.data_ptr(), 2 * s.H, 3 * s.hid, st));
-  r.logits = product(r.qkv, r.gate_w.t(), at::cat({p[kIB], p[kFB]}));
+  r.logits = product(r.qkv, transposed(r.gate_w), at::cat({p[kIB], p[kFB]}));
   r.log_i = empty_like_of(x, {s.M, s.H}, at::kFloat);
   r.log_f = empty_like_of(x, {s.M, s.H}, at::kFloat);
   r.ks = empty_like_of(x, {s.M, s.hid}, bf);
@@ -80,7 +82,8 @@ Result forward(const Tensor& x, const variable_list& p, const Tensor& c0, const 
   r.g = empty_like_of(x, {s.M, s.hid}, bf);
   check("mlstm_out_fwd", l::mlstm_out_fwd(r.h.data_ptr(), r.u.data_ptr(), column(r.up, s.hid), 2 * s.hid, p[kNorm].data_ptr(), p[kSkip].data_ptr(), r.g.data_ptr(), s.M,
                                           s.H, s.d, st));
-  r.y = product(r.g, p[kOut].t()).view({s.B, s.T, p[kOut].size(0)});
+  r.y = empty_like_of(x, {s.B, s.T, p[kOut].size(0)}, bf);
+  product_into(r.g, transposed(p[kOut]), matrix(r.y, s.M, p[kOut].size(0)));
   return r;
 }
 
@@ -116,19 +119,19 @@ struct MlstmLayer : torch::autograd::Function<MlstmLayer> {
     const int64_t out = p[kOut].size(0);
     const auto given = [&](int i) { return gout[i].defined() ? gout[i].contiguous() : Tensor(); };
     const Tensor gc = given(0), gn = given(1), gm = given(2);
-    const Tensor gy = (gout[4].defined() ? gout[4].contiguous() : empty_like_of(x, {s.M, out}, bf).zero_()).view({s.M, out});
+    const Tensor gy = matrix(gout[4].defined() ? gout[4].contiguous() : empty_like_of(x, {s.M, out}, bf).zero_(), s.M, out);
     // inputs of the node: x, the parameters, then what there is of the carry
     variable_list grads(1 + kParams + 6);
     const int first = 1 + kParams;
     const bool need_state = c0.defined() || n0.defined() || m0.defined();
     Tensor gc0, gn0, gm0;
     if (need_state) {
-      gc0 = empty_like_of(x, {s.B, s.H, s.d, s.d}, at::kFloat);
-      gn0 = empty_like_of(x, {s.B, s.H, s.d}, at::kFloat);
-      gm0 = empty_like_of(x, {s.B, s.H}, at::kFloat);
+      gc0 = empty_like_of(x, {s.B, 1, s.H, s.d, s.d}, at::kFloat);
+      gn0 = empty_like_of(x, {s.B, 1, s.H, s.d, 1}, at::kFloat);
+      gm0 = empty_like_of(x, {s.B, 1, s.H, 1, 1}, at::kFloat);
     }
     const Tensor gg = product(gy, p[kOut]);
-    grads[1 + kOut] = product(gy.t(), g);
+    grads[1 + kOut] = product(transposed(gy), g);
     const Tensor gh = empty_like_of(x, {s.M, s.hid}, bf), gu = empty_like_of(x, {s.M, s.hid}, bf), gks = empty_like_of(x, {s.M, s.hid}, bf), gx = empty_like_of(x, {s.M, s.hid}, bf);
     const Tensor gup = empty_like_of(x, {s.M, 2 * s.hid}, bf), gqkv = empty_like_of(x, {s.M, 3 * s.hid}, bf), glogits = empty_like_of(x, {s.M, 2 * s.H}, bf);
     const Tensor gli = empty_like_of(x, {s.M, s.H}, at::kFloat), glf = empty_like_of(x, {s.M, s.H}, at::kFloat);
@@ -147,14 +150,14 @@ struct MlstmLayer : torch::autograd::Function<MlstmLayer> {
     check("mlstm_gates_bwd", l::mlstm_gates_bwd(logits.data_ptr(), ptr(gli), ptr(glf), gks.data_ptr(), s.scale(), column(gqkv, s.d), 3 * s.hid, 3 * s.d,
                                                 glogits.data_ptr(), part_gate, s.M, s.H, s.d, st));
     product_into(glogits, gate_w, gqkv, Tensor(), true);
-    const Tensor ggate = product(glogits.t(), qkv);
-    grads[1 + kIW] = ggate.narrow(0, 0, s.H);
-    grads[1 + kFW] = ggate.narrow(0, s.H, s.H);
+    const Tensor ggate = product(transposed(glogits), qkv);
+    grads[1 + kIW] = piece(ggate, 0, {s.H, 3 * s.hid});
+    grads[1 + kFW] = piece(ggate, 3ll * s.hid * s.H, {s.H, 3 * s.hid});
     const Tensor gqk = parts(gqkv, 0, 2, s), gvalue = parts(gqkv, 2, 1, s);
-    const Tensor gqk_w = product(gqk.transpose(1, 2), heads(u, 0, s));
-    grads[1 + kQ] = gqk_w.narrow(1, 0, s.d);
-    grads[1 + kK] = gqk_w.narrow(1, s.d, s.d);
-    grads[1 + kV] = product(gvalue.transpose(1, 2), heads(up, 0, s));
+    const Tensor gqk_w = product(swapped(gqk), heads(u, 0, s));
+    grads[1 + kQ] = view_of(gqk_w, 0, {s.H, s.d, s.d}, {2 * s.d * s.d, s.d, 1});
+    grads[1 + kK] = view_of(gqk_w, s.d * s.d, {s.H, s.d, s.d}, {2 * s.d * s.d, s.d, 1});
+    grads[1 + kV] = product(swapped(gvalue), heads(up, 0, s));
     product_into(gqk, qk_w, heads(gu, 0, s), Tensor(), true);
     product_into(gvalue, p[kV], heads(gx, 0, s));
     check("mlstm_conv_bwd", l::mlstm_conv_bwd(up.data_ptr(), 2 * s.hid, p[kConvW].data_ptr(), p[kConvB].data_ptr(), gu.data_ptr(), gx.data_ptr(), gup.data_ptr(), part_conv, s.B,
@@ -164,18 +167,21 @@ struct MlstmLayer : torch::autograd::Function<MlstmLayer> {
     check("column_sums", l::column_sums(jobs, 3, st));
     const Tensor small = sums.to(bf);
     int64_t at = 0;
-    const auto piece = [&](int i, int64_t n) {
-      grads[1 + i] = small.narrow(0, at, n).view(p[i].sizes());
+    const auto give = [&](int i, int64_t n) {
+      grads[1 + i] = piece(small, at, p[i].sizes());
       at += n;
     };
-    piece(kNorm, s.hid);
-    piece(kSkip, s.hid);
-    piece(kIB, s.H);
-    piece(kFB, s.H);
-    piece(kConvW, 4 * s.hid);
-    piece(kConvB, s.hid);
-    grads[1 + kUp] = product(gup.t(), x.view({s.M, s.F}));
-    if (ctx->needs_input_grad(0)) grads[0] = product(gup, p[kUp]).view(x.sizes());
+    give(kNorm, s.hid);
+    give(kSkip, s.hid);
+    give(kIB, s.H);
+    give(kFB, s.H);
+    give(kConvW, 4 * s.hid);
+    give(kConvB, s.hid);
+    grads[1 + kUp] = product(transposed(gup), matrix(x, s.M, s.F));
+    if (ctx->needs_input_grad(0)) {
+      grads[0] = empty_like_of(x, x.sizes(), bf);
+      product_into(gup, p[kUp], matrix(grads[0], s.M, s.F));
+    }
     if (c0.defined()) grads[first] = gc0;
     if (n0.defined()) grads[first + 1] = gn0;
     if (m0.defined()) grads[first + 2] = gm0;
@@ -196,12 +202,10 @@ pybind11::object mlstm_layer(const Tensor& x_in, const variable_list& p, const O
       p[kConvW].sizes() != at::IntArrayRef({hid, 1, 4}) || p[kOut].size(1) != hid || x_in.size(0) * H > 0x7fffffff)
     return pybind11::none();
   const c10::cuda::CUDAGuard guard(x_in.device());
-  const auto leaf = [&](const OptTensor& t, at::IntArrayRef sizes, const char* name) {
-    return t && t->defined() ? dev(t->reshape(sizes), at::kFloat, name) : Tensor();
-  };
   const int64_t B = x_in.size(0);
-  const Tensor x = x_in.contiguous(), done = done_bytes(done_in);
-  const Tensor c0 = leaf(c_in, {B, H, d, d}, "c0"), f0 = leaf(f_in, {B, H}, "f0"), n0 = leaf(n_in, {B, H, d}, "n0"), m0 = leaf(m_in, {B, H}, "m0");
+  const Tensor x = x_in.contiguous(), done = done_bytes(done_in, x.size(0) * x.size(1));
+  const Tensor c0 = carry_leaf(c_in, B * hid * d, at::kFloat, "c0"), f0 = carry_leaf(f_in, B * H, at::kFloat, "f0"), n0 = carry_leaf(n_in, B * hid, at::kFloat, "n0"),
+               m0 = carry_leaf(m_in, B * H, at::kFloat, "m0");
   bool grad = x.requires_grad();
   for (const Tensor& t : p) grad |= t.requires_grad();
   for (const Tensor& t : {c0, n0, m0}) grad |= t.defined() && t.requires_grad();
@@ -215,7 +219,7 @@ pybind11::object mlstm_layer(const Tensor& x_in, const variable_list& p, const O
     const Result r = forward(x, p, c0, n0, m0, f0, done, shape_of(x, p), eps, false);
     c = r.c_last; n = r.n_last; m = r.m_last; f = r.f_last; y = r.y;
   }
-  return pybind11::cast(std::make_tuple(c.unsqueeze(1), f.view({B, 1, H, 1, 1}), n.view({B, 1, H, d, 1}), m.view({B, 1, H, 1, 1}), y));
+  return pybind11::cast(std::make_tuple(c, f, n, m, y));
 }
 
 }  // namespace

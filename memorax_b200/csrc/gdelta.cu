@@ -85,6 +85,7 @@ constexpr uint32_t kColS = 0, kColY = 128, kColU = 128, kColQK = 192, kColO = 19
 constexpr int kFwdThreads = 256;
 
 __global__ void __launch_bounds__(kFwdThreads, 2) gdelta_fwd_kernel(const __grid_constant__ FwdParams p) {
+  enter_kernel();
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   FwdSmem& sm = *reinterpret_cast<FwdSmem*>(smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -436,7 +437,7 @@ int forward(const void* q, const void* k, const void* v, long long ld_v, const f
   cudaError_t e = cudaFuncSetAttribute(gdelta_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(sizeof(FwdSmem)));
   if (e != cudaSuccess) return static_cast<int>(e);
-  gdelta_fwd_kernel<<<B * H, kFwdThreads, sizeof(FwdSmem), stream>>>(prm);
+  mxk::launch_kernel(gdelta_fwd_kernel, B * H, kFwdThreads, sizeof(FwdSmem), stream, prm);
   return launch_status();
 }
 

@@ -161,6 +161,7 @@ __device__ __forceinline__ void issue_chunk_loads(BwdSmem& sm, const BwdParams& 
 constexpr int kBwdThreads = 256;
 
 __global__ void __launch_bounds__(kBwdThreads) gdelta_bwd_kernel(const __grid_constant__ BwdParams p) {
+  enter_kernel();
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   BwdSmem& sm = *reinterpret_cast<BwdSmem*>(smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -682,7 +683,7 @@ int backward(const void* q, const void* k, const void* v, const float* alpha, co
   cudaError_t e = cudaFuncSetAttribute(gdelta_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(sizeof(BwdSmem)));
   if (e != cudaSuccess) return static_cast<int>(e);
-  gdelta_bwd_kernel<<<B * H, kBwdThreads, sizeof(BwdSmem), stream>>>(prm);
+  mxk::launch_kernel(gdelta_bwd_kernel, B * H, kBwdThreads, sizeof(BwdSmem), stream, prm);
   return launch_status();
 }
 

@@ -61,6 +61,7 @@ constexpr uint32_t kPrepTmemCols = 32;
 constexpr uint32_t kUpper = 16u << 16;
 
 __global__ void __launch_bounds__(kThreads, 4) gdelta_prep_kernel(const __grid_constant__ PrepParams p) {
+  enter_kernel();
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   PrepSmem& sm = *reinterpret_cast<PrepSmem*>(smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -271,7 +272,7 @@ int launch_prep(const void* k, const float* alpha, const float* beta, const uint
   if (e != cudaSuccess) return static_cast<int>(e);
   const long long items = static_cast<long long>(B) * H * prm.nchunks;
   if (items > 0x7fffffffLL) return MXK_ERR_DIMS;
-  gdelta_prep_kernel<<<static_cast<unsigned>(items), kThreads, sizeof(PrepSmem), stream>>>(prm);
+  mxk::launch_kernel(gdelta_prep_kernel, static_cast<unsigned>(items), kThreads, sizeof(PrepSmem), stream, prm);
   return launch_status();
 }
 

@@ -52,6 +52,7 @@ __device__ __forceinline__ void arrive(uint64_t* bar) {
 
 template <int BN, bool A_ROWS, bool B_ROWS>
 __global__ void __launch_bounds__(kThreads, 1) gemm16_kernel(const __grid_constant__ Params p) {
+  enter_kernel();
   using L = Layout<BN>;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* const full = reinterpret_cast<uint64_t*>(smem + L::kBars);
@@ -207,6 +208,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm16_kernel(const __grid_consta
 __global__ void __launch_bounds__(256) reduce_splits_kernel(const float* __restrict__ partial, int splits, long long all, int M, int N,
                                                             const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ c,
                                                             long long ldc, long long c_batch_stride, bool accumulate) {
+  enter_kernel();
   const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
   if (i >= all) return;
   float s[4] = {0.f, 0.f, 0.f, 0.f};
@@ -257,7 +259,7 @@ template <int BN, bool A_ROWS, bool B_ROWS>
 int launch(const Params& p, cudaStream_t stream) {
   if (const int st = allow_smem<gemm16_kernel<BN, A_ROWS, B_ROWS>>(Layout<BN>::kBytes); st != MXK_OK) return st;
   const long long tiles = static_cast<long long>((p.M + kBM - 1) / kBM) * ((p.N + BN - 1) / BN) * p.batch * p.splits;
-  gemm16_kernel<BN, A_ROWS, B_ROWS><<<static_cast<unsigned>(min(tiles, static_cast<long long>(kNumSMs))), kThreads, Layout<BN>::kBytes, stream>>>(p);
+  mxk::launch_kernel(gemm16_kernel<BN, A_ROWS, B_ROWS>, static_cast<unsigned>(min(tiles, static_cast<long long>(kNumSMs))), kThreads, Layout<BN>::kBytes, stream, p);
   return launch_status();
 }
 template <int BN>
@@ -299,7 +301,7 @@ int run(const Matrix& a, bool a_rows, const Matrix& b, bool b_rows, const void* 
   const int st = pl.bn == 128 ? launch_bn<128>(p, a_rows, b_rows, stream) : launch_bn<64>(p, a_rows, b_rows, stream);
   if (st != MXK_OK || pl.splits == 1) return st;
   const long long all = static_cast<long long>(batch) * M * N;
-  reduce_splits_kernel<<<static_cast<unsigned>((all + 255) / 256), 256, 0, stream>>>(p.partial, pl.splits, all, M, N, p.bias, p.c, ldc,
+  mxk::launch_kernel(reduce_splits_kernel, static_cast<unsigned>((all + 255) / 256), 256, 0, stream, p.partial, pl.splits, all, M, N, p.bias, p.c, ldc,
                                                                                      c_batch_stride, accumulate);
   return launch_status();
 }

@@ -219,6 +219,7 @@ struct Roles {
 
 template <int BN, bool kOuter>
 __global__ void __launch_bounds__(Roles<BN, kOuter>::kThreads, 1) gemm32_kernel(const __grid_constant__ Params p) {
+  enter_kernel();
   using L = Layout<BN>;
   using R = Roles<BN, kOuter>;
   constexpr int kProducerWarps = R::kProducerWarps, kEpilogueWarps = R::kEpilogueWarps, kMmaWarp = R::kMmaWarp;
@@ -430,6 +431,7 @@ __global__ void __launch_bounds__(Roles<BN, kOuter>::kThreads, 1) gemm32_kernel(
 // C = sum over splits of the partial products (fixed order: bit-reproducible) + epilogue
 __global__ void __launch_bounds__(256) reduce_splits_kernel(const float* __restrict__ partial, int splits, int M, int N,
                                                             float* __restrict__ c, long long ldc, Epilogue ep) {
+  enter_kernel();
   const long long n_all = static_cast<long long>(M) * N;
   const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
   if (i >= n_all) return;
@@ -486,7 +488,7 @@ Plan plan(int M, int N, int K) {
 template <int BN, bool kOuter>
 int launch(const Params& p, int tiles, cudaStream_t stream) {
   if (const int st = allow_smem<gemm32_kernel<BN, kOuter>>(Layout<BN>::kBytes); st != MXK_OK) return st;
-  gemm32_kernel<BN, kOuter><<<min(tiles, kNumSMs), Roles<BN, kOuter>::kThreads, Layout<BN>::kBytes, stream>>>(p);
+  mxk::launch_kernel(gemm32_kernel<BN, kOuter>, min(tiles, kNumSMs), Roles<BN, kOuter>::kThreads, Layout<BN>::kBytes, stream, p);
   return launch_status();
 }
 
@@ -508,7 +510,7 @@ int run(Params& p, float* ws, size_t ws_bytes, int* partials, cudaStream_t strea
   if (partials) *partials = pl.splits;
   if (st != MXK_OK || pl.splits == 1 || partials) return st;
   const long long n_all = static_cast<long long>(p.M) * p.N;
-  reduce_splits_kernel<<<static_cast<unsigned>((n_all + 255) / 256), 256, 0, stream>>>(ws, pl.splits, p.M, p.N, p.c, p.ldc, p.ep);
+  mxk::launch_kernel(reduce_splits_kernel, static_cast<unsigned>((n_all + 255) / 256), 256, 0, stream, ws, pl.splits, p.M, p.N, p.c, p.ldc, p.ep);
   return launch_status();
 }
 
@@ -520,6 +522,7 @@ struct SplitParams {
 
 // One thread per eight k of a weight row: reads them (zero past the matrix), writes one vector of each plane.
 __global__ void __launch_bounds__(256) split_weights_kernel(const __grid_constant__ SplitParams sp) {
+  enter_kernel();
   int j = 0;
   while (static_cast<int>(blockIdx.x) >= sp.first_block[j + 1]) ++j;
   if (j == 4) {
@@ -591,7 +594,7 @@ int split_weights(const WeightJob* jobs, int count, const LambdaJob& lambda, cud
   sp.first_block[5] = 0x7fffffff;
   sp.lambda = lambda;
   if (blocks == 0) return MXK_OK;
-  split_weights_kernel<<<blocks, 256, 0, stream>>>(sp);
+  mxk::launch_kernel(split_weights_kernel, blocks, 256, 0, stream, sp);
   return launch_status();
 }
 

@@ -44,6 +44,7 @@ __global__ void __launch_bounds__(kRowWarps * 32)
 norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gamma,
                 const __nv_bfloat16* __restrict__ beta, __nv_bfloat16* __restrict__ y, float* __restrict__ mean,
                 float* __restrict__ rstd, long long rows, int D, float eps) {
+  enter_kernel();
   const float inv_d = 1.f / static_cast<float>(D);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float g[V][8], b[V][8];
@@ -90,6 +91,7 @@ __global__ void __launch_bounds__(kRowWarps * 32)
 norm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gamma, const float* __restrict__ mean,
                 const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ dy, __nv_bfloat16* __restrict__ dx,
                 float* __restrict__ part, long long rows, int D) {
+  enter_kernel();
   const float inv_d = 1.f / static_cast<float>(D);
   __shared__ float red[kRowWarps][V * 256];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -146,6 +148,7 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
 // every eighth partial, then thread row 0 adds the eight sums in order.
 __global__ void __launch_bounds__(256)
 norm_bwd_reduce_kernel(const float* __restrict__ part, float* __restrict__ dgamma, float* __restrict__ dbeta, int blocks, int D) {
+  enter_kernel();
   __shared__ float red[2][8][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + tx;
@@ -173,6 +176,7 @@ norm_bwd_reduce_kernel(const float* __restrict__ part, float* __restrict__ dgamm
 // are added in a fixed order, and the block's sums go to part[ry][col]; the second kernel adds the row blocks in order.
 __global__ void __launch_bounds__(256)
 colsum_partial_kernel(const uint4* __restrict__ x, float* __restrict__ part, long long rows, int cols8, int rows_per_block) {
+  enter_kernel();
   __shared__ float red[8][32][9];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int v = blockIdx.x * 32 + tx;
@@ -218,6 +222,7 @@ colsum_partial_kernel(const uint4* __restrict__ x, float* __restrict__ part, lon
 // A block owns 32 columns; its eight thread rows each add every eighth row block, then thread row 0 adds the eight sums in order.
 __global__ void __launch_bounds__(256)
 colsum_final_kernel(const float* __restrict__ part, __nv_bfloat16* __restrict__ out, int row_blocks, int cols) {
+  enter_kernel();
   __shared__ float red[8][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + tx;
@@ -242,6 +247,7 @@ __device__ __forceinline__ float tanh_fast(float x) {
 }
 __global__ void __launch_bounds__(256)
 gelu_fwd_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, long long n8) {
+  enter_kernel();
   const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
   if (i >= n8) return;
   float f[8];
@@ -257,6 +263,7 @@ gelu_fwd_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, long long n8
 // dx = dy * d/dx gelu(x)
 __global__ void __launch_bounds__(256)
 gelu_bwd_kernel(const uint4* __restrict__ x, const uint4* __restrict__ dy, uint4* __restrict__ dx, long long n8) {
+  enter_kernel();
   const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
   if (i >= n8) return;
   float f[8], g[8];
@@ -276,6 +283,7 @@ gelu_bwd_kernel(const uint4* __restrict__ x, const uint4* __restrict__ dy, uint4
 __global__ void __launch_bounds__(256)
 gated_residual_fwd_kernel(const uint4* __restrict__ x, const uint4* __restrict__ g, const uint4* __restrict__ o,
                           uint4* __restrict__ y, long long n8) {
+  enter_kernel();
   const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
   if (i >= n8) return;
   float xf[8], gf[8], of[8];
@@ -290,6 +298,7 @@ gated_residual_fwd_kernel(const uint4* __restrict__ x, const uint4* __restrict__
 __global__ void __launch_bounds__(256)
 gated_residual_bwd_kernel(const uint4* __restrict__ dy, const uint4* __restrict__ g, const uint4* __restrict__ o,
                           uint4* __restrict__ dg, uint4* __restrict__ d_o, long long n8) {
+  enter_kernel();
   const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
   if (i >= n8) return;
   float yf[8], gf[8], of[8];
@@ -310,6 +319,7 @@ gated_residual_bwd_kernel(const uint4* __restrict__ dy, const uint4* __restrict_
 template <int LPH, bool BWD>
 __global__ void __launch_bounds__(256)
 l2norm_kernel(const uint4* __restrict__ x, const uint4* __restrict__ dy, uint4* __restrict__ out, long long nvec, float eps) {
+  enter_kernel();
   const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
   const bool in = i < nvec;
   float xf[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, df[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -386,10 +396,10 @@ int mxk_colsum_bf16(const void* x, void* out, void* workspace, size_t workspace_
   const int nrb = colsum_row_blocks(rows, cols), cols8 = cols / 8;
   const int rpb = static_cast<int>((rows + nrb - 1) / nrb);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  colsum_partial_kernel<<<dim3((cols8 + 31) / 32, nrb), 256, 0, s>>>(static_cast<const uint4*>(x), static_cast<float*>(workspace),
+  mxk::launch_kernel(colsum_partial_kernel, dim3((cols8 + 31) / 32, nrb), 256, 0, s, static_cast<const uint4*>(x), static_cast<float*>(workspace),
                                                                       rows, cols8, rpb);
   if (int st = launch_status()) return st;
-  colsum_final_kernel<<<(cols + 31) / 32, 256, 0, s>>>(static_cast<const float*>(workspace), static_cast<__nv_bfloat16*>(out), nrb, cols);
+  mxk::launch_kernel(colsum_final_kernel, (cols + 31) / 32, 256, 0, s, static_cast<const float*>(workspace), static_cast<__nv_bfloat16*>(out), nrb, cols);
   return launch_status();
 }
 
@@ -410,8 +420,8 @@ int mxk_norm_bf16_fwd(const void* x, const void* gamma, const void* beta, void* 
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int blocks = norm_blocks(rows, 8), threads = kRowWarps * 32;
 #define MXK_NORM_FWD(V)                                                                                        \
-  if (rms) norm_fwd_kernel<V, true><<<blocks, threads, 0, s>>>(xp, gp, nullptr, yp, nullptr, rstd, rows, D, eps); \
-  else norm_fwd_kernel<V, false><<<blocks, threads, 0, s>>>(xp, gp, bp, yp, mean, rstd, rows, D, eps);
+  if (rms) mxk::launch_kernel(norm_fwd_kernel<V, true>, blocks, threads, 0, s, xp, gp, nullptr, yp, nullptr, rstd, rows, D, eps); \
+  else mxk::launch_kernel(norm_fwd_kernel<V, false>, blocks, threads, 0, s, xp, gp, bp, yp, mean, rstd, rows, D, eps);
   switch ((D + 255) / 256) {
     case 1: MXK_NORM_FWD(1) break;
     case 2: MXK_NORM_FWD(2) break;
@@ -438,8 +448,8 @@ int mxk_norm_bf16_bwd(const void* x, const void* gamma, const float* mean, const
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int blocks = norm_blocks(rows), threads = kRowWarps * 32;
 #define MXK_NORM_BWD(V)                                                                                  \
-  if (rms) norm_bwd_kernel<V, true><<<blocks, threads, 0, s>>>(xp, gp, nullptr, rstd, dyp, dxp, part, rows, D); \
-  else norm_bwd_kernel<V, false><<<blocks, threads, 0, s>>>(xp, gp, mean, rstd, dyp, dxp, part, rows, D);
+  if (rms) mxk::launch_kernel(norm_bwd_kernel<V, true>, blocks, threads, 0, s, xp, gp, nullptr, rstd, dyp, dxp, part, rows, D); \
+  else mxk::launch_kernel(norm_bwd_kernel<V, false>, blocks, threads, 0, s, xp, gp, mean, rstd, dyp, dxp, part, rows, D);
   switch ((D + 255) / 256) {
     case 1: MXK_NORM_BWD(1) break;
     case 2: MXK_NORM_BWD(2) break;
@@ -448,7 +458,7 @@ int mxk_norm_bf16_bwd(const void* x, const void* gamma, const float* mean, const
   }
 #undef MXK_NORM_BWD
   if (int st = launch_status()) return st;
-  norm_bwd_reduce_kernel<<<(D + 31) / 32, 256, 0, s>>>(part, dgamma, rms ? nullptr : dbeta, blocks, D);
+  mxk::launch_kernel(norm_bwd_reduce_kernel, (D + 31) / 32, 256, 0, s, part, dgamma, rms ? nullptr : dbeta, blocks, D);
   return launch_status();
 }
 
@@ -461,8 +471,8 @@ int mxk_gelu_bf16(const void* x, const void* dy, void* out, long long n, mxk_str
   const long long n8 = n / 8;
   const unsigned blocks = static_cast<unsigned>((n8 + 255) / 256);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (dy) gelu_bwd_kernel<<<blocks, 256, 0, s>>>(static_cast<const uint4*>(x), static_cast<const uint4*>(dy), static_cast<uint4*>(out), n8);
-  else gelu_fwd_kernel<<<blocks, 256, 0, s>>>(static_cast<const uint4*>(x), static_cast<uint4*>(out), n8);
+  if (dy) mxk::launch_kernel(gelu_bwd_kernel, blocks, 256, 0, s, static_cast<const uint4*>(x), static_cast<const uint4*>(dy), static_cast<uint4*>(out), n8);
+  else mxk::launch_kernel(gelu_fwd_kernel, blocks, 256, 0, s, static_cast<const uint4*>(x), static_cast<uint4*>(out), n8);
   return launch_status();
 }
 
@@ -473,8 +483,7 @@ int mxk_gated_residual_bf16_fwd(const void* x, const void* g, const void* o, voi
   for (const void* p : {x, g, o, (const void*)y})
     if (!aligned16(p)) return MXK_ERR_ALIGN;
   const long long n8 = n / 8;
-  gated_residual_fwd_kernel<<<static_cast<unsigned>((n8 + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const uint4*>(x), static_cast<const uint4*>(g), static_cast<const uint4*>(o), static_cast<uint4*>(y), n8);
+  mxk::launch_kernel(gated_residual_fwd_kernel, static_cast<unsigned>((n8 + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream), static_cast<const uint4*>(x), static_cast<const uint4*>(g), static_cast<const uint4*>(o), static_cast<uint4*>(y), n8);
   return launch_status();
 }
 
@@ -486,8 +495,7 @@ int mxk_gated_residual_bf16_bwd(const void* dy, const void* g, const void* o, vo
   for (const void* p : {dy, g, o, (const void*)dg, (const void*)d_o})
     if (!aligned16(p)) return MXK_ERR_ALIGN;
   const long long n8 = n / 8;
-  gated_residual_bwd_kernel<<<static_cast<unsigned>((n8 + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const uint4*>(dy), static_cast<const uint4*>(g), static_cast<const uint4*>(o), static_cast<uint4*>(dg),
+  mxk::launch_kernel(gated_residual_bwd_kernel, static_cast<unsigned>((n8 + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream), static_cast<const uint4*>(dy), static_cast<const uint4*>(g), static_cast<const uint4*>(o), static_cast<uint4*>(dg),
       static_cast<uint4*>(d_o), n8);
   return launch_status();
 }
@@ -507,11 +515,11 @@ int mxk_l2norm_heads_bf16(const void* x, const void* dy, void* out, long long ve
   const uint4* dp = static_cast<const uint4*>(dy);
   uint4* op = static_cast<uint4*>(out);
   if (head_dim == 64) {
-    if (dy) l2norm_kernel<8, true><<<blocks, 256, 0, s>>>(xp, dp, op, nvec, eps);
-    else l2norm_kernel<8, false><<<blocks, 256, 0, s>>>(xp, nullptr, op, nvec, eps);
+    if (dy) mxk::launch_kernel(l2norm_kernel<8, true>, blocks, 256, 0, s, xp, dp, op, nvec, eps);
+    else mxk::launch_kernel(l2norm_kernel<8, false>, blocks, 256, 0, s, xp, nullptr, op, nvec, eps);
   } else {
-    if (dy) l2norm_kernel<16, true><<<blocks, 256, 0, s>>>(xp, dp, op, nvec, eps);
-    else l2norm_kernel<16, false><<<blocks, 256, 0, s>>>(xp, nullptr, op, nvec, eps);
+    if (dy) mxk::launch_kernel(l2norm_kernel<16, true>, blocks, 256, 0, s, xp, dp, op, nvec, eps);
+    else mxk::launch_kernel(l2norm_kernel<16, false>, blocks, 256, 0, s, xp, nullptr, op, nvec, eps);
   }
   return launch_status();
 }

@@ -94,6 +94,7 @@ constexpr int kAhead = MXK_LINATTN_AHEAD;
 // kFull: head dimension = the tile width (compile-time bounds); otherwise a multiple of 8 below it.
 template <bool kFull>
 __global__ void __launch_bounds__(kThreads, 4) linattn_fwd_kernel(const __grid_constant__ FwdParams p) {
+  enter_kernel();
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   FwdSmem& sm = *reinterpret_cast<FwdSmem*>(smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -415,7 +416,7 @@ int forward(const void* q, const void* k, const void* v, long long ld, const flo
   auto kernel = d == kD ? linattn_fwd_kernel<true> : linattn_fwd_kernel<false>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(FwdSmem)));
   if (e != cudaSuccess) return static_cast<int>(e);
-  kernel<<<B * H, kThreads, sizeof(FwdSmem), stream>>>(prm);
+  mxk::launch_kernel(kernel, B * H, kThreads, sizeof(FwdSmem), stream, prm);
   return launch_status();
 }
 

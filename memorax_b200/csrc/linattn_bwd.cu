@@ -128,6 +128,7 @@ __device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w 
 // kFull: head dimension = the tile width (compile-time bounds); otherwise a multiple of 8 below it.
 template <bool kFull>
 __global__ void __launch_bounds__(kBwdThreads, 2) linattn_bwd_kernel(const __grid_constant__ BwdParams p) {
+  enter_kernel();
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   BwdSmem& sm = *reinterpret_cast<BwdSmem*>(smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -554,7 +555,7 @@ int backward(const void* q, const void* k, const void* v, long long ld, const vo
   auto kernel = d == kD ? linattn_bwd_kernel<true> : linattn_bwd_kernel<false>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(BwdSmem)));
   if (e != cudaSuccess) return static_cast<int>(e);
-  kernel<<<B * H, kBwdThreads, sizeof(BwdSmem), stream>>>(prm);
+  mxk::launch_kernel(kernel, B * H, kBwdThreads, sizeof(BwdSmem), stream, prm);
   return launch_status();
 }
 

@@ -149,6 +149,7 @@ linrec_fwd_kernel(const float* __restrict__ a, int a_tinv, const float* __restri
                   const float* __restrict__ h0, const float* __restrict__ a0,
                   const uint8_t* __restrict__ done, float* __restrict__ h,
                   float* __restrict__ a_last, int B, int T, int row) {
+  enter_kernel();
   const int per_row = row / W;
   const long long gid = static_cast<long long>(blockIdx.x) * kBlock + threadIdx.x;
   if (gid >= static_cast<long long>(B) * per_row) return;
@@ -222,6 +223,7 @@ linrec_fwd_tsplit_kernel(const float* __restrict__ a, int a_tinv, const float* _
                          const float* __restrict__ h0, const float* __restrict__ a0,
                          const uint8_t* __restrict__ done, float* __restrict__ h, float* __restrict__ a_last,
                          int B, int T, int row) {
+  enter_kernel();
   __shared__ float sp[kSegs][32 * W], sq[kSegs][32 * W], sd[kSegs][32 * W];
   __shared__ int sr[kSegs][32];
   const int cx = threadIdx.x & 31, seg = threadIdx.x >> 5;
@@ -303,6 +305,7 @@ linrec_bwd_tsplit_kernel(const float* __restrict__ a, int a_tinv, const float* _
                          const float* __restrict__ gh, const float* __restrict__ gh_last,
                          float* __restrict__ gb, float* __restrict__ ga, float* __restrict__ ga_partial,
                          float* __restrict__ gh0, int B, int T, int row, int conj_ops) {
+  enter_kernel();
   __shared__ float sp[kSegs][32 * W], sq[kSegs][32 * W];
   const int cx = threadIdx.x & 31, seg = threadIdx.x >> 5;
   const long long ch = (static_cast<long long>(blockIdx.x) * 32 + cx) * W;
@@ -410,6 +413,7 @@ linrec_bwd_kernel(const float* __restrict__ a, int a_tinv, const float* __restri
                   const float* __restrict__ gh, const float* __restrict__ gh_last,
                   float* __restrict__ gb, float* __restrict__ ga, float* __restrict__ ga_partial,
                   float* __restrict__ gh0, int B, int T, int row, int conj_ops) {
+  enter_kernel();
   const int per_row = row / W;
   const long long gid = static_cast<long long>(blockIdx.x) * kBlock + threadIdx.x;
   if (gid >= static_cast<long long>(B) * per_row) return;
@@ -484,6 +488,7 @@ linrec_bwd_kernel(const float* __restrict__ a, int a_tinv, const float* __restri
 // 0 adds the eight partials in order.
 __global__ void __launch_bounds__(kBlock)
 reduce_rows_kernel(const float* __restrict__ partial, float* __restrict__ out, int B, int row) {
+  enter_kernel();
   __shared__ float part[8][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int col = blockIdx.x * 32 + tx;
@@ -508,6 +513,7 @@ loglinrec_fwd_kernel(const float* __restrict__ ls, const float* __restrict__ d,
                      const float* __restrict__ x0, const float* __restrict__ a0,
                      const uint8_t* __restrict__ done, float* __restrict__ x, float* __restrict__ y,
                      float* __restrict__ a_last, int B, int T, int row) {
+  enter_kernel();
   const int per_row = row / W;
   const long long gid = static_cast<long long>(blockIdx.x) * kBlock + threadIdx.x;
   if (gid >= static_cast<long long>(B) * per_row) return;
@@ -574,6 +580,7 @@ loglinrec_bwd_kernel(const float* __restrict__ d, const float* __restrict__ ht, 
                      const float* __restrict__ gx, const float* __restrict__ gy,
                      const float* __restrict__ gx_last, float* __restrict__ gls,
                      float* __restrict__ gd, float* __restrict__ gx0, int B, int T, int row) {
+  enter_kernel();
   const int per_row = row / W;
   const long long gid = static_cast<long long>(blockIdx.x) * kBlock + threadIdx.x;
   if (gid >= static_cast<long long>(B) * per_row) return;
@@ -699,19 +706,19 @@ int linrec_fwd(const float* a, int a_tinv, const float* b, const float* h0, cons
     const unsigned threads = 32 * kSegs;
     if constexpr (CPLX) {
       const unsigned blocks = static_cast<unsigned>((total / 2 + 31) / 32);
-      if (len <= 8) linrec_fwd_tsplit_kernel<true, 8, 2><<<blocks, threads, 0, s>>>(a, a_tinv, b, h0, a0, done, h, a_last, B, T, row);
-      else linrec_fwd_tsplit_kernel<true, 16, 2><<<blocks, threads, 0, s>>>(a, a_tinv, b, h0, a0, done, h, a_last, B, T, row);
+      if (len <= 8) mxk::launch_kernel(linrec_fwd_tsplit_kernel<true, 8, 2>, blocks, threads, 0, s, a, a_tinv, b, h0, a0, done, h, a_last, B, T, row);
+      else mxk::launch_kernel(linrec_fwd_tsplit_kernel<true, 16, 2>, blocks, threads, 0, s, a, a_tinv, b, h0, a0, done, h, a_last, B, T, row);
     } else {
       bool wide = (D % 4 == 0) && len <= 8;   // 16-byte lanes keep 8 steps x (a, b) in registers
       for (const void* ptr : {(const void*)a, (const void*)b, (const void*)h0, (const void*)a0, (const void*)h, (const void*)a_last})
         if (ptr && !aligned16(ptr)) wide = false;
       if (wide) {
         const unsigned blocks = static_cast<unsigned>((total / 4 + 31) / 32);
-        linrec_fwd_tsplit_kernel<false, 8, 4><<<blocks, threads, 0, s>>>(a, a_tinv, b, h0, a0, done, h, a_last, B, T, row);
+        mxk::launch_kernel(linrec_fwd_tsplit_kernel<false, 8, 4>, blocks, threads, 0, s, a, a_tinv, b, h0, a0, done, h, a_last, B, T, row);
       } else {
         const unsigned blocks = static_cast<unsigned>((total + 31) / 32);
-        if (len <= 8) linrec_fwd_tsplit_kernel<false, 8, 1><<<blocks, threads, 0, s>>>(a, a_tinv, b, h0, a0, done, h, a_last, B, T, row);
-        else linrec_fwd_tsplit_kernel<false, 16, 1><<<blocks, threads, 0, s>>>(a, a_tinv, b, h0, a0, done, h, a_last, B, T, row);
+        if (len <= 8) mxk::launch_kernel(linrec_fwd_tsplit_kernel<false, 8, 1>, blocks, threads, 0, s, a, a_tinv, b, h0, a0, done, h, a_last, B, T, row);
+        else mxk::launch_kernel(linrec_fwd_tsplit_kernel<false, 16, 1>, blocks, threads, 0, s, a, a_tinv, b, h0, a0, done, h, a_last, B, T, row);
       }
     }
     return launch_status();
@@ -722,11 +729,11 @@ int linrec_fwd(const float* a, int a_tinv, const float* b, const float* h0, cons
   const unsigned blocks = w == 4 ? blocks_for(total / 4) : blocks_for(total / kN);
   const bool small = blocks <= 3u * kNumSMs;
   if (w == 4) {
-    if (small) linrec_fwd_kernel<CPLX, 4, 2 * MXK_LINREC_UNROLL_F, 2><<<blocks, kBlock, 0, s>>>(a, a_tinv, b, h0, a0, done, h, a_last, B, T, row);
-    else linrec_fwd_kernel<CPLX, 4><<<blocks, kBlock, 0, s>>>(a, a_tinv, b, h0, a0, done, h, a_last, B, T, row);
+    if (small) mxk::launch_kernel(linrec_fwd_kernel<CPLX, 4, 2 * MXK_LINREC_UNROLL_F, 2>, blocks, kBlock, 0, s, a, a_tinv, b, h0, a0, done, h, a_last, B, T, row);
+    else mxk::launch_kernel(linrec_fwd_kernel<CPLX, 4>, blocks, kBlock, 0, s, a, a_tinv, b, h0, a0, done, h, a_last, B, T, row);
   } else {
-    if (small) linrec_fwd_kernel<CPLX, kN, 4 * MXK_LINREC_UNROLL_F, 2><<<blocks, kBlock, 0, s>>>(a, a_tinv, b, h0, a0, done, h, a_last, B, T, row);
-    else linrec_fwd_kernel<CPLX, kN><<<blocks, kBlock, 0, s>>>(a, a_tinv, b, h0, a0, done, h, a_last, B, T, row);
+    if (small) mxk::launch_kernel(linrec_fwd_kernel<CPLX, kN, 4 * MXK_LINREC_UNROLL_F, 2>, blocks, kBlock, 0, s, a, a_tinv, b, h0, a0, done, h, a_last, B, T, row);
+    else mxk::launch_kernel(linrec_fwd_kernel<CPLX, kN>, blocks, kBlock, 0, s, a, a_tinv, b, h0, a0, done, h, a_last, B, T, row);
   }
   return launch_status();
 }
@@ -747,11 +754,9 @@ int linrec_last(const float* a, int a_tinv, const float* b, const float* h0, con
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   constexpr int kN = CPLX ? 2 : 1;
   if (w == 4)
-    linrec_fwd_kernel<CPLX, 4, 2 * MXK_LINREC_UNROLL_F, 2, true><<<blocks_for(total / 4), kBlock, 0, s>>>(
-        a, a_tinv, b, h0, nullptr, done, h_last, nullptr, B, T, row);
+    mxk::launch_kernel(linrec_fwd_kernel<CPLX, 4, 2 * MXK_LINREC_UNROLL_F, 2, true>, blocks_for(total / 4), kBlock, 0, s, a, a_tinv, b, h0, nullptr, done, h_last, nullptr, B, T, row);
   else
-    linrec_fwd_kernel<CPLX, kN, 4 * MXK_LINREC_UNROLL_F, 2, true><<<blocks_for(total / kN), kBlock, 0, s>>>(
-        a, a_tinv, b, h0, nullptr, done, h_last, nullptr, B, T, row);
+    mxk::launch_kernel(linrec_fwd_kernel<CPLX, kN, 4 * MXK_LINREC_UNROLL_F, 2, true>, blocks_for(total / kN), kBlock, 0, s, a, a_tinv, b, h0, nullptr, done, h_last, nullptr, B, T, row);
   return launch_status();
 }
 
@@ -781,24 +786,24 @@ int linrec_bwd(const float* a, int a_tinv, const float* h, const float* h0, cons
     constexpr int kW = CPLX ? 2 : 1;
     const unsigned blocks = static_cast<unsigned>((total / kW + 31) / 32), threads = 32 * kSegs;
     if ((T + kSegs - 1) / kSegs <= 8)
-      linrec_bwd_tsplit_kernel<CPLX, 8, kW><<<blocks, threads, 0, s>>>(a, a_tinv, h, h0, done, gh, gh_last, gb, ga_full, partial, gh0, B, T, row, conj_ops);
+      mxk::launch_kernel(linrec_bwd_tsplit_kernel<CPLX, 8, kW>, blocks, threads, 0, s, a, a_tinv, h, h0, done, gh, gh_last, gb, ga_full, partial, gh0, B, T, row, conj_ops);
     else
-      linrec_bwd_tsplit_kernel<CPLX, 16, kW><<<blocks, threads, 0, s>>>(a, a_tinv, h, h0, done, gh, gh_last, gb, ga_full, partial, gh0, B, T, row, conj_ops);
+      mxk::launch_kernel(linrec_bwd_tsplit_kernel<CPLX, 16, kW>, blocks, threads, 0, s, a, a_tinv, h, h0, done, gh, gh_last, gb, ga_full, partial, gh0, B, T, row, conj_ops);
   } else {
     constexpr int kN = CPLX ? 2 : 1;
     const unsigned blocks = w == 4 ? blocks_for(total / 4) : blocks_for(total / kN);
     const bool small = blocks <= 3u * kNumSMs;   // see linrec_fwd
     if (w == 4) {
-      if (small) linrec_bwd_kernel<CPLX, 4, 2 * MXK_LINREC_UNROLL_B, 2><<<blocks, kBlock, 0, s>>>(a, a_tinv, h, h0, done, gh, gh_last, gb, ga_full, partial, gh0, B, T, row, conj_ops);
-      else linrec_bwd_kernel<CPLX, 4><<<blocks, kBlock, 0, s>>>(a, a_tinv, h, h0, done, gh, gh_last, gb, ga_full, partial, gh0, B, T, row, conj_ops);
+      if (small) mxk::launch_kernel(linrec_bwd_kernel<CPLX, 4, 2 * MXK_LINREC_UNROLL_B, 2>, blocks, kBlock, 0, s, a, a_tinv, h, h0, done, gh, gh_last, gb, ga_full, partial, gh0, B, T, row, conj_ops);
+      else mxk::launch_kernel(linrec_bwd_kernel<CPLX, 4>, blocks, kBlock, 0, s, a, a_tinv, h, h0, done, gh, gh_last, gb, ga_full, partial, gh0, B, T, row, conj_ops);
     } else {
-      if (small) linrec_bwd_kernel<CPLX, kN, 4 * MXK_LINREC_UNROLL_B, 2><<<blocks, kBlock, 0, s>>>(a, a_tinv, h, h0, done, gh, gh_last, gb, ga_full, partial, gh0, B, T, row, conj_ops);
-      else linrec_bwd_kernel<CPLX, kN><<<blocks, kBlock, 0, s>>>(a, a_tinv, h, h0, done, gh, gh_last, gb, ga_full, partial, gh0, B, T, row, conj_ops);
+      if (small) mxk::launch_kernel(linrec_bwd_kernel<CPLX, kN, 4 * MXK_LINREC_UNROLL_B, 2>, blocks, kBlock, 0, s, a, a_tinv, h, h0, done, gh, gh_last, gb, ga_full, partial, gh0, B, T, row, conj_ops);
+      else mxk::launch_kernel(linrec_bwd_kernel<CPLX, kN>, blocks, kBlock, 0, s, a, a_tinv, h, h0, done, gh, gh_last, gb, ga_full, partial, gh0, B, T, row, conj_ops);
     }
   }
   if (int st = launch_status()) return st;
   if (partial) {
-    reduce_rows_kernel<<<(row + 31) / 32, kBlock, 0, s>>>(partial, ga, B, row);
+    mxk::launch_kernel(reduce_rows_kernel, (row + 31) / 32, kBlock, 0, s, partial, ga, B, row);
     return launch_status();
   }
   return MXK_OK;
@@ -914,9 +919,9 @@ int mxk_loglinrec_f32_fwd(const float* ls, const float* d, const float* x0, cons
   const int w = pick_width(total, D, false, {ls, d, x0, a0, x, y, a_last});
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (w == 4)
-    loglinrec_fwd_kernel<4, false><<<blocks_for(total / 4), kBlock, 0, s>>>(ls, d, x0, a0, done, x, y, a_last, B, T, D);
+    mxk::launch_kernel(loglinrec_fwd_kernel<4, false>, blocks_for(total / 4), kBlock, 0, s, ls, d, x0, a0, done, x, y, a_last, B, T, D);
   else
-    loglinrec_fwd_kernel<1, false><<<blocks_for(total), kBlock, 0, s>>>(ls, d, x0, a0, done, x, y, a_last, B, T, D);
+    mxk::launch_kernel(loglinrec_fwd_kernel<1, false>, blocks_for(total), kBlock, 0, s, ls, d, x0, a0, done, x, y, a_last, B, T, D);
   return launch_status();
 }
 
@@ -932,9 +937,9 @@ int mxk_mingru_f32_fwd(const float* z, const float* h_tilde, const float* x0, co
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (!mingru_walks(B, D)) return layers::mingru_fwd(z, h_tilde, nullptr, nullptr, nullptr, 0, D, x0, a0, done, x, y, a_last, B, T, D, s);
   if (w == 4)
-    loglinrec_fwd_kernel<4, true><<<blocks_for(total / 4), kBlock, 0, s>>>(z, h_tilde, x0, a0, done, x, y, a_last, B, T, D);
+    mxk::launch_kernel(loglinrec_fwd_kernel<4, true>, blocks_for(total / 4), kBlock, 0, s, z, h_tilde, x0, a0, done, x, y, a_last, B, T, D);
   else
-    loglinrec_fwd_kernel<1, true><<<blocks_for(total), kBlock, 0, s>>>(z, h_tilde, x0, a0, done, x, y, a_last, B, T, D);
+    mxk::launch_kernel(loglinrec_fwd_kernel<1, true>, blocks_for(total), kBlock, 0, s, z, h_tilde, x0, a0, done, x, y, a_last, B, T, D);
   return launch_status();
 }
 
@@ -951,9 +956,9 @@ int mxk_loglinrec_f32_bwd(const float* d, const float* x, const float* x0, const
   const int w = pick_width(total, D, false, {d, x, x0, gx, gy, gx_last, gls, gd, gx0});
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (w == 4)
-    loglinrec_bwd_kernel<4, false><<<blocks_for(total / 4), kBlock, 0, s>>>(d, nullptr, x, x0, done, gx, gy, gx_last, gls, gd, gx0, B, T, D);
+    mxk::launch_kernel(loglinrec_bwd_kernel<4, false>, blocks_for(total / 4), kBlock, 0, s, d, nullptr, x, x0, done, gx, gy, gx_last, gls, gd, gx0, B, T, D);
   else
-    loglinrec_bwd_kernel<1, false><<<blocks_for(total), kBlock, 0, s>>>(d, nullptr, x, x0, done, gx, gy, gx_last, gls, gd, gx0, B, T, D);
+    mxk::launch_kernel(loglinrec_bwd_kernel<1, false>, blocks_for(total), kBlock, 0, s, d, nullptr, x, x0, done, gx, gy, gx_last, gls, gd, gx0, B, T, D);
   return launch_status();
 }
 
@@ -971,9 +976,9 @@ int mxk_mingru_f32_bwd(const float* z, const float* h_tilde, const float* x, con
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (!mingru_walks(B, D)) return layers::mingru_bwd(z, h_tilde, D, x, nullptr, x0, done, gx, gy, gx_last, gz, gh, gx0, B, T, D, s);
   if (w == 4)
-    loglinrec_bwd_kernel<4, true><<<blocks_for(total / 4), kBlock, 0, s>>>(z, h_tilde, x, x0, done, gx, gy, gx_last, gz, gh, gx0, B, T, D);
+    mxk::launch_kernel(loglinrec_bwd_kernel<4, true>, blocks_for(total / 4), kBlock, 0, s, z, h_tilde, x, x0, done, gx, gy, gx_last, gz, gh, gx0, B, T, D);
   else
-    loglinrec_bwd_kernel<1, true><<<blocks_for(total), kBlock, 0, s>>>(z, h_tilde, x, x0, done, gx, gy, gx_last, gz, gh, gx0, B, T, D);
+    mxk::launch_kernel(loglinrec_bwd_kernel<1, true>, blocks_for(total), kBlock, 0, s, z, h_tilde, x, x0, done, gx, gy, gx_last, gz, gh, gx0, B, T, D);
   return launch_status();
 }
 

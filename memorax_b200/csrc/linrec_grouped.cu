@@ -27,6 +27,7 @@ __global__ void __launch_bounds__(kBlockG, kMinBlocks)
 linrec_grouped_fwd_kernel(const float* __restrict__ a, const float* __restrict__ b, const float* __restrict__ h0,
                           const float* __restrict__ a0, const uint8_t* __restrict__ done, float* __restrict__ h,
                           float* __restrict__ a_last, int B, int T, int D, int G, int group) {
+  enter_kernel();
   const int per_row = D / 4;
   const long long gid = static_cast<long long>(blockIdx.x) * kBlockG + threadIdx.x;
   if (gid >= static_cast<long long>(B) * per_row) return;
@@ -82,6 +83,7 @@ linrec_grouped_bwd_kernel(const float* __restrict__ a, const float* __restrict__
                           const uint8_t* __restrict__ done, const float* __restrict__ gh,
                           const float* __restrict__ gh_last, float* __restrict__ gb, float* __restrict__ ga_part,
                           float* __restrict__ gh0, int B, int T, int D, int G, int group) {
+  enter_kernel();
   const int per_row = D / 4;
   const long long gid = static_cast<long long>(blockIdx.x) * kBlockG + threadIdx.x;
   if (gid >= static_cast<long long>(B) * per_row) return;   // D % 128 == 0: whole warps leave together
@@ -143,6 +145,7 @@ linrec_grouped_bwd_kernel(const float* __restrict__ a, const float* __restrict__
 // ga[i] = sum of the wpg partials of (b, t, group) i, in index order.
 __global__ void __launch_bounds__(kBlockG)
 sum_group_partials_kernel(const float* __restrict__ part, float* __restrict__ ga, long long n, int wpg) {
+  enter_kernel();
   const long long i = static_cast<long long>(blockIdx.x) * kBlockG + threadIdx.x;
   if (i >= n) return;
   float s = part[i * wpg];
@@ -181,9 +184,9 @@ int mxk_linrec_f32_grouped_fwd(const float* a, const float* b, const float* h0, 
   const unsigned blocks = static_cast<unsigned>((threads + kBlockG - 1) / kBlockG);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (blocks <= 3u * kNumSMs)
-    linrec_grouped_fwd_kernel<8, 2><<<blocks, kBlockG, 0, s>>>(a, b, h0, a0, done, h, a_last, B, T, D, G, D / G);
+    mxk::launch_kernel(linrec_grouped_fwd_kernel<8, 2>, blocks, kBlockG, 0, s, a, b, h0, a0, done, h, a_last, B, T, D, G, D / G);
   else
-    linrec_grouped_fwd_kernel<4, 4><<<blocks, kBlockG, 0, s>>>(a, b, h0, a0, done, h, a_last, B, T, D, G, D / G);
+    mxk::launch_kernel(linrec_grouped_fwd_kernel<4, 4>, blocks, kBlockG, 0, s, a, b, h0, a0, done, h, a_last, B, T, D, G, D / G);
   return launch_status();
 }
 
@@ -197,8 +200,7 @@ int mxk_linrec_f32_grouped_last(const float* a, const float* b, const float* h0,
   if (reinterpret_cast<uintptr_t>(a) & 3u) return MXK_ERR_ALIGN;
   const long long threads = static_cast<long long>(B) * (D / 4);
   const unsigned blocks = static_cast<unsigned>((threads + kBlockG - 1) / kBlockG);
-  linrec_grouped_fwd_kernel<8, 2, true><<<blocks, kBlockG, 0, static_cast<cudaStream_t>(stream)>>>(
-      a, b, h0, nullptr, done, h_last, nullptr, B, T, D, G, D / G);
+  mxk::launch_kernel(linrec_grouped_fwd_kernel<8, 2, true>, blocks, kBlockG, 0, static_cast<cudaStream_t>(stream), a, b, h0, nullptr, done, h_last, nullptr, B, T, D, G, D / G);
   return launch_status();
 }
 
@@ -222,13 +224,13 @@ int mxk_linrec_f32_grouped_bwd(const float* a, const float* h, const float* h0, 
   const long long threads = static_cast<long long>(B) * (D / 4);
   const unsigned blocks = static_cast<unsigned>((threads + kBlockG - 1) / kBlockG);
   if (blocks <= 3u * kNumSMs)
-    linrec_grouped_bwd_kernel<8, 2><<<blocks, kBlockG, 0, s>>>(a, h, h0, done, gh, gh_last, gb, part, gh0, B, T, D, G, D / G);
+    mxk::launch_kernel(linrec_grouped_bwd_kernel<8, 2>, blocks, kBlockG, 0, s, a, h, h0, done, gh, gh_last, gb, part, gh0, B, T, D, G, D / G);
   else
-    linrec_grouped_bwd_kernel<4, 4><<<blocks, kBlockG, 0, s>>>(a, h, h0, done, gh, gh_last, gb, part, gh0, B, T, D, G, D / G);
+    mxk::launch_kernel(linrec_grouped_bwd_kernel<4, 4>, blocks, kBlockG, 0, s, a, h, h0, done, gh, gh_last, gb, part, gh0, B, T, D, G, D / G);
   if (int st = launch_status()) return st;
   if (ga && wpg > 1) {
     const long long n = static_cast<long long>(B) * T * G;
-    sum_group_partials_kernel<<<static_cast<unsigned>((n + kBlockG - 1) / kBlockG), kBlockG, 0, s>>>(part, ga, n, wpg);
+    mxk::launch_kernel(sum_group_partials_kernel, static_cast<unsigned>((n + kBlockG - 1) / kBlockG), kBlockG, 0, s, part, ga, n, wpg);
     return launch_status();
   }
   return MXK_OK;

@@ -16,6 +16,7 @@ __global__ void __launch_bounds__(128) lru_step_state_kernel(LruWeights w, const
                                                              const float* __restrict__ h0, const float* __restrict__ a0,
                                                              const uint8_t* __restrict__ done, float* __restrict__ h,
                                                              float* __restrict__ a_last, int B, int F, int N) {
+  enter_kernel();
   const int lane = threadIdx.x & 31, warp = blockIdx.x * 4 + (threadIdx.x >> 5);
   const int units = (N + 1) / 2;
   const int n0 = (warp % units) * 2, m0 = (warp / units) * 8;
@@ -49,6 +50,7 @@ __global__ void __launch_bounds__(128) lru_step_state_kernel(LruWeights w, const
 __global__ void __launch_bounds__(128) lru_step_read_kernel(LruWeights w, const float* __restrict__ x,
                                                             const float* __restrict__ h, float* __restrict__ y, int B,
                                                             int F, int N) {
+  enter_kernel();
   const int lane = threadIdx.x & 31, warp = blockIdx.x * 4 + (threadIdx.x >> 5);
   const int units = (F + 3) / 4;
   const int f0 = (warp % units) * 4, m0 = (warp / units) * 8;
@@ -84,6 +86,7 @@ constexpr int kSkipBlocks = 2 * kNumSMs;
 // HBM-bound: one read of both operands; a block takes every gridDim.x-th group of rows, its threads the columns.
 __global__ void __launch_bounds__(256) skip_grad_kernel(const float* __restrict__ gy, const float* __restrict__ x,
                                                         float* __restrict__ partial, long long rows, int F) {
+  enter_kernel();
   __shared__ float sums[256];
   const int per = F < 256 ? 256 / F : 1;   // rows side by side in a block
   const int width = min(F, 256);
@@ -120,6 +123,7 @@ __global__ void __launch_bounds__(256) skip_grad_kernel(const float* __restrict_
 // Blocks 0..N-1: hidden unit n (its rows of the input projection, and lambda); N..N+F-1: feature f (its row of the
 // read-out and its skip weight).  Sums over splits run in a fixed order.
 __global__ void __launch_bounds__(128) lru_param_grads_kernel(LruWeights w, LruGrads g, int F, int N) {
+  enter_kernel();
   __shared__ float red[128];
   const int tid = threadIdx.x;
   const auto block_sum = [&](float v) {
@@ -220,6 +224,7 @@ __device__ __forceinline__ float2 cmul_add(float2 a, float2 b, float2 c) {
 __global__ void __launch_bounds__(128) lru_sens_units_kernel(LruWeights w, const float* __restrict__ lambda,
                                                              const float* __restrict__ h, const float* __restrict__ h0,
                                                              const uint8_t* __restrict__ done, LruSensitivities s, int T, int N) {
+  enter_kernel();
   const int b = blockIdx.y, n = blockIdx.x * 128 + threadIdx.x;
   const int r = last_reset(done ? done + static_cast<size_t>(b) * T : nullptr, T);
   if (n >= N) return;
@@ -257,6 +262,7 @@ constexpr int kSensUnits = 8, kSensSteps = 64, kSensFeatures = 128;
 __global__ void __launch_bounds__(256) lru_sens_inputs_kernel(LruWeights w, const float* __restrict__ lambda,
                                                               const float* __restrict__ u, const uint8_t* __restrict__ done,
                                                               LruSensitivities s, int T, int F, int N) {
+  enter_kernel();
   __shared__ __align__(16) float us[kSensSteps][kSensFeatures];
   __shared__ float2 pw[kSensUnits][kSensSteps + 1];
   const int b = blockIdx.z, n0 = blockIdx.x * kSensUnits, f0 = blockIdx.y * kSensFeatures;
@@ -326,6 +332,7 @@ struct ColumnSums {
 };
 // 32 columns per block; 32 groups of rows (few rows per thread: latency-bound), added in order
 __global__ void __launch_bounds__(1024) column_sums_kernel(const __grid_constant__ ColumnSums p) {
+  enter_kernel();
   __shared__ float part[32][33];
   int j = 0;
   while (static_cast<int>(blockIdx.x) >= p.first_block[j + 1]) ++j;
@@ -356,7 +363,7 @@ int column_sums(const ColumnSum* jobs, int count, cudaStream_t stream) {
     p.first_block[j + 1] = p.first_block[j] + (jobs[j].cols + 31) / 32;
   }
   for (int j = count; j < 4; ++j) p.first_block[j + 1] = 0x7fffffff;
-  column_sums_kernel<<<p.first_block[count], 1024, 0, stream>>>(p);
+  mxk::launch_kernel(column_sums_kernel, p.first_block[count], 1024, 0, stream, p);
   return launch_status();
 }
 
@@ -365,29 +372,29 @@ int lru_step(const LruWeights& w, const float* x, const float* h0, const float* 
   if (B <= 0 || F <= 0 || N <= 0) return MXK_ERR_DIMS;
   const long long groups = (B + 7) / 8;
   const long long warps_h = groups * ((N + 1) / 2), warps_y = groups * ((F + 3) / 4);
-  lru_step_state_kernel<<<static_cast<unsigned>((warps_h + 3) / 4), 128, 0, stream>>>(w, x, h0, a0, done, h, a_last, B, F, N);
-  lru_step_read_kernel<<<static_cast<unsigned>((warps_y + 3) / 4), 128, 0, stream>>>(w, x, h, y, B, F, N);
+  mxk::launch_kernel(lru_step_state_kernel, static_cast<unsigned>((warps_h + 3) / 4), 128, 0, stream, w, x, h0, a0, done, h, a_last, B, F, N);
+  mxk::launch_kernel(lru_step_read_kernel, static_cast<unsigned>((warps_y + 3) / 4), 128, 0, stream, w, x, h, y, B, F, N);
   return launch_status();
 }
 
 int skip_grad_blocks(long long rows) { return static_cast<int>(rows < kSkipBlocks ? rows : kSkipBlocks); }
 
 int skip_grad(const float* gy, const float* x, float* partial, long long rows, int F, cudaStream_t stream) {
-  skip_grad_kernel<<<skip_grad_blocks(rows), 256, 0, stream>>>(gy, x, partial, rows, F);
+  mxk::launch_kernel(skip_grad_kernel, skip_grad_blocks(rows), 256, 0, stream, gy, x, partial, rows, F);
   return launch_status();
 }
 
 int lru_param_grads(const LruWeights& w, const LruGrads& g, int F, int N, cudaStream_t stream) {
-  lru_param_grads_kernel<<<N + F, 128, 0, stream>>>(w, g, F, N);
+  mxk::launch_kernel(lru_param_grads_kernel, N + F, 128, 0, stream, w, g, F, N);
   return launch_status();
 }
 
 int lru_sensitivities(const LruWeights& w, const float* lambda, const float* h, const float* h0, const float* u,
                       const uint8_t* done, const LruSensitivities& s, int B, int T, int F, int N, cudaStream_t stream) {
   if (B <= 0 || T <= 0 || F <= 0 || N <= 0 || B > 65535) return MXK_ERR_DIMS;
-  lru_sens_units_kernel<<<dim3((N + 127) / 128, B), 128, 0, stream>>>(w, lambda, h, h0, done, s, T, N);
+  mxk::launch_kernel(lru_sens_units_kernel, dim3((N + 127) / 128, B), 128, 0, stream, w, lambda, h, h0, done, s, T, N);
   const dim3 grid((N + kSensUnits - 1) / kSensUnits, (F + kSensFeatures - 1) / kSensFeatures, B);
-  lru_sens_inputs_kernel<<<grid, 256, 0, stream>>>(w, lambda, u, done, s, T, F, N);
+  mxk::launch_kernel(lru_sens_inputs_kernel, grid, 256, 0, stream, w, lambda, u, done, s, T, F, N);
   return launch_status();
 }
 

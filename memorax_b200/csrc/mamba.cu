@@ -101,6 +101,7 @@ __global__ void __launch_bounds__(128) mamba_scan_fwd_kernel(MambaParams w, cons
                                                              const uint8_t* __restrict__ done, float* __restrict__ y_pre,
                                                              float* __restrict__ h_last, float* __restrict__ a_last,
                                                              float* __restrict__ states, int T, int H) {
+  enter_kernel();
   __shared__ __align__(16) FwdSmem sm;
   const int tid = threadIdx.x, lane = tid & 31, q = tid >> 5;
   const int b = blockIdx.x / H, h = blockIdx.x % H, hid = H * 16;
@@ -210,6 +211,7 @@ __global__ void __launch_bounds__(384, 2) mamba_scan_bwd_kernel(MambaParams w, c
                                                                 const float* __restrict__ gy_pre,
                                                                 const float* __restrict__ gh_last, float* __restrict__ gproj,
                                                                 float* __restrict__ gh0, float* __restrict__ partial, int T, int H) {
+  enter_kernel();
   extern __shared__ __align__(16) uint8_t raw_smem[];
   BwdSmem& sm = *reinterpret_cast<BwdSmem*>(raw_smem);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -436,6 +438,7 @@ constexpr int kGateBlocks = 4 * kNumSMs;
 __global__ void __launch_bounds__(256) mamba_gate_fwd_kernel(MambaParams w, const float* __restrict__ proj, long long ld,
                                                              const float* __restrict__ y_pre, float* __restrict__ z,
                                                              long long tokens, int hid) {
+  enter_kernel();
   const int lane = threadIdx.x & 31;
   const long long tok = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
   if (tok >= tokens) return;
@@ -455,6 +458,7 @@ __global__ void __launch_bounds__(256) mamba_gate_bwd_kernel(MambaParams w, cons
                                                              const float* __restrict__ y_pre, const float* __restrict__ gz,
                                                              float* __restrict__ gy_pre, float* __restrict__ gproj,
                                                              float* __restrict__ norm_partial, long long tokens, int hid) {
+  enter_kernel();
   extern __shared__ float acc[];   // [8 warps][hid]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int i = threadIdx.x; i < 8 * hid; i += 256) acc[i] = 0.f;
@@ -503,7 +507,7 @@ int mamba_gate_blocks(long long tokens) {
 int mamba_scan_fwd(const MambaParams& w, const float* proj, long long ld, const float* h0, const float* a0, const uint8_t* done,
                    float* y_pre, float* h_last, float* a_last, float* states, int B, int T, int H, cudaStream_t stream) {
   if (B <= 0 || T <= 0 || H <= 0) return MXK_ERR_DIMS;
-  mamba_scan_fwd_kernel<<<B * H, 128, 0, stream>>>(w, proj, ld, h0, a0, done, y_pre, h_last, a_last, states, T, H);
+  mxk::launch_kernel(mamba_scan_fwd_kernel, B * H, 128, 0, stream, w, proj, ld, h0, a0, done, y_pre, h_last, a_last, states, T, H);
   return launch_status();
 }
 
@@ -512,14 +516,14 @@ int mamba_scan_bwd(const MambaParams& w, const float* proj, long long ld, const 
                    float* partial, int B, int T, int H, cudaStream_t stream) {
   if (B <= 0 || T <= 0 || H <= 0) return MXK_ERR_DIMS;
   if (const int st = allow_smem<mamba_scan_bwd_kernel>(sizeof(BwdSmem)); st != MXK_OK) return st;
-  mamba_scan_bwd_kernel<<<B * H, 384, sizeof(BwdSmem), stream>>>(w, proj, ld, done, states, gy_pre, gh_last, gproj, gh0, partial,
+  mxk::launch_kernel(mamba_scan_bwd_kernel, B * H, 384, sizeof(BwdSmem), stream, w, proj, ld, done, states, gy_pre, gh_last, gproj, gh0, partial,
                                                                  T, H);
   return launch_status();
 }
 
 int mamba_gate_fwd(const MambaParams& w, const float* proj, long long ld, const float* y_pre, float* z, long long tokens, int H,
                    cudaStream_t stream) {
-  mamba_gate_fwd_kernel<<<static_cast<unsigned>((tokens + 7) / 8), 256, 0, stream>>>(w, proj, ld, y_pre, z, tokens, 16 * H);
+  mxk::launch_kernel(mamba_gate_fwd_kernel, static_cast<unsigned>((tokens + 7) / 8), 256, 0, stream, w, proj, ld, y_pre, z, tokens, 16 * H);
   return launch_status();
 }
 
@@ -528,7 +532,7 @@ int mamba_gate_bwd(const MambaParams& w, const float* proj, long long ld, const 
   const int hid = 16 * H, bytes = 8 * hid * static_cast<int>(sizeof(float));
   if (bytes > 48 * 1024)
     if (const int st = allow_smem<mamba_gate_bwd_kernel>(bytes); st != MXK_OK) return st;
-  mamba_gate_bwd_kernel<<<mamba_gate_blocks(tokens), 256, bytes, stream>>>(w, proj, ld, y_pre, gz, gy_pre, gproj, norm_partial, tokens, hid);
+  mxk::launch_kernel(mamba_gate_bwd_kernel, mamba_gate_blocks(tokens), 256, bytes, stream, w, proj, ld, y_pre, gz, gy_pre, gproj, norm_partial, tokens, hid);
   return launch_status();
 }
 

@@ -69,6 +69,7 @@ mingru_fwd_kernel(const float* __restrict__ z, const float* ht, float* ht_kink, 
                   const float* __restrict__ dense_w, int F, long long ld, const float* __restrict__ x0,
                   const float* __restrict__ a0, const uint8_t* __restrict__ done, float* __restrict__ x, float* __restrict__ y,
                   float* __restrict__ a_last, int B, int T, int D, int turn_len) {
+  enter_kernel();
   __shared__ float sa[kSegs][32], sq[kSegs][32], sd[kSegs][32];
   __shared__ unsigned sr[kSegs];   // reset bits of a stretch
   __shared__ float carry_x[32], carry_a[32];
@@ -212,6 +213,7 @@ mingru_bwd_kernel(const float* __restrict__ z, const float* __restrict__ ht, lon
                   const float* __restrict__ y, const float* __restrict__ x0, const uint8_t* __restrict__ done,
                   const float* __restrict__ gx, const float* __restrict__ gy, const float* __restrict__ gx_last,
                   float* __restrict__ gz, float* __restrict__ gh, float* __restrict__ gx0, int B, int T, int D, int turn_len) {
+  enter_kernel();
   __shared__ float sp[kSegs][32], sq[kSegs][32];
   __shared__ float carry[32];
   const int lane = threadIdx.x & 31, seg = threadIdx.x >> 5;
@@ -335,6 +337,7 @@ __global__ void __launch_bounds__(128)
 mingru_step_kernel(const float* __restrict__ in, const float* __restrict__ w_z, const float* __restrict__ w_h,
                    const float* __restrict__ x0, const float* __restrict__ a0, const uint8_t* __restrict__ done,
                    float* __restrict__ x, float* __restrict__ y, float* __restrict__ a_last, int B, int F, int D) {
+  enter_kernel();
   const int lane = threadIdx.x & 31, warp = blockIdx.x * 4 + (threadIdx.x >> 5);
   const int units = (D + 1) / 2;
   const int d0 = (warp % units) * 2, m0 = (warp / units) * 8;
@@ -368,7 +371,7 @@ int mingru_fwd(const float* z, const float* h_tilde, float* h_kink, const float*
                long long ld, const float* x0, const float* a0, const uint8_t* done,
                float* x, float* y, float* a_last, int B, int T, int D, cudaStream_t stream) {
   if (const int st = check_dims(B, T, D)) return st;
-  mingru_fwd_kernel<<<blocks_of(B, D), 32 * kSegs, 0, stream>>>(z, h_tilde, h_kink, dense_in, dense_w, F, ld, x0,
+  mxk::launch_kernel(mingru_fwd_kernel, blocks_of(B, D), 32 * kSegs, 0, stream, z, h_tilde, h_kink, dense_in, dense_w, F, ld, x0,
                                                                 a0, done, x, y, a_last, B, T, D, turn_length(T));
   return launch_status();
 }
@@ -377,7 +380,7 @@ int mingru_bwd(const float* z, const float* h_tilde, long long ld, const float* 
                const float* gx, const float* gy, const float* gx_last, float* gz, float* gh, float* gx0, int B, int T, int D,
                cudaStream_t stream) {
   if (const int st = check_dims(B, T, D)) return st;
-  mingru_bwd_kernel<<<blocks_of(B, D), 32 * kSegs, 0, stream>>>(z, h_tilde, ld, x, y, x0, done, gx, gy, gx_last, gz, gh, gx0,
+  mxk::launch_kernel(mingru_bwd_kernel, blocks_of(B, D), 32 * kSegs, 0, stream, z, h_tilde, ld, x, y, x0, done, gx, gy, gx_last, gz, gh, gx0,
                                                                 B, T, D, turn_length(T));
   return launch_status();
 }
@@ -386,7 +389,7 @@ int mingru_step(const float* in, const float* w_z, const float* w_h, const float
                 float* x, float* y, float* a_last, int B, int F, int D, cudaStream_t stream) {
   if (B <= 0 || F <= 0 || D <= 0) return MXK_ERR_DIMS;
   const long long warps = static_cast<long long>((B + 7) / 8) * ((D + 1) / 2);
-  mingru_step_kernel<<<static_cast<unsigned>((warps + 3) / 4), 128, 0, stream>>>(in, w_z, w_h, x0, a0, done, x, y, a_last, B, F, D);
+  mxk::launch_kernel(mingru_step_kernel, static_cast<unsigned>((warps + 3) / 4), 128, 0, stream, in, w_z, w_h, x0, a0, done, x, y, a_last, B, F, D);
   return launch_status();
 }
 

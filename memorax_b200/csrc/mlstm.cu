@@ -119,6 +119,7 @@ __device__ __forceinline__ void gate_step(bool reset, float li, float lf, float&
 // lanes per column): the kernel is bound by instruction throughput at low occupancy, not by per-step latency.
 template <int D, int SPLIT>
 __global__ void __launch_bounds__(D * SPLIT) mlstm_fwd_kernel(const MlstmParams p) {
+  enter_kernel();
   constexpr int L = D / SPLIT, NT = D * SPLIT, NW = NT / 32;
   __shared__ __align__(16) float rows[3][kTS][D];
   __shared__ float sli[kTS], slf[kTS];
@@ -184,6 +185,7 @@ __global__ void __launch_bounds__(D * SPLIT) mlstm_fwd_kernel(const MlstmParams 
 // ----------------------------------------------------------------- backward
 template <int D, int SPLIT>
 __global__ void __launch_bounds__(D * SPLIT) mlstm_bwd_kernel(const MlstmParams p) {
+  enter_kernel();
   constexpr int L = D / SPLIT, NT = D * SPLIT, NW = NT / 32;
   __shared__ __align__(16) float rows[4][kTS][D];      // q, k, v, dh of the staged steps
   __shared__ float sli[kTS], slf[kTS];
@@ -386,7 +388,7 @@ __global__ void __launch_bounds__(D * SPLIT) mlstm_bwd_kernel(const MlstmParams 
 
 template <typename K>
 int launch(K kernel, const MlstmParams& p, int threads, mxk_stream_t stream) {
-  kernel<<<p.B * p.H, threads, 0, static_cast<cudaStream_t>(stream)>>>(p);
+  mxk::launch_kernel(kernel, p.B * p.H, threads, 0, static_cast<cudaStream_t>(stream), p);
   return launch_status();
 }
 

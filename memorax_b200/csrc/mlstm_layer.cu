@@ -44,6 +44,7 @@ template <int kRun>   // tokens per thread
 __global__ void __launch_bounds__(256) conv_fwd_kernel(const bf16* __restrict__ up, long long ld, const bf16* __restrict__ conv_w,
                                                        const bf16* __restrict__ conv_b, bf16* __restrict__ u, int B, int T, int hid,
                                                        int runs) {
+  enter_kernel();
   const int groups = hid / 8;
   const long long id = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
   const int c = static_cast<int>(id % groups) * 8;
@@ -96,6 +97,7 @@ __global__ void __launch_bounds__(256) conv_bwd_kernel(const bf16* __restrict__ 
                                                        const bf16* __restrict__ conv_b, const bf16* __restrict__ gu,
                                                        const bf16* __restrict__ gx, bf16* __restrict__ gup,
                                                        float* __restrict__ partial, int B, int T, int hid, int runs, int lanes) {
+  enter_kernel();
   extern __shared__ float red[];   // [channel][taps + bias] sums of the block's runs, one run group at a time
   const int groups = hid / 8;
   // a block: `lanes` channel groups (a divisor of both 256 and groups) x 256 / lanes runs
@@ -208,6 +210,7 @@ __global__ void __launch_bounds__(256) conv_bwd_kernel(const bf16* __restrict__ 
 __global__ void __launch_bounds__(256) gates_fwd_kernel(const bf16* __restrict__ logits, const bf16* __restrict__ k, long long ld,
                                                         float scale, float* __restrict__ log_i, float* __restrict__ log_f,
                                                         bf16* __restrict__ ks, long long tokens, int H, int hid8, int hp, unsigned vec_blocks) {
+  enter_kernel();
   if (blockIdx.x < vec_blocks) {
     const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
     const long long tok = i / hid8;
@@ -236,6 +239,7 @@ __global__ void __launch_bounds__(256) gates_bwd_kernel(const bf16* __restrict__
                                                         const bf16* __restrict__ gks, float scale, bf16* __restrict__ gk, long long ld,
                                                         bf16* __restrict__ glogits, float* __restrict__ partial, long long tokens,
                                                         int H, int hid8, int hp, unsigned vec_blocks) {
+  enter_kernel();
   __shared__ float red[256];
   if (blockIdx.x < vec_blocks) {
     const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
@@ -283,6 +287,7 @@ template <int LPH>
 __global__ void __launch_bounds__(256) out_fwd_kernel(const bf16* __restrict__ h, const bf16* __restrict__ u, const bf16* __restrict__ z,
                                                       long long ld, const bf16* __restrict__ norm_w, const bf16* __restrict__ skip,
                                                       bf16* __restrict__ g, long long tokens, int hid8) {
+  enter_kernel();
   const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
   const long long tok = i / hid8;
   const int c = static_cast<int>(i % hid8) * 8;
@@ -314,6 +319,7 @@ __global__ void __launch_bounds__(256) out_bwd_kernel(const bf16* __restrict__ g
                                                       const bf16* __restrict__ skip, bf16* __restrict__ gh, bf16* __restrict__ gz,
                                                       long long ld_gz, bf16* __restrict__ gu, float* __restrict__ partial,
                                                       long long tokens, int hid8) {
+  enter_kernel();
   __shared__ float red[256 * 16];
   const int per = 256 / hid8;
   const int c = (threadIdx.x % hid8) * 8, ro = threadIdx.x / hid8;
@@ -400,8 +406,7 @@ int mlstm_conv_fwd(const void* up, long long ld, const void* conv_w, const void*
   const int run = run_of(B, T, hid), runs = runs_of(T, run);
   const long long threads = static_cast<long long>(B) * runs * (hid / 8);
   const auto go = [&](auto kernel) {
-    kernel<<<static_cast<unsigned>((threads + 255) / 256), 256, 0, stream>>>(
-        static_cast<const bf16*>(up), ld, static_cast<const bf16*>(conv_w), static_cast<const bf16*>(conv_b), static_cast<bf16*>(u), B, T, hid, runs);
+    mxk::launch_kernel(kernel, static_cast<unsigned>((threads + 255) / 256), 256, 0, stream, static_cast<const bf16*>(up), ld, static_cast<const bf16*>(conv_w), static_cast<const bf16*>(conv_b), static_cast<bf16*>(u), B, T, hid, runs);
     return launch_status();
   };
   return run == 16 ? go(conv_fwd_kernel<16>) : go(conv_fwd_kernel<4>);
@@ -417,8 +422,7 @@ int mlstm_conv_bwd(const void* up, long long ld, const void* conv_w, const void*
   const int lanes = conv_lanes(hid), bytes = lanes * 8 * (kTaps + 1) * static_cast<int>(sizeof(float));
   const int run = run_of(B, T, hid), runs = runs_of(T, run);
   const auto go = [&](auto kernel) {
-    kernel<<<dim3(mlstm_conv_blocks(B, T, hid), hid / 8 / lanes), 256, bytes, stream>>>(
-        static_cast<const bf16*>(up), ld, static_cast<const bf16*>(conv_w), static_cast<const bf16*>(conv_b), static_cast<const bf16*>(gu),
+    mxk::launch_kernel(kernel, dim3(mlstm_conv_blocks(B, T, hid), hid / 8 / lanes), 256, bytes, stream, static_cast<const bf16*>(up), ld, static_cast<const bf16*>(conv_w), static_cast<const bf16*>(conv_b), static_cast<const bf16*>(gu),
         static_cast<const bf16*>(gx), static_cast<bf16*>(gup), partial, B, T, hid, runs, lanes);
     return launch_status();
   };
@@ -429,7 +433,7 @@ int mlstm_gates_fwd(const void* logits, const void* k, long long ld, int hp, flo
                     float* log_i, float* log_f, void* k_scaled, long long tokens, int H, int d, cudaStream_t stream) {
   const int hid8 = H * d / 8;
   const unsigned vb = static_cast<unsigned>((tokens * hid8 + 255) / 256), gb = static_cast<unsigned>((tokens * H + 255) / 256);
-  gates_fwd_kernel<<<vb + gb, 256, 0, stream>>>(static_cast<const bf16*>(logits), static_cast<const bf16*>(k), ld, scale, log_i, log_f, static_cast<bf16*>(k_scaled), tokens, H, hid8, hp, vb);
+  mxk::launch_kernel(gates_fwd_kernel, vb + gb, 256, 0, stream, static_cast<const bf16*>(logits), static_cast<const bf16*>(k), ld, scale, log_i, log_f, static_cast<bf16*>(k_scaled), tokens, H, hid8, hp, vb);
   return launch_status();
 }
 
@@ -444,7 +448,7 @@ int mlstm_gates_bwd(const void* logits, const float* glog_i, const float* glog_f
   if (H > 128) return MXK_ERR_UNSUPPORTED;
   const int hid8 = H * d / 8;
   const unsigned vb = static_cast<unsigned>((tokens * hid8 + 255) / 256), gb = static_cast<unsigned>(mlstm_gate_blocks(tokens));
-  gates_bwd_kernel<<<vb + gb, 256, 0, stream>>>(static_cast<const bf16*>(logits), glog_i, glog_f,
+  mxk::launch_kernel(gates_bwd_kernel, vb + gb, 256, 0, stream, static_cast<const bf16*>(logits), glog_i, glog_f,
                                                 static_cast<const bf16*>(gk_scaled), scale, static_cast<bf16*>(gk), ld, static_cast<bf16*>(glogits),
                                                 partial, tokens, H, hid8, hp, vb);
   return launch_status();
@@ -455,7 +459,7 @@ int mlstm_out_fwd(const void* h, const void* u, const void* z, long long ld, con
   const int hid8 = H * d / 8;
   const unsigned blocks = static_cast<unsigned>((tokens * hid8 + 255) / 256);
   const auto go = [&](auto kernel) {
-    kernel<<<blocks, 256, 0, stream>>>(static_cast<const bf16*>(h), static_cast<const bf16*>(u), static_cast<const bf16*>(z), ld,
+    mxk::launch_kernel(kernel, blocks, 256, 0, stream, static_cast<const bf16*>(h), static_cast<const bf16*>(u), static_cast<const bf16*>(z), ld,
                                        static_cast<const bf16*>(norm_w), static_cast<const bf16*>(skip), static_cast<bf16*>(g), tokens, hid8);
     return launch_status();
   };
@@ -472,8 +476,7 @@ int mlstm_out_bwd(const void* gg, const void* h, const void* u, const void* z, l
   const int hid8 = H * d / 8;
   if (hid8 > 256 || 256 % hid8) return MXK_ERR_UNSUPPORTED;
   const auto go = [&](auto kernel) {
-    kernel<<<mlstm_out_blocks(tokens, hid8 * 8), 256, 0, stream>>>(
-        static_cast<const bf16*>(gg), static_cast<const bf16*>(h), static_cast<const bf16*>(u), static_cast<const bf16*>(z), ld,
+    mxk::launch_kernel(kernel, mlstm_out_blocks(tokens, hid8 * 8), 256, 0, stream, static_cast<const bf16*>(gg), static_cast<const bf16*>(h), static_cast<const bf16*>(u), static_cast<const bf16*>(z), ld,
         static_cast<const bf16*>(norm_w), static_cast<const bf16*>(skip), static_cast<bf16*>(gh), static_cast<bf16*>(gz), ld_gz,
         static_cast<bf16*>(gu), partial, tokens, hid8);
     return launch_status();

@@ -79,6 +79,7 @@ constexpr uint32_t kTmemCols = 128;
 constexpr uint32_t kUpper = 16u << 16;
 
 __global__ void __launch_bounds__(kThreads, 4) mlstm_tc_fwd_kernel(const __grid_constant__ FwdParams p) {
+  enter_kernel();
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   FwdSmem& sm = *reinterpret_cast<FwdSmem*>(smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -369,7 +370,7 @@ int forward(const void* q, const void* k, const void* v, long long ld_qv, long l
   cudaError_t e = cudaFuncSetAttribute(mlstm_tc_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(sizeof(FwdSmem)));
   if (e != cudaSuccess) return static_cast<int>(e);
-  mlstm_tc_fwd_kernel<<<B * H, kThreads, sizeof(FwdSmem), stream>>>(prm);
+  mxk::launch_kernel(mlstm_tc_fwd_kernel, B * H, kThreads, sizeof(FwdSmem), stream, prm);
   return launch_status();
 }
 

@@ -190,6 +190,7 @@ __device__ __forceinline__ void chunk_gate_grads(const ChunkGates& g, const Gate
 }
 
 __global__ void __launch_bounds__(kBwdThreads, 2) mlstm_tc_bwd_kernel(const __grid_constant__ BwdParams p) {
+  enter_kernel();
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   BwdSmem& sm = *reinterpret_cast<BwdSmem*>(smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -709,7 +710,7 @@ int backward(const void* q, const void* k, const void* v, long long ld_qv, long 
   cudaError_t e = cudaFuncSetAttribute(mlstm_tc_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(sizeof(BwdSmem)));
   if (e != cudaSuccess) return static_cast<int>(e);
-  mlstm_tc_bwd_kernel<<<B * H, kBwdThreads, sizeof(BwdSmem), stream>>>(prm);
+  mxk::launch_kernel(mlstm_tc_bwd_kernel, B * H, kBwdThreads, sizeof(BwdSmem), stream, prm);
   return launch_status();
 }
 

@@ -34,6 +34,32 @@ inline int allow_smem(int bytes) {
   return MXK_OK;
 }
 
+// Kernel launch that may be set up while the kernel in front of it still runs (programmatic dependent launch: 0.7-1 us
+// less between two small kernels).  Every kernel of this library begins with enter_kernel(), which waits for the kernels in
+// front before anything is read or written, so the order of effects on a stream is the usual one.
+template <typename... P, typename... A>
+inline int launch_kernel(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  return launch_status();
+}
+
+// First statement of every kernel, executed by all threads.  A grid of at most two blocks per SM lets its successor's
+// blocks take their places at once; a larger one would have them pile up on the SMs that empty first.
+__device__ __forceinline__ void enter_kernel() {
+  if (gridDim.x * gridDim.y * gridDim.z <= 2u * kNumSMs) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // 16-byte streaming accesses: data that is touched once should not displace
 // reusable lines (the carried state, chunk tiles) from L1/L2.
 __device__ __forceinline__ float4 ld_stream(const float4* p) { return __ldcs(p); }
