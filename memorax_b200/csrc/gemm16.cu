@@ -52,7 +52,7 @@ __device__ __forceinline__ void arrive(uint64_t* bar) {
 
 template <int BN, bool A_ROWS, bool B_ROWS>
 __global__ void __launch_bounds__(kThreads, 1) gemm16_kernel(const __grid_constant__ Params p) {
-  enter_kernel();
+  enter_kernel(((p.M + kBM - 1) / kBM) * ((p.N + BN - 1) / BN) * p.batch * p.splits <= static_cast<int>(gridDim.x));
   using L = Layout<BN>;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* const full = reinterpret_cast<uint64_t*>(smem + L::kBars);

@@ -219,7 +219,7 @@ struct Roles {
 
 template <int BN, bool kOuter>
 __global__ void __launch_bounds__(Roles<BN, kOuter>::kThreads, 1) gemm32_kernel(const __grid_constant__ Params p) {
-  enter_kernel();
+  enter_kernel(((p.M + kBM - 1) / kBM) * ((p.N + BN - 1) / BN) * p.splits <= static_cast<int>(gridDim.x) && p.k_split <= 2 * kSegment);
   using L = Layout<BN>;
   using R = Roles<BN, kOuter>;
   constexpr int kProducerWarps = R::kProducerWarps, kEpilogueWarps = R::kEpilogueWarps, kMmaWarp = R::kMmaWarp;

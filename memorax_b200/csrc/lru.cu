@@ -12,20 +12,23 @@ namespace {
 // depth of the memory pipeline are what counts, so every warp computes eight sequences x four outputs with its lanes
 // across the contraction (the 12 loads of an iteration are independent), and nothing but the state makes a round trip
 // through memory between the two launches.  (16 sequences, F = 128, N = 256: 25 launches, 250 us on the host -> 2.)
+template <int kSplit>
 __global__ void __launch_bounds__(128) lru_step_state_kernel(LruWeights w, const float* __restrict__ x,
                                                              const float* __restrict__ h0, const float* __restrict__ a0,
                                                              const uint8_t* __restrict__ done, float* __restrict__ h,
                                                              float* __restrict__ a_last, int B, int F, int N) {
   enter_kernel();
-  const int lane = threadIdx.x & 31, warp = blockIdx.x * 4 + (threadIdx.x >> 5);
+  const TilePlace<kSplit> at_tile;
+  const int lane = at_tile.lane;
   const int units = (N + 1) / 2;
-  const int n0 = (warp % units) * 2, m0 = (warp / units) * 8;
+  const int n0 = (at_tile.tile % units) * 2, m0 = (at_tile.tile / units) * 8;
   if (m0 >= B) return;
   WarpTile acc;
   const float* rows[4] = {w.b_re + static_cast<size_t>(n0) * F, w.b_im + static_cast<size_t>(n0) * F,
                           w.b_re + static_cast<size_t>(min(n0 + 1, N - 1)) * F, w.b_im + static_cast<size_t>(min(n0 + 1, N - 1)) * F};
-  acc.accumulate(x + static_cast<size_t>(m0) * F, F, min(8, B - m0), rows, F, lane);
-  const float v = acc.reduce(lane);
+  acc.accumulate(x + static_cast<size_t>(m0) * F, F, min(8, B - m0), rows, F, at_tile.first, at_tile.step);
+  float v = acc.reduce(lane);
+  if (!join_warps<kSplit>(v, lane)) return;
   // this lane: sequence m, component j & 1 of unit n
   const int m = m0 + (lane >> 2), n = n0 + ((lane >> 1) & 1), im = lane & 1;
   if (m >= B || n >= N) return;
@@ -47,17 +50,20 @@ __global__ void __launch_bounds__(128) lru_step_state_kernel(LruWeights w, const
   }
 }
 
+template <int kSplit>
 __global__ void __launch_bounds__(128) lru_step_read_kernel(LruWeights w, const float* __restrict__ x,
                                                             const float* __restrict__ h, float* __restrict__ y, int B,
                                                             int F, int N) {
   enter_kernel();
-  const int lane = threadIdx.x & 31, warp = blockIdx.x * 4 + (threadIdx.x >> 5);
+  const TilePlace<kSplit> at_tile;
+  const int lane = at_tile.lane;
   const int units = (F + 3) / 4;
-  const int f0 = (warp % units) * 4, m0 = (warp / units) * 8;
+  const int f0 = (at_tile.tile % units) * 4, m0 = (at_tile.tile / units) * 8;
   if (m0 >= B) return;
   const int mv = min(8, B - m0);
   WarpTile acc;
-  for (int n = lane; n < N; n += 32) {
+#pragma unroll 2
+  for (int n = at_tile.first; n < N; n += at_tile.step) {
     float2 hv[8];
     float cr[4], ci[4];
 #pragma unroll
@@ -74,7 +80,8 @@ __global__ void __launch_bounds__(128) lru_step_read_kernel(LruWeights w, const 
 #pragma unroll
       for (int j = 0; j < 4; ++j) acc.v[i * 4 + j] = fmaf(hv[i].x, cr[j], fmaf(-hv[i].y, ci[j], acc.v[i * 4 + j]));
   }
-  const float v = acc.reduce(lane);
+  float v = acc.reduce(lane);
+  if (!join_warps<kSplit>(v, lane)) return;
   const int m = m0 + (lane >> 2), f = f0 + (lane & 3);
   if (m >= B || f >= F) return;
   const size_t at = static_cast<size_t>(m) * F + f;
@@ -220,32 +227,39 @@ __device__ __forceinline__ float2 cmul_add(float2 a, float2 b, float2 c) {
   return make_float2(fmaf(a.x, b.x, fmaf(-a.y, b.y, c.x)), fmaf(a.x, b.y, fmaf(a.y, b.x, c.y)));
 }
 
-// nu, theta, gamma: one thread per (sequence, unit); latency-bound, so eight states are in flight per thread.
-__global__ void __launch_bounds__(128) lru_sens_units_kernel(LruWeights w, const float* __restrict__ lambda,
-                                                             const float* __restrict__ h, const float* __restrict__ h0,
-                                                             const uint8_t* __restrict__ done, LruSensitivities s, int T, int N) {
-  enter_kernel();
-  const int b = blockIdx.y, n = blockIdx.x * 128 + threadIdx.x;
-  const int r = last_reset(done ? done + static_cast<size_t>(b) * T : nullptr, T);
-  if (n >= N) return;
-  const float2* hs = reinterpret_cast<const float2*>(h) + static_cast<size_t>(b) * T * N + n;
-  const size_t at = static_cast<size_t>(b) * N + n;
-  const float2 l = reinterpret_cast<const float2*>(lambda)[n];
-  const float2 start = h0 ? reinterpret_cast<const float2*>(h0)[at] : make_float2(0.f, 0.f);
-  // R_t = lambda R_{t-1} + lambda h_{t-1} from step r + 1 on (R = 0 at a reset), or from the carried state
+// nu, theta, gamma of 32 units: with s0 the first step after the last reset (0 without one, and then the carried state is
+// "step -1"), the sum over s >= s0 of lambda^(T-1-s) h_s is cut into eight stretches of time, one per warp, each by Horner's
+// rule with eight states in flight (one thread per unit walking all of T was a chain of L2 round trips: 20 us at T = 64).
+__device__ __forceinline__ void unit_sensitivities(const LruWeights& w, const float* __restrict__ lambda, const float* __restrict__ h,
+                                                   const float* __restrict__ h0, const LruSensitivities& s, int b, int n0, int r,
+                                                   int T, int N) {
+  __shared__ float2 part[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n = n0 + lane;
+  const bool in = n < N;
+  const size_t at = static_cast<size_t>(b) * N + (in ? n : 0);
+  const float2 l = reinterpret_cast<const float2*>(lambda)[in ? n : 0];
+  const float2* hs = reinterpret_cast<const float2*>(h) + static_cast<size_t>(b) * T * N + (in ? n : 0);
+  const int s0 = max(r, 0), len = (T - 1 - s0 + 7) / 8;
+  const int from = min(T - 1, s0 + warp * len), to = min(T - 1, from + len);
   float2 acc = make_float2(0.f, 0.f);
-  if (r < 0) acc = cmul(l, start);
   constexpr int kDeep = 8;
-  for (int t0 = r < 0 ? 1 : r + 1; t0 < T; t0 += kDeep) {
-    float2 prev[kDeep];
+  for (int t = from; t < to; t += kDeep) {
+    float2 v[kDeep];
 #pragma unroll
     for (int u = 0; u < kDeep; ++u)
-      if (t0 + u < T) prev[u] = __ldg(hs + static_cast<size_t>(t0 + u - 1) * N);
+      if (t + u < to) v[u] = __ldg(hs + static_cast<size_t>(t + u) * N);
 #pragma unroll
     for (int u = 0; u < kDeep; ++u)
-      if (t0 + u < T) acc = cmul(l, make_float2(acc.x + prev[u].x, acc.y + prev[u].y));
+      if (t + u < to) acc = cmul(l, make_float2(acc.x + v[u].x, acc.y + v[u].y));
   }
+  part[warp][lane] = cmul(power(l, T - 1 - to), acc);
+  __syncthreads();
+  if (warp > 0 || !in) return;
+  const float2 start = h0 ? reinterpret_cast<const float2*>(h0)[at] : make_float2(0.f, 0.f);
   const float2 p = r < 0 ? power(l, T) : make_float2(0.f, 0.f);
+  acc = cmul(p, start);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) { acc.x += part[i][lane].x; acc.y += part[i][lane].y; }
   const float en = expf(w.nu_log[n]), et = expf(w.theta_log[n]);
   const auto old = [&](const float* q) { return reinterpret_cast<const float2*>(q)[at]; };
   const float2 last = hs[static_cast<size_t>(T - 1) * N], g0 = old(s.gamma);
@@ -254,74 +268,89 @@ __global__ void __launch_bounds__(128) lru_sens_units_kernel(LruWeights w, const
   reinterpret_cast<float2*>(s.gamma_out)[at] = cmul_add(p, make_float2(g0.x - start.x, g0.y - start.y), last);
 }
 
-// B: a block owns one sequence, eight units and 128 features; a warp one unit, a lane four features.  The powers of
-// lambda are made once per block, so a step costs two multiply-adds per entry, and only the old and the new
-// sensitivities touch memory: HBM-bound at large N F, else bound by the multiply-adds.  (64 sequences x 64 steps, 64
-// features, 128 units: the materialised Jacobians took 490 us of kernels in 76 launches.)
-constexpr int kSensUnits = 8, kSensSteps = 64, kSensFeatures = 128;
-__global__ void __launch_bounds__(256) lru_sens_inputs_kernel(LruWeights w, const float* __restrict__ lambda,
-                                                              const float* __restrict__ u, const uint8_t* __restrict__ done,
-                                                              LruSensitivities s, int T, int F, int N) {
+// B: a block owns one sequence, 256 / kLanes units and 4 kLanes features; kLanes lanes share a unit, four features each.
+// The powers of lambda are made once per block, so a step costs one packed multiply-add per entry, and only the old and the
+// new sensitivities touch memory: HBM-bound at large N F, else bound by the multiply-adds.  The blocks behind them take the
+// other leaves.  (64 sequences x 64 steps, 64 features, 128 units: the materialised Jacobians took 490 us of kernels in 76
+// launches.)
+constexpr int kSensSteps = 64;
+template <int kLanes>
+__global__ void __launch_bounds__(256) lru_sensitivities_kernel(LruWeights w, const float* __restrict__ lambda,
+                                                                const float* __restrict__ h, const float* __restrict__ h0,
+                                                                const float* __restrict__ u, const uint8_t* __restrict__ done,
+                                                                LruSensitivities s, int T, int F, int N, int input_blocks) {
   enter_kernel();
-  __shared__ __align__(16) float us[kSensSteps][kSensFeatures];
-  __shared__ float2 pw[kSensUnits][kSensSteps + 1];
-  const int b = blockIdx.z, n0 = blockIdx.x * kSensUnits, f0 = blockIdx.y * kSensFeatures;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n = n0 + warp, f = f0 + lane * 4;
-  const int r = last_reset(done ? done + static_cast<size_t>(b) * T : nullptr, T);
-  const int first = max(r, 0);
-  for (int i = threadIdx.x; i < kSensUnits * (kSensSteps + 1); i += 256) {
-    const int un = i / (kSensSteps + 1), k = i % (kSensSteps + 1);
-    if (n0 + un < N) pw[un][k] = power(reinterpret_cast<const float2*>(lambda)[n0 + un], k);
+  constexpr int kUnits = 256 / kLanes, kFeatures = 4 * kLanes;
+  __shared__ __align__(16) float us[kSensSteps][kFeatures];
+  __shared__ float2 pw[kUnits][kSensSteps + 1];
+  const int b = blockIdx.y;
+  const uint8_t* drow = done ? done + static_cast<size_t>(b) * T : nullptr;
+  if (static_cast<int>(blockIdx.x) >= input_blocks) {
+    unit_sensitivities(w, lambda, h, h0, s, b, (blockIdx.x - input_blocks) * 32, last_reset(drow, T), T, N);
+    return;
   }
-  float re[4] = {0.f, 0.f, 0.f, 0.f}, im[4] = {0.f, 0.f, 0.f, 0.f};
+  const int unit_groups = (N + kUnits - 1) / kUnits;
+  const int n0 = (blockIdx.x % unit_groups) * kUnits, f0 = (blockIdx.x / unit_groups) * kFeatures;
+  const int un = threadIdx.x / kLanes, lf = threadIdx.x % kLanes;
+  const int n = n0 + un, f = f0 + lf * 4;
+  const bool in = n < N && f < F, wide = F % 4 == 0;
+  const size_t at = (static_cast<size_t>(b) * N + (in ? n : 0)) * F + (in ? f : 0);
+  float4 ore[2] = {}, oim[2] = {};   // old sensitivities, on their way while the sums are formed
+  if (in && wide) {
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      ore[e] = ld_stream(reinterpret_cast<const float4*>(s.b_re + 2 * at) + e);
+      oim[e] = ld_stream(reinterpret_cast<const float4*>(s.b_im + 2 * at) + e);
+    }
+  }
+  const int r = last_reset(drow, T);
+  const int first = max(r, 0);
+  for (int i = threadIdx.x; i < kUnits * (kSensSteps + 1); i += 256) {
+    const int ui = i / (kSensSteps + 1), k = i % (kSensSteps + 1);
+    if (n0 + ui < N) pw[ui][k] = power(reinterpret_cast<const float2*>(lambda)[n0 + ui], k);
+  }
+  float2 acc[4] = {};
   const float* ub = u + static_cast<size_t>(b) * T * F;
   for (int t0 = first; t0 < T; t0 += kSensSteps) {
     const int len = min(kSensSteps, T - t0);
     __syncthreads();
-    for (int i = threadIdx.x; i < len * kSensFeatures; i += 256) {
-      const int t = i / kSensFeatures, c = i % kSensFeatures;
-      us[t][c] = f0 + c < F ? ub[static_cast<size_t>(t0 + t) * F + f0 + c] : 0.f;
+    for (int i = threadIdx.x; i < len * kFeatures; i += 256) {
+      const int t = i / kFeatures, c = i % kFeatures;
+      us[t][c] = f0 + c < F ? __ldg(ub + static_cast<size_t>(t0 + t) * F + f0 + c) : 0.f;
     }
     __syncthreads();
-    if (n >= N || f >= F) continue;
-    const float2 shift = pw[warp][len];   // what earlier steps have decayed by at the end of this stretch
+    const float2 shift = pw[un][len];   // what earlier steps have decayed by at the end of this stretch
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float2 v = cmul(shift, make_float2(re[e], im[e]));
-      re[e] = v.x;
-      im[e] = v.y;
-    }
+    for (int e = 0; e < 4; ++e) acc[e] = cmul(shift, acc[e]);
 #pragma unroll 8
     for (int t = 0; t < len; ++t) {
-      const float4 x = *reinterpret_cast<const float4*>(&us[t][lane * 4]);
-      const float2 p = pw[warp][len - 1 - t];
-      re[0] = fmaf(p.x, x.x, re[0]); im[0] = fmaf(p.y, x.x, im[0]);
-      re[1] = fmaf(p.x, x.y, re[1]); im[1] = fmaf(p.y, x.y, im[1]);
-      re[2] = fmaf(p.x, x.z, re[2]); im[2] = fmaf(p.y, x.z, im[2]);
-      re[3] = fmaf(p.x, x.w, re[3]); im[3] = fmaf(p.y, x.w, im[3]);
+      const float4 x = *reinterpret_cast<const float4*>(&us[t][lf * 4]);
+      const float2 p = pw[un][len - 1 - t];
+      acc[0] = __ffma2_rn(p, make_float2(x.x, x.x), acc[0]);
+      acc[1] = __ffma2_rn(p, make_float2(x.y, x.y), acc[1]);
+      acc[2] = __ffma2_rn(p, make_float2(x.z, x.z), acc[2]);
+      acc[3] = __ffma2_rn(p, make_float2(x.w, x.w), acc[3]);
     }
   }
-  if (n >= N || f >= F) return;
+  if (!in) return;
   const float gamma = expf(w.gamma_log[n]);
   const float2 p = r < 0 ? power(reinterpret_cast<const float2*>(lambda)[n], T) : make_float2(0.f, 0.f);
-  const size_t at = (static_cast<size_t>(b) * N + n) * F + f;
-  const auto one = [&](const float2 o, float x, float y) { return cmul_add(p, o, make_float2(x, y)); };
-  if (F % 4 == 0) {   // sixteen-byte accesses: two complex entries each
+  const auto re = [&](float2 o, int e) { return cmul_add(p, o, make_float2(gamma * acc[e].x, gamma * acc[e].y)); };
+  const auto im = [&](float2 o, int e) { return cmul_add(p, o, make_float2(-gamma * acc[e].y, gamma * acc[e].x)); };
+  if (wide) {   // sixteen-byte accesses: two complex entries each
 #pragma unroll
-    for (int e = 0; e < 4; e += 2) {
-      const float4 o = ld_stream(reinterpret_cast<const float4*>(s.b_re + 2 * (at + e)));
-      const float4 q = ld_stream(reinterpret_cast<const float4*>(s.b_im + 2 * (at + e)));
-      const float2 v0 = one({o.x, o.y}, gamma * re[e], gamma * im[e]), v1 = one({o.z, o.w}, gamma * re[e + 1], gamma * im[e + 1]);
-      const float2 y0 = one({q.x, q.y}, -gamma * im[e], gamma * re[e]), y1 = one({q.z, q.w}, -gamma * im[e + 1], gamma * re[e + 1]);
-      *reinterpret_cast<float4*>(s.b_re_out + 2 * (at + e)) = make_float4(v0.x, v0.y, v1.x, v1.y);
-      *reinterpret_cast<float4*>(s.b_im_out + 2 * (at + e)) = make_float4(y0.x, y0.y, y1.x, y1.y);
+    for (int e = 0; e < 2; ++e) {
+      const float2 v0 = re({ore[e].x, ore[e].y}, 2 * e), v1 = re({ore[e].z, ore[e].w}, 2 * e + 1);
+      const float2 y0 = im({oim[e].x, oim[e].y}, 2 * e), y1 = im({oim[e].z, oim[e].w}, 2 * e + 1);
+      reinterpret_cast<float4*>(s.b_re_out + 2 * at)[e] = make_float4(v0.x, v0.y, v1.x, v1.y);
+      reinterpret_cast<float4*>(s.b_im_out + 2 * at)[e] = make_float4(y0.x, y0.y, y1.x, y1.y);
     }
   } else {
-    for (int e = 0; e < 4 && f + e < F; ++e) {
-      const float2 o = reinterpret_cast<const float2*>(s.b_re)[at + e], q = reinterpret_cast<const float2*>(s.b_im)[at + e];
-      reinterpret_cast<float2*>(s.b_re_out)[at + e] = one(o, gamma * re[e], gamma * im[e]);
-      reinterpret_cast<float2*>(s.b_im_out)[at + e] = one(q, -gamma * im[e], gamma * re[e]);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      if (f + e >= F) break;
+      reinterpret_cast<float2*>(s.b_re_out)[at + e] = re(reinterpret_cast<const float2*>(s.b_re)[at + e], e);
+      reinterpret_cast<float2*>(s.b_im_out)[at + e] = im(reinterpret_cast<const float2*>(s.b_im)[at + e], e);
     }
   }
 }
@@ -371,9 +400,11 @@ int lru_step(const LruWeights& w, const float* x, const float* h0, const float* 
              float* a_last, float* y, int B, int F, int N, cudaStream_t stream) {
   if (B <= 0 || F <= 0 || N <= 0) return MXK_ERR_DIMS;
   const long long groups = (B + 7) / 8;
-  const long long warps_h = groups * ((N + 1) / 2), warps_y = groups * ((F + 3) / 4);
-  mxk::launch_kernel(lru_step_state_kernel, static_cast<unsigned>((warps_h + 3) / 4), 128, 0, stream, w, x, h0, a0, done, h, a_last, B, F, N);
-  mxk::launch_kernel(lru_step_read_kernel, static_cast<unsigned>((warps_y + 3) / 4), 128, 0, stream, w, x, h, y, B, F, N);
+  const long long tiles_h = groups * ((N + 1) / 2), tiles_y = groups * ((F + 3) / 4);
+  const auto state = few_tiles(tiles_h) ? lru_step_state_kernel<4> : lru_step_state_kernel<1>;
+  const auto read = few_tiles(tiles_y) ? lru_step_read_kernel<4> : lru_step_read_kernel<1>;
+  mxk::launch_kernel(state, tile_blocks(tiles_h), 128, 0, stream, w, x, h0, a0, done, h, a_last, B, F, N);
+  mxk::launch_kernel(read, tile_blocks(tiles_y), 128, 0, stream, w, x, h, y, B, F, N);
   return launch_status();
 }
 
@@ -392,10 +423,14 @@ int lru_param_grads(const LruWeights& w, const LruGrads& g, int F, int N, cudaSt
 int lru_sensitivities(const LruWeights& w, const float* lambda, const float* h, const float* h0, const float* u,
                       const uint8_t* done, const LruSensitivities& s, int B, int T, int F, int N, cudaStream_t stream) {
   if (B <= 0 || T <= 0 || F <= 0 || N <= 0 || B > 65535) return MXK_ERR_DIMS;
-  mxk::launch_kernel(lru_sens_units_kernel, dim3((N + 127) / 128, B), 128, 0, stream, w, lambda, h, h0, done, s, T, N);
-  const dim3 grid((N + kSensUnits - 1) / kSensUnits, (F + kSensFeatures - 1) / kSensFeatures, B);
-  mxk::launch_kernel(lru_sens_inputs_kernel, grid, 256, 0, stream, w, lambda, u, done, s, T, F, N);
-  return launch_status();
+  // lanes per unit: as many as four features each need, so that narrow inputs leave none idle
+  const auto go = [&](auto kernel, int lanes) {
+    const int units = 256 / lanes, inputs = ((N + units - 1) / units) * ((F + 4 * lanes - 1) / (4 * lanes));
+    return mxk::launch_kernel(kernel, dim3(inputs + (N + 31) / 32, B), 256, 0, stream, w, lambda, h, h0, u, done, s, T, F, N, inputs);
+  };
+  if (F <= 32) return go(lru_sensitivities_kernel<8>, 8);
+  if (F <= 64) return go(lru_sensitivities_kernel<16>, 16);
+  return go(lru_sensitivities_kernel<32>, 32);
 }
 
 }  // namespace layers

@@ -333,20 +333,23 @@ int turn_length(int T) {
   return (T + turns - 1) / turns;
 }
 
+template <int kSplit>
 __global__ void __launch_bounds__(128)
 mingru_step_kernel(const float* __restrict__ in, const float* __restrict__ w_z, const float* __restrict__ w_h,
                    const float* __restrict__ x0, const float* __restrict__ a0, const uint8_t* __restrict__ done,
                    float* __restrict__ x, float* __restrict__ y, float* __restrict__ a_last, int B, int F, int D) {
   enter_kernel();
-  const int lane = threadIdx.x & 31, warp = blockIdx.x * 4 + (threadIdx.x >> 5);
+  const TilePlace<kSplit> at_tile;
+  const int lane = at_tile.lane;
   const int units = (D + 1) / 2;
-  const int d0 = (warp % units) * 2, m0 = (warp / units) * 8;
+  const int d0 = (at_tile.tile % units) * 2, m0 = (at_tile.tile / units) * 8;
   if (m0 >= B) return;
   const size_t r0 = static_cast<size_t>(d0) * F, r1 = static_cast<size_t>(min(d0 + 1, D - 1)) * F;
   const float* rows[4] = {w_z + r0, w_h + r0, w_z + r1, w_h + r1};
   WarpTile acc;
-  acc.accumulate(in + static_cast<size_t>(m0) * F, F, min(8, B - m0), rows, F, lane);
-  const float v = acc.reduce(lane);
+  acc.accumulate(in + static_cast<size_t>(m0) * F, F, min(8, B - m0), rows, F, at_tile.first, at_tile.step);
+  float v = acc.reduce(lane);
+  if (!join_warps<kSplit>(v, lane)) return;
   const float other = __shfl_xor_sync(0xffffffffu, v, 1);
   const int m = m0 + (lane >> 2), d = d0 + ((lane >> 1) & 1);
   if ((lane & 1) || m >= B || d >= D) return;   // even lanes hold z, their neighbours h~
@@ -388,8 +391,9 @@ int mingru_bwd(const float* z, const float* h_tilde, long long ld, const float* 
 int mingru_step(const float* in, const float* w_z, const float* w_h, const float* x0, const float* a0, const uint8_t* done,
                 float* x, float* y, float* a_last, int B, int F, int D, cudaStream_t stream) {
   if (B <= 0 || F <= 0 || D <= 0) return MXK_ERR_DIMS;
-  const long long warps = static_cast<long long>((B + 7) / 8) * ((D + 1) / 2);
-  mxk::launch_kernel(mingru_step_kernel, static_cast<unsigned>((warps + 3) / 4), 128, 0, stream, in, w_z, w_h, x0, a0, done, x, y, a_last, B, F, D);
+  const long long tiles = static_cast<long long>((B + 7) / 8) * ((D + 1) / 2);
+  mxk::launch_kernel(few_tiles(tiles) ? mingru_step_kernel<4> : mingru_step_kernel<1>, tile_blocks(tiles), 128, 0, stream, in, w_z, w_h, x0, a0, done,
+                     x, y, a_last, B, F, D);
   return launch_status();
 }
 

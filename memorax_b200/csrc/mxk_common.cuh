@@ -54,9 +54,10 @@ inline int launch_kernel(void (*kernel)(P...), dim3 grid, dim3 block, size_t sme
 }
 
 // First statement of every kernel, executed by all threads.  A grid of at most two blocks per SM lets its successor's
-// blocks take their places at once; a larger one would have them pile up on the SMs that empty first.
-__device__ __forceinline__ void enter_kernel() {
-  if (gridDim.x * gridDim.y * gridDim.z <= 2u * kNumSMs) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+// blocks take their places at once (`brief`: a persistent kernel says whether its blocks have one piece of work only); a
+// larger or longer one would have them wait, or pile up on the SMs that empty first (3 % of the 1024 x 1024 LRU layer).
+__device__ __forceinline__ void enter_kernel(bool brief = true) {
+  if (brief && gridDim.x * gridDim.y * gridDim.z <= 2u * kNumSMs) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 

@@ -1,5 +1,6 @@
-// Small float32 products y[m][n] = sum_k x[m][k] w[n][k]: a warp computes 8 rows of x times 4 rows of w, its lanes
-// spread over k.
+// Small float32 products y[m][n] = sum_k x[m][k] w[n][k]: kSplit warps compute 8 rows of x times 4 rows of w, their lanes
+// spread over k.  Blocks of four warps; four to a tile while there are few tiles (the loop over k is a chain of L2 round
+// trips: 16 x 256 x 128 took 7.2 us with one warp per tile), one where the tiles fill the machine anyway.
 #pragma once
 
 namespace mxk {
@@ -12,9 +13,9 @@ struct WarpTile {
   }
   // x: first of `rows` rows (1..8; the others repeat the last one), `ld` apart; w: the four weight rows
   __device__ __forceinline__ void accumulate(const float* __restrict__ x, long long ld, int rows, const float* const (&w)[4],
-                                             int K, int lane) {
+                                             int K, int first, int step) {
 #pragma unroll 2
-    for (int k = lane; k < K; k += 32) {
+    for (int k = first; k < K; k += step) {
       float xv[8], wv[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) wv[j] = __ldg(w[j] + k);
@@ -40,5 +41,33 @@ struct WarpTile {
     return v[0];
   }
 };
+
+// Where a thread of a block of four warps works: its tile, and its share of k.
+template <int kSplit>
+struct TilePlace {
+  int tile, first, step, lane;
+  __device__ __forceinline__ TilePlace() {
+    const int warp = threadIdx.x >> 5;
+    lane = threadIdx.x & 31;
+    tile = kSplit == 4 ? static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x) * 4 + warp;
+    first = kSplit == 4 ? warp * 32 + lane : lane;
+    step = 32 * kSplit;
+  }
+};
+// The sum of a tile's warps, in the first of them; the others are done.
+template <int kSplit>
+__device__ __forceinline__ bool join_warps(float& v, int lane) {
+  if constexpr (kSplit == 4) {
+    __shared__ float part[3][32];
+    const int warp = threadIdx.x >> 5;
+    if (warp > 0) part[warp - 1][lane] = v;
+    __syncthreads();
+    if (warp > 0) return false;
+    v += (part[0][lane] + part[1][lane]) + part[2][lane];
+  }
+  return true;
+}
+inline bool few_tiles(long long tiles) { return tiles <= 8 * 148; }
+inline unsigned tile_blocks(long long tiles) { return static_cast<unsigned>(few_tiles(tiles) ? tiles : (tiles + 3) / 4); }
 
 }  // namespace mxk

@@ -61,8 +61,8 @@ def test_lru_layer_matches_the_oracle(shape, with_carry):
         assert err(got, ref) <= 1e-4
 
 
-# stretches of 64 steps, groups of 8 units and of 128 features; with and without a reset in a sequence
-@pytest.mark.parametrize("shape", [(2, 1, 4, 3), (3, 64, 33, 9), (2, 65, 130, 16), (4, 150, 8, 130)])
+# stretches of 64 steps, eight pieces of time for the leaves per unit, 8 / 16 / 32 units by 128 / 64 / 32 features; with and without a reset in a sequence
+@pytest.mark.parametrize("shape", [(2, 1, 4, 3), (3, 64, 33, 9), (2, 65, 130, 16), (4, 150, 8, 130), (2, 9, 48, 33)])
 @pytest.mark.parametrize("p_done", [0.0, 0.03])
 def test_fused_rtrl_segment_matches_the_oracle(shape, p_done):
     from memorax_b200.memoroid import LRUCell, Memoroid
