@@ -55,10 +55,13 @@ struct Params {
   int* status;
 };
 
+// BN = 256: two CTAs share a 256 x 256 tile (cta_group::2), each with its 128 rows of A and half of the rows of B.
 template <int BN>
 struct Layout {
-  static constexpr int kStages = BN == 256 ? 3 : (BN == 128 ? 4 : 5);
-  static constexpr int kPlaneA = kBM * kBK * 2, kPlaneB = BN * kBK * 2;   // bytes
+  static constexpr bool kPair = BN == 256;
+  static constexpr int kRowsB = kPair ? BN / 2 : BN;   // rows of B in this CTA
+  static constexpr int kStages = BN == 64 ? 5 : 4;
+  static constexpr int kPlaneA = kBM * kBK * 2, kPlaneB = kRowsB * kBK * 2;   // bytes
   static constexpr int kStage = 3 * (kPlaneA + kPlaneB);
   static constexpr int kBarriers = kStages * kStage;
   static constexpr int kBytes = kBarriers + 256;
@@ -80,20 +83,6 @@ __device__ __forceinline__ void load8(const float* p, int valid, int vec, float*
   } else {
 #pragma unroll
     for (int e = 0; e < 8; ++e) x[e] = e < valid ? __ldg(p + e) : 0.f;
-  }
-}
-
-// What this thread has stored before (not through the read-only path).
-__device__ __forceinline__ void load8_own(const float* p, int valid, int vec, float* x) {
-  if (valid >= 8 && vec == 8) {
-    asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]), "=f"(x[4]), "=f"(x[5]), "=f"(x[6]), "=f"(x[7])
-                 : "l"(p)
-                 : "memory");
-  } else {
-    const volatile float* q = p;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) x[e] = e < valid ? q[e] : 0.f;
   }
 }
 
@@ -208,24 +197,45 @@ __device__ __forceinline__ void store8(float* p, int valid, int vec, const float
   }
 }
 
+// Adds to what this thread has stored (or added) there before: fire and forget, and in program order, so the sums are the
+// same every time.  (A load, an addition and a store cost 26 k cycles per drained 128 x 256 tile.)
+__device__ __forceinline__ void add8(float* p, int valid, int vec, const float* x) {
+  if (valid >= 8 && vec >= 4) {
+#pragma unroll
+    for (int h = 0; h < 8; h += 4)
+      asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1,%2,%3,%4};" ::"l"(p + h), "f"(x[h]), "f"(x[h + 1]), "f"(x[h + 2]), "f"(x[h + 3])
+                   : "memory");
+  } else {
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+      if (e < valid) asm volatile("red.relaxed.gpu.global.add.f32 [%0], %1;" ::"l"(p + e), "f"(x[e]) : "memory");
+  }
+}
+
 // kOuter: C = A^T B, both operands contracted over their rows and converted here; else C = A W^T, W from its image.
 template <int BN, bool kOuter>
 struct Roles {
   // (a seventeenth warp is the last that leaves 96 registers a thread)
-  static constexpr int kProducerWarps = kOuter ? 12 : 8, kEpilogueWarps = kOuter ? 4 : 8;
+  static constexpr int kProducerWarps = !kOuter ? 8 : (BN == 256 ? 16 : 12), kEpilogueWarps = kOuter ? 4 : 8;
   static constexpr int kMmaWarp = kProducerWarps + kEpilogueWarps;
   static constexpr int kThreads = 32 * (kMmaWarp + 1);
 };
 
 template <int BN, bool kOuter>
 __global__ void __launch_bounds__(Roles<BN, kOuter>::kThreads, 1) gemm32_kernel(const __grid_constant__ Params p) {
-  enter_kernel(((p.M + kBM - 1) / kBM) * ((p.N + BN - 1) / BN) * p.splits <= static_cast<int>(gridDim.x) && p.k_split <= 2 * kSegment);
   using L = Layout<BN>;
+  constexpr bool kPair = L::kPair;
+  constexpr int kTileM = kPair ? 2 * kBM : kBM;
+  const int mt = (p.M + kTileM - 1) / kTileM, nt = (p.N + BN - 1) / BN;
+  const int tiles = mt * nt * p.splits;
+  const int first_tile = kPair ? blockIdx.x / 2 : blockIdx.x, tile_step = kPair ? gridDim.x / 2 : gridDim.x;
+  enter_kernel(tiles <= tile_step && p.k_split <= 2 * kSegment);
+  const int rank = kPair ? static_cast<int>(cluster_rank()) : 0;
   using R = Roles<BN, kOuter>;
   constexpr int kProducerWarps = R::kProducerWarps, kEpilogueWarps = R::kEpilogueWarps, kMmaWarp = R::kMmaWarp;
   constexpr int kColumnParts = kEpilogueWarps / 4;   // epilogue warps that share the rows, and the columns between them
   using TileA = Tile<kOuter, kBM, kProducerWarps>;
-  using TileB = Tile<true, BN, kProducerWarps>;
+  using TileB = Tile<true, L::kRowsB, kProducerWarps>;
   constexpr int kStages = L::kStages;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* const bars = reinterpret_cast<uint64_t*>(smem + L::kBarriers);
@@ -233,29 +243,35 @@ __global__ void __launch_bounds__(Roles<BN, kOuter>::kThreads, 1) gemm32_kernel(
   uint64_t* const empty = bars + kStages;      // MMA -> producers
   uint64_t* const acc_full = bars + 2 * kStages;       // MMA -> epilogue
   uint64_t* const acc_empty = bars + 2 * kStages + 2;  // epilogue -> MMA
-  uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 4);
+  uint64_t* const peer_full = bars + 2 * kStages + 4;  // rank 0: the other CTA's stage is full
+  uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * kStages + 4);
+  const auto wait = [](uint64_t* bar, uint32_t parity, bool& timed_out) {
+    if (kPair) mbar_wait_cluster_flag(bar, parity, timed_out);
+    else mbar_wait_flag(bar, parity, timed_out);
+  };
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (tid == 0) {
-    for (int s = 0; s < kStages; ++s) { mbar_init(&full[s], kProducerWarps + (kOuter ? 0 : 1)); mbar_init(&empty[s], 1); }
-    for (int s = 0; s < 2; ++s) { mbar_init(&acc_full[s], 1); mbar_init(&acc_empty[s], kEpilogueWarps); }
+    for (int s = 0; s < kStages; ++s) { mbar_init(&full[s], kProducerWarps + (kOuter ? 0 : 1)); mbar_init(&empty[s], 1); mbar_init(&peer_full[s], 1); }
+    for (int s = 0; s < 2; ++s) { mbar_init(&acc_full[s], 1); mbar_init(&acc_empty[s], kEpilogueWarps * (kPair ? 2 : 1)); }
     mbar_init_fence();
   }
-  if (warp == kMmaWarp) tmem_alloc(tmem_slot, L::kTmem);
+  if (warp == kMmaWarp) {
+    if (kPair) tmem_alloc_pair(tmem_slot, L::kTmem);
+    else tmem_alloc(tmem_slot, L::kTmem);
+  }
   fence_before_sync();
   __syncthreads();
+  if (kPair) cluster_sync();   // the other CTA's barriers are there
   fence_after_sync();
   const uint32_t tmem = *tmem_slot;
   bool timed_out = false;
-
-  const int mt = (p.M + kBM - 1) / kBM, nt = (p.N + BN - 1) / BN;
-  const int tiles = mt * nt * p.splits;
 
   if (warp >= kEpilogueWarps && warp < kMmaWarp) {
     // ------------------------------------------------------------ producers
     const int pw = warp - kEpilogueWarps;
     const int k_images = (p.K + kBK - 1) / kBK;
-    int tile = blockIdx.x;
+    int tile = first_tile;
     int stage = 0;
     uint32_t parity = 1;   // a fresh barrier's previous phase counts as complete
     TileA ta;
@@ -264,8 +280,8 @@ __global__ void __launch_bounds__(Roles<BN, kOuter>::kThreads, 1) gemm32_kernel(
     bool a_inner = false, b_inner = false;
     auto tile_begin = [&](int t) {
       const int mn = t % (mt * nt), sp = t / (mt * nt);
-      n0 = (mn % nt) * BN;
-      m0 = (mn / nt) * kBM;
+      n0 = (mn % nt) * BN + rank * L::kRowsB;   // of this CTA's part of B
+      m0 = (mn / nt) * kTileM + rank * kBM;
       k0 = sp * p.k_split;
       k_end = min(p.K, k0 + p.k_split);
       ta.begin(p.a, p.lda, pw, lane, m0, k0);
@@ -274,7 +290,7 @@ __global__ void __launch_bounds__(Roles<BN, kOuter>::kThreads, 1) gemm32_kernel(
     auto bounds = [&]() {
       const bool k_in = k0 + kBK <= k_end;
       a_inner = p.a_wide && k_in && m0 + kBM <= p.M;
-      b_inner = p.b_wide && k_in && n0 + BN <= p.N;
+      b_inner = p.b_wide && k_in && n0 + L::kRowsB <= p.N;
     };
     if (tile < tiles) {
       tile_begin(tile);
@@ -287,11 +303,11 @@ __global__ void __launch_bounds__(Roles<BN, kOuter>::kThreads, 1) gemm32_kernel(
       }
     }
     while (tile < tiles) {
-      const uint8_t* const image = kOuter ? nullptr : p.image + (static_cast<size_t>(n0 / BN) * k_images + k0 / kBK) * (3 * L::kPlaneB);
+      const uint8_t* const image = kOuter ? nullptr : p.image + (static_cast<size_t>(n0 / L::kRowsB) * k_images + k0 / kBK) * (3 * L::kPlaneB);
       // the block after this one, whose loads are issued as this one's registers are released
       k0 += kBK;
       if (k0 >= k_end) {
-        tile += gridDim.x;
+        tile += tile_step;
         if (tile < tiles) tile_begin(tile);
       } else {
         ta.advance(p.lda);
@@ -299,7 +315,7 @@ __global__ void __launch_bounds__(Roles<BN, kOuter>::kThreads, 1) gemm32_kernel(
       }
       const bool more = tile < tiles;
       bounds();
-      mbar_wait_flag(&empty[stage], parity, timed_out);
+      wait(&empty[stage], parity, timed_out);
       uint8_t* const base = smem + stage * L::kStage;
       if (!kOuter && pw == 0 && lane == 0) {
         tma::expect_bytes(&full[stage], 3 * L::kPlaneB);
@@ -325,49 +341,60 @@ __global__ void __launch_bounds__(Roles<BN, kOuter>::kThreads, 1) gemm32_kernel(
   } else if (warp == kMmaWarp) {
     // ------------------------------------------------------------ tensor core
     const bool leader = elect_one();
-    const uint32_t idesc = idesc_bf16(kBM, BN, kOuter, kOuter);
+    const uint32_t idesc = idesc_bf16(kTileM, BN, kOuter, kOuter);
     int stage = 0;
     uint32_t parity = 0;
     int turn = 0;
-    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    for (int tile = first_tile; tile < tiles; tile += tile_step) {
       const int sp = tile / (mt * nt);
       const int k_len = min(p.K, (sp + 1) * p.k_split) - sp * p.k_split;
       for (int seg = 0; seg < k_len; seg += kSegment, ++turn) {
         const int blocks = (min(k_len - seg, kSegment) + kBK - 1) / kBK;
         const int buf = turn % L::kAccs;
-        mbar_wait_flag(&acc_empty[buf], ((turn / L::kAccs) & 1) ^ 1, timed_out);
+        if (rank == 0) wait(&acc_empty[buf], ((turn / L::kAccs) & 1) ^ 1, timed_out);
         fence_after_sync();
         const uint32_t acc = tmem + buf * 2 * BN, acc_small = acc + BN;
         for (int kb = 0; kb < blocks; ++kb) {
-          mbar_wait_flag(&full[stage], parity, timed_out);
+          wait(&full[stage], parity, timed_out);
+          if (kPair && rank != 0) {   // this CTA's stage is full: the other one issues
+            if (leader) arrive_at_leader(&peer_full[stage]);
+            __syncwarp();
+            if (++stage == kStages) { stage = 0; parity ^= 1; }
+            continue;
+          }
+          if (kPair) wait(&peer_full[stage], parity, timed_out);
           fence_after_sync();
           const uint32_t sa = smem_u32(smem + stage * L::kStage), sb = sa + 3 * L::kPlaneA;
-          constexpr uint32_t kRowsA = kOuter ? kBK : kBM, kRowsB = kOuter ? kBK : BN;
+          constexpr uint32_t kRowsA = kOuter ? kBK : kBM, kRowsB = kOuter ? kBK : L::kRowsB;
           const Operand a0{sa, kRowsA, kOuter}, a1{sa + L::kPlaneA, kRowsA, kOuter}, a2{sa + 2 * L::kPlaneA, kRowsA, kOuter};
           const Operand b0{sb, kRowsB, kOuter}, b1{sb + L::kPlaneB, kRowsB, kOuter}, b2{sb + 2 * L::kPlaneB, kRowsB, kOuter};
-          gemm<kBK / 16>(acc_small, a2, b0, idesc, kb > 0, leader);
-          gemm<kBK / 16>(acc_small, a0, b2, idesc, true, leader);
-          gemm<kBK / 16>(acc_small, a1, b1, idesc, true, leader);
-          gemm<kBK / 16>(acc_small, a1, b0, idesc, true, leader);
-          gemm<kBK / 16>(acc_small, a0, b1, idesc, true, leader);
-          gemm<kBK / 16>(acc, a0, b0, idesc, kb > 0, leader);
-          if (leader) commit(&empty[stage]);
+          const auto product = [&](uint32_t d, const Operand& a, const Operand& b, bool accumulate) {
+            if (kPair) gemm_pair<kBK / 16>(d, a, b, idesc, accumulate, leader);
+            else gemm<kBK / 16>(d, a, b, idesc, accumulate, leader);
+          };
+          product(acc_small, a2, b0, kb > 0);
+          product(acc_small, a0, b2, true);
+          product(acc_small, a1, b1, true);
+          product(acc_small, a1, b0, true);
+          product(acc_small, a0, b1, true);
+          product(acc, a0, b0, kb > 0);
+          if (leader) (kPair ? commit_pair : commit)(&empty[stage]);
           if (++stage == kStages) { stage = 0; parity ^= 1; }
         }
-        if (leader) commit(&acc_full[buf]);
+        if (leader && rank == 0) (kPair ? commit_pair : commit)(&acc_full[buf]);
       }
     }
     // the last commits may still be on their way to barriers in this CTA's shared memory
     for (int s = 0; s < kStages; ++s) {
-      mbar_wait_flag(&empty[stage], parity ^ 1, timed_out);
+      wait(&empty[stage], parity ^ 1, timed_out);
       if (++stage == kStages) { stage = 0; parity ^= 1; }
     }
   } else if (warp < kEpilogueWarps) {
     // ------------------------------------------------------------ epilogue
     int turn = 0;
-    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    for (int tile = first_tile; tile < tiles; tile += tile_step) {
       const int mn = tile % (mt * nt), sp = tile / (mt * nt);
-      const int n0 = (mn % nt) * BN, m0 = (mn / nt) * kBM;
+      const int n0 = (mn % nt) * BN, m0 = (mn / nt) * kTileM + rank * kBM;
       const int m = m0 + (warp & 3) * 32 + lane;
       const bool in = m < p.M;
       const bool split = p.splits > 1;
@@ -378,7 +405,7 @@ __global__ void __launch_bounds__(Roles<BN, kOuter>::kThreads, 1) gemm32_kernel(
       for (int seg = 0; seg < k_len; seg += kSegment, ++turn) {
         const int buf = turn % L::kAccs;
         const bool last = seg + kSegment >= k_len;
-        mbar_wait_flag(&acc_full[buf], (turn / L::kAccs) & 1, timed_out);
+        wait(&acc_full[buf], (turn / L::kAccs) & 1, timed_out);
         fence_after_sync();
         const uint32_t src = tmem + buf * 2 * BN + (static_cast<uint32_t>((warp & 3) * 32) << 16);
 #pragma unroll 1
@@ -396,11 +423,6 @@ __global__ void __launch_bounds__(Roles<BN, kOuter>::kThreads, 1) gemm32_kernel(
             const int n = n0 + c + g * 8, valid = in ? p.N - n : 0;
             if (valid <= 0) continue;
             float ad[8];
-            if (seg > 0) {   // this thread's own earlier segment of the contraction
-              load8_own(crow + n, valid, p.c_vec, ad);
-#pragma unroll
-              for (int e = 0; e < 8; ++e) v[g * 8 + e] += ad[e];
-            }
             if (last && !split && p.ep.bias) {
 #pragma unroll
               for (int e = 0; e < 8; ++e)
@@ -412,12 +434,16 @@ __global__ void __launch_bounds__(Roles<BN, kOuter>::kThreads, 1) gemm32_kernel(
               for (int e = 0; e < 8; ++e)
                 v[g * 8 + e] = fmaf(ad[e], (p.ep.add_scale && e < valid) ? __ldg(p.ep.add_scale + n + e) : 1.f, v[g * 8 + e]);
             }
-            store8(crow + n, valid, p.c_vec, v + g * 8);
+            if (seg > 0) add8(crow + n, valid, p.c_vec, v + g * 8);   // to this thread's own earlier segments
+            else store8(crow + n, valid, p.c_vec, v + g * 8);
           }
         }
         fence_before_sync();
         __syncwarp();
-        if (lane == 0) arrive(&acc_empty[buf]);
+        if (lane == 0) {
+          if (kPair) arrive_at_leader(&acc_empty[buf]);
+          else arrive(&acc_empty[buf]);
+        }
       }
     }
   }
@@ -425,7 +451,11 @@ __global__ void __launch_bounds__(Roles<BN, kOuter>::kThreads, 1) gemm32_kernel(
   if (timed_out && p.status) atomicExch(p.status, 1);
   fence_before_sync();
   __syncthreads();
-  if (warp == kMmaWarp) tmem_dealloc(tmem, L::kTmem);
+  if (kPair) cluster_sync();   // nothing reaches into the other CTA any more
+  if (warp == kMmaWarp) {
+    if (kPair) tmem_dealloc_pair(tmem, L::kTmem);
+    else tmem_dealloc(tmem, L::kTmem);
+  }
 }
 
 // C = sum over splits of the partial products (fixed order: bit-reproducible) + epilogue
@@ -465,12 +495,14 @@ struct Plan {
   int bn, splits, k_split;
 };
 Plan plan(int M, int N, int K) {
-  const int mt = (M + kBM - 1) / kBM;
   Plan pl{256, 1, 0};
-  const auto tiles = [&](int bn) { return static_cast<long long>(mt) * ((N + bn - 1) / bn); };
+  const auto tiles = [&](int bn) {   // CTAs that one pass over C occupies
+    const int tm = bn == 256 ? 2 * kBM : kBM;
+    return static_cast<long long>((M + tm - 1) / tm) * ((N + bn - 1) / bn) * (tm / kBM);
+  };
   const int kblocks = (K + kBK - 1) / kBK;
   if (N <= 64) pl.bn = 64;
-  else if (N <= 128) pl.bn = 128;
+  else if (N <= 128 || M <= 128) pl.bn = 128;
   int max_splits = max(1, kblocks / 8);
   // without enough k to split, narrower tiles are the only way to occupy more SMs
   while (pl.bn > 64 && tiles(pl.bn) * max_splits < kNumSMs) pl.bn /= 2;
@@ -488,8 +520,8 @@ Plan plan(int M, int N, int K) {
 template <int BN, bool kOuter>
 int launch(const Params& p, int tiles, cudaStream_t stream) {
   if (const int st = allow_smem<gemm32_kernel<BN, kOuter>>(Layout<BN>::kBytes); st != MXK_OK) return st;
-  mxk::launch_kernel(gemm32_kernel<BN, kOuter>, min(tiles, kNumSMs), Roles<BN, kOuter>::kThreads, Layout<BN>::kBytes, stream, p);
-  return launch_status();
+  return mxk::launch_kernel_clusters(gemm32_kernel<BN, kOuter>, Layout<BN>::kPair ? 2 : 1, min(tiles, kNumSMs), Roles<BN, kOuter>::kThreads,
+                                     Layout<BN>::kBytes, stream, p);
 }
 
 template <bool kOuter>
@@ -503,7 +535,8 @@ int run(Params& p, float* ws, size_t ws_bytes, int* partials, cudaStream_t strea
   p.ep_vec = p.ep.add ? vec_of(p.ep.add, p.ep.ld_add) : 1;
   p.a_wide = vec_of(p.a, p.lda) == 8;
   p.b_wide = kOuter && vec_of(p.b, p.ldb) == 8;
-  const int tiles = ((p.M + kBM - 1) / kBM) * ((p.N + pl.bn - 1) / pl.bn) * pl.splits;
+  const int tm = pl.bn == 256 ? 2 * kBM : kBM;
+  const int tiles = ((p.M + tm - 1) / tm) * ((p.N + pl.bn - 1) / pl.bn) * pl.splits * (tm / kBM);   // in CTAs
   const int st = pl.bn == 256   ? launch<256, kOuter>(p, tiles, stream)
                  : pl.bn == 128 ? launch<128, kOuter>(p, tiles, stream)
                                 : launch<64, kOuter>(p, tiles, stream);
@@ -562,10 +595,12 @@ __global__ void __launch_bounds__(256) split_weights_kernel(const __grid_constan
     x[e] = (n < jb.N && k + e < jb.K) ? (jb.transposed ? at(k + e, n) : at(n, k + e)) : 0.f;
   uint4 hi, mid, lo;
   split8(x, hi, mid, lo);
-  uint4* const dst = static_cast<uint4*>(jb.image) + (static_cast<size_t>(n_tile) * kb + k_block) * (3 * bn * 4) + kg * bn + n_in;
+  // a tile of 256 columns is cut into the halves that its two CTAs hold
+  const int cut = bn == 256 ? 128 : bn, part = n_tile * (bn / cut) + n_in / cut;
+  uint4* const dst = static_cast<uint4*>(jb.image) + (static_cast<size_t>(part) * kb + k_block) * (3 * cut * 4) + kg * cut + n_in % cut;
   dst[0] = hi;
-  dst[bn * 4] = mid;
-  dst[2 * bn * 4] = lo;
+  dst[cut * 4] = mid;
+  dst[2 * cut * 4] = lo;
 }
 
 }  // namespace

@@ -38,19 +38,27 @@ inline int allow_smem(int bytes) {
 // less between two small kernels).  Every kernel of this library begins with enter_kernel(), which waits for the kernels in
 // front before anything is read or written, so the order of effects on a stream is the usual one.
 template <typename... P, typename... A>
-inline int launch_kernel(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
+inline int launch_kernel_clusters(void (*kernel)(P...), unsigned cluster, dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                  A&&... args) {
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
   return launch_status();
+}
+template <typename... P, typename... A>
+inline int launch_kernel(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+  return launch_kernel_clusters(kernel, 1, grid, block, smem, stream, static_cast<A&&>(args)...);
 }
 
 // First statement of every kernel, executed by all threads.  A grid of at most two blocks per SM lets its successor's

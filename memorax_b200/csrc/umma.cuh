@@ -140,6 +140,59 @@ __device__ __forceinline__ void commit(uint64_t* bar) {
                : "memory");
 }
 
+// ---- cta_group::2: two CTAs of a cluster work on one M = 256 tile; each holds its 128 rows of A and of the accumulator and
+//      half of the rows of B.  Issued by the CTA of rank 0; descriptors are offsets that hold in both. ----
+__device__ __forceinline__ void mma_bf16_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
+                                              uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
+      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+template <int KSTEPS>
+__device__ __forceinline__ void gemm_pair(uint32_t tmem_d, const Operand& a, const Operand& b, uint32_t idesc, bool accumulate,
+                                          bool leader) {
+  const uint64_t da = a.desc(0), db = b.desc(0);
+  const uint32_t adv_a = a.advance(), adv_b = b.advance();
+#pragma unroll
+  for (int k = 0; k < KSTEPS; ++k) {
+    if (leader)
+      mma_bf16_pair(tmem_d, da + static_cast<uint64_t>(k * adv_a), db + static_cast<uint64_t>(k * adv_b), idesc,
+                    (accumulate || k > 0) ? 1u : 0u);
+  }
+}
+// Arrives on the barrier of this offset in both CTAs.
+__device__ __forceinline__ void commit_pair(uint64_t* bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+      "h"(static_cast<uint16_t>(3))
+      : "memory");
+}
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_slot, uint32_t columns) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_slot)), "r"(columns) : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t tmem, uint32_t columns) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(columns) : "memory");
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+}
+// Arrives on the barrier of this offset in the CTA of rank 0.
+__device__ __forceinline__ void arrive_at_leader(uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, 0;\n\t"
+      "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [ra];\n\t}\n" ::"r"(smem_u32(bar))
+      : "memory");
+}
+
 __device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 // Makes generic-proxy shared-memory writes visible to the tensor core (async proxy).
@@ -182,6 +235,20 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int li
 // drains in about a second instead of a second per wait.
 __device__ __forceinline__ void mbar_wait_flag(uint64_t* bar, uint32_t parity, bool& timed_out) {
   if (!mbar_wait(bar, parity, timed_out ? 1 : 1024)) timed_out = true;
+}
+
+// The same for a barrier that another CTA of the cluster arrives on.
+__device__ __forceinline__ void mbar_wait_cluster_flag(uint64_t* bar, uint32_t parity, bool& timed_out) {
+  uint32_t ok = 0;
+  const int limit = timed_out ? 1 : 1024;
+  for (int it = 0; it < limit && !ok; ++it) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(1000000u)
+        : "memory");
+  }
+  if (!ok) timed_out = true;
 }
 
 // ---- TMEM <-> registers (each thread: its own lane, 8 consecutive columns) ----

@@ -7,9 +7,10 @@ from oracle import memoroid_oracle as mo
 pytestmark = pytest.mark.gpu
 
 
-# edges of the 128 x {64,128,256} tiles and of the 32-deep stages, split contractions, unaligned rows
+# edges of the 128 x {64,128} and the paired 256 x 256 tiles and of the 32-deep stages, split contractions, accumulators
+# drained in between, unaligned rows
 @pytest.mark.parametrize("m,n,k", [(1, 1, 1), (127, 64, 31), (129, 65, 33), (257, 257, 100), (300, 776, 513), (128, 256, 4000),
-                                   (20000, 512, 96)])
+                                   (20000, 512, 96), (20001, 520, 300), (20000, 300, 1100)])
 def test_linear_f32_and_its_gradients_match_float64(m, n, k):
     from memorax_b200 import _C, ops
     g = torch.Generator("cuda").manual_seed(m + n + k)
