@@ -9,9 +9,12 @@
 // the conversion below writes 48, against 128 available, so shared memory binds a little before the pipe does.
 //
 // One persistent CTA per SM, warp-specialised:
-//   8 / 4 warps  epilogue: accumulators (TMEM) -> global, one row per thread, 32-byte stores
-//   8 / 12 warps producers: global float32 -> registers (a stage ahead) -> three bf16 planes in shared memory
-//   1 warp       issues the MMAs (12 per stage of 32 k)
+//   epilogue   accumulators (TMEM) -> global in whole lines, see to_lines()
+//   producers  global float32 -> registers (a stage ahead) -> three bf16 planes in shared memory
+//   1 warp     issues the MMAs (12 per stage of 32 k)
+// Eight warps each for the first two; where one CTA converts both operands alone, 12 producers and 4 epilogue warps.
+// Measured: 24000 x 1024 x 512 at 198 TFLOP/s, its weight gradient at 178 (167 when a pair had 16 producers and 4 epilogue
+// warps: the drains of long sums then held the pipe up).
 // Weights are split once, by split_weights, into images of the shared-memory stage, which arrive by one bulk copy per
 // stage: with both operands converted here the producers bound the kernel (127 TFLOP/s at 65536 x 1024 x 256).  A
 // gradient of a weight contracts two activations and converts both.
@@ -212,11 +215,32 @@ __device__ __forceinline__ void add8(float* p, int valid, int vec, const float* 
   }
 }
 
+// v: 32 consecutive columns of row `lane`.  Afterwards v[8 j ..] are columns 8 (lane & 3) .. + 7 of row (lane & 28) + j, so
+// that a store instruction writes whole 128-byte lines: with a row per lane it touched 32 lines for 32 bytes each, and a
+// 128 x 256 accumulator took 7.9 k cycles to drain instead of the 5 k that its bytes need.
+__device__ __forceinline__ void to_lines(float* v, int lane) {
+#pragma unroll
+  for (int o = 1; o <= 2; o <<= 1) {
+    const bool high = (lane & o) != 0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (u & o) continue;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {   // units u and u + o: keep one, trade the other
+        float &a = v[u * 8 + e], &b = v[(u + o) * 8 + e];
+        const float got = __shfl_xor_sync(0xffffffffu, high ? a : b, o);
+        a = high ? got : a;
+        b = high ? b : got;
+      }
+    }
+  }
+}
+
 // kOuter: C = A^T B, both operands contracted over their rows and converted here; else C = A W^T, W from its image.
 template <int BN, bool kOuter>
 struct Roles {
   // (a seventeenth warp is the last that leaves 96 registers a thread)
-  static constexpr int kProducerWarps = !kOuter ? 8 : (BN == 256 ? 16 : 12), kEpilogueWarps = kOuter ? 4 : 8;
+  static constexpr int kProducerWarps = !kOuter || BN == 256 ? 8 : 12, kEpilogueWarps = kOuter && BN != 256 ? 4 : 8;
   static constexpr int kMmaWarp = kProducerWarps + kEpilogueWarps;
   static constexpr int kThreads = 32 * (kMmaWarp + 1);
 };
@@ -395,12 +419,10 @@ __global__ void __launch_bounds__(Roles<BN, kOuter>::kThreads, 1) gemm32_kernel(
     for (int tile = first_tile; tile < tiles; tile += tile_step) {
       const int mn = tile % (mt * nt), sp = tile / (mt * nt);
       const int n0 = (mn % nt) * BN, m0 = (mn / nt) * kTileM + rank * kBM;
-      const int m = m0 + (warp & 3) * 32 + lane;
-      const bool in = m < p.M;
+      const int m = m0 + (warp & 3) * 32 + (lane & 28);   // first of the four rows this lane stores, see to_lines()
       const bool split = p.splits > 1;
-      float* const crow = split ? p.partial + (static_cast<size_t>(sp) * p.M + (in ? m : 0)) * p.N
-                                : p.c + static_cast<long long>(in ? m : 0) * p.ldc;
-      const float* const arow = (p.ep.add && !split) ? p.ep.add + static_cast<long long>(in ? m : 0) * p.ep.ld_add : nullptr;
+      float* const c0 = split ? p.partial + static_cast<size_t>(sp) * p.M * p.N : p.c;
+      const long long ldc = split ? p.N : p.ldc;
       const int k_len = min(p.K, (sp + 1) * p.k_split) - sp * p.k_split;
       for (int seg = 0; seg < k_len; seg += kSegment, ++turn) {
         const int buf = turn % L::kAccs;
@@ -411,31 +433,42 @@ __global__ void __launch_bounds__(Roles<BN, kOuter>::kThreads, 1) gemm32_kernel(
 #pragma unroll 1
         for (int c = (warp >> 2) * (BN / kColumnParts); c < ((warp >> 2) + 1) * (BN / kColumnParts); c += 32) {
           if (n0 + c >= p.N) break;
-          float v[32], w[32];
+          float v[32];
           __syncwarp();
           tmem_ld32(src + c, v);
-          tmem_ld32(src + BN + c, w);
-          tmem_ld_wait();
 #pragma unroll
-          for (int e = 0; e < 32; ++e) v[e] += w[e];
+          for (int h = 0; h < 32; h += 16) {
+            float w[16];
+            tmem_ld8(src + BN + c + h, w);
+            tmem_ld8(src + BN + c + h + 8, w + 8);
+            tmem_ld_wait();
 #pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            const int n = n0 + c + g * 8, valid = in ? p.N - n : 0;
+            for (int e = 0; e < 16; ++e) v[h + e] += w[e];
+          }
+          to_lines(v, lane);
+          const int n = n0 + c + (lane & 3) * 8;
+          float* dst = c0 + m * ldc + n;
+#pragma unroll
+          for (int j = 0; j < 4; ++j, dst += ldc) {
+            const int valid = m + j < p.M ? p.N - n : 0;
             if (valid <= 0) continue;
-            float ad[8];
-            if (last && !split && p.ep.bias) {
+            float* const x = v + j * 8;
+            if (last && !split) {
+              if (p.ep.bias) {
 #pragma unroll
-              for (int e = 0; e < 8; ++e)
-                if (e < valid) v[g * 8 + e] += __ldg(p.ep.bias + n + e);
-            }
-            if (last && arow) {
-              load8(arow + n, valid, p.ep_vec, ad);
+                for (int e = 0; e < 8; ++e)
+                  if (e < valid) x[e] += __ldg(p.ep.bias + n + e);
+              }
+              if (p.ep.add) {
+                float ad[8];
+                load8(p.ep.add + (m + j) * p.ep.ld_add + n, valid, p.ep_vec, ad);
 #pragma unroll
-              for (int e = 0; e < 8; ++e)
-                v[g * 8 + e] = fmaf(ad[e], (p.ep.add_scale && e < valid) ? __ldg(p.ep.add_scale + n + e) : 1.f, v[g * 8 + e]);
+                for (int e = 0; e < 8; ++e)
+                  x[e] = fmaf(ad[e], (p.ep.add_scale && e < valid) ? __ldg(p.ep.add_scale + n + e) : 1.f, x[e]);
+              }
             }
-            if (seg > 0) add8(crow + n, valid, p.c_vec, v + g * 8);   // to this thread's own earlier segments
-            else store8(crow + n, valid, p.c_vec, v + g * 8);
+            if (seg > 0) add8(dst, valid, p.c_vec, x);   // to this thread's own earlier segments
+            else store8(dst, valid, p.c_vec, x);
           }
         }
         fence_before_sync();
