@@ -1,4 +1,4 @@
-// Gated delta rule, forward, on the sm_100a tensor cores (math in gdelta_common.cuh).
+// Gated delta rule, forward, heads of 128, on the sm_100a tensor cores (math in gdelta_common.cuh; heads of 64: gdelta64.cu).
 //
 // One CTA (256 threads, two warpgroups) owns one (batch, head) sequence and walks its
 // 64-token chunks in order with the fp32 state S (128 x 128) resident in tensor memory;
@@ -14,6 +14,7 @@
 #include <cstddef>
 
 #include "attention.cuh"
+#include "gdelta64.cuh"
 #include "gdelta_common.cuh"
 #include "tma.cuh"
 
@@ -37,8 +38,6 @@ struct FwdParams {
   const uint4* tprime;        // T' of every chunk, written by the preparation kernel
   int* status;
   int B, T, H;
-  int d;                      // head dimension in memory: 128, or 64 (the upper half of every tile is then the
-                              // tensor maps' zero fill and the state's rows / columns 64..127 stay zero)
   CUtensorMap map_k, map_q, map_v;   // 64-token tiles as SW tiles (two 64-column blocks)
   CUtensorMap map_o;                 // 64-token tiles row-major
 };
@@ -113,7 +112,7 @@ __global__ void __launch_bounds__(kFwdThreads, 2) gdelta_fwd_kernel(const __grid
 
   // carried state: thread (v, wg) owns S[v][64 wg .. 64 wg + 63]
   {
-    const float* s0 = (p.s0 && vt < p.d && wg * 64 < p.d) ? p.s0 + (static_cast<size_t>(bh) * p.d + vt) * p.d + wg * 64 : nullptr;
+    const float* s0 = p.s0 ? p.s0 + (static_cast<size_t>(bh) * kD + vt) * kD + wg * 64 : nullptr;
     float vals[64];   // all loads first: the TMEM stores below are compiler memory barriers
 #pragma unroll
     for (int c4 = 0; c4 < 16; ++c4) {
@@ -155,11 +154,9 @@ __global__ void __launch_bounds__(kFwdThreads, 2) gdelta_fwd_kernel(const __grid
       tma::prefetch_plain_tile(&p.map_k, (cc + 1) * kC, h, b, 0);
       tma::prefetch_plain_tile(&p.map_q, (cc + 1) * kC, h, b, 0);
       tma::prefetch_plain_tile(&p.map_v, (cc + 1) * kC, h, b, 0);
-      if (p.d > 64) {
-        tma::prefetch_plain_tile(&p.map_k, (cc + 1) * kC, h, b, 64);
-        tma::prefetch_plain_tile(&p.map_q, (cc + 1) * kC, h, b, 64);
-        tma::prefetch_plain_tile(&p.map_v, (cc + 1) * kC, h, b, 64);
-      }
+      tma::prefetch_plain_tile(&p.map_k, (cc + 1) * kC, h, b, 64);
+      tma::prefetch_plain_tile(&p.map_q, (cc + 1) * kC, h, b, 64);
+      tma::prefetch_plain_tile(&p.map_v, (cc + 1) * kC, h, b, 64);
       tma::prefetch_bulk(p.tprime + (static_cast<size_t>(bh) * nchunks + cc + 1) * kAinvVecs, kAinvVecs * 16);
     }
   };
@@ -362,7 +359,7 @@ __global__ void __launch_bounds__(kFwdThreads, 2) gdelta_fwd_kernel(const __grid
 #pragma unroll
       for (int e = 0; e < 32; ++e) otile[(wg * 32 + e) * kD + vt] = __float2bfloat16(o[e]);
       const bool last = (c == nchunks - 1);
-      float* sl = (last && p.s_last && vt < p.d && wg * 64 < p.d) ? p.s_last + (static_cast<size_t>(bh) * p.d + vt) * p.d + wg * 64 : nullptr;
+      float* sl = (last && p.s_last) ? p.s_last + (static_cast<size_t>(bh) * kD + vt) * kD + wg * 64 : nullptr;
 #pragma unroll
       for (int c8 = 0; c8 < 8; ++c8) {
         sm.s[(wg * 8 + c8) * kD + vt] = pack8_bf16(st + c8 * 8);
@@ -415,6 +412,14 @@ int forward(const void* q, const void* k, const void* v, long long ld_v, const f
     if (ptr && !aligned16(ptr)) return MXK_ERR_ALIGN;
   if (!workspace || workspace_bytes < mxk_gdelta_workspace_bytes(B, T, H, d)) return MXK_ERR_WORKSPACE;
   if (!aligned16(workspace)) return MXK_ERR_ALIGN;
+  if (d == 64) {
+    heads64::Forward prm{alpha, s0, done, s_last, static_cast<uint4*>(chunk_states), static_cast<const uint4*>(workspace), status, T, H};
+    if (!tma::make_sw_map(&prm.map_k, k, B, T, H, kC) || !tma::make_sw_map(&prm.map_q, q, B, T, H, kC) ||
+        !tma::make_sw_map(&prm.map_v, v, B, T, H, kC, d, ld_v) || !tma::make_sw_map(&prm.map_o, o, B, T, H, kC))
+      return MXK_ERR_UNSUPPORTED;
+    const int st = launch_prep(k, alpha, beta, done, workspace, status, B, T, H, d, stream);
+    return st != MXK_OK ? st : heads64::launch_forward(prm, B * H, stream);
+  }
   FwdParams prm;
   prm.q = static_cast<const __nv_bfloat16*>(q);
   prm.k = static_cast<const __nv_bfloat16*>(k);
@@ -428,7 +433,7 @@ int forward(const void* q, const void* k, const void* v, long long ld_v, const f
   prm.chunk_states = static_cast<uint4*>(chunk_states);
   prm.tprime = static_cast<const uint4*>(workspace);
   prm.status = status;
-  prm.B = B; prm.T = T; prm.H = H; prm.d = d;
+  prm.B = B; prm.T = T; prm.H = H;
   if (!tma::make_sw_map(&prm.map_k, k, B, T, H, kC, d) || !tma::make_sw_map(&prm.map_q, q, B, T, H, kC, d) ||
       !tma::make_sw_map(&prm.map_v, v, B, T, H, kC, d, ld_v) || !tma::make_plain_map(&prm.map_o, o, B, T, H, d, kC, kD))
     return MXK_ERR_UNSUPPORTED;
@@ -449,7 +454,7 @@ extern "C" {
 size_t mxk_gdelta_chunk_states_bytes(int B, int T, int H, int d) {
   if (B <= 0 || T <= 0 || H <= 0 || (d != mxk::gdelta::kD && d != 64)) return 0;
   const size_t nchunks = (static_cast<size_t>(T) + mxk::gdelta::kC - 1) / mxk::gdelta::kC;
-  return static_cast<size_t>(B) * H * nchunks * mxk::gdelta::kResidualVecs * sizeof(uint4);
+  return static_cast<size_t>(B) * H * nchunks * (d == 64 ? mxk::gdelta::heads64::kResidualVecs64 : mxk::gdelta::kResidualVecs) * sizeof(uint4);
 }
 
 size_t mxk_gdelta_workspace_bytes(int B, int T, int H, int d) {

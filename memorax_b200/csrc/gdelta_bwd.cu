@@ -1,4 +1,4 @@
-// Gated delta rule, backward, on the sm_100a tensor cores.
+// Gated delta rule, backward, heads of 128, on the sm_100a tensor cores (heads of 64: gdelta64_bwd.cu).
 //
 // One CTA (256 threads) owns one (batch, head) sequence and walks its 64-token
 // chunks right to left with the fp32 cotangent of the state, dS (128 x 128),
@@ -20,6 +20,7 @@
 // owns one value column, as in the forward kernel; dQ and dK are accumulated transposed too
 // ([feature][token], M = 128 products: the full tensor datapath instead of half of it).
 #include "attention.cuh"
+#include "gdelta64.cuh"
 #include "gdelta_common.cuh"
 #include "tma.cuh"
 
@@ -48,7 +49,6 @@ struct BwdParams {
   float* ds0;
   int* status;
   int B, T, H;
-  int d;                              // head dimension in memory: 128, or 64 (see the forward kernel)
   CUtensorMap map_k, map_q, map_do;   // 64-token tiles as SW tiles (two 64-column blocks)
   CUtensorMap map_dq, map_dk;         // the same for the outputs
   CUtensorMap map_dv;                 // 64-token tiles row-major
@@ -145,11 +145,9 @@ __device__ __forceinline__ void issue_chunk_loads(BwdSmem& sm, const BwdParams& 
     tma::prefetch_plain_tile(&p.map_k, tp, h, b, 0);
     tma::prefetch_plain_tile(&p.map_q, tp, h, b, 0);
     tma::prefetch_plain_tile(&p.map_do, tp, h, b, 0);
-    if (p.d > 64) {
-      tma::prefetch_plain_tile(&p.map_k, tp, h, b, 64);
-      tma::prefetch_plain_tile(&p.map_q, tp, h, b, 64);
-      tma::prefetch_plain_tile(&p.map_do, tp, h, b, 64);
-    }
+    tma::prefetch_plain_tile(&p.map_k, tp, h, b, 64);
+    tma::prefetch_plain_tile(&p.map_q, tp, h, b, 64);
+    tma::prefetch_plain_tile(&p.map_do, tp, h, b, 64);
     tma::prefetch_bulk(src - kResidualVecs, kResidualVecs * 16);
     tma::prefetch_bulk(tp_src - kAinvVecs, kAinvVecs * 16);
   }
@@ -196,7 +194,7 @@ __global__ void __launch_bounds__(kBwdThreads) gdelta_bwd_kernel(const __grid_co
   linattn::DoneFlags flags_next = linattn::load_done_flags(drow, (nchunks - 1) * kC, p.T, lane);
   // cotangent of the next carry: thread (v, wg) owns dS[v][64 wg .. 64 wg + 63]
   {
-    const float* g0 = (p.ds_last && vt < p.d && wg * 64 < p.d) ? p.ds_last + (static_cast<size_t>(bh) * p.d + vt) * p.d + wg * 64 : nullptr;
+    const float* g0 = p.ds_last ? p.ds_last + (static_cast<size_t>(bh) * kD + vt) * kD + wg * 64 : nullptr;
     float vals[64];   // all loads first: the TMEM stores below are compiler memory barriers
 #pragma unroll
     for (int c4 = 0; c4 < 16; ++c4) {
@@ -575,7 +573,7 @@ __global__ void __launch_bounds__(kBwdThreads) gdelta_bwd_kernel(const __grid_co
           reinterpret_cast<__nv_bfloat16*>(&dk_stage[sw_slot(wg * 32 + e, vt >> 3)])[vt & 7] = __float2bfloat16(acc[e]);
       }
       const float g_last = sm.cd.g[kC - 1];
-      float* out0 = (c == 0 && p.ds0 && vt < p.d) ? p.ds0 + (static_cast<size_t>(bh) * p.d + vt) * p.d : nullptr;
+      float* out0 = (c == 0 && p.ds0) ? p.ds0 + (static_cast<size_t>(bh) * kD + vt) * kD : nullptr;
 #pragma unroll
       for (int q2 = 0; q2 < 2; ++q2) {
         const int q4 = wg * 2 + q2;
@@ -588,7 +586,7 @@ __global__ void __launch_bounds__(kBwdThreads) gdelta_bwd_kernel(const __grid_co
         for (int c8 = 0; c8 < 4; ++c8) {
           tmem_st8(lane_base + kColDS + q4 * 32 + c8 * 8, s + c8 * 8);
           sm.ds[(q4 * 4 + c8) * kD + vt] = pack8_bf16(s + c8 * 8);
-          if (out0 && q4 * 32 < p.d) {
+          if (out0) {
             *reinterpret_cast<float4*>(out0 + q4 * 32 + c8 * 8) = make_float4(s[c8 * 8], s[c8 * 8 + 1], s[c8 * 8 + 2], s[c8 * 8 + 3]);
             *reinterpret_cast<float4*>(out0 + q4 * 32 + c8 * 8 + 4) = make_float4(s[c8 * 8 + 4], s[c8 * 8 + 5], s[c8 * 8 + 6], s[c8 * 8 + 7]);
           }
@@ -602,10 +600,8 @@ __global__ void __launch_bounds__(kBwdThreads) gdelta_bwd_kernel(const __grid_co
     if (tid == 0) {
       tma::store_plain_tile(&p.map_dq, sm.r1, t0, h, b, 0);
       tma::store_plain_tile(&p.map_dk, sm.lt, t0, h, b, 0);
-      if (p.d > 64) {   // a 64-wide head has no second column block in memory
-        tma::store_plain_tile(&p.map_dq, sm.r1 + kSwBlockVecs, t0, h, b, 64);
-        tma::store_plain_tile(&p.map_dk, reinterpret_cast<uint4*>(sm.lt) + kSwBlockVecs, t0, h, b, 64);
-      }
+      tma::store_plain_tile(&p.map_dq, sm.r1 + kSwBlockVecs, t0, h, b, 64);
+      tma::store_plain_tile(&p.map_dk, reinterpret_cast<uint4*>(sm.lt) + kSwBlockVecs, t0, h, b, 64);
       tma::commit_group();
     }
   }
@@ -652,6 +648,15 @@ int backward(const void* q, const void* k, const void* v, const float* alpha, co
   for (const void* ptr : {q, k, v, d_o, chunk_states, workspace, (const void*)dq, (const void*)dk, (const void*)dv,
                           (const void*)ds_last, (const void*)ds0})
     if (ptr && !aligned16(ptr)) return MXK_ERR_ALIGN;
+  if (d == 64) {
+    heads64::Backward prm{alpha, beta, done, static_cast<const uint4*>(chunk_states), static_cast<const uint4*>(workspace), ds_last, dalpha,
+                          dbeta, ds0, status, T, H};
+    if (!tma::make_sw_map(&prm.map_k, k, B, T, H, kC) || !tma::make_sw_map(&prm.map_q, q, B, T, H, kC) ||
+        !tma::make_sw_map(&prm.map_do, d_o, B, T, H, kC) || !tma::make_sw_map(&prm.map_dq, dq, B, T, H, kC) ||
+        !tma::make_sw_map(&prm.map_dk, dk, B, T, H, kC) || !tma::make_sw_map(&prm.map_dv, dv, B, T, H, kC, d, ld_dv))
+      return MXK_ERR_UNSUPPORTED;
+    return heads64::launch_backward(prm, B * H, stream);
+  }
   BwdParams prm;
   prm.q = static_cast<const __nv_bfloat16*>(q);
   prm.k = static_cast<const __nv_bfloat16*>(k);
@@ -670,7 +675,7 @@ int backward(const void* q, const void* k, const void* v, const float* alpha, co
   prm.dbeta = dbeta;
   prm.ds0 = ds0;
   prm.status = status;
-  prm.B = B; prm.T = T; prm.H = H; prm.d = d;
+  prm.B = B; prm.T = T; prm.H = H;
   prm.phase_cycles = nullptr;
   if (g_gd_phase_on) {
     void* sym = nullptr;
