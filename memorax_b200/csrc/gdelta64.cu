@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(kThreads64, 3) gdelta64_fwd_kernel(const __gri
     fence_after_sync();
 
     {
-      const int lo = row_first_key(dm, me.row);
+      const uint32_t seen = keys_seen(dm, me.row, me.c0);
       const float cum_t = sm.cum[me.row], gt = sm.g[me.row], gm = sm.gam[me.row];
       float qk[16], y[16];
       load16(me.tmem + kQK, qk);
@@ -127,8 +127,7 @@ __global__ void __launch_bounds__(kThreads64, 3) gdelta64_fwd_kernel(const __gri
       tmem_ld_wait();
 #pragma unroll
       for (int e = 0; e < 16; ++e) {
-        const int j = me.c0 + e;
-        qk[e] = (j >= lo && j <= me.row) ? __expf(cum_t - sm.cum[j]) * qk[e] : 0.f;
+        qk[e] *= decay_between(cum_t, sm.cum[me.c0 + e], seen, e);
         y[e] *= -gt;
       }
 #pragma unroll

@@ -77,8 +77,8 @@ __device__ __forceinline__ Gates load_gates(const float* alpha, const float* bet
   }
   return g;
 }
-// cum, g and gam of a chunk, by one warp.
-__device__ __forceinline__ void chunk_decay(const Gates& ga, uint64_t dm, int lane, float* cum, float* g, float* gam) {
+// cum of tokens 2 lane, 2 lane + 1, by one warp.
+__device__ __forceinline__ float2 cumulative(const Gates& ga, int lane) {
   const float l1 = __logf(ga.a[1]);
   float s = __logf(ga.a[0]) + l1;
 #pragma unroll
@@ -86,11 +86,16 @@ __device__ __forceinline__ void chunk_decay(const Gates& ga, uint64_t dm, int la
     const float o = __shfl_up_sync(0xffffffffu, s, off);
     if (lane >= off) s += o;
   }
-  const float last = __shfl_sync(0xffffffffu, s, 31);
+  return make_float2(s - l1, s);
+}
+// cum, g and gam of a chunk, by one warp.
+__device__ __forceinline__ void chunk_decay(const Gates& ga, uint64_t dm, int lane, float* cum, float* g, float* gam) {
+  const float2 s = cumulative(ga, lane);
+  const float last = __shfl_sync(0xffffffffu, s.y, 31);
 #pragma unroll
   for (int e = 0; e < 2; ++e) {
     const int t = 2 * lane + e;
-    const float c = e ? s : s - l1;
+    const float c = e ? s.y : s.x;
     cum[t] = c;
     g[t] = row_live(dm, t) ? __expf(c) : 0.f;
     gam[t] = row_keep(dm, t) ? __expf(last - c) : 0.f;

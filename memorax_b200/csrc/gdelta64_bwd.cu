@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(kThreads64, 2) gdelta64_bwd_kernel(const __gri
     fence_after_sync();
 
     // ---- epilogue A ----
-    const int lo = row_first_key(dm, me.row);
+    const uint32_t seen = keys_seen(dm, me.row, me.c0);
     const float cum_t = sm.cum[me.row], gt = sm.g[me.row], gm = sm.gam[me.row];
     float dg = 0.f;
     {
@@ -149,10 +149,7 @@ __global__ void __launch_bounds__(kThreads64, 2) gdelta64_bwd_kernel(const __gri
       load16(me.tmem + kOI, oi);
       tmem_ld_wait();
 #pragma unroll
-      for (int e = 0; e < 16; ++e) {
-        const int j = me.c0 + e;
-        qk[e] = (j >= lo && j <= me.row) ? __expf(cum_t - sm.cum[j]) * qk[e] : 0.f;
-      }
+      for (int e = 0; e < 16; ++e) qk[e] *= decay_between(cum_t, sm.cum[me.c0 + e], seen, e);
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         sm.p[(me.ch + i) * kC + me.row] = pack8_bf16(qk + 8 * i);
@@ -303,7 +300,7 @@ __global__ void __launch_bounds__(kThreads64, 2) gdelta64_bwd_kernel(const __gri
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
           const int j = me.c0 + 8 * i + e;
-          const float gtj = (j >= lo && j <= me.row) ? __expf(cum_t - sm.cum[j]) : 0.f;
+          const float gtj = decay_between(cum_t, sm.cum[j], seen, 8 * i + e);
           const float dl = j < me.row ? -w[e] : 0.f;
           ev[8 * i + e] = (x[e] * qk[e] + dl * kk[e]) * gtj;
           rs += ev[8 * i + e];

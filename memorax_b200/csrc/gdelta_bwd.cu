@@ -267,9 +267,9 @@ __global__ void __launch_bounds__(kBwdThreads) gdelta_bwd_kernel(const __grid_co
 
     // ---- epilogue A1: tril(G o QK^T) (bf16); every thread owns 16 keys of its token row ----
     {
-      const int lo = row_first_key(dm, row);
       const float cum_t = sm.cd.cum[row];
       const int j0 = (upper ? 32 : 0) + wg * 16;
+      const uint32_t seen = keys_seen(dm, row, j0);
       float qk[16];
       tmem_ld_row<16>(lane_base + kColQK + wg * 16, qk);
 #pragma unroll
@@ -277,9 +277,8 @@ __global__ void __launch_bounds__(kBwdThreads) gdelta_bwd_kernel(const __grid_co
         float pm[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-          const int x = jq * 8 + e, j = j0 + x;
-          const bool in = (j >= lo && j <= row);
-          pm[e] = in ? __expf(cum_t - sm.cd.cum[j]) * qk[x] : 0.f;
+          const int x = jq * 8 + e;
+          pm[e] = decay_between(cum_t, sm.cd.cum[j0 + x], seen, x) * qk[x];
         }
         sm.p[((j0 >> 3) + jq) * kC + row] = pack8_bf16(pm);
       }
@@ -424,9 +423,9 @@ __global__ void __launch_bounds__(kBwdThreads) gdelta_bwd_kernel(const __grid_co
     {
       uint4* dpg = reinterpret_cast<uint4*>(sm.lt);           // [j/8][t][8]
       uint4* dlg = dpg + kPanC * kC;
-      const int lo = row_first_key(dm, row);
       const float cum_t = sm.cd.cum[row], beta_t = sm.cd.beta[row];
       const int j0 = (upper ? 32 : 0) + wg * 16;
+      const uint32_t seen = keys_seen(dm, row, j0);
       float rs = 0.f, wtt = 0.f;
       float kk[16], qk[16], dp[16], w[16];
       tmem_ld_row<16>(lane_base + kColKK + wg * 16, kk);
@@ -440,8 +439,7 @@ __global__ void __launch_bounds__(kBwdThreads) gdelta_bwd_kernel(const __grid_co
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
           const int x = jq * 8 + e, j = j0 + x;
-          const bool in = (j >= lo && j <= row);
-          const float gtj = in ? __expf(cum_t - sm.cd.cum[j]) : 0.f;
+          const float gtj = decay_between(cum_t, sm.cd.cum[j], seen, x);
           const float dl = (j < row) ? -w[x] : 0.f;
           wtt = (j == row) ? w[x] : wtt;   // the diagonal of W', held by exactly one thread per row
           a8[e] = dp[x] * gtj;

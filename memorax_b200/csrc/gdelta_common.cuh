@@ -53,6 +53,15 @@ __device__ __forceinline__ float sw_bf16_at(const uint4* tile, int t, int c) {
   return __bfloat162float(p[c & 7]);
 }
 
+// Bit e: key j0 + e is one that token `row` of a chunk sees (no reset in between), up to itself.
+__device__ __forceinline__ uint32_t keys_seen(uint64_t dm, int row, int j0) {
+  return static_cast<uint32_t>(((2ull << row) - (1ull << row_first_key(dm, row))) >> j0);
+}
+// G_tj = exp(cum_t - cum_j) where bit e is set, 0 elsewhere; selected before the exponential, which a branch would skip.
+__device__ __forceinline__ float decay_between(float cum_t, float cum_j, uint32_t seen, int e) {
+  return __expf((seen >> e) & 1u ? cum_t - cum_j : -INFINITY);
+}
+
 struct ChunkDecay {
   float alpha[kC], beta[kC], cum[kC], g[kC], gam[kC];
 };
@@ -104,59 +113,6 @@ __device__ __forceinline__ void chunk_decay_from_regs(ChunkDecay& cd, float2 ab,
 __device__ __forceinline__ float bf16_at(const uint4* plain, int t, int c) {
   const __nv_bfloat16* p = reinterpret_cast<const __nv_bfloat16*>(plain);
   return __bfloat162float(p[t * kD + c]);
-}
-
-// Unit-triangular solves, one independent column per thread, on packed fp32
-// pairs (fma.rn.f32x2): r2[i] = (r[2i], r[2i+1]).
-//
-// forward_substitute: r holds the right-hand side on entry and the solution of
-// (I + diag(beta) L) u = r on exit; nlt[j * 64 + t] = -beta_t L_tj (zero for t <= j).
-// The template form eliminates columns J0 .. J1 - 1 from rows < T1 only, so that a solve
-// can be blocked: rows 0..31 first (<0, 31, 32>), then -- once the 32 x 32 off-diagonal
-// block times the first half has been added to rows 32..63 -- the rest (<32, 63, 64>).
-template <int J0, int J1, int T1>
-__device__ __forceinline__ void forward_substitute_range(float2* r2, const float* nlt) {
-  const float4* lt4 = reinterpret_cast<const float4*>(nlt);
-#pragma unroll
-  for (int j = J0; j < J1; ++j) {
-    const float uj = (j & 1) ? r2[j >> 1].y : r2[j >> 1].x;
-    const float2 u2 = make_float2(uj, uj);
-#pragma unroll
-    for (int m = (j + 1) / 4; m < T1 / 4; ++m) {
-      const float4 l = lt4[j * (kC / 4) + m];
-      r2[2 * m] = __ffma2_rn(make_float2(l.x, l.y), u2, r2[2 * m]);
-      r2[2 * m + 1] = __ffma2_rn(make_float2(l.z, l.w), u2, r2[2 * m + 1]);
-    }
-  }
-}
-__device__ __forceinline__ void forward_substitute(float2* r2, const float* nlt) {
-  forward_substitute_range<0, kC - 1, kC>(r2, nlt);
-}
-
-// backward_substitute: r holds dU on entry and (I + diag(beta) L)^-T dU on exit;
-// nl[i * kStride + t] = -beta_i L_it (zero for t >= i), kStride a multiple of 4.
-// The range form eliminates rows I1 down to I0 from the entries t >= T0 only (T0 a multiple of 4),
-// so that the solve can be blocked like the forward one: rows 63..33 over entries 32.. first
-// (<63, 33, 32>), then -- once the off-diagonal block times the second half has been added to
-// entries 0..31 -- rows 31..1 (<31, 1, 0>).
-template <int kStride, int I1, int I0, int T0>
-__device__ __forceinline__ void backward_substitute_range(float2* r2, const float* nl) {
-  const float4* l4 = reinterpret_cast<const float4*>(nl);
-#pragma unroll
-  for (int i = I1; i >= I0; --i) {
-    const float xi = (i & 1) ? r2[i >> 1].y : r2[i >> 1].x;
-    const float2 x2 = make_float2(xi, xi);
-#pragma unroll
-    for (int m = T0 / 4; m <= (i - 1) / 4; ++m) {
-      const float4 c = l4[i * (kStride / 4) + m];
-      r2[2 * m] = __ffma2_rn(make_float2(c.x, c.y), x2, r2[2 * m]);
-      r2[2 * m + 1] = __ffma2_rn(make_float2(c.z, c.w), x2, r2[2 * m + 1]);
-    }
-  }
-}
-template <int kStride>
-__device__ __forceinline__ void backward_substitute(float2* r2, const float* nl) {
-  backward_substitute_range<kStride, kC - 1, 1, 0>(r2, nl);
 }
 
 }  // namespace gdelta
