@@ -205,19 +205,26 @@ __global__ void __launch_bounds__(kThreads, 1) gemm16_kernel(const __grid_consta
   if (warp == 1) tmem_dealloc(tmem, 2 * BN);
 }
 
+// Eight threads an element, each with every eighth split and eight of those loads in flight; their sums are added in a fixed
+// order.  (One thread an element took 18 to 32 us for the 37 to 74 splits of a narrow weight gradient.)
 __global__ void __launch_bounds__(256) reduce_splits_kernel(const float* __restrict__ partial, int splits, long long all, int M, int N,
                                                             const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ c,
                                                             long long ldc, long long c_batch_stride, bool accumulate) {
   enter_kernel();
-  const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
-  if (i >= all) return;
-  float s[4] = {0.f, 0.f, 0.f, 0.f};
-  int k = 0;
-  for (; k + 4 <= splits; k += 4)
+  __shared__ float red[8][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const long long i = static_cast<long long>(blockIdx.x) * 32 + tx;
+  float s = 0.f;
+  if (i < all) {
+#pragma unroll 8
+    for (int k = ty; k < splits; k += 8) s += partial[k * all + i];
+  }
+  red[ty][tx] = s;
+  __syncthreads();
+  if (ty != 0 || i >= all) return;
+  float v = red[0][tx];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) s[u] += partial[(k + u) * all + i];
-  for (; k < splits; ++k) s[0] += partial[k * all + i];
-  float v = (s[0] + s[1]) + (s[2] + s[3]);
+  for (int k = 1; k < 8; ++k) v += red[k][tx];
   const int n = static_cast<int>(i % N);
   const long long row = i / N;
   __nv_bfloat16* const dst = c + row / M * c_batch_stride + row % M * ldc + n;
@@ -301,7 +308,7 @@ int run(const Matrix& a, bool a_rows, const Matrix& b, bool b_rows, const void* 
   const int st = pl.bn == 128 ? launch_bn<128>(p, a_rows, b_rows, stream) : launch_bn<64>(p, a_rows, b_rows, stream);
   if (st != MXK_OK || pl.splits == 1) return st;
   const long long all = static_cast<long long>(batch) * M * N;
-  mxk::launch_kernel(reduce_splits_kernel, static_cast<unsigned>((all + 255) / 256), 256, 0, stream, p.partial, pl.splits, all, M, N, p.bias, p.c, ldc,
+  mxk::launch_kernel(reduce_splits_kernel, static_cast<unsigned>((all + 31) / 32), 256, 0, stream, p.partial, pl.splits, all, M, N, p.bias, p.c, ldc,
                                                                                      c_batch_stride, accumulate);
   return launch_status();
 }

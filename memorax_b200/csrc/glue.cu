@@ -144,17 +144,20 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
   }
 }
 
-// Adds the per-block partial rows in a fixed order: a block owns 32 columns, its eight thread rows each add
-// every eighth partial, then thread row 0 adds the eight sums in order.
-__global__ void __launch_bounds__(256)
+// Adds the per-block partial rows in a fixed order: a block owns 32 columns, its 32 thread rows each add every 32nd
+// partial, then thread row 0 adds the 32 sums in order.  (The loads come from other SMs' writes, most of a microsecond each:
+// eight thread rows took 30 to 40 us for 296 partials.)
+constexpr int kReduceRows = 32;
+__global__ void __launch_bounds__(32 * kReduceRows)
 norm_bwd_reduce_kernel(const float* __restrict__ part, float* __restrict__ dgamma, float* __restrict__ dbeta, int blocks, int D) {
   enter_kernel();
-  __shared__ float red[2][8][33];
+  __shared__ float red[2][kReduceRows][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + tx;
   float sg = 0.f, sb = 0.f;
   if (c < D) {
-    for (int b = ty; b < blocks; b += 8) {
+#pragma unroll 5
+    for (int b = ty; b < blocks; b += kReduceRows) {
       sg += part[(static_cast<size_t>(b) * 2) * D + c];
       if (dbeta) sb += part[(static_cast<size_t>(b) * 2 + 1) * D + c];
     }
@@ -165,7 +168,7 @@ norm_bwd_reduce_kernel(const float* __restrict__ part, float* __restrict__ dgamm
   if (ty == 0 && c < D) {
     float tg = red[0][0][tx], tb = red[1][0][tx];
 #pragma unroll
-    for (int i = 1; i < 8; ++i) { tg += red[0][i][tx]; tb += red[1][i][tx]; }
+    for (int i = 1; i < kReduceRows; ++i) { tg += red[0][i][tx]; tb += red[1][i][tx]; }
     dgamma[c] = tg;
     if (dbeta) dbeta[c] = tb;
   }
@@ -458,7 +461,7 @@ int mxk_norm_bf16_bwd(const void* x, const void* gamma, const float* mean, const
   }
 #undef MXK_NORM_BWD
   if (int st = launch_status()) return st;
-  mxk::launch_kernel(norm_bwd_reduce_kernel, (D + 31) / 32, 256, 0, s, part, dgamma, rms ? nullptr : dbeta, blocks, D);
+  mxk::launch_kernel(norm_bwd_reduce_kernel, (D + 31) / 32, 32 * kReduceRows, 0, s, part, dgamma, rms ? nullptr : dbeta, blocks, D);
   return launch_status();
 }
 
