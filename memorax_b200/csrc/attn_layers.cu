@@ -255,31 +255,63 @@ __global__ void __launch_bounds__(kStepThreads) gdelta_step_kernel(const __nv_bf
 }
 
 // ------------------------------------------------------------------------------------- delta rule: inputs, gates
-// HBM-bound.  LPH lanes hold one head vector, 16 bytes each; the blocks past the vectors take the gates.
+// HBM-bound.  LPH lanes hold one head vector, 16 bytes each; the first blocks take the gates, whose loads are few and slow
+// (after the vectors they were a tail of their own).  A thread walks over kWalk vectors at a time, all loaded before the
+// first is used, and divides only once: a 64-bit division per vector took as long as its 16 bytes.
+constexpr int kWalk = 4;
+struct Walk {   // vector i of the q and k columns is (token, column) = (i / width, i % width)
+  long long tok;
+  int c, width, dtok, dc;
+  __device__ __forceinline__ Walk(unsigned block, unsigned blocks, int w) : width(w) {
+    const long long i = static_cast<long long>(block) * 256 + threadIdx.x, step = static_cast<long long>(blocks) * 256;
+    tok = i / w;
+    c = static_cast<int>(i % w);
+    dtok = static_cast<int>(step / w);
+    dc = static_cast<int>(step % w);
+  }
+  __device__ __forceinline__ void next() {
+    tok += dtok;
+    c += dc;
+    if (c >= width) { c -= width; ++tok; }
+  }
+};
+
 template <int LPH>
 __global__ void __launch_bounds__(256) delta_inputs_kernel(const __nv_bfloat16* __restrict__ qkvg, long long ld,
                                                            const __nv_bfloat16* __restrict__ gate_bias, uint4* __restrict__ q,
                                                            uint4* __restrict__ k, float* __restrict__ alpha,
-                                                           float* __restrict__ beta, long long tokens, int H, unsigned vec_blocks) {
+                                                           float* __restrict__ beta, long long tokens, int H, unsigned gate_blocks) {
   enter_kernel();
   const int hid8 = H * LPH;
-  if (blockIdx.x < vec_blocks) {
-    const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
-    const long long tok = i / (2 * hid8);
-    const int c = static_cast<int>(i % (2 * hid8));
-    float x[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    if (tok < tokens) unpack8_bf16(ld_stream(reinterpret_cast<const uint4*>(qkvg + tok * ld + c * 8)), x);
-    float ss = 0.f;
+  if (blockIdx.x >= gate_blocks) {
+    Walk w(blockIdx.x - gate_blocks, gridDim.x - gate_blocks, 2 * hid8);
+    // (of a warp's lanes the first is the last to run out)
+    while (__shfl_sync(0xffffffffu, w.tok, 0) < tokens) {
+      uint4 raw[kWalk];
+      uint4* dst[kWalk];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) ss = fmaf(x[e], x[e], ss);
+      for (int u = 0; u < kWalk; ++u) {
+        const bool in = w.tok < tokens;
+        raw[u] = in ? ld_stream(reinterpret_cast<const uint4*>(qkvg + w.tok * ld + w.c * 8)) : make_uint4(0, 0, 0, 0);
+        dst[u] = in ? (w.c < hid8 ? q : k) + w.tok * hid8 + (w.c < hid8 ? w.c : w.c - hid8) : nullptr;
+        w.next();
+      }
 #pragma unroll
-    for (int off = 1; off < LPH; off <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
-    const float inv = 1.f / fmaxf(sqrtf(ss), 1e-12f);
+      for (int u = 0; u < kWalk; ++u) {
+        float x[8], ss = 0.f;
+        unpack8_bf16(raw[u], x);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) x[e] *= inv;
-    if (tok < tokens) (c < hid8 ? q : k)[tok * hid8 + (c < hid8 ? c : c - hid8)] = pack8_bf16(x);
+        for (int e = 0; e < 8; ++e) ss = fmaf(x[e], x[e], ss);
+#pragma unroll
+        for (int off = 1; off < LPH; off <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+        const float inv = 1.f / fmaxf(sqrtf(ss), 1e-12f);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[e] *= inv;
+        if (dst[u]) *dst[u] = pack8_bf16(x);
+      }
+    }
   } else {
-    const long long i = static_cast<long long>(blockIdx.x - vec_blocks) * 256 + threadIdx.x;
+    const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
     if (i >= tokens * H) return;
     const long long tok = i / H;
     const int h = static_cast<int>(i % H);
@@ -295,39 +327,51 @@ __global__ void __launch_bounds__(256) delta_inputs_bwd_kernel(const __nv_bfloat
                                                                const uint4* __restrict__ dq, const uint4* __restrict__ dk,
                                                                const float* __restrict__ dalpha, const float* __restrict__ dbeta,
                                                                __nv_bfloat16* __restrict__ g, float* __restrict__ partial,
-                                                               long long tokens, int H, unsigned vec_blocks) {
+                                                               long long tokens, int H, unsigned gate_blocks) {
   enter_kernel();
   __shared__ float red[256];
   const int hid8 = H * LPH, hid = hid8 * 8;
-  if (blockIdx.x < vec_blocks) {
-    const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
-    const long long tok = i / (2 * hid8);
-    const int c = static_cast<int>(i % (2 * hid8));
-    float x[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, d[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    if (tok < tokens) {
-      unpack8_bf16(ld_stream(reinterpret_cast<const uint4*>(qkvg + tok * ld + c * 8)), x);
-      unpack8_bf16(ld_stream((c < hid8 ? dq : dk) + tok * hid8 + (c < hid8 ? c : c - hid8)), d);
+  if (blockIdx.x >= gate_blocks) {
+    Walk w(blockIdx.x - gate_blocks, gridDim.x - gate_blocks, 2 * hid8);
+    while (__shfl_sync(0xffffffffu, w.tok, 0) < tokens) {
+      uint4 xr[kWalk], dr[kWalk];
+      uint4* dst[kWalk];
+#pragma unroll
+      for (int u = 0; u < kWalk; ++u) {
+        const bool in = w.tok < tokens;
+        const long long at = w.tok * ld + w.c * 8;
+        xr[u] = in ? ld_stream(reinterpret_cast<const uint4*>(qkvg + at)) : make_uint4(0, 0, 0, 0);
+        dr[u] = in ? ld_stream((w.c < hid8 ? dq : dk) + w.tok * hid8 + (w.c < hid8 ? w.c : w.c - hid8)) : make_uint4(0, 0, 0, 0);
+        dst[u] = in ? reinterpret_cast<uint4*>(g + at) : nullptr;
+        w.next();
+      }
+#pragma unroll
+      for (int u = 0; u < kWalk; ++u) {
+        float x[8], d[8], ss = 0.f, sd = 0.f;
+        unpack8_bf16(xr[u], x);
+        unpack8_bf16(dr[u], d);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) { ss = fmaf(x[e], x[e], ss); sd = fmaf(x[e], d[e], sd); }
+#pragma unroll
+        for (int off = 1; off < LPH; off <<= 1) {
+          ss += __shfl_xor_sync(0xffffffffu, ss, off);
+          sd += __shfl_xor_sync(0xffffffffu, sd, off);
+        }
+        const float inv = 1.f / fmaxf(sqrtf(ss), 1e-12f), ydy = sd * inv;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[e] = inv * (d[e] - x[e] * inv * ydy);
+        if (dst[u]) *dst[u] = pack8_bf16(x);
+      }
     }
-    float ss = 0.f, sd = 0.f;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) { ss = fmaf(x[e], x[e], ss); sd = fmaf(x[e], d[e], sd); }
-#pragma unroll
-    for (int off = 1; off < LPH; off <<= 1) {
-      ss += __shfl_xor_sync(0xffffffffu, ss, off);
-      sd += __shfl_xor_sync(0xffffffffu, sd, off);
-    }
-    const float inv = 1.f / fmaxf(sqrtf(ss), 1e-12f), ydy = sd * inv;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) x[e] = inv * (d[e] - x[e] * inv * ydy);
-    if (tok < tokens) *reinterpret_cast<uint4*>(g + tok * ld + c * 8) = pack8_bf16(x);
     return;
   }
   // gates: columns 0..H-1 beta, H..2H-1 decay, then the padding
   const int cols = static_cast<int>(ld) - 3 * hid, per = 256 / cols;
   const int c = threadIdx.x % cols, ro = threadIdx.x / cols;
-  const unsigned blocks = gridDim.x - vec_blocks, blk = blockIdx.x - vec_blocks;
+  const unsigned blocks = gate_blocks, blk = blockIdx.x;
   float sum = 0.f;
   if (ro < per)
+#pragma unroll 4
     for (long long tok = static_cast<long long>(blk) * per + ro; tok < tokens; tok += static_cast<long long>(blocks) * per) {
       float v = 0.f;
       if (c < 2 * H) {
@@ -347,6 +391,10 @@ __global__ void __launch_bounds__(256) delta_inputs_bwd_kernel(const __nv_bfloat
 }
 
 constexpr int kGateBlocks = 2 * kNumSMs;
+unsigned walk_blocks(long long vecs) {   // a wave of eight blocks an SM
+  const long long need = (vecs + 256 * kWalk - 1) / (256 * kWalk);
+  return static_cast<unsigned>(need < 8 * kNumSMs ? need : 8 * kNumSMs);
+}
 
 }  // namespace
 
@@ -395,11 +443,11 @@ int gdelta_step(const void* qkvg, long long ld, const void* gate_bias, const flo
 int delta_inputs(const void* qkvg, long long ld, const void* gate_bias, void* q, void* k, float* alpha, float* beta,
                  long long tokens, int H, int d, cudaStream_t stream) {
   const long long vecs = tokens * 2 * H * (d / 8);
-  const unsigned vb = static_cast<unsigned>((vecs + 255) / 256), gb = static_cast<unsigned>((tokens * H + 255) / 256);
+  const unsigned vb = walk_blocks(vecs), gb = static_cast<unsigned>((tokens * H + 255) / 256);
   const auto* x = static_cast<const __nv_bfloat16*>(qkvg);
   const auto* bias = static_cast<const __nv_bfloat16*>(gate_bias);
-  if (d == 64) mxk::launch_kernel(delta_inputs_kernel<8>, vb + gb, 256, 0, stream, x, ld, bias, static_cast<uint4*>(q), static_cast<uint4*>(k), alpha, beta, tokens, H, vb);
-  else if (d == 128) mxk::launch_kernel(delta_inputs_kernel<16>, vb + gb, 256, 0, stream, x, ld, bias, static_cast<uint4*>(q), static_cast<uint4*>(k), alpha, beta, tokens, H, vb);
+  if (d == 64) mxk::launch_kernel(delta_inputs_kernel<8>, vb + gb, 256, 0, stream, x, ld, bias, static_cast<uint4*>(q), static_cast<uint4*>(k), alpha, beta, tokens, H, gb);
+  else if (d == 128) mxk::launch_kernel(delta_inputs_kernel<16>, vb + gb, 256, 0, stream, x, ld, bias, static_cast<uint4*>(q), static_cast<uint4*>(k), alpha, beta, tokens, H, gb);
   else return MXK_ERR_UNSUPPORTED;
   return launch_status();
 }
@@ -413,12 +461,12 @@ int delta_inputs_bwd(const void* qkvg, long long ld, const void* gate_bias, cons
                      const float* dbeta, void* g, float* partial, long long tokens, int H, int d, cudaStream_t stream) {
   if (ld - 3 * H * d > 256 || ld - 3 * H * d < 2 * H) return MXK_ERR_UNSUPPORTED;
   const long long vecs = tokens * 2 * H * (d / 8);
-  const unsigned vb = static_cast<unsigned>((vecs + 255) / 256), gb = static_cast<unsigned>(delta_gate_blocks(tokens));
+  const unsigned vb = walk_blocks(vecs), gb = static_cast<unsigned>(delta_gate_blocks(tokens));
   const auto* x = static_cast<const __nv_bfloat16*>(qkvg);
   const auto* bias = static_cast<const __nv_bfloat16*>(gate_bias);
   auto* out = static_cast<__nv_bfloat16*>(g);
-  if (d == 64) mxk::launch_kernel(delta_inputs_bwd_kernel<8>, vb + gb, 256, 0, stream, x, ld, bias, static_cast<const uint4*>(dq), static_cast<const uint4*>(dk), dalpha, dbeta, out, partial, tokens, H, vb);
-  else if (d == 128) mxk::launch_kernel(delta_inputs_bwd_kernel<16>, vb + gb, 256, 0, stream, x, ld, bias, static_cast<const uint4*>(dq), static_cast<const uint4*>(dk), dalpha, dbeta, out, partial, tokens, H, vb);
+  if (d == 64) mxk::launch_kernel(delta_inputs_bwd_kernel<8>, vb + gb, 256, 0, stream, x, ld, bias, static_cast<const uint4*>(dq), static_cast<const uint4*>(dk), dalpha, dbeta, out, partial, tokens, H, gb);
+  else if (d == 128) mxk::launch_kernel(delta_inputs_bwd_kernel<16>, vb + gb, 256, 0, stream, x, ld, bias, static_cast<const uint4*>(dq), static_cast<const uint4*>(dk), dalpha, dbeta, out, partial, tokens, H, gb);
   else return MXK_ERR_UNSUPPORTED;
   return launch_status();
 }
