@@ -390,7 +390,9 @@ int mxk_adam_bf16_master(void* params, float* master, const void* grads, float* 
  * elements (n % 8 == 0): out = gelu(x), or with dy != NULL out = dy * gelu'(x).
  * Column sums of x (rows, cols) bf16 -> out (cols) bf16, added in fp32 in a fixed order through
  * `workspace` (mxk_colsum_workspace_bytes): the bias gradient of a Dense layer (the reference's
- * nn.Dense under autodiff); cols % 8 == 0, else MXK_ERR_UNSUPPORTED.
+ * nn.Dense under autodiff); cols % 8 == 0, else MXK_ERR_UNSUPPORTED.  The _bwd_bias forms add up what they
+ * write as they write it (dbias: column sums of dx and of dg).  mxk_norm_bf16_bwd_add: dx += add1 + add2,
+ * the cotangents of two other readers of a LayerNorm's input (rms == 0; both or neither).
  * ------------------------------------------------------------------------- */
 size_t mxk_norm_bwd_workspace_bytes(long long rows, int D);
 int mxk_norm_bf16_fwd(const void* x, const void* gamma, const void* beta, void* y, float* mean, float* rstd,
@@ -398,12 +400,19 @@ int mxk_norm_bf16_fwd(const void* x, const void* gamma, const void* beta, void* 
 int mxk_norm_bf16_bwd(const void* x, const void* gamma, const float* mean, const float* rstd, const void* dy, void* dx,
                       float* dgamma, float* dbeta, void* workspace, size_t workspace_bytes, long long rows, int D, int rms,
                       mxk_stream_t stream);
+int mxk_norm_bf16_bwd_add(const void* x, const void* gamma, const float* mean, const float* rstd, const void* dy, const void* add1,
+                          const void* add2, void* dx, float* dgamma, float* dbeta, void* workspace, size_t workspace_bytes,
+                          long long rows, int D, int rms, mxk_stream_t stream);
 int mxk_gated_residual_bf16_fwd(const void* x, const void* g, const void* o, void* y, long long n, mxk_stream_t stream);
 int mxk_gated_residual_bf16_bwd(const void* dy, const void* g, const void* o, void* dg, void* d_o, long long n,
                                 mxk_stream_t stream);
 int mxk_l2norm_heads_bf16(const void* x, const void* dy, void* out, long long vectors, int head_dim, float eps,
                           mxk_stream_t stream);
+int mxk_gated_residual_bf16_bwd_bias(const void* dy, const void* g, const void* o, void* dg, void* d_o, void* dbias, void* workspace,
+                                     size_t workspace_bytes, long long rows, int cols, mxk_stream_t stream);
 int mxk_gelu_bf16(const void* x, const void* dy, void* out, long long n, mxk_stream_t stream);
+int mxk_gelu_bf16_bwd_bias(const void* x, const void* dy, void* dx, void* dbias, void* workspace, size_t workspace_bytes,
+                           long long rows, int cols, mxk_stream_t stream);
 size_t mxk_colsum_workspace_bytes(long long rows, int cols);
 int mxk_colsum_bf16(const void* x, void* out, void* workspace, size_t workspace_bytes, long long rows, int cols,
                     mxk_stream_t stream);

@@ -52,6 +52,9 @@ SIGNATURES = {
     "mxk_norm_bf16_fwd": (_i, [_p, _p, _p, _p, _p, _p, ctypes.c_longlong, _i, _f, _i, _p]),
     "mxk_norm_bf16_bwd": (_i, [_p] * 9 + [_z, ctypes.c_longlong, _i, _i, _p]),
     "mxk_gated_residual_bf16_fwd": (_i, [_p, _p, _p, _p, ctypes.c_longlong, _p]),
+    "mxk_norm_bf16_bwd_add": (_i, [_p] * 11 + [_z, ctypes.c_longlong, _i, _i, _p]),
+    "mxk_gated_residual_bf16_bwd_bias": (_i, [_p] * 7 + [_z, ctypes.c_longlong, _i, _p]),
+    "mxk_gelu_bf16_bwd_bias": (_i, [_p] * 5 + [_z, ctypes.c_longlong, _i, _p]),
     "mxk_gated_residual_bf16_bwd": (_i, [_p, _p, _p, _p, _p, ctypes.c_longlong, _p]),
     "mxk_l2norm_heads_bf16": (_i, [_p, _p, _p, ctypes.c_longlong, _i, _f, _p]),
     "mxk_mlstm_bf16_chunk_states_bytes": (_z, [_i, _i, _i, _i]),

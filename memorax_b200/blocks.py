@@ -32,14 +32,31 @@ class Dense(nn.Linear):
         return ops.dense(x, self.weight, self.bias)
 
 
+def _plain(module, kind):
+    """A module of exactly this kind without hooks: what a composition may call through its parts."""
+    return type(module) is kind and not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks
+                                         or module._backward_pre_hooks)
+
+
 class GatedResidual(nn.Module):
     def __init__(self, module, features):
         super().__init__()
         self.module, self.gate = module, Dense(features, features)
 
     def forward(self, inputs, done=None, initial_carry=None):
-        carry, out = self.module(inputs, done, initial_carry)
-        return carry, ops.gated_residual(inputs, self.gate(inputs), out)
+        fork = None
+        if _plain(self.module, PreNorm):   # the norm, the gate and the sum read the same inputs
+            norm = self.module.norm
+            fork = ops.norm_fork(inputs, norm.weight, norm.bias, norm.eps)
+        if fork is not None:
+            normed, inputs, gated = fork
+            carry, out = self.module.module(normed, done, initial_carry)
+        else:
+            gated = inputs
+            carry, out = self.module(inputs, done, initial_carry)
+        if _plain(self.gate, Dense):
+            return carry, ops.gated_dense(inputs, gated, self.gate, out)
+        return carry, ops.gated_residual(inputs, self.gate(gated), out)
 
 
 class FFN(nn.Module):
@@ -48,7 +65,7 @@ class FFN(nn.Module):
         self.up, self.down = Dense(features, features * expansion_factor), Dense(features * expansion_factor, features)
 
     def forward(self, inputs, done=None, initial_carry=None):
-        return None, self.down(ops.gelu(self.up(inputs)))
+        return None, self.down(ops.dense_gelu(inputs, self.up) if _plain(self.up, Dense) else ops.gelu(self.up(inputs)))
 
 
 class Stack(nn.Module):

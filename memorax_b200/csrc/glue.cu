@@ -85,12 +85,14 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
   }
 }
 
-// dx per row; per-block partial sums of dgamma (and dbeta) into part[block][2][D].
+// dx per row, plus add1 + add2 where a LayerNorm's input has two more readers; per-block partial sums of dgamma (and dbeta)
+// into part[block][2][D].
 template <int V, bool RMS>
 __global__ void __launch_bounds__(kRowWarps * 32)
 norm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gamma, const float* __restrict__ mean,
-                const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ dy, __nv_bfloat16* __restrict__ dx,
-                float* __restrict__ part, long long rows, int D) {
+                const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ add1,
+                const __nv_bfloat16* __restrict__ add2, __nv_bfloat16* __restrict__ dx, float* __restrict__ part, long long rows,
+                int D) {
   enter_kernel();
   const float inv_d = 1.f / static_cast<float>(D);
   __shared__ float red[kRowWarps][V * 256];
@@ -105,6 +107,11 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
     float xv[V][8], dv[V][8];
     load_row<V>(x + r * D, lane, D, xv);
     load_row<V>(dy + r * D, lane, D, dv);
+    float a1[V][8], a2[V][8];
+    if (!RMS && add1) {
+      load_row<V>(add1 + r * D, lane, D, a1);
+      load_row<V>(add2 + r * D, lane, D, a2);
+    }
     const float mu = RMS ? 0.f : mean[r], rs = rstd[r];
     float s1 = 0.f, s2 = 0.f;
 #pragma unroll
@@ -124,7 +131,10 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
 #pragma unroll
     for (int v = 0; v < V; ++v)
 #pragma unroll
-      for (int e = 0; e < 8; ++e) xv[v][e] = rs * (dv[v][e] - s1 - xv[v][e] * s2);
+      for (int e = 0; e < 8; ++e) {
+        xv[v][e] = rs * (dv[v][e] - s1 - xv[v][e] * s2);
+        if (!RMS && add1) xv[v][e] += a1[v][e] + a2[v][e];
+      }
     store_row<V>(dx + r * D, lane, D, xv);
   }
   // block partials: the eight warps' sums added in warp order
@@ -174,12 +184,14 @@ norm_bwd_reduce_kernel(const float* __restrict__ part, float* __restrict__ dgamm
   }
 }
 
-// Column sums of a (rows, cols) bf16 matrix in fp32 -- the bias gradient of a Dense layer.  Block (cx, ry) owns 256
-// columns x a contiguous range of rows: its thread (tx, ty) adds 8 columns of every eighth row, the eight thread rows
-// are added in a fixed order, and the block's sums go to part[ry][col]; the second kernel adds the row blocks in order.
-__global__ void __launch_bounds__(256)
-colsum_partial_kernel(const uint4* __restrict__ x, float* __restrict__ part, long long rows, int cols8, int rows_per_block) {
+// Column sums of a (rows, cols) bf16 matrix in fp32 -- the bias gradient of a Dense layer -- either as it is (ReadOp) or as
+// the pass that makes it writes it (GeluBwdOp, GatedBwdOp: a pass of its own would read the matrix again).  Block (cx, ry)
+// owns 256 columns x a contiguous range of rows: its thread (tx, ty) takes 8 columns of every eighth row, the eight thread
+// rows are added in a fixed order, and the block's sums go to part[ry][col]; a second kernel adds the row blocks in order.
+template <class Op>
+__global__ void __launch_bounds__(256) colsum_partial_kernel(const Op op, float* __restrict__ part, long long rows, int cols8, int rows_per_block) {
   enter_kernel();
+  constexpr int kInFlight = Op::kInFlight;   // rows whose loads are issued together
   __shared__ float red[8][32][9];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int v = blockIdx.x * 32 + tx;
@@ -190,21 +202,21 @@ colsum_partial_kernel(const uint4* __restrict__ x, float* __restrict__ part, lon
   for (int e = 0; e < 8; ++e) acc[e] = 0.f;
   if (v < cols8) {
     long long r = r0 + ty;
-    for (; r + 56 < r1; r += 64) {   // eight independent loads in flight
-      uint4 raw[8];
+    for (; r + 8 * (kInFlight - 1) < r1; r += 8 * kInFlight) {
+      typename Op::Raw raw[kInFlight];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) raw[u] = ld_stream(x + (r + 8 * u) * cols8 + v);
+      for (int u = 0; u < kInFlight; ++u) raw[u] = op.load((r + 8 * u) * cols8 + v);
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
+      for (int u = 0; u < kInFlight; ++u) {
         float f[8];
-        umma::unpack8_bf16(raw[u], f);
+        op.apply(raw[u], (r + 8 * u) * cols8 + v, f);
 #pragma unroll
         for (int e = 0; e < 8; ++e) acc[e] += f[e];
       }
     }
     for (; r < r1; r += 8) {
       float f[8];
-      umma::unpack8_bf16(ld_stream(x + r * cols8 + v), f);
+      op.apply(op.load(r * cols8 + v), r * cols8 + v, f);
 #pragma unroll
       for (int e = 0; e < 8; ++e) acc[e] += f[e];
     }
@@ -222,6 +234,14 @@ colsum_partial_kernel(const uint4* __restrict__ x, float* __restrict__ part, lon
     part[static_cast<size_t>(blockIdx.y) * cols8 * 8 + col] = t;
   }
 }
+struct ReadOp {
+  static constexpr int kInFlight = 8;
+  using Raw = uint4;
+  const uint4* x;
+  __device__ __forceinline__ Raw load(long long i) const { return ld_stream(x + i); }
+  __device__ __forceinline__ void apply(const Raw& raw, long long, float* f) const { umma::unpack8_bf16(raw, f); }
+};
+
 // A block owns 32 columns; its eight thread rows each add every eighth row block, then thread row 0 adds the eight sums in order.
 __global__ void __launch_bounds__(256)
 colsum_final_kernel(const float* __restrict__ part, __nv_bfloat16* __restrict__ out, int row_blocks, int cols) {
@@ -263,15 +283,11 @@ gelu_fwd_kernel(const uint4* __restrict__ x, uint4* __restrict__ y, long long n8
   }
   y[i] = umma::pack8_bf16(f);
 }
-// dx = dy * d/dx gelu(x)
-__global__ void __launch_bounds__(256)
-gelu_bwd_kernel(const uint4* __restrict__ x, const uint4* __restrict__ dy, uint4* __restrict__ dx, long long n8) {
-  enter_kernel();
-  const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
-  if (i >= n8) return;
-  float f[8], g[8];
-  umma::unpack8_bf16(ld_stream(x + i), f);
-  umma::unpack8_bf16(ld_stream(dy + i), g);
+// g <- dy * d/dx gelu(x)
+__device__ __forceinline__ void gelu_grad8(uint4 x, uint4 dy, float* g) {
+  float f[8];
+  umma::unpack8_bf16(x, f);
+  umma::unpack8_bf16(dy, g);
 #pragma unroll
   for (int e = 0; e < 8; ++e) {
     const float v = f[e], v2 = v * v;
@@ -279,8 +295,27 @@ gelu_bwd_kernel(const uint4* __restrict__ x, const uint4* __restrict__ dy, uint4
     const float dt = (1.f - t * t) * 0.7978845608f * fmaf(3.f * 0.044715f, v2, 1.f);
     g[e] *= 0.5f * (1.f + t) + 0.5f * v * dt;
   }
+}
+__global__ void __launch_bounds__(256)
+gelu_bwd_kernel(const uint4* __restrict__ x, const uint4* __restrict__ dy, uint4* __restrict__ dx, long long n8) {
+  enter_kernel();
+  const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
+  if (i >= n8) return;
+  float g[8];
+  gelu_grad8(ld_stream(x + i), ld_stream(dy + i), g);
   dx[i] = umma::pack8_bf16(g);
 }
+struct GeluBwdOp {
+  static constexpr int kInFlight = 4;
+  struct Raw { uint4 x, dy; };
+  const uint4 *x, *dy;
+  uint4* dx;
+  __device__ __forceinline__ Raw load(long long i) const { return {ld_stream(x + i), ld_stream(dy + i)}; }
+  __device__ __forceinline__ void apply(const Raw& r, long long i, float* g) const {
+    gelu_grad8(r.x, r.dy, g);
+    dx[i] = umma::pack8_bf16(g);
+  }
+};
 
 // y = x + sigmoid(g) * o
 __global__ void __launch_bounds__(256)
@@ -297,26 +332,43 @@ gated_residual_fwd_kernel(const uint4* __restrict__ x, const uint4* __restrict__
   for (int e = 0; e < 8; ++e) xf[e] = fmaf(1.f / (1.f + __expf(-gf[e])), of[e], xf[e]);
   y[i] = umma::pack8_bf16(xf);
 }
-// do = dy * sigmoid(g), dg = dy * o * sigmoid(g) (1 - sigmoid(g)); dx = dy needs no kernel
-__global__ void __launch_bounds__(256)
-gated_residual_bwd_kernel(const uint4* __restrict__ dy, const uint4* __restrict__ g, const uint4* __restrict__ o,
-                          uint4* __restrict__ dg, uint4* __restrict__ d_o, long long n8) {
-  enter_kernel();
-  const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
-  if (i >= n8) return;
-  float yf[8], gf[8], of[8];
-  umma::unpack8_bf16(dy[i], yf);
-  umma::unpack8_bf16(g[i], gf);
-  umma::unpack8_bf16(o[i], of);
+// gf <- dg = dy * o * sigmoid(g) (1 - sigmoid(g)), of <- do = dy * sigmoid(g); dx = dy needs no kernel
+__device__ __forceinline__ void gated_grad8(uint4 dy, uint4 g, uint4 o, float* gf, float* of) {
+  float yf[8];
+  umma::unpack8_bf16(dy, yf);
+  umma::unpack8_bf16(g, gf);
+  umma::unpack8_bf16(o, of);
 #pragma unroll
   for (int e = 0; e < 8; ++e) {
     const float s = 1.f / (1.f + __expf(-gf[e]));
     gf[e] = yf[e] * of[e] * s * (1.f - s);
     of[e] = yf[e] * s;
   }
+}
+__global__ void __launch_bounds__(256)
+gated_residual_bwd_kernel(const uint4* __restrict__ dy, const uint4* __restrict__ g, const uint4* __restrict__ o,
+                          uint4* __restrict__ dg, uint4* __restrict__ d_o, long long n8) {
+  enter_kernel();
+  const long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
+  if (i >= n8) return;
+  float gf[8], of[8];
+  gated_grad8(dy[i], g[i], o[i], gf, of);
   dg[i] = umma::pack8_bf16(gf);
   d_o[i] = umma::pack8_bf16(of);
 }
+struct GatedBwdOp {
+  static constexpr int kInFlight = 4;
+  struct Raw { uint4 dy, g, o; };
+  const uint4 *dy, *g, *o;
+  uint4 *dg, *d_o;
+  __device__ __forceinline__ Raw load(long long i) const { return {dy[i], ld_stream(g + i), ld_stream(o + i)}; }
+  __device__ __forceinline__ void apply(const Raw& r, long long i, float* gf) const {
+    float of[8];
+    gated_grad8(r.dy, r.g, r.o, gf, of);
+    dg[i] = umma::pack8_bf16(gf);
+    d_o[i] = umma::pack8_bf16(of);
+  }
+};
 
 // Per-head L2 normalisation: LPH = hd / 8 lanes hold one head vector (16 bytes each).
 template <int LPH, bool BWD>
@@ -378,6 +430,22 @@ int colsum_row_blocks(long long rows, int cols) {
   return static_cast<int>(want < 1 ? 1 : want);
 }
 
+template <class Op>
+int colsum(const Op& op, void* out, void* workspace, size_t workspace_bytes, long long rows, int cols, mxk_stream_t stream) {
+  if (rows <= 0 || cols <= 0) return MXK_ERR_DIMS;
+  if (cols % 8) return MXK_ERR_UNSUPPORTED;
+  if ((reinterpret_cast<uintptr_t>(out) % 2) || (workspace && !aligned16(workspace))) return MXK_ERR_ALIGN;
+  if (!workspace || workspace_bytes < mxk_colsum_workspace_bytes(rows, cols)) return MXK_ERR_WORKSPACE;
+  const int nrb = colsum_row_blocks(rows, cols), cols8 = cols / 8;
+  const int rpb = static_cast<int>((rows + nrb - 1) / nrb);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  float* const part = static_cast<float*>(workspace);
+  mxk::launch_kernel(colsum_partial_kernel<Op>, dim3((cols8 + 31) / 32, nrb), 256, 0, s, op, part, rows, cols8, rpb);
+  if (int st = launch_status()) return st;
+  mxk::launch_kernel(colsum_final_kernel, (cols + 31) / 32, 256, 0, s, static_cast<const float*>(part), static_cast<__nv_bfloat16*>(out), nrb, cols);
+  return launch_status();
+}
+
 }  // namespace
 }  // namespace mxk
 
@@ -390,20 +458,28 @@ size_t mxk_colsum_workspace_bytes(long long rows, int cols) {
 
 int mxk_colsum_bf16(const void* x, void* out, void* workspace, size_t workspace_bytes, long long rows, int cols,
                     mxk_stream_t stream) {
-  using namespace mxk;
   if (!x || !out) return MXK_ERR_NULL;
-  if (rows <= 0 || cols <= 0) return MXK_ERR_DIMS;
-  if (cols % 8) return MXK_ERR_UNSUPPORTED;
-  if (!aligned16(x) || (reinterpret_cast<uintptr_t>(out) % 2) || (workspace && !aligned16(workspace))) return MXK_ERR_ALIGN;
-  if (!workspace || workspace_bytes < mxk_colsum_workspace_bytes(rows, cols)) return MXK_ERR_WORKSPACE;
-  const int nrb = colsum_row_blocks(rows, cols), cols8 = cols / 8;
-  const int rpb = static_cast<int>((rows + nrb - 1) / nrb);
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  mxk::launch_kernel(colsum_partial_kernel, dim3((cols8 + 31) / 32, nrb), 256, 0, s, static_cast<const uint4*>(x), static_cast<float*>(workspace),
-                                                                      rows, cols8, rpb);
-  if (int st = launch_status()) return st;
-  mxk::launch_kernel(colsum_final_kernel, (cols + 31) / 32, 256, 0, s, static_cast<const float*>(workspace), static_cast<__nv_bfloat16*>(out), nrb, cols);
-  return launch_status();
+  if (!mxk::aligned16(x)) return MXK_ERR_ALIGN;
+  return mxk::colsum(mxk::ReadOp{static_cast<const uint4*>(x)}, out, workspace, workspace_bytes, rows, cols, stream);
+}
+
+int mxk_gelu_bf16_bwd_bias(const void* x, const void* dy, void* dx, void* dbias, void* workspace, size_t workspace_bytes,
+                           long long rows, int cols, mxk_stream_t stream) {
+  if (!x || !dy || !dx || !dbias) return MXK_ERR_NULL;
+  for (const void* p : {x, dy, (const void*)dx})
+    if (!mxk::aligned16(p)) return MXK_ERR_ALIGN;
+  const mxk::GeluBwdOp op{static_cast<const uint4*>(x), static_cast<const uint4*>(dy), static_cast<uint4*>(dx)};
+  return mxk::colsum(op, dbias, workspace, workspace_bytes, rows, cols, stream);
+}
+
+int mxk_gated_residual_bf16_bwd_bias(const void* dy, const void* g, const void* o, void* dg, void* d_o, void* dbias, void* workspace,
+                                     size_t workspace_bytes, long long rows, int cols, mxk_stream_t stream) {
+  if (!dy || !g || !o || !dg || !d_o || !dbias) return MXK_ERR_NULL;
+  for (const void* p : {dy, g, o, (const void*)dg, (const void*)d_o})
+    if (!mxk::aligned16(p)) return MXK_ERR_ALIGN;
+  const mxk::GatedBwdOp op{static_cast<const uint4*>(dy), static_cast<const uint4*>(g), static_cast<const uint4*>(o), static_cast<uint4*>(dg),
+                           static_cast<uint4*>(d_o)};
+  return mxk::colsum(op, dbias, workspace, workspace_bytes, rows, cols, stream);
 }
 
 size_t mxk_norm_bwd_workspace_bytes(long long rows, int D) {
@@ -438,21 +514,29 @@ int mxk_norm_bf16_fwd(const void* x, const void* gamma, const void* beta, void* 
 int mxk_norm_bf16_bwd(const void* x, const void* gamma, const float* mean, const float* rstd, const void* dy, void* dx,
                       float* dgamma, float* dbeta, void* workspace, size_t workspace_bytes, long long rows, int D, int rms,
                       mxk_stream_t stream) {
+  return mxk_norm_bf16_bwd_add(x, gamma, mean, rstd, dy, nullptr, nullptr, dx, dgamma, dbeta, workspace, workspace_bytes, rows, D, rms, stream);
+}
+
+int mxk_norm_bf16_bwd_add(const void* x, const void* gamma, const float* mean, const float* rstd, const void* dy, const void* add1,
+                          const void* add2, void* dx, float* dgamma, float* dbeta, void* workspace, size_t workspace_bytes,
+                          long long rows, int D, int rms, mxk_stream_t stream) {
   using namespace mxk;
   if (int st = check_norm(x, gamma, dx, rows, D)) return st;
-  if (!rstd || !dy || !dgamma || (!rms && (!mean || !dbeta))) return MXK_ERR_NULL;
+  if (!rstd || !dy || !dgamma || (!rms && (!mean || !dbeta)) || !add1 != !add2) return MXK_ERR_NULL;
+  if (rms && add1) return MXK_ERR_UNSUPPORTED;
   if (!workspace || workspace_bytes < mxk_norm_bwd_workspace_bytes(rows, D)) return MXK_ERR_WORKSPACE;
-  if (!aligned16(dy) || (reinterpret_cast<uintptr_t>(workspace) & 3u)) return MXK_ERR_ALIGN;
+  if (!aligned16(dy) || !aligned16(add1) || !aligned16(add2) || (reinterpret_cast<uintptr_t>(workspace) & 3u)) return MXK_ERR_ALIGN;
   const auto* xp = static_cast<const __nv_bfloat16*>(x);
   const auto* gp = static_cast<const __nv_bfloat16*>(gamma);
   const auto* dyp = static_cast<const __nv_bfloat16*>(dy);
+  const auto *a1 = static_cast<const __nv_bfloat16*>(add1), *a2 = static_cast<const __nv_bfloat16*>(add2);
   auto* dxp = static_cast<__nv_bfloat16*>(dx);
   float* part = static_cast<float*>(workspace);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int blocks = norm_blocks(rows), threads = kRowWarps * 32;
 #define MXK_NORM_BWD(V)                                                                                  \
-  if (rms) mxk::launch_kernel(norm_bwd_kernel<V, true>, blocks, threads, 0, s, xp, gp, nullptr, rstd, dyp, dxp, part, rows, D); \
-  else mxk::launch_kernel(norm_bwd_kernel<V, false>, blocks, threads, 0, s, xp, gp, mean, rstd, dyp, dxp, part, rows, D);
+  if (rms) mxk::launch_kernel(norm_bwd_kernel<V, true>, blocks, threads, 0, s, xp, gp, nullptr, rstd, dyp, nullptr, nullptr, dxp, part, rows, D); \
+  else mxk::launch_kernel(norm_bwd_kernel<V, false>, blocks, threads, 0, s, xp, gp, mean, rstd, dyp, a1, a2, dxp, part, rows, D);
   switch ((D + 255) / 256) {
     case 1: MXK_NORM_BWD(1) break;
     case 2: MXK_NORM_BWD(2) break;

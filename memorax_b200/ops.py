@@ -601,7 +601,7 @@ class FusedNorm(torch.autograd.Function):
         return y
 
     @staticmethod
-    def backward(ctx, dy):
+    def backward(ctx, dy, add1=None, add2=None):
         x, weight, mean, rstd = ctx.saved_tensors
         dim = x.shape[-1]
         rows = x.numel() // dim
@@ -611,10 +611,33 @@ class FusedNorm(torch.autograd.Function):
         dbeta = None if ctx.rms else torch.empty(dim, dtype=torch.float32, device=x.device)
         ws_bytes = _lib.lib.mxk_norm_bwd_workspace_bytes(rows, dim)
         ws = torch.empty(ws_bytes, dtype=torch.uint8, device=x.device)
-        _lib.call("mxk_norm_bf16_bwd", _ptr(x), _ptr(weight), _ptr(mean), _ptr(rstd), _ptr(dy), _ptr(dx), _ptr(dgamma),
-                  _ptr(dbeta), _ptr(ws), ws_bytes, rows, dim, int(ctx.rms), _stream())
+        _lib.call("mxk_norm_bf16_bwd_add", _ptr(x), _ptr(weight), _ptr(mean), _ptr(rstd), _ptr(dy), _ptr(add1), _ptr(add2),
+                  _ptr(dx), _ptr(dgamma), _ptr(dbeta), _ptr(ws), ws_bytes, rows, dim, int(ctx.rms), _stream())
         return (dx, dgamma.to(weight.dtype), dbeta.to(weight.dtype) if (dbeta is not None and ctx.has_bias) else None,
                 None, None)
+
+
+class NormFork(torch.autograd.Function):
+    """``(LayerNorm(x), x, x)`` for an ``x`` that two others read besides the norm: the three cotangents are added by the
+    norm's backward pass (autograd would add them in two passes of its own, three tensors each)."""
+
+    @staticmethod
+    def forward(ctx, x, weight, bias, eps):
+        y = FusedNorm.forward(ctx, x, weight, bias, eps, False)
+        return y, x.view_as(x), x.view_as(x)
+
+    @staticmethod
+    def backward(ctx, dy, d1, d2):
+        dx, dw, db, _, _ = FusedNorm.backward(ctx, dy, d1.contiguous(), d2.contiguous())
+        return dx, dw, db, None
+
+
+def norm_fork(x, weight, bias, eps):
+    """``(layer_norm(x), x, x)``, or ``None`` where the fused backward pass does not apply."""
+    if (torch.is_grad_enabled() and x.requires_grad and _glue_ok(x, x.shape[-1]) and weight.dtype == torch.bfloat16
+            and bias is not None and x.is_contiguous() and _aligned(x, weight, bias)):
+        return NormFork.apply(x, weight, bias, eps)
+    return None
 
 
 def layer_norm(x, weight, bias, eps=1e-5):
@@ -743,6 +766,80 @@ def dense(x, weight, bias=None):
             and bias.dtype == torch.bfloat16 and weight.shape[0] % 8 == 0 and torch.is_grad_enabled()):
         return DenseBias.apply(x, weight, bias)
     return F.linear(x, weight, bias)
+
+
+def _dense_grads(ctx, dy, x, weight):
+    """Cotangents of the input and the weight of ``x W^T`` for the Functions whose inputs start with ``(x, weight)``."""
+    dy2 = dy.reshape(-1, dy.shape[-1])
+    dx = torch.matmul(dy, weight) if ctx.needs_input_grad[0] else None
+    dw = torch.mm(dy2.t(), x.reshape(-1, x.shape[-1])) if ctx.needs_input_grad[1] else None
+    return dx, dw
+
+
+def _bias_workspace(x):
+    rows, cols = x.numel() // x.shape[-1], x.shape[-1]
+    ws_bytes = _lib.lib.mxk_colsum_workspace_bytes(rows, cols)
+    ws = torch.empty(ws_bytes, dtype=torch.uint8, device=x.device)
+    return torch.empty(cols, dtype=torch.bfloat16, device=x.device), ws, ws_bytes, rows, cols
+
+
+class DenseGelu(torch.autograd.Function):
+    """``gelu(x W^T + b)``; the bias gradient is added up by the pass that writes the GELU's cotangent."""
+
+    @staticmethod
+    def forward(ctx, x, weight, bias):
+        a = F.linear(x, weight, bias)
+        y = torch.empty_like(a)
+        _lib.call("mxk_gelu_bf16", _ptr(a), None, _ptr(y), a.numel(), _stream())
+        ctx.save_for_backward(x, weight, a)
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        x, weight, a = ctx.saved_tensors
+        da, dy = torch.empty_like(a), dy.contiguous()
+        db, ws, ws_bytes, rows, cols = _bias_workspace(a)
+        _lib.call("mxk_gelu_bf16_bwd_bias", _ptr(a), _ptr(dy), _ptr(da), _ptr(db), _ptr(ws), ws_bytes, rows, cols, _stream())
+        return (*_dense_grads(ctx, da, x, weight), db)
+
+
+class GatedDense(torch.autograd.Function):
+    """``x + sigmoid(z W^T + b) * o``; the bias gradient is added up by the pass that writes the gate's cotangent."""
+
+    @staticmethod
+    def forward(ctx, z, weight, bias, x, o):
+        g, x, o = F.linear(z, weight, bias), x.contiguous(), o.contiguous()
+        y = torch.empty_like(x)
+        _lib.call("mxk_gated_residual_bf16_fwd", _ptr(x), _ptr(g), _ptr(o), _ptr(y), x.numel(), _stream())
+        ctx.save_for_backward(z, weight, g, o)
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        z, weight, g, o = ctx.saved_tensors
+        dy, dg, d_o = dy.contiguous(), torch.empty_like(g), torch.empty_like(o)
+        db, ws, ws_bytes, rows, cols = _bias_workspace(g)
+        _lib.call("mxk_gated_residual_bf16_bwd_bias", _ptr(dy), _ptr(g), _ptr(o), _ptr(dg), _ptr(d_o), _ptr(db), _ptr(ws), ws_bytes,
+                  rows, cols, _stream())
+        return (*_dense_grads(ctx, dg, z, weight), db, dy, d_o)
+
+
+def _trains(x, layer):
+    """Whether a Dense layer over bf16 CUDA rows is in a backward pass that wants its bias gradient."""
+    return (torch.is_grad_enabled() and layer.bias is not None and x.is_cuda and x.numel() > 0 and layer.weight.shape[0] % 8 == 0
+            and layer.bias.requires_grad and x.dtype == layer.weight.dtype == layer.bias.dtype == torch.bfloat16)
+
+
+def dense_gelu(x, layer):
+    """``gelu(layer(x))``."""
+    return DenseGelu.apply(x, layer.weight, layer.bias) if _trains(x, layer) else gelu(dense(x, layer.weight, layer.bias))
+
+
+def gated_dense(x, z, layer, o):
+    """``x + sigmoid(layer(z)) * o``."""
+    if _trains(z, layer) and x.is_cuda and x.dtype == o.dtype == torch.bfloat16 and x.shape == o.shape == (*z.shape[:-1], layer.weight.shape[0]):
+        return GatedDense.apply(z, layer.weight, layer.bias, x, o)
+    return gated_residual(x, dense(z, layer.weight, layer.bias), o)
 
 
 def l2norm_heads(x, head_dim, eps=1e-12):
