@@ -17,7 +17,6 @@
 //          j the column.
 // The forward kernel then forms U = T' (V - diag(g) K S_in^T) and the backward kernel dR = T'^T dU as
 // plain tensor-core products.
-#include "gdelta64.cuh"
 #include "gdelta_common.cuh"
 #include "tma.cuh"
 
@@ -53,9 +52,9 @@ struct PrepSmem {
   float cum[kC], beta[kC];
   uint64_t bar_load, bar_mma;
   uint32_t tmem;
-  alignas(1024) uint4 k[kPanD * kC];   // K, SW tiles (one or two 64-column blocks)
+  alignas(1024) uint4 k[2 * kSquareVecs];   // K, SW tiles (one or two 64-column blocks)
 };
-constexpr int smem_bytes(int blocks) { return static_cast<int>(offsetof(PrepSmem, k)) + blocks * kSwBlockVecs * 16; }
+constexpr int smem_bytes(int blocks) { return static_cast<int>(offsetof(PrepSmem, k)) + blocks * kSquareVecs * 16; }
 static_assert(smem_bytes(1) <= 44 * 1024 && smem_bytes(2) <= 56 * 1024, "five CTAs per SM for heads of 64, four for 128");
 
 #ifdef MXK_TIMING
@@ -67,7 +66,7 @@ namespace {
 #define MXK_TP(i) do {} while (0)
 #endif
 constexpr uint32_t kPrepTmemCols = 32;
-constexpr uint32_t kUpper = 16u << 16;
+constexpr int kThreads = 128;
 
 // acc[0 .. 1] += a * (four consecutive values)
 __device__ __forceinline__ void axpy(float a, float4 x, float2* acc) {
@@ -82,7 +81,7 @@ __global__ void __launch_bounds__(kThreads, 5) gdelta_prep_kernel(const __grid_c
   PrepSmem& sm = *reinterpret_cast<PrepSmem*>(smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bool upper = lane >= 16;
-  const int row = warp * 16 + (lane & 15);   // token row owned in the M = 64 accumulator
+  const int row = warp * 16 + (lane & 15);   // token row owned in the accumulator
 
 #ifdef MXK_TIMING
   long long t_prev_ = clock64();
@@ -101,15 +100,15 @@ __global__ void __launch_bounds__(kThreads, 5) gdelta_prep_kernel(const __grid_c
   bool timed_out = false;
   MXK_TP(0);
 
-  heads64::Gates gates{};
+  Gates gates{};
   linattn::DoneFlags flags;
   const auto fetch = [&](int item) {
     const int c = item % p.nchunks, bh = item / p.nchunks, b = bh / p.H, h = bh % p.H, t0 = c * kC;
     if (tid == 0) {
-      tma::expect_bytes(&sm.bar_load, p.blocks * kSwBlockVecs * 16);
-      for (int i = 0; i < p.blocks; ++i) tma::load_plain_tile(sm.k + i * kSwBlockVecs, &p.map_k, &sm.bar_load, t0, h, b, 64 * i);
+      tma::expect_bytes(&sm.bar_load, p.blocks * kSquareVecs * 16);
+      for (int i = 0; i < p.blocks; ++i) tma::load_plain_tile(sm.k + i * kSquareVecs, &p.map_k, &sm.bar_load, t0, h, b, 64 * i);
     }
-    if (warp == 1) gates = heads64::load_gates(p.alpha, p.beta, static_cast<size_t>(b) * p.T, p.H, h, t0, p.T, lane);
+    if (warp == 1) gates = load_gates(p.alpha, p.beta, static_cast<size_t>(b) * p.T, p.H, h, t0, p.T, lane);
     flags = linattn::load_done_flags(p.done ? p.done + static_cast<size_t>(b) * p.T : nullptr, t0, p.T, lane);
   };
   float* const xm = sm.x;
@@ -127,15 +126,15 @@ __global__ void __launch_bounds__(kThreads, 5) gdelta_prep_kernel(const __grid_c
       fence_after_sync();
       // keys 0..31 land in lanes 0..15 of each warp's TMEM quarter, keys 32..63 in lanes 16..31 of the same columns
       for (int i = 0; i < p.blocks; ++i) {
-        const uint32_t at = smem_u32(sm.k + i * kSwBlockVecs);
+        const uint32_t at = smem_u32(sm.k + i * kSquareVecs);
         gemm<4>(tmem, sw_operand(at, false), sw_operand(at, false), id_half, i > 0, leader);
-        gemm<4>(tmem + kUpper, sw_operand(at, false), sw_operand(at + 32 * 128, false), id_half, i > 0, leader);
+        gemm<4>(tmem + kUpperLanes, sw_operand(at, false), sw_operand(at + 32 * 128, false), id_half, i > 0, leader);
       }
       if (leader) commit(&sm.bar_mma);
       if (tid == 0) tma::wait_group_read<0>();   // the previous T' has left `tp`
       __syncwarp();
     } else if (warp == 1) {
-      const float2 cum = heads64::cumulative(gates, lane);
+      const float2 cum = cumulative(gates, lane);
       *reinterpret_cast<float2*>(&sm.cum[2 * lane]) = cum;
       *reinterpret_cast<float2*>(&sm.beta[2 * lane]) = make_float2(gates.b[0], gates.b[1]);
     }
