@@ -88,9 +88,12 @@ __global__ void __launch_bounds__(128) lru_step_read_kernel(LruWeights w, const 
   y[at] = fmaf(x[at], w.d[f], v);
 }
 
-constexpr int kSkipBlocks = 2 * kNumSMs;
+constexpr int kSkipBlocks = 4 * kNumSMs;
 
-// HBM-bound: one read of both operands; a block takes every gridDim.x-th group of rows, its threads the columns.
+// HBM-bound: one read of both operands; a block takes every gridDim.x-th group of rows, its threads the columns.  Four blocks
+// an SM with eight rows of both operands in flight per thread are the 64 KiB that HBM wants outstanding (16 KiB: 45 us for
+// 65536 x 256).
+constexpr int kSkipRows = 8;
 __global__ void __launch_bounds__(256) skip_grad_kernel(const float* __restrict__ gy, const float* __restrict__ x,
                                                         float* __restrict__ partial, long long rows, int F) {
   enter_kernel();
@@ -104,15 +107,15 @@ __global__ void __launch_bounds__(256) skip_grad_kernel(const float* __restrict_
     if (ro < per && c < F) {
       const long long step = static_cast<long long>(gridDim.x) * per;
       long long r = static_cast<long long>(blockIdx.x) * per + ro;
-      for (; r + 3 * step < rows; r += 4 * step) {
-        float a[4], b[4];
+      for (; r + (kSkipRows - 1) * step < rows; r += kSkipRows * step) {
+        float a[kSkipRows], b[kSkipRows];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < kSkipRows; ++u) {
           a[u] = ld_stream(gy + (r + u * step) * F + c);
           b[u] = x ? ld_stream(x + (r + u * step) * F + c) : 1.f;
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) s[u] = fmaf(a[u], b[u], s[u]);
+        for (int u = 0; u < kSkipRows; ++u) s[u & 3] = fmaf(a[u], b[u], s[u & 3]);
       }
       for (; r < rows; r += step) s[0] = fmaf(gy[r * F + c], x ? x[r * F + c] : 1.f, s[0]);
     }
@@ -150,7 +153,7 @@ __global__ void __launch_bounds__(128) lru_param_grads_kernel(LruWeights w, LruG
     for (int f = tid; f < F; f += 128) {
       float re = 0.f, im = 0.f;
       const float* p = g.in_partial + static_cast<size_t>(2) * n * F + f;
-#pragma unroll 4
+#pragma unroll 6
       for (int s = 0; s < g.in_splits; ++s) { re += p[s * plane]; im += p[s * plane + F]; }
       re *= scale;
       im *= scale;
@@ -173,7 +176,7 @@ __global__ void __launch_bounds__(128) lru_param_grads_kernel(LruWeights w, LruG
     for (int n = tid; n < N; n += 128) {
       float re = 0.f, im = 0.f;
       const float2* p = reinterpret_cast<const float2*>(g.out_partial + static_cast<size_t>(f) * 2 * N) + n;
-#pragma unroll 4
+#pragma unroll 6
       for (int s = 0; s < g.out_splits; ++s) { const float2 v = p[s * (plane / 2)]; re += v.x; im += v.y; }
       const size_t at = static_cast<size_t>(f) * N + n;
       g.g_c_re[at] = re;
