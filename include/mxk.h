@@ -318,9 +318,7 @@ int mxk_mlstm_bf16_bwd(const void* q, const void* k, const void* v, const float*
  * i.e. Memoroid.scan_fn (memoroid.py:60-91) over the elements
  * (alpha (I - beta k k^T), beta v k^T) with the operator (M_i M_j, U_i M_j + U_j).
  *
- *   q, k, v   (B,T,H,d) bf16, contiguous, d = 128 or 64 (a 64-wide head runs on the
- *             128-wide tiles with their upper half zero-filled by the tensor maps: half the
- *             memory traffic, the arithmetic of d = 128); k is expected L2-normalised
+ *   q, k, v   (B,T,H,d) bf16, contiguous, d = 128 or 64; k is expected L2-normalised
  *   alpha     (B,T,H) fp32 in (0, 1];  beta (B,T,H) fp32
  *   s0        (B,H,d_v,d_k) fp32 carried state, NULL = zeros
  *   o         (B,T,H,d) bf16 out;  s_last (B,H,d_v,d_k) fp32 out, optional
