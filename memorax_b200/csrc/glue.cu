@@ -25,12 +25,23 @@ __device__ __forceinline__ float warp_sum(float x) {
 
 // V = ceil(D / 256) 16-byte vectors per lane; lane l owns elements [v * 256 + l * 8, + 8), those past D read as zero.
 template <int V>
-__device__ __forceinline__ void load_row(const __nv_bfloat16* row, int lane, int D, float (*x)[8]) {
+__device__ __forceinline__ void load_raw(const __nv_bfloat16* row, int lane, int D, uint4* x) {
 #pragma unroll
   for (int v = 0; v < V; ++v) {
     const int at = v * 256 + lane * 8;
-    umma::unpack8_bf16(at < D ? *reinterpret_cast<const uint4*>(row + at) : make_uint4(0, 0, 0, 0), x[v]);
+    x[v] = at < D ? *reinterpret_cast<const uint4*>(row + at) : make_uint4(0, 0, 0, 0);
   }
+}
+template <int V>
+__device__ __forceinline__ void unpack_row(const uint4* raw, float (*x)[8]) {
+#pragma unroll
+  for (int v = 0; v < V; ++v) umma::unpack8_bf16(raw[v], x[v]);
+}
+template <int V>
+__device__ __forceinline__ void load_row(const __nv_bfloat16* row, int lane, int D, float (*x)[8]) {
+  uint4 raw[V];
+  load_raw<V>(row, lane, D, raw);
+  unpack_row<V>(raw, x);
 }
 template <int V>
 __device__ __forceinline__ void store_row(__nv_bfloat16* row, int lane, int D, const float (*y)[8]) {
@@ -86,9 +97,11 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
 }
 
 // dx per row, plus add1 + add2 where a LayerNorm's input has two more readers; per-block partial sums of dgamma (and dbeta)
-// into part[block][2][D].
+// into part[block][2][D].  A warp's next row is on its way while it works on the present one: few rows fit an SM beside the
+// column sums in registers, and without that they left HBM waiting (65536 x 256: 31 us, 16 KiB an SM outstanding).
+constexpr int norm_bwd_blocks_per_sm(int v) { return v == 1 ? 3 : v == 2 ? 2 : 1; }
 template <int V, bool RMS>
-__global__ void __launch_bounds__(kRowWarps * 32)
+__global__ void __launch_bounds__(kRowWarps * 32, norm_bwd_blocks_per_sm(V))
 norm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gamma, const float* __restrict__ mean,
                 const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ add1,
                 const __nv_bfloat16* __restrict__ add2, __nv_bfloat16* __restrict__ dx, float* __restrict__ part, long long rows,
@@ -103,16 +116,27 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
   for (int v = 0; v < V; ++v)
 #pragma unroll
     for (int e = 0; e < 8; ++e) dg[v][e] = db[v][e] = 0.f;
-  for (long long r = static_cast<long long>(blockIdx.x) * kRowWarps + warp; r < rows; r += static_cast<long long>(gridDim.x) * kRowWarps) {
+  const long long step = static_cast<long long>(gridDim.x) * kRowWarps;
+  long long r = static_cast<long long>(blockIdx.x) * kRowWarps + warp;
+  uint4 xr[V], dr[V];
+  if (r < rows) {
+    load_raw<V>(x + r * D, lane, D, xr);
+    load_raw<V>(dy + r * D, lane, D, dr);
+  }
+  for (; r < rows; r += step) {
     float xv[V][8], dv[V][8];
-    load_row<V>(x + r * D, lane, D, xv);
-    load_row<V>(dy + r * D, lane, D, dv);
-    float a1[V][8], a2[V][8];
-    if (!RMS && add1) {
-      load_row<V>(add1 + r * D, lane, D, a1);
-      load_row<V>(add2 + r * D, lane, D, a2);
-    }
+    uint4 a1[V], a2[V];
+    unpack_row<V>(xr, xv);
+    unpack_row<V>(dr, dv);
     const float mu = RMS ? 0.f : mean[r], rs = rstd[r];
+    if (!RMS && add1) {
+      load_raw<V>(add1 + r * D, lane, D, a1);
+      load_raw<V>(add2 + r * D, lane, D, a2);
+    }
+    if (r + step < rows) {
+      load_raw<V>(x + (r + step) * D, lane, D, xr);
+      load_raw<V>(dy + (r + step) * D, lane, D, dr);
+    }
     float s1 = 0.f, s2 = 0.f;
 #pragma unroll
     for (int v = 0; v < V; ++v)
@@ -131,10 +155,17 @@ norm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
 #pragma unroll
     for (int v = 0; v < V; ++v)
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        xv[v][e] = rs * (dv[v][e] - s1 - xv[v][e] * s2);
-        if (!RMS && add1) xv[v][e] += a1[v][e] + a2[v][e];
+      for (int e = 0; e < 8; ++e) xv[v][e] = rs * (dv[v][e] - s1 - xv[v][e] * s2);
+    if (!RMS && add1) {
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        float f1[8], f2[8];
+        umma::unpack8_bf16(a1[v], f1);
+        umma::unpack8_bf16(a2[v], f2);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) xv[v][e] += f1[e] + f2[e];
       }
+    }
     store_row<V>(dx + r * D, lane, D, xv);
   }
   // block partials: the eight warps' sums added in warp order
@@ -412,9 +443,10 @@ int check_norm(const void* x, const void* gamma, const void* y, long long rows, 
   return MXK_OK;
 }
 
-// Blocks of the backward row pass: two per SM -- enough rows per warp to amortise the partial row every
-// block writes, few enough partials for the fixed-order reduction.  The forward pass takes eight per SM.
-int norm_blocks(long long rows, int per_sm = 2) {
+// Blocks of the row passes.  Backward: those that fit an SM, two at least -- enough rows per warp to amortise the partial row
+// every block writes, few enough partials for the fixed-order reduction.  The forward pass takes eight per SM.
+int norm_bwd_per_sm(int D) { return D <= 256 ? norm_bwd_blocks_per_sm(1) : 2; }
+int norm_blocks(long long rows, int per_sm) {
   const long long want = (rows + kRowWarps - 1) / kRowWarps;
   const long long cap = static_cast<long long>(per_sm) * kNumSMs;
   return static_cast<int>(want < cap ? want : cap);
@@ -484,7 +516,7 @@ int mxk_gated_residual_bf16_bwd_bias(const void* dy, const void* g, const void* 
 
 size_t mxk_norm_bwd_workspace_bytes(long long rows, int D) {
   if (rows <= 0 || D <= 0) return 0;
-  return static_cast<size_t>(mxk::norm_blocks(rows)) * 2 * D * sizeof(float);
+  return static_cast<size_t>(mxk::norm_blocks(rows, mxk::norm_bwd_per_sm(D))) * 2 * D * sizeof(float);
 }
 
 int mxk_norm_bf16_fwd(const void* x, const void* gamma, const void* beta, void* y, float* mean, float* rstd,
@@ -533,7 +565,7 @@ int mxk_norm_bf16_bwd_add(const void* x, const void* gamma, const float* mean, c
   auto* dxp = static_cast<__nv_bfloat16*>(dx);
   float* part = static_cast<float*>(workspace);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const int blocks = norm_blocks(rows), threads = kRowWarps * 32;
+  const int blocks = norm_blocks(rows, norm_bwd_per_sm(D)), threads = kRowWarps * 32;
 #define MXK_NORM_BWD(V)                                                                                  \
   if (rms) mxk::launch_kernel(norm_bwd_kernel<V, true>, blocks, threads, 0, s, xp, gp, nullptr, rstd, dyp, nullptr, nullptr, dxp, part, rows, D); \
   else mxk::launch_kernel(norm_bwd_kernel<V, false>, blocks, threads, 0, s, xp, gp, mean, rstd, dyp, a1, a2, dxp, part, rows, D);
