@@ -288,10 +288,11 @@ struct DeltaLayer : torch::autograd::Function<DeltaLayer> {
                                                        bytes(done), ptr(gs), gq.data_ptr(), gk.data_ptr(), cols_out(gproj, 2 * hid), s.ld, ptr(ga), ptr(gb),
                                                        need_s0 ? ptr(grads[9]) : nullptr, status_ptr(x), s.B, s.T, s.H, s.d, stream()));
     const int rows = l::delta_gate_blocks(s.M);
-    const Tensor part = empty_like_of(x, {rows + 1, 2 * s.H}, at::kFloat);
+    const Tensor part = empty_like_of(x, {rows, 2 * s.H}, at::kFloat);
     check("delta_inputs_bwd", l::delta_inputs_bwd(proj.data_ptr(), s.ld, gate_b.data_ptr(), gq.data_ptr(), gk.data_ptr(), ptr(ga), ptr(gb), gproj.data_ptr(), ptr(part), s.M, s.H,
                                                   s.d, stream()));
-    const l::ColumnSum sum{ptr(part), rows, 2 * s.H, ptr(part) + static_cast<size_t>(rows) * 2 * s.H};
+    grads[5] = empty_like_of(x, {2 * s.H}, at::kBFloat16);
+    const l::ColumnSum sum{ptr(part), rows, 2 * s.H, nullptr, grads[5].data_ptr()};
     check("column_sums", l::column_sums(&sum, 1, stream()));
     if (ctx->needs_input_grad(0)) {
       grads[0] = empty_like_of(x, x.sizes(), at::kBFloat16);
@@ -300,7 +301,6 @@ struct DeltaLayer : torch::autograd::Function<DeltaLayer> {
     const Tensor rows_in = matrix(x, s.M, s.F), gw = product(transposed(matrix(gproj, s.M, 3 * hid, s.ld)), rows_in);
     for (int i = 0; i < 3; ++i) grads[1 + i] = piece(gw, i * hid * s.F, {hid, s.F});
     grads[4] = product(transposed(matrix(gproj, s.M, 2 * s.H, s.ld, 3 * hid)), rows_in);
-    grads[5] = part[rows].to(at::kBFloat16);
     grads[6] = t.norm_w;
     grads[7] = t.out_w;
     grads[8] = t.out_b;

@@ -56,16 +56,16 @@ Result forward(const Tensor& x, const variable_list& p, const Tensor& c0, const 
   r.u = empty_like_of(x, {s.M, s.hid}, bf);
   check("mlstm_conv_fwd", l::mlstm_conv_fwd(r.up.data_ptr(), 2 * s.hid, p[kConvW].data_ptr(), p[kConvB].data_ptr(), r.u.data_ptr(), s.B, s.T, s.hid, st));
   r.qkv = empty_like_of(x, {s.M, 3 * s.hid}, bf);
-  r.qk_w = at::cat({p[kQ], p[kK]}, 1);   // (H, 2d, d)
+  const int64_t gate_w_size = 6ll * s.H * s.hid;
+  const Tensor gates = empty_like_of(x, {gate_w_size + 2 * s.H}, bf);
+  r.qk_w = empty_like_of(x, {s.H, 2 * s.d, s.d}, bf);
+  r.gate_w = piece(gates, 0, {2 * s.H, 3 * s.hid});
+  const Tensor gate_b = piece(gates, gate_w_size, {2 * s.H});
+  check("mlstm_weights", l::mlstm_weights(p[kQ].data_ptr(), p[kK].data_ptr(), p[kIW].data_ptr(), p[kFW].data_ptr(), p[kIB].data_ptr(), p[kFB].data_ptr(),
+                                          r.qk_w.data_ptr(), r.gate_w.data_ptr(), gate_b.data_ptr(), s.H, s.d, st));
   product_into(heads(r.u, 0, s), swapped(r.qk_w), parts(r.qkv, 0, 2, s));
   product_into(heads(r.up, 0, s), swapped(p[kV]), parts(r.qkv, 2, 1, s));
-  r.gate_w = empty_like_of(x, {2 * s.H, 3 * s.hid}, bf);
-  l::WeightRows rows{};
-  rows.count = 2;
-  rows.ptr[0] = p[kIW].data_ptr(); rows.ptr[1] = p[kFW].data_ptr();
-  rows.rows[0] = rows.rows[1] = s.H;
-  check("stack_rows", l::stack_rows(rows, r.gate_w.data_ptr(), 2 * s.H, 3 * s.hid, st));
-  r.logits = product(r.qkv, transposed(r.gate_w), at::cat({p[kIB], p[kFB]}));
+  r.logits = product(r.qkv, transposed(r.gate_w), gate_b);
   r.log_i = empty_like_of(x, {s.M, s.H}, at::kFloat);
   r.log_f = empty_like_of(x, {s.M, s.H}, at::kFloat);
   r.ks = empty_like_of(x, {s.M, s.hid}, bf);
@@ -162,10 +162,10 @@ struct MlstmLayer : torch::autograd::Function<MlstmLayer> {
     product_into(gvalue, p[kV], heads(gx, 0, s));
     check("mlstm_conv_bwd", l::mlstm_conv_bwd(up.data_ptr(), 2 * s.hid, p[kConvW].data_ptr(), p[kConvB].data_ptr(), gu.data_ptr(), gx.data_ptr(), gup.data_ptr(), part_conv, s.B,
                                               s.T, s.hid, st));
-    const Tensor sums = empty_like_of(x, {cols[0] + cols[1] + cols[2]}, at::kFloat);
-    const l::ColumnSum jobs[3] = {{part_out, out_rows, cols[0], ptr(sums)}, {part_gate, gate_rows, cols[1], ptr(sums) + cols[0]}, {part_conv, conv_rows, cols[2], ptr(sums) + cols[0] + cols[1]}};
+    const Tensor small = empty_like_of(x, {cols[0] + cols[1] + cols[2]}, bf);
+    const l::ColumnSum jobs[3] = {{part_out, out_rows, cols[0], nullptr, small.data_ptr()}, {part_gate, gate_rows, cols[1], nullptr, column(small, cols[0])},
+                                  {part_conv, conv_rows, cols[2], nullptr, column(small, cols[0] + cols[1])}};
     check("column_sums", l::column_sums(jobs, 3, st));
-    const Tensor small = sums.to(bf);
     int64_t at = 0;
     const auto give = [&](int i, int64_t n) {
       grads[1 + i] = piece(small, at, p[i].sizes());

@@ -67,6 +67,7 @@ struct ColumnSum {
   const float* src;
   int rows, cols;
   float* dst;
+  void* dst16 = nullptr;   // given: the sums leave in bf16, here
 };
 int column_sums(const ColumnSum* jobs, int count, cudaStream_t stream);   // at most four
 
@@ -128,6 +129,10 @@ int delta_inputs_bwd(const void* qkvg, long long ld, const void* gate_bias, cons
 // u (tokens, hid) = silu(conv(x)), x the first `hid` columns of up (tokens, ld); weights (hid, 4), bias (hid)
 int mlstm_conv_fwd(const void* up, long long ld, const void* conv_w, const void* conv_b, void* u, int B, int T, int hid,
                    cudaStream_t stream);
+// The weights as the layer's products take them, one launch: qk_w (H, 2d, d) = q over k of each head, gate_w (2H, 3 H d) and
+// gate_b (2H) = input gate over forget gate.
+int mlstm_weights(const void* q, const void* k, const void* i_w, const void* f_w, const void* i_b, const void* f_b, void* qk_w, void* gate_w,
+                  void* gate_b, int H, int d, cudaStream_t stream);
 // logits (tokens, 2H) -> log_i, log_f = log sigmoid (tokens, H); k_scaled = k scale, k a slice with pitch ld
 // between steps and hp between heads
 int mlstm_gates_fwd(const void* logits, const void* k, long long ld, int hp, float scale,

@@ -1,5 +1,7 @@
 // The LRU layer's own kernels: a fused single time step (acting), and the gradients of its parameters from those of the
 // real projection matrices.
+#include <cuda_bf16.h>
+
 #include "layers.cuh"
 #include "mxk_common.cuh"
 #include "warp_tile.cuh"
@@ -381,7 +383,8 @@ __global__ void __launch_bounds__(1024) column_sums_kernel(const __grid_constant
     float t = part[0][tx];
 #pragma unroll
     for (int i = 1; i < 32; ++i) t += part[i][tx];
-    jb.dst[col] = t;
+    if (jb.dst16) static_cast<__nv_bfloat16*>(jb.dst16)[col] = __float2bfloat16(t);
+    else jb.dst[col] = t;
   }
 }
 

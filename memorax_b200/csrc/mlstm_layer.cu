@@ -207,6 +207,24 @@ __global__ void __launch_bounds__(256) conv_bwd_kernel(const bf16* __restrict__ 
   }
 }
 
+__global__ void __launch_bounds__(256) weights_kernel(const uint4* __restrict__ q, const uint4* __restrict__ k, const uint4* __restrict__ i_w,
+                                                      const uint4* __restrict__ f_w, const bf16* __restrict__ i_b,
+                                                      const bf16* __restrict__ f_b, uint4* __restrict__ qk_w, uint4* __restrict__ gate_w,
+                                                      bf16* __restrict__ gate_b, int H, int head8, int gate8) {
+  enter_kernel();
+  const int heads = H * head8;
+  int i = blockIdx.x * 256 + threadIdx.x;
+  if (i < 2 * H) gate_b[i] = i < H ? i_b[i] : f_b[i - H];
+  if (i < 2 * heads) {
+    const bool is_k = i >= heads;
+    if (is_k) i -= heads;
+    qk_w[(2 * (i / head8) + is_k) * head8 + i % head8] = (is_k ? k : q)[i];
+  } else if (i - 2 * heads < 2 * gate8) {
+    i -= 2 * heads;
+    gate_w[i] = i < gate8 ? i_w[i] : f_w[i - gate8];
+  }
+}
+
 __global__ void __launch_bounds__(256) gates_fwd_kernel(const bf16* __restrict__ logits, const bf16* __restrict__ k, long long ld,
                                                         float scale, float* __restrict__ log_i, float* __restrict__ log_f,
                                                         bf16* __restrict__ ks, long long tokens, int H, int hid8, int hp, unsigned vec_blocks) {
@@ -427,6 +445,15 @@ int mlstm_conv_bwd(const void* up, long long ld, const void* conv_w, const void*
     return launch_status();
   };
   return run == 16 ? go(conv_bwd_kernel<16>) : go(conv_bwd_kernel<4>);
+}
+
+int mlstm_weights(const void* q, const void* k, const void* i_w, const void* f_w, const void* i_b, const void* f_b, void* qk_w, void* gate_w,
+                  void* gate_b, int H, int d, cudaStream_t stream) {
+  const int head8 = d * d / 8, gate8 = H * 3 * H * d / 8, all = 2 * H * head8 + 2 * gate8;
+  const auto vecs = [](const void* p) { return static_cast<const uint4*>(p); };
+  mxk::launch_kernel(weights_kernel, (all + 255) / 256, 256, 0, stream, vecs(q), vecs(k), vecs(i_w), vecs(f_w), static_cast<const bf16*>(i_b),
+                     static_cast<const bf16*>(f_b), static_cast<uint4*>(qk_w), static_cast<uint4*>(gate_w), static_cast<bf16*>(gate_b), H, head8, gate8);
+  return launch_status();
 }
 
 int mlstm_gates_fwd(const void* logits, const void* k, long long ld, int hp, float scale,
