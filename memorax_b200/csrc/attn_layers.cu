@@ -43,8 +43,8 @@ __global__ void __launch_bounds__(256) stack_rows_kernel(WeightRows w, uint4* __
 // mma.sync fragments, eight consecutive k per lane and load -- the order of k inside a product is free, so those eight
 // serve two k16 steps -- and nothing waits before the last product but the loads themselves.
 __global__ void __launch_bounds__(128) small_product_kernel(const __nv_bfloat16* __restrict__ x, WeightRows w,
-                                                            const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ c,
-                                                            long long ldc, int M, int N, int K) {
+                                                            const __nv_bfloat16* __restrict__ bias, int bias_from,
+                                                            __nv_bfloat16* __restrict__ c, long long ldc, int M, int N, int K) {
   enter_kernel();
   __shared__ float part[4][16][33];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(128) small_product_kernel(const __nv_bfloat16*
     const int r = i >> 5, n = i & 31;
     if (m0 + r < M && n0 + n < N) {
       float v = (part[0][r][n] + part[1][r][n]) + (part[2][r][n] + part[3][r][n]);
-      if (bias) v += bf(bias + n0 + n);
+      if (bias && n0 + n >= bias_from) v += bf(bias + n0 + n - bias_from);
       c[(m0 + r) * ldc + n0 + n] = __float2bfloat16(v);
     }
   }
@@ -187,7 +187,6 @@ __global__ void __launch_bounds__(kStepThreads) linattn_step_kernel(const __nv_b
 
 template <int D>
 __global__ void __launch_bounds__(kStepThreads) gdelta_step_kernel(const __nv_bfloat16* __restrict__ qkvg, long long ld,
-                                                                   const __nv_bfloat16* __restrict__ gate_bias,
                                                                    const float* __restrict__ s0, const uint8_t* __restrict__ done,
                                                                    const __nv_bfloat16* __restrict__ norm_w, float norm_eps,
                                                                    __nv_bfloat16* __restrict__ y, float* __restrict__ s_last, int H) {
@@ -201,8 +200,8 @@ __global__ void __launch_bounds__(kStepThreads) gdelta_step_kernel(const __nv_bf
   const __nv_bfloat16* row = qkvg + b * ld;
   for (int i = tid; i < 3 * hid / 8; i += kStepThreads) unpack8_bf16(*reinterpret_cast<const uint4*>(row + i * 8), sm + i * 8);
   for (int h = tid; h < H; h += kStepThreads) {
-    beta[h] = sigmoid(bf(row + 3 * hid + h) + bf(gate_bias + h));
-    alpha[h] = keep ? __expf(-softplus(bf(row + 3 * hid + H + h) + bf(gate_bias + H + h))) : 0.f;
+    beta[h] = sigmoid(bf(row + 3 * hid + h));
+    alpha[h] = keep ? __expf(-softplus(bf(row + 3 * hid + H + h))) : 0.f;
   }
   __syncthreads();
   for (int i = tid >> 5; i < 2 * H; i += kStepThreads / 32) {   // a warp per head vector of q and k
@@ -278,8 +277,7 @@ struct Walk {   // vector i of the q and k columns is (token, column) = (i / wid
 
 template <int LPH>
 __global__ void __launch_bounds__(256) delta_inputs_kernel(const __nv_bfloat16* __restrict__ qkvg, long long ld,
-                                                           const __nv_bfloat16* __restrict__ gate_bias, uint4* __restrict__ q,
-                                                           uint4* __restrict__ k, float* __restrict__ alpha,
+                                                           uint4* __restrict__ q, uint4* __restrict__ k, float* __restrict__ alpha,
                                                            float* __restrict__ beta, long long tokens, int H, unsigned gate_blocks) {
   enter_kernel();
   const int hid8 = H * LPH;
@@ -316,14 +314,13 @@ __global__ void __launch_bounds__(256) delta_inputs_kernel(const __nv_bfloat16* 
     const long long tok = i / H;
     const int h = static_cast<int>(i % H);
     const __nv_bfloat16* g = qkvg + tok * ld + 3 * hid8 * 8;
-    beta[i] = sigmoid(bf(g + h) + bf(gate_bias + h));
-    alpha[i] = __expf(-softplus(bf(g + H + h) + bf(gate_bias + H + h)));
+    beta[i] = sigmoid(bf(g + h));
+    alpha[i] = __expf(-softplus(bf(g + H + h)));
   }
 }
 
 template <int LPH>
 __global__ void __launch_bounds__(256) delta_inputs_bwd_kernel(const __nv_bfloat16* __restrict__ qkvg, long long ld,
-                                                               const __nv_bfloat16* __restrict__ gate_bias,
                                                                const uint4* __restrict__ dq, const uint4* __restrict__ dk,
                                                                const float* __restrict__ dalpha, const float* __restrict__ dbeta,
                                                                __nv_bfloat16* __restrict__ g, float* __restrict__ partial,
@@ -375,8 +372,8 @@ __global__ void __launch_bounds__(256) delta_inputs_bwd_kernel(const __nv_bfloat
     for (long long tok = static_cast<long long>(blk) * per + ro; tok < tokens; tok += static_cast<long long>(blocks) * per) {
       float v = 0.f;
       if (c < 2 * H) {
-        const float z = bf(qkvg + tok * ld + 3 * hid + c) + bf(gate_bias + c), s = sigmoid(z);
-        v = c < H ? dbeta[tok * H + c] * s * (1.f - s) : -dalpha[tok * H + c - H] * __expf(-softplus(z)) * s;
+        const float z = bf(qkvg + tok * ld + 3 * hid + c), s = sigmoid(z);
+        v = round_bf(c < H ? dbeta[tok * H + c] * s * (1.f - s) : -dalpha[tok * H + c - H] * __expf(-softplus(z)) * s);
       }
       g[tok * ld + 3 * hid + c] = __float2bfloat16(v);
       sum += v;
@@ -405,11 +402,11 @@ int stack_rows(const WeightRows& w, void* dst, int padded, int K, cudaStream_t s
   return launch_status();
 }
 
-int small_product(const void* x, const WeightRows& w, const void* bias, void* c, long long ldc, int M, int K, cudaStream_t stream) {
+int small_product(const void* x, const WeightRows& w, const void* bias, int bias_from, void* c, long long ldc, int M, int K, cudaStream_t stream) {
   if (K % 32 || M <= 0 || w.count < 1 || w.count > kMaxWeights) return MXK_ERR_UNSUPPORTED;
   int N = 0;
   for (int i = 0; i < w.count; ++i) N += w.rows[i];
-  mxk::launch_kernel(small_product_kernel, dim3((N + 31) / 32, (M + 15) / 16), 128, 0, stream, static_cast<const __nv_bfloat16*>(x), w, static_cast<const __nv_bfloat16*>(bias), static_cast<__nv_bfloat16*>(c), ldc, M, N, K);
+  mxk::launch_kernel(small_product_kernel, dim3((N + 31) / 32, (M + 15) / 16), 128, 0, stream, static_cast<const __nv_bfloat16*>(x), w, static_cast<const __nv_bfloat16*>(bias), bias_from, static_cast<__nv_bfloat16*>(c), ldc, M, N, K);
   return launch_status();
 }
 
@@ -426,28 +423,26 @@ int linattn_step(const void* qkv, long long ld, const float* s0, const float* z0
   return launch_status();
 }
 
-int gdelta_step(const void* qkvg, long long ld, const void* gate_bias, const float* s0, const uint8_t* done, const void* norm_w,
+int gdelta_step(const void* qkvg, long long ld, const float* s0, const uint8_t* done, const void* norm_w,
                 float norm_eps, void* y, float* s_last, int B, int H, int d, cudaStream_t stream) {
   const int bytes = (4 * H * d + 2 * H) * static_cast<int>(sizeof(float));
   const auto* x = static_cast<const __nv_bfloat16*>(qkvg);
-  const auto* gb = static_cast<const __nv_bfloat16*>(gate_bias);
   const auto* nw = static_cast<const __nv_bfloat16*>(norm_w);
   auto* out = static_cast<__nv_bfloat16*>(y);
   if (bytes > 48 * 1024) return MXK_ERR_UNSUPPORTED;
-  if (d == 128) mxk::launch_kernel(gdelta_step_kernel<128>, B, kStepThreads, bytes, stream, x, ld, gb, s0, done, nw, norm_eps, out, s_last, H);
-  else if (d == 64) mxk::launch_kernel(gdelta_step_kernel<64>, B, kStepThreads, bytes, stream, x, ld, gb, s0, done, nw, norm_eps, out, s_last, H);
+  if (d == 128) mxk::launch_kernel(gdelta_step_kernel<128>, B, kStepThreads, bytes, stream, x, ld, s0, done, nw, norm_eps, out, s_last, H);
+  else if (d == 64) mxk::launch_kernel(gdelta_step_kernel<64>, B, kStepThreads, bytes, stream, x, ld, s0, done, nw, norm_eps, out, s_last, H);
   else return MXK_ERR_UNSUPPORTED;
   return launch_status();
 }
 
-int delta_inputs(const void* qkvg, long long ld, const void* gate_bias, void* q, void* k, float* alpha, float* beta,
+int delta_inputs(const void* qkvg, long long ld, void* q, void* k, float* alpha, float* beta,
                  long long tokens, int H, int d, cudaStream_t stream) {
   const long long vecs = tokens * 2 * H * (d / 8);
   const unsigned vb = walk_blocks(vecs), gb = static_cast<unsigned>((tokens * H + 255) / 256);
   const auto* x = static_cast<const __nv_bfloat16*>(qkvg);
-  const auto* bias = static_cast<const __nv_bfloat16*>(gate_bias);
-  if (d == 64) mxk::launch_kernel(delta_inputs_kernel<8>, vb + gb, 256, 0, stream, x, ld, bias, static_cast<uint4*>(q), static_cast<uint4*>(k), alpha, beta, tokens, H, gb);
-  else if (d == 128) mxk::launch_kernel(delta_inputs_kernel<16>, vb + gb, 256, 0, stream, x, ld, bias, static_cast<uint4*>(q), static_cast<uint4*>(k), alpha, beta, tokens, H, gb);
+  if (d == 64) mxk::launch_kernel(delta_inputs_kernel<8>, vb + gb, 256, 0, stream, x, ld, static_cast<uint4*>(q), static_cast<uint4*>(k), alpha, beta, tokens, H, gb);
+  else if (d == 128) mxk::launch_kernel(delta_inputs_kernel<16>, vb + gb, 256, 0, stream, x, ld, static_cast<uint4*>(q), static_cast<uint4*>(k), alpha, beta, tokens, H, gb);
   else return MXK_ERR_UNSUPPORTED;
   return launch_status();
 }
@@ -457,16 +452,15 @@ int delta_gate_blocks(long long tokens) {
   return static_cast<int>(need < kGateBlocks ? need : kGateBlocks);
 }
 
-int delta_inputs_bwd(const void* qkvg, long long ld, const void* gate_bias, const void* dq, const void* dk, const float* dalpha,
+int delta_inputs_bwd(const void* qkvg, long long ld, const void* dq, const void* dk, const float* dalpha,
                      const float* dbeta, void* g, float* partial, long long tokens, int H, int d, cudaStream_t stream) {
   if (ld - 3 * H * d > 256 || ld - 3 * H * d < 2 * H) return MXK_ERR_UNSUPPORTED;
   const long long vecs = tokens * 2 * H * (d / 8);
   const unsigned vb = walk_blocks(vecs), gb = static_cast<unsigned>(delta_gate_blocks(tokens));
   const auto* x = static_cast<const __nv_bfloat16*>(qkvg);
-  const auto* bias = static_cast<const __nv_bfloat16*>(gate_bias);
   auto* out = static_cast<__nv_bfloat16*>(g);
-  if (d == 64) mxk::launch_kernel(delta_inputs_bwd_kernel<8>, vb + gb, 256, 0, stream, x, ld, bias, static_cast<const uint4*>(dq), static_cast<const uint4*>(dk), dalpha, dbeta, out, partial, tokens, H, gb);
-  else if (d == 128) mxk::launch_kernel(delta_inputs_bwd_kernel<16>, vb + gb, 256, 0, stream, x, ld, bias, static_cast<const uint4*>(dq), static_cast<const uint4*>(dk), dalpha, dbeta, out, partial, tokens, H, gb);
+  if (d == 64) mxk::launch_kernel(delta_inputs_bwd_kernel<8>, vb + gb, 256, 0, stream, x, ld, static_cast<const uint4*>(dq), static_cast<const uint4*>(dk), dalpha, dbeta, out, partial, tokens, H, gb);
+  else if (d == 128) mxk::launch_kernel(delta_inputs_bwd_kernel<16>, vb + gb, 256, 0, stream, x, ld, static_cast<const uint4*>(dq), static_cast<const uint4*>(dk), dalpha, dbeta, out, partial, tokens, H, gb);
   else return MXK_ERR_UNSUPPORTED;
   return launch_status();
 }

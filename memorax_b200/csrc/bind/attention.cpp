@@ -31,10 +31,11 @@ l::WeightRows rows_of(const variable_list& w, size_t count) {
 }
 
 // x (M, F) -> (M, ld), columns past the weights zero; `stacked` keeps the joint weight for the backward pass
-Tensor project(const Tensor& x, const variable_list& w, size_t count, const Shape& s, Tensor* stacked) {
+// `bias`: of the columns behind q | k | v, added before they are rounded
+Tensor project(const Tensor& x, const variable_list& w, size_t count, const Shape& s, Tensor* stacked, const Tensor& bias = Tensor()) {
   const Tensor proj = empty_like_of(x, {s.M, s.ld}, at::kBFloat16);
   if (!stacked && s.M <= kFewRows && s.F % 32 == 0) {
-    check("small_product", l::small_product(x.data_ptr(), rows_of(w, count), nullptr, proj.data_ptr(), s.ld, s.M, s.F, stream()));
+    check("small_product", l::small_product(x.data_ptr(), rows_of(w, count), ptr<void>(bias), static_cast<int>(3 * s.hid), proj.data_ptr(), s.ld, s.M, s.F, stream()));
     return proj;
   }
   const Tensor joint = empty_like_of(x, {s.ld, s.F}, at::kBFloat16);
@@ -42,9 +43,9 @@ Tensor project(const Tensor& x, const variable_list& w, size_t count, const Shap
   // tiles fit q | k | v; the few columns behind them would cost a tile column (65536 x 3088 x 512 in the library: 198 us
   // against 160 for 3072 and 17 for 16)
   const Tensor rows = matrix(x, s.M, s.F);
-  const int64_t main = 3 * s.hid, rest = s.ld - main;
+  const int64_t main = 3 * s.hid, rest = bias.defined() ? bias.size(0) : 0;
   product_into(rows, transposed(matrix(joint, main, s.F)), matrix(proj, s.M, main, s.ld));
-  if (rest) product_into(rows, transposed(matrix(joint, rest, s.F, 0, main * s.F)), matrix(proj, s.M, rest, s.ld, main));
+  if (rest) product_into(rows, transposed(matrix(joint, rest, s.F, 0, main * s.F)), matrix(proj, s.M, rest, s.ld, main), bias);
   if (stacked) *stacked = joint;
   return proj;
 }
@@ -52,7 +53,7 @@ Tensor project(const Tensor& x, const variable_list& w, size_t count, const Shap
 Tensor output(const Tensor& n, const Tensor& w, const Tensor& bias, const Shape& s, bool few) {
   if (few && s.M <= kFewRows && s.hid % 32 == 0) {
     const Tensor y = empty_like_of(n, {s.B, s.T, s.out}, at::kBFloat16);
-    check("small_product", l::small_product(n.data_ptr(), rows_of({w}, 1), bias.data_ptr(), y.data_ptr(), s.out, s.M, s.hid, stream()));
+    check("small_product", l::small_product(n.data_ptr(), rows_of({w}, 1), bias.data_ptr(), 0, y.data_ptr(), s.out, s.M, s.hid, stream()));
     return y;
   }
   const Tensor y = empty_like_of(n, {s.B, s.T, s.out}, at::kBFloat16);
@@ -229,10 +230,10 @@ struct DeltaResult {
 DeltaResult delta_forward(const Tensor& x, const variable_list& p, const Tensor& s0, const Tensor& done, const Shape& s, double norm_eps, bool keep) {
   DeltaResult r;
   r.s_last = empty_like_of(x, {s.B, 1, s.H, s.d, s.d}, at::kFloat);
-  r.proj = project(x, p, 4, s, keep ? &r.joint : nullptr);
+  r.proj = project(x, p, 4, s, keep ? &r.joint : nullptr, p[kGateB]);
   if (s.T == 1 && !keep && s.hid <= 2048) {
     const Tensor n = empty_like_of(x, {s.M, s.hid}, at::kBFloat16);
-    check("gdelta_step", l::gdelta_step(r.proj.data_ptr(), s.ld, p[kGateB].data_ptr(), ptr(s0), bytes(done), p[kDNorm].data_ptr(), norm_eps, n.data_ptr(),
+    check("gdelta_step", l::gdelta_step(r.proj.data_ptr(), s.ld, ptr(s0), bytes(done), p[kDNorm].data_ptr(), norm_eps, n.data_ptr(),
                                         ptr(r.s_last), s.B, s.H, s.d, stream()));
     r.y = output(n, p[kDOutW], p[kDOutB], s, true);
     return r;
@@ -245,7 +246,7 @@ DeltaResult delta_forward(const Tensor& x, const variable_list& p, const Tensor&
   if (keep) r.states = scratch(x, mxk_gdelta_chunk_states_bytes(s.B, s.T, s.H, s.d));
   const size_t ws_bytes = mxk_gdelta_workspace_bytes(s.B, s.T, s.H, s.d);
   r.ws = scratch(x, ws_bytes);
-  check("delta_inputs", l::delta_inputs(r.proj.data_ptr(), s.ld, p[kGateB].data_ptr(), r.q.data_ptr(), r.k.data_ptr(), ptr(r.alpha), ptr(r.beta), s.M, s.H, s.d, stream()));
+  check("delta_inputs", l::delta_inputs(r.proj.data_ptr(), s.ld, r.q.data_ptr(), r.k.data_ptr(), ptr(r.alpha), ptr(r.beta), s.M, s.H, s.d, stream()));
   check("mxk_gdelta_bf16_fwd", mxk::gdelta::forward(r.q.data_ptr(), r.k.data_ptr(), cols_of(r.proj, 2 * s.hid), s.ld, ptr(r.alpha), ptr(r.beta), ptr(s0), bytes(done),
                                                     r.o.data_ptr(), ptr(r.s_last), ptr<void>(r.states), r.ws.data_ptr(), ws_bytes, status_ptr(x), s.B, s.T, s.H,
                                                     s.d, stream()));
@@ -265,21 +266,21 @@ struct DeltaLayer : torch::autograd::Function<DeltaLayer> {
     ctx->set_materialize_grads(false);
     ctx->saved_data["heads"] = heads;
     ctx->saved_data["s0"] = s0.defined();
-    ctx->save_for_backward({x, gate_b, norm_w, out_w, done, r.proj, r.joint, r.q, r.k, r.alpha, r.beta, r.states, r.ws, r.o, r.tail.n, r.tail.rstd});
+    ctx->save_for_backward({x, norm_w, out_w, done, r.proj, r.joint, r.q, r.k, r.alpha, r.beta, r.states, r.ws, r.o, r.tail.n, r.tail.rstd});
     return {r.s_last, r.y};
   }
 
   static variable_list backward(AutogradContext* ctx, const variable_list& gout) {
     const variable_list saved = ctx->get_saved_variables();
-    const Tensor &x = saved[0], &gate_b = saved[1], &norm_w = saved[2], &out_w = saved[3], &done = saved[4], &proj = saved[5], &joint = saved[6];
-    const Tensor &q = saved[7], &k = saved[8], &alpha = saved[9], &beta = saved[10], &states = saved[11], &ws = saved[12], &o = saved[13];
+    const Tensor &x = saved[0], &norm_w = saved[1], &out_w = saved[2], &done = saved[3], &proj = saved[4], &joint = saved[5];
+    const Tensor &q = saved[6], &k = saved[7], &alpha = saved[8], &beta = saved[9], &states = saved[10], &ws = saved[11], &o = saved[12];
     const c10::cuda::CUDAGuard guard(x.device());
     const int64_t hid = out_w.size(1);
     const Shape s = shape_of(x, ctx->saved_data["heads"].toInt(), hid, out_w.size(0), 2 * ctx->saved_data["heads"].toInt());
     const Tensor gy = matrix(gout[1].defined() ? gout[1].contiguous() : empty_like_of(x, {s.M, s.out}, at::kBFloat16).zero_(), s.M, s.out);
     const Tensor gs = gout[0].defined() ? gout[0].contiguous() : Tensor();
     const bool need_s0 = ctx->saved_data["s0"].toBool() && ctx->needs_input_grad(9);
-    const TailGrads t = tail_backward(gy, o, saved[14], saved[15], norm_w, out_w, s);
+    const TailGrads t = tail_backward(gy, o, saved[13], saved[14], norm_w, out_w, s);
     const Tensor gproj = empty_like_of(x, proj.sizes(), at::kBFloat16), gq = empty_like_of(x, q.sizes(), at::kBFloat16), gk = empty_like_of(x, k.sizes(), at::kBFloat16);
     const Tensor ga = empty_like_of(x, alpha.sizes(), at::kFloat), gb = empty_like_of(x, beta.sizes(), at::kFloat);
     variable_list grads(13);
@@ -289,7 +290,7 @@ struct DeltaLayer : torch::autograd::Function<DeltaLayer> {
                                                        need_s0 ? ptr(grads[9]) : nullptr, status_ptr(x), s.B, s.T, s.H, s.d, stream()));
     const int rows = l::delta_gate_blocks(s.M);
     const Tensor part = empty_like_of(x, {rows, 2 * s.H}, at::kFloat);
-    check("delta_inputs_bwd", l::delta_inputs_bwd(proj.data_ptr(), s.ld, gate_b.data_ptr(), gq.data_ptr(), gk.data_ptr(), ptr(ga), ptr(gb), gproj.data_ptr(), ptr(part), s.M, s.H,
+    check("delta_inputs_bwd", l::delta_inputs_bwd(proj.data_ptr(), s.ld, gq.data_ptr(), gk.data_ptr(), ptr(ga), ptr(gb), gproj.data_ptr(), ptr(part), s.M, s.H,
                                                   s.d, stream()));
     grads[5] = empty_like_of(x, {2 * s.H}, at::kBFloat16);
     const l::ColumnSum sum{ptr(part), rows, 2 * s.H, nullptr, grads[5].data_ptr()};

@@ -108,21 +108,22 @@ struct WeightRows {                 // bf16 matrices (rows[i], K) on top of each
 // dst (padded, K): the stacked rows, then zeros
 int stack_rows(const WeightRows& w, void* dst, int padded, int K, cudaStream_t stream);
 // c (M, ldc) = x (M, K) w^T (+ bias (N) or null) for few rows; K a multiple of 32, columns past the stacked rows untouched
-int small_product(const void* x, const WeightRows& w, const void* bias, void* c, long long ldc, int M, int K, cudaStream_t stream);
+// `bias` belongs to the columns from bias_from on.
+int small_product(const void* x, const WeightRows& w, const void* bias, int bias_from, void* c, long long ldc, int M, int K, cudaStream_t stream);
 // One step of linear attention with its RMSNorm: qkv (B, ld) holds q | k | v of H heads of d (32 or 64); y (B, H d) bf16.
 int linattn_step(const void* qkv, long long ld, const float* s0, const float* z0, const uint8_t* done, const void* norm_w,
                  float norm_eps, float eps, void* y, float* s_last, float* z_last, int B, int H, int d, cudaStream_t stream);
 // One step of the gated delta rule with the normalisation of q and k, the gates and the RMSNorm: qkvg (B, ld) holds
 // q | k | v | beta logits (H) | decay logits (H); d 64 or 128.
-int gdelta_step(const void* qkvg, long long ld, const void* gate_bias, const float* s0, const uint8_t* done, const void* norm_w,
+int gdelta_step(const void* qkvg, long long ld, const float* s0, const uint8_t* done, const void* norm_w,
                 float norm_eps, void* y, float* s_last, int B, int H, int d, cudaStream_t stream);
 // The same normalisation and gates over whole segments: q, k (tokens, H d) bf16, alpha, beta (tokens, H).
-int delta_inputs(const void* qkvg, long long ld, const void* gate_bias, void* q, void* k, float* alpha, float* beta,
+int delta_inputs(const void* qkvg, long long ld, void* q, void* k, float* alpha, float* beta,
                  long long tokens, int H, int d, cudaStream_t stream);
 // dq, dk, dalpha, dbeta -> the q, k and gate columns of g (tokens, ld) (and zeros from `used` to ld);
 // partial: delta_gate_blocks rows of 2 H (the gates' bias gradient).
 int delta_gate_blocks(long long tokens);
-int delta_inputs_bwd(const void* qkvg, long long ld, const void* gate_bias, const void* dq, const void* dk, const float* dalpha,
+int delta_inputs_bwd(const void* qkvg, long long ld, const void* dq, const void* dk, const float* dalpha,
                      const float* dbeta, void* g, float* partial, long long tokens, int H, int d, cudaStream_t stream);
 
 // ---- mLSTM in bf16, mlstm_layer.cu: what is elementwise around its products and its chunk kernels ------------------
