@@ -11,6 +11,8 @@
 //   products 3: O += P U, S += U^T (gam K)
 //   epilogue 3: output tile (one TMA store), bf16 operand copy of the new state
 // Bound: the serial chain of three groups of products a chunk, hidden by two (D = 128) or three (D = 64) CTAs per SM.
+// Measured: 512 x 256 steps, 8 heads of 64: 222 us (408 padded to 128); 128 x 512 steps, 8 heads of 128: 222 us (229 with
+// features on the rows).
 #include <cstddef>
 
 #include "attention.cuh"

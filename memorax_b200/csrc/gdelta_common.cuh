@@ -53,7 +53,8 @@ __host__ __device__ constexpr int residual_vecs(int d) { return state_vecs(d) + 
 __device__ __forceinline__ uint32_t keys_seen(uint64_t dm, int row, int j0) {
   return static_cast<uint32_t>(((2ull << row) - (1ull << row_first_key(dm, row))) >> j0);
 }
-// G_tj = exp(cum_t - cum_j) where bit e is set, 0 elsewhere; selected before the exponential, which a branch would skip.
+// G_tj = exp(cum_t - cum_j) where bit e is set, 0 elsewhere; selected before the exponential: around it the
+// selection became a branch per key, half the time of an epilogue (backward, heads of 64: 517 us a launch against 428).
 __device__ __forceinline__ float decay_between(float cum_t, float cum_j, uint32_t seen, int e) {
   return __expf((seen >> e) & 1u ? cum_t - cum_j : -INFINITY);
 }

@@ -216,7 +216,8 @@ norm_bwd_reduce_kernel(const float* __restrict__ part, float* __restrict__ dgamm
 }
 
 // Column sums of a (rows, cols) bf16 matrix in fp32 -- the bias gradient of a Dense layer -- either as it is (ReadOp) or as
-// the pass that makes it writes it (GeluBwdOp, GatedBwdOp: a pass of its own would read the matrix again).  Block (cx, ry)
+// the pass that makes it writes it (GeluBwdOp, GatedBwdOp: a pass of its own would read the matrix again, 80 us for 131072 x
+// 2048).  Block (cx, ry)
 // owns 256 columns x a contiguous range of rows: its thread (tx, ty) takes 8 columns of every eighth row, the eight thread
 // rows are added in a fixed order, and the block's sums go to part[ry][col]; a second kernel adds the row blocks in order.
 template <class Op>
