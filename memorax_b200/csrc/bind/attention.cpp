@@ -138,7 +138,8 @@ LinResult linattn_forward(const Tensor& x, const variable_list& p, const Tensor&
   r.s_last = empty_like_of(x, {s.B, 1, s.H, s.d, s.d}, at::kFloat);
   r.z_last = empty_like_of(x, {s.B, 1, s.H, s.d}, at::kFloat);
   r.proj = project(x, p, 3, s, keep ? &r.joint : nullptr);
-  if (s.T == 1 && !keep && (s.d == 64 || s.d == 32) && s.hid <= 2048) {
+  // (the chunk kernels take a state from any address)
+  if (s.T == 1 && !keep && (s.d == 64 || s.d == 32) && s.hid <= 2048 && aligned16(s0)) {
     const Tensor n = empty_like_of(x, {s.M, s.hid}, at::kBFloat16);
     check("linattn_step", l::linattn_step(r.proj.data_ptr(), s.ld, ptr(s0), ptr(z0), bytes(done), p[kNorm].data_ptr(), norm_eps, eps, n.data_ptr(),
                                           ptr(r.s_last), ptr(r.z_last), s.B, s.H, s.d, stream()));
@@ -231,7 +232,8 @@ DeltaResult delta_forward(const Tensor& x, const variable_list& p, const Tensor&
   DeltaResult r;
   r.s_last = empty_like_of(x, {s.B, 1, s.H, s.d, s.d}, at::kFloat);
   r.proj = project(x, p, 4, s, keep ? &r.joint : nullptr, p[kGateB]);
-  if (s.T == 1 && !keep && s.hid <= 2048) {
+  // (the chunk kernels report a state that is not aligned)
+  if (s.T == 1 && !keep && s.hid <= 2048 && aligned16(s0)) {
     const Tensor n = empty_like_of(x, {s.M, s.hid}, at::kBFloat16);
     check("gdelta_step", l::gdelta_step(r.proj.data_ptr(), s.ld, ptr(s0), bytes(done), p[kDNorm].data_ptr(), norm_eps, n.data_ptr(),
                                         ptr(r.s_last), s.B, s.H, s.d, stream()));

@@ -20,6 +20,8 @@ inline cudaStream_t stream() { return at::cuda::getCurrentCUDAStream().stream();
 
 template <typename T = float>
 inline T* ptr(const Tensor& t) { return t.defined() ? static_cast<T*>(t.data_ptr()) : nullptr; }
+// What kernels with 16-byte accesses ask of a tensor that a caller brings (one cut out of a larger buffer may start anywhere).
+inline bool aligned16(const Tensor& t) { return !t.defined() || reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; }
 inline const uint8_t* bytes(const Tensor& t) { return t.defined() ? static_cast<const uint8_t*>(t.data_ptr()) : nullptr; }
 
 // The per-device word that a kernel whose bounded wait gave up sets to 1.

@@ -68,3 +68,28 @@ def test_one_step_equals_a_segment_of_one(kind, heads, dim, bsz, with_carry):
         want_c, want = MemoroidCellBase.layer(model.cell, x, done, carry)
     for g, w in zip([got, *got_c], [want, *want_c]):
         _close(g, w, 1e-2)
+
+
+# a carry cut out of a flat buffer starts at any float: linear attention takes it, the delta rule's kernels refuse it
+@pytest.mark.parametrize("kind,heads,dim", [("linattn", 4, 64), ("linattn", 2, 32), ("deltanet", 2, 64), ("deltanet", 8, 128)])
+@pytest.mark.parametrize("offset", [1, 2, 3])
+def test_one_step_from_a_carry_at_any_address(kind, heads, dim, offset):
+    from memorax_b200._lib import MxkError
+    from memorax_b200.memoroid import DeltaNetCell, LinearAttentionCell, Memoroid
+    torch.manual_seed(2)
+    bsz, feat = 5, 128
+    model = Memoroid((LinearAttentionCell if kind == "linattn" else DeltaNetCell)(feat, dim, heads)).cuda().bfloat16()
+    x, done = torch.randn(bsz, 1, feat, device="cuda").bfloat16(), torch.zeros(bsz, 1, dtype=torch.bool, device="cuda")
+    s0 = 0.3 * torch.randn(bsz, 1, heads, dim, dim, device="cuda")
+    flat = torch.zeros(s0.numel() + 4, device="cuda")
+    cut = flat[offset:offset + s0.numel()].view_as(s0).copy_(s0)
+    rest = (torch.rand(bsz, 1, heads, dim, device="cuda"),) if kind == "linattn" else ()
+    with torch.no_grad():
+        if kind == "deltanet":
+            with pytest.raises(MxkError):
+                model(x, done, (cut,))
+            return
+        want_c, want = model(x, done, (s0, *rest))
+        got_c, got = model(x, done, (cut, *rest))
+    for g, w in zip([got, *got_c], [want, *want_c]):
+        _close(g, w, 1e-2)
