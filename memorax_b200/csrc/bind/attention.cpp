@@ -34,7 +34,7 @@ l::WeightRows rows_of(const variable_list& w, size_t count) {
 // `bias`: of the columns behind q | k | v, added before they are rounded
 Tensor project(const Tensor& x, const variable_list& w, size_t count, const Shape& s, Tensor* stacked, const Tensor& bias = Tensor()) {
   const Tensor proj = empty_like_of(x, {s.M, s.ld}, at::kBFloat16);
-  if (!stacked && s.M <= kFewRows && s.F % 32 == 0) {
+  if (!stacked && s.M <= kFewRows && s.F % 32 == 0 && aligned16(x)) {
     check("small_product", l::small_product(x.data_ptr(), rows_of(w, count), ptr<void>(bias), static_cast<int>(3 * s.hid), proj.data_ptr(), s.ld, s.M, s.F, stream()));
     return proj;
   }

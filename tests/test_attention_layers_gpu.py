@@ -93,3 +93,22 @@ def test_one_step_from_a_carry_at_any_address(kind, heads, dim, offset):
         got_c, got = model(x, done, (cut, *rest))
     for g, w in zip([got, *got_c], [want, *want_c]):
         _close(g, w, 1e-2)
+
+
+# inputs cut out of a larger buffer start at any bf16: not for the 16-byte loads of the small products
+@pytest.mark.parametrize("kind,heads,dim", [("linattn", 4, 64), ("deltanet", 2, 64)])
+@pytest.mark.parametrize("bsz,steps", [(7, 1), (2, 70)])
+@pytest.mark.parametrize("offset", [1, 4])
+def test_inputs_at_any_address(kind, heads, dim, bsz, steps, offset):
+    from memorax_b200.memoroid import DeltaNetCell, LinearAttentionCell, Memoroid
+    torch.manual_seed(3)
+    feat = 128
+    model = Memoroid((LinearAttentionCell if kind == "linattn" else DeltaNetCell)(feat, dim, heads)).cuda().bfloat16()
+    x, done = torch.randn(bsz, steps, feat, device="cuda").bfloat16(), torch.rand(bsz, steps, device="cuda") < 0.1
+    flat = torch.zeros(x.numel() + 8, device="cuda", dtype=torch.bfloat16)
+    cut = flat[offset:offset + x.numel()].view_as(x).copy_(x)
+    with torch.no_grad():
+        want_c, want = model(x, done)
+        got_c, got = model(cut, done)
+    for g, w in zip([got, *got_c], [want, *want_c]):
+        _close(g, w, 1e-2)
