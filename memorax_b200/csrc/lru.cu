@@ -283,7 +283,8 @@ template <int kLanes>
 __global__ void __launch_bounds__(256) lru_sensitivities_kernel(LruWeights w, const float* __restrict__ lambda,
                                                                 const float* __restrict__ h, const float* __restrict__ h0,
                                                                 const float* __restrict__ u, const uint8_t* __restrict__ done,
-                                                                LruSensitivities s, int T, int F, int N, int input_blocks) {
+                                                                LruSensitivities s, int T, int F, int N, int input_blocks,
+                                                                bool wide) {
   enter_kernel();
   constexpr int kUnits = 256 / kLanes, kFeatures = 4 * kLanes;
   __shared__ __align__(16) float us[kSensSteps][kFeatures];
@@ -298,7 +299,7 @@ __global__ void __launch_bounds__(256) lru_sensitivities_kernel(LruWeights w, co
   const int n0 = (blockIdx.x % unit_groups) * kUnits, f0 = (blockIdx.x / unit_groups) * kFeatures;
   const int un = threadIdx.x / kLanes, lf = threadIdx.x % kLanes;
   const int n = n0 + un, f = f0 + lf * 4;
-  const bool in = n < N && f < F, wide = F % 4 == 0;
+  const bool in = n < N && f < F;
   const size_t at = (static_cast<size_t>(b) * N + (in ? n : 0)) * F + (in ? f : 0);
   float4 ore[2] = {}, oim[2] = {};   // old sensitivities, on their way while the sums are formed
   if (in && wide) {
@@ -429,10 +430,13 @@ int lru_param_grads(const LruWeights& w, const LruGrads& g, int F, int N, cudaSt
 int lru_sensitivities(const LruWeights& w, const float* lambda, const float* h, const float* h0, const float* u,
                       const uint8_t* done, const LruSensitivities& s, int B, int T, int F, int N, cudaStream_t stream) {
   if (B <= 0 || T <= 0 || F <= 0 || N <= 0 || B > 65535) return MXK_ERR_DIMS;
+  // sixteen-byte accesses to the sensitivities of B: whole vectors per unit, from where they may start
+  bool wide = F % 4 == 0;
+  for (const float* p : {s.b_re, s.b_im, static_cast<const float*>(s.b_re_out), static_cast<const float*>(s.b_im_out)}) wide = wide && aligned16(p);
   // lanes per unit: as many as four features each need, so that narrow inputs leave none idle
   const auto go = [&](auto kernel, int lanes) {
     const int units = 256 / lanes, inputs = ((N + units - 1) / units) * ((F + 4 * lanes - 1) / (4 * lanes));
-    return mxk::launch_kernel(kernel, dim3(inputs + (N + 31) / 32, B), 256, 0, stream, w, lambda, h, h0, u, done, s, T, F, N, inputs);
+    return mxk::launch_kernel(kernel, dim3(inputs + (N + 31) / 32, B), 256, 0, stream, w, lambda, h, h0, u, done, s, T, F, N, inputs, wide);
   };
   if (F <= 32) return go(lru_sensitivities_kernel<8>, 8);
   if (F <= 64) return go(lru_sensitivities_kernel<16>, 16);

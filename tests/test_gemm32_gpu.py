@@ -86,3 +86,22 @@ def test_fused_rtrl_segment_matches_the_oracle(shape, p_done):
     assert err(h, h_ref) <= 1e-5 and err(y, y_ref) <= 1e-5
     for name in s_ref:
         assert err(out[name], s_ref[name]) <= 1e-5, name
+
+
+# sensitivities cut out of a flat buffer start at any complex number; the wide accesses are for 16-byte boundaries
+@pytest.mark.parametrize("feat", [8, 6])
+def test_fused_rtrl_segment_from_sensitivities_at_any_address(feat):
+    from memorax_b200.memoroid import LRUCell, Memoroid
+    torch.manual_seed(4)
+    bsz, steps, hidden = 3, 20, 40
+    model = Memoroid(LRUCell(feat, hidden).cuda())
+    c64 = lambda *s: torch.view_as_complex(torch.randn(*s, 2, device="cuda"))
+    x, done = torch.randn(bsz, steps, feat, device="cuda"), torch.rand(bsz, steps, device="cuda") < 0.1
+    carry = (c64(bsz, 1, hidden), torch.ones(bsz, 1, hidden, dtype=torch.complex64, device="cuda"))
+    sens = {k: c64(*v.shape) for k, v in model.initialize_sensitivity(None, (bsz, feat)).items()}
+    cut = {k: torch.zeros(v.numel() + 1, dtype=torch.complex64, device="cuda")[1:].view_as(v).copy_(v) for k, v in sens.items()}
+    with torch.no_grad():
+        *_, want = model.local_jacobian(x, done, carry, sens)
+        *_, got = model.local_jacobian(x, done, carry, cut)
+    for k in want:
+        assert torch.equal(got[k], want[k]), k
