@@ -12,7 +12,7 @@ import torch
 from torch import nn
 
 from . import ops
-from .memoroid import DeltaNetCell, Memoroid
+from .memoroid import DeltaNetCell, Memoroid, plain
 
 
 class PreNorm(nn.Module):
@@ -32,12 +32,6 @@ class Dense(nn.Linear):
         return ops.dense(x, self.weight, self.bias)
 
 
-def _plain(module, kind):
-    """A module of exactly this kind without hooks: what a composition may call through its parts."""
-    return type(module) is kind and not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks
-                                         or module._backward_pre_hooks)
-
-
 class GatedResidual(nn.Module):
     def __init__(self, module, features):
         super().__init__()
@@ -45,7 +39,7 @@ class GatedResidual(nn.Module):
 
     def forward(self, inputs, done=None, initial_carry=None):
         fork = None
-        if _plain(self.module, PreNorm):   # the norm, the gate and the sum read the same inputs
+        if plain(self.module, PreNorm):   # the norm, the gate and the sum read the same inputs
             norm = self.module.norm
             fork = ops.norm_fork(inputs, norm.weight, norm.bias, norm.eps)
         if fork is not None:
@@ -54,7 +48,7 @@ class GatedResidual(nn.Module):
         else:
             gated = inputs
             carry, out = self.module(inputs, done, initial_carry)
-        if _plain(self.gate, Dense):
+        if plain(self.gate, Dense):
             return carry, ops.gated_dense(inputs, gated, self.gate, out)
         return carry, ops.gated_residual(inputs, self.gate(gated), out)
 
@@ -65,7 +59,7 @@ class FFN(nn.Module):
         self.up, self.down = Dense(features, features * expansion_factor), Dense(features * expansion_factor, features)
 
     def forward(self, inputs, done=None, initial_carry=None):
-        return None, self.down(ops.dense_gelu(inputs, self.up) if _plain(self.up, Dense) else ops.gelu(self.up(inputs)))
+        return None, self.down(ops.dense_gelu(inputs, self.up) if plain(self.up, Dense) else ops.gelu(self.up(inputs)))
 
 
 class Stack(nn.Module):

@@ -27,21 +27,52 @@ import math
 import torch
 from torch import nn
 from torch.nn import functional as F
+from torch.nn.modules.module import _has_any_global_hook
 
 from . import _C, ops
 
 
-def _weights_of(module, names):
-    """Parameters by ``submodule.kind`` out of the module dictionaries (an attribute lookup through ``nn.Module`` per
-    parameter costs more than a launch), or None where a submodule is not the plain kind the native layers know."""
+def plain(module, kind):
+    """Whether calling ``module`` runs ``kind.forward`` and nothing else: exactly this class, without hooks (weight norm and
+    pruning are hooks too) and without a ``forward`` of its own.  Only such a module may be called through its parts."""
+    return (type(module) is kind and not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks
+                                          or module._backward_pre_hooks)
+            and "forward" not in module.__dict__ and not _has_any_global_hook())
+
+
+def native_params(cell, kind, spec):
+    """The parameters that the native layer of a ``kind`` takes, or None where the layer has to be composed: the cell or one
+    of its submodules is not plain, or has other parameters than these.  ``spec`` names them in order: (submodule or None for
+    the cell's own, its class, names).  They come out of the module dictionaries: an attribute lookup through ``nn.Module``
+    per parameter costs more than a launch."""
+    if not plain(cell, kind):
+        return None
     out = []
-    for name in names:
-        sub, kind = name.split(".")
-        sub = module._modules[sub]
-        if type(sub) not in (nn.Linear, nn.RMSNorm):
-            return None
-        out.append(sub._parameters[kind])
-    return None if any(t is None for t in out) else out
+    for sub, sub_kind, names in spec:
+        module = cell
+        if sub is not None:
+            module = cell._modules.get(sub)
+            if not plain(module, sub_kind):
+                return None
+            for name, param in module._parameters.items():
+                if param is not None and name not in names:   # (a bias that the cell was not built with)
+                    return None
+        for name in names:
+            param = module._parameters.get(name)
+            if param is None:
+                return None
+            out.append(param)
+    return out
+
+
+def _causal_taps(conv, taps):
+    """Whether a Conv1d is the causal convolution that the native layers know: ``taps`` steps one apart, zeros in front."""
+    return (conv.kernel_size, conv.stride, conv.padding, conv.dilation, conv.padding_mode) == ((taps,), (1,), (taps - 1,), (1,), "zeros")
+
+
+def _normed(norm, x):
+    """``norm(x)`` for an RMSNorm, through the fused kernels where nothing but its forward would run."""
+    return ops.rms_norm(x, norm.weight, norm.eps) if plain(norm, nn.RMSNorm) and norm.eps is not None else norm(x)
 
 
 def get_input_shape(inputs):
@@ -269,7 +300,7 @@ class _ComplexDiagonalCell(MemoroidCellBase):
 
 # ---------------------------------------------------------------------- LRU
 _LRU_SENSITIVITIES = ("B_imag", "B_real", "gamma_log", "nu_log", "theta_log")
-_LRU_PARAMS = ("nu_log", "theta_log", "gamma_log", "B_real", "B_imag", "C_real", "C_imag", "D")
+_LRU_PARAMS = ((None, None, ("nu_log", "theta_log", "gamma_log", "B_real", "B_imag", "C_real", "C_imag", "D")),)
 
 
 class LRUCell(_ComplexDiagonalCell):
@@ -292,9 +323,10 @@ class LRUCell(_ComplexDiagonalCell):
     def layer(self, inputs, done, initial_carry, **kwargs):
         """Projections, scan and read-out as one native call (float32); its backward pass is one autograd node.  A
         subclass, or a call the fused layer does not cover, is composed from its parts."""
-        if type(self) is LRUCell and not kwargs:
+        params = native_params(self, LRUCell, _LRU_PARAMS) if not kwargs else None
+        if params is not None:
             h0, a0 = (None, None) if initial_carry is None else initial_carry
-            out = _C.lru_layer(inputs, [self._parameters[name] for name in _LRU_PARAMS], h0, a0, done)
+            out = _C.lru_layer(inputs, params, h0, a0, done)
             if out is not None:
                 return (out[0], out[1]), out[2]
         return super().layer(inputs, done, initial_carry, **kwargs)
@@ -302,10 +334,12 @@ class LRUCell(_ComplexDiagonalCell):
     def jacobian_segment(self, inputs, done, carry, sensitivity):
         """The segment without gradients: the local Jacobians are never formed, the sensitivities are updated from the
         states and the inputs by two kernels."""
-        if type(self) is not LRUCell or done is None or sensitivity.keys() != set(_LRU_SENSITIVITIES):
+        if done is None or sensitivity.keys() != set(_LRU_SENSITIVITIES):
             return None
-        out = _C.lru_rtrl(inputs, [self._parameters[name] for name in _LRU_PARAMS], carry[0], carry[1], done,
-                          [sensitivity[name] for name in _LRU_SENSITIVITIES])
+        params = native_params(self, LRUCell, _LRU_PARAMS)
+        if params is None:
+            return None
+        out = _C.lru_rtrl(inputs, params, carry[0], carry[1], done, [sensitivity[name] for name in _LRU_SENSITIVITIES])
         return None if out is None else ((out[0], out[1]), out[2], dict(zip(_LRU_SENSITIVITIES, out[3])))
 
     def diag_lambda(self):
@@ -355,6 +389,9 @@ class MinGRUPreactivations(tuple):
     """(z, h_tilde): what ``MinGRUCell`` hands its fused scan instead of the (log_state, decay) elements."""
 
 
+_MINGRU_PARAMS = (("z", nn.Linear, ("weight",)), ("h", nn.Linear, ("weight",)))
+
+
 class MinGRUCell(MemoroidCellBase):
     """Log-space minimal GRU (min_gru.py:14-90).  With ``fused_gates`` (default) the gate math of
     min_gru.py:52-61 runs inside the scan kernels: ``forward`` returns the two Dense pre-activations and the
@@ -374,11 +411,10 @@ class MinGRUCell(MemoroidCellBase):
 
     def layer(self, inputs, done, initial_carry, **kwargs):
         """Dense layers, gates, scan and read-out as one native call (float32); see ``LRUCell.layer``."""
-        z, h = self._modules["z"], self._modules["h"]
-        if (type(self) is MinGRUCell and self.fused_gates and not kwargs and type(z) is nn.Linear and type(h) is nn.Linear
-                and z.bias is None and h.bias is None):
+        params = native_params(self, MinGRUCell, _MINGRU_PARAMS) if not kwargs and self.fused_gates else None
+        if params is not None:
             x0, a0 = (None, None) if initial_carry is None else initial_carry
-            out = _C.mingru_layer(inputs, z._parameters["weight"], h._parameters["weight"], x0, a0, done)
+            out = _C.mingru_layer(inputs, *params, x0, a0, done)
             if out is not None:
                 return (out[0], out[1]), out[2]
         return super().layer(inputs, done, initial_carry, **kwargs)
@@ -419,8 +455,8 @@ class MinGRUCell(MemoroidCellBase):
 
 
 # --------------------------------------------------------- linear attention
-_LINATTN_PARAMS = ("query.weight", "key.weight", "value.weight", "norm.weight", "output_projection.weight",
-                   "output_projection.bias")
+_LINATTN_PARAMS = (("query", nn.Linear, ("weight",)), ("key", nn.Linear, ("weight",)), ("value", nn.Linear, ("weight",)),
+                   ("norm", nn.RMSNorm, ("weight",)), ("output_projection", nn.Linear, ("weight", "bias")))
 
 
 class LinearAttentionCell(MemoroidCellBase):
@@ -439,10 +475,10 @@ class LinearAttentionCell(MemoroidCellBase):
 
     def layer(self, inputs, done, initial_carry, **kwargs):
         """The whole layer as one native call (bf16); other dtypes, and subclasses, are composed from their parts."""
-        weights = _weights_of(self, _LINATTN_PARAMS) if type(self) is LinearAttentionCell and not kwargs else None
-        if weights is not None:
+        params = native_params(self, LinearAttentionCell, _LINATTN_PARAMS) if not kwargs else None
+        if params is not None and self._modules["norm"].eps is not None:
             s0, z0 = (None, None) if initial_carry is None else initial_carry
-            out = _C.linattn_layer(inputs, weights, s0, z0, done, self.num_heads, self.eps, self._modules["norm"].eps)
+            out = _C.linattn_layer(inputs, params, s0, z0, done, self.num_heads, self.eps, self._modules["norm"].eps)
             if out is not None:
                 return (out[0], out[1]), out[2]
         return super().layer(inputs, done, initial_carry, **kwargs)
@@ -474,13 +510,14 @@ class LinearAttentionCell(MemoroidCellBase):
         bf = torch.bfloat16
         o, s_last, z_last = ops.LinAttn.apply(q.to(bf), k.to(bf), v.to(bf), s0, z0, done, self.eps, True)
         o = o.reshape(*o.shape[:2], -1).to(inputs.dtype)
-        y = ops.dense(ops.rms_norm(o, self.norm.weight, self.norm.eps), self.output_projection.weight, self.output_projection.bias)
+        y = ops.dense(_normed(self.norm, o), self.output_projection.weight, self.output_projection.bias)
         return (s_last[:, None], z_last[:, None]), y
 
 
 # ------------------------------------------------------- gated delta rule
-_DELTANET_PARAMS = ("query.weight", "key.weight", "value.weight", "gate.weight", "gate.bias", "norm.weight",
-                    "output_projection.weight", "output_projection.bias")
+_DELTANET_PARAMS = (("query", nn.Linear, ("weight",)), ("key", nn.Linear, ("weight",)), ("value", nn.Linear, ("weight",)),
+                    ("gate", nn.Linear, ("weight", "bias")), ("norm", nn.RMSNorm, ("weight",)),
+                    ("output_projection", nn.Linear, ("weight", "bias")))
 
 
 class DeltaNetCell(MemoroidCellBase):
@@ -508,9 +545,9 @@ class DeltaNetCell(MemoroidCellBase):
 
     def layer(self, inputs, done, initial_carry, **kwargs):
         """The whole layer as one native call (bf16); see ``LinearAttentionCell.layer``."""
-        weights = _weights_of(self, _DELTANET_PARAMS) if type(self) is DeltaNetCell and not kwargs else None
-        if weights is not None:
-            out = _C.deltanet_layer(inputs, weights, None if initial_carry is None else initial_carry[0], done, self.num_heads,
+        params = native_params(self, DeltaNetCell, _DELTANET_PARAMS) if not kwargs else None
+        if params is not None and self._modules["norm"].eps is not None:
+            out = _C.deltanet_layer(inputs, params, None if initial_carry is None else initial_carry[0], done, self.num_heads,
                                     self._modules["norm"].eps)
             if out is not None:
                 return (out[0],), out[1]
@@ -542,11 +579,16 @@ class DeltaNetCell(MemoroidCellBase):
         bf = torch.bfloat16
         o, s_last = ops.GatedDelta.apply(q.to(bf), k.to(bf), v.to(bf), alpha.contiguous(), beta.contiguous(), s0, done)
         o = o.reshape(*o.shape[:2], -1).to(inputs.dtype)
-        return (s_last[:, None],), ops.dense(ops.rms_norm(o, self.norm.weight, self.norm.eps), self.output_projection.weight,
-                                          self.output_projection.bias)
+        return (s_last[:, None],), ops.dense(_normed(self.norm, o), self.output_projection.weight, self.output_projection.bias)
 
 
 # -------------------------------------------------------------------- mLSTM
+_MLSTM_PARAMS = (("up_projection", nn.Linear, ("weight",)), ("causal_conv", nn.Conv1d, ("weight", "bias")),
+                 (None, None, ("query", "key", "value")), ("i_gate", nn.Linear, ("weight", "bias")),
+                 ("f_gate", nn.Linear, ("weight", "bias")), (None, None, ("learnable_skip", "norm_weight")),
+                 ("output_projection", nn.Linear, ("weight",)))
+
+
 class mLSTMCell(MemoroidCellBase):
     """Matrix-memory LSTM (mlstm.py:31-240): gated linear attention with a per-head scalar forget gate and
     the running-max stabiliser.  Projections as the reference (up-projection, causal depthwise convolution +
@@ -585,14 +627,10 @@ class mLSTMCell(MemoroidCellBase):
 
     def layer(self, inputs, done, initial_carry, **kwargs):
         """On the tensor cores in bf16 the whole layer is one native call; everything else is composed from its parts."""
-        if type(self) is mLSTMCell and self.tensor_cores and not kwargs:
+        params = native_params(self, mLSTMCell, _MLSTM_PARAMS) if self.tensor_cores and not kwargs else None
+        if params is not None and _causal_taps(self._modules["causal_conv"], 4):
             c0, f0, n0, m0 = (None,) * 4 if initial_carry is None else initial_carry
-            own, sub = self._parameters, self._modules
-            of = lambda name, kind="weight": sub[name]._parameters[kind]
-            out = _C.mlstm_layer(inputs, [of("up_projection"), of("causal_conv"), of("causal_conv", "bias"), own["query"], own["key"],
-                                          own["value"], of("i_gate"), of("i_gate", "bias"), of("f_gate"), of("f_gate", "bias"),
-                                          own["learnable_skip"], own["norm_weight"], of("output_projection")], c0, f0, n0, m0, done,
-                                 self.eps)
+            out = _C.mlstm_layer(inputs, params, c0, f0, n0, m0, done, self.eps)
             if out is not None:
                 return out[:4], out[4]
         return super().layer(inputs, done, initial_carry, **kwargs)
@@ -726,6 +764,11 @@ class S5Cell(_ComplexDiagonalCell):
 
 
 # -------------------------------------------------------------------- Mamba
+_MAMBA_PARAMS = ((None, None, ("A_log", "D", "dt_bias")), ("input_projection", nn.Linear, ("weight",)), ("B", nn.Linear, ("weight",)),
+                 ("C", nn.Linear, ("weight",)), ("dt", nn.Linear, ("weight",)), ("conv", nn.Conv1d, ("weight", "bias")),
+                 ("norm", nn.RMSNorm, ("weight",)), ("output_projection", nn.Linear, ("weight", "bias")))
+
+
 class MambaCell(MemoroidCellBase):
     """Selective state-space cell (mamba.py:33-150): per head a (state_dim x head_dim) matrix
     state with one scalar decay per (b, t, head).  Elements and read-out follow the
@@ -759,13 +802,12 @@ class MambaCell(MemoroidCellBase):
     def layer(self, inputs, done, initial_carry, **kwargs):
         """The whole layer as one native call (float32, heads of 16 x 16 states, four taps): the (B, T, H, N, P) elements
         and states are never formed.  Other shapes, and subclasses, are composed from their parts."""
-        if type(self) is MambaCell and not kwargs and (self.head_dim, self.state_dim, self.conv_dim) == (16, 16, 4):
+        params = None
+        if not kwargs and (self.head_dim, self.state_dim, self.conv_dim) == (16, 16, 4):
+            params = native_params(self, MambaCell, _MAMBA_PARAMS)
+        if params is not None and self._modules["norm"].eps is not None and _causal_taps(self._modules["conv"], 4):
             h0, a0 = (None, None) if initial_carry is None else initial_carry
-            own, sub = self._parameters, self._modules
-            of = lambda name, kind="weight": sub[name]._parameters[kind]
-            out = _C.mamba_layer(inputs, [own["A_log"], own["D"], own["dt_bias"], of("input_projection"), of("B"), of("C"), of("dt"),
-                                          of("conv"), of("conv", "bias"), of("norm"), of("output_projection"),
-                                          of("output_projection", "bias")], h0, a0, done, self.norm.eps)
+            out = _C.mamba_layer(inputs, params, h0, a0, done, self._modules["norm"].eps)
             if out is not None:
                 return (out[0], out[1]), out[2]
         return super().layer(inputs, done, initial_carry, **kwargs)
