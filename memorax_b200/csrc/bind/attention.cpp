@@ -207,9 +207,11 @@ variable_list LinAttnLayer::backward(AutogradContext* ctx, const variable_list& 
 pybind11::object linattn_layer(const Tensor& x_in, const variable_list& p, const OptTensor& s0_in, const OptTensor& z0_in, const OptTensor& done_in,
                                int64_t heads, double eps, double norm_eps) {
   if (!all_bf16(x_in, p) || p.size() != kLinParams) return pybind11::none();
-  const int64_t hid = p[kQ].size(0), F = x_in.size(2), d = hid / heads;
-  if (d * heads != hid || d % 8 || d < 8 || d > 64 || hid > 1024 || F % 8 || p[kQ].size(1) != F || p[kOutW].size(1) != hid || p[kOutW].size(0) % 8 ||
-      x_in.size(0) * heads > 0x7fffffff)
+  if (p[kQ].dim() != 2 || p[kOutW].dim() != 2 || heads < 1) return pybind11::none();
+  const int64_t hid = p[kQ].size(0), F = x_in.size(2), d = hid / heads, out_dim = p[kOutW].size(0);
+  if (d * heads != hid || d % 8 || d < 8 || d > 64 || hid > 1024 || F % 8 || out_dim % 8 || x_in.size(0) * heads > 0x7fffffff) return pybind11::none();
+  if (!shaped(p[kQ], {hid, F}) || !shaped(p[kK], {hid, F}) || !shaped(p[kV], {hid, F}) || !shaped(p[kNorm], {hid}) || !shaped(p[kOutW], {out_dim, hid}) ||
+      !shaped(p[kOutB], {out_dim}))
     return pybind11::none();
   const c10::cuda::CUDAGuard guard(x_in.device());
   const Tensor x = x_in.contiguous(), s0 = carry_leaf(s0_in, x.size(0) * hid * d, at::kFloat, "s0"), z0 = carry_leaf(z0_in, x.size(0) * hid, at::kFloat, "z0"), done = done_bytes(done_in, x.size(0) * x.size(1));
@@ -314,9 +316,11 @@ struct DeltaLayer : torch::autograd::Function<DeltaLayer> {
 // -> (s_last (B,1,H,d,d), y (B,T,F)), or None
 pybind11::object deltanet_layer(const Tensor& x_in, const variable_list& p, const OptTensor& s0_in, const OptTensor& done_in, int64_t heads, double norm_eps) {
   if (!all_bf16(x_in, p) || p.size() != kDeltaParams) return pybind11::none();
-  const int64_t hid = p[kDq].size(0), F = x_in.size(2), d = hid / heads;
-  if (d * heads != hid || (d != 64 && d != 128) || hid > 1024 || heads > 64 || F % 8 || p[kDq].size(1) != F || p[kDOutW].size(1) != hid || p[kDOutW].size(0) % 8 ||
-      p[kGateW].size(0) != 2 * heads || x_in.size(0) * heads > 0x7fffffff)
+  if (p[kDq].dim() != 2 || p[kDOutW].dim() != 2 || heads < 1) return pybind11::none();
+  const int64_t hid = p[kDq].size(0), F = x_in.size(2), d = hid / heads, out_dim = p[kDOutW].size(0);
+  if (d * heads != hid || (d != 64 && d != 128) || hid > 1024 || heads > 64 || F % 8 || out_dim % 8 || x_in.size(0) * heads > 0x7fffffff) return pybind11::none();
+  if (!shaped(p[kDq], {hid, F}) || !shaped(p[kDk], {hid, F}) || !shaped(p[kDv], {hid, F}) || !shaped(p[kGateW], {2 * heads, F}) || !shaped(p[kGateB], {2 * heads}) ||
+      !shaped(p[kDNorm], {hid}) || !shaped(p[kDOutW], {out_dim, hid}) || !shaped(p[kDOutB], {out_dim}))
     return pybind11::none();
   const c10::cuda::CUDAGuard guard(x_in.device());
   const Tensor x = x_in.contiguous(), s0 = carry_leaf(s0_in, x.size(0) * hid * d, at::kFloat, "s0"), done = done_bytes(done_in, x.size(0) * x.size(1));

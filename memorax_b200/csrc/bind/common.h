@@ -83,6 +83,7 @@ inline Tensor last_state(const Tensor& h) {
   const int64_t B = h.size(0), T = h.size(1), N = h.size(2);
   return view_of(h, (T - 1) * N, {B, 1, N}, {T * N, N, 1});
 }
+inline bool shaped(const Tensor& t, at::IntArrayRef sizes) { return t.sizes() == sizes; }
 inline size_t align_up(size_t n) { return (n + 255) & ~static_cast<size_t>(255); }
 
 // One allocation cut into 256-byte aligned pieces.

@@ -166,8 +166,14 @@ struct LruLayer : torch::autograd::Function<LruLayer> {
 bool native(const Tensor& x, const variable_list& params) {
   if (!x.is_cuda() || x.dim() != 3 || x.numel() == 0 || !x.is_floating_point() || x.scalar_type() == at::kDouble ||
       (x.size(1) > 1 && at::globalContext().allowTF32CuBLAS()) || at::autocast::is_autocast_enabled(at::kCUDA) ||
-      x.size(0) * x.size(1) > 0x7fffffff || params[3].dim() != 2 || x.size(2) != params[3].size(1))
+      x.size(0) * x.size(1) > 0x7fffffff || params.size() != kParams || params[3].dim() != 2)
     return false;
+  const int64_t N = params[3].size(0), F = x.size(2);
+  for (int i : {0, 1, 2})
+    if (!shaped(params[i], {N})) return false;
+  for (int i : {3, 4})
+    if (!shaped(params[i], {N, F}) || !shaped(params[i + 2], {F, N})) return false;
+  if (!shaped(params[7], {F})) return false;
   for (const Tensor& p : params)
     if (p.scalar_type() != at::kFloat || p.device() != x.device() || !p.is_contiguous()) return false;
   return true;

@@ -151,9 +151,11 @@ pybind11::object mamba_layer(const Tensor& x_in, const variable_list& p, const O
     return pybind11::none();
   for (const Tensor& t : p)
     if (t.scalar_type() != at::kFloat || t.device() != x_in.device() || !t.is_contiguous()) return pybind11::none();
-  const int64_t H = p[kALog].size(0), F = x_in.size(2);
-  if (p[kIn].sizes() != at::IntArrayRef({32 * H, F}) || p[kB].sizes() != at::IntArrayRef({16 * H, F}) || p[kC].sizes() != at::IntArrayRef({16 * H, F}) ||
-      p[kDt].sizes() != at::IntArrayRef({H, F}) || p[kConvW].sizes() != at::IntArrayRef({48 * H, 1, 4}) || p[kOutW].size(1) != 16 * H || x_in.size(0) * H > 0x7fffffff)
+  if (p[kALog].dim() != 1 || p[kOutW].dim() != 2) return pybind11::none();
+  const int64_t H = p[kALog].size(0), F = x_in.size(2), out_dim = p[kOutW].size(0);
+  if (!shaped(p[kD], {H}) || !shaped(p[kDtBias], {H}) || !shaped(p[kIn], {32 * H, F}) || !shaped(p[kB], {16 * H, F}) || !shaped(p[kC], {16 * H, F}) ||
+      !shaped(p[kDt], {H, F}) || !shaped(p[kConvW], {48 * H, 1, 4}) || !shaped(p[kConvB], {48 * H}) || !shaped(p[kNormW], {16 * H}) ||
+      !shaped(p[kOutW], {out_dim, 16 * H}) || !shaped(p[kOutB], {out_dim}) || x_in.size(0) * H > 0x7fffffff)
     return pybind11::none();
   const c10::cuda::CUDAGuard guard(x_in.device());
   const Tensor x = x_in.contiguous(), h0 = carry_leaf(h0_in, x.size(0) * H * 256, at::kFloat, "h0"), a0 = carry_leaf(a0_in, x.size(0) * H, at::kFloat, "a0"), done = done_bytes(done_in, x.size(0) * x.size(1));

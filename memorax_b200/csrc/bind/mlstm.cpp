@@ -197,9 +197,12 @@ pybind11::object mlstm_layer(const Tensor& x_in, const variable_list& p, const O
     return pybind11::none();
   for (const Tensor& t : p)
     if (t.scalar_type() != at::kBFloat16 || t.device() != x_in.device() || !t.is_contiguous() || (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15)) return pybind11::none();
-  const int64_t H = p[kQ].size(0), d = p[kQ].size(1), hid = H * d, F = x_in.size(2);
-  if ((d != 16 && d != 32 && d != 64) || H > 64 || hid > 2048 || 256 % (hid / 8 > 0 ? hid / 8 : 1) || p[kUp].sizes() != at::IntArrayRef({2 * hid, F}) ||
-      p[kConvW].sizes() != at::IntArrayRef({hid, 1, 4}) || p[kOut].size(1) != hid || x_in.size(0) * H > 0x7fffffff)
+  if (p[kQ].dim() != 3 || p[kOut].dim() != 2) return pybind11::none();
+  const int64_t H = p[kQ].size(0), d = p[kQ].size(1), hid = H * d, F = x_in.size(2), out_dim = p[kOut].size(0);
+  if ((d != 16 && d != 32 && d != 64) || H > 64 || hid > 2048 || 256 % (hid / 8 > 0 ? hid / 8 : 1) || x_in.size(0) * H > 0x7fffffff) return pybind11::none();
+  if (!shaped(p[kUp], {2 * hid, F}) || !shaped(p[kConvW], {hid, 1, 4}) || !shaped(p[kConvB], {hid}) || !shaped(p[kQ], {H, d, d}) || !shaped(p[kK], {H, d, d}) ||
+      !shaped(p[kV], {H, d, d}) || !shaped(p[kIW], {H, 3 * hid}) || !shaped(p[kIB], {H}) || !shaped(p[kFW], {H, 3 * hid}) || !shaped(p[kFB], {H}) ||
+      !shaped(p[kSkip], {hid}) || !shaped(p[kNorm], {H, d}) || !shaped(p[kOut], {out_dim, hid}))
     return pybind11::none();
   const c10::cuda::CUDAGuard guard(x_in.device());
   const int64_t B = x_in.size(0);
