@@ -206,7 +206,7 @@ variable_list LinAttnLayer::backward(AutogradContext* ctx, const variable_list& 
 // -> (s_last (B,1,H,d,d), z_last (B,1,H,d), y (B,T,F)), or None where the caller has to compose the layer
 pybind11::object linattn_layer(const Tensor& x_in, const variable_list& p, const OptTensor& s0_in, const OptTensor& z0_in, const OptTensor& done_in,
                                int64_t heads, double eps, double norm_eps) {
-  if (!all_bf16(x_in, p) || p.size() != kLinParams) return pybind11::none();
+  if (!all_bf16(x_in, p) || p.size() != kLinParams || followed(x_in, p, s0_in, z0_in)) return pybind11::none();
   if (p[kQ].dim() != 2 || p[kOutW].dim() != 2 || heads < 1) return pybind11::none();
   const int64_t hid = p[kQ].size(0), F = x_in.size(2), d = hid / heads, out_dim = p[kOutW].size(0);
   if (d * heads != hid || d % 8 || d < 8 || d > 64 || hid > 1024 || F % 8 || out_dim % 8 || x_in.size(0) * heads > 0x7fffffff) return pybind11::none();
@@ -315,7 +315,7 @@ struct DeltaLayer : torch::autograd::Function<DeltaLayer> {
 
 // -> (s_last (B,1,H,d,d), y (B,T,F)), or None
 pybind11::object deltanet_layer(const Tensor& x_in, const variable_list& p, const OptTensor& s0_in, const OptTensor& done_in, int64_t heads, double norm_eps) {
-  if (!all_bf16(x_in, p) || p.size() != kDeltaParams) return pybind11::none();
+  if (!all_bf16(x_in, p) || p.size() != kDeltaParams || followed(x_in, p, s0_in)) return pybind11::none();
   if (p[kDq].dim() != 2 || p[kDOutW].dim() != 2 || heads < 1) return pybind11::none();
   const int64_t hid = p[kDq].size(0), F = x_in.size(2), d = hid / heads, out_dim = p[kDOutW].size(0);
   if (d * heads != hid || (d != 64 && d != 128) || hid > 1024 || heads > 64 || F % 8 || out_dim % 8 || x_in.size(0) * heads > 0x7fffffff) return pybind11::none();

@@ -5,6 +5,7 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/extension.h>
 
 #include <optional>
@@ -20,6 +21,17 @@ inline cudaStream_t stream() { return at::cuda::getCurrentCUDAStream().stream();
 
 template <typename T = float>
 inline T* ptr(const Tensor& t) { return t.defined() ? static_cast<T*>(t.data_ptr()) : nullptr; }
+// A trace would hold a native call's results as constants, and forward-mode tangents end at one: such calls are composed, and
+// the autograd functions they are composed of refuse them.
+inline bool followed(const Tensor& t) { return t.defined() && t._fw_grad(0).defined(); }
+inline bool followed(const OptTensor& t) { return t && followed(*t); }
+template <typename... T>
+inline bool followed(const Tensor& x, at::ArrayRef<Tensor> params, const T&... carry) {
+  if (torch::jit::tracer::isTracing() || followed(x) || (followed(carry) || ...)) return true;
+  for (const Tensor& p : params)
+    if (followed(p)) return true;
+  return false;
+}
 // What kernels with 16-byte accesses ask of a tensor that a caller brings (one cut out of a larger buffer may start anywhere).
 inline bool aligned16(const Tensor& t) { return !t.defined() || reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; }
 inline const uint8_t* bytes(const Tensor& t) { return t.defined() ? static_cast<const uint8_t*>(t.data_ptr()) : nullptr; }

@@ -188,7 +188,7 @@ bool wants_grad(const Tensor& x, const variable_list& params, const Tensor& h0) 
 // -> (last state (B,1,N), decay leaf (B,1,N), y (B,T,F)), or None
 pybind11::object lru_layer(const Tensor& x_in, const variable_list& params, const OptTensor& h0_in, const OptTensor& a0_in,
                            const OptTensor& done_in) {
-  if (!native(x_in, params)) return pybind11::none();
+  if (!native(x_in, params) || followed(x_in, params, h0_in, a0_in)) return pybind11::none();
   const c10::cuda::CUDAGuard guard(x_in.device());
   const Tensor x = (x_in.scalar_type() == at::kFloat ? x_in : x_in.to(at::kFloat)).contiguous();
   const Tensor h0 = carry_leaf(h0_in, x.size(0) * params[0].size(0), at::kComplexFloat, "h0"), a0 = carry_leaf(a0_in, x.size(0) * params[0].size(0), at::kComplexFloat, "a0"), done = done_bytes(done_in, x.size(0) * x.size(1));
@@ -205,7 +205,7 @@ pybind11::object lru_layer(const Tensor& x_in, const variable_list& params, cons
 // theta_log), or None
 pybind11::object lru_rtrl(const Tensor& x_in, const variable_list& params, const OptTensor& h0_in, const OptTensor& a0_in,
                           const OptTensor& done_in, const variable_list& sens_in) {
-  if (!native(x_in, params) || sens_in.size() != 5 || x_in.size(0) > 65535) return pybind11::none();
+  if (!native(x_in, params) || sens_in.size() != 5 || x_in.size(0) > 65535 || followed(x_in, params, h0_in, a0_in) || followed(x_in, sens_in)) return pybind11::none();
   const int B = x_in.size(0), T = x_in.size(1), F = x_in.size(2), N = params[0].size(0);
   const c10::cuda::CUDAGuard guard(x_in.device());
   const Tensor x = (x_in.scalar_type() == at::kFloat ? x_in : x_in.to(at::kFloat)).contiguous();

@@ -98,7 +98,8 @@ pybind11::object mingru_layer(const Tensor& in_, const Tensor& w_z, const Tensor
   const auto fits = [&](const Tensor& t) { return t.is_cuda() && t.scalar_type() == at::kFloat && t.device() == in_.device(); };
   if (!fits(in_) || !fits(w_z) || !fits(w_h) || in_.dim() != 3 || in_.numel() == 0 || w_z.dim() != 2 || w_z.sizes() != w_h.sizes() ||
       !w_z.is_contiguous() || !w_h.is_contiguous() || in_.size(2) != w_z.size(1) || in_.size(0) * in_.size(1) > 0x7fffffff ||
-      (in_.size(1) > 1 && at::globalContext().allowTF32CuBLAS()) || at::autocast::is_autocast_enabled(at::kCUDA))
+      (in_.size(1) > 1 && at::globalContext().allowTF32CuBLAS()) || at::autocast::is_autocast_enabled(at::kCUDA) ||
+      followed(in_, {w_z, w_h}, x0_in, a0_in))
     return pybind11::none();
   const c10::cuda::CUDAGuard guard(in_.device());
   const Tensor in = in_.contiguous(), x0 = carry_leaf(x0_in, in.size(0) * w_z.size(0), at::kFloat, "x0"), a0 = carry_leaf(a0_in, in.size(0) * w_z.size(0), at::kFloat, "a0"), done = done_bytes(done_in, in.size(0) * in.size(1));

@@ -193,7 +193,7 @@ struct MlstmLayer : torch::autograd::Function<MlstmLayer> {
 pybind11::object mlstm_layer(const Tensor& x_in, const variable_list& p, const OptTensor& c_in, const OptTensor& f_in, const OptTensor& n_in, const OptTensor& m_in,
                              const OptTensor& done_in, double eps) {
   if (!x_in.is_cuda() || x_in.scalar_type() != at::kBFloat16 || x_in.dim() != 3 || x_in.numel() == 0 || p.size() != kParams ||
-      x_in.size(0) * x_in.size(1) > 0x7fffffff || at::autocast::is_autocast_enabled(at::kCUDA))
+      x_in.size(0) * x_in.size(1) > 0x7fffffff || at::autocast::is_autocast_enabled(at::kCUDA) || followed(x_in, p, c_in, f_in, n_in, m_in))
     return pybind11::none();
   for (const Tensor& t : p)
     if (t.scalar_type() != at::kBFloat16 || t.device() != x_in.device() || !t.is_contiguous() || (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15)) return pybind11::none();

@@ -54,3 +54,49 @@ def test_a_skip_weight_for_all_features():
     model.cell.D = nn.Parameter(torch.full((1,), 0.7, device="cuda"))
     _, got = model(x, done)
     assert float((got - want).detach().abs().max()) <= 1e-5 * float(want.detach().abs().max())
+
+
+CELLS = {"lru": lambda m: m.LRUCell(32, 16), "s5": lambda m: m.S5Cell(32, 16), "mingru": lambda m: m.MinGRUCell(32), "mamba": lambda m: m.MambaCell(32, num_heads=2),
+         "linattn": lambda m: m.LinearAttentionCell(32, 64, 2).bfloat16(), "deltanet": lambda m: m.DeltaNetCell(32, 64, 2).bfloat16(),
+         "mlstm": lambda m: m.mLSTMCell(32, 64, num_heads=2, tensor_cores=True).bfloat16()}
+
+
+# the kernels have neither tangents nor a graph form: both are refused, not dropped
+@pytest.mark.parametrize("kind", CELLS)
+@pytest.mark.parametrize("what", ["inputs", "carry", "parameter"])
+def test_forward_mode_is_refused(kind, what):
+    import torch.autograd.forward_ad as fwd
+    from memorax_b200 import memoroid
+    torch.manual_seed(0)
+    model = memoroid.Memoroid(CELLS[kind](memoroid)).cuda().requires_grad_(False)
+    x, done = torch.randn(2, 5, 32, device="cuda", dtype=torch.float32 if kind in ("lru", "s5", "mingru", "mamba") else torch.bfloat16), torch.zeros(2, 5, device="cuda")
+    carry = [c.cuda() for c in model.initialize_carry(None, (2, 32))]
+    with fwd.dual_level():
+        dual = lambda t: fwd.make_dual(t, torch.ones_like(t))
+        if what == "inputs":
+            x = dual(x)
+        elif what == "carry":
+            carry[0] = dual(carry[0])
+        else:   # the cell's own parameter, or a Dense layer's
+            holder = model.cell if model.cell._parameters else next(m for m in model.cell.children() if isinstance(m, nn.Linear))
+            name = next(iter(holder._parameters))
+            holder._parameters[name] = dual(holder._parameters[name])
+        with pytest.raises(NotImplementedError):
+            model(x, done, tuple(carry))
+
+
+@pytest.mark.filterwarnings("ignore::torch.jit.TracerWarning")
+@pytest.mark.parametrize("kind", CELLS)
+def test_a_trace_is_refused_or_follows_its_inputs(kind):
+    from memorax_b200 import memoroid
+    torch.manual_seed(0)
+    model = memoroid.Memoroid(CELLS[kind](memoroid)).cuda().requires_grad_(False)
+    dtype = torch.float32 if kind in ("lru", "s5", "mingru", "mamba") else torch.bfloat16
+    x, other = (torch.randn(2, 5, 32, device="cuda", dtype=dtype) for _ in range(2))
+    done = torch.zeros(2, 5, device="cuda")
+    try:
+        traced = torch.jit.trace(lambda x, done: model(x, done)[1], (x, done), check_trace=False)
+    except RuntimeError:
+        return
+    want = model(other, done)[1].float()
+    assert float((traced(other, done).float() - want).norm()) <= 1e-5 * float(want.norm())
