@@ -163,6 +163,7 @@ pybind11::object mamba_layer(const Tensor& x_in, const variable_list& p, const O
   bool grad = x.requires_grad() || (h0.defined() && h0.requires_grad());
   for (const Tensor& t : p) grad |= t.requires_grad();
   if (at::GradMode::is_enabled() && grad) {
+    if (H > l::kMambaGradHeads) return pybind11::none();
     const variable_list out = MambaLayer::apply(x, p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7], p[8], p[9], p[10], p[11], opt(h0), opt(a0), opt(done), eps);
     return pybind11::cast(std::make_tuple(out[0], out[1], out[2]));
   }

@@ -264,7 +264,7 @@ bool encode(CUtensorMap* map, const Matrix& m, int cols, int rows, int batch, in
 
 template <int BN, bool A_ROWS, bool B_ROWS>
 int launch(const Params& p, cudaStream_t stream) {
-  if (const int st = allow_smem<gemm16_kernel<BN, A_ROWS, B_ROWS>>(Layout<BN>::kBytes); st != MXK_OK) return st;
+  if (const int st = allow_smem<gemm16_kernel<BN, A_ROWS, B_ROWS>, Layout<BN>::kBytes>(); st != MXK_OK) return st;
   const long long tiles = static_cast<long long>((p.M + kBM - 1) / kBM) * ((p.N + BN - 1) / BN) * p.batch * p.splits;
   mxk::launch_kernel(gemm16_kernel<BN, A_ROWS, B_ROWS>, static_cast<unsigned>(min(tiles, static_cast<long long>(kNumSMs))), kThreads, Layout<BN>::kBytes, stream, p);
   return launch_status();

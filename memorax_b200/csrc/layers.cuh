@@ -88,7 +88,8 @@ int mamba_scan_fwd(const MambaParams& w, const float* proj, long long ld, const 
 // z = RMSNorm(y_pre) silu(gate)
 int mamba_gate_fwd(const MambaParams& w, const float* proj, long long ld, const float* y_pre, float* z, long long tokens, int H,
                    cudaStream_t stream);
-// gz -> gy_pre and the gate columns of gproj; norm_partial: mamba_gate_blocks rows of 16 H
+// gz -> gy_pre and the gate columns of gproj, for at most kMambaGradHeads heads (each warp keeps a row of sums in shared memory); norm_partial: mamba_gate_blocks rows of 16 H
+constexpr int kMambaGradHeads = 454;
 int mamba_gate_blocks(long long tokens);
 int mamba_gate_bwd(const MambaParams& w, const float* proj, long long ld, const float* y_pre, const float* gz, float* gy_pre,
                    float* gproj, float* norm_partial, long long tokens, int H, cudaStream_t stream);

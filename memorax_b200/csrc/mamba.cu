@@ -515,7 +515,7 @@ int mamba_scan_bwd(const MambaParams& w, const float* proj, long long ld, const 
                    const float* gy_pre, const float* gh_last, float* gproj, float* gh0,
                    float* partial, int B, int T, int H, cudaStream_t stream) {
   if (B <= 0 || T <= 0 || H <= 0) return MXK_ERR_DIMS;
-  if (const int st = allow_smem<mamba_scan_bwd_kernel>(sizeof(BwdSmem)); st != MXK_OK) return st;
+  if (const int st = allow_smem<mamba_scan_bwd_kernel, sizeof(BwdSmem)>(); st != MXK_OK) return st;
   mxk::launch_kernel(mamba_scan_bwd_kernel, B * H, 384, sizeof(BwdSmem), stream, w, proj, ld, done, states, gy_pre, gh_last, gproj, gh0, partial,
                                                                  T, H);
   return launch_status();
@@ -529,9 +529,11 @@ int mamba_gate_fwd(const MambaParams& w, const float* proj, long long ld, const 
 
 int mamba_gate_bwd(const MambaParams& w, const float* proj, long long ld, const float* y_pre, const float* gz, float* gy_pre,
                    float* gproj, float* norm_partial, long long tokens, int H, cudaStream_t stream) {
+  if (H > kMambaGradHeads) return MXK_ERR_UNSUPPORTED;
   const int hid = 16 * H, bytes = 8 * hid * static_cast<int>(sizeof(float));
+  static_assert(8 * 16 * sizeof(float) * kMambaGradHeads <= kMaxSmem, "a row of sums per warp");
   if (bytes > 48 * 1024)
-    if (const int st = allow_smem<mamba_gate_bwd_kernel>(bytes); st != MXK_OK) return st;
+    if (const int st = allow_smem<mamba_gate_bwd_kernel, kMaxSmem>(); st != MXK_OK) return st;
   mxk::launch_kernel(mamba_gate_bwd_kernel, mamba_gate_blocks(tokens), 256, bytes, stream, w, proj, ld, y_pre, gz, gy_pre, gproj, norm_partial, tokens, hid);
   return launch_status();
 }

@@ -19,16 +19,19 @@ inline int launch_status() {
   return e == cudaSuccess ? MXK_OK : static_cast<int>(e);
 }
 
-// Raises a kernel's dynamic shared memory limit, once per kernel and device (the call costs as much as a launch).
-template <auto kKernel>
-inline int allow_smem(int bytes) {
+// Raises a kernel's dynamic shared memory limit, once per kernel and device (the call costs as much as a launch) -- hence to
+// a constant: the most that any launch of the kernel asks for.
+constexpr int kMaxSmem = 227 * 1024;
+template <auto kKernel, int kBytes>
+inline int allow_smem() {
+  static_assert(kBytes <= kMaxSmem, "shared memory of an SM");
   static std::atomic<uint64_t> done{0};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return static_cast<int>(e);
   const uint64_t bit = dev < 64 ? 1ull << dev : 0;
   if (done.load(std::memory_order_acquire) & bit) return MXK_OK;
-  e = cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  e = cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes);
   if (e != cudaSuccess) return static_cast<int>(e);
   done.fetch_or(bit, std::memory_order_release);
   return MXK_OK;

@@ -48,3 +48,21 @@ def test_mamba_layer_and_its_gradients(shape, with_carry):
         assert err(got, r) <= 1e-5
     for name, got, r in zip(["x", *(n for n, _ in cell.named_parameters()), "h0"], grads, want):
         assert err(got, r) <= 1e-4, (name, err(got, r))
+
+
+# the gate's backward pass keeps 512 bytes of shared memory a head: more of it in a later call than in an earlier one, and
+# on both sides of what an SM has
+def test_head_counts_one_after_another():
+    from memorax_b200.memoroid import MambaCell, Memoroid, MemoroidCellBase
+    bsz, steps, feat = 2, 9, 8
+    for heads in (97, 100, 200, 454, 455):
+        torch.manual_seed(heads)
+        cell = MambaCell(feat, num_heads=heads).cuda()
+        x, done = torch.randn(bsz, steps, feat, device="cuda", requires_grad=True), torch.rand(bsz, steps, device="cuda") < 0.1
+        gy, wrt = torch.randn(bsz, steps, feat, device="cuda"), [x, *cell.parameters()]
+        runs = []
+        for layer in (Memoroid(cell), lambda *a: MemoroidCellBase.layer(cell, *a)):
+            _, y = layer(x, done, None)
+            runs.append([y, *torch.autograd.grad(y, wrt, gy)])
+        for got, want in zip(*runs):
+            assert float((got - want).detach().abs().max()) <= 1e-4 * max(0.05, float(want.detach().abs().max())), heads
