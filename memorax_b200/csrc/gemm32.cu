@@ -553,8 +553,9 @@ Plan plan(int M, int N, int K) {
 template <int BN, bool kOuter>
 int launch(const Params& p, int tiles, cudaStream_t stream) {
   if (const int st = allow_smem<gemm32_kernel<BN, kOuter>, Layout<BN>::kBytes>(); st != MXK_OK) return st;
-  return mxk::launch_kernel_clusters(gemm32_kernel<BN, kOuter>, Layout<BN>::kPair ? 2 : 1, min(tiles, kNumSMs), Roles<BN, kOuter>::kThreads,
-                                     Layout<BN>::kBytes, stream, p);
+  mxk::launch_kernel_clusters(gemm32_kernel<BN, kOuter>, Layout<BN>::kPair ? 2 : 1, min(tiles, kNumSMs), Roles<BN, kOuter>::kThreads,
+                              Layout<BN>::kBytes, stream, p);
+  return launch_status();
 }
 
 template <bool kOuter>

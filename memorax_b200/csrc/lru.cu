@@ -436,7 +436,8 @@ int lru_sensitivities(const LruWeights& w, const float* lambda, const float* h, 
   // lanes per unit: as many as four features each need, so that narrow inputs leave none idle
   const auto go = [&](auto kernel, int lanes) {
     const int units = 256 / lanes, inputs = ((N + units - 1) / units) * ((F + 4 * lanes - 1) / (4 * lanes));
-    return mxk::launch_kernel(kernel, dim3(inputs + (N + 31) / 32, B), 256, 0, stream, w, lambda, h, h0, u, done, s, T, F, N, inputs, wide);
+    mxk::launch_kernel(kernel, dim3(inputs + (N + 31) / 32, B), 256, 0, stream, w, lambda, h, h0, u, done, s, T, F, N, inputs, wide);
+    return launch_status();
   };
   if (F <= 32) return go(lru_sensitivities_kernel<8>, 8);
   if (F <= 64) return go(lru_sensitivities_kernel<16>, 16);

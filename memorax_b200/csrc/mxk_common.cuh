@@ -14,6 +14,7 @@ constexpr int kNumSMs = 148;  // B200: 2 dies x 74 SMs; grids are sized against 
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
+// Of the launches since the last call (cudaGetLastError forgets what it reports): once, behind the last launch.
 inline int launch_status() {
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? MXK_OK : static_cast<int>(e);
@@ -39,9 +40,10 @@ inline int allow_smem() {
 
 // Kernel launch that may be set up while the kernel in front of it still runs (programmatic dependent launch: 0.7-1 us
 // less between two small kernels).  Every kernel of this library begins with enter_kernel(), which waits for the kernels in
-// front before anything is read or written, so the order of effects on a stream is the usual one.
+// front before anything is read or written, so the order of effects on a stream is the usual one.  What became of a launch
+// is launch_status()'s to say.
 template <typename... P, typename... A>
-inline int launch_kernel_clusters(void (*kernel)(P...), unsigned cluster, dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+inline void launch_kernel_clusters(void (*kernel)(P...), unsigned cluster, dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                                   A&&... args) {
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -57,11 +59,10 @@ inline int launch_kernel_clusters(void (*kernel)(P...), unsigned cluster, dim3 g
   cfg.attrs = attr;
   cfg.numAttrs = cluster > 1 ? 2 : 1;
   cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
-  return launch_status();
 }
 template <typename... P, typename... A>
-inline int launch_kernel(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
-  return launch_kernel_clusters(kernel, 1, grid, block, smem, stream, static_cast<A&&>(args)...);
+inline void launch_kernel(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+  launch_kernel_clusters(kernel, 1, grid, block, smem, stream, static_cast<A&&>(args)...);
 }
 
 // First statement of every kernel, executed by all threads.  A grid of at most two blocks per SM lets its successor's

@@ -111,3 +111,13 @@ def test_gelu_tanh_form(n):
     (dxr,) = torch.autograd.grad(yr, xr, dy.double())
     assert float((y.double() - yr).abs().max()) <= 2 ** -8 * float(yr.abs().max()) + 2e-3
     assert float((dx.double() - dxr).abs().max()) <= 2 ** -8 * float(dxr.abs().max()) + 4e-3
+
+
+def test_a_launch_that_fails_is_reported_once():
+    """2^43 elements make a grid of 2^32 blocks, which is none in the launch's 32 bits: the runtime refuses an empty grid, and
+    the status has to say so; the next call starts clean."""
+    from memorax_b200 import _lib, ops
+    x, y = torch.zeros(64, device="cuda", dtype=torch.bfloat16), torch.ones(64, device="cuda", dtype=torch.bfloat16)
+    call = lambda n: _lib.lib.mxk_gelu_bf16(x.data_ptr(), None, y.data_ptr(), n, ops._stream())
+    assert call(1 << 43) > 0
+    assert call(64) == 0 and not y.any()
