@@ -40,11 +40,17 @@ Result forward(const Tensor& in, const Tensor& w_z, const Tensor& w_h, const Ten
   r.zh = empty_like_of(in, {B, T, 2 * D}, at::kFloat);
   Arena mem;
   const size_t image = mem.take(g::image_bytes(M, 2 * D, F)), ws_bytes = g::workspace_bytes(M, 2 * D, F), ws = mem.take(ws_bytes);
+  const size_t norms = keep ? mem.take(sizeof(float) * (static_cast<size_t>(M) + D)) : 0;
   mem.alloc(in);
+  mxk::layers::NearKink kink;
+  if (keep) {   // (only gradients tell the two sides of the kink apart)
+    kink = {ptr(r.zh) + D, ptr(in), ptr(w_h), mem.at(norms), F};
+    check("row_norms", mxk::layers::row_norms(ptr(in), M, ptr(w_h), D, F, mem.at(norms), stream()));
+  }
   const g::WeightJob job{stacked(w_z, w_h), false, 2 * D, F, g::tile_width(M, 2 * D, F), mem.at<void>(image)};
   check("split_weights", g::split_weights(&job, 1, {}, stream()));
   check("run_weights", g::run_weights(ptr(in), F, job.image, ptr(r.zh), 2 * D, M, 2 * D, F, {}, mem.at(ws), ws_bytes, status_ptr(in), stream()));
-  check("mingru_fwd", mxk::layers::mingru_fwd(ptr(r.zh), ptr(r.zh) + D, keep ? ptr(r.zh) + D : nullptr, ptr(in), ptr(w_h), F, 2 * D, ptr(x0), ptr(a0), bytes(done), ptr(r.x), ptr(r.y), ptr(r.a_last), B, T, D, stream()));
+  check("mingru_fwd", mxk::layers::mingru_fwd(ptr(r.zh), ptr(r.zh) + D, kink, 2 * D, ptr(x0), ptr(a0), bytes(done), ptr(r.x), ptr(r.y), ptr(r.a_last), B, T, D, stream()));
   return r;
 }
 

@@ -48,12 +48,17 @@ int lru_sensitivities(const LruWeights& w, const float* lambda, const float* h, 
                       const uint8_t* done, const LruSensitivities& s, int B, int T, int F, int N, cudaStream_t stream);
 
 // ---- MinGRU, mingru.cu -----------------------------------------------------------------------------------------
+// out: the two-norms of the rows of a, then of those of b, each row F long.
+int row_norms(const float* a, long long rows_a, const float* b, long long rows_b, int F, float* out, cudaStream_t stream);
+// The elements of h_tilde whose sign is not sure are replaced by the product in (B, T, F) w (D, F)^T in plain float32 order.
+struct NearKink {
+  float* h = nullptr;             // = h_tilde, writable; null: they stay as they are
+  const float *in = nullptr, *w = nullptr, *norms = nullptr;   // norms: row_norms of in and w
+  int F = 0;
+};
 // z and h_tilde are (B, T, D) with rows of both (and of their cotangents) `ld` floats apart; the rest is dense.
-// With `h_kink` (= h_tilde, writable) elements too close to zero for their sign to be sure are replaced by the product
-// dense_in (B, T, F) dense_w (D, F)^T in plain float32 order.
-int mingru_fwd(const float* z, const float* h_tilde, float* h_kink, const float* dense_in, const float* dense_w, int F,
-               long long ld, const float* x0, const float* a0, const uint8_t* done,
-               float* x, float* y, float* a_last, int B, int T, int D, cudaStream_t stream);
+int mingru_fwd(const float* z, const float* h_tilde, const NearKink& kink, long long ld, const float* x0, const float* a0,
+               const uint8_t* done, float* x, float* y, float* a_last, int B, int T, int D, cudaStream_t stream);
 // y: the read-out exp(x), or null
 int mingru_bwd(const float* z, const float* h_tilde, long long ld, const float* x, const float* y, const float* x0, const uint8_t* done,
                const float* gx, const float* gy, const float* gx_last, float* gz, float* gh, float* gx0, int B, int T, int D,

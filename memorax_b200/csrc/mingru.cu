@@ -26,14 +26,44 @@ constexpr int kSegs = 16, kSteps = 8;
 
 // d log g / dh~ jumps at h~ = 0 (from 1/2 to 2), so an element whose sign hangs on the rounding of its dot product is
 // decided by the plain float32 sum in the order of k: the branch, and with it the gradient, does not depend on how the
-// product was tiled.  (Two such sums differ by about 2e-7 at
-// unit scale and 512 terms; one element in 200 000 is looked at.)
-constexpr float kNearKink = 1.f / 262144.f;
+// product was tiled.  Two such sums of terms with random signs differ by about 0.6 x 2^-24 |in| |w|; those below eight
+// times 2^-24 |in| |w| are looked at (one in 100 000 at 512 terms), whatever the scale of the inputs and of the weights.
+// A sum that is zero because its terms are needs no decision: a row or a channel of zeros has no such range, and where
+// zeros of both meet (one-hot inputs, pruned weights) a stretch has several of them, which chance does not give without as
+// many others in the range (an element in 4e7 is zero).  Without that distinction zeros cost 27 ms a pass at 96 x 250 x 512.
+constexpr float kNearKink = 8.f / 16777216.f;
 __device__ __noinline__ float dot_in_order(const float* __restrict__ in, const float* __restrict__ w, int F) {
   float acc = 0.f;
 #pragma unroll 32
   for (int k = 0; k < F; ++k) acc = fmaf(in[k], w[k], acc);
   return acc;
+}
+
+// Two-norms of the rows of a (rows_a, F), then of those of b (rows_b, F); a warp each.  0 where the squares leave float32's
+// range: the gates are saturated there.  HBM-bound: one read of a.
+__global__ void __launch_bounds__(256) row_norms_kernel(const float* __restrict__ a, long long rows_a, const float* __restrict__ b,
+                                                        long long rows_b, int F, bool wide, float* __restrict__ out) {
+  enter_kernel();
+  const long long row = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (row >= rows_a + rows_b) return;
+  const float* const p = row < rows_a ? a + row * F : b + (row - rows_a) * F;
+  float s[4] = {};
+  if (wide) {
+#pragma unroll 4
+    for (int k = lane * 4; k < F; k += 128) {
+      const float4 v = __ldg(reinterpret_cast<const float4*>(p + k));
+      s[0] = fmaf(v.x, v.x, s[0]); s[1] = fmaf(v.y, v.y, s[1]);
+      s[2] = fmaf(v.z, v.z, s[2]); s[3] = fmaf(v.w, v.w, s[3]);
+    }
+  } else {
+#pragma unroll 4
+    for (int k = lane; k < F; k += 32) s[0] = fmaf(p[k], p[k], s[0]);
+  }
+  float sum = (s[0] + s[1]) + (s[2] + s[3]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if (lane == 0) out[row] = sum < INFINITY ? sqrtf(sum) : 0.f;
 }
 
 // Largest |z|, |h~| and carried x for which the linear form stays inside float32: every state is at least e^-40, and what
@@ -66,9 +96,9 @@ __device__ __forceinline__ unsigned reset_mask(const uint8_t* drow, int t_begin,
 
 __global__ void __launch_bounds__(32 * kSegs, 2)
 mingru_fwd_kernel(const float* __restrict__ z, const float* ht, float* ht_kink, const float* __restrict__ dense_in,
-                  const float* __restrict__ dense_w, int F, long long ld, const float* __restrict__ x0,
-                  const float* __restrict__ a0, const uint8_t* __restrict__ done, float* __restrict__ x, float* __restrict__ y,
-                  float* __restrict__ a_last, int B, int T, int D, int turn_len) {
+                  const float* __restrict__ dense_w, const float* __restrict__ norms, int F, long long ld,
+                  const float* __restrict__ x0, const float* __restrict__ a0, const uint8_t* __restrict__ done,
+                  float* __restrict__ x, float* __restrict__ y, float* __restrict__ a_last, int B, int T, int D, int turn_len) {
   enter_kernel();
   __shared__ float sa[kSegs][32], sq[kSegs][32], sd[kSegs][32];
   __shared__ unsigned sr[kSegs];   // reset bits of a stretch
@@ -83,6 +113,7 @@ mingru_fwd_kernel(const float* __restrict__ z, const float* ht, float* ht_kink, 
     carry_x[lane] = (in && x0) ? x0[static_cast<size_t>(b) * D + d] : -INFINITY;
     carry_a[lane] = (in && a0) ? a0[static_cast<size_t>(b) * D + d] : 0.f;
   }
+  const float range = (ht_kink && in) ? kNearKink * __ldg(norms + static_cast<long long>(B) * T + d) : 0.f;
   for (int turn = 0; turn < T; turn += turn_len) {
     const int t_begin = turn + seg * len, t_end = min(min(T, turn + turn_len), t_begin + len);
     const int count = t_end - t_begin;   // steps of this warp (may be negative)
@@ -100,20 +131,27 @@ mingru_fwd_kernel(const float* __restrict__ z, const float* ht, float* ht_kink, 
       }
     }
     const unsigned resets = reset_mask(drow, t_begin, count, lane);
-    float most = 0.f, least = 1.f;
+    float most = 0.f;
 #pragma unroll
-    for (int i = 0; i < kSteps; ++i) {
-      most = fmaxf(most, fmaxf(fabsf(lv[i]), fabsf(dv[i])));
-      least = fminf(least, fabsf(dv[i]));
-    }
-    if (ht_kink && least < kNearKink) {
+    for (int i = 0; i < kSteps; ++i) most = fmaxf(most, fmaxf(fabsf(lv[i]), fabsf(dv[i])));
+    if (ht_kink) {
+      const long long token0 = static_cast<long long>(b) * T + t_begin;
+      const float norm = lane < count ? __ldg(norms + token0 + lane) : 0.f;
+      unsigned near = 0, zero = 0;
 #pragma unroll
-      for (int i = 0; i < kSteps; ++i)
-        if (fabsf(dv[i]) < kNearKink) {
-          const long long token = static_cast<long long>(b) * T + t_begin + i;
-          dv[i] = dot_in_order(dense_in + token * F, dense_w + static_cast<long long>(d) * F, F);
-          ht_kink[token * ld + d] = dv[i];
-        }
+      for (int i = 0; i < kSteps; ++i) {
+        if (fabsf(dv[i]) < range * __shfl_sync(0xffffffffu, norm, i)) near |= 1u << i;
+        if (dv[i] == 0.f) zero |= 1u << i;
+      }
+      if (__any_sync(0xffffffffu, near != 0)) {
+        if (__reduce_add_sync(0xffffffffu, __popc(near & zero) - __popc(near & ~zero)) > 1) near &= ~zero;
+#pragma unroll
+        for (int i = 0; i < kSteps; ++i)
+          if (near >> i & 1u) {
+            dv[i] = dot_in_order(dense_in + (token0 + i) * F, dense_w + static_cast<long long>(d) * F, F);
+            ht_kink[(token0 + i) * ld + d] = dv[i];
+          }
+      }
     }
     const bool linear = !__syncthreads_or(!(most <= kSafe) || (seg == 0 && !(carry_x[lane] <= kSafe)));
     const size_t out0 = (static_cast<size_t>(b) * T + t_begin) * D + d;
@@ -370,11 +408,16 @@ int check_dims(int B, int T, int D) {
 
 }  // namespace
 
-int mingru_fwd(const float* z, const float* h_tilde, float* h_kink, const float* dense_in, const float* dense_w, int F,
-               long long ld, const float* x0, const float* a0, const uint8_t* done,
-               float* x, float* y, float* a_last, int B, int T, int D, cudaStream_t stream) {
+int row_norms(const float* a, long long rows_a, const float* b, long long rows_b, int F, float* out, cudaStream_t stream) {
+  const bool wide = F % 4 == 0 && aligned16(a) && aligned16(b);
+  mxk::launch_kernel(row_norms_kernel, static_cast<unsigned>((rows_a + rows_b + 7) / 8), 256, 0, stream, a, rows_a, b, rows_b, F, wide, out);
+  return launch_status();
+}
+
+int mingru_fwd(const float* z, const float* h_tilde, const NearKink& kink, long long ld, const float* x0, const float* a0,
+               const uint8_t* done, float* x, float* y, float* a_last, int B, int T, int D, cudaStream_t stream) {
   if (const int st = check_dims(B, T, D)) return st;
-  mxk::launch_kernel(mingru_fwd_kernel, blocks_of(B, D), 32 * kSegs, 0, stream, z, h_tilde, h_kink, dense_in, dense_w, F, ld, x0,
+  mxk::launch_kernel(mingru_fwd_kernel, blocks_of(B, D), 32 * kSegs, 0, stream, z, h_tilde, kink.h, kink.in, kink.w, kink.norms, kink.F, ld, x0,
                                                                 a0, done, x, y, a_last, B, T, D, turn_length(T));
   return launch_status();
 }

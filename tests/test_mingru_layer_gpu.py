@@ -39,3 +39,72 @@ def test_mingru_layer_matches_the_oracle(shape, with_carry, scale):
         assert err(got, ref) <= 1e-5
     for got, ref in zip(grads, want):
         assert err(got, ref) <= 1e-4
+
+
+# g's slope jumps at zero: an element whose product is rounding only takes the side of the plain float32 sum in the order
+# of k, at every scale.  Weights orthogonal to the inputs up to rounding; every step starts afresh, so that the gradient of
+# a channel's weights is sigmoid(z) g'(h~) x with g' = 1 or 1/4.
+@pytest.mark.parametrize("scale", [1e-6, 1.0, 60.0, 1e4])
+@pytest.mark.parametrize("w_scale", [1e-4, 1.0])
+def test_the_side_of_the_kink_is_that_of_the_sum_in_order(scale, w_scale):
+    from memorax_b200.memoroid import MinGRUCell, Memoroid
+    torch.manual_seed(0)
+    steps, feat, dim, t = 3, 512, 64, 1
+    cell = MinGRUCell(dim, in_features=feat)
+    x = scale * torch.randn(1, steps, feat)
+    xt = x[0, t].double()
+    with torch.no_grad():
+        w = cell.h.weight.double()
+        cell.h.weight.copy_(w_scale * (w - (w @ xt)[:, None] * xt / (xt @ xt)))
+        cell.z.weight.zero_()
+    terms = (cell.h.weight.double() * xt).detach()     # exact: 24 x 24 bits
+    acc = torch.zeros(dim)
+    for k in range(feat):
+        acc = (acc.double() + terms[:, k]).float()
+    assert bool(((acc >= 0) != (terms.sum(1) >= 0)).any())   # the order of the sum does decide
+    cell, x = cell.cuda(), x.cuda()
+    gy = torch.zeros(1, steps, dim, device="cuda")
+    gy[:, t] = 1
+    _, y = Memoroid(cell)(x, torch.ones(1, steps, device="cuda"), None)
+    (gw,) = torch.autograd.grad(y, [cell.h.weight], gy)
+    slope = (gw.cpu().double() @ xt) / (xt @ xt) / 0.5
+    want = torch.where(acc >= 0, 1.0, 0.25).double()
+    assert float((slope - want).abs().max()) <= 1e-3
+
+
+# elements that are zero or tiny because the inputs or the weights are need no second look, which costs thousands of cycles
+@pytest.mark.parametrize("case", ["zero inputs", "small inputs", "padding", "zero channels", "small channels", "one-hot inputs, pruned weights"])
+def test_no_input_is_slow(case):
+    from memorax_b200.memoroid import MinGRUCell, Memoroid
+    torch.manual_seed(0)
+    bsz, steps, dim = 32, 128, 256
+    cell = MinGRUCell(dim).cuda()
+    model, done = Memoroid(cell), torch.zeros(bsz, steps, device="cuda")
+    x = torch.randn(bsz, steps, dim, device="cuda")
+
+    def time(x):
+        x, times = x.requires_grad_(), []
+        for _ in range(8):
+            start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            start.record()
+            model(x, done)
+            end.record()
+            end.synchronize()
+            times.append(start.elapsed_time(end))
+        return min(times)
+    usual = time(x.clone())
+    rows, w = torch.rand(dim, 1, device="cuda"), cell.h.weight.detach()
+    if case == "zero inputs":
+        x.zero_()
+    elif case == "small inputs":
+        x *= 1e-6
+    elif case == "padding":
+        x[:, 100:] = 0
+    elif case == "zero channels":
+        w *= rows > 0.1
+    elif case == "small channels":
+        w *= torch.where(rows > 0.1, 1.0, 1e-6)
+    else:
+        x = torch.zeros_like(x).scatter_(2, torch.randint(0, dim, (bsz, steps, 1), device="cuda"), 1.0)
+        w *= torch.rand_like(w) > 0.5
+    assert time(x) <= 3 * usual
