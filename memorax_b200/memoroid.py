@@ -32,33 +32,41 @@ from torch.nn.modules.module import _has_any_global_hook
 from . import _C, ops
 
 
+def _plain(module, kind):
+    if type(module) is not kind:
+        return False
+    own = module.__dict__
+    return not (own["_forward_hooks"] or own["_forward_pre_hooks"] or own["_backward_hooks"] or own["_backward_pre_hooks"]
+                or "forward" in own)
+
+
 def plain(module, kind):
     """Whether calling ``module`` runs ``kind.forward`` and nothing else: exactly this class, without hooks (weight norm and
     pruning are hooks too) and without a ``forward`` of its own.  Only such a module may be called through its parts."""
-    return (type(module) is kind and not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks
-                                          or module._backward_pre_hooks)
-            and "forward" not in module.__dict__ and not _has_any_global_hook())
+    return _plain(module, kind) and not _has_any_global_hook()
 
 
 def native_params(cell, kind, spec):
     """The parameters that the native layer of a ``kind`` takes, or None where the layer has to be composed: the cell or one
     of its submodules is not plain, or has other parameters than these.  ``spec`` names them in order: (submodule or None for
-    the cell's own, its class, names).  They come out of the module dictionaries: an attribute lookup through ``nn.Module``
-    per parameter costs more than a launch."""
-    if not plain(cell, kind):
+    the cell's own, its class, names).  They come out of the module dictionaries: attribute lookups through ``nn.Module``
+    take as long as an acting step's launches."""
+    if not _plain(cell, kind) or _has_any_global_hook():
         return None
-    out = []
+    own, out = cell.__dict__, []
     for sub, sub_kind, names in spec:
-        module = cell
-        if sub is not None:
-            module = cell._modules.get(sub)
-            if not plain(module, sub_kind):
+        if sub is None:
+            params = own["_parameters"]
+        else:
+            module = own["_modules"].get(sub)
+            if not _plain(module, sub_kind):
                 return None
-            for name, param in module._parameters.items():
-                if param is not None and name not in names:   # (a bias that the cell was not built with)
+            params = module.__dict__["_parameters"]
+            for name in params:
+                if name not in names and params[name] is not None:   # (a bias that the cell was not built with)
                     return None
         for name in names:
-            param = module._parameters.get(name)
+            param = params.get(name)
             if param is None:
                 return None
             out.append(param)
