@@ -112,3 +112,34 @@ def test_inputs_at_any_address(kind, heads, dim, bsz, steps, offset):
         got_c, got = model(cut, done)
     for g, w in zip([got, *got_c], [want, *want_c]):
         _close(g, w, 1e-2)
+
+
+# The native delta-rule layer adds in other orders than the composed one before it rounds to bf16.  Neither is the exact one:
+# both are as far from float64 as bf16 makes them, and no further from each other than two such errors are.
+@pytest.mark.parametrize("heads,dim", [(4, 64), (2, 128)])
+def test_native_gradients_are_as_close_to_float64_as_the_composed_ones(heads, dim):
+    import torch.nn.functional as F
+    from memorax_b200.memoroid import DeltaNetCell, Memoroid
+    from oracle import memoroid_oracle as mo
+    torch.manual_seed(4)
+    bsz, steps, feat = 17, 132, 256
+    model = Memoroid(DeltaNetCell(feat, dim, heads)).cuda().bfloat16()
+    x = torch.randn(bsz, steps, feat, device="cuda").bfloat16().requires_grad_()
+    done = torch.rand(bsz, steps, device="cuda") < 0.02
+    gy = torch.randn_like(x)
+    wrt = [x, *model.parameters()]
+    runs = [_run(model, x, done, None, gy, [torch.zeros(bsz, 1, heads, dim, dim, device="cuda")], wrt, native=n)[2:] for n in (True, False)]
+    p = {k: v.detach().double().cpu().requires_grad_() for k, v in model.cell.named_parameters()}
+    xd = x.detach().double().cpu().requires_grad_()
+    head = lambda name: F.linear(xd, p[name + ".weight"]).view(bsz, steps, heads, dim)
+    b_logit, a_logit = F.linear(xd, p["gate.weight"], p["gate.bias"]).chunk(2, dim=-1)
+    o, _ = mo.gdelta_seq(F.normalize(head("query"), dim=-1), F.normalize(head("key"), dim=-1), head("value"), torch.exp(-F.softplus(a_logit)),
+                         torch.sigmoid(b_logit), torch.zeros(bsz, heads, dim, dim, dtype=torch.float64), done.cpu().double())
+    o = F.rms_norm(o.reshape(bsz, steps, -1), (heads * dim,), p["norm.weight"], 1e-6)
+    y = F.linear(o, p["output_projection.weight"], p["output_projection.bias"])
+    want = torch.autograd.grad(y, [xd, *(p[k] for k, _ in model.cell.named_parameters())], gy.double().cpu())
+    for (name, _), native, composed, ref in zip([("x", None), *model.cell.named_parameters()], *runs, want):
+        native, composed = native.double().cpu(), composed.double().cpu()
+        off = [float((t - ref).norm() / ref.norm()) for t in (native, composed)]
+        apart = float((native - composed).norm() / ref.norm())
+        assert off[0] <= 1.1 * off[1] + 2 ** -10 and apart <= off[0] + off[1], (name, off, apart)

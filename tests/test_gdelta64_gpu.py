@@ -1,7 +1,8 @@
 """Gated delta rule, heads of 64, at the sizes where its chunks and sequences end: one step, one short of, at and one past
 a chunk, several chunks with every barrier phase wrapping, resets everywhere, and more sequences than fit on the chip at
-once.  Same oracle and tolerances as the heads of 128,
-except that dalpha, a sum of cancelling terms of bf16 states, has twice as much."""
+once.  Same oracle and tolerances as the heads of 128.  A first step's dalpha is <dS0, S0> / alpha, 64 x 64 products of
+bf16-rounded factors that largely cancel: it has the rounding of that sum on top, four times its standard deviation of
+0.8 x 2^-9 |dS0 o S0| / alpha (both factors off by up to 2^-9, evenly spread)."""
 import pytest
 import torch
 
@@ -31,6 +32,9 @@ def test_against_the_oracle(shape, p_done, carry):
     assert max_abs(o.float(), o_ref) <= ATOL
     assert max_abs(s_last, s_ref) <= 1e-2 * max(1.0, float(s_ref.detach().abs().max()))
     outs = ops.gdelta_bwd(*x, d_o.cuda(), states, done.cuda(), cu(ds_last), check=True)
+    first = 4 * 0.8 * 2 ** -9 * float(((leaves[5].grad * leaves[5].detach()).flatten(2).norm(dim=2) / alpha[:, 0]).max())
     for got, leaf, name in zip(outs, leaves, ["dq", "dk", "dv", "dalpha", "dbeta", "ds0"]):
-        err, tol = max_abs(got.float(), leaf.grad), GRAD_RTOL * (2 if name == "dalpha" else 1) * max(1.0, float(leaf.grad.abs().max()))
+        err, tol = max_abs(got.float(), leaf.grad), GRAD_RTOL * max(1.0, float(leaf.grad.abs().max()))
+        if name == "dalpha":
+            tol = max(tol, first)
         assert err <= tol, f"{name}: {err:.4f} > {tol:.4f}"
