@@ -63,25 +63,6 @@ inline bool make_panel_map(CUtensorMap* map, const void* base, int B, int T, int
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Map whose loads write `rows` x box_cols tiles row-major, [t][box_cols].  Coordinates: {0, h, t0, b}.
-// box_cols (default D) may exceed D: the columns past D are zero-filled on loads and clipped on stores,
-// which is how a head of 64 columns is served by a kernel built for 128.
-inline bool make_plain_map(CUtensorMap* map, const void* base, int B, int T, int H, int D, int rows, int box_cols = 0,
-                           long long ld = 0, long long hp = 0) {
-  EncodeTiledFn enc = encode_tiled_fn();
-  if (!enc) return false;
-  if (box_cols <= 0) box_cols = D;
-  const cuuint64_t row_bytes = static_cast<cuuint64_t>(ld > 0 ? ld : static_cast<long long>(H) * D) * 2;
-  const cuuint64_t dims[4] = {static_cast<cuuint64_t>(D), static_cast<cuuint64_t>(H), static_cast<cuuint64_t>(T),
-                              static_cast<cuuint64_t>(B)};
-  const cuuint64_t strides[3] = {static_cast<cuuint64_t>(hp > 0 ? hp : D) * 2, row_bytes, row_bytes * T};
-  const cuuint32_t box[4] = {static_cast<cuuint32_t>(box_cols), 1, static_cast<cuuint32_t>(rows), 1};
-  const cuuint32_t elem[4] = {1, 1, 1, 1};
-  return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, elem,
-             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 // Map whose loads write `rows` x 64 column blocks of a [B][T][H][D] tensor as 128-byte-swizzled row-major
 // lines (umma.cuh "SW tiles"): 128-byte pieces, about five times faster per byte than the panel map.
 // Coordinates {c0, h, t0, b} with c0 the first column of the block (a multiple of 64); the destination
@@ -113,6 +94,7 @@ __device__ __forceinline__ void load_panel_tile(void* dst, const CUtensorMap* ma
       "l"(reinterpret_cast<uint64_t>(map)), "r"(umma::smem_u32(bar)), "r"(0), "r"(t0), "r"(0), "r"(h), "r"(b)
       : "memory");
 }
+// Tile load through a 4-D map (make_sw_map).
 __device__ __forceinline__ void load_plain_tile(void* dst, const CUtensorMap* map, uint64_t* bar, int t0, int h, int b,
                                                 int c0 = 0) {
   asm volatile(
@@ -148,7 +130,7 @@ __device__ __forceinline__ void prefetch_bulk(const void* src, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
 // ---- shared -> global (bulk groups of the issuing thread) ----
-// Tile store through a plain map; rows past the end of the sequence are clipped.
+// Tile store through a 4-D map (make_sw_map); rows past the end of the sequence are clipped.
 __device__ __forceinline__ void store_plain_tile(const CUtensorMap* map, const void* src, int t0, int h, int b,
                                                  int c0 = 0) {
   asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"(
