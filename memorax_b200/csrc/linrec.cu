@@ -684,8 +684,12 @@ inline int check_dims(int B, int T, int D) {
   return MXK_OK;
 }
 
-// One thread per channel is the better form of the MinGRU scan from five full blocks per SM on (256 x 256 x 1024 forward +
-// backward: 0.73 ms against 0.82 split over time; 96 x 250 x 512: 0.25 ms against 0.15).
+// One thread per channel (walking all of T) against time split over a block's warps, in the bare MinGRU scan: forward and
+// backward in microseconds, walking | split: 256 x 256 x 1024: 287 + 353 | 298 + 384; 512 x 256 x 512: 294 + 354 | 298 + 385;
+// 512 x 128 x 512: 151 + 178 | 150 + 186; 1024 x 64 x 512: 150 + 189 | 233 + 269 (stretches of four steps fill half of a split
+// thread's registers); 96 x 250 x 512: 116 + 136 | 62 + 74.  The line is five full blocks of channels per SM.  The layer
+// (mingru_layer) splits at every size: the walking kernels know neither the pitch of its joint pre-activations nor the
+// decisions near the kink.
 inline bool mingru_walks(int B, int D) { return static_cast<long long>(B) * D >= 5LL * kNumSMs * kBlock; }
 
 template <bool CPLX>
