@@ -297,10 +297,11 @@ class TrainC5:
     p_done = 0.005
     seed = 1234 + 5
     dominant = "train_step"
-    # this library's kernels per step: per layer 3 delta-rule launches (prep, fwd, bwd), 9 norm launches (three norms:
-    # fwd, bwd, bwd reduce), 4 gated-residual, 4 L2-normalise, 12 column-sum launches (six biased Dense layers x 2);
-    # plus the embedding's column sum (2) and the Adam step
-    launches_per_step = 4 * (3 + 9 + 4 + 4 + 12) + 2 + 1
+    # this library's kernels per step, counted from a launch list: per layer the delta rule (prep, fwd, bwd) with its inputs
+    # (2), joint weights, gate products (2 and a sum over splits) and gate bias sums, 9 norm launches (three norms: fwd, bwd,
+    # bwd reduce), GELU and two gates, and five passes with bias sums (GELU, two gates, two Dense layers; 2 each); plus the
+    # embedding's bias sum (2) and the Adam step
+    launches_per_step = 4 * (3 + 2 + 1 + 3 + 1 + 9 + 3 + 5 * 2) + 2 + 1
     dominant_traffic_bytes = None
     cpu_sample_batch = 2
 
@@ -499,15 +500,15 @@ class MinGruA7:
 
 class RtrlN3:
     """One RTRL segment of the LRU cell (Memoroid.local_jacobian, memoroid.py:143-176 with lru.py:110-139): scan,
-    read-out, the five local Jacobians and their propagation to the sensitivities after the last step.  B=64
+    read-out, and the sensitivities after the last step (the five local Jacobians are never formed).  B=64
     sequences x T=64 steps, F=64 features, N=128 hidden units, fp32 / complex64, done ~ Bernoulli(0.01)."""
     name = "n3_rtrl_lru_segment"
     dtype = "c64"
     B, T, F, N = 64, 64, 64, 128
     p_done = 0.01
     seed = 1234 + 10
-    dominant = "linrec_fwd_kernel"
-    launches_per_step = 6
+    dominant = "lru_sensitivities_kernel"
+    launches_per_step = 5   # split weights, projection, scan, read-out, sensitivities
     dominant_traffic_bytes = None
     cpu_sample_batch = 8
     roofline_of_step = True
@@ -534,19 +535,18 @@ class RtrlN3:
         return self.model
 
     def algorithmic_bytes(self):
-        # the formulation's own traffic: the two (B,T,N,F) complex Jacobians of the input matrix written and read once,
-        # the three (B,T,N) ones likewise, inputs in, read-out and sensitivities out
-        big = 2 * 8 * self.B * self.T * self.N * self.F
-        small = 3 * 8 * self.B * self.T * self.N
-        return 2 * (big + small) + 8 * self.B * self.T * self.F + 8 * self.B * self.N * (2 * self.F + 3)
+        # what a segment cannot do without: inputs in, read-out out, weights, both leaves of the carry and the sensitivities
+        # in and out
+        weights = 4 * (4 * self.N * self.F + 3 * self.N + self.F)
+        return (8 * self.B * self.T * self.F + self.B * self.T + weights + 32 * self.B * self.N +
+                16 * self.B * self.N * (2 * self.F + 3))
 
     def roofline(self, step_ms):
         hbm, _, kind = measured_peaks()
         byts = self.algorithmic_bytes()
         return {"bound": "hbm", "achieved": byts / (step_ms * 1e-3) / 1e9, "peak": hbm, "unit": "GB/s",
                 "frac": byts / (step_ms * 1e-3) / 1e9 / hbm, "peak_kind": f"of {kind}", "algorithmic_bytes_per_step": byts,
-                "note": "whole segment: library GEMMs and PyTorch elementwise ops build the Jacobians, this repository's "
-                        "kernels run the scan and the five last-state-only propagations"}
+                "note": "whole segment: five dependent launches of this repository's kernels, bound by their latencies"}
 
     def step(self, x, ops, mark=None):
         model = self._model(x["x"].device)
