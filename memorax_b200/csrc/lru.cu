@@ -2,6 +2,8 @@
 // real projection matrices.
 #include <cuda_bf16.h>
 
+#include <type_traits>
+
 #include "layers.cuh"
 #include "mxk_common.cuh"
 #include "warp_tile.cuh"
@@ -278,13 +280,14 @@ __device__ __forceinline__ void unit_sensitivities(const LruWeights& w, const fl
 // new sensitivities touch memory: HBM-bound at large N F, else bound by the multiply-adds.  The blocks behind them take the
 // other leaves.  (64 sequences x 64 steps, 64 features, 128 units: the materialised Jacobians took 490 us of kernels in 76
 // launches.)
+// kWide: sixteen-byte accesses to the sensitivities of B (known when compiled, the old ones' loads stay in front of the sums:
+// 3 us of 44 for the whole segment).
 constexpr int kSensSteps = 64;
-template <int kLanes>
+template <int kLanes, bool kWide>
 __global__ void __launch_bounds__(256) lru_sensitivities_kernel(LruWeights w, const float* __restrict__ lambda,
                                                                 const float* __restrict__ h, const float* __restrict__ h0,
                                                                 const float* __restrict__ u, const uint8_t* __restrict__ done,
-                                                                LruSensitivities s, int T, int F, int N, int input_blocks,
-                                                                bool wide) {
+                                                                LruSensitivities s, int T, int F, int N, int input_blocks) {
   enter_kernel();
   constexpr int kUnits = 256 / kLanes, kFeatures = 4 * kLanes;
   __shared__ __align__(16) float us[kSensSteps][kFeatures];
@@ -302,7 +305,7 @@ __global__ void __launch_bounds__(256) lru_sensitivities_kernel(LruWeights w, co
   const bool in = n < N && f < F;
   const size_t at = (static_cast<size_t>(b) * N + (in ? n : 0)) * F + (in ? f : 0);
   float4 ore[2] = {}, oim[2] = {};   // old sensitivities, on their way while the sums are formed
-  if (in && wide) {
+  if (kWide && in) {
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       ore[e] = ld_stream(reinterpret_cast<const float4*>(s.b_re + 2 * at) + e);
@@ -343,7 +346,7 @@ __global__ void __launch_bounds__(256) lru_sensitivities_kernel(LruWeights w, co
   const float2 p = r < 0 ? power(reinterpret_cast<const float2*>(lambda)[n], T) : make_float2(0.f, 0.f);
   const auto re = [&](float2 o, int e) { return cmul_add(p, o, make_float2(gamma * acc[e].x, gamma * acc[e].y)); };
   const auto im = [&](float2 o, int e) { return cmul_add(p, o, make_float2(-gamma * acc[e].y, gamma * acc[e].x)); };
-  if (wide) {   // sixteen-byte accesses: two complex entries each
+  if (kWide) {   // two complex entries each
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const float2 v0 = re({ore[e].x, ore[e].y}, 2 * e), v1 = re({ore[e].z, ore[e].w}, 2 * e + 1);
@@ -430,18 +433,20 @@ int lru_param_grads(const LruWeights& w, const LruGrads& g, int F, int N, cudaSt
 int lru_sensitivities(const LruWeights& w, const float* lambda, const float* h, const float* h0, const float* u,
                       const uint8_t* done, const LruSensitivities& s, int B, int T, int F, int N, cudaStream_t stream) {
   if (B <= 0 || T <= 0 || F <= 0 || N <= 0 || B > 65535) return MXK_ERR_DIMS;
-  // sixteen-byte accesses to the sensitivities of B: whole vectors per unit, from where they may start
+  // whole vectors per unit, from where they may start
   bool wide = F % 4 == 0;
   for (const float* p : {s.b_re, s.b_im, static_cast<const float*>(s.b_re_out), static_cast<const float*>(s.b_im_out)}) wide = wide && aligned16(p);
   // lanes per unit: as many as four features each need, so that narrow inputs leave none idle
-  const auto go = [&](auto kernel, int lanes) {
-    const int units = 256 / lanes, inputs = ((N + units - 1) / units) * ((F + 4 * lanes - 1) / (4 * lanes));
-    mxk::launch_kernel(kernel, dim3(inputs + (N + 31) / 32, B), 256, 0, stream, w, lambda, h, h0, u, done, s, T, F, N, inputs, wide);
+  const auto go = [&](auto lanes_c) {
+    constexpr int lanes = decltype(lanes_c)::value, units = 256 / lanes;
+    const int inputs = ((N + units - 1) / units) * ((F + 4 * lanes - 1) / (4 * lanes));
+    mxk::launch_kernel(wide ? lru_sensitivities_kernel<lanes, true> : lru_sensitivities_kernel<lanes, false>, dim3(inputs + (N + 31) / 32, B), 256, 0,
+                       stream, w, lambda, h, h0, u, done, s, T, F, N, inputs);
     return launch_status();
   };
-  if (F <= 32) return go(lru_sensitivities_kernel<8>, 8);
-  if (F <= 64) return go(lru_sensitivities_kernel<16>, 16);
-  return go(lru_sensitivities_kernel<32>, 32);
+  if (F <= 32) return go(std::integral_constant<int, 8>{});
+  if (F <= 64) return go(std::integral_constant<int, 16>{});
+  return go(std::integral_constant<int, 32>{});
 }
 
 }  // namespace layers
