@@ -115,5 +115,6 @@ void bind_lru(pybind11::module_& m);
 void bind_mamba(pybind11::module_& m);
 void bind_mingru(pybind11::module_& m);
 void bind_mlstm(pybind11::module_& m);
+void bind_modules(pybind11::module_& m);
 
 }  // namespace mxk_host

@@ -38,4 +38,5 @@ PYBIND11_MODULE(_C, m) {
   bind_mamba(m);
   bind_mingru(m);
   bind_mlstm(m);
+  bind_modules(m);
 }

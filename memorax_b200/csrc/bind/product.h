@@ -8,8 +8,9 @@
 
 namespace mxk_host {
 
-// 2 M N K above which a product is the library's.  On the GPU its two-SM tiles are always the faster form (by 1.1 to 1.4,
-// 1.3 to 3 for weight gradients); below the line a layer's pass waits for the host, which a library call holds up for longer.
+// 2 M N K above which a product is the library's.  On the GPU its two-SM tiles are the faster form at nearly every size
+// (by 1.1 to 1.6, up to 3.4 for weight gradients); below the line a pass waits for the host, which a library call holds up for
+// longer.
 // Passes with gradients, with the line at 1e8 | 4e9 | 8e9 | 2e10, in microseconds: linear attention (4 heads of 64), 4096 x 256:
 // 207 | 166 | 167 | 168; 8192 x 512: 207 | 188 | 164 | 166; 16384 x 512: 210 | 205 | 186 | 181; 65536 x 512: 452 | 450 | 451 |
 // 474.  Delta rule, 8192 x 512, 4 heads of 128: 261 | 253 | 249 | 386 (rows of its joint projection are not 32-byte aligned,

@@ -27,50 +27,15 @@ import math
 import torch
 from torch import nn
 from torch.nn import functional as F
-from torch.nn.modules.module import _has_any_global_hook
 
 from . import _C, ops
 
 
-def _plain(module, kind):
-    if type(module) is not kind:
-        return False
-    own = module.__dict__
-    return not (own["_forward_hooks"] or own["_forward_pre_hooks"] or own["_backward_hooks"] or own["_backward_pre_hooks"]
-                or "forward" in own)
-
-
-def plain(module, kind):
-    """Whether calling ``module`` runs ``kind.forward`` and nothing else: exactly this class, without hooks (weight norm and
-    pruning are hooks too) and without a ``forward`` of its own.  Only such a module may be called through its parts."""
-    return _plain(module, kind) and not _has_any_global_hook()
-
-
-def native_params(cell, kind, spec):
-    """The parameters that the native layer of a ``kind`` takes, or None where the layer has to be composed: the cell or one
-    of its submodules is not plain, or has other parameters than these.  ``spec`` names them in order: (submodule or None for
-    the cell's own, its class, names).  They come out of the module dictionaries: attribute lookups through ``nn.Module``
-    take as long as an acting step's launches."""
-    if not _plain(cell, kind) or _has_any_global_hook():
-        return None
-    own, out = cell.__dict__, []
-    for sub, sub_kind, names in spec:
-        if sub is None:
-            params = own["_parameters"]
-        else:
-            module = own["_modules"].get(sub)
-            if not _plain(module, sub_kind):
-                return None
-            params = module.__dict__["_parameters"]
-            for name in params:
-                if name not in names and params[name] is not None:   # (a bias that the cell was not built with)
-                    return None
-        for name in names:
-            param = params.get(name)
-            if param is None:
-                return None
-            out.append(param)
-    return out
+#: Whether calling a module runs its class's forward and nothing else: exactly that class, without hooks (weight norm and
+#: pruning are hooks too) and without a ``forward`` of its own.  Only such a module may be called through its parts.
+plain = _C.plain
+#: The parameters that a native layer takes, out of a plain cell and its plain submodules, or None where it has to be composed.
+native_params = _C.native_params
 
 
 def _causal_taps(conv, taps):
