@@ -32,6 +32,11 @@ inline bool followed(const Tensor& x, at::ArrayRef<Tensor> params, const T&... c
     if (followed(p)) return true;
   return false;
 }
+// Float32 products in TF32 were asked for, by either of torch's settings (its query of the older one raises where only the
+// newer one was used).
+inline bool tf32_products() {
+  return at::globalContext().float32Precision(at::Float32Backend::CUDA, at::Float32Op::MATMUL) == at::Float32Precision::TF32;
+}
 // What kernels with 16-byte accesses ask of a tensor that a caller brings (one cut out of a larger buffer may start anywhere).
 inline bool aligned16(const Tensor& t) { return !t.defined() || reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; }
 inline const uint8_t* bytes(const Tensor& t) { return t.defined() ? static_cast<const uint8_t*>(t.data_ptr()) : nullptr; }

@@ -62,7 +62,7 @@ struct Linear32 : torch::autograd::Function<Linear32> {
 Tensor linear_f32(const Tensor& x, const Tensor& w, const OptTensor& bias) {
   const auto fits = [&](const Tensor& t) { return t.is_cuda() && t.scalar_type() == at::kFloat && t.device() == x.device(); };
   if (!fits(x) || !fits(w) || (bias && !fits(*bias)) || w.dim() != 2 || x.size(-1) != w.size(1) || x.numel() == 0 || w.numel() == 0 ||
-      x.numel() / x.size(-1) > 0x7fffffff || at::globalContext().allowTF32CuBLAS() || at::autocast::is_autocast_enabled(at::kCUDA) || followed(x, {w}, bias))
+      x.numel() / x.size(-1) > 0x7fffffff || tf32_products() || at::autocast::is_autocast_enabled(at::kCUDA) || followed(x, {w}, bias))
     return at::linear(x, w, bias);
   const c10::cuda::CUDAGuard guard(x.device());
   return Linear32::apply(x.contiguous(), w.contiguous(), bias ? OptTensor(bias->contiguous()) : std::nullopt);

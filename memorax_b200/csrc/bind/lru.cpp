@@ -165,7 +165,7 @@ struct LruLayer : torch::autograd::Function<LruLayer> {
 // the caller composes from its parts.
 bool native(const Tensor& x, const variable_list& params) {
   if (!x.is_cuda() || x.dim() != 3 || x.numel() == 0 || !x.is_floating_point() || x.scalar_type() == at::kDouble ||
-      (x.size(1) > 1 && at::globalContext().allowTF32CuBLAS()) || at::autocast::is_autocast_enabled(at::kCUDA) ||
+      (x.size(1) > 1 && tf32_products()) || at::autocast::is_autocast_enabled(at::kCUDA) ||
       x.size(0) * x.size(1) > 0x7fffffff || params.size() != kParams || params[3].dim() != 2)
     return false;
   const int64_t N = params[3].size(0), F = x.size(2);

@@ -147,7 +147,7 @@ struct MambaLayer : torch::autograd::Function<MambaLayer> {
 // -> (last state (B,1,H,16,16), decay leaf (B,1,H,1,1), y (B,T,F)), or None where the caller has to compose the layer
 pybind11::object mamba_layer(const Tensor& x_in, const variable_list& p, const OptTensor& h0_in, const OptTensor& a0_in, const OptTensor& done_in, double eps) {
   if (!x_in.is_cuda() || x_in.scalar_type() != at::kFloat || x_in.dim() != 3 || x_in.numel() == 0 || x_in.size(0) * x_in.size(1) > 0x7fffffff ||
-      at::globalContext().allowTF32CuBLAS() || at::autocast::is_autocast_enabled(at::kCUDA) || p.size() != kParams ||
+      tf32_products() || at::autocast::is_autocast_enabled(at::kCUDA) || p.size() != kParams ||
       followed(x_in, p, h0_in, a0_in))
     return pybind11::none();
   for (const Tensor& t : p)

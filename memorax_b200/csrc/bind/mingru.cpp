@@ -104,7 +104,7 @@ pybind11::object mingru_layer(const Tensor& in_, const Tensor& w_z, const Tensor
   const auto fits = [&](const Tensor& t) { return t.is_cuda() && t.scalar_type() == at::kFloat && t.device() == in_.device(); };
   if (!fits(in_) || !fits(w_z) || !fits(w_h) || in_.dim() != 3 || in_.numel() == 0 || w_z.dim() != 2 || w_z.sizes() != w_h.sizes() ||
       !w_z.is_contiguous() || !w_h.is_contiguous() || in_.size(2) != w_z.size(1) || in_.size(0) * in_.size(1) > 0x7fffffff ||
-      (in_.size(1) > 1 && at::globalContext().allowTF32CuBLAS()) || at::autocast::is_autocast_enabled(at::kCUDA) ||
+      (in_.size(1) > 1 && tf32_products()) || at::autocast::is_autocast_enabled(at::kCUDA) ||
       followed(in_, {w_z, w_h}, x0_in, a0_in))
     return pybind11::none();
   const c10::cuda::CUDAGuard guard(in_.device());

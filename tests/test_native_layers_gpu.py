@@ -100,3 +100,23 @@ def test_a_trace_is_refused_or_follows_its_inputs(kind):
         return
     want = model(other, done)[1].float()
     assert float((traced(other, done).float() - want).norm()) <= 1e-5 * float(want.norm())
+
+
+# products in TF32 are the library's, whichever of torch's two settings asked for them
+@pytest.mark.parametrize("setting", ["older", "newer"])
+@pytest.mark.parametrize("kind", ["lru", "s5", "mingru", "mamba"])
+def test_tf32_products_are_composed(kind, setting):
+    from memorax_b200 import memoroid
+    torch.manual_seed(0)
+    model = memoroid.Memoroid(CELLS[kind](memoroid)).cuda().requires_grad_(False)
+    x, done = torch.randn(2, 5, 32, device="cuda"), torch.zeros(2, 5, device="cuda")
+    exact = model(x, done)[1]
+    matmul = torch.backends.cuda.matmul
+    name, value = ("allow_tf32", True) if setting == "older" else ("fp32_precision", "tf32")
+    before = getattr(matmul, name)
+    try:
+        setattr(matmul, name, value)
+        got, want = model(x, done)[1], memoroid.MemoroidCellBase.layer(model.cell, x, done, None)[1]
+    finally:
+        setattr(matmul, name, before)
+    assert torch.equal(got, want) and not torch.equal(got, exact)
