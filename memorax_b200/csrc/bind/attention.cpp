@@ -178,8 +178,8 @@ variable_list LinAttnLayer::backward(AutogradContext* ctx, const variable_list& 
   const c10::cuda::CUDAGuard guard(x.device());
   const int64_t hid = out_w.size(1);
   const Shape s = shape_of(x, ctx->saved_data["heads"].toInt(), hid, out_w.size(0), 0);
-  const Tensor gy = matrix(gout[2].defined() ? gout[2].contiguous() : empty_like_of(x, {s.M, s.out}, at::kBFloat16).zero_(), s.M, s.out);
-  const Tensor gs = gout[0].defined() ? gout[0].contiguous() : Tensor(), gz = gout[1].defined() ? gout[1].contiguous() : Tensor();
+  const Tensor gy = matrix(gout[2].defined() ? dense(gout[2]) : empty_like_of(x, {s.M, s.out}, at::kBFloat16).zero_(), s.M, s.out);
+  const Tensor gs = gout[0].defined() ? dense(gout[0]) : Tensor(), gz = gout[1].defined() ? dense(gout[1]) : Tensor();
   const bool has_s = ctx->saved_data["s0"].toBool(), has_z = ctx->saved_data["z0"].toBool();
   const bool need_s = (has_s && ctx->needs_input_grad(7)) || (has_z && ctx->needs_input_grad(has_s ? 8 : 7));
   const TailGrads t = tail_backward(gy, o, saved[8], saved[9], norm_w, out_w, s);
@@ -214,7 +214,7 @@ pybind11::object linattn_layer(const Tensor& x_in, const variable_list& p, const
       !shaped(p[kOutB], {out_dim}))
     return pybind11::none();
   const c10::cuda::CUDAGuard guard(x_in.device());
-  const Tensor x = x_in.contiguous(), s0 = carry_leaf(s0_in, x.size(0) * hid * d, at::kFloat, "s0"), z0 = carry_leaf(z0_in, x.size(0) * hid, at::kFloat, "z0"), done = done_bytes(done_in, x.size(0) * x.size(1));
+  const Tensor x = dense(x_in), s0 = carry_leaf(s0_in, x.size(0) * hid * d, at::kFloat, "s0"), z0 = carry_leaf(z0_in, x.size(0) * hid, at::kFloat, "z0"), done = done_bytes(done_in, x.size(0) * x.size(1));
   if (wants_grad(x, p, {s0, z0})) {
     const variable_list out = LinAttnLayer::apply(x, p[0], p[1], p[2], p[3], p[4], p[5], opt(s0), opt(z0), opt(done), heads, eps, norm_eps);
     return pybind11::cast(std::make_tuple(out[0], out[1], out[2]));
@@ -281,8 +281,8 @@ struct DeltaLayer : torch::autograd::Function<DeltaLayer> {
     const c10::cuda::CUDAGuard guard(x.device());
     const int64_t hid = out_w.size(1);
     const Shape s = shape_of(x, ctx->saved_data["heads"].toInt(), hid, out_w.size(0), 2 * ctx->saved_data["heads"].toInt());
-    const Tensor gy = matrix(gout[1].defined() ? gout[1].contiguous() : empty_like_of(x, {s.M, s.out}, at::kBFloat16).zero_(), s.M, s.out);
-    const Tensor gs = gout[0].defined() ? gout[0].contiguous() : Tensor();
+    const Tensor gy = matrix(gout[1].defined() ? dense(gout[1]) : empty_like_of(x, {s.M, s.out}, at::kBFloat16).zero_(), s.M, s.out);
+    const Tensor gs = gout[0].defined() ? dense(gout[0]) : Tensor();
     const bool need_s0 = ctx->saved_data["s0"].toBool() && ctx->needs_input_grad(9);
     const TailGrads t = tail_backward(gy, o, saved[13], saved[14], norm_w, out_w, s);
     const Tensor gproj = empty_like_of(x, proj.sizes(), at::kBFloat16), gq = empty_like_of(x, q.sizes(), at::kBFloat16), gk = empty_like_of(x, k.sizes(), at::kBFloat16);
@@ -323,7 +323,7 @@ pybind11::object deltanet_layer(const Tensor& x_in, const variable_list& p, cons
       !shaped(p[kDNorm], {hid}) || !shaped(p[kDOutW], {out_dim, hid}) || !shaped(p[kDOutB], {out_dim}))
     return pybind11::none();
   const c10::cuda::CUDAGuard guard(x_in.device());
-  const Tensor x = x_in.contiguous(), s0 = carry_leaf(s0_in, x.size(0) * hid * d, at::kFloat, "s0"), done = done_bytes(done_in, x.size(0) * x.size(1));
+  const Tensor x = dense(x_in), s0 = carry_leaf(s0_in, x.size(0) * hid * d, at::kFloat, "s0"), done = done_bytes(done_in, x.size(0) * x.size(1));
   if (wants_grad(x, p, {s0})) {
     const variable_list out = DeltaLayer::apply(x, p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7], opt(s0), opt(done), heads, norm_eps);
     return pybind11::cast(std::make_tuple(out[0], out[1]));

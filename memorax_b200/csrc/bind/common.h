@@ -52,10 +52,12 @@ void check(const char* fn, int status);
 // an autograd node takes what may be missing as an optional
 inline OptTensor opt(const Tensor& t) { return t.defined() ? OptTensor(t) : std::nullopt; }
 
+// Dense memory that holds the values themselves: a conjugated (negated) view is a bit on the same memory, contiguous or not.
+inline Tensor dense(const Tensor& t) { return (t.is_conj() || t.is_neg() ? t.resolve_conj().resolve_neg() : t).contiguous(); }
 inline Tensor dev(const OptTensor& t, at::ScalarType dtype, const char* name) {
   if (!t || !t->defined()) return Tensor();
   TORCH_CHECK_VALUE(t->is_cuda(), name, " must be a CUDA tensor (memorax_b200 has no CPU path)");
-  return (t->scalar_type() == dtype ? *t : t->to(dtype)).contiguous();
+  return dense(t->scalar_type() == dtype ? *t : t->to(dtype));
 }
 // (B,T) flags of any dtype -> bytes
 inline Tensor done_bytes(const OptTensor& done, int64_t steps) {

@@ -40,7 +40,7 @@ struct Linear32 : torch::autograd::Function<Linear32> {
   }
   static variable_list backward(AutogradContext* ctx, const variable_list& gout) {
     const auto saved = ctx->get_saved_variables();
-    const Tensor &x = saved[0], &w = saved[1], gy = gout[0].contiguous();
+    const Tensor &x = saved[0], &w = saved[1], gy = dense(gout[0]);
     const c10::cuda::CUDAGuard guard(x.device());
     const int K = x.size(-1), N = w.size(0), M = x.numel() / K;
     variable_list grads(3);
@@ -65,7 +65,7 @@ Tensor linear_f32(const Tensor& x, const Tensor& w, const OptTensor& bias) {
       x.numel() / x.size(-1) > 0x7fffffff || tf32_products() || at::autocast::is_autocast_enabled(at::kCUDA) || followed(x, {w}, bias))
     return at::linear(x, w, bias);
   const c10::cuda::CUDAGuard guard(x.device());
-  return Linear32::apply(x.contiguous(), w.contiguous(), bias ? OptTensor(bias->contiguous()) : std::nullopt);
+  return Linear32::apply(dense(x), dense(w), bias ? OptTensor(dense(*bias)) : std::nullopt);
 }
 
 // a (.., M, K) b (.., K, N) (+ bias) (+ c) in bf16 through this repository's kernel

@@ -105,8 +105,8 @@ struct LruLayer : torch::autograd::Function<LruLayer> {
     bool need_params = false;
     for (int i = 1; i <= kParams; ++i) need_params |= ctx->needs_input_grad(i);
     const bool need_x = ctx->needs_input_grad(0), need_h0 = h0.defined() && ctx->needs_input_grad(9);
-    const Tensor gh_last = gout[0].defined() ? gout[0].contiguous() : Tensor();
-    const Tensor gy = gout[2].defined() ? gout[2].contiguous() : at::zeros_like(x);
+    const Tensor gh_last = gout[0].defined() ? dense(gout[0]) : Tensor();
+    const Tensor gy = gout[2].defined() ? dense(gout[2]) : at::zeros_like(x);
 
     Tensor gx = empty_like_of(x, x.sizes(), at::kFloat);
     Tensor gh0 = need_h0 ? empty_like_of(x, {B, 1, N}, at::kComplexFloat) : Tensor();
@@ -190,7 +190,7 @@ pybind11::object lru_layer(const Tensor& x_in, const variable_list& params, cons
                            const OptTensor& done_in) {
   if (!native(x_in, params) || followed(x_in, params, h0_in, a0_in)) return pybind11::none();
   const c10::cuda::CUDAGuard guard(x_in.device());
-  const Tensor x = (x_in.scalar_type() == at::kFloat ? x_in : x_in.to(at::kFloat)).contiguous();
+  const Tensor x = dense(x_in.scalar_type() == at::kFloat ? x_in : x_in.to(at::kFloat));
   const Tensor h0 = carry_leaf(h0_in, x.size(0) * params[0].size(0), at::kComplexFloat, "h0"), a0 = carry_leaf(a0_in, x.size(0) * params[0].size(0), at::kComplexFloat, "a0"), done = done_bytes(done_in, x.size(0) * x.size(1));
   if (wants_grad(x, params, h0)) {
     const variable_list out = LruLayer::apply(x, params[0], params[1], params[2], params[3], params[4], params[5], params[6],
@@ -208,7 +208,7 @@ pybind11::object lru_rtrl(const Tensor& x_in, const variable_list& params, const
   if (!native(x_in, params) || sens_in.size() != 5 || x_in.size(0) > 65535 || followed(x_in, params, h0_in, a0_in) || followed(x_in, sens_in)) return pybind11::none();
   const int B = x_in.size(0), T = x_in.size(1), F = x_in.size(2), N = params[0].size(0);
   const c10::cuda::CUDAGuard guard(x_in.device());
-  const Tensor x = (x_in.scalar_type() == at::kFloat ? x_in : x_in.to(at::kFloat)).contiguous();
+  const Tensor x = dense(x_in.scalar_type() == at::kFloat ? x_in : x_in.to(at::kFloat));
   const Tensor h0 = carry_leaf(h0_in, x.size(0) * params[0].size(0), at::kComplexFloat, "h0"), a0 = carry_leaf(a0_in, x.size(0) * params[0].size(0), at::kComplexFloat, "a0"), done = done_bytes(done_in, x.size(0) * x.size(1));
   bool grad = wants_grad(x, params, h0);
   variable_list sens, out;

@@ -96,8 +96,8 @@ struct MambaLayer : torch::autograd::Function<MambaLayer> {
     const auto s = stream();
     const l::MambaParams w = scan_params(p, ctx->saved_data["eps"].toDouble());
     const bool need_x = ctx->needs_input_grad(0), need_h0 = ctx->saved_data["h0"].toBool() && ctx->needs_input_grad(13);
-    const Tensor gh_last = gout[0].defined() ? gout[0].contiguous() : Tensor();
-    const Tensor gy = gout[2].defined() ? gout[2].contiguous() : empty_like_of(x, {B, T, out}, at::kFloat).zero_();
+    const Tensor gh_last = gout[0].defined() ? dense(gout[0]) : Tensor();
+    const Tensor gy = gout[2].defined() ? dense(gout[2]) : empty_like_of(x, {B, T, out}, at::kFloat).zero_();
     variable_list grads(17);
     if (need_x) grads[0] = empty_like_of(x, x.sizes(), at::kFloat);
     if (need_h0) grads[13] = empty_like_of(x, {B, 1, H, 16, 16}, at::kFloat);
@@ -159,7 +159,7 @@ pybind11::object mamba_layer(const Tensor& x_in, const variable_list& p, const O
       !shaped(p[kOutW], {out_dim, 16 * H}) || !shaped(p[kOutB], {out_dim}) || x_in.size(0) * H > 0x7fffffff)
     return pybind11::none();
   const c10::cuda::CUDAGuard guard(x_in.device());
-  const Tensor x = x_in.contiguous(), h0 = carry_leaf(h0_in, x.size(0) * H * 256, at::kFloat, "h0"), a0 = carry_leaf(a0_in, x.size(0) * H, at::kFloat, "a0"), done = done_bytes(done_in, x.size(0) * x.size(1));
+  const Tensor x = dense(x_in), h0 = carry_leaf(h0_in, x.size(0) * H * 256, at::kFloat, "h0"), a0 = carry_leaf(a0_in, x.size(0) * H, at::kFloat, "a0"), done = done_bytes(done_in, x.size(0) * x.size(1));
   bool grad = x.requires_grad() || (h0.defined() && h0.requires_grad());
   for (const Tensor& t : p) grad |= t.requires_grad();
   if (at::GradMode::is_enabled() && grad) {

@@ -72,8 +72,8 @@ struct MinGruLayer : torch::autograd::Function<MinGruLayer> {
     const int B = in.size(0), T = in.size(1), F = in.size(2), D = w_z.size(0), M = B * T;
     const bool need_in = ctx->needs_input_grad(0), need_w = ctx->needs_input_grad(1) || ctx->needs_input_grad(2);
     const bool need_x0 = x0.defined() && ctx->needs_input_grad(3);
-    const Tensor gx_last = gout[0].defined() ? gout[0].contiguous() : Tensor();
-    const Tensor gy = gout[2].defined() ? gout[2].contiguous() : at::zeros_like(x);
+    const Tensor gx_last = gout[0].defined() ? dense(gout[0]) : Tensor();
+    const Tensor gy = gout[2].defined() ? dense(gout[2]) : at::zeros_like(x);
     variable_list grads(6);
     if (need_x0) grads[3] = empty_like_of(in, {B, 1, D}, at::kFloat);
     if (need_in) grads[0] = empty_like_of(in, in.sizes(), at::kFloat);
@@ -108,7 +108,7 @@ pybind11::object mingru_layer(const Tensor& in_, const Tensor& w_z, const Tensor
       followed(in_, {w_z, w_h}, x0_in, a0_in))
     return pybind11::none();
   const c10::cuda::CUDAGuard guard(in_.device());
-  const Tensor in = in_.contiguous(), x0 = carry_leaf(x0_in, in.size(0) * w_z.size(0), at::kFloat, "x0"), a0 = carry_leaf(a0_in, in.size(0) * w_z.size(0), at::kFloat, "a0"), done = done_bytes(done_in, in.size(0) * in.size(1));
+  const Tensor in = dense(in_), x0 = carry_leaf(x0_in, in.size(0) * w_z.size(0), at::kFloat, "x0"), a0 = carry_leaf(a0_in, in.size(0) * w_z.size(0), at::kFloat, "a0"), done = done_bytes(done_in, in.size(0) * in.size(1));
   if (at::GradMode::is_enabled() && (in.requires_grad() || w_z.requires_grad() || w_h.requires_grad() || (x0.defined() && x0.requires_grad()))) {
     const variable_list out = MinGruLayer::apply(in, w_z, w_h, opt(x0), opt(a0), opt(done));
     return pybind11::cast(std::make_tuple(out[0], out[1], out[2]));

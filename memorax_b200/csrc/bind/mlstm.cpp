@@ -117,9 +117,9 @@ struct MlstmLayer : torch::autograd::Function<MlstmLayer> {
     const auto bf = at::kBFloat16;
     const auto st = stream();
     const int64_t out = p[kOut].size(0);
-    const auto given = [&](int i) { return gout[i].defined() ? gout[i].contiguous() : Tensor(); };
+    const auto given = [&](int i) { return gout[i].defined() ? dense(gout[i]) : Tensor(); };
     const Tensor gc = given(0), gn = given(1), gm = given(2);
-    const Tensor gy = matrix(gout[4].defined() ? gout[4].contiguous() : empty_like_of(x, {s.M, out}, bf).zero_(), s.M, out);
+    const Tensor gy = matrix(gout[4].defined() ? dense(gout[4]) : empty_like_of(x, {s.M, out}, bf).zero_(), s.M, out);
     // inputs of the node: x, the parameters, then what there is of the carry
     variable_list grads(1 + kParams + 6);
     const int first = 1 + kParams;
@@ -206,7 +206,7 @@ pybind11::object mlstm_layer(const Tensor& x_in, const variable_list& p, const O
     return pybind11::none();
   const c10::cuda::CUDAGuard guard(x_in.device());
   const int64_t B = x_in.size(0);
-  const Tensor x = x_in.contiguous(), done = done_bytes(done_in, x.size(0) * x.size(1));
+  const Tensor x = dense(x_in), done = done_bytes(done_in, x.size(0) * x.size(1));
   const Tensor c0 = carry_leaf(c_in, B * hid * d, at::kFloat, "c0"), f0 = carry_leaf(f_in, B * H, at::kFloat, "f0"), n0 = carry_leaf(n_in, B * hid, at::kFloat, "n0"),
                m0 = carry_leaf(m_in, B * H, at::kFloat, "m0");
   bool grad = x.requires_grad();

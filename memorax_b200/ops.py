@@ -33,6 +33,8 @@ def _dev(t, dtype, name):
         raise ValueError(f"{name} must be a CUDA tensor (memorax_b200 has no CPU path)")
     if t.dtype != dtype:
         t = t.to(dtype)
+    if t.is_conj() or t.is_neg():     # a view's bit, which the memory does not show
+        t = t.resolve_conj().resolve_neg()
     return t.contiguous()
 
 

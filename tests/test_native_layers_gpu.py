@@ -120,3 +120,23 @@ def test_tf32_products_are_composed(kind, setting):
     finally:
         setattr(matmul, name, before)
     assert torch.equal(got, want) and not torch.equal(got, exact)
+
+
+# conj() only sets a bit: the memory that a kernel would read is the unconjugated tensor's
+@pytest.mark.parametrize("kind", ["lru", "s5"])
+def test_conjugated_views_are_what_they_show(kind):
+    from memorax_b200 import memoroid, ops
+    torch.manual_seed(0)
+    model = memoroid.Memoroid(CELLS[kind](memoroid)).cuda()
+    x, done = torch.randn(2, 5, 32, device="cuda"), torch.zeros(2, 5, device="cuda")
+    c64 = lambda: torch.view_as_complex(torch.randn(2, 1, 16, 2, device="cuda")).conj()
+    state, one, cotangent = c64(), torch.ones(2, 1, 16, dtype=torch.complex64, device="cuda"), c64()
+    params = list(model.parameters())
+    runs = []
+    for view in (lambda t: t, lambda t: t.resolve_conj()):
+        (h, _), y = model(x, done, (view(state), one))
+        runs.append([h, y, *torch.autograd.grad(h, params, view(cotangent), allow_unused=True)])
+    for got, want in zip(*runs):
+        assert (got is None and want is None) or torch.equal(got, want)
+    a, b = state[0, 0], c64().expand(2, 3, 16).resolve_conj().conj()
+    assert torch.equal(ops.linrec_fwd(a, b)[0], ops.linrec_fwd(a.resolve_conj(), b.resolve_conj())[0])
