@@ -23,18 +23,19 @@ g::Weight stacked(const Tensor& w_z, const Tensor& w_h) {
 }
 
 struct Result {
-  Tensor x, y, a_last, zh;   // zh: both pre-activations, (B, T, 2D)
+  Tensor y, x_last, a_last;
+  Tensor zh, states, forms;   // for the backward pass; zh: both pre-activations, (B, T, 2D)
 };
 
 Result forward(const Tensor& in, const Tensor& w_z, const Tensor& w_h, const Tensor& x0, const Tensor& a0, const Tensor& done,
                bool keep) {
   const int B = in.size(0), T = in.size(1), F = in.size(2), D = w_z.size(0), M = B * T;
   Result r;
-  r.x = empty_like_of(in, {B, T, D}, at::kFloat);
   r.y = empty_like_of(in, {B, T, D}, at::kFloat);
+  r.x_last = empty_like_of(in, {B, 1, D}, at::kFloat);
   r.a_last = empty_like_of(in, {B, 1, D}, at::kFloat);
   if (T == 1 && !keep) {
-    check("mingru_step", mxk::layers::mingru_step(ptr(in), ptr(w_z), ptr(w_h), ptr(x0), ptr(a0), bytes(done), ptr(r.x), ptr(r.y), ptr(r.a_last), B, F, D, stream()));
+    check("mingru_step", mxk::layers::mingru_step(ptr(in), ptr(w_z), ptr(w_h), ptr(x0), ptr(a0), bytes(done), ptr(r.x_last), ptr(r.y), ptr(r.a_last), B, F, D, stream()));
     return r;
   }
   r.zh = empty_like_of(in, {B, T, 2 * D}, at::kFloat);
@@ -44,13 +45,16 @@ Result forward(const Tensor& in, const Tensor& w_z, const Tensor& w_h, const Ten
   mem.alloc(in);
   mxk::layers::NearKink kink;
   if (keep) {   // (only gradients tell the two sides of the kink apart)
+    r.states = empty_like_of(in, {B, T, D}, at::kFloat);
+    r.forms = scratch(in, mxk::layers::mingru_forms(B, T, D));
     kink = {ptr(r.zh) + D, ptr(in), ptr(w_h), mem.at(norms), F};
     check("row_norms", mxk::layers::row_norms(ptr(in), M, ptr(w_h), D, F, mem.at(norms), stream()));
   }
   const g::WeightJob job{stacked(w_z, w_h), false, 2 * D, F, g::tile_width(M, 2 * D, F), mem.at<void>(image)};
   check("split_weights", g::split_weights(&job, 1, {}, stream()));
   check("run_weights", g::run_weights(ptr(in), F, job.image, ptr(r.zh), 2 * D, M, 2 * D, F, {}, mem.at(ws), ws_bytes, status_ptr(in), stream()));
-  check("mingru_fwd", mxk::layers::mingru_fwd(ptr(r.zh), ptr(r.zh) + D, kink, 2 * D, ptr(x0), ptr(a0), bytes(done), ptr(r.x), ptr(r.y), ptr(r.a_last), B, T, D, stream()));
+  check("mingru_fwd", mxk::layers::mingru_fwd(ptr(r.zh), ptr(r.zh) + D, kink, 2 * D, ptr(x0), ptr(a0), bytes(done), ptr(r.states), ptr<uint8_t>(r.forms), ptr(r.y),
+                                              ptr(r.x_last), ptr(r.a_last), B, T, D, stream()));
   return r;
 }
 
@@ -60,20 +64,21 @@ struct MinGruLayer : torch::autograd::Function<MinGruLayer> {
     const Tensor x0 = x0_in.value_or(Tensor()), a0 = a0_in.value_or(Tensor()), done = done_in.value_or(Tensor());
     Result r = mxk_host::forward(in, w_z, w_h, x0, a0, done, true);
     ctx->set_materialize_grads(false);
-    ctx->save_for_backward({in, w_z, w_h, x0, done, r.x, r.zh, r.y});
+    // (not the read-out, which the caller may change in place)
+    ctx->save_for_backward({in, w_z, w_h, x0, done, r.zh, r.states, r.forms});
     ctx->mark_non_differentiable({r.a_last});
-    return {last_state(r.x).clone(), r.a_last, r.y};
+    return {r.x_last, r.a_last, r.y};
   }
 
   static variable_list backward(AutogradContext* ctx, const variable_list& gout) {
     const variable_list saved = ctx->get_saved_variables();
-    const Tensor &in = saved[0], &w_z = saved[1], &w_h = saved[2], &x0 = saved[3], &done = saved[4], &x = saved[5], &zh = saved[6];
+    const Tensor &in = saved[0], &w_z = saved[1], &w_h = saved[2], &x0 = saved[3], &done = saved[4], &zh = saved[5], &states = saved[6];
     const c10::cuda::CUDAGuard guard(in.device());
     const int B = in.size(0), T = in.size(1), F = in.size(2), D = w_z.size(0), M = B * T;
     const bool need_in = ctx->needs_input_grad(0), need_w = ctx->needs_input_grad(1) || ctx->needs_input_grad(2);
     const bool need_x0 = x0.defined() && ctx->needs_input_grad(3);
     const Tensor gx_last = gout[0].defined() ? dense(gout[0]) : Tensor();
-    const Tensor gy = gout[2].defined() ? dense(gout[2]) : at::zeros_like(x);
+    const Tensor gy = gout[2].defined() ? dense(gout[2]) : empty_like_of(in, {B, T, D}, at::kFloat).zero_();
     variable_list grads(6);
     if (need_x0) grads[3] = empty_like_of(in, {B, 1, D}, at::kFloat);
     if (need_in) grads[0] = empty_like_of(in, in.sizes(), at::kFloat);
@@ -82,7 +87,7 @@ struct MinGruLayer : torch::autograd::Function<MinGruLayer> {
     const size_t gzh = mem.take(sizeof(float) * 2 * D * M), image = mem.take(g::image_bytes(M, F, 2 * D));
     const size_t ws_bytes = std::max(g::workspace_bytes(M, F, 2 * D), g::workspace_bytes(2 * D, F, M)), ws = mem.take(ws_bytes);
     mem.alloc(in);
-    check("mingru_bwd", mxk::layers::mingru_bwd(ptr(zh), ptr(zh) + D, 2 * D, ptr(x), ptr(saved[7]), ptr(x0), bytes(done), nullptr, ptr(gy), ptr(gx_last), mem.at(gzh),
+    check("mingru_bwd", mxk::layers::mingru_bwd(ptr(zh), ptr(zh) + D, 2 * D, ptr(states), bytes(saved[7]), ptr(x0), bytes(done), nullptr, ptr(gy), ptr(gx_last), mem.at(gzh),
                                                 mem.at(gzh) + D, need_x0 ? ptr(grads[3]) : nullptr, B, T, D, stream()));
     if (need_in) {
       const g::WeightJob job{stacked(w_z, w_h), true, F, 2 * D, g::tile_width(M, F, 2 * D), mem.at<void>(image)};
@@ -114,7 +119,7 @@ pybind11::object mingru_layer(const Tensor& in_, const Tensor& w_z, const Tensor
     return pybind11::cast(std::make_tuple(out[0], out[1], out[2]));
   }
   const Result r = forward(in, w_z, w_h, x0, a0, done, false);
-  return pybind11::cast(std::make_tuple(last_state(r.x), r.a_last, r.y));
+  return pybind11::cast(std::make_tuple(r.x_last, r.a_last, r.y));
 }
 
 }  // namespace

@@ -57,10 +57,13 @@ struct NearKink {
   int F = 0;
 };
 // z and h_tilde are (B, T, D) with rows of both (and of their cotangents) `ld` floats apart; the rest is dense.
+// states (or null): the log states; with `forms` (mingru_forms bytes) each block leaves a turn's as it had them, linear or log,
+// for the backward pass, and says which.  y: the read-out; x_last, a_last: the next carry.  Each may be null.
+size_t mingru_forms(int B, int T, int D);
 int mingru_fwd(const float* z, const float* h_tilde, const NearKink& kink, long long ld, const float* x0, const float* a0,
-               const uint8_t* done, float* x, float* y, float* a_last, int B, int T, int D, cudaStream_t stream);
-// y: the read-out exp(x), or null
-int mingru_bwd(const float* z, const float* h_tilde, long long ld, const float* x, const float* y, const float* x0, const uint8_t* done,
+               const uint8_t* done, float* states, uint8_t* forms, float* y, float* x_last, float* a_last, int B, int T, int D,
+               cudaStream_t stream);
+int mingru_bwd(const float* z, const float* h_tilde, long long ld, const float* states, const uint8_t* forms, const float* x0, const uint8_t* done,
                const float* gx, const float* gy, const float* gx_last, float* gz, float* gh, float* gx0, int B, int T, int D,
                cudaStream_t stream);
 // One time step of the layer: the two Dense layers w_z, w_h (D, F), the gates and the recurrence.

@@ -939,7 +939,7 @@ int mxk_mingru_f32_fwd(const float* z, const float* h_tilde, const float* x0, co
   const long long total = static_cast<long long>(B) * D;
   const int w = pick_width(total, D, false, {z, h_tilde, x0, a0, x, y, a_last});
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (!mingru_walks(B, D)) return layers::mingru_fwd(z, h_tilde, {}, D, x0, a0, done, x, y, a_last, B, T, D, s);
+  if (!mingru_walks(B, D)) return layers::mingru_fwd(z, h_tilde, {}, D, x0, a0, done, x, nullptr, y, nullptr, a_last, B, T, D, s);
   if (w == 4)
     mxk::launch_kernel(loglinrec_fwd_kernel<4, true>, blocks_for(total / 4), kBlock, 0, s, z, h_tilde, x0, a0, done, x, y, a_last, B, T, D);
   else

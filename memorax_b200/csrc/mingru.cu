@@ -7,7 +7,7 @@
 // no relative precision and needs one logarithm per element instead of a logaddexp; where a pre-activation or the carry
 // is so large that exp could leave float32's range (kSafe), the block takes the log form for that stretch of time.
 //
-// Bound: HBM (16 / 28 bytes per element; 30 / 53 us for 12.3 M elements) and about five special-function evaluations
+// Bound: HBM (16 / 24 bytes per element; 30 / 45 us for 12.3 M elements) and about five special-function evaluations
 // per element, which have to overlap: time is split over sixteen warps of a block.  A block owns 32 channels of one
 // sequence; every thread loads its stretch of at most kSteps steps, folds it into one affine map of the incoming value
 // (forward: the state, backward: the carried cotangent; a reset cuts the map's slope), the sixteen maps are chained
@@ -23,6 +23,8 @@ namespace layers {
 namespace {
 
 constexpr int kSegs = 16, kSteps = 8;
+// How a block took a turn, and left its states with `forms`.
+constexpr uint8_t kLinear = 0, kLog = 1;
 
 // d log g / dh~ jumps at h~ = 0 (from 1/2 to 2), so an element whose sign hangs on the rounding of its dot product is
 // decided by the plain float32 sum in the order of k: the branch, and with it the gradient, does not depend on how the
@@ -98,7 +100,8 @@ __global__ void __launch_bounds__(32 * kSegs, 2)
 mingru_fwd_kernel(const float* __restrict__ z, const float* ht, float* ht_kink, const float* __restrict__ dense_in,
                   const float* __restrict__ dense_w, const float* __restrict__ norms, int F, long long ld,
                   const float* __restrict__ x0, const float* __restrict__ a0, const uint8_t* __restrict__ done,
-                  float* __restrict__ x, float* __restrict__ y, float* __restrict__ a_last, int B, int T, int D, int turn_len) {
+                  float* __restrict__ states, uint8_t* __restrict__ forms, float* __restrict__ y, float* __restrict__ x_last,
+                  float* __restrict__ a_last, int B, int T, int D, int turn_len) {
   enter_kernel();
   __shared__ float sa[kSegs][32], sq[kSegs][32], sd[kSegs][32];
   __shared__ unsigned sr[kSegs];   // reset bits of a stretch
@@ -113,6 +116,7 @@ mingru_fwd_kernel(const float* __restrict__ z, const float* ht, float* ht_kink, 
     carry_x[lane] = (in && x0) ? x0[static_cast<size_t>(b) * D + d] : -INFINITY;
     carry_a[lane] = (in && a0) ? a0[static_cast<size_t>(b) * D + d] : 0.f;
   }
+  const auto form_at = [&](int turn_no) { return static_cast<size_t>(blockIdx.x) * ((T + turn_len - 1) / turn_len) + turn_no; };
   const float range = (ht_kink && in) ? kNearKink * __ldg(norms + static_cast<long long>(B) * T + d) : 0.f;
   for (int turn = 0; turn < T; turn += turn_len) {
     const int t_begin = turn + seg * len, t_end = min(min(T, turn + turn_len), t_begin + len);
@@ -155,6 +159,7 @@ mingru_fwd_kernel(const float* __restrict__ z, const float* ht, float* ht_kink, 
     }
     const bool linear = !__syncthreads_or(!(most <= kSafe) || (seg == 0 && !(carry_x[lane] <= kSafe)));
     const size_t out0 = (static_cast<size_t>(b) * T + t_begin) * D + d;
+    if (forms && threadIdx.x == 0) forms[form_at(turn / turn_len)] = linear ? kLinear : kLog;
     if (linear) {
       // h -> A h + Q; dec: decays since the last reset
       float A = 1.f, Q = 0.f, dec = 0.f, prod = 1.f;
@@ -178,18 +183,16 @@ mingru_fwd_kernel(const float* __restrict__ z, const float* ht, float* ht_kink, 
       float cur = exp_ls(carry_x[lane]);
       __syncthreads();
       for (int s2 = 0; s2 < seg; ++s2) cur = fmaf(sa[s2][lane], cur, sq[s2][lane]);
-      float last = 0.f;
-      float *px = x + out0, *py = y + out0;
+      float *ps = states + out0, *py = y + out0;
 #pragma unroll
       for (int i = 0; i < kSteps; ++i) {
         if (i < count) {
           cur = (resets >> i & 1u) ? lv[i] : fmaf(dv[i], cur, lv[i]);
-          last = log_safe(cur);
           if (in) {
-            st_stream(px, last);
+            if (states) st_stream(ps, forms ? cur : log_safe(cur));
             if (y) st_stream(py, cur);
           }
-          px += D;
+          ps += D;
           py += D;
         }
       }
@@ -198,7 +201,7 @@ mingru_fwd_kernel(const float* __restrict__ z, const float* ht, float* ht_kink, 
         float acc = carry_a[lane];
         for (int s2 = 0; s2 < kSegs; ++s2) acc = sr[s2] ? sd[s2][lane] : acc + sd[s2][lane];
         carry_a[lane] = acc;
-        carry_x[lane] = last;
+        carry_x[lane] = log_safe(cur);
       }
       __syncthreads();
       continue;
@@ -229,7 +232,7 @@ mingru_fwd_kernel(const float* __restrict__ z, const float* ht, float* ht_kink, 
       if (i < count) {
         cur = (resets >> i & 1u) ? lv[i] : log_add_exp(dv[i] + cur, lv[i]);
         if (in) {
-          st_stream(x + out0 + static_cast<size_t>(i) * D, cur);
+          if (states) st_stream(states + out0 + static_cast<size_t>(i) * D, cur);
           if (y) st_stream(y + out0 + static_cast<size_t>(i) * D, exp_ls(cur));
         }
       }
@@ -242,13 +245,16 @@ mingru_fwd_kernel(const float* __restrict__ z, const float* ht, float* ht_kink, 
     }
     __syncthreads();
   }
-  if (seg == 0 && in && a_last) a_last[static_cast<size_t>(b) * D + d] = carry_a[lane];
+  if (seg == 0 && in) {
+    if (x_last) x_last[static_cast<size_t>(b) * D + d] = carry_x[lane];
+    if (a_last) a_last[static_cast<size_t>(b) * D + d] = carry_a[lane];
+  }
 }
 
-// y: the states exp(x) where the caller has them (else they are formed here)
+// states, forms: as the forward kernel left them (without forms: log states)
 __global__ void __launch_bounds__(32 * kSegs, 2)
-mingru_bwd_kernel(const float* __restrict__ z, const float* __restrict__ ht, long long ld, const float* __restrict__ x,
-                  const float* __restrict__ y, const float* __restrict__ x0, const uint8_t* __restrict__ done,
+mingru_bwd_kernel(const float* __restrict__ z, const float* __restrict__ ht, long long ld, const float* __restrict__ states,
+                  const uint8_t* __restrict__ forms, const float* __restrict__ x0, const uint8_t* __restrict__ done,
                   const float* __restrict__ gx, const float* __restrict__ gy, const float* __restrict__ gx_last,
                   float* __restrict__ gz, float* __restrict__ gh, float* __restrict__ gx0, int B, int T, int D, int turn_len) {
   enter_kernel();
@@ -266,17 +272,20 @@ mingru_bwd_kernel(const float* __restrict__ z, const float* __restrict__ ht, lon
     const int count = t_end - t_begin;   // steps of this warp (may be negative)
     const size_t at0 = (static_cast<size_t>(b) * T + t_begin) * D + d;
     const long long io0 = (static_cast<long long>(b) * T + t_begin) * ld + d;
-    const float* const state = y ? y : x;
+    // how this turn's states are stored, and the one in front of this warp's first step
+    const auto stored = [&](int turn_no) { return forms ? forms[static_cast<size_t>(blockIdx.x) * ((T + turn_len - 1) / turn_len) + turn_no] : kLog; };
+    const bool logs = stored(turn / turn_len) == kLog;
+    const bool prev_log = t_begin == 0 || (t_begin > turn ? logs : stored(turn / turn_len - 1) == kLog);
     float zv[kSteps], hv[kSteps], sv[kSteps], e[kSteps], w[kSteps], prev = 0.f;
     {
-      const float *pz = z + io0, *ph = ht + io0, *ps = state + at0, *pg = gy + at0;
+      const float *pz = z + io0, *ph = ht + io0, *ps = states + at0, *pg = gy + at0;
       if (in && count > 0) prev = t_begin > 0 ? ps[-D] : (x0 ? x0[static_cast<size_t>(b) * D + d] : -INFINITY);
 #pragma unroll
       for (int i = 0; i < kSteps; ++i) {
         const bool on = in && i < count;
         zv[i] = on ? ld_stream(pz) : 0.f;
         hv[i] = on ? ld_stream(ph) : 0.f;
-        sv[i] = on ? ld_stream(ps) : 1.f;
+        sv[i] = on ? ld_stream(ps) : (logs ? 0.f : 1.f);
         e[i] = (on && gy) ? ld_stream(pg) : 0.f;
         pz += ld;
         ph += ld;
@@ -285,18 +294,21 @@ mingru_bwd_kernel(const float* __restrict__ z, const float* __restrict__ ht, lon
       }
     }
     const unsigned resets = reset_mask(drow, t_begin, count, lane);
-    float most = (t_begin == 0 && x0) ? fmaxf(prev, 0.f) : 0.f;
+    bool linear = !logs;
+    if (!forms) {
+      float most = (t_begin == 0 && x0) ? fmaxf(prev, 0.f) : 0.f;
 #pragma unroll
-    for (int i = 0; i < kSteps; ++i) most = fmaxf(most, fmaxf(fabsf(zv[i]), fabsf(hv[i])));
-    const bool linear = !__syncthreads_or(!(most <= kSafe));
+      for (int i = 0; i < kSteps; ++i) most = fmaxf(most, fmaxf(fabsf(zv[i]), fabsf(hv[i])));
+      linear = !__syncthreads_or(!(most <= kSafe));
+    }
     // w_t = share of the incoming state in x_t; carry' = w (e + carry), right to left
     float P = 1.f, Q = 0.f;
     if (linear) {
-      if (!y) {
+      if (logs) {
 #pragma unroll
         for (int i = 0; i < kSteps; ++i) sv[i] = exp_ls(sv[i]);
       }
-      if (!y || t_begin == 0) prev = exp_ls(prev);
+      if (prev_log) prev = exp_ls(prev);
       if (gx && in) {
 #pragma unroll
         for (int i = 0; i < kSteps; ++i) e[i] = i < count ? fmaf(e[i], sv[i], gx[at0 + static_cast<size_t>(i) * D]) : 0.f;
@@ -317,20 +329,17 @@ mingru_bwd_kernel(const float* __restrict__ z, const float* __restrict__ ht, lon
       }
     } else {
       // log form, from the log states
-      float xv[kSteps];
-#pragma unroll
-      for (int i = 0; i < kSteps; ++i) xv[i] = (in && t_begin + i < t_end) ? x[at0 + static_cast<size_t>(i) * D] : 0.f;
-      if (y && t_begin > 0 && in && t_begin < t_end) prev = x[at0 - D];
+      if (!prev_log) prev = logf(prev);
 #pragma unroll
       for (int i = kSteps - 1; i >= 0; --i) {
         w[i] = 0.f;
         if (i < count) {
-          e[i] = e[i] != 0.f ? e[i] * exp_ls(xv[i]) : 0.f;
+          e[i] = e[i] != 0.f ? e[i] * exp_ls(sv[i]) : 0.f;
           if (gx && in) e[i] += gx[at0 + static_cast<size_t>(i) * D];
           const float ez = exp_ls(-fabsf(zv[i]));
           if (!(resets >> i & 1u)) {
-            const float p = -(fmaxf(zv[i], 0.f) + log1p_ls(ez)) + (i > 0 ? xv[i > 0 ? i - 1 : 0] : prev);
-            w[i] = p == -INFINITY ? 0.f : exp_ls(p - xv[i]);
+            const float p = -(fmaxf(zv[i], 0.f) + log1p_ls(ez)) + (i > 0 ? sv[i > 0 ? i - 1 : 0] : prev);
+            w[i] = p == -INFINITY ? 0.f : exp_ls(p - sv[i]);
           }
           zv[i] = (zv[i] >= 0.f ? 1.f : ez) / (1.f + ez);
           Q = w[i] * (e[i] + Q);
@@ -415,18 +424,21 @@ int row_norms(const float* a, long long rows_a, const float* b, long long rows_b
 }
 
 int mingru_fwd(const float* z, const float* h_tilde, const NearKink& kink, long long ld, const float* x0, const float* a0,
-               const uint8_t* done, float* x, float* y, float* a_last, int B, int T, int D, cudaStream_t stream) {
+               const uint8_t* done, float* states, uint8_t* forms, float* y, float* x_last, float* a_last, int B, int T, int D,
+               cudaStream_t stream) {
   if (const int st = check_dims(B, T, D)) return st;
   mxk::launch_kernel(mingru_fwd_kernel, blocks_of(B, D), 32 * kSegs, 0, stream, z, h_tilde, kink.h, kink.in, kink.w, kink.norms, kink.F, ld, x0,
-                                                                a0, done, x, y, a_last, B, T, D, turn_length(T));
+                     a0, done, states, forms, y, x_last, a_last, B, T, D, turn_length(T));
   return launch_status();
 }
 
-int mingru_bwd(const float* z, const float* h_tilde, long long ld, const float* x, const float* y, const float* x0, const uint8_t* done,
+size_t mingru_forms(int B, int T, int D) { return static_cast<size_t>(blocks_of(B, D)) * ((T + turn_length(T) - 1) / turn_length(T)); }
+
+int mingru_bwd(const float* z, const float* h_tilde, long long ld, const float* states, const uint8_t* forms, const float* x0, const uint8_t* done,
                const float* gx, const float* gy, const float* gx_last, float* gz, float* gh, float* gx0, int B, int T, int D,
                cudaStream_t stream) {
   if (const int st = check_dims(B, T, D)) return st;
-  mxk::launch_kernel(mingru_bwd_kernel, blocks_of(B, D), 32 * kSegs, 0, stream, z, h_tilde, ld, x, y, x0, done, gx, gy, gx_last, gz, gh, gx0,
+  mxk::launch_kernel(mingru_bwd_kernel, blocks_of(B, D), 32 * kSegs, 0, stream, z, h_tilde, ld, states, forms, x0, done, gx, gy, gx_last, gz, gh, gx0,
                                                                 B, T, D, turn_length(T));
   return launch_status();
 }

@@ -108,3 +108,37 @@ def test_no_input_is_slow(case):
         x = torch.zeros_like(x).scatter_(2, torch.randint(0, dim, (bsz, steps, 1), device="cuda"), 1.0)
         w *= torch.rand_like(w) > 0.5
     assert time(x) <= 3 * usual
+
+
+# three turns of 100 steps, in linear or in log form by the size of their pre-activations: the state between two turns is in
+# the form of the one it was left by
+@pytest.mark.parametrize("large", [(0,), (1,), (2,), (0, 1), (1, 2), (0, 2)])
+@pytest.mark.parametrize("with_carry", [False, True])
+def test_turns_in_different_forms(large, with_carry):
+    from memorax_b200.memoroid import MinGRUCell, Memoroid
+    bsz, steps, feat, dim = 2, 300, 16, 40
+    torch.manual_seed(0)
+    cell = MinGRUCell(dim, in_features=feat).cuda()
+    x = torch.randn(bsz, steps, feat, device="cuda")
+    for turn in large:
+        x[:, turn * 100:turn * 100 + 100] *= 40
+    x.requires_grad_()
+    done = torch.rand(bsz, steps, device="cuda") < 0.01
+    carry = (3 * torch.randn(bsz, 1, dim, device="cuda").requires_grad_(), torch.zeros(bsz, 1, dim, device="cuda")) if with_carry else None
+    gy, gl = torch.randn(bsz, steps, dim, device="cuda"), torch.randn(bsz, 1, dim, device="cuda")
+    wrt = [x, cell.z.weight, cell.h.weight] + ([carry[0]] if with_carry else [])
+    (h, _), y = Memoroid(cell)(x, done, carry)
+    grads = torch.autograd.grad((y, h), wrt, (gy, gl))
+    with torch.no_grad():
+        (h_n, _), y_n = Memoroid(cell)(x, done, carry)
+    assert torch.equal(h_n, h) and torch.equal(y_n, y)
+    d64 = lambda t: t.detach().cpu().double()
+    xd, wz, wh = (d64(t).requires_grad_() for t in wrt[:3])
+    x0 = d64(carry[0])[:, 0].requires_grad_() if with_carry else torch.full((bsz, dim), -float("inf"), dtype=torch.float64)
+    z, ht, sp = xd @ wz.t(), xd @ wh.t(), torch.nn.functional.softplus
+    xs, _ = mo.mingru_seq(-sp(-z) + torch.where(ht >= 0, torch.log(torch.relu(ht) + 0.5), -sp(-ht)), -sp(z), x0, d64(done), None)
+    want = torch.autograd.grad((xs.exp(), xs[:, -1:]), [xd, wz, wh] + ([x0] if with_carry else []), (d64(gy), d64(gl)))
+    err = lambda got, ref: float((got.detach().cpu().reshape(ref.shape) - ref.detach()).abs().max()) / max(1e-30, float(ref.detach().abs().max()))
+    assert err(h, xs[:, -1]) <= 1e-5 and err(y, xs.exp()) <= 1e-5
+    for got, ref in zip(grads, want):
+        assert err(got, ref) <= 1e-4

@@ -140,3 +140,20 @@ def test_conjugated_views_are_what_they_show(kind):
         assert (got is None and want is None) or torch.equal(got, want)
     a, b = state[0, 0], c64().expand(2, 3, 16).resolve_conj().conj()
     assert torch.equal(ops.linrec_fwd(a, b)[0], ops.linrec_fwd(a.resolve_conj(), b.resolve_conj())[0])
+
+
+# nothing that a layer returns to be read is needed by its backward pass: it may be changed in place
+@pytest.mark.parametrize("kind", CELLS)
+def test_the_read_out_may_be_changed_in_place(kind):
+    from memorax_b200 import memoroid
+    torch.manual_seed(0)
+    model = memoroid.Memoroid(CELLS[kind](memoroid)).cuda()
+    dtype = next(model.parameters()).dtype
+    x, done = torch.randn(2, 5, 32, device="cuda").to(dtype).requires_grad_(), torch.zeros(2, 5, device="cuda")
+    wrt = [x, *model.parameters()]
+    _, y = model(x, done)
+    want = torch.autograd.grad(2 * y, wrt, torch.ones_like(y))
+    _, y = model(x, done)
+    got = torch.autograd.grad(y.mul_(2), wrt, torch.ones_like(y))
+    for g, w in zip(got, want):
+        assert torch.equal(g, w)
