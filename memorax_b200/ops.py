@@ -827,8 +827,9 @@ class GatedDense(torch.autograd.Function):
 
 
 def _trains(x, layer):
-    """Whether a Dense layer over bf16 CUDA rows is in a backward pass that wants its bias gradient."""
-    return (torch.is_grad_enabled() and layer.bias is not None and x.is_cuda and x.numel() > 0 and layer.weight.shape[0] % 8 == 0
+    """Whether a Dense layer over bf16 CUDA rows is in a backward pass that wants its bias gradient (and gives bf16: under
+    autocast its product may have another type)."""
+    return (torch.is_grad_enabled() and not torch.is_autocast_enabled("cuda") and layer.bias is not None and x.is_cuda and x.numel() > 0 and layer.weight.shape[0] % 8 == 0
             and layer.bias.requires_grad and x.dtype == layer.weight.dtype == layer.bias.dtype == torch.bfloat16)
 
 

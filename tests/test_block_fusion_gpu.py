@@ -34,3 +34,17 @@ def test_joint_passes_equal_the_parts(features, rows):
     for name, a, b in zip(names, got[0][1:], got[1][1:]):
         scale = float(b.float().abs().max())
         assert float((a.float() - b.float()).abs().max()) <= 1.5e-2 * scale + 1e-6, name
+
+
+def test_products_of_another_type_under_autocast():
+    """Autocast gives a Dense layer's product its own type: the fused passes, which read bf16, leave it to the general ones."""
+    from memorax_b200 import ops
+    from memorax_b200.blocks import Dense
+    torch.manual_seed(0)
+    layer = Dense(32, 64).cuda().bfloat16()
+    x, o = torch.randn(5, 32, device="cuda").bfloat16(), torch.randn(5, 64, device="cuda").bfloat16()
+    with torch.autocast("cuda", dtype=torch.float16):
+        up, gated = ops.dense_gelu(x, layer), ops.gated_dense(o, x, layer, o)
+    a = x.double() @ layer.weight.double().t() + layer.bias.double()
+    near = lambda got, want: float((got.double() - want).detach().abs().max()) <= 2e-2 * float(want.detach().abs().max())
+    assert near(up, torch.nn.functional.gelu(a, approximate="tanh")) and near(gated, o.double() * (1 + torch.sigmoid(a)))
