@@ -747,11 +747,11 @@ class MambaCell(MemoroidCellBase):
     state with one scalar decay per (b, t, head).  Elements and read-out follow the
     reference -- ``h_t = (dt B_t) (x) x_t`` (mamba.py:109-117), operator
     ``(decay_j h_i + h_j, decay_j decay_i)`` (:119-122), ``y = C . h + D x`` gated by
-    ``silu(z)`` after an RMSNorm (:124-135) -- and, like the reference, the scan runs over the
-    materialised (B, T, H, N, P) elements: here as ONE real linear-recurrence launch over
-    H*N*P channels instead of ~2 log2(T) passes.  When a head's N*P state elements are a multiple of
-    128 (the default 16 x 16 is) the kernels read the per-head decay (B,T,H) directly and reduce its
-    gradient per head (``ops.LinRecGrouped``); otherwise the decay is expanded (``ops.LinRec``)."""
+    ``silu(z)`` after an RMSNorm (:124-135).  With 16 x 16 states a head and four taps in float32 the layer is one
+    native call that never forms the (B, T, H, N, P) elements or states.  Composed, the scan runs over the materialised
+    elements like the reference's, as ONE real linear-recurrence launch over H*N*P channels instead of ~2 log2(T) passes:
+    when a head's N*P state elements are a multiple of 128 the kernels read the per-head decay (B,T,H) directly and reduce
+    its gradient per head (``ops.LinRecGrouped``); otherwise the decay is expanded (``ops.LinRec``)."""
 
     def __init__(self, features, num_heads=8, head_dim=16, state_dim=16, conv_dim=4, in_features=None):
         super().__init__()
