@@ -5,6 +5,7 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/autograd/forward_grad.h>
 #include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/extension.h>
 
@@ -27,7 +28,9 @@ inline bool followed(const Tensor& t) { return t.defined() && t._fw_grad(0).defi
 inline bool followed(const OptTensor& t) { return t && followed(*t); }
 template <typename... T>
 inline bool followed(const Tensor& x, at::ArrayRef<Tensor> params, const T&... carry) {
-  if (torch::jit::tracer::isTracing() || followed(x) || (followed(carry) || ...)) return true;
+  if (torch::jit::tracer::isTracing()) return true;
+  if (!torch::autograd::ForwardADLevel::try_get_by_idx(0)) return false;   // (nobody has tangents)
+  if (followed(x) || (followed(carry) || ...)) return true;
   for (const Tensor& p : params)
     if (followed(p)) return true;
   return false;
