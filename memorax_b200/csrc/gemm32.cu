@@ -89,19 +89,27 @@ __device__ __forceinline__ void load8(const float* p, int valid, int vec, float*
   }
 }
 
+// Two floats to bf16, to the nearest; what lies beyond bf16's largest number, the largest floats and infinity, becomes that
+// number (an infinite plane times a zero one would be NaN).
+__device__ __forceinline__ uint32_t pack_finite(float lo, float hi) {
+  uint32_t v;
+  asm("cvt.rn.satfinite.bf16x2.f32 %0, %1, %2;" : "=r"(v) : "f"(hi), "f"(lo));
+  return v;
+}
+
 // hi / mid / lo bf16 planes of eight floats
 __device__ __forceinline__ void split8(const float* x, uint4& hi, uint4& mid, uint4& lo) {
   uint32_t h[4], m[4], l[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     float a = x[2 * i], b = x[2 * i + 1];
-    h[i] = pack_bf16(a, b);
+    h[i] = pack_finite(a, b);
     a -= __uint_as_float(h[i] << 16);
     b -= __uint_as_float(h[i] & 0xFFFF0000u);
-    m[i] = pack_bf16(a, b);
+    m[i] = pack_finite(a, b);
     a -= __uint_as_float(m[i] << 16);
     b -= __uint_as_float(m[i] & 0xFFFF0000u);
-    l[i] = pack_bf16(a, b);
+    l[i] = pack_finite(a, b);
   }
   hi = make_uint4(h[0], h[1], h[2], h[3]);
   mid = make_uint4(m[0], m[1], m[2], m[3]);

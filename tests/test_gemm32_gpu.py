@@ -105,3 +105,17 @@ def test_fused_rtrl_segment_from_sensitivities_at_any_address(feat):
         *_, got = model.local_jacobian(x, done, carry, cut)
     for k in want:
         assert torch.equal(got[k], want[k]), k
+
+
+# the largest floats lie beyond bf16's largest number, and masks are made of them
+@pytest.mark.parametrize("m,n,k", [(3, 5, 32), (130, 70, 100), (300, 256, 512)])
+def test_products_of_the_largest_floats(m, n, k):
+    from memorax_b200 import _C
+    torch.manual_seed(0)
+    x, w = torch.randn(m, k, device="cuda"), torch.randn(n, k, device="cuda") / k
+    x[0, :3], x[-1, k // 2] = torch.finfo(torch.float32).min, torch.finfo(torch.float32).max
+    got, want = _C.linear_f32(x, w), x.double() @ w.double().t()
+    assert float(((got - want).abs() / want.abs().amax(1, keepdim=True)).max()) <= 1e-6
+    x[1, 0] = float("inf")
+    got = _C.linear_f32(x, w)
+    assert not got.isnan().any() and bool((got[1].sign() == w[:, 0].sign()).all()) and float(got[1].abs().min()) > 1e30
