@@ -262,13 +262,16 @@ __device__ __forceinline__ void unit_sensitivities(const LruWeights& w, const fl
   part[warp][lane] = cmul(power(l, T - 1 - to), acc);
   __syncthreads();
   if (warp > 0 || !in) return;
-  const float2 start = h0 ? reinterpret_cast<const float2*>(h0)[at] : make_float2(0.f, 0.f);
-  const float2 p = r < 0 ? power(l, T) : make_float2(0.f, 0.f);
+  // (what a reset cuts off does not enter, finite or not)
+  const bool kept = r < 0;
+  const float2 none = make_float2(0.f, 0.f);
+  const float2 start = h0 && kept ? reinterpret_cast<const float2*>(h0)[at] : none;
+  const float2 p = kept ? power(l, T) : none;
   acc = cmul(p, start);
 #pragma unroll
   for (int i = 0; i < 8; ++i) { acc.x += part[i][lane].x; acc.y += part[i][lane].y; }
   const float en = expf(w.nu_log[n]), et = expf(w.theta_log[n]);
-  const auto old = [&](const float* q) { return reinterpret_cast<const float2*>(q)[at]; };
+  const auto old = [&](const float* q) { return kept ? reinterpret_cast<const float2*>(q)[at] : none; };
   const float2 last = hs[static_cast<size_t>(T - 1) * N], g0 = old(s.gamma);
   reinterpret_cast<float2*>(s.nu_out)[at] = cmul_add(p, old(s.nu), make_float2(-en * acc.x, -en * acc.y));
   reinterpret_cast<float2*>(s.theta_out)[at] = cmul_add(p, old(s.theta), make_float2(-et * acc.y, et * acc.x));
@@ -344,8 +347,9 @@ __global__ void __launch_bounds__(256) lru_sensitivities_kernel(LruWeights w, co
   if (!in) return;
   const float gamma = expf(w.gamma_log[n]);
   const float2 p = r < 0 ? power(reinterpret_cast<const float2*>(lambda)[n], T) : make_float2(0.f, 0.f);
-  const auto re = [&](float2 o, int e) { return cmul_add(p, o, make_float2(gamma * acc[e].x, gamma * acc[e].y)); };
-  const auto im = [&](float2 o, int e) { return cmul_add(p, o, make_float2(-gamma * acc[e].y, gamma * acc[e].x)); };
+  const auto add_old = [&](float2 o, float2 v) { return r < 0 ? cmul_add(p, o, v) : v; };
+  const auto re = [&](float2 o, int e) { return add_old(o, make_float2(gamma * acc[e].x, gamma * acc[e].y)); };
+  const auto im = [&](float2 o, int e) { return add_old(o, make_float2(-gamma * acc[e].y, gamma * acc[e].x)); };
   if (kWide) {   // two complex entries each
 #pragma unroll
     for (int e = 0; e < 2; ++e) {

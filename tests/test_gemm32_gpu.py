@@ -119,3 +119,24 @@ def test_products_of_the_largest_floats(m, n, k):
     x[1, 0] = float("inf")
     got = _C.linear_f32(x, w)
     assert not got.isnan().any() and bool((got[1].sign() == w[:, 0].sign()).all()) and float(got[1].abs().min()) > 1e30
+
+
+# an episode that has gone wrong ends at its reset
+@pytest.mark.parametrize("feat", [8, 6])
+def test_fused_rtrl_segment_forgets_at_a_reset(feat):
+    from memorax_b200.memoroid import LRUCell, Memoroid
+    torch.manual_seed(5)
+    bsz, steps, hidden = 2, 20, 40
+    model = Memoroid(LRUCell(feat, hidden).cuda())
+    x, done = torch.randn(bsz, steps, feat, device="cuda"), torch.zeros(bsz, steps, device="cuda")
+    done[:, 7] = 1
+    x[:, 3] = float("nan")
+    bad = lambda *s: torch.full(s, float("nan"), dtype=torch.complex64, device="cuda")
+    sens = {k: bad(*v.shape) for k, v in model.initialize_sensitivity(None, (bsz, feat)).items()}
+    ones = torch.ones(bsz, 1, hidden, dtype=torch.complex64, device="cuda")
+    with torch.no_grad():
+        (h, _), _, got = model.local_jacobian(x, done, (bad(bsz, 1, hidden), ones), sens)
+        zero = {k: torch.zeros_like(v) for k, v in sens.items()}
+        (h2, _), _, want = model.local_jacobian(x[:, 7:], done[:, 7:], (torch.zeros_like(ones), ones), zero)
+    for k in want:
+        assert float((got[k] - want[k]).abs().max()) <= 1e-5 * float(want[k].abs().max()), k
