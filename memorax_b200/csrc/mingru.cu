@@ -182,7 +182,8 @@ mingru_fwd_kernel(const float* __restrict__ z, const float* ht, float* ht_kink, 
       if (lane == 0) sr[seg] = resets;
       float cur = exp_ls(carry_x[lane]);
       __syncthreads();
-      for (int s2 = 0; s2 < seg; ++s2) cur = fmaf(sa[s2][lane], cur, sq[s2][lane]);
+      // (a stretch with a reset forgets what comes in, finite or not)
+      for (int s2 = 0; s2 < seg; ++s2) cur = sr[s2] ? sq[s2][lane] : fmaf(sa[s2][lane], cur, sq[s2][lane]);
       float *ps = states + out0, *py = y + out0;
 #pragma unroll
       for (int i = 0; i < kSteps; ++i) {
@@ -225,7 +226,7 @@ mingru_fwd_kernel(const float* __restrict__ z, const float* ht, float* ht_kink, 
     if (lane == 0) sr[seg] = resets;
     __syncthreads();
     float cur = carry_x[lane];
-    for (int s2 = 0; s2 < seg; ++s2) cur = log_add_exp(sa[s2][lane] + cur, sq[s2][lane]);
+    for (int s2 = 0; s2 < seg; ++s2) cur = sr[s2] ? sq[s2][lane] : log_add_exp(sa[s2][lane] + cur, sq[s2][lane]);
     __syncthreads();   // every segment has read the carry
 #pragma unroll
     for (int i = 0; i < kSteps; ++i) {

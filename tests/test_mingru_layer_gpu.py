@@ -142,3 +142,31 @@ def test_turns_in_different_forms(large, with_carry):
     assert err(h, xs[:, -1]) <= 1e-5 and err(y, xs.exp()) <= 1e-5
     for got, ref in zip(grads, want):
         assert err(got, ref) <= 1e-4
+
+
+# a step that is not finite spoils its episode, and ends with it: in the same stretch of steps, turn, and in a later one
+@pytest.mark.parametrize("steps,bad,reset", [(20, 3, 9), (100, 10, 12), (100, 3, 70), (300, 50, 60), (300, 50, 250)])
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("raw", [False, True])
+@pytest.mark.parametrize("with_carry", [False, True])
+def test_a_broken_episode_ends_at_its_reset(steps, bad, reset, value, raw, with_carry):
+    from memorax_b200.memoroid import MinGRUCell, Memoroid, MemoroidCellBase
+    torch.manual_seed(0)
+    bsz, dim = 2, 40
+    cell = MinGRUCell(dim).cuda()
+    layer = (lambda *a: MemoroidCellBase.layer(cell, *a)) if raw else Memoroid(cell)
+    x = torch.randn(bsz, steps, dim, device="cuda")
+    x[:, bad] = value
+    x.requires_grad_()
+    done = torch.zeros(bsz, steps, device="cuda")
+    done[:, reset] = 1
+    gy = torch.zeros(bsz, steps, dim, device="cuda")
+    gy[:, reset:] = torch.randn(bsz, steps - reset, dim, device="cuda")
+    carry = (torch.full((bsz, 1, dim), value, device="cuda"), torch.zeros(bsz, 1, dim, device="cuda")) if with_carry else None
+    (h, a), y = layer(x, done, carry)
+    (gx,) = torch.autograd.grad(y, x, gy)
+    rest = x.detach()[:, reset:].requires_grad_()
+    (h2, a2), y2 = layer(rest, done[:, reset:], None)
+    (gx2,) = torch.autograd.grad(y2, rest, gy[:, reset:])
+    for got, want in ((h, h2), (a, a2), (y[:, reset:], y2), (gx[:, reset:], gx2)):
+        assert float((got - want).detach().abs().max()) <= 1e-5 * max(1.0, float(want.detach().abs().max()))
