@@ -1,4 +1,5 @@
-// float32 matrix products on the tensor cores (tcgen05).
+// float32 matrix products on the tensor cores (tcgen05): products with a weight of at most 255 contracted elements, and
+// those of two activations.  (Longer ones with a weight: gemm32_f16.cu.)
 //
 // A float32 number is the exact sum of three bf16 numbers (8 + 8 + 8 mantissa bits: hi + mid + lo), so a product
 // of float32 matrices is a sum of bf16 products accumulated in float32.  The six largest of the nine are kept;
@@ -25,10 +26,10 @@
 // the number of additions, 3.3e-6 of the result's norm after 192), so the five small products go to an accumulator of
 // their own, whose truncations are 2^-8 as large, and the hi*hi accumulator is drained after at most kSegment k and
 // summed in float32 registers from there on.  Errors against float64 are then those of a float32 FMA kernel.
-#include "gemm32.cuh"
-#include "mxk_common.cuh"
+#include <algorithm>
+
+#include "gemm32_common.cuh"
 #include "tma.cuh"
-#include "umma.cuh"
 
 namespace mxk {
 namespace gemm32 {
@@ -73,21 +74,6 @@ struct Layout {
   static constexpr int kAccs = BN == 256 ? 1 : 2;
   static constexpr uint32_t kTmem = kAccs * 2 * BN;
 };
-
-__device__ __forceinline__ void load8(const float* p, int valid, int vec, float* x) {
-  if (valid >= 8 && vec == 8) {
-    asm volatile("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]), "=f"(x[4]), "=f"(x[5]), "=f"(x[6]), "=f"(x[7])
-                 : "l"(p));
-  } else if (valid >= 8 && vec == 4) {
-    const float4 u = __ldg(reinterpret_cast<const float4*>(p)), v = __ldg(reinterpret_cast<const float4*>(p) + 1);
-    x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w;
-    x[4] = v.x; x[5] = v.y; x[6] = v.z; x[7] = v.w;
-  } else {
-#pragma unroll
-    for (int e = 0; e < 8; ++e) x[e] = e < valid ? __ldg(p + e) : 0.f;
-  }
-}
 
 // Two floats to bf16, to the nearest; what lies beyond bf16's largest number, the largest floats and infinity, becomes that
 // number (an infinite plane times a zero one would be NaN).
@@ -173,10 +159,6 @@ struct Tile {
   }
 };
 
-__device__ __forceinline__ void arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* out) {
   uint32_t r[32];
   asm volatile(
@@ -191,21 +173,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* out) {
       : "memory");
 #pragma unroll
   for (int i = 0; i < 32; ++i) out[i] = __uint_as_float(r[i]);
-}
-
-__device__ __forceinline__ void store8(float* p, int valid, int vec, const float* x) {
-  if (valid >= 8 && vec == 8) {
-    asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "f"(x[0]), "f"(x[1]), "f"(x[2]),
-                 "f"(x[3]), "f"(x[4]), "f"(x[5]), "f"(x[6]), "f"(x[7])
-                 : "memory");
-  } else if (valid >= 8 && vec == 4) {
-    reinterpret_cast<float4*>(p)[0] = make_float4(x[0], x[1], x[2], x[3]);
-    reinterpret_cast<float4*>(p)[1] = make_float4(x[4], x[5], x[6], x[7]);
-  } else {
-#pragma unroll
-    for (int e = 0; e < 8; ++e)
-      if (e < valid) p[e] = x[e];
-  }
 }
 
 // Adds to what this thread has stored (or added) there before: fire and forget, and in program order, so the sums are the
@@ -522,12 +489,17 @@ __global__ void __launch_bounds__(256) reduce_splits_kernel(const float* __restr
   c[m * ldc + n] = acc;
 }
 
-int vec_of(const void* p, long long ld) {
-  const uintptr_t a = reinterpret_cast<uintptr_t>(p);
-  if (a % 32 == 0 && ld % 8 == 0) return 8;
-  if (a % 16 == 0 && ld % 4 == 0) return 4;
-  return 1;
+int reduce_splits(const float* partial, int splits, int M, int N, float* c, long long ldc, const Epilogue& ep, cudaStream_t stream) {
+  const long long n_all = static_cast<long long>(M) * N;
+  mxk::launch_kernel(reduce_splits_kernel, static_cast<unsigned>((n_all + 255) / 256), 256, 0, stream, partial, splits, M, N, c, ldc, ep);
+  return launch_status();
 }
+
+// Products with a weight of more than this many k go to gemm32_f16.cu, half the work of the tensor cores: 131 against 184 us at
+// 65536 x 1024 x 256.  Below, three bf16 planes are the more precise form: errors against float64 at K = 64 / 128 / 256 with normal
+// entries 0.7 / 1.2 / 2.3e-7, of two float16 planes 1.35 / 1.4 / 1.4e-7.
+constexpr int kShortK = 255;
+__host__ __device__ constexpr bool two_planes(int K) { return K > kShortK; }
 
 // Width of a tile and how often the contraction is split: a tile of 256 columns halves the shared-memory traffic per
 // product, but only where enough tiles are left to give every SM one; a contraction is split when even the narrowest
@@ -584,9 +556,7 @@ int run(Params& p, float* ws, size_t ws_bytes, int* partials, cudaStream_t strea
                                 : launch<64, kOuter>(p, tiles, stream);
   if (partials) *partials = pl.splits;
   if (st != MXK_OK || pl.splits == 1 || partials) return st;
-  const long long n_all = static_cast<long long>(p.M) * p.N;
-  mxk::launch_kernel(reduce_splits_kernel, static_cast<unsigned>((n_all + 255) / 256), 256, 0, stream, ws, pl.splits, p.M, p.N, p.c, p.ldc, p.ep);
-  return launch_status();
+  return reduce_splits(ws, pl.splits, p.M, p.N, p.c, p.ldc, p.ep, stream);
 }
 
 struct SplitParams {
@@ -611,6 +581,7 @@ __global__ void __launch_bounds__(256) split_weights_kernel(const __grid_constan
     return;
   }
   const WeightJob& jb = sp.job[j];
+  if (two_planes(jb.K)) return f16::split_rows(jb, blockIdx.x - sp.first_block[j]);
   const int bn = jb.bn, kb = (jb.K + kBK - 1) / kBK;
   const long long id = static_cast<long long>(blockIdx.x - sp.first_block[j]) * 256 + threadIdx.x;
   // id = ((n_tile * kb + k_block) * 4 + k_group) * bn + n: consecutive threads write consecutive vectors
@@ -619,22 +590,8 @@ __global__ void __launch_bounds__(256) split_weights_kernel(const __grid_constan
   const int kg = static_cast<int>(rest & 3), k_block = static_cast<int>((rest >> 2) % kb);
   const int n_tile = static_cast<int>((rest >> 2) / kb);
   if (n_tile * bn >= jb.N) return;
-  const int n = n_tile * bn + n_in, k = k_block * kBK + kg * 8;
-  const auto at = [&](int row, int col) -> float {
-    if (jb.w.form == Form::kComplexRows)
-      return jb.w.ptr[row & 1][static_cast<long long>(row >> 1) * jb.w.ld + col] * (jb.w.log_scale ? expf(jb.w.log_scale[row >> 1]) : 1.f);
-    if (jb.w.form == Form::kComplexCols) {
-      const float v = jb.w.ptr[col & 1][static_cast<long long>(row) * jb.w.ld + (col >> 1)];
-      return (col & 1) ? -v : v;
-    }
-    int start = 0, s = 0;
-    for (; s < jb.w.count - 1 && row >= jb.w.row_end[s]; ++s) start = jb.w.row_end[s];
-    return jb.w.ptr[s][static_cast<long long>(row - start) * jb.w.ld + col];
-  };
   float x[8];
-#pragma unroll
-  for (int e = 0; e < 8; ++e)
-    x[e] = (n < jb.N && k + e < jb.K) ? (jb.transposed ? at(k + e, n) : at(n, k + e)) : 0.f;
+  weight_vector(jb, n_tile * bn + n_in, k_block * 4 + kg, x);
   uint4 hi, mid, lo;
   split8(x, hi, mid, lo);
   // a tile of 256 columns is cut into the halves that its two CTAs hold
@@ -647,11 +604,12 @@ __global__ void __launch_bounds__(256) split_weights_kernel(const __grid_constan
 
 }  // namespace
 
-int tile_width(int M, int N, int K) { return plan(M, N, K).bn; }
+int tile_width(int M, int N, int K) { return two_planes(K) ? f16::plan(M, N, K).bn : plan(M, N, K).bn; }
 
 size_t image_bytes(int M, int N, int K) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  const int bn = plan(M, N, K).bn;
+  const int bn = tile_width(M, N, K);
+  if (two_planes(K)) return f16::image_bytes(bn, N, K);
   return static_cast<size_t>((N + bn - 1) / bn) * ((K + kBK - 1) / kBK) * (3 * bn * kBK * 2);
 }
 
@@ -664,7 +622,7 @@ int split_weights(const WeightJob* jobs, int count, const LambdaJob& lambda, cud
     if (!aligned16(jb.image)) return MXK_ERR_ALIGN;
     sp.job[j] = jb;
     const long long vectors = static_cast<long long>((jb.N + jb.bn - 1) / jb.bn) * jb.bn * ((jb.K + kBK - 1) / kBK) * 4;
-    sp.first_block[j + 1] = sp.first_block[j] + static_cast<int>((vectors + 255) / 256);
+    sp.first_block[j + 1] = sp.first_block[j] + (two_planes(jb.K) ? (jb.N + jb.bn - 1) / jb.bn * (jb.bn / f16::kSplitRows) : static_cast<int>((vectors + 255) / 256));
   }
   for (int j = count; j < 4; ++j) sp.first_block[j + 1] = sp.first_block[count];
   const int blocks = sp.first_block[4] + (lambda.N + 255) / 256;
@@ -677,8 +635,9 @@ int split_weights(const WeightJob* jobs, int count, const LambdaJob& lambda, cud
 
 size_t workspace_bytes(int M, int N, int K) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  const Plan pl = plan(M, N, K);
-  return pl.splits > 1 ? static_cast<size_t>(pl.splits) * M * N * sizeof(float) : 0;
+  // (of a weight's product or of two activations')
+  const int splits = std::max(plan(M, N, K).splits, two_planes(K) ? f16::plan(M, N, K).splits : 1);
+  return splits > 1 ? static_cast<size_t>(splits) * M * N * sizeof(float) : 0;
 }
 
 int run_weights(const float* a, long long lda, const void* image, float* c, long long ldc, int M, int N, int K,
@@ -686,6 +645,12 @@ int run_weights(const float* a, long long lda, const void* image, float* c, long
   if (!a || !image || !c) return MXK_ERR_NULL;
   if (M <= 0 || N <= 0 || K <= 0) return MXK_ERR_DIMS;
   if (!aligned16(image)) return MXK_ERR_ALIGN;
+  if (two_planes(K)) {
+    const f16::Plan pl = f16::plan(M, N, K);
+    if (pl.splits > 1 && (!ws || ws_bytes < static_cast<size_t>(pl.splits) * M * N * sizeof(float))) return MXK_ERR_WORKSPACE;
+    const int st = f16::launch_weights(pl, a, lda, image, c, ldc, M, N, K, ep, ws, status, stream);
+    return st != MXK_OK || pl.splits == 1 ? st : reduce_splits(ws, pl.splits, M, N, c, ldc, ep, stream);
+  }
   Params p{};
   p.a = a; p.lda = lda;
   p.image = static_cast<const uint8_t*>(image);

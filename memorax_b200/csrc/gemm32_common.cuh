@@ -1,0 +1,227 @@
+// What the two kernels of float32 products share (gemm32.cu: three bf16 planes, gemm32_f16.cu: two scaled float16 planes).
+#pragma once
+
+#include <cuda_fp16.h>
+
+#include "gemm32.cuh"
+#include "mxk_common.cuh"
+#include "umma.cuh"
+
+namespace mxk {
+namespace gemm32 {
+
+__device__ __forceinline__ void load8(const float* p, int valid, int vec, float* x) {
+  if (valid >= 8 && vec == 8) {
+    asm volatile("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]), "=f"(x[4]), "=f"(x[5]), "=f"(x[6]), "=f"(x[7])
+                 : "l"(p));
+  } else if (valid >= 8 && vec == 4) {
+    const float4 u = __ldg(reinterpret_cast<const float4*>(p)), v = __ldg(reinterpret_cast<const float4*>(p) + 1);
+    x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w;
+    x[4] = v.x; x[5] = v.y; x[6] = v.z; x[7] = v.w;
+  } else {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) x[e] = e < valid ? __ldg(p + e) : 0.f;
+  }
+}
+
+__device__ __forceinline__ void store8(float* p, int valid, int vec, const float* x) {
+  if (valid >= 8 && vec == 8) {
+    asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "f"(x[0]), "f"(x[1]), "f"(x[2]),
+                 "f"(x[3]), "f"(x[4]), "f"(x[5]), "f"(x[6]), "f"(x[7])
+                 : "memory");
+  } else if (valid >= 8 && vec == 4) {
+    reinterpret_cast<float4*>(p)[0] = make_float4(x[0], x[1], x[2], x[3]);
+    reinterpret_cast<float4*>(p)[1] = make_float4(x[4], x[5], x[6], x[7]);
+  } else {
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+      if (e < valid) p[e] = x[e];
+  }
+}
+
+__device__ __forceinline__ void arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(umma::smem_u32(bar)) : "memory");
+}
+
+inline int vec_of(const void* p, long long ld) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+  if (a % 32 == 0 && ld % 8 == 0) return 8;
+  if (a % 16 == 0 && ld % 4 == 0) return 4;
+  return 1;
+}
+
+// Eight elements along k from k = 8 g on of W's row n, zero past the matrix.  (What kind of weight it is, is asked once, so that
+// the eight loads are under way together.)
+__device__ __forceinline__ void weight_vector(const WeightJob& jb, int n, int g, float* x) {
+  const int k = g * 8, valid = n < jb.N ? jb.K - k : 0;
+  const Weight& w = jb.w;
+  const auto loads = [&](const float* p, long long step) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) x[e] = e < valid ? __ldg(p + e * step) : 0.f;
+  };
+  const auto pairs = [&](const float* p0, const float* p1, long long step) {   // even and odd elements
+#pragma unroll
+    for (int e = 0; e < 8; ++e) x[e] = e < valid ? __ldg((e & 1 ? p1 : p0) + (e >> 1) * step) : 0.f;
+  };
+  if (w.form == Form::kComplexRows) {
+    if (!jb.transposed) {
+      loads(w.ptr[n & 1] + static_cast<long long>(n >> 1) * w.ld + k, 1);
+      const float s = w.log_scale && valid > 0 ? expf(__ldg(w.log_scale + (n >> 1))) : 1.f;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) x[e] *= s;
+    } else {
+      const long long at = static_cast<long long>(k >> 1) * w.ld + n;
+      pairs(w.ptr[0] + at, w.ptr[1] + at, w.ld);
+#pragma unroll
+      for (int e = 0; e < 8; e += 2) {
+        const float s = w.log_scale && e < valid ? expf(__ldg(w.log_scale + ((k + e) >> 1))) : 1.f;
+        x[e] *= s;
+        x[e + 1] *= s;
+      }
+    }
+  } else if (w.form == Form::kComplexCols) {
+    if (!jb.transposed) {
+      const long long at = static_cast<long long>(n) * w.ld + (k >> 1);
+      pairs(w.ptr[0] + at, w.ptr[1] + at, 1);
+#pragma unroll
+      for (int e = 1; e < 8; e += 2) x[e] = -x[e];
+    } else {
+      loads(w.ptr[n & 1] + static_cast<long long>(k) * w.ld + (n >> 1), w.ld);
+      if (n & 1) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[e] = -x[e];
+      }
+    }
+  } else {
+    const auto piece = [&](int row, int& start) {
+      int s = 0;
+      start = 0;
+      for (; s < w.count - 1 && row >= w.row_end[s]; ++s) start = w.row_end[s];
+      return s;
+    };
+    int start;
+    if (!jb.transposed) {
+      const int s = piece(n, start);
+      loads(w.ptr[s] + static_cast<long long>(n - start) * w.ld + k, 1);
+    } else {
+      const int s = piece(k, start);
+      if (s == w.count - 1 || k + 7 < w.row_end[s]) {
+        loads(w.ptr[s] + static_cast<long long>(k - start) * w.ld + n, w.ld);
+      } else {
+#pragma unroll 1
+        for (int e = 0; e < 8; ++e) {
+          const int q = piece(k + e, start);
+          const float v = e < valid ? __ldg(w.ptr[q] + static_cast<long long>(k + e - start) * w.ld + n) : 0.f;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) x[i] = i == e ? v : x[i];
+        }
+      }
+    }
+  }
+}
+
+// ---- two float16 planes (gemm32_f16.cu) ----
+namespace f16 {
+
+constexpr int kSplitRows = 4;   // rows of a weight that a block of split_rows splits, with 64 threads each
+constexpr int kBK = 64;
+
+struct Plan {
+  int bn, splits, k_split;
+};
+Plan plan(int M, int N, int K);
+// Planes of an image: two for every tile of `bn` rows and stage of kBK, to the end of the last of each; the exponents of the
+// rows' units follow.
+__host__ __device__ inline size_t planes_bytes(int bn, int N, int K) { return static_cast<size_t>((N + bn - 1) / bn) * ((K + kBK - 1) / kBK) * (2 * bn * kBK * 2); }
+inline size_t image_bytes(int bn, int N, int K) { return planes_bytes(bn, N, K) + static_cast<size_t>((N + bn - 1) / bn) * bn * sizeof(int); }
+// C = A W^T; `partial` (splits x M x N) takes the parts of a split contraction.
+int launch_weights(const Plan& pl, const float* a, long long lda, const void* image, float* c, long long ldc, int M, int N, int K, const Epilogue& ep,
+                   float* partial, int* status, cudaStream_t stream);
+
+constexpr float kLo = 2048.f;     // lo planes are this much larger than what they stand for
+constexpr int kTargetExp = 14;    // the largest element of a row is scaled to [2^14, 2^15)
+
+__device__ __forceinline__ float pow2(int e) { return __uint_as_float(static_cast<uint32_t>(e + 127) << 23); }   // e in [-126, 127]
+// x 2^e for |e| <= 252, rounded once where the result is a normal number
+__device__ __forceinline__ float scale_by(float x, int e) {
+  const int h = e >> 1;
+  return x * pow2(h) * pow2(e - h);
+}
+
+// Exponent of the unit in which a stretch with this largest magnitude is kept: [-126, 113].  (Infinity counts as the largest number.)
+__device__ __forceinline__ int unit_of(float most) {
+  const int e = static_cast<int>(__float_as_uint(most) >> 23);
+  return min(max(e, 1 + kTargetExp), 254) - 127 - kTargetExp;
+}
+__device__ __forceinline__ float scale_of(int unit) { return pow2(-unit); }
+// Two floats to float16, to the nearest; what does not fit, infinity alone, becomes the largest number (an infinite plane times a
+// zero one would be NaN).
+__device__ __forceinline__ uint32_t pack_half(float lo, float hi) {
+  uint32_t v;
+  asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(v) : "f"(hi), "f"(lo));
+  return v;
+}
+
+// hi and lo planes of two scaled floats
+__device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo) {
+  hi = pack_half(a, b);
+  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hi));
+  lo = pack_half((a - f.x) * kLo, (b - f.y) * kLo);
+}
+__device__ __forceinline__ void split8(const float* x, float s, uint4& hi, uint4& lo) {
+  split2(x[0] * s, x[1] * s, hi.x, lo.x);
+  split2(x[2] * s, x[3] * s, hi.y, lo.y);
+  split2(x[4] * s, x[5] * s, hi.z, lo.z);
+  split2(x[6] * s, x[7] * s, hi.w, lo.w);
+}
+
+// Column of a 32-column block in which W's row `n` of the block is placed, so that the eight values that a thread reads from a
+// lane with tmem_ld_16x32 are consecutive columns of C and its stores fill whole lines.
+__device__ __forceinline__ int placed(int n) { return 8 * ((n >> 1) & 3) + 2 * (n >> 3) + (n & 1); }
+
+// A block splits four rows of a weight: 64 threads a row look for its largest element, then each writes the planes of every 64th
+// vector of eight k.  Bound: the latency of its loads, all of them under way together up to 1024 k (1024 x 256: 4.6 us).
+__device__ __forceinline__ void split_rows(const WeightJob& jb, int block) {
+  constexpr int kParts = 256 / kSplitRows, kHeld = 2;
+  __shared__ float most_of[kParts][kSplitRows];
+  const int kb = (jb.K + kBK - 1) / kBK, groups = kb * (kBK / 8);
+  const int row_in = threadIdx.x % kSplitRows, part = threadIdx.x / kSplitRows, n = block * kSplitRows + row_in;
+  float x[kHeld][8], most = 0.f;
+  const auto load = [&](int g0) {
+#pragma unroll
+    for (int i = 0; i < kHeld; ++i) weight_vector(jb, n, g0 + i * kParts, x[i]);   // (zero past the matrix)
+  };
+  for (int g0 = part; g0 < groups; g0 += kHeld * kParts) {
+    load(g0);
+#pragma unroll
+    for (int i = 0; i < kHeld * 8; ++i) most = fmaxf(most, fabsf(x[i >> 3][i & 7]));
+  }
+  most_of[part][row_in] = most;
+  __syncthreads();
+#pragma unroll 8
+  for (int i = 0; i < kParts; ++i) most = fmaxf(most, most_of[i][row_in]);
+  const int unit = unit_of(most);
+  const float scale = scale_of(unit);
+  // a tile of 256 or 128 columns is cut into the halves that its two CTAs hold
+  const int cut = jb.bn == 64 ? 64 : jb.bn / 2, tile_row = n % cut;
+  uint4* const dst = static_cast<uint4*>(jb.image) + static_cast<size_t>(n / cut) * kb * (2 * cut * (kBK / 8)) + (tile_row & ~31) + placed(tile_row & 31);
+  for (int g0 = part; g0 < groups; g0 += kHeld * kParts) {
+    if (groups > kHeld * kParts) load(g0);
+#pragma unroll
+    for (int i = 0; i < kHeld; ++i) {
+      const int g = g0 + i * kParts;
+      if (g >= groups) break;
+      uint4 hi, lo;
+      split8(x[i], scale, hi, lo);
+      uint4* const d = dst + static_cast<size_t>(g / (kBK / 8)) * (2 * cut * (kBK / 8)) + (g % (kBK / 8)) * cut;
+      d[0] = hi;
+      d[cut * (kBK / 8)] = lo;
+    }
+  }
+  if (part == 0) reinterpret_cast<int*>(static_cast<uint8_t*>(jb.image) + planes_bytes(jb.bn, jb.N, jb.K))[n] = unit;
+}
+
+}  // namespace f16
+}  // namespace gemm32
+}  // namespace mxk

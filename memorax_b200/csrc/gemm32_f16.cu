@@ -1,0 +1,615 @@
+// float32 products with a weight on the tensor cores (tcgen05), contractions of 256 elements and more.
+//
+// A float32 number, scaled by a power of two, is the sum of two float16 numbers (hi + lo, 11 + 11 mantissa bits and lo's sign) to
+// within 2^-23 of itself, so a product of float32 matrices is three float16 products, hi*hi + hi*lo + lo*hi, accumulated in
+// float32; lo*lo is below 2^-24 of |a||b|.  (The sum of three bf16 numbers, which needs no scales, takes six: gemm32.cu.)
+//
+// Scales.  A row of the weight is scaled so that its largest element is in [2^14, 2^15).  A row of A takes the scale of its first
+// kBK elements, with room for elements 2^kHeadroom larger; where one later does not fit, the producers begin a new scale at that
+// stage (`event`), the accumulator of the small products is drained and the row's sum brought to the new unit.  lo is kept 2^11
+// times as large: full precision down to 2^-23 of the largest element, and an error of 2^-44 of it below that.
+//
+// Precision: the tensor core truncates when it adds to a float32 accumulator (3e-8 of the sum per addition of 16 k), so the hi*hi
+// accumulator lives for one stage of 64 k, two in contractions from 384 on, and is summed up in float32 registers; the two small
+// products have an accumulator of their own, whose truncations are 2^-11 as large, for the whole tile.  Errors against float64,
+// relative 2-norm (three bf16 planes, drained every 512 k, in brackets; below 256 k they are the more precise form):
+//   4096 x 1024 x 256     normal entries 1.4e-7 (2.3e-7)   lognormal, sigma 3: 1.5e-7 (3.3e-7)
+//   4096 x 256 x 512                     2.1e-7 (4.7e-7)                       1.2e-7 (6.1e-7)
+//   4096 x 256 x 1024                    2.1e-7 (4.7e-7)                       1.4e-7 (4.5e-7)
+//
+// Bound: the tensor pipe at three float16 products per float32 product (1.66 PFLOP/s / 3 = 554 TFLOP/s; 463 with the waves of
+// 65536 x 256 x 1024 and all but the products left out), and C's way to memory.  Beside it shared memory: a stage of 256 columns
+// is 96 KB read by the pipe in 1536 cycles, 64 KB of tiles and 32 KB of planes written and 32 KB of float32 read.
+//
+// One persistent CTA per SM, warp-specialised:
+//   8 warps    epilogue: accumulators (TMEM) -> sums in registers -> global, whole lines
+//   8 warps    producers: float32 tiles, two or three stages ahead in shared memory -> scaled float16 planes
+//   1 warp     issues the MMAs (12 per stage of 64 k), 1 warp the copies of the weight's image, 1 warp those of A (TMA)
+// Registers are dealt out by setmaxnreg: a thread of the epilogue holds up to 128 sums.  (A loaded straight from global memory
+// into the producers' registers: 142 us at 65536 x 256 x 1024, its loads then wait for room in an L1 of 28 KB.)
+// Measured, without the splitting of the weight (three bf16 planes before): 65536 x 1024 x 256 131 us (184), 65536 x 256 x 1024
+// 102 us (173), 24000 x 1024 x 512 90 us (126), 65536 x 128 x 256 29 us (40).
+#include <algorithm>
+
+#include "gemm32_common.cuh"
+#include "tma.cuh"
+
+namespace mxk {
+namespace gemm32 {
+namespace f16 {
+namespace {
+
+using namespace umma;
+
+constexpr int kBM = 128;
+constexpr int kSlots = 8;      // stages whose units and events are kept: more than producers are ahead of the epilogue
+constexpr int kHeadroom = 6;   // powers of two that a row may grow by after its first stage
+constexpr int kLongRuns = 384; // from here on the hi*hi accumulator lives for two stages
+
+struct Params {
+  CUtensorMap map_a;     // kWide: boxes of 128 rows x 32 k
+  const float* a;
+  long long lda;
+  const uint8_t* image;
+  const int* unit_w;     // exponents of the units of W's rows, to the end of the last tile
+  float* c;
+  long long ldc;
+  int M, N, K;
+  int k_split;           // k per split (a multiple of kBK)
+  int splits;            // more than one: c is [splits][M][N]
+  int run;               // stages that the hi*hi accumulator lives for
+  Epilogue ep;           // of a contraction that is not split
+  int* status;
+};
+
+// kPair: two CTAs share a tile of 256 rows (cta_group::2), each with its 128 rows of A and half of the rows of W.
+template <int BN>
+struct Config {
+  static constexpr bool kPair = BN != 64;
+  static constexpr int kTileM = kPair ? 2 * kBM : kBM;
+  static constexpr int kRowsB = kPair ? BN / 2 : BN;   // rows of W in this CTA
+  static constexpr int kPlaneA = kBM * kBK * 2, kPlaneB = kRowsB * kBK * 2;   // bytes
+  static constexpr int kStage = 2 * (kPlaneA + kPlaneB);
+  static constexpr int kStages = kRowsB == 128 ? 2 : 3;
+  static constexpr int kRaw = kBM * kBK * 4, kRaws = kRowsB == 128 ? 3 : 2;   // float32 tiles of A: two halves of 32 k, rows of 128 bytes
+  // accumulators: BN columns for hi*hi and BN for the small products, twice where TMEM has room
+  static constexpr int kSets = BN == 256 ? 1 : 2;
+  static constexpr uint32_t kTmem = kSets * 2 * BN;
+  static constexpr int kRawAt = kStages * kStage;
+  static constexpr int kUnits = kRawAt + kRaws * kRaw;      // int8 [kSlots][128], units of the rows of A
+  static constexpr int kEvents = kUnits + kSlots * 128;     // [kSlots]
+  static constexpr int kBarriers = kEvents + kSlots * 4;
+  static constexpr int kBytes = kBarriers + (3 * kStages + 2 * kRaws + 4 * kSets + 2) * 8;
+  static constexpr int kEpilogueWarps = 8, kProducerWarps = 8;
+  static constexpr int kMmaWarp = kEpilogueWarps + kProducerWarps, kImageWarp = kMmaWarp + 1, kRawWarp = kMmaWarp + 2;
+  static constexpr int kThreads = 32 * (kMmaWarp + 4);   // warpgroups deal registers: 640 threads of 96
+  static constexpr int kRegsEpilogue = BN == 256 ? 168 : 152, kRegsProducer = BN == 256 ? 56 : 64, kRegsMma = BN == 256 ? 32 : 48;
+  static_assert(kEpilogueWarps * kRegsEpilogue + kProducerWarps * kRegsProducer + 4 * kRegsMma == kThreads / 32 * 96, "the launch's registers");
+};
+
+template <int N> __device__ __forceinline__ void more_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void fewer_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+
+// Arrives on the barrier of this offset in the CTA of rank 0: tensor memory has been read (tcgen05 fences order that; a release
+// at cluster scope would wait for every access to global memory under way, 1900 cycles).
+__device__ __forceinline__ void arrive_read(uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, 0;\n\t"
+      "mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [ra];\n\t}\n" ::"r"(smem_u32(bar))
+      : "memory");
+}
+// The same after writes to shared memory that the tensor core is to read.
+__device__ __forceinline__ void arrive_written(uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, 0;\n\t"
+      "mbarrier.arrive.shared::cluster.b64 _, [ra];\n\t}\n" ::"r"(smem_u32(bar))
+      : "memory");
+}
+// Stores to CTA `rank` of the cluster.
+__device__ __forceinline__ void store_at(uint32_t* p, int rank, uint32_t v) {
+  asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, %1;\n\tst.shared::cluster.u32 [ra], %2;\n\t}\n" ::"r"(smem_u32(p)), "r"(rank), "r"(v) : "memory");
+}
+
+// 16 TMEM lanes x 32 columns: r[4 j + 2 h + e] is lane (lane / 4) + 8 h, column 8 j + 2 (lane % 4) + e.
+__device__ __forceinline__ void tmem_ld_16x32(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+// Four floats of shared memory, read here and nowhere else: a plain load may be repeated where its values are used, after the tile
+// has been given back.
+__device__ __forceinline__ void read_once(const void* p, float* x) {
+  asm volatile("ld.volatile.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]) : "r"(smem_u32(p)) : "memory");
+}
+__device__ __forceinline__ void load_box(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y)
+      : "memory");
+}
+
+// kWide: rows of A begin on 16-byte boundaries, those of C on 32-byte ones.  kEp: something is added on the way out.
+// (The instruction cache is small beside this much unrolled code: what is rare is a rolled loop over a copy of the sums in
+// local memory, or another instantiation.)
+template <int BN, bool kWide, bool kEp>
+__global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(const __grid_constant__ Params p) {
+  using L = Config<BN>;
+  constexpr bool kPair = L::kPair;
+  constexpr int kStages = L::kStages, kSets = L::kSets, kTileM = L::kTileM, kRowsB = L::kRowsB;
+  constexpr int kEpilogueWarps = L::kEpilogueWarps, kProducerWarps = L::kProducerWarps, kMmaWarp = L::kMmaWarp;
+  const int mt = (p.M + kTileM - 1) / kTileM, nt = (p.N + BN - 1) / BN;
+  const int tiles = mt * nt * p.splits;
+  const int first_tile = kPair ? blockIdx.x / 2 : blockIdx.x, tile_step = kPair ? gridDim.x / 2 : gridDim.x;
+  enter_kernel(tiles <= tile_step && p.k_split <= 1024);
+  const int rank = kPair ? static_cast<int>(cluster_rank()) : 0;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint64_t* const full = reinterpret_cast<uint64_t*>(smem + L::kBarriers);   // producers and the image's copy -> MMA; rank 1: the copy alone
+  uint64_t* const empty = full + kStages;          // MMA -> producers, copies
+  uint64_t* const peer_full = empty + kStages;     // rank 0: the other CTA's part of the image is there
+  uint64_t* const main_full = peer_full + kStages; // MMA -> epilogue, the hi*hi accumulator
+  uint64_t* const main_empty = main_full + kSets;  // epilogue -> MMA
+  uint64_t* const low_full = main_empty + kSets;   // the same for the small products
+  uint64_t* const low_empty = low_full + kSets;
+  uint64_t* const raw_full = low_empty + kSets;    // copies -> producers, a float32 tile
+  uint64_t* const raw_empty = raw_full + L::kRaws;
+  uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(raw_empty + L::kRaws);
+  int8_t* const units = reinterpret_cast<int8_t*>(smem + L::kUnits);
+  uint32_t* const events = reinterpret_cast<uint32_t*>(smem + L::kEvents);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+
+  if (tid == 0) {
+    for (int s = 0; s < kStages; ++s) { mbar_init(&full[s], (rank == 0 ? kProducerWarps * (kPair ? 2 : 1) : 0) + 1); mbar_init(&empty[s], 1); mbar_init(&peer_full[s], 1); }
+    for (int s = 0; s < kSets; ++s) {
+      mbar_init(&main_full[s], 1); mbar_init(&low_full[s], 1);
+      mbar_init(&main_empty[s], kEpilogueWarps * (kPair ? 2 : 1)); mbar_init(&low_empty[s], kEpilogueWarps * (kPair ? 2 : 1));
+    }
+    for (int s = 0; s < L::kRaws; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], kProducerWarps); }
+    mbar_init_fence();
+  }
+  if (tid < kSlots) events[tid] = 0;
+  if (warp == kMmaWarp) {
+    if (kPair) tmem_alloc_pair(tmem_slot, L::kTmem);
+    else tmem_alloc(tmem_slot, L::kTmem);
+  }
+  fence_before_sync();
+  __syncthreads();
+  if (kPair) cluster_sync();   // the other CTA's barriers are there
+  fence_after_sync();
+  const uint32_t tmem = *tmem_slot;
+  bool timed_out = false;
+  const auto wait = [&](uint64_t* bar, uint32_t parity) { mbar_wait_flag(bar, parity, timed_out); };
+  const auto k_length = [&](int tile) {
+    const int sp = tile / (mt * nt);
+    return min(p.K, (sp + 1) * p.k_split) - sp * p.k_split;
+  };
+  // Whether a row of the tile begins a new unit at this stage; the same in both CTAs.  (Read after a barrier that the producers'
+  // arrivals of the stage lead to; a slot is written again only when its stage has been drained.)
+  const auto event_at = [&](int turn) { return *const_cast<volatile uint32_t*>(events + turn % kSlots) == turn + 1u; };
+
+  if (warp < kEpilogueWarps) {
+    // ------------------------------------------------------------ epilogue
+    more_registers<L::kRegsEpilogue>();
+    constexpr int kChunks = BN / 64;   // of 32 columns
+    const int col0 = (warp >> 2) * (BN / 2), row0 = (warp & 3) * 32 + (lane >> 2);   // this thread: rows row0 + 8 i
+    float sum[kChunks][4][8];          // columns 32 c + 8 (lane % 4) + e
+    int turn = 0, main_turn = 0, low_turn = 0;   // stages, accumulators
+    for (int tile = first_tile; tile < tiles; tile += tile_step) {
+      const int mn = tile % (mt * nt), sp = tile / (mt * nt);
+      const int n0 = (mn % nt) * BN + col0, m0 = (mn / nt) * kTileM + rank * kBM + row0;
+      const int k_len = k_length(tile);
+      int unit[4] = {};   // of the rows' sums: 2^unit
+      int4 unit_w = make_int4(0, 0, 0, 0);   // of four of W's rows a lane, for the end of the tile
+      if (lane < BN / 8) unit_w = __ldg(reinterpret_cast<const int4*>(p.unit_w + n0) + lane);
+#pragma unroll
+      for (int c = 0; c < kChunks; ++c)
+#pragma unroll
+        for (int i = 0; i < 32; ++i) sum[c][i >> 3][i & 7] = 0.f;
+      bool drained = false;   // the small products that an event ended
+#pragma unroll 1
+      for (int seg = 0;;) {   // one accumulator a turn: hi*hi of a run of stages, the small products before an event and at the end
+        const int slot = turn % kSlots;
+        bool low = seg >= k_len;
+        if (!low) {
+          wait(&main_full[main_turn % kSets], (main_turn / kSets) & 1);
+          low = seg > 0 && !drained && event_at(turn);
+        }
+        const int set = (low ? low_turn : main_turn) % kSets;
+        const float f = low ? 1.f / kLo : 1.f;
+        if (low) wait(&low_full[set], (low_turn / kSets) & 1);
+        fence_after_sync();
+        const uint32_t src = tmem + set * 2 * BN + (low ? BN : 0) + col0 + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+#pragma unroll
+        for (int c = 0; c < kChunks; ++c)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {   // rows 16 h + lane / 4, + 8
+            uint32_t r[16];
+            tmem_ld_16x32(src + c * 32 + (static_cast<uint32_t>(16 * h) << 16), r);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                float& x = sum[c][2 * h + (i >> 1)][2 * j + (i & 1)];
+                x = fmaf(__uint_as_float(r[4 * j + i]), f, x);
+              }
+          }
+        fence_before_sync();
+        __syncwarp();
+        if (lane == 0) {
+          uint64_t* const bar = low ? &low_empty[set] : &main_empty[set];
+          if (kPair) arrive_read(bar);
+          else arrive(bar);
+        }
+        if (!low) {
+          if (seg == 0) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) unit[i] = units[slot * 128 + row0 + 8 * i];
+          }
+          ++main_turn;
+          drained = false;
+          // the run's stages: one where an event began it, fewer than p.run where one ended it
+          const int most = seg > 0 && event_at(turn) ? 1 : p.run;
+          int n = 0;
+          do {
+            ++n;
+            seg += kBK;
+            ++turn;
+          } while (n < most && seg < k_len && !event_at(turn));
+          continue;
+        }
+        ++low_turn;
+        if (seg >= k_len) break;
+        drained = true;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int u = units[slot * 128 + row0 + 8 * i];   // no smaller than before
+          const float r = pow2(max(unit[i] - u, -126));
+          unit[i] = u;
+#pragma unroll
+          for (int c = 0; c < kChunks; ++c)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) sum[c][i][e] *= r;
+        }
+      }
+      float* const dst = p.c + (p.splits > 1 ? static_cast<size_t>(sp) * p.M * p.N : 0);
+      // units whose powers are factors that leave room for the sums, and a whole tile
+      bool plain = true;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) plain &= abs(unit[i]) <= 60;
+      plain &= max(max(abs(unit_w.x), abs(unit_w.y)), max(abs(unit_w.z), abs(unit_w.w))) <= 60;
+      if (kWide && __all_sync(0xffffffffu, plain) && m0 - row0 + kBM <= p.M && n0 + BN / 2 <= p.N) {
+        float fr[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) fr[i] = pow2(unit[i]);
+        float* out = dst + m0 * p.ldc + n0 + (lane & 3) * 8;
+#pragma unroll
+        for (int c = 0; c < kChunks; ++c, out += 32) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {   // four columns
+            const int n = n0 + c * 32 + (lane & 3) * 8 + 4 * h;
+            float fc[4], bias[4], scale[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const int mine = e == 0 ? unit_w.x : e == 1 ? unit_w.y : e == 2 ? unit_w.z : unit_w.w;
+              fc[e] = pow2(__shfl_sync(0xffffffffu, mine, c * 8 + (lane & 3) * 2 + h));
+              if (kEp) {
+                bias[e] = p.ep.bias ? __ldg(p.ep.bias + n + e) : 0.f;
+                scale[e] = p.ep.add_scale ? __ldg(p.ep.add_scale + n + e) : 1.f;
+              }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              float* const x = sum[c][i] + 4 * h;
+#pragma unroll
+              for (int e = 0; e < 4; ++e) x[e] = x[e] * fr[i] * fc[e];
+              if (kEp) {
+                const float4 ad = p.ep.add ? __ldg(reinterpret_cast<const float4*>(p.ep.add + (m0 + 8 * i) * p.ep.ld_add + n)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                x[0] = fmaf(ad.x, scale[0], x[0] + bias[0]);
+                x[1] = fmaf(ad.y, scale[1], x[1] + bias[1]);
+                x[2] = fmaf(ad.z, scale[2], x[2] + bias[2]);
+                x[3] = fmaf(ad.w, scale[3], x[3] + bias[3]);
+              }
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) store8(out + 8 * i * p.ldc, 8, 8, sum[c][i]);
+        }
+      } else {
+        float copy[kChunks * 32];
+        int copy_unit[4];
+#pragma unroll
+        for (int i = 0; i < kChunks * 32; ++i) copy[i] = sum[i >> 5][i >> 3 & 3][i & 7];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) copy_unit[i] = unit[i];
+#pragma unroll 1
+        for (int q = 0; q < kChunks * 4; ++q) {   // vectors of eight columns
+          const int i = q & 3, m = m0 + 8 * i, n = n0 + (q >> 2) * 32 + (lane & 3) * 8;
+          const int valid = m < p.M ? p.N - n : 0;
+          float x[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            x[e] = copy[q * 8 + e];
+            if (e >= valid) continue;
+            x[e] = scale_by(x[e], copy_unit[i] + __ldg(p.unit_w + n + e));
+            if (kEp && p.ep.bias) x[e] += __ldg(p.ep.bias + n + e);
+            if (kEp && p.ep.add) x[e] = fmaf(__ldg(p.ep.add + m * p.ep.ld_add + n + e), p.ep.add_scale ? __ldg(p.ep.add_scale + n + e) : 1.f, x[e]);
+          }
+          store8(dst + m * p.ldc + n, valid, kWide ? 8 : 1, x);
+        }
+      }
+    }
+  } else if (warp < kMmaWarp) {
+    // ------------------------------------------------------------ producers
+    fewer_registers<L::kRegsProducer>();
+    // A warp converts 16 rows, in blocks of 8 rows x 32 k; a lane owns 8 consecutive k of a row, eight consecutive lanes eight rows
+    // (no bank conflicts on either side: the float32 tile is swizzled).
+    const int pw = warp - kEpilogueWarps, r0 = pw * 16 + (lane & 7);
+    int stage = 0, raw = 0, turn = 0;
+    uint32_t parity = 1, raw_parity = 0;   // a fresh barrier's previous phase counts as complete
+    int unit[2] = {};             // of this lane's rows
+    for (int tile = first_tile; tile < tiles; tile += tile_step) {
+      const int k_len = k_length(tile);
+#pragma unroll 1
+      for (int seg = 0; seg < k_len; seg += kBK, ++turn) {
+        float x[2][2][8];
+        wait(&raw_full[raw], raw_parity);
+        const uint8_t* const src = smem + L::kRawAt + raw * L::kRaw + r0 * 128;
+#pragma unroll
+        for (int g = 0; g < 2; ++g)
+#pragma unroll
+          for (int b = 0; b < 2; ++b)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              read_once(src + b * (L::kRaw / 2) + g * 1024 + (((lane >> 3) * 2 + h) ^ (lane & 7)) * 16, x[g][b] + 4 * h);
+            }
+        float most[2];
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+          float m[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) m[e] = fmaxf(fabsf(x[g][0][e]), fabsf(x[g][1][e]));
+          most[g] = fmaxf(fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3])), fmaxf(fmaxf(m[4], m[5]), fmaxf(m[6], m[7])));
+          most[g] = fmaxf(most[g], __shfl_xor_sync(0xffffffffu, most[g], 8));
+          most[g] = fmaxf(most[g], __shfl_xor_sync(0xffffffffu, most[g], 16));
+        }
+        // The tile may be overwritten once every lane has its values: the vote takes the maxima, and those take all of them.
+        if (!__any_sync(0xffffffffu, most[0] < 0.f || most[1] < 0.f) && lane == 0) arrive(&raw_empty[raw]);
+        if (++raw == L::kRaws) { raw = 0; raw_parity ^= 1; }
+        const int slot = turn % kSlots;
+        bool event = false;
+        float s[2];
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+          const int u = unit_of(most[g]);
+          if (seg == 0 || u > unit[g]) {
+            event |= seg > 0;
+            unit[g] = u + kHeadroom;
+          }
+          s[g] = scale_of(unit[g]);
+        }
+        wait(&empty[stage], parity);
+        uint8_t* const base = smem + stage * L::kStage + ((lane >> 3) * kBM + r0) * 16;
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+          if (lane < 8) units[slot * 128 + r0 + g * 8] = static_cast<int8_t>(unit[g]);
+#pragma unroll
+          for (int b = 0; b < 2; ++b) {
+            uint4 hi, lo;
+            split8(x[g][b], s[g], hi, lo);
+            uint8_t* const dst = base + (b * 4 * kBM + g * 8) * 16;
+            *reinterpret_cast<uint4*>(dst) = hi;
+            *reinterpret_cast<uint4*>(dst + L::kPlaneA) = lo;
+          }
+        }
+        if (event) {   // before the arrivals that let the MMAs of this stage begin
+          for (int r = 0; r < (kPair ? 2 : 1); ++r) store_at(events + slot, r, turn + 1u);
+          asm volatile("fence.acq_rel.cluster;" ::: "memory");
+        }
+        fence_smem_to_async();
+        __syncwarp();
+        if (lane == 0) {
+          if (kPair) arrive_written(&full[stage]);
+          else arrive(&full[stage]);
+        }
+        if (++stage == kStages) { stage = 0; parity ^= 1; }
+      }
+    }
+  } else {
+    fewer_registers<L::kRegsMma>();   // (a whole warpgroup's)
+    if (warp == kMmaWarp) {
+      // ---------------------------------------------------------- tensor core
+      const bool leader = elect_one();
+      const uint32_t idesc = idesc_f16(kTileM, BN, false, false);
+      int stage = 0, turn = 0, main_turn = 0, low_turn = 0;
+      uint32_t parity = 0;
+      const auto done = [&](uint64_t* bar) {
+        if (leader) (kPair ? commit_pair : commit)(bar);
+      };
+      for (int tile = first_tile; tile < tiles; tile += tile_step) {
+        const int k_len = k_length(tile);
+        bool low_open = false;
+        int run = 0;   // stages in the hi*hi accumulator
+        for (int seg = 0; seg < k_len; seg += kBK, ++turn) {
+          wait(&full[stage], parity);
+          if (kPair && rank != 0) {   // the other CTA issues
+            if (leader) arrive_written(&peer_full[stage]);
+            __syncwarp();
+            if (++stage == kStages) { stage = 0; parity ^= 1; }
+            continue;
+          }
+          if (kPair) wait(&peer_full[stage], parity);
+          const bool event = seg > 0 && event_at(turn);
+          if (event) {
+            if (run > 0) done(&main_full[main_turn++ % kSets]);
+            run = 0;
+            done(&low_full[low_turn % kSets]);
+            ++low_turn;
+            low_open = false;
+          }
+          const uint32_t sa = smem_u32(smem + stage * L::kStage), sb = sa + 2 * L::kPlaneA;
+          const Operand a0{sa, kBM, false}, a1{sa + L::kPlaneA, kBM, false}, b0{sb, kRowsB, false}, b1{sb + L::kPlaneB, kRowsB, false};
+          const int steps = min(kBK, k_len - seg + 15) / 16;   // of 16 k
+          const auto product = [&](uint32_t d, const Operand& a, const Operand& b, bool accumulate) {
+            const uint64_t da = a.desc(0), db = b.desc(0);
+#pragma unroll
+            for (int k = 0; k < kBK / 16; ++k)
+              if (leader && k < steps)
+                (kPair ? mma_bf16_pair : mma_bf16)(d, da + static_cast<uint64_t>(k * a.advance()), db + static_cast<uint64_t>(k * b.advance()), idesc,
+                                                  (accumulate || k > 0) ? 1u : 0u);
+          };
+          const int set = main_turn % kSets;
+          const uint32_t acc = tmem + set * 2 * BN, low = tmem + (low_turn % kSets) * 2 * BN + BN;
+          if (run == 0) wait(&main_empty[set], ((main_turn / kSets) & 1) ^ 1);
+          fence_after_sync();
+          product(acc, a0, b0, run > 0);
+          // (a run that an event begins is one stage: the epilogue learns of the event by its end, and until it has drained the
+          // small products' accumulator the next one cannot be begun)
+          if (++run == p.run || event || seg + kBK >= k_len) {
+            done(&main_full[set]);
+            ++main_turn;
+            run = 0;
+          }
+          if (!low_open) {
+            wait(&low_empty[low_turn % kSets], ((low_turn / kSets) & 1) ^ 1);
+            fence_after_sync();
+          }
+          product(low, a0, b1, low_open);
+          product(low, a1, b0, true);
+          low_open = true;
+          done(&empty[stage]);
+          if (++stage == kStages) { stage = 0; parity ^= 1; }
+        }
+        if (rank == 0) done(&low_full[low_turn % kSets]);
+        ++low_turn;
+      }
+      // the last commits may still be on their way to barriers in this CTA's shared memory
+      for (int s = 0; s < kStages; ++s) {
+        wait(&empty[stage], parity ^ 1);
+        if (++stage == kStages) { stage = 0; parity ^= 1; }
+      }
+    } else if (warp == L::kImageWarp && lane == 0) {
+      // ---------------------------------------------------------- the weight's image
+      const int k_images = (p.K + kBK - 1) / kBK;
+      int stage = 0;
+      uint32_t parity = 1;
+      for (int tile = first_tile; tile < tiles; tile += tile_step) {
+        const int n0 = (tile % nt) * BN + rank * kRowsB, k0 = tile / (mt * nt) * p.k_split, k_len = k_length(tile);
+        const uint8_t* image = p.image + (static_cast<size_t>(n0 / kRowsB) * k_images + k0 / kBK) * (2 * L::kPlaneB);
+        for (int seg = 0; seg < k_len; seg += kBK, image += 2 * L::kPlaneB) {
+          wait(&empty[stage], parity);
+          tma::expect_bytes(&full[stage], 2 * L::kPlaneB);
+          tma::load_bulk(smem + stage * L::kStage + 2 * L::kPlaneA, image, 2 * L::kPlaneB, &full[stage]);
+          if (++stage == kStages) { stage = 0; parity ^= 1; }
+        }
+      }
+    } else if (warp == L::kRawWarp && (!kWide || lane == 0)) {
+      // ---------------------------------------------------------- float32 tiles of A
+      int raw = 0;
+      uint32_t parity = 1;
+      for (int tile = first_tile; tile < tiles; tile += tile_step) {
+        const int m0 = tile % (mt * nt) / nt * kTileM + rank * kBM, k0 = tile / (mt * nt) * p.k_split, k_len = k_length(tile);
+        for (int seg = 0; seg < k_len; seg += kBK) {
+          wait(&raw_empty[raw], parity);
+          uint8_t* const dst = smem + L::kRawAt + raw * L::kRaw;
+          if (kWide) {
+            tma::expect_bytes(&raw_full[raw], L::kRaw);
+            load_box(dst, &p.map_a, &raw_full[raw], k0 + seg, m0);   // zeros past the matrix
+            load_box(dst + L::kRaw / 2, &p.map_a, &raw_full[raw], k0 + seg + 32, m0);
+          } else {
+#pragma unroll 4
+            for (int r = 0; r < kBM; ++r)
+#pragma unroll
+              for (int b = 0; b < 2; ++b) {
+                const int m = m0 + r, k = k0 + seg + b * 32 + lane;
+                const float v = m < p.M && k < p.K ? __ldg(p.a + m * p.lda + k) : 0.f;
+                *reinterpret_cast<float*>(dst + b * (L::kRaw / 2) + r * 128 + ((lane >> 2) ^ (r & 7)) * 16 + (lane & 3) * 4) = v;
+              }
+            __syncwarp();
+            if (lane == 0) arrive(&raw_full[raw]);
+          }
+          if (++raw == L::kRaws) { raw = 0; parity ^= 1; }
+        }
+      }
+    }
+    __syncwarp();
+  }
+
+  if (timed_out && p.status) atomicExch(p.status, 1);
+  fence_before_sync();
+  __syncthreads();
+  if (kPair) cluster_sync();   // nothing reaches into the other CTA any more
+  if (warp == kMmaWarp) {
+    if (kPair) tmem_dealloc_pair(tmem, L::kTmem);
+    else tmem_dealloc(tmem, L::kTmem);
+  }
+}
+
+int tile_m(int bn) { return bn == 64 ? kBM : 2 * kBM; }
+int tile_ctas(int bn) { return bn == 64 ? 1 : 2; }
+
+template <int BN, bool kWide, bool kEp>
+int launch(const Params& p, long long ctas, cudaStream_t stream) {
+  using L = Config<BN>;
+  if (const int st = allow_smem<gemm32_f16_kernel<BN, kWide, kEp>, L::kBytes>(); st != MXK_OK) return st;
+  mxk::launch_kernel_clusters(gemm32_f16_kernel<BN, kWide, kEp>, L::kPair ? 2 : 1, static_cast<unsigned>(std::min(ctas, static_cast<long long>(kNumSMs))),
+                              L::kThreads, L::kBytes, stream, p);
+  return launch_status();
+}
+template <int BN>
+int launch(const Params& p, bool wide, long long ctas, cudaStream_t stream) {
+  if (!wide) return launch<BN, false, true>(p, ctas, stream);
+  return p.ep.bias || p.ep.add ? launch<BN, true, true>(p, ctas, stream) : launch<BN, true, false>(p, ctas, stream);
+}
+
+}  // namespace
+
+// 256 x 256 on a pair of SMs reads the least shared memory per product, 256 x 128 where that leaves SMs without a tile or N is
+// small, 128 x 64 on one SM where that one does, too.  A contraction is split when even the narrowest tiles leave SMs idle and
+// each part still has enough stages to fill the pipeline (four).
+Plan plan(int M, int N, int K) {
+  Plan pl{256, 1, 0};
+  const auto ctas = [&] { return static_cast<long long>((M + tile_m(pl.bn) - 1) / tile_m(pl.bn)) * ((N + pl.bn - 1) / pl.bn) * tile_ctas(pl.bn); };
+  const int kblocks = (K + kBK - 1) / kBK, most = std::max(1, kblocks / 4);
+  if (N <= 64 || M <= 128) pl.bn = 64;
+  else if (N <= 128) pl.bn = 128;
+  // without enough k to split, narrower tiles are the only way to occupy more SMs
+  while (pl.bn > 64 && ctas() * most < kNumSMs) pl.bn /= 2;
+  if (ctas() < kNumSMs && most > 1) pl.splits = static_cast<int>(std::min(static_cast<long long>(most), kNumSMs / ctas()));
+  const int per = (kblocks + pl.splits - 1) / pl.splits;
+  pl.k_split = per * kBK;
+  pl.splits = (kblocks + per - 1) / per;
+  return pl;
+}
+
+int launch_weights(const Plan& pl, const float* a, long long lda, const void* image, float* c, long long ldc, int M, int N, int K, const Epilogue& ep,
+                   float* partial, int* status, cudaStream_t stream) {
+  Params p{};
+  p.a = a; p.lda = lda;
+  p.image = static_cast<const uint8_t*>(image);
+  p.unit_w = reinterpret_cast<const int*>(p.image + planes_bytes(pl.bn, N, K));
+  p.c = pl.splits > 1 ? partial : c;
+  p.ldc = pl.splits > 1 ? N : ldc;
+  p.M = M; p.N = N; p.K = K;
+  p.k_split = pl.k_split; p.splits = pl.splits;
+  p.run = K < kLongRuns ? 1 : 2;
+  if (pl.splits == 1) p.ep = ep;
+  p.status = status;
+  const bool wide = vec_of(a, lda) >= 4 && vec_of(p.c, p.ldc) == 8 && (!p.ep.add || vec_of(p.ep.add, p.ep.ld_add) >= 4);
+  if (wide) {
+    tma::EncodeTiledFn enc = tma::encode_tiled_fn();
+    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(K), static_cast<cuuint64_t>(M)}, strides[1] = {static_cast<cuuint64_t>(lda) * 4};
+    const cuuint32_t box[2] = {32, kBM}, elem[2] = {1, 1};
+    if (!enc || enc(&p.map_a, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(a), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+      return MXK_ERR_UNSUPPORTED;
+  }
+  const long long ctas = static_cast<long long>((M + tile_m(pl.bn) - 1) / tile_m(pl.bn)) * ((N + pl.bn - 1) / pl.bn) * pl.splits * tile_ctas(pl.bn);
+  return pl.bn == 256 ? launch<256>(p, wide, ctas, stream) : pl.bn == 128 ? launch<128>(p, wide, ctas, stream) : launch<64>(p, wide, ctas, stream);
+}
+
+}  // namespace f16
+}  // namespace gemm32
+}  // namespace mxk

@@ -1,0 +1,92 @@
+"""float32 products of long contractions with a weight: scaled float16 planes, units that change along a row."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+# Elementwise, relative to sum |a||b|: two operands to 2^-23 each and the product of their small parts, 2^-24; eight truncating
+# additions of at most 2^-23 to each accumulator, and the float32 sums of the accumulators, 2^-24 each for K / 128 of them.
+# Elements far below the largest of their row are kept to 2^-44 of that (A, with its room to grow; W: 2^-50): a row's largest
+# element may meet an almost vanishing weight.
+BOUND, FLOOR_A, FLOOR_W = 2.0 ** -20 + 2.0 ** -21, 2.0 ** -44, 2.0 ** -50
+
+
+def product(x, w, b=None):
+    from memorax_b200 import _C, ops
+    got = _C.linear_f32(x, w, b)
+    ops.check_status()
+    return got
+
+
+# tiles of 256 and 128 columns on pairs and of 64 on one SM, their edges, stages of 64 k and runs of two, split contractions,
+# rows that start anywhere
+@pytest.mark.parametrize("m,n,k", [(1, 1, 256), (127, 64, 257), (129, 130, 320), (300, 776, 513), (9000, 256, 264), (20000, 128, 384),
+                                   (20001, 520, 300), (4097, 300, 1100)])
+@pytest.mark.parametrize("kind", ["plain", "grows", "leaps", "wide range", "zeros first"])
+def test_products_stay_within_the_bound_of_their_terms(m, n, k, kind):
+    g = torch.Generator("cuda").manual_seed(m + n + k)
+    x, w, b = (torch.randn(*s, generator=g, device="cuda") for s in ((m, k), (n, k), (n,)))
+    at = torch.arange(k, device="cuda")
+    if kind == "grows":         # every stage takes a new unit in some row, in steps of 2^9, over the range of float32
+        x *= 2.0 ** (9.0 * (at // 64) * (torch.arange(m, device="cuda")[:, None] % 3) - 60).clamp(max=40)
+    elif kind == "leaps":       # one element far above its row, at any place
+        x[torch.arange(m, device="cuda"), torch.randint(k, (m,), generator=g, device="cuda")] *= 2.0 ** 40
+    elif kind == "wide range":  # rows and columns of very different sizes
+        x *= 2.0 ** torch.randint(-60, 61, (m, 1), generator=g, device="cuda")
+        w *= 2.0 ** torch.randint(-60, 61, (n, 1), generator=g, device="cuda")
+    elif kind == "zeros first":
+        x[:, :130] = 0
+        x[::3] = 0
+    got = product(x, w, b).double()
+    want, scale = x.double() @ w.double().t() + b.double(), x.abs().double() @ w.abs().double().t() + b.abs().double()
+    bound = BOUND * scale + FLOOR_A * x.abs().amax(1, keepdim=True).double() * w.abs().double().sum(1)
+    bound += FLOOR_W * x.abs().double().sum(1, keepdim=True) * w.abs().amax(1).double()
+    assert bool(((got - want).abs() <= bound).all()), float(((got - want).abs() / bound.clamp(min=1e-300)).max())
+
+
+def test_a_broken_row_stays_alone():
+    torch.manual_seed(0)
+    x, w = torch.randn(300, 512, device="cuda"), torch.randn(260, 512, device="cuda") / 512
+    want = product(x, w)
+    x[7, 300], x[9, 3], w[11, 5] = float("nan"), float("inf"), float("nan")
+    got = product(x, w)
+    assert bool(got[7].isnan().all()) and bool(got[:, 11].isnan().all())
+    keep_r, keep_c = [i for i in range(300) if i not in (7, 9)], [i for i in range(260) if i != 11]
+    assert torch.equal(got[keep_r][:, keep_c], want[keep_r][:, keep_c])
+    assert not got[9][keep_c].isnan().any() and bool((got[9].sign() == w[:, 3].sign())[keep_c].all()) and float(got[9][keep_c].abs().min()) > 1e30
+
+
+# the weights of the layers: complex pairs along rows and along columns, stacked ones whose pieces end inside a vector, each also
+# transposed (the gradients of the inputs); against the same layers in float64
+@pytest.mark.parametrize("cell", ["lru", "mingru"])
+@pytest.mark.parametrize("feat,width", [(256, 128), (261, 131), (520, 300)])
+def test_layers_with_long_contractions(cell, feat, width):
+    from memorax_b200.memoroid import LRUCell, Memoroid, MinGRUCell
+    torch.manual_seed(feat)
+    bsz, steps = 3, 50
+    made = (LRUCell(feat, width, r_min=0.5, r_max=0.9, max_phase=0.6) if cell == "lru" else MinGRUCell(width, in_features=feat)).cuda()
+    x = torch.randn(bsz, steps, feat, device="cuda", requires_grad=True)
+    gy = torch.randn(bsz, steps, feat if cell == "lru" else width, device="cuda")
+    _, y = Memoroid(made)(x, torch.zeros(bsz, steps, device="cuda"), None)
+    wrt = [x, *made.parameters()]
+    grads = torch.autograd.grad(y, wrt, gy)
+    xd, p = x.detach().double().requires_grad_(), {n: v.detach().double().requires_grad_() for n, v in made.named_parameters()}
+    if cell == "lru":
+        lam = torch.exp(torch.complex(-torch.exp(p["nu_log"]), torch.exp(p["theta_log"])))
+        bu = xd.to(torch.complex128) @ (torch.complex(p["B_real"], p["B_imag"]) * torch.exp(p["gamma_log"])[:, None]).t()
+        h, out = torch.zeros_like(bu[:, 0]), []
+        for t in range(steps):
+            h = lam * h + bu[:, t]
+            out.append(h)
+        want_y = (torch.stack(out, 1) @ torch.complex(p["C_real"], p["C_imag"]).t()).real + p["D"] * xd
+    else:
+        z, ht = xd @ p["z.weight"].t(), xd @ p["h.weight"].t()
+        g = torch.where(ht >= 0, torch.relu(ht) + 0.5, torch.sigmoid(ht))
+        h, out = torch.zeros_like(z[:, 0]), []
+        for t in range(steps):
+            h = torch.sigmoid(-z[:, t]) * h + torch.sigmoid(z[:, t]) * g[:, t]
+            out.append(h)
+        want_y = torch.stack(out, 1)
+    want = torch.autograd.grad(want_y, [xd, *p.values()], gy.double())
+    for name, a, b in zip(["y", "x", *p], [y, *grads], [want_y, *want]):
+        assert float((a.detach().double() - b).norm() / b.norm()) <= 2e-6, name
