@@ -1,5 +1,5 @@
-// float32 matrix products on the tensor cores (tcgen05): products with a weight of at most 255 contracted elements, and
-// those of two activations.  (Longer ones with a weight: gemm32_f16.cu.)
+// float32 matrix products on the tensor cores (tcgen05): contractions of at most 255 elements, and the host side of all of them.
+// (Longer ones: gemm32_f16.cu, gemm32_f16_outer.cu.)
 //
 // A float32 number is the exact sum of three bf16 numbers (8 + 8 + 8 mantissa bits: hi + mid + lo), so a product
 // of float32 matrices is a sum of bf16 products accumulated in float32.  The six largest of the nine are kept;
@@ -14,18 +14,14 @@
 //   producers  global float32 -> registers (a stage ahead) -> three bf16 planes in shared memory
 //   1 warp     issues the MMAs (12 per stage of 32 k)
 // Eight warps each for the first two; where one CTA converts both operands alone, 12 producers and 4 epilogue warps.
-// Measured: 24000 x 1024 x 512 at 198 TFLOP/s, its weight gradient at 178 (167 when a pair had 16 producers and 4 epilogue
-// warps: the drains of long sums then held the pipe up).
 // Weights are split once, by split_weights, into images of the shared-memory stage, which arrive by one bulk copy per
-// stage: with both operands converted here the producers bound the kernel (127 TFLOP/s at 65536 x 1024 x 256).  A
-// gradient of a weight contracts two activations and converts both.
+// stage.  A gradient of a weight contracts two activations and converts both.
 // Operand planes are in the panel format of umma.cuh, which serves contraction over columns and over rows alike, so
 // nothing is transposed.
 //
 // Precision: the tensor core truncates when it adds to a float32 accumulator (measured: the error grows linearly with
 // the number of additions, 3.3e-6 of the result's norm after 192), so the five small products go to an accumulator of
-// their own, whose truncations are 2^-8 as large, and the hi*hi accumulator is drained after at most kSegment k and
-// summed in float32 registers from there on.  Errors against float64 are then those of a float32 FMA kernel.
+// their own, whose truncations are 2^-8 as large.  Errors against float64 are then those of a float32 FMA kernel.
 #include <algorithm>
 
 #include "gemm32_common.cuh"
@@ -38,7 +34,6 @@ namespace {
 using namespace umma;
 
 constexpr int kBM = 128, kBK = 32;
-constexpr int kSegment = 512;   // k between two drains of the accumulators
 
 struct Params {
   const float* a;
@@ -51,9 +46,6 @@ struct Params {
   long long ldc;
   int c_vec;
   int M, N, K;
-  int k_split;           // k per split (a multiple of kBK)
-  int splits;
-  float* partial;        // [splits][M][N] when splits > 1
   Epilogue ep;
   int ep_vec;
   int* status;
@@ -175,21 +167,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* out) {
   for (int i = 0; i < 32; ++i) out[i] = __uint_as_float(r[i]);
 }
 
-// Adds to what this thread has stored (or added) there before: fire and forget, and in program order, so the sums are the
-// same every time.  (A load, an addition and a store cost 26 k cycles per drained 128 x 256 tile.)
-__device__ __forceinline__ void add8(float* p, int valid, int vec, const float* x) {
-  if (valid >= 8 && vec >= 4) {
-#pragma unroll
-    for (int h = 0; h < 8; h += 4)
-      asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1,%2,%3,%4};" ::"l"(p + h), "f"(x[h]), "f"(x[h + 1]), "f"(x[h + 2]), "f"(x[h + 3])
-                   : "memory");
-  } else {
-#pragma unroll
-    for (int e = 0; e < 8; ++e)
-      if (e < valid) asm volatile("red.relaxed.gpu.global.add.f32 [%0], %1;" ::"l"(p + e), "f"(x[e]) : "memory");
-  }
-}
-
 // v: 32 consecutive columns of row `lane`.  Afterwards v[8 j ..] are columns 8 (lane & 3) .. + 7 of row (lane & 28) + j, so
 // that a store instruction writes whole 128-byte lines: with a row per lane it touched 32 lines for 32 bytes each, and a
 // 128 x 256 accumulator took 7.9 k cycles to drain instead of the 5 k that its bytes need.
@@ -226,9 +203,9 @@ __global__ void __launch_bounds__(Roles<BN, kOuter>::kThreads, 1) gemm32_kernel(
   constexpr bool kPair = L::kPair;
   constexpr int kTileM = kPair ? 2 * kBM : kBM;
   const int mt = (p.M + kTileM - 1) / kTileM, nt = (p.N + BN - 1) / BN;
-  const int tiles = mt * nt * p.splits;
+  const int tiles = mt * nt;
   const int first_tile = kPair ? blockIdx.x / 2 : blockIdx.x, tile_step = kPair ? gridDim.x / 2 : gridDim.x;
-  enter_kernel(tiles <= tile_step && p.k_split <= 2 * kSegment);
+  enter_kernel(tiles <= tile_step);
   const int rank = kPair ? static_cast<int>(cluster_rank()) : 0;
   using R = Roles<BN, kOuter>;
   constexpr int kProducerWarps = R::kProducerWarps, kEpilogueWarps = R::kEpilogueWarps, kMmaWarp = R::kMmaWarp;
@@ -275,14 +252,13 @@ __global__ void __launch_bounds__(Roles<BN, kOuter>::kThreads, 1) gemm32_kernel(
     uint32_t parity = 1;   // a fresh barrier's previous phase counts as complete
     TileA ta;
     TileB tb;
-    int m0 = 0, n0 = 0, k0 = 0, k_end = 0;
+    const int k_end = p.K;
+    int m0 = 0, n0 = 0, k0 = 0;
     bool a_inner = false, b_inner = false;
     auto tile_begin = [&](int t) {
-      const int mn = t % (mt * nt), sp = t / (mt * nt);
-      n0 = (mn % nt) * BN + rank * L::kRowsB;   // of this CTA's part of B
-      m0 = (mn / nt) * kTileM + rank * kBM;
-      k0 = sp * p.k_split;
-      k_end = min(p.K, k0 + p.k_split);
+      n0 = (t % nt) * BN + rank * L::kRowsB;   // of this CTA's part of B
+      m0 = (t / nt) * kTileM + rank * kBM;
+      k0 = 0;
       ta.begin(p.a, p.lda, pw, lane, m0, k0);
       if (kOuter) tb.begin(p.b, p.ldb, pw, lane, n0, k0);
     };
@@ -344,44 +320,40 @@ __global__ void __launch_bounds__(Roles<BN, kOuter>::kThreads, 1) gemm32_kernel(
     int stage = 0;
     uint32_t parity = 0;
     int turn = 0;
-    for (int tile = first_tile; tile < tiles; tile += tile_step) {
-      const int sp = tile / (mt * nt);
-      const int k_len = min(p.K, (sp + 1) * p.k_split) - sp * p.k_split;
-      for (int seg = 0; seg < k_len; seg += kSegment, ++turn) {
-        const int blocks = (min(k_len - seg, kSegment) + kBK - 1) / kBK;
-        const int buf = turn % L::kAccs;
-        if (rank == 0) wait(&acc_empty[buf], ((turn / L::kAccs) & 1) ^ 1, timed_out);
-        fence_after_sync();
-        const uint32_t acc = tmem + buf * 2 * BN, acc_small = acc + BN;
-        for (int kb = 0; kb < blocks; ++kb) {
-          wait(&full[stage], parity, timed_out);
-          if (kPair && rank != 0) {   // this CTA's stage is full: the other one issues
-            if (leader) arrive_at_leader(&peer_full[stage]);
-            __syncwarp();
-            if (++stage == kStages) { stage = 0; parity ^= 1; }
-            continue;
-          }
-          if (kPair) wait(&peer_full[stage], parity, timed_out);
-          fence_after_sync();
-          const uint32_t sa = smem_u32(smem + stage * L::kStage), sb = sa + 3 * L::kPlaneA;
-          constexpr uint32_t kRowsA = kOuter ? kBK : kBM, kRowsB = kOuter ? kBK : L::kRowsB;
-          const Operand a0{sa, kRowsA, kOuter}, a1{sa + L::kPlaneA, kRowsA, kOuter}, a2{sa + 2 * L::kPlaneA, kRowsA, kOuter};
-          const Operand b0{sb, kRowsB, kOuter}, b1{sb + L::kPlaneB, kRowsB, kOuter}, b2{sb + 2 * L::kPlaneB, kRowsB, kOuter};
-          const auto product = [&](uint32_t d, const Operand& a, const Operand& b, bool accumulate) {
-            if (kPair) gemm_pair<kBK / 16>(d, a, b, idesc, accumulate, leader);
-            else gemm<kBK / 16>(d, a, b, idesc, accumulate, leader);
-          };
-          product(acc_small, a2, b0, kb > 0);
-          product(acc_small, a0, b2, true);
-          product(acc_small, a1, b1, true);
-          product(acc_small, a1, b0, true);
-          product(acc_small, a0, b1, true);
-          product(acc, a0, b0, kb > 0);
-          if (leader) (kPair ? commit_pair : commit)(&empty[stage]);
+    for (int tile = first_tile; tile < tiles; tile += tile_step, ++turn) {
+      const int blocks = (p.K + kBK - 1) / kBK;
+      const int buf = turn % L::kAccs;
+      if (rank == 0) wait(&acc_empty[buf], ((turn / L::kAccs) & 1) ^ 1, timed_out);
+      fence_after_sync();
+      const uint32_t acc = tmem + buf * 2 * BN, acc_small = acc + BN;
+      for (int kb = 0; kb < blocks; ++kb) {
+        wait(&full[stage], parity, timed_out);
+        if (kPair && rank != 0) {   // this CTA's stage is full: the other one issues
+          if (leader) arrive_at_leader(&peer_full[stage]);
+          __syncwarp();
           if (++stage == kStages) { stage = 0; parity ^= 1; }
+          continue;
         }
-        if (leader && rank == 0) (kPair ? commit_pair : commit)(&acc_full[buf]);
+        if (kPair) wait(&peer_full[stage], parity, timed_out);
+        fence_after_sync();
+        const uint32_t sa = smem_u32(smem + stage * L::kStage), sb = sa + 3 * L::kPlaneA;
+        constexpr uint32_t kRowsA = kOuter ? kBK : kBM, kRowsB = kOuter ? kBK : L::kRowsB;
+        const Operand a0{sa, kRowsA, kOuter}, a1{sa + L::kPlaneA, kRowsA, kOuter}, a2{sa + 2 * L::kPlaneA, kRowsA, kOuter};
+        const Operand b0{sb, kRowsB, kOuter}, b1{sb + L::kPlaneB, kRowsB, kOuter}, b2{sb + 2 * L::kPlaneB, kRowsB, kOuter};
+        const auto product = [&](uint32_t d, const Operand& a, const Operand& b, bool accumulate) {
+          if (kPair) gemm_pair<kBK / 16>(d, a, b, idesc, accumulate, leader);
+          else gemm<kBK / 16>(d, a, b, idesc, accumulate, leader);
+        };
+        product(acc_small, a2, b0, kb > 0);
+        product(acc_small, a0, b2, true);
+        product(acc_small, a1, b1, true);
+        product(acc_small, a1, b0, true);
+        product(acc_small, a0, b1, true);
+        product(acc, a0, b0, kb > 0);
+        if (leader) (kPair ? commit_pair : commit)(&empty[stage]);
+        if (++stage == kStages) { stage = 0; parity ^= 1; }
       }
+      if (leader && rank == 0) (kPair ? commit_pair : commit)(&acc_full[buf]);
     }
     // the last commits may still be on their way to barriers in this CTA's shared memory
     for (int s = 0; s < kStages; ++s) {
@@ -391,67 +363,56 @@ __global__ void __launch_bounds__(Roles<BN, kOuter>::kThreads, 1) gemm32_kernel(
   } else if (warp < kEpilogueWarps) {
     // ------------------------------------------------------------ epilogue
     int turn = 0;
-    for (int tile = first_tile; tile < tiles; tile += tile_step) {
-      const int mn = tile % (mt * nt), sp = tile / (mt * nt);
-      const int n0 = (mn % nt) * BN, m0 = (mn / nt) * kTileM + rank * kBM;
+    for (int tile = first_tile; tile < tiles; tile += tile_step, ++turn) {
+      const int n0 = (tile % nt) * BN, m0 = (tile / nt) * kTileM + rank * kBM;
       const int m = m0 + (warp & 3) * 32 + (lane & 28);   // first of the four rows this lane stores, see to_lines()
-      const bool split = p.splits > 1;
-      float* const c0 = split ? p.partial + static_cast<size_t>(sp) * p.M * p.N : p.c;
-      const long long ldc = split ? p.N : p.ldc;
-      const int k_len = min(p.K, (sp + 1) * p.k_split) - sp * p.k_split;
-      for (int seg = 0; seg < k_len; seg += kSegment, ++turn) {
-        const int buf = turn % L::kAccs;
-        const bool last = seg + kSegment >= k_len;
-        wait(&acc_full[buf], (turn / L::kAccs) & 1, timed_out);
-        fence_after_sync();
-        const uint32_t src = tmem + buf * 2 * BN + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+      const int buf = turn % L::kAccs;
+      wait(&acc_full[buf], (turn / L::kAccs) & 1, timed_out);
+      fence_after_sync();
+      const uint32_t src = tmem + buf * 2 * BN + (static_cast<uint32_t>((warp & 3) * 32) << 16);
 #pragma unroll 1
-        for (int c = (warp >> 2) * (BN / kColumnParts); c < ((warp >> 2) + 1) * (BN / kColumnParts); c += 32) {
-          if (n0 + c >= p.N) break;
-          float v[32];
-          __syncwarp();
-          tmem_ld32(src + c, v);
-#pragma unroll
-          for (int h = 0; h < 32; h += 16) {
-            float w[16];
-            tmem_ld8(src + BN + c + h, w);
-            tmem_ld8(src + BN + c + h + 8, w + 8);
-            tmem_ld_wait();
-#pragma unroll
-            for (int e = 0; e < 16; ++e) v[h + e] += w[e];
-          }
-          to_lines(v, lane);
-          const int n = n0 + c + (lane & 3) * 8;
-          float* dst = c0 + m * ldc + n;
-#pragma unroll
-          for (int j = 0; j < 4; ++j, dst += ldc) {
-            const int valid = m + j < p.M ? p.N - n : 0;
-            if (valid <= 0) continue;
-            float* const x = v + j * 8;
-            if (last && !split) {
-              if (p.ep.bias) {
-#pragma unroll
-                for (int e = 0; e < 8; ++e)
-                  if (e < valid) x[e] += __ldg(p.ep.bias + n + e);
-              }
-              if (p.ep.add) {
-                float ad[8];
-                load8(p.ep.add + (m + j) * p.ep.ld_add + n, valid, p.ep_vec, ad);
-#pragma unroll
-                for (int e = 0; e < 8; ++e)
-                  x[e] = fmaf(ad[e], (p.ep.add_scale && e < valid) ? __ldg(p.ep.add_scale + n + e) : 1.f, x[e]);
-              }
-            }
-            if (seg > 0) add8(dst, valid, p.c_vec, x);   // to this thread's own earlier segments
-            else store8(dst, valid, p.c_vec, x);
-          }
-        }
-        fence_before_sync();
+      for (int c = (warp >> 2) * (BN / kColumnParts); c < ((warp >> 2) + 1) * (BN / kColumnParts); c += 32) {
+        if (n0 + c >= p.N) break;
+        float v[32];
         __syncwarp();
-        if (lane == 0) {
-          if (kPair) arrive_at_leader(&acc_empty[buf]);
-          else arrive(&acc_empty[buf]);
+        tmem_ld32(src + c, v);
+#pragma unroll
+        for (int h = 0; h < 32; h += 16) {
+          float w[16];
+          tmem_ld8(src + BN + c + h, w);
+          tmem_ld8(src + BN + c + h + 8, w + 8);
+          tmem_ld_wait();
+#pragma unroll
+          for (int e = 0; e < 16; ++e) v[h + e] += w[e];
         }
+        to_lines(v, lane);
+        const int n = n0 + c + (lane & 3) * 8;
+        float* dst = p.c + m * p.ldc + n;
+#pragma unroll
+        for (int j = 0; j < 4; ++j, dst += p.ldc) {
+          const int valid = m + j < p.M ? p.N - n : 0;
+          if (valid <= 0) continue;
+          float* const x = v + j * 8;
+          if (p.ep.bias) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+              if (e < valid) x[e] += __ldg(p.ep.bias + n + e);
+          }
+          if (p.ep.add) {
+            float ad[8];
+            load8(p.ep.add + (m + j) * p.ep.ld_add + n, valid, p.ep_vec, ad);
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+              x[e] = fmaf(ad[e], (p.ep.add_scale && e < valid) ? __ldg(p.ep.add_scale + n + e) : 1.f, x[e]);
+          }
+          store8(dst, valid, p.c_vec, x);
+        }
+      }
+      fence_before_sync();
+      __syncwarp();
+      if (lane == 0) {
+        if (kPair) arrive_at_leader(&acc_empty[buf]);
+        else arrive(&acc_empty[buf]);
       }
     }
   }
@@ -501,33 +462,16 @@ int reduce_splits(const float* partial, int splits, int M, int N, float* c, long
 constexpr int kShortK = 255;
 __host__ __device__ constexpr bool two_planes(int K) { return K > kShortK; }
 
-// Width of a tile and how often the contraction is split: a tile of 256 columns halves the shared-memory traffic per
-// product, but only where enough tiles are left to give every SM one; a contraction is split when even the narrowest
-// tiles leave SMs idle and each part still has enough steps to fill the pipeline (8 stages of 32).
-struct Plan {
-  int bn, splits, k_split;
-};
-Plan plan(int M, int N, int K) {
-  Plan pl{256, 1, 0};
+// Width of a tile: 256 columns halve the shared-memory traffic per product, but only where enough tiles are left to give every SM
+// one.  Narrower tiles are the only way to occupy more SMs.
+int tile_columns(int M, int N) {
   const auto tiles = [&](int bn) {   // CTAs that one pass over C occupies
     const int tm = bn == 256 ? 2 * kBM : kBM;
     return static_cast<long long>((M + tm - 1) / tm) * ((N + bn - 1) / bn) * (tm / kBM);
   };
-  const int kblocks = (K + kBK - 1) / kBK;
-  if (N <= 64) pl.bn = 64;
-  else if (N <= 128 || M <= 128) pl.bn = 128;
-  int max_splits = max(1, kblocks / 8);
-  // without enough k to split, narrower tiles are the only way to occupy more SMs
-  while (pl.bn > 64 && tiles(pl.bn) * max_splits < kNumSMs) pl.bn /= 2;
-  const long long t = tiles(pl.bn);
-  if (t < kNumSMs && max_splits > 1) {
-    pl.splits = static_cast<int>(min(static_cast<long long>(max_splits), kNumSMs / t));
-    if (pl.splits < 1) pl.splits = 1;
-  }
-  const int per = (kblocks + pl.splits - 1) / pl.splits;
-  pl.k_split = per * kBK;
-  pl.splits = (kblocks + per - 1) / per;
-  return pl;
+  int bn = N <= 64 ? 64 : N <= 128 || M <= 128 ? 128 : 256;
+  while (bn > 64 && tiles(bn) < kNumSMs) bn /= 2;
+  return bn;
 }
 
 template <int BN, bool kOuter>
@@ -539,24 +483,14 @@ int launch(const Params& p, int tiles, cudaStream_t stream) {
 }
 
 template <bool kOuter>
-int run(Params& p, float* ws, size_t ws_bytes, int* partials, cudaStream_t stream) {
-  const Plan pl = plan(p.M, p.N, p.K);
-  if (pl.splits > 1 && (!ws || ws_bytes < static_cast<size_t>(pl.splits) * p.M * p.N * sizeof(float))) return MXK_ERR_WORKSPACE;
-  p.k_split = pl.k_split;
-  p.splits = pl.splits;
-  p.partial = ws;
-  p.c_vec = pl.splits > 1 ? vec_of(ws, p.N) : vec_of(p.c, p.ldc);
+int run(Params& p, cudaStream_t stream) {
+  const int bn = tile_columns(p.M, p.N), tm = bn == 256 ? 2 * kBM : kBM;
+  p.c_vec = vec_of(p.c, p.ldc);
   p.ep_vec = p.ep.add ? vec_of(p.ep.add, p.ep.ld_add) : 1;
   p.a_wide = vec_of(p.a, p.lda) == 8;
   p.b_wide = kOuter && vec_of(p.b, p.ldb) == 8;
-  const int tm = pl.bn == 256 ? 2 * kBM : kBM;
-  const int tiles = ((p.M + tm - 1) / tm) * ((p.N + pl.bn - 1) / pl.bn) * pl.splits * (tm / kBM);   // in CTAs
-  const int st = pl.bn == 256   ? launch<256, kOuter>(p, tiles, stream)
-                 : pl.bn == 128 ? launch<128, kOuter>(p, tiles, stream)
-                                : launch<64, kOuter>(p, tiles, stream);
-  if (partials) *partials = pl.splits;
-  if (st != MXK_OK || pl.splits == 1 || partials) return st;
-  return reduce_splits(ws, pl.splits, p.M, p.N, p.c, p.ldc, p.ep, stream);
+  const int tiles = ((p.M + tm - 1) / tm) * ((p.N + bn - 1) / bn) * (tm / kBM);   // in CTAs
+  return bn == 256 ? launch<256, kOuter>(p, tiles, stream) : bn == 128 ? launch<128, kOuter>(p, tiles, stream) : launch<64, kOuter>(p, tiles, stream);
 }
 
 struct SplitParams {
@@ -604,7 +538,7 @@ __global__ void __launch_bounds__(256) split_weights_kernel(const __grid_constan
 
 }  // namespace
 
-int tile_width(int M, int N, int K) { return two_planes(K) ? f16::plan(M, N, K).bn : plan(M, N, K).bn; }
+int tile_width(int M, int N, int K) { return two_planes(K) ? f16::plan(M, N, K).bn : tile_columns(M, N); }
 
 size_t image_bytes(int M, int N, int K) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
@@ -636,7 +570,7 @@ int split_weights(const WeightJob* jobs, int count, const LambdaJob& lambda, cud
 size_t workspace_bytes(int M, int N, int K) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   // (of a weight's product or of two activations')
-  const int splits = std::max(plan(M, N, K).splits, two_planes(K) ? f16::plan(M, N, K).splits : 1);
+  const int splits = two_planes(K) ? std::max(f16::plan(M, N, K).splits, f16::plan_outer(M, N, K).splits) : 1;
   return splits > 1 ? static_cast<size_t>(splits) * M * N * sizeof(float) : 0;
 }
 
@@ -658,20 +592,28 @@ int run_weights(const float* a, long long lda, const void* image, float* c, long
   p.M = M; p.N = N; p.K = K;
   p.ep = ep;
   p.status = status;
-  return run<false>(p, ws, ws_bytes, nullptr, stream);
+  return run<false>(p, stream);
 }
 
 int run_outer(const float* a, long long lda, const float* b, long long ldb, float* c, long long ldc, int M, int N, int K,
               float* ws, size_t ws_bytes, int* partials, int* status, cudaStream_t stream) {
   if (!a || !b || !c) return MXK_ERR_NULL;
   if (M <= 0 || N <= 0 || K <= 0) return MXK_ERR_DIMS;
+  if (two_planes(K)) {
+    const f16::Plan pl = f16::plan_outer(M, N, K);
+    if (pl.splits > 1 && (!ws || ws_bytes < static_cast<size_t>(pl.splits) * M * N * sizeof(float))) return MXK_ERR_WORKSPACE;
+    const int st = f16::launch_outer(pl, a, lda, b, ldb, c, ldc, M, N, K, ws, status, stream);
+    if (partials) *partials = pl.splits;
+    return st != MXK_OK || pl.splits == 1 || partials ? st : reduce_splits(ws, pl.splits, M, N, c, ldc, {}, stream);
+  }
   Params p{};
   p.a = a; p.lda = lda;
   p.b = b; p.ldb = ldb;
   p.c = c; p.ldc = ldc;
   p.M = M; p.N = N; p.K = K;
   p.status = status;
-  return run<true>(p, ws, ws_bytes, partials, stream);
+  if (partials) *partials = 1;
+  return run<true>(p, stream);
 }
 
 }  // namespace gemm32

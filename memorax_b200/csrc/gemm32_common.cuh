@@ -5,6 +5,7 @@
 
 #include "gemm32.cuh"
 #include "mxk_common.cuh"
+#include "tma.cuh"
 #include "umma.cuh"
 
 namespace mxk {
@@ -138,6 +139,10 @@ inline size_t image_bytes(int bn, int N, int K) { return planes_bytes(bn, N, K) 
 // C = A W^T; `partial` (splits x M x N) takes the parts of a split contraction.
 int launch_weights(const Plan& pl, const float* a, long long lda, const void* image, float* c, long long ldc, int M, int N, int K, const Epilogue& ep,
                    float* partial, int* status, cudaStream_t stream);
+// C = A^T B, both stored [K][..] (gemm32_f16_outer.cu).
+Plan plan_outer(int M, int N, int K);
+int launch_outer(const Plan& pl, const float* a, long long lda, const float* b, long long ldb, float* c, long long ldc, int M, int N, int K, float* partial,
+                 int* status, cudaStream_t stream);
 
 constexpr float kLo = 2048.f;     // lo planes are this much larger than what they stand for
 constexpr int kTargetExp = 14;    // the largest element of a row is scaled to [2^14, 2^15)
@@ -179,6 +184,59 @@ __device__ __forceinline__ void split8(const float* x, float s, uint4& hi, uint4
 // Column of a 32-column block in which W's row `n` of the block is placed, so that the eight values that a thread reads from a
 // lane with tmem_ld_16x32 are consecutive columns of C and its stores fill whole lines.
 __device__ __forceinline__ int placed(int n) { return 8 * ((n >> 1) & 3) + 2 * (n >> 3) + (n & 1); }
+
+constexpr int kBM = 128;
+constexpr int kSlots = 8;      // stages whose units and events are kept: more than producers are ahead of the epilogue
+constexpr int kHeadroom = 6;   // powers of two that a row may grow by after its first stage
+
+template <int N> __device__ __forceinline__ void more_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void fewer_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+
+// Arrives on the barrier of this offset in the CTA of rank 0: tensor memory has been read (tcgen05 fences order that; a release
+// at cluster scope would wait for every access to global memory under way, 1900 cycles).
+__device__ __forceinline__ void arrive_read(uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, 0;\n\t"
+      "mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [ra];\n\t}\n" ::"r"(umma::smem_u32(bar))
+      : "memory");
+}
+// The same after writes to shared memory that the tensor core is to read.
+__device__ __forceinline__ void arrive_written(uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, 0;\n\t"
+      "mbarrier.arrive.shared::cluster.b64 _, [ra];\n\t}\n" ::"r"(umma::smem_u32(bar))
+      : "memory");
+}
+// Stores to CTA `rank` of the cluster.
+__device__ __forceinline__ void store_at(uint32_t* p, int rank, uint32_t v) {
+  asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, %1;\n\tst.shared::cluster.u32 [ra], %2;\n\t}\n" ::"r"(umma::smem_u32(p)), "r"(rank), "r"(v) : "memory");
+}
+
+// 16 TMEM lanes x 32 columns: r[4 j + 2 h + e] is lane (lane / 4) + 8 h, column 8 j + 2 (lane % 4) + e.
+__device__ __forceinline__ void tmem_ld_16x32(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+// Four floats of shared memory, read here and nowhere else: a plain load may be repeated where its values are used, after the tile
+// has been given back.
+__device__ __forceinline__ void read_once(const void* p, float* x) {
+  asm volatile("ld.volatile.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]) : "r"(umma::smem_u32(p)) : "memory");
+}
+__device__ __forceinline__ float read_once(const void* p) {
+  float x;
+  asm volatile("ld.volatile.shared.f32 %0, [%1];" : "=f"(x) : "r"(umma::smem_u32(p)) : "memory");
+  return x;
+}
+__device__ __forceinline__ void load_box(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(umma::smem_u32(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(umma::smem_u32(bar)), "r"(x), "r"(y)
+      : "memory");
+}
 
 // A block splits four rows of a weight: 64 threads a row look for its largest element, then each writes the planes of every 64th
 // vector of eight k.  Bound: the latency of its loads, all of them under way together up to 1024 k (1024 x 256: 4.6 us).

@@ -2,7 +2,8 @@
 //
 // A float32 number, scaled by a power of two, is the sum of two float16 numbers (hi + lo, 11 + 11 mantissa bits and lo's sign) to
 // within 2^-23 of itself, so a product of float32 matrices is three float16 products, hi*hi + hi*lo + lo*hi, accumulated in
-// float32; lo*lo is below 2^-24 of |a||b|.  (The sum of three bf16 numbers, which needs no scales, takes six: gemm32.cu.)
+// float32; lo*lo is below 2^-22 of |a||b|, and mostly below 2^-24.  (The sum of three bf16 numbers, which needs no scales, takes
+// six: gemm32.cu.)
 //
 // Scales.  A row of the weight is scaled so that its largest element is in [2^14, 2^15).  A row of A takes the scale of its first
 // kBK elements, with room for elements 2^kHeadroom larger; where one later does not fit, the producers begin a new scale at that
@@ -41,9 +42,6 @@ namespace {
 
 using namespace umma;
 
-constexpr int kBM = 128;
-constexpr int kSlots = 8;      // stages whose units and events are kept: more than producers are ahead of the epilogue
-constexpr int kHeadroom = 6;   // powers of two that a row may grow by after its first stage
 constexpr int kLongRuns = 384; // from here on the hi*hi accumulator lives for two stages
 
 struct Params {
@@ -54,6 +52,8 @@ struct Params {
   const int* unit_w;     // exponents of the units of W's rows, to the end of the last tile
   float* c;
   long long ldc;
+  int c_vec;             // floats per aligned access to a row
+  bool vectors;          // eight of C's, four of what is added
   int M, N, K;
   int k_split;           // k per split (a multiple of kBK)
   int splits;            // more than one: c is [splits][M][N]
@@ -87,51 +87,8 @@ struct Config {
   static_assert(kEpilogueWarps * kRegsEpilogue + kProducerWarps * kRegsProducer + 4 * kRegsMma == kThreads / 32 * 96, "the launch's registers");
 };
 
-template <int N> __device__ __forceinline__ void more_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
-template <int N> __device__ __forceinline__ void fewer_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
-
-// Arrives on the barrier of this offset in the CTA of rank 0: tensor memory has been read (tcgen05 fences order that; a release
-// at cluster scope would wait for every access to global memory under way, 1900 cycles).
-__device__ __forceinline__ void arrive_read(uint64_t* bar) {
-  asm volatile(
-      "{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, 0;\n\t"
-      "mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [ra];\n\t}\n" ::"r"(smem_u32(bar))
-      : "memory");
-}
-// The same after writes to shared memory that the tensor core is to read.
-__device__ __forceinline__ void arrive_written(uint64_t* bar) {
-  asm volatile(
-      "{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, 0;\n\t"
-      "mbarrier.arrive.shared::cluster.b64 _, [ra];\n\t}\n" ::"r"(smem_u32(bar))
-      : "memory");
-}
-// Stores to CTA `rank` of the cluster.
-__device__ __forceinline__ void store_at(uint32_t* p, int rank, uint32_t v) {
-  asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, %1;\n\tst.shared::cluster.u32 [ra], %2;\n\t}\n" ::"r"(smem_u32(p)), "r"(rank), "r"(v) : "memory");
-}
-
-// 16 TMEM lanes x 32 columns: r[4 j + 2 h + e] is lane (lane / 4) + 8 h, column 8 j + 2 (lane % 4) + e.
-__device__ __forceinline__ void tmem_ld_16x32(uint32_t taddr, uint32_t* r) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-}
-// Four floats of shared memory, read here and nowhere else: a plain load may be repeated where its values are used, after the tile
-// has been given back.
-__device__ __forceinline__ void read_once(const void* p, float* x) {
-  asm volatile("ld.volatile.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]) : "r"(smem_u32(p)) : "memory");
-}
-__device__ __forceinline__ void load_box(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y)
-      : "memory");
-}
-
-// kWide: rows of A begin on 16-byte boundaries, those of C on 32-byte ones.  kEp: something is added on the way out.
+// kWide: rows of A begin on 16-byte boundaries; where they do not, the producers read them element by element.  kEp: something is
+// added on the way out.
 // (The instruction cache is small beside this much unrolled code: what is rare is a rolled loop over a copy of the sums in
 // local memory, or another instantiation.)
 template <int BN, bool kWide, bool kEp>
@@ -275,12 +232,12 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
         }
       }
       float* const dst = p.c + (p.splits > 1 ? static_cast<size_t>(sp) * p.M * p.N : 0);
-      // units whose powers are factors that leave room for the sums, and a whole tile
+      // units whose powers are factors that leave room for the sums (a row of zeros has the smallest), and a whole tile
       bool plain = true;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) plain &= abs(unit[i]) <= 60;
-      plain &= max(max(abs(unit_w.x), abs(unit_w.y)), max(abs(unit_w.z), abs(unit_w.w))) <= 60;
-      if (kWide && __all_sync(0xffffffffu, plain) && m0 - row0 + kBM <= p.M && n0 + BN / 2 <= p.N) {
+      for (int i = 0; i < 4; ++i) plain &= unit[i] <= 60;
+      plain &= max(max(unit_w.x, unit_w.y), max(unit_w.z, unit_w.w)) <= 60;
+      if (p.vectors && __all_sync(0xffffffffu, plain) && m0 - row0 + kBM <= p.M && n0 + BN / 2 <= p.N) {
         float fr[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) fr[i] = pow2(unit[i]);
@@ -337,7 +294,7 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
             if (kEp && p.ep.bias) x[e] += __ldg(p.ep.bias + n + e);
             if (kEp && p.ep.add) x[e] = fmaf(__ldg(p.ep.add + m * p.ep.ld_add + n + e), p.ep.add_scale ? __ldg(p.ep.add_scale + n + e) : 1.f, x[e]);
           }
-          store8(dst + m * p.ldc + n, valid, kWide ? 8 : 1, x);
+          store8(dst + m * p.ldc + n, valid, p.c_vec, x);
         }
       }
     }
@@ -355,14 +312,21 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
 #pragma unroll 1
       for (int seg = 0; seg < k_len; seg += kBK, ++turn) {
         float x[2][2][8];
-        wait(&raw_full[raw], raw_parity);
+        if (kWide) wait(&raw_full[raw], raw_parity);
         const uint8_t* const src = smem + L::kRawAt + raw * L::kRaw + r0 * 128;
+        const int m = tile % (mt * nt) / nt * kTileM + rank * kBM + r0, k = tile / (mt * nt) * p.k_split + seg + (lane >> 3) * 8;
 #pragma unroll
         for (int g = 0; g < 2; ++g)
 #pragma unroll
           for (int b = 0; b < 2; ++b)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
+              if (!kWide) {
+                const float* const from = p.a + (m + 8 * g) * p.lda + k + 32 * b + 4 * h;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) x[g][b][4 * h + e] = m + 8 * g < p.M && k + 32 * b + 4 * h + e < p.K ? __ldg(from + e) : 0.f;
+                continue;
+              }
               read_once(src + b * (L::kRaw / 2) + g * 1024 + (((lane >> 3) * 2 + h) ^ (lane & 7)) * 16, x[g][b] + 4 * h);
             }
         float most[2];
@@ -376,7 +340,7 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
           most[g] = fmaxf(most[g], __shfl_xor_sync(0xffffffffu, most[g], 16));
         }
         // The tile may be overwritten once every lane has its values: the vote takes the maxima, and those take all of them.
-        if (!__any_sync(0xffffffffu, most[0] < 0.f || most[1] < 0.f) && lane == 0) arrive(&raw_empty[raw]);
+        if (kWide && !__any_sync(0xffffffffu, most[0] < 0.f || most[1] < 0.f) && lane == 0) arrive(&raw_empty[raw]);
         if (++raw == L::kRaws) { raw = 0; raw_parity ^= 1; }
         const int slot = turn % kSlots;
         bool event = false;
@@ -505,7 +469,7 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
           if (++stage == kStages) { stage = 0; parity ^= 1; }
         }
       }
-    } else if (warp == L::kRawWarp && (!kWide || lane == 0)) {
+    } else if (kWide && warp == L::kRawWarp && lane == 0) {
       // ---------------------------------------------------------- float32 tiles of A
       int raw = 0;
       uint32_t parity = 1;
@@ -514,22 +478,9 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
         for (int seg = 0; seg < k_len; seg += kBK) {
           wait(&raw_empty[raw], parity);
           uint8_t* const dst = smem + L::kRawAt + raw * L::kRaw;
-          if (kWide) {
-            tma::expect_bytes(&raw_full[raw], L::kRaw);
-            load_box(dst, &p.map_a, &raw_full[raw], k0 + seg, m0);   // zeros past the matrix
-            load_box(dst + L::kRaw / 2, &p.map_a, &raw_full[raw], k0 + seg + 32, m0);
-          } else {
-#pragma unroll 4
-            for (int r = 0; r < kBM; ++r)
-#pragma unroll
-              for (int b = 0; b < 2; ++b) {
-                const int m = m0 + r, k = k0 + seg + b * 32 + lane;
-                const float v = m < p.M && k < p.K ? __ldg(p.a + m * p.lda + k) : 0.f;
-                *reinterpret_cast<float*>(dst + b * (L::kRaw / 2) + r * 128 + ((lane >> 2) ^ (r & 7)) * 16 + (lane & 3) * 4) = v;
-              }
-            __syncwarp();
-            if (lane == 0) arrive(&raw_full[raw]);
-          }
+          tma::expect_bytes(&raw_full[raw], L::kRaw);
+          load_box(dst, &p.map_a, &raw_full[raw], k0 + seg, m0);   // zeros past the matrix
+          load_box(dst + L::kRaw / 2, &p.map_a, &raw_full[raw], k0 + seg + 32, m0);
           if (++raw == L::kRaws) { raw = 0; parity ^= 1; }
         }
       }
@@ -560,7 +511,7 @@ int launch(const Params& p, long long ctas, cudaStream_t stream) {
 }
 template <int BN>
 int launch(const Params& p, bool wide, long long ctas, cudaStream_t stream) {
-  if (!wide) return launch<BN, false, true>(p, ctas, stream);
+  if (!wide) return launch<BN, false, true>(p, ctas, stream);   // (rare enough to do without a form of its own for no addition)
   return p.ep.bias || p.ep.add ? launch<BN, true, true>(p, ctas, stream) : launch<BN, true, false>(p, ctas, stream);
 }
 
@@ -597,7 +548,9 @@ int launch_weights(const Plan& pl, const float* a, long long lda, const void* im
   p.run = K < kLongRuns ? 1 : 2;
   if (pl.splits == 1) p.ep = ep;
   p.status = status;
-  const bool wide = vec_of(a, lda) >= 4 && vec_of(p.c, p.ldc) == 8 && (!p.ep.add || vec_of(p.ep.add, p.ep.ld_add) >= 4);
+  p.c_vec = vec_of(p.c, p.ldc);
+  p.vectors = p.c_vec == 8 && (!p.ep.add || vec_of(p.ep.add, p.ep.ld_add) >= 4);
+  const bool wide = vec_of(a, lda) >= 4;
   if (wide) {
     tma::EncodeTiledFn enc = tma::encode_tiled_fn();
     const cuuint64_t dims[2] = {static_cast<cuuint64_t>(K), static_cast<cuuint64_t>(M)}, strides[1] = {static_cast<cuuint64_t>(lda) * 4};

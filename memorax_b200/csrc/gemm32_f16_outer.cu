@@ -1,0 +1,457 @@
+// float32 products of two activations, C = A^T B (the gradient of a weight), contractions of 256 tokens and more, on the tensor
+// cores: scaled float16 planes as in gemm32_f16.cu.
+//
+// Both operands are contracted over their rows and converted here.  Scales are per column: that of its first kBK tokens in a tile,
+// with room for elements 2^kHeadroom larger; where one later does not fit, a new unit begins at that stage (`event`) and the
+// accumulators are closed before it.  They live for one stage, two in contractions from 512 on, in any case (eight truncating
+// additions), and are then added to float32 sums in registers, which are kept in the columns' units.  Errors against float64,
+// relative 2-norm, normal entries: 2.1e-7 at 4096 tokens, 2.4e-7 at 24000 (three bf16 planes, drained every 512 tokens: 4.3e-7 and
+// 4.7e-7); lognormal, sigma 3: 1.1e-7 (4.0e-7).
+//
+// Bound: the producers.  A stage of 256 x 128 is 768 cycles of the tensor pipe and 12288 numbers to convert, about 1200 cycles of
+// the issue slots, and takes 2400: the twelve warps wait for the same barriers and are in the same phase of their work.
+// Measured (three bf16 planes before): 1024 x 256 over 65536 tokens 151 us (185), 1024 x 512 over 24000 114 us (137), 520 x 512
+// over 8192 36 us (38).
+//
+// One persistent CTA per SM, pairs on tiles of 256 x 128, or alone on 128 x 64:
+//   8 warps    epilogue: accumulators (TMEM) -> sums in registers -> global
+//   12 warps   producers: 32 columns x 32 tokens of a stage each, eight warps for A and four for B
+//   1 warp     issues the MMAs (12 per stage of 64 tokens), 1 warp the copies of both float32 tiles (TMA)
+#include <algorithm>
+
+#include "gemm32_common.cuh"
+
+namespace mxk {
+namespace gemm32 {
+namespace f16 {
+namespace {
+
+using namespace umma;
+
+constexpr int kLongRuns = 512;   // tokens from which on the accumulators live for two stages
+
+struct Params {
+  CUtensorMap map_a, map_b;   // kWide: boxes of 64 tokens x 32 columns
+  const float *a, *b;
+  long long lda, ldb;
+  float* c;
+  long long ldc;
+  int c_vec;             // floats per aligned access to a row
+  int M, N, K;
+  int k_split;           // tokens per split (a multiple of kBK)
+  int splits;            // more than one: c is [splits][M][N]
+  int run;               // stages that the accumulators live for
+  int* status;
+};
+
+// kPair: two CTAs share a tile of 256 rows (cta_group::2), each with 128 columns of A and 64 of B.
+template <bool kPair>
+struct Config {
+  static constexpr int kTileM = kPair ? 2 * kBM : kBM, kBN = kPair ? 128 : 64, kColsB = 64;   // columns of B in this CTA
+  static constexpr int kPlaneA = kBM * kBK * 2, kPlaneB = kColsB * kBK * 2;   // bytes
+  static constexpr int kStage = 2 * (kPlaneA + kPlaneB), kStages = 2;
+  static constexpr int kBox = 32 * kBK * 4, kRaw = (kBM + kColsB) / 32 * kBox, kRaws = 2;   // float32 tiles: boxes of 32 columns, rows of 128 bytes
+  static constexpr int kSets = 2;   // accumulators: kBN columns for hi*hi and kBN for the small products, twice
+  static constexpr uint32_t kTmem = kSets * 2 * kBN;
+  static constexpr int kRawAt = kStages * kStage;
+  static constexpr int kUnits = kRawAt + kRaws * kRaw;             // int8 [kSlots][128 + 128], units of the columns of A and B
+  static constexpr int kMax = kUnits + kSlots * 256;               // float [2][6][2][32], maxima of the halves of a stage
+  static constexpr int kEvents = kMax + 2 * 6 * 2 * 32 * 4;        // [kSlots]
+  static constexpr int kBarriers = kEvents + kSlots * 4;
+  static constexpr int kBytes = kBarriers + (2 * kStages + 2 * kRaws + 2 * kSets + kSlots + 2) * 8;
+  static constexpr int kEpilogueWarps = 8, kProducerWarps = 12, kWarpsA = 8;
+  static constexpr int kMmaWarp = kEpilogueWarps + kProducerWarps, kRawWarp = kMmaWarp + 1;
+  static constexpr int kThreads = 32 * (kMmaWarp + 4);   // warpgroups deal registers: 768 threads of 80
+  static constexpr int kRegsEpilogue = 104, kRegsProducer = 80, kRegsMma = 32;
+  static_assert(kEpilogueWarps * kRegsEpilogue + kProducerWarps * kRegsProducer + 4 * kRegsMma == kThreads / 32 * 80, "the launch's registers");
+};
+
+// Sixteen bytes to the other CTA of the pair, counted by the barrier of this offset there.
+__device__ __forceinline__ void send16(void* p, uint64_t* bar, int rank, uint4 v) {
+  asm volatile(
+      "{\n\t.reg .b32 ra, rb;\n\tmapa.shared::cluster.u32 ra, %0, %2;\n\tmapa.shared::cluster.u32 rb, %1, %2;\n\t"
+      "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [ra], {%3, %4, %5, %6}, [rb];\n\t}\n" ::"r"(smem_u32(p)),
+      "r"(smem_u32(bar)), "r"(rank), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
+      : "memory");
+}
+
+template <bool kPair, bool kWide>
+__global__ void __launch_bounds__(Config<kPair>::kThreads, 1) gemm32_f16_outer_kernel(const __grid_constant__ Params p) {
+  using L = Config<kPair>;
+  constexpr int kStages = L::kStages, kSets = L::kSets, kTileM = L::kTileM, BN = L::kBN;
+  constexpr int kEpilogueWarps = L::kEpilogueWarps, kProducerWarps = L::kProducerWarps, kMmaWarp = L::kMmaWarp;
+  const int mt = (p.M + kTileM - 1) / kTileM, nt = (p.N + BN - 1) / BN;
+  const int tiles = mt * nt * p.splits;
+  const int first_tile = kPair ? blockIdx.x / 2 : blockIdx.x, tile_step = kPair ? gridDim.x / 2 : gridDim.x;
+  enter_kernel(tiles <= tile_step && p.k_split <= 1024);
+  const int rank = kPair ? static_cast<int>(cluster_rank()) : 0;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint64_t* const full = reinterpret_cast<uint64_t*>(smem + L::kBarriers);   // rank 0: producers of both CTAs -> MMA
+  uint64_t* const empty = full + kStages;        // MMA -> producers
+  uint64_t* const acc_full = empty + kStages;    // MMA -> epilogue
+  uint64_t* const acc_empty = acc_full + kSets;  // epilogue -> MMA
+  uint64_t* const peer_units = acc_empty + kSets;   // the other CTA's units of B's columns
+  uint64_t* const raw_full = peer_units + kSlots;   // copies -> producers, the float32 tiles
+  uint64_t* const raw_empty = raw_full + L::kRaws;
+  uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(raw_empty + L::kRaws);
+  int8_t* const units = reinterpret_cast<int8_t*>(smem + L::kUnits);
+  uint32_t* const events = reinterpret_cast<uint32_t*>(smem + L::kEvents);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+
+  if (tid == 0) {
+    for (int s = 0; s < kStages; ++s) { mbar_init(&full[s], kProducerWarps * (kPair ? 2 : 1)); mbar_init(&empty[s], 1); }
+    for (int s = 0; s < kSets; ++s) { mbar_init(&acc_full[s], 1); mbar_init(&acc_empty[s], kEpilogueWarps * (kPair ? 2 : 1)); }
+    for (int s = 0; s < kSlots; ++s) mbar_init(&peer_units[s], 1);
+    for (int s = 0; s < L::kRaws; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], kProducerWarps); }
+    mbar_init_fence();
+  }
+  if (tid < kSlots) events[tid] = 0;
+  if (warp == kMmaWarp) {
+    if (kPair) tmem_alloc_pair(tmem_slot, L::kTmem);
+    else tmem_alloc(tmem_slot, L::kTmem);
+  }
+  fence_before_sync();
+  __syncthreads();
+  if (kPair) cluster_sync();   // the other CTA's barriers are there
+  fence_after_sync();
+  const uint32_t tmem = *tmem_slot;
+  bool timed_out = false;
+  const auto wait = [&](uint64_t* bar, uint32_t parity) { mbar_wait_flag(bar, parity, timed_out); };
+  const auto k_length = [&](int tile) {
+    const int sp = tile / (mt * nt);
+    return min(p.K, (sp + 1) * p.k_split) - sp * p.k_split;
+  };
+  // Whether a column of the tile begins a new unit at this stage; the same in both CTAs.
+  const auto event_at = [&](int turn) { return *const_cast<volatile uint32_t*>(events + turn % kSlots) == turn + 1u; };
+
+  if (warp < kEpilogueWarps) {
+    // ------------------------------------------------------------ epilogue
+    more_registers<L::kRegsEpilogue>();
+    constexpr int kChunks = BN / 64;   // of 32 columns
+    const int col0 = (warp >> 2) * (BN / 2), row0 = (warp & 3) * 32 + (lane >> 2);   // this thread: rows row0 + 8 i
+    float sum[kChunks][4][8];          // [2 j + e]: column 32 c + 8 j + 2 (lane % 4) + e
+    int turn = 0, run = 0;
+    for (int tile = first_tile; tile < tiles; tile += tile_step) {
+      const int mn = tile % (mt * nt), sp = tile / (mt * nt);
+      const int n0 = (mn % nt) * BN + col0, m0 = (mn / nt) * kTileM + rank * kBM + row0;
+      const int k_len = k_length(tile);
+#pragma unroll
+      for (int c = 0; c < kChunks; ++c)
+#pragma unroll
+        for (int i = 0; i < 32; ++i) sum[c][i >> 3][i & 7] = 0.f;
+      const int8_t* unit = nullptr;   // of the sums: a slot, whose units are those of the stages after it up to the next event
+#pragma unroll 1
+      for (int seg = 0; seg < k_len; ++run) {
+        const int set = run % kSets;
+        wait(&acc_full[set], (run / kSets) & 1);
+        fence_after_sync();
+        if (seg == 0 || event_at(turn)) {
+          const int8_t* const next = units + turn % kSlots * 256;
+          if (kPair) wait(&peer_units[turn % kSlots], (turn / kSlots) & 1);
+          if (seg > 0) {   // the sums are brought to the new units, none of which is smaller
+#pragma unroll
+            for (int c = 0; c < kChunks; ++c)
+#pragma unroll
+              for (int e = 0; e < 8; ++e) {
+                const int at = 128 + col0 + c * 32 + (e >> 1) * 8 + (lane & 3) * 2 + (e & 1);
+                const float r = pow2(max(unit[at] - next[at], -126));
+#pragma unroll
+                for (int i = 0; i < 4; ++i) sum[c][i][e] *= r;
+              }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float r = pow2(max(unit[row0 + 8 * i] - next[row0 + 8 * i], -126));
+#pragma unroll
+              for (int c = 0; c < kChunks; ++c)
+#pragma unroll
+                for (int e = 0; e < 8; ++e) sum[c][i][e] *= r;
+            }
+          }
+        }
+        unit = units + turn % kSlots * 256;
+        const uint32_t src = tmem + set * 2 * BN + col0 + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+#pragma unroll
+        for (int c = 0; c < kChunks; ++c)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {   // rows 16 h + lane / 4, + 8
+            uint32_t r[16], q[16];
+            tmem_ld_16x32(src + c * 32 + (static_cast<uint32_t>(16 * h) << 16), r);
+            tmem_ld_16x32(src + BN + c * 32 + (static_cast<uint32_t>(16 * h) << 16), q);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+              for (int i = 0; i < 4; ++i) sum[c][2 * h + (i >> 1)][2 * j + (i & 1)] += fmaf(__uint_as_float(q[4 * j + i]), 1.f / kLo, __uint_as_float(r[4 * j + i]));
+          }
+        fence_before_sync();
+        __syncwarp();
+        if (lane == 0) {
+          if (kPair) arrive_read(&acc_empty[set]);
+          else arrive(&acc_empty[set]);
+        }
+        int n = 0;   // an event ends a run
+        do {
+          ++n;
+          seg += kBK;
+          ++turn;
+        } while (n < p.run && seg < k_len && !event_at(turn));
+      }
+      float* const dst = p.c + (p.splits > 1 ? static_cast<size_t>(sp) * p.M * p.N : 0);
+      int unit_row[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) unit_row[i] = unit[row0 + 8 * i];
+#pragma unroll
+      for (int c = 0; c < kChunks; ++c)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int nc = c * 32 + j * 8 + (lane & 3) * 2, n = n0 + nc;
+          const char2 unit_col = *reinterpret_cast<const char2*>(unit + 128 + col0 + nc);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int m = m0 + 8 * i;
+            const float2 v = make_float2(scale_by(sum[c][i][2 * j], unit_row[i] + unit_col.x), scale_by(sum[c][i][2 * j + 1], unit_row[i] + unit_col.y));
+            if (m >= p.M || n >= p.N) continue;
+            float* const out = dst + m * p.ldc + n;
+            if (p.c_vec >= 4 && n + 1 < p.N) {
+              *reinterpret_cast<float2*>(out) = v;
+            } else {
+              out[0] = v.x;
+              if (n + 1 < p.N) out[1] = v.y;
+            }
+          }
+        }
+    }
+  } else if (warp < kMmaWarp) {
+    // ------------------------------------------------------------ producers
+    fewer_registers<L::kRegsProducer>();
+    // A warp converts 32 columns x 32 tokens, a column a lane, and leaves vectors of eight tokens: what was contracted over rows
+    // becomes K-major on the way, with a scale a lane.  Another warp has the stage's other 32 tokens; the two exchange their maxima.
+    const int pw = warp - kEpilogueWarps;
+    const bool is_b = pw >= L::kWarpsA;
+    const int block = is_b ? pw & 1 : pw & 3, half = is_b ? (pw - L::kWarpsA) >> 1 : pw >> 2, partners = is_b ? 4 + block : block;
+    const int col = block * 32 + lane, rows = is_b ? L::kColsB : kBM, plane = is_b ? L::kPlaneB : L::kPlaneA;
+    const int unit_at = is_b ? 128 + rank * L::kColsB + block * 32 : block * 32;   // of this warp's first column in a slot's units
+    float* const maxima = reinterpret_cast<float*>(smem + L::kMax) + partners * 64;
+    int stage = 0, raw = 0, turn = 0;
+    uint32_t parity = 1, raw_parity = 0;
+    int unit = 0;   // of this lane's column
+    float x[32];
+    const auto load = [&](int tile, int seg) {
+      if (kWide) {
+        wait(&raw_full[raw], raw_parity);
+        const uint8_t* const src = smem + L::kRawAt + raw * L::kRaw + ((is_b ? kBM / 32 : 0) + block) * L::kBox + half * 4096 + (lane & 3) * 4;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) x[i] = read_once(src + i * 128 + ((lane >> 2) ^ (i & 7)) * 16);
+      } else {
+        const int mn = tile % (mt * nt), k = tile / (mt * nt) * p.k_split + half * 32 + seg;
+        const int c = (is_b ? (mn % nt) * BN + rank * L::kColsB : (mn / nt) * kTileM + rank * kBM) + col, end = is_b ? p.N : p.M;
+        const long long ld = is_b ? p.ldb : p.lda;
+        const float* const from = (is_b ? p.b : p.a) + k * ld + c;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) x[i] = k + i < p.K && c < end ? __ldg(from + i * ld) : 0.f;
+      }
+    };
+    if (first_tile < tiles) load(first_tile, 0);
+    for (int tile = first_tile; tile < tiles; tile += tile_step) {
+      const int k_len = k_length(tile);
+#pragma unroll 1
+      for (int seg = 0; seg < k_len; seg += kBK, ++turn) {
+        float m[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) m[i] = fmaxf(fmaxf(fabsf(x[i]), fabsf(x[i + 8])), fmaxf(fabsf(x[i + 16]), fabsf(x[i + 24])));
+        const float own = fmaxf(fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3])), fmaxf(fmaxf(m[4], m[5]), fmaxf(m[6], m[7])));
+        float* const now = maxima + (turn & 1) * (6 * 64);
+        now[half * 32 + lane] = own;
+        asm volatile("bar.sync %0, 64;" ::"r"(1 + partners) : "memory");
+        // (every lane has all of its values, or its maximum would not be there)
+        if (kWide && lane == 0) arrive(&raw_empty[raw]);
+        if (++raw == L::kRaws) { raw = 0; raw_parity ^= 1; }
+        const int slot = turn % kSlots, u = unit_of(fmaxf(own, now[(half ^ 1) * 32 + lane]));
+        bool event = false;
+        if (seg == 0 || u > unit) {
+          event = seg > 0;
+          unit = u + kHeadroom;
+        }
+        const float scale = scale_of(unit);
+        wait(&empty[stage], parity);
+        int8_t* const told = units + slot * 256 + unit_at;
+        if (half == 0) told[lane] = static_cast<int8_t>(unit);
+        uint8_t* const dst = smem + stage * L::kStage + (is_b ? 2 * L::kPlaneA : 0) + (half * 4 * rows + col) * 16;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          uint4 hi, lo;
+          split8(x + 8 * j, scale, hi, lo);
+          *reinterpret_cast<uint4*>(dst + j * rows * 16) = hi;
+          *reinterpret_cast<uint4*>(dst + j * rows * 16 + plane) = lo;
+        }
+        // the next stage's values, on their way under what is left of this one
+        if (seg + kBK < k_len) load(tile, seg + kBK);
+        else if (tile + tile_step < tiles) load(tile + tile_step, 0);
+        if (event) {   // before the arrivals that let the MMAs of this stage begin
+          for (int r = 0; r < (kPair ? 2 : 1); ++r) store_at(events + slot, r, turn + 1u);
+          asm volatile("fence.acq_rel.cluster;" ::: "memory");
+        }
+        fence_smem_to_async();
+        __syncwarp();
+        if (kPair && is_b && half == 0 && lane < 2) send16(told + 16 * lane, &peer_units[slot], rank ^ 1, *reinterpret_cast<const volatile uint4*>(told + 16 * lane));
+        if (lane == 0) {
+          if (kPair && pw == 0) tma::expect_bytes(&peer_units[slot], L::kColsB);
+          if (kPair) arrive_written(&full[stage]);
+          else arrive(&full[stage]);
+        }
+        if (++stage == kStages) { stage = 0; parity ^= 1; }
+      }
+    }
+  } else {
+    fewer_registers<L::kRegsMma>();   // (a whole warpgroup's)
+    if (warp == kMmaWarp) {
+      // ---------------------------------------------------------- tensor core
+      const bool leader = elect_one();
+      const uint32_t idesc = idesc_f16(kTileM, BN, false, false);
+      int stage = 0, turn = 0, runs = 0;
+      uint32_t parity = 0;
+      const auto done = [&](uint64_t* bar) {
+        if (leader) (kPair ? commit_pair : commit)(bar);
+      };
+        for (int tile = first_tile; tile < tiles; tile += tile_step) {
+          const int k_len = k_length(tile);
+          int run = 0;   // stages in the accumulators
+          for (int seg = 0; seg < k_len; seg += kBK, ++turn) {
+            if (rank != 0) {   // the other CTA issues; its commits reach this one's barriers
+              wait(&empty[stage], parity);
+              if (++stage == kStages) { stage = 0; parity ^= 1; }
+              continue;
+            }
+            wait(&full[stage], parity);
+            if (seg > 0 && run > 0 && event_at(turn)) {
+              done(&acc_full[runs++ % kSets]);
+              run = 0;
+            }
+            const int set = runs % kSets;
+            if (run == 0) wait(&acc_empty[set], ((runs / kSets) & 1) ^ 1);
+            fence_after_sync();
+            const uint32_t sa = smem_u32(smem + stage * L::kStage), sb = sa + 2 * L::kPlaneA, acc = tmem + set * 2 * BN;
+            const Operand a0{sa, kBM, false}, a1{sa + L::kPlaneA, kBM, false}, b0{sb, L::kColsB, false}, b1{sb + L::kPlaneB, L::kColsB, false};
+            const int steps = min(kBK, k_len - seg + 15) / 16;   // of 16 tokens
+            const auto product = [&](uint32_t d, const Operand& a, const Operand& b, bool accumulate) {
+              const uint64_t da = a.desc(0), db = b.desc(0);
+#pragma unroll
+              for (int k = 0; k < kBK / 16; ++k)
+                if (leader && k < steps)
+                  (kPair ? mma_bf16_pair : mma_bf16)(d, da + static_cast<uint64_t>(k * a.advance()), db + static_cast<uint64_t>(k * b.advance()), idesc,
+                                                    (accumulate || k > 0) ? 1u : 0u);
+            };
+            product(acc, a0, b0, run > 0);
+            product(acc + BN, a0, b1, run > 0);
+            product(acc + BN, a1, b0, true);
+            done(&empty[stage]);
+            if (++run == p.run || seg + kBK >= k_len) {
+              done(&acc_full[set]);
+              ++runs;
+              run = 0;
+            }
+            if (++stage == kStages) { stage = 0; parity ^= 1; }
+          }
+        }
+        // the last commits may still be on their way to barriers in this CTA's shared memory
+        for (int s = 0; rank == 0 && s < kStages; ++s) {
+          wait(&empty[stage], parity ^ 1);
+          if (++stage == kStages) { stage = 0; parity ^= 1; }
+        }
+    } else if (kWide && warp == L::kRawWarp && lane == 0) {
+      // ---------------------------------------------------------- float32 tiles
+      int raw = 0;
+      uint32_t parity = 1;
+      for (int tile = first_tile; tile < tiles; tile += tile_step) {
+        const int mn = tile % (mt * nt), m0 = mn / nt * kTileM + rank * kBM, n0 = mn % nt * BN + rank * L::kColsB, k0 = tile / (mt * nt) * p.k_split;
+        const int k_len = k_length(tile);
+        for (int seg = 0; seg < k_len; seg += kBK) {
+          wait(&raw_empty[raw], parity);
+          uint8_t* dst = smem + L::kRawAt + raw * L::kRaw;
+          tma::expect_bytes(&raw_full[raw], L::kRaw);
+          for (int c = 0; c < kBM; c += 32, dst += L::kBox) load_box(dst, &p.map_a, &raw_full[raw], m0 + c, k0 + seg);   // zeros past the matrix
+          for (int c = 0; c < L::kColsB; c += 32, dst += L::kBox) load_box(dst, &p.map_b, &raw_full[raw], n0 + c, k0 + seg);
+          if (++raw == L::kRaws) { raw = 0; parity ^= 1; }
+        }
+      }
+    }
+    __syncwarp();
+  }
+
+  if (timed_out && p.status) atomicExch(p.status, 1);
+  fence_before_sync();
+  __syncthreads();
+  if (kPair) cluster_sync();   // nothing reaches into the other CTA any more
+  if (warp == kMmaWarp) {
+    if (kPair) tmem_dealloc_pair(tmem, L::kTmem);
+    else tmem_dealloc(tmem, L::kTmem);
+  }
+}
+
+int tile_m(int bn) { return bn == 64 ? kBM : 2 * kBM; }
+int tile_ctas(int bn) { return bn == 64 ? 1 : 2; }
+
+template <bool kPair, bool kWide>
+int launch(const Params& p, long long ctas, cudaStream_t stream) {
+  using L = Config<kPair>;
+  if (const int st = allow_smem<gemm32_f16_outer_kernel<kPair, kWide>, L::kBytes>(); st != MXK_OK) return st;
+  mxk::launch_kernel_clusters(gemm32_f16_outer_kernel<kPair, kWide>, kPair ? 2 : 1, static_cast<unsigned>(std::min(ctas, static_cast<long long>(kNumSMs))),
+                              L::kThreads, L::kBytes, stream, p);
+  return launch_status();
+}
+
+}  // namespace
+
+// Pairs, unless one SM's tile is all there is.  The contraction is split so that the SMs' rounds of tiles take the fewest stages (three
+// more for a tile's begin and end), each part four stages at least: 1024 x 512 x 24000 in nine parts, two rounds of 42 stages, instead of
+// one round of 94 on 64 of the 74 pairs.
+Plan plan_outer(int M, int N, int K) {
+  Plan pl{M <= 128 || N <= 64 ? 64 : 128, 1, 0};
+  const auto ctas = [&] { return static_cast<long long>((M + tile_m(pl.bn) - 1) / tile_m(pl.bn)) * ((N + pl.bn - 1) / pl.bn) * tile_ctas(pl.bn); };
+  const int kblocks = (K + kBK - 1) / kBK, most = std::max(1, kblocks / 4);
+  if (pl.bn == 128 && ctas() * most < kNumSMs) pl.bn = 64;
+  const long long tiles = ctas() / tile_ctas(pl.bn), slots = kNumSMs / tile_ctas(pl.bn);
+  if (tiles < slots) {
+    long long best = -1;
+    for (int n = 1; n <= most && n <= 32; ++n) {
+      const long long cost = (tiles * n + slots - 1) / slots * ((kblocks + n - 1) / n + 3);
+      if (best < 0 || cost < best) { best = cost; pl.splits = n; }
+    }
+  }
+  const int per = (kblocks + pl.splits - 1) / pl.splits;
+  pl.k_split = per * kBK;
+  pl.splits = (kblocks + per - 1) / per;
+  return pl;
+}
+
+int launch_outer(const Plan& pl, const float* a, long long lda, const float* b, long long ldb, float* c, long long ldc, int M, int N, int K, float* partial,
+                 int* status, cudaStream_t stream) {
+  Params p{};
+  p.a = a; p.lda = lda;
+  p.b = b; p.ldb = ldb;
+  p.c = pl.splits > 1 ? partial : c;
+  p.ldc = pl.splits > 1 ? N : ldc;
+  p.c_vec = vec_of(p.c, p.ldc);
+  p.M = M; p.N = N; p.K = K;
+  p.k_split = pl.k_split; p.splits = pl.splits;
+  p.run = K < kLongRuns ? 1 : 2;
+  p.status = status;
+  const bool wide = vec_of(a, lda) >= 4 && vec_of(b, ldb) >= 4;
+  if (wide) {
+    tma::EncodeTiledFn enc = tma::encode_tiled_fn();
+    const auto map = [&](CUtensorMap* m, const float* q, int cols, long long ld) {
+      const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(K)}, strides[1] = {static_cast<cuuint64_t>(ld) * 4};
+      const cuuint32_t box[2] = {32, kBK}, elem[2] = {1, 1};
+      return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(q), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    };
+    if (!enc || !map(&p.map_a, a, M, lda) || !map(&p.map_b, b, N, ldb)) return MXK_ERR_UNSUPPORTED;
+  }
+  const long long ctas = static_cast<long long>((M + tile_m(pl.bn) - 1) / tile_m(pl.bn)) * ((N + pl.bn - 1) / pl.bn) * pl.splits * tile_ctas(pl.bn);
+  if (pl.bn == 128) return wide ? launch<true, true>(p, ctas, stream) : launch<true, false>(p, ctas, stream);
+  return wide ? launch<false, true>(p, ctas, stream) : launch<false, false>(p, ctas, stream);
+}
+
+}  // namespace f16
+}  // namespace gemm32
+}  // namespace mxk

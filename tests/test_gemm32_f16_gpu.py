@@ -4,11 +4,12 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-# Elementwise, relative to sum |a||b|: two operands to 2^-23 each and the product of their small parts, 2^-24; eight truncating
-# additions of at most 2^-23 to each accumulator, and the float32 sums of the accumulators, 2^-24 each for K / 128 of them.
-# Elements far below the largest of their row are kept to 2^-44 of that (A, with its room to grow; W: 2^-50): a row's largest
-# element may meet an almost vanishing weight.
-BOUND, FLOOR_A, FLOOR_W = 2.0 ** -20 + 2.0 ** -21, 2.0 ** -44, 2.0 ** -50
+# Elementwise, relative to sum |a||b|: two operands to 2^-23 each and the product of their small parts, 2^-22; eight truncating
+# additions of at most 2^-23 to each accumulator, and the float32 sums of the accumulators, 2^-24 each for K / 64 of them.
+# Elements far below the largest of their row are kept to 2^-44 of that (A, with its room to grow; W: 2^-50), and the product that
+# is left out, of the largest's small part (2^-11) and what is below a float16 number of theirs (2^-33, 2^-39), is as much again: a
+# row's largest element may meet an almost vanishing weight.
+BOUND, FLOOR_A, FLOOR_W = 2.0 ** -20 + 2.0 ** -21, 2.0 ** -43, 2.0 ** -49
 
 
 def product(x, w, b=None):
@@ -42,6 +43,48 @@ def test_products_stay_within_the_bound_of_their_terms(m, n, k, kind):
     bound = BOUND * scale + FLOOR_A * x.abs().amax(1, keepdim=True).double() * w.abs().double().sum(1)
     bound += FLOOR_W * x.abs().double().sum(1, keepdim=True) * w.abs().amax(1).double()
     assert bool(((got - want).abs() <= bound).all()), float(((got - want).abs() / bound.clamp(min=1e-300)).max())
+
+
+# rows that begin anywhere: activations cut out of a larger buffer, widths that are no multiple of four
+@pytest.mark.parametrize("m,n,k", [(300, 70, 257), (9000, 256, 320), (20000, 260, 514)])
+def test_rows_at_any_address(m, n, k):
+    torch.manual_seed(m)
+    x, w = torch.empty(m * k + 1, device="cuda")[1:].view(m, k).normal_(), torch.randn(n, k, device="cuda")
+    got, want, scale = product(x, w).double(), x.double() @ w.double().t(), x.abs().double() @ w.abs().double().t()
+    assert bool(((got - want).abs() <= BOUND * scale).all())
+
+
+# the gradient of a weight contracts the tokens of two activations, with units per column: tiles of 256 x 128 on pairs and 128 x 64
+# alone, their edges, runs of two stages, splits, columns that grow from stage to stage, leap, differ, begin with zeros, or start anywhere
+@pytest.mark.parametrize("tokens,m,n", [(256, 1, 1), (257, 64, 127), (1000, 130, 70), (4097, 256, 300), (24000, 520, 260), (300, 2000, 1100)])
+@pytest.mark.parametrize("kind", ["plain", "grows", "leaps", "wide range", "zeros first", "any address"])
+def test_gradients_of_weights_stay_within_the_bound_of_their_terms(tokens, m, n, kind):
+    from memorax_b200 import _C, ops
+    g = torch.Generator("cuda").manual_seed(tokens + m + n)
+    a, b = (torch.randn(tokens, s, generator=g, device="cuda") for s in (m, n))
+    at = torch.arange(tokens, device="cuda")[:, None]
+    if kind == "grows":
+        for t in (a, b):
+            t *= 2.0 ** (9.0 * (at // 64) * (torch.arange(t.shape[1], device="cuda") % 3) - 60).clamp(max=0)
+    elif kind == "leaps":
+        for t in (a, b):
+            t[torch.randint(tokens, (t.shape[1],), generator=g, device="cuda"), torch.arange(t.shape[1], device="cuda")] *= 2.0 ** 30
+    elif kind == "wide range":
+        for t in (a, b):
+            t *= 2.0 ** torch.randint(-60, 56, (1, t.shape[1]), generator=g, device="cuda")   # (sums of 24000 terms stay below 2^128)
+    elif kind == "zeros first":
+        a[:130], b[:70], a[:, ::3] = 0, 0, 0
+    elif kind == "any address":
+        a = torch.empty(tokens * m + 1, device="cuda")[1:].view(tokens, m).copy_(a)
+    w = torch.zeros(m, n, device="cuda", requires_grad=True)
+    y = _C.linear_f32(b, w, None)
+    got = torch.autograd.grad(y, w, a)[0].double()
+    ops.check_status()
+    ad, bd = a.double(), b.double()
+    bound = BOUND * (ad.abs().t() @ bd.abs())
+    bound += FLOOR_A * (ad.abs().amax(0)[:, None] * bd.abs().sum(0) + ad.abs().sum(0)[:, None] * bd.abs().amax(0))
+    bad = (got - ad.t() @ bd).abs() > bound
+    assert not bool(bad.any()), (int(bad.sum()), float(((got - ad.t() @ bd).abs() / bound.clamp(min=1e-300)).max()))
 
 
 def test_a_broken_row_stays_alone():
