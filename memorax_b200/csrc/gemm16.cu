@@ -28,7 +28,8 @@ struct Params {
   float* partial;        // [split][batch][M][N] when splits > 1
   long long ldc, c_batch_stride;
   int batch, M, N, K, k_split, splits;
-  bool accumulate, wide;  // wide: 32-byte aligned output rows
+  bool accumulate;
+  int vec;               // elements of C per aligned access to a row: 16, 8 or 1
   int* status;
 };
 
@@ -174,22 +175,34 @@ __global__ void __launch_bounds__(kThreads, 1) gemm16_kernel(const __grid_consta
               for (int e = 0; e < 16; ++e)
                 if (e < valid) v[e] += __bfloat162float(p.bias[n + e]);
             }
-            if (p.accumulate) {
+            // (sums into existing rows, and rows on 16 bytes only, element by element: 26 us at 6000 x 768 x 8 instead of 11,
+            // 14 at 4 x 6000 x 64 x 128 instead of 7)
+            if (valid >= 16 && p.vec >= 8) {
+              if (p.accumulate) {
+                float had[16];
+                unpack8_bf16(*reinterpret_cast<const uint4*>(dst), had);
+                unpack8_bf16(*reinterpret_cast<const uint4*>(dst + 8), had + 8);
 #pragma unroll
-              for (int e = 0; e < 16; ++e)
-                if (e < valid) v[e] += __bfloat162float(dst[e]);
-            }
-            if (valid >= 16 && p.wide) {
-              uint32_t w[8];
+                for (int e = 0; e < 16; ++e) v[e] += had[e];
+              }
+              if (p.vec == 16) {
+                uint32_t w[8];
 #pragma unroll
-              for (int e = 0; e < 8; ++e) w[e] = pack_bf16(v[2 * e], v[2 * e + 1]);
-              asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]),
-                           "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
-                           : "memory");
+                for (int e = 0; e < 8; ++e) w[e] = pack_bf16(v[2 * e], v[2 * e + 1]);
+                asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]),
+                             "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                             : "memory");
+              } else {
+                *reinterpret_cast<uint4*>(dst) = pack8_bf16(v);
+                *reinterpret_cast<uint4*>(dst + 8) = pack8_bf16(v + 8);
+              }
             } else {
 #pragma unroll
-              for (int e = 0; e < 16; ++e)
-                if (e < valid) dst[e] = __float2bfloat16(v[e]);
+              for (int e = 0; e < 16; ++e) {
+                if (e >= valid) continue;
+                if (p.accumulate) v[e] += __bfloat162float(dst[e]);
+                dst[e] = __float2bfloat16(v[e]);
+              }
             }
           }
         }
@@ -205,32 +218,60 @@ __global__ void __launch_bounds__(kThreads, 1) gemm16_kernel(const __grid_consta
   if (warp == 1) tmem_dealloc(tmem, 2 * BN);
 }
 
-// Eight threads an element, each with every eighth split and eight of those loads in flight; their sums are added in a fixed
-// order.  (One thread an element took 18 to 32 us for the 37 to 74 splits of a narrow weight gradient.)
+// Four elements a thread; of many splits every eighth goes to one of eight threads (one thread for all of the 37 to 74 splits of a
+// narrow weight gradient: 18 to 32 us), and their sums are added in a fixed order.  `kVec`: rows of four elements on aligned places.
+// (An element a thread, always eight to an element: 4096 x 256 x 768 in two splits took 30 us with its product, 8.5 now.)
+template <int kParts, int kVec>
 __global__ void __launch_bounds__(256) reduce_splits_kernel(const float* __restrict__ partial, int splits, long long all, int M, int N,
                                                             const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ c,
                                                             long long ldc, long long c_batch_stride, bool accumulate) {
   enter_kernel();
-  __shared__ float red[8][33];
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const long long i = static_cast<long long>(blockIdx.x) * 32 + tx;
-  float s = 0.f;
+  constexpr int kLanes = 256 / kParts;
+  __shared__ float red[kParts > 1 ? kParts : 1][kLanes][kVec];
+  const int tx = threadIdx.x % kLanes, ty = threadIdx.x / kLanes;
+  const long long i = (static_cast<long long>(blockIdx.x) * kLanes + tx) * kVec;
+  float v[kVec] = {};
   if (i < all) {
+    const float* const from = partial + i;
 #pragma unroll 8
-    for (int k = ty; k < splits; k += 8) s += partial[k * all + i];
+    for (int k = ty; k < splits; k += kParts) {
+      if constexpr (kVec == 4) {
+        const float4 u = *reinterpret_cast<const float4*>(from + k * all);
+        v[0] += u.x; v[1] += u.y; v[2] += u.z; v[3] += u.w;
+      } else {
+        v[0] += from[k * all];
+      }
+    }
   }
-  red[ty][tx] = s;
-  __syncthreads();
-  if (ty != 0 || i >= all) return;
-  float v = red[0][tx];
+  if constexpr (kParts > 1) {
 #pragma unroll
-  for (int k = 1; k < 8; ++k) v += red[k][tx];
+    for (int e = 0; e < kVec; ++e) red[ty][tx][e] = v[e];
+    __syncthreads();
+    if (ty != 0) return;
+#pragma unroll
+    for (int k = 1; k < kParts; ++k)
+#pragma unroll
+      for (int e = 0; e < kVec; ++e) v[e] += red[k][tx][e];
+  }
+  if (i >= all) return;
   const int n = static_cast<int>(i % N);
   const long long row = i / N;
   __nv_bfloat16* const dst = c + row / M * c_batch_stride + row % M * ldc + n;
-  if (bias) v += __bfloat162float(bias[n]);
-  if (accumulate) v += __bfloat162float(*dst);
-  *dst = __float2bfloat16(v);
+#pragma unroll
+  for (int e = 0; e < kVec; ++e) {
+    if (bias) v[e] += __bfloat162float(bias[n + e]);
+    if (accumulate) v[e] += __bfloat162float(dst[e]);
+  }
+  if constexpr (kVec == 4) *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]));
+  else *dst = __float2bfloat16(v[0]);
+}
+template <int kParts>
+void reduce_splits(const Params& p, cudaStream_t stream) {
+  const long long all = static_cast<long long>(p.batch) * p.M * p.N;
+  const bool vec = p.N % 4 == 0 && p.ldc % 4 == 0 && p.c_batch_stride % 4 == 0 && reinterpret_cast<uintptr_t>(p.c) % 8 == 0;
+  const long long per_block = 256 / kParts * (vec ? 4 : 1);
+  mxk::launch_kernel(vec ? reduce_splits_kernel<kParts, 4> : reduce_splits_kernel<kParts, 1>, static_cast<unsigned>((all + per_block - 1) / per_block), 256, 0, stream, p.partial, p.splits, all,
+                     p.M, p.N, p.bias, p.c, p.ldc, p.c_batch_stride, p.accumulate);
 }
 
 // Narrow tiles where wide ones would leave SMs idle; a contraction is split when even those do and each part still has
@@ -303,13 +344,13 @@ int run(const Matrix& a, bool a_rows, const Matrix& b, bool b_rows, const void* 
   p.batch = batch; p.M = M; p.N = N; p.K = K;
   p.k_split = pl.k_split; p.splits = pl.splits;
   p.accumulate = accumulate;
-  p.wide = (reinterpret_cast<uintptr_t>(c) % 32 == 0) && ldc % 16 == 0 && c_batch_stride % 16 == 0;
+  const auto rows_on = [&](int elements) { return reinterpret_cast<uintptr_t>(c) % (2 * elements) == 0 && ldc % elements == 0 && c_batch_stride % elements == 0; };
+  p.vec = rows_on(16) ? 16 : rows_on(8) ? 8 : 1;
   p.status = status;
   const int st = pl.bn == 128 ? launch_bn<128>(p, a_rows, b_rows, stream) : launch_bn<64>(p, a_rows, b_rows, stream);
   if (st != MXK_OK || pl.splits == 1) return st;
-  const long long all = static_cast<long long>(batch) * M * N;
-  mxk::launch_kernel(reduce_splits_kernel, static_cast<unsigned>((all + 31) / 32), 256, 0, stream, p.partial, pl.splits, all, M, N, p.bias, p.c, ldc,
-                                                                                     c_batch_stride, accumulate);
+  if (pl.splits > 8) reduce_splits<8>(p, stream);
+  else reduce_splits<1>(p, stream);
   return launch_status();
 }
 

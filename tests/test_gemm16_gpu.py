@@ -37,3 +37,21 @@ def test_batched_product_on_strided_heads(tokens, heads, dim):
     gw = _C.product_bf16(part.transpose(1, 2), u)
     want = part.double().transpose(1, 2) @ u.double()
     assert float((gw.double() - want).norm() / want.norm()) <= 4e-3
+
+
+# sums into rows on 32, 16 and 2 bytes, and the sum of few and of many splits into them, four elements at a time and one
+@pytest.mark.parametrize("n,ld,at", [(96, 96, 0), (96, 104, 8), (96, 99, 1), (100, 104, 4), (41, 41, 0)])
+@pytest.mark.parametrize("k", [40, 640, 6000])
+def test_sums_into_rows_at_any_address(n, ld, at, k):
+    from memorax_b200 import _C, ops
+    g = torch.Generator("cuda").manual_seed(n + k)
+    mk = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    a, b, held = mk(130, k), mk(k, -(-n // 8) * 8)[:, :n], mk(130 * ld + at)
+    c, before = held[at:].view(130, ld)[:, :n], held.clone()
+    want = a.double() @ b.double() + c.double()
+    _C.product_bf16(a, b, None, c)
+    assert float((c.double() - want).norm() / want.norm()) <= 4e-3
+    rest = torch.ones_like(held, dtype=torch.bool)
+    rest[at:].view(130, ld)[:, :n] = False
+    assert torch.equal(held[rest], before[rest])
+    ops.check_status()
