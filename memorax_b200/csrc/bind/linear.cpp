@@ -76,10 +76,19 @@ Tensor product_bf16(const Tensor& a, const Tensor& b, const OptTensor& bias, con
   return *c;
 }
 
+// c[i] = a[i] b[i], in one launch where the kernel takes them all
+void products_bf16(const std::vector<Tensor>& a, const std::vector<Tensor>& b, const std::vector<Tensor>& c) {
+  const c10::cuda::CUDAGuard guard(a.at(0).device());
+  std::vector<Product> products;
+  for (size_t i = 0; i < a.size(); ++i) products.push_back({a[i], b.at(i), c.at(i)});
+  products_into(products);
+}
+
 }  // namespace
 
 void bind_linear(pybind11::module_& m) {
   m.def("product_bf16", &product_bf16, pybind11::arg("a"), pybind11::arg("b"), pybind11::arg("bias") = pybind11::none(), pybind11::arg("c") = pybind11::none());
+  m.def("products_bf16", &products_bf16);
   m.def("linear_f32", &linear_f32, pybind11::arg("x"), pybind11::arg("w"), pybind11::arg("bias") = pybind11::none()); }
 
 }  // namespace mxk_host

@@ -63,8 +63,7 @@ Result forward(const Tensor& x, const variable_list& p, const Tensor& c0, const 
   const Tensor gate_b = piece(gates, gate_w_size, {2 * s.H});
   check("mlstm_weights", l::mlstm_weights(p[kQ].data_ptr(), p[kK].data_ptr(), p[kIW].data_ptr(), p[kFW].data_ptr(), p[kIB].data_ptr(), p[kFB].data_ptr(),
                                           r.qk_w.data_ptr(), r.gate_w.data_ptr(), gate_b.data_ptr(), s.H, s.d, st));
-  product_into(heads(r.u, 0, s), swapped(r.qk_w), parts(r.qkv, 0, 2, s));
-  product_into(heads(r.up, 0, s), swapped(p[kV]), parts(r.qkv, 2, 1, s));
+  products_into({{heads(r.u, 0, s), swapped(r.qk_w), parts(r.qkv, 0, 2, s)}, {heads(r.up, 0, s), swapped(p[kV]), parts(r.qkv, 2, 1, s)}});
   r.logits = product(r.qkv, transposed(r.gate_w), gate_b);
   r.log_i = empty_like_of(x, {s.M, s.H}, at::kFloat);
   r.log_f = empty_like_of(x, {s.M, s.H}, at::kFloat);
@@ -131,7 +130,6 @@ struct MlstmLayer : torch::autograd::Function<MlstmLayer> {
       gm0 = empty_like_of(x, {s.B, 1, s.H, 1, 1}, at::kFloat);
     }
     const Tensor gg = product(gy, p[kOut]);
-    grads[1 + kOut] = product(transposed(gy), g);
     const Tensor gh = empty_like_of(x, {s.M, s.hid}, bf), gu = empty_like_of(x, {s.M, s.hid}, bf), gks = empty_like_of(x, {s.M, s.hid}, bf), gx = empty_like_of(x, {s.M, s.hid}, bf);
     const Tensor gup = empty_like_of(x, {s.M, 2 * s.hid}, bf), gqkv = empty_like_of(x, {s.M, 3 * s.hid}, bf), glogits = empty_like_of(x, {s.M, 2 * s.H}, bf);
     const Tensor gli = empty_like_of(x, {s.M, s.H}, at::kFloat), glf = empty_like_of(x, {s.M, s.H}, at::kFloat);
@@ -150,16 +148,8 @@ struct MlstmLayer : torch::autograd::Function<MlstmLayer> {
     check("mlstm_gates_bwd", l::mlstm_gates_bwd(logits.data_ptr(), ptr(gli), ptr(glf), gks.data_ptr(), s.scale(), column(gqkv, s.d), 3 * s.hid, 3 * s.d,
                                                 glogits.data_ptr(), part_gate, s.M, s.H, s.d, st));
     product_into(glogits, gate_w, gqkv, Tensor(), true);
-    const Tensor ggate = product(transposed(glogits), qkv);
-    grads[1 + kIW] = piece(ggate, 0, {s.H, 3 * s.hid});
-    grads[1 + kFW] = piece(ggate, 3ll * s.hid * s.H, {s.H, 3 * s.hid});
     const Tensor gqk = parts(gqkv, 0, 2, s), gvalue = parts(gqkv, 2, 1, s);
-    const Tensor gqk_w = product(swapped(gqk), heads(u, 0, s));
-    grads[1 + kQ] = view_of(gqk_w, 0, {s.H, s.d, s.d}, {2 * s.d * s.d, s.d, 1});
-    grads[1 + kK] = view_of(gqk_w, s.d * s.d, {s.H, s.d, s.d}, {2 * s.d * s.d, s.d, 1});
-    grads[1 + kV] = product(swapped(gvalue), heads(up, 0, s));
-    product_into(gqk, qk_w, heads(gu, 0, s), Tensor(), true);
-    product_into(gvalue, p[kV], heads(gx, 0, s));
+    products_into({{gqk, qk_w, heads(gu, 0, s), true}, {gvalue, p[kV], heads(gx, 0, s)}});
     check("mlstm_conv_bwd", l::mlstm_conv_bwd(up.data_ptr(), 2 * s.hid, p[kConvW].data_ptr(), p[kConvB].data_ptr(), gu.data_ptr(), gx.data_ptr(), gup.data_ptr(), part_conv, s.B,
                                               s.T, s.hid, st));
     const Tensor small = empty_like_of(x, {cols[0] + cols[1] + cols[2]}, bf);
@@ -177,7 +167,17 @@ struct MlstmLayer : torch::autograd::Function<MlstmLayer> {
     give(kFB, s.H);
     give(kConvW, 4 * s.hid);
     give(kConvB, s.hid);
-    grads[1 + kUp] = product(transposed(gup), matrix(x, s.M, s.F));
+    const Tensor ggate = empty_like_of(x, {2 * s.H, 3 * s.hid}, bf), gqk_w = empty_like_of(x, {s.H, 2 * s.d, s.d}, bf);
+    for (int i : {kOut, kV, kUp}) grads[1 + i] = empty_like_of(x, p[i].sizes(), bf);
+    products_into({{transposed(gup), matrix(x, s.M, s.F), grads[1 + kUp]},
+                   {transposed(gy), g, grads[1 + kOut]},
+                   {transposed(glogits), qkv, ggate},
+                   {swapped(gqk), heads(u, 0, s), gqk_w},
+                   {swapped(gvalue), heads(up, 0, s), grads[1 + kV]}});
+    grads[1 + kIW] = piece(ggate, 0, {s.H, 3 * s.hid});
+    grads[1 + kFW] = piece(ggate, 3ll * s.hid * s.H, {s.H, 3 * s.hid});
+    grads[1 + kQ] = view_of(gqk_w, 0, {s.H, s.d, s.d}, {2 * s.d * s.d, s.d, 1});
+    grads[1 + kK] = view_of(gqk_w, s.d * s.d, {s.H, s.d, s.d}, {2 * s.d * s.d, s.d, 1});
     if (ctx->needs_input_grad(0)) {
       grads[0] = empty_like_of(x, x.sizes(), bf);
       product_into(gup, p[kUp], matrix(grads[0], s.M, s.F));

@@ -18,9 +18,12 @@ namespace mxk_host {
 // 289; 65536 x 512: 2586 | 2994 | 2950 | 3045 (the sums into existing tensors, which the line does not tell apart).
 constexpr double kLibraryFlops = 8e9;
 
-// c = a b (+ bias) (+ c when `accumulate`) over the last two dimensions; a (M, K), b (K, N), c (M, N), or the same with a
-// leading batch dimension: any views whose rows or columns are contiguous.
-inline void product_into(const Tensor& a, const Tensor& b, const Tensor& c, const Tensor& bias = Tensor(), bool accumulate = false) {
+// A product over the last two dimensions as the kernel's job; `fits`: whether it is one for the kernel.
+struct AsJob {
+  mxk::gemm16::Job job;
+  bool a_rows, b_rows, fits;
+};
+inline AsJob as_job(const Tensor& a, const Tensor& b, const Tensor& c, const Tensor& bias, bool accumulate) {
   namespace g = mxk::gemm16;
   const int n = static_cast<int>(c.dim()), r = n - 2, q = n - 1;
   const int64_t batch = n == 3 ? c.size(0) : 1, M = c.size(r), N = c.size(q), K = a.size(q);
@@ -30,16 +33,26 @@ inline void product_into(const Tensor& a, const Tensor& b, const Tensor& c, cons
     by_rows = row_major != k_is_col;
     return g::Matrix{t.data_ptr(), row_major ? t.stride(r) : t.stride(q), n == 3 ? t.stride(0) : 0};
   };
-  bool a_rows, b_rows;
-  const g::Matrix ma = rows_of(a, a_rows, true), mb = rows_of(b, b_rows, false);
+  AsJob j;
+  const g::Matrix ma = rows_of(a, j.a_rows, true), mb = rows_of(b, j.b_rows, false);
   const auto fits = [&](const Tensor& t, const g::Matrix& m) {
     return (t.stride(r) == 1 || t.stride(q) == 1) && m.ld % 8 == 0 && m.batch_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(m.ptr) & 15) == 0;
   };
-  if (2.0 * batch * M * N * K <= kLibraryFlops && fits(a, ma) && fits(b, mb) && c.stride(q) == 1) {
-    const size_t bytes = g::workspace_bytes(batch, M, N, K);
+  j.fits = 2.0 * batch * M * N * K <= kLibraryFlops && fits(a, ma) && fits(b, mb) && c.stride(q) == 1;
+  j.job = {ma, mb, bias.defined() ? bias.data_ptr() : nullptr, c.data_ptr(), c.stride(r), n == 3 ? c.stride(0) : 0, accumulate,
+           static_cast<int>(batch), static_cast<int>(M), static_cast<int>(N), static_cast<int>(K)};
+  return j;
+}
+
+// c = a b (+ bias) (+ c when `accumulate`) over the last two dimensions; a (M, K), b (K, N), c (M, N), or the same with a
+// leading batch dimension: any views whose rows or columns are contiguous.
+inline void product_into(const Tensor& a, const Tensor& b, const Tensor& c, const Tensor& bias = Tensor(), bool accumulate = false) {
+  namespace g = mxk::gemm16;
+  const int n = static_cast<int>(c.dim());
+  if (const AsJob j = as_job(a, b, c, bias, accumulate); j.fits) {
+    const size_t bytes = g::workspace_bytes(j.job.batch, j.job.M, j.job.N, j.job.K);
     const Tensor ws = bytes ? scratch(c, bytes) : Tensor();
-    check("gemm16", g::run(ma, a_rows, mb, b_rows, bias.defined() ? bias.data_ptr() : nullptr, c.data_ptr(), c.stride(r), n == 3 ? c.stride(0) : 0, accumulate, batch, M, N, K,
-                           ptr<void>(ws), bytes, status_ptr(c), stream()));
+    check("gemm16", g::run(j.job, j.a_rows, j.b_rows, ptr<void>(ws), bytes, status_ptr(c), stream()));
     return;
   }
   Tensor out = c;
@@ -53,6 +66,33 @@ inline void product_into(const Tensor& a, const Tensor& b, const Tensor& c, cons
   } else {
     at::mm_out(out, a, b);
   }
+}
+// Products that do not depend on one another: one launch where all of them are the kernel's and stored alike.
+struct Product {
+  Tensor a, b, c;
+  bool accumulate = false;
+};
+inline void products_into(const std::vector<Product>& products) {
+  namespace g = mxk::gemm16;
+  g::Job jobs[g::kMaxGroup];
+  int count = 0;
+  bool a_rows = false, b_rows = false, together = products.size() <= g::kMaxGroup;
+  for (const Product& p : products) {
+    if (!together) break;
+    const AsJob j = as_job(p.a, p.b, p.c, Tensor(), p.accumulate);
+    together = j.fits && (count == 0 || (j.a_rows == a_rows && j.b_rows == b_rows));
+    a_rows = j.a_rows;
+    b_rows = j.b_rows;
+    jobs[count++] = j.job;
+  }
+  if (!together) {
+    for (const Product& p : products) product_into(p.a, p.b, p.c, Tensor(), p.accumulate);
+    return;
+  }
+  const size_t bytes = g::group_workspace_bytes(jobs, count);
+  const Tensor& like = products.front().c;
+  const Tensor ws = bytes ? scratch(like, bytes) : Tensor();
+  check("gemm16 group", g::run_group(jobs, count, a_rows, b_rows, ptr<void>(ws), bytes, status_ptr(like), stream()));
 }
 inline Tensor product(const Tensor& a, const Tensor& b, const Tensor& bias = Tensor()) {
   auto sizes = a.sizes().vec();

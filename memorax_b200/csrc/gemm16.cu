@@ -8,6 +8,8 @@
 // the largest products stay with the library's two-SM tiles.
 #include <cuda_bf16.h>
 
+#include <algorithm>
+
 #include "gemm16.cuh"
 #include "mxk_common.cuh"
 #include "tma.cuh"
@@ -21,7 +23,7 @@ using namespace umma;
 
 constexpr int kBM = 128, kBK = 64, kStages = 4, kThreads = 192;
 
-struct Params {
+struct Problem {
   CUtensorMap map_a, map_b;
   __nv_bfloat16* c;
   const __nv_bfloat16* bias;
@@ -30,6 +32,12 @@ struct Params {
   int batch, M, N, K, k_split, splits;
   bool accumulate;
   int vec;               // elements of C per aligned access to a row: 16, 8 or 1
+  int first_tile;        // of the launch's
+};
+template <int kCount>
+struct Params {
+  Problem problem[kCount];
+  int count, tiles;
   int* status;
 };
 
@@ -51,9 +59,32 @@ __device__ __forceinline__ void arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-template <int BN, bool A_ROWS, bool B_ROWS>
-__global__ void __launch_bounds__(kThreads, 1) gemm16_kernel(const __grid_constant__ Params p) {
-  enter_kernel(((p.M + kBM - 1) / kBM) * ((p.N + BN - 1) / BN) * p.batch * p.splits <= static_cast<int>(gridDim.x));
+// The tile of a launch that a role works at.
+template <int BN>
+struct Tile {
+  int q = 0;   // problem
+  int sp, z, m0, n0, k0, k_end;
+  template <int kCount>
+  __device__ __forceinline__ const Problem& at(const Params<kCount>& all, int tile) {
+    if (kCount > 1)
+      while (q + 1 < all.count && tile >= all.problem[q + 1].first_tile) ++q;
+    const Problem& p = all.problem[q];
+    const int mt = (p.M + kBM - 1) / kBM, nt = (p.N + BN - 1) / BN, per_split = mt * nt * p.batch, i = tile - p.first_tile, r = i % per_split;
+    sp = i / per_split;
+    z = r / (mt * nt);
+    n0 = (r % nt) * BN;
+    m0 = (r / nt % mt) * kBM;
+    k0 = sp * p.k_split;
+    k_end = min(p.K, k0 + p.k_split);
+    return p;
+  }
+};
+
+// kCount: several problems of the same orders share a launch (a chain of short ones waits for the host: the mLSTM layer's five weight
+// gradients in one launch and one sum of their splits instead of ten).
+template <int BN, bool A_ROWS, bool B_ROWS, int kCount>
+__global__ void __launch_bounds__(kThreads, 1) gemm16_kernel(const __grid_constant__ Params<kCount> all) {
+  enter_kernel(all.tiles <= static_cast<int>(gridDim.x));
   using L = Layout<BN>;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* const full = reinterpret_cast<uint64_t*>(smem + L::kBars);
@@ -73,18 +104,17 @@ __global__ void __launch_bounds__(kThreads, 1) gemm16_kernel(const __grid_consta
   fence_after_sync();
   const uint32_t tmem = *slot;
   bool timed_out = false;
-  const int mt = (p.M + kBM - 1) / kBM, nt = (p.N + BN - 1) / BN, per_split = mt * nt * p.batch;
-  const int tiles = per_split * p.splits;
+  const int tiles = all.tiles;
+  Tile<BN> at;
 
   if (warp == 0) {
     int stage = 0;
     uint32_t parity = 1;
     const bool leader = elect_one();
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-      const int sp = tile / per_split, r = tile % per_split, z = r / (mt * nt);
-      const int n0 = (r % nt) * BN, m0 = (r / nt % mt) * kBM;
-      const int k_end = min(p.K, (sp + 1) * p.k_split);
-      for (int k0 = sp * p.k_split; k0 < k_end; k0 += kBK) {
+      const Problem& p = at.at(all, tile);
+      const int n0 = at.n0, m0 = at.m0, z = at.z;
+      for (int k0 = at.k0; k0 < at.k_end; k0 += kBK) {
         mbar_wait_flag(&empty[stage], parity, timed_out);
         if (leader) {
           uint8_t* const sa = smem + stage * L::kStage;
@@ -113,13 +143,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemm16_kernel(const __grid_consta
     int stage = 0, turn = 0;
     uint32_t parity = 0;
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++turn) {
-      const int sp = tile / per_split;
-      const int k_end = min(p.K, (sp + 1) * p.k_split);
+      at.at(all, tile);
       const int buf = turn & 1;
       mbar_wait_flag(&acc_empty[buf], ((turn >> 1) & 1) ^ 1, timed_out);
       fence_after_sync();
       bool first = true;
-      for (int k0 = sp * p.k_split; k0 < k_end; k0 += kBK) {
+      for (int k0 = at.k0; k0 < at.k_end; k0 += kBK) {
         mbar_wait_flag(&full[stage], parity, timed_out);
         fence_after_sync();
         const uint32_t sa = smem_u32(smem + stage * L::kStage), sb = sa + L::kA;
@@ -138,8 +167,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm16_kernel(const __grid_consta
     const int sub = warp & 3;   // tensor-memory lanes this warp may read
     int turn = 0;
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++turn) {
-      const int sp = tile / per_split, r = tile % per_split, z = r / (mt * nt);
-      const int n0 = (r % nt) * BN, m = (r / nt % mt) * kBM + sub * 32 + lane;
+      const Problem& p = at.at(all, tile);
+      const int sp = at.sp, z = at.z, n0 = at.n0, m = at.m0 + sub * 32 + lane;
       const bool in = m < p.M;
       const int buf = turn & 1;
       mbar_wait_flag(&acc_full[buf], (turn >> 1) & 1, timed_out);
@@ -212,7 +241,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm16_kernel(const __grid_consta
       if (lane == 0) arrive(&acc_empty[buf]);
     }
   }
-  if (timed_out && p.status) atomicExch(p.status, 1);
+  if (timed_out && all.status) atomicExch(all.status, 1);
   fence_before_sync();
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem, 2 * BN);
@@ -221,25 +250,40 @@ __global__ void __launch_bounds__(kThreads, 1) gemm16_kernel(const __grid_consta
 // Four elements a thread; of many splits every eighth goes to one of eight threads (one thread for all of the 37 to 74 splits of a
 // narrow weight gradient: 18 to 32 us), and their sums are added in a fixed order.  `kVec`: rows of four elements on aligned places.
 // (An element a thread, always eight to an element: 4096 x 256 x 768 in two splits took 30 us with its product, 8.5 now.)
-template <int kParts, int kVec>
-__global__ void __launch_bounds__(256) reduce_splits_kernel(const float* __restrict__ partial, int splits, long long all, int M, int N,
-                                                            const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ c,
-                                                            long long ldc, long long c_batch_stride, bool accumulate) {
+struct Sum {
+  const float* partial;
+  const __nv_bfloat16* bias;
+  __nv_bfloat16* c;
+  long long all, ldc, c_batch_stride;   // all: elements
+  int splits, M, N, first_block;
+  bool accumulate;
+};
+template <int kCount>
+struct Sums {
+  Sum sum[kCount];
+  int count;
+};
+template <int kParts, int kVec, int kCount>
+__global__ void __launch_bounds__(256) reduce_splits_kernel(const __grid_constant__ Sums<kCount> sums) {
   enter_kernel();
   constexpr int kLanes = 256 / kParts;
   __shared__ float red[kParts > 1 ? kParts : 1][kLanes][kVec];
+  int q = 0;
+  if (kCount > 1)
+    while (q + 1 < sums.count && static_cast<int>(blockIdx.x) >= sums.sum[q + 1].first_block) ++q;
+  const Sum& p = sums.sum[q];
   const int tx = threadIdx.x % kLanes, ty = threadIdx.x / kLanes;
-  const long long i = (static_cast<long long>(blockIdx.x) * kLanes + tx) * kVec;
+  const long long i = (static_cast<long long>(blockIdx.x - p.first_block) * kLanes + tx) * kVec;
   float v[kVec] = {};
-  if (i < all) {
-    const float* const from = partial + i;
+  if (i < p.all) {
+    const float* const from = p.partial + i;
 #pragma unroll 8
-    for (int k = ty; k < splits; k += kParts) {
+    for (int k = ty; k < p.splits; k += kParts) {
       if constexpr (kVec == 4) {
-        const float4 u = *reinterpret_cast<const float4*>(from + k * all);
+        const float4 u = *reinterpret_cast<const float4*>(from + k * p.all);
         v[0] += u.x; v[1] += u.y; v[2] += u.z; v[3] += u.w;
       } else {
-        v[0] += from[k * all];
+        v[0] += from[k * p.all];
       }
     }
   }
@@ -253,25 +297,46 @@ __global__ void __launch_bounds__(256) reduce_splits_kernel(const float* __restr
 #pragma unroll
       for (int e = 0; e < kVec; ++e) v[e] += red[k][tx][e];
   }
-  if (i >= all) return;
-  const int n = static_cast<int>(i % N);
-  const long long row = i / N;
-  __nv_bfloat16* const dst = c + row / M * c_batch_stride + row % M * ldc + n;
+  if (i >= p.all) return;
+  const int n = static_cast<int>(i % p.N);
+  const long long row = i / p.N;
+  __nv_bfloat16* const dst = p.c + row / p.M * p.c_batch_stride + row % p.M * p.ldc + n;
 #pragma unroll
   for (int e = 0; e < kVec; ++e) {
-    if (bias) v[e] += __bfloat162float(bias[n + e]);
-    if (accumulate) v[e] += __bfloat162float(dst[e]);
+    if (p.bias) v[e] += __bfloat162float(p.bias[n + e]);
+    if (p.accumulate) v[e] += __bfloat162float(dst[e]);
   }
   if constexpr (kVec == 4) *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]));
   else *dst = __float2bfloat16(v[0]);
 }
-template <int kParts>
-void reduce_splits(const Params& p, cudaStream_t stream) {
-  const long long all = static_cast<long long>(p.batch) * p.M * p.N;
-  const bool vec = p.N % 4 == 0 && p.ldc % 4 == 0 && p.c_batch_stride % 4 == 0 && reinterpret_cast<uintptr_t>(p.c) % 8 == 0;
-  const long long per_block = 256 / kParts * (vec ? 4 : 1);
-  mxk::launch_kernel(vec ? reduce_splits_kernel<kParts, 4> : reduce_splits_kernel<kParts, 1>, static_cast<unsigned>((all + per_block - 1) / per_block), 256, 0, stream, p.partial, p.splits, all,
-                     p.M, p.N, p.bias, p.c, p.ldc, p.c_batch_stride, p.accumulate);
+
+bool by_fours(const Problem& p) { return p.N % 4 == 0 && p.ldc % 4 == 0 && p.c_batch_stride % 4 == 0 && reinterpret_cast<uintptr_t>(p.c) % 8 == 0; }
+
+template <int kParts, int kVec, int kCount>
+void launch_sums(const Params<kCount>& params, cudaStream_t stream) {
+  Sums<kCount> sums{};
+  long long blocks = 0;
+  for (int i = 0; i < params.count; ++i) {
+    const Problem& p = params.problem[i];
+    if (p.splits == 1) continue;
+    const long long all = static_cast<long long>(p.batch) * p.M * p.N;
+    sums.sum[sums.count++] = {p.partial, p.bias, p.c, all, p.ldc, p.c_batch_stride, p.splits, p.M, p.N, static_cast<int>(blocks), p.accumulate};
+    blocks += (all + 256 / kParts * kVec - 1) / (256 / kParts * kVec);
+  }
+  mxk::launch_kernel(reduce_splits_kernel<kParts, kVec, kCount>, static_cast<unsigned>(blocks), 256, 0, stream, sums);
+}
+template <int kCount>
+void reduce_splits(const Params<kCount>& params, cudaStream_t stream) {
+  int most = 1;
+  bool fours = true;
+  for (int i = 0; i < params.count; ++i)
+    if (params.problem[i].splits > 1) {
+      most = std::max(most, params.problem[i].splits);
+      fours &= by_fours(params.problem[i]);
+    }
+  if (most == 1) return;
+  if (fours) most > 8 ? launch_sums<8, 4>(params, stream) : launch_sums<1, 4>(params, stream);
+  else most > 8 ? launch_sums<8, 1>(params, stream) : launch_sums<1, 1>(params, stream);
 }
 
 // Narrow tiles where wide ones would leave SMs idle; a contraction is split when even those do and each part still has
@@ -303,17 +368,58 @@ bool encode(CUtensorMap* map, const Matrix& m, int cols, int rows, int batch, in
              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int BN, bool A_ROWS, bool B_ROWS>
-int launch(const Params& p, cudaStream_t stream) {
-  if (const int st = allow_smem<gemm16_kernel<BN, A_ROWS, B_ROWS>, Layout<BN>::kBytes>(); st != MXK_OK) return st;
-  const long long tiles = static_cast<long long>((p.M + kBM - 1) / kBM) * ((p.N + BN - 1) / BN) * p.batch * p.splits;
-  mxk::launch_kernel(gemm16_kernel<BN, A_ROWS, B_ROWS>, static_cast<unsigned>(min(tiles, static_cast<long long>(kNumSMs))), kThreads, Layout<BN>::kBytes, stream, p);
+template <int BN, bool A_ROWS, bool B_ROWS, int kCount>
+int launch(const Params<kCount>& p, cudaStream_t stream) {
+  if (const int st = allow_smem<gemm16_kernel<BN, A_ROWS, B_ROWS, kCount>, Layout<BN>::kBytes>(); st != MXK_OK) return st;
+  mxk::launch_kernel(gemm16_kernel<BN, A_ROWS, B_ROWS, kCount>, static_cast<unsigned>(std::min(p.tiles, kNumSMs)), kThreads, Layout<BN>::kBytes, stream, p);
   return launch_status();
 }
-template <int BN>
-int launch_bn(const Params& p, bool a_rows, bool b_rows, cudaStream_t s) {
+template <int BN, int kCount>
+int launch(const Params<kCount>& p, bool a_rows, bool b_rows, cudaStream_t s) {
   if (a_rows) return b_rows ? launch<BN, true, true>(p, s) : launch<BN, true, false>(p, s);
   return b_rows ? launch<BN, false, true>(p, s) : launch<BN, false, false>(p, s);
+}
+
+// What a launch is told of a job; MXK_OK, or what is wrong with it.
+int fill(Problem& p, const Job& j, bool a_rows, bool b_rows, const Plan& pl, float* partial) {
+  if (!j.a.ptr || !j.b.ptr || !j.c) return MXK_ERR_NULL;
+  if (j.batch <= 0 || j.M <= 0 || j.N <= 0 || j.K <= 0) return MXK_ERR_DIMS;
+  if (!aligned16(j.a.ptr) || !aligned16(j.b.ptr) || j.a.ld % 8 || j.b.ld % 8 || j.a.batch_stride % 8 || j.b.batch_stride % 8) return MXK_ERR_ALIGN;
+  if (!encode(&p.map_a, j.a, a_rows ? j.M : j.K, a_rows ? j.K : j.M, j.batch, a_rows ? kBK : kBM) ||
+      !encode(&p.map_b, j.b, b_rows ? j.N : j.K, b_rows ? j.K : j.N, j.batch, b_rows ? kBK : pl.bn))
+    return MXK_ERR_UNSUPPORTED;
+  p.c = static_cast<__nv_bfloat16*>(j.c);
+  p.bias = static_cast<const __nv_bfloat16*>(j.bias);
+  p.partial = partial;
+  p.ldc = j.ldc;
+  p.c_batch_stride = j.c_batch_stride;
+  p.batch = j.batch; p.M = j.M; p.N = j.N; p.K = j.K;
+  p.k_split = pl.k_split; p.splits = pl.splits;
+  p.accumulate = j.accumulate;
+  const auto rows_on = [&](int elements) { return reinterpret_cast<uintptr_t>(j.c) % (2 * elements) == 0 && j.ldc % elements == 0 && j.c_batch_stride % elements == 0; };
+  p.vec = rows_on(16) ? 16 : rows_on(8) ? 8 : 1;
+  return MXK_OK;
+}
+int tiles_of(const Job& j, int bn) { return (j.M + kBM - 1) / kBM * ((j.N + bn - 1) / bn) * j.batch; }
+int steps_of(const Job& j) { return (j.K + kBK - 1) / kBK; }
+size_t partial_floats(const Job& j, const Plan& pl) { return pl.splits > 1 ? (static_cast<size_t>(pl.splits) * j.batch * j.M * j.N + 7) / 8 * 8 : 0; }
+
+// The most steps of a tile's contraction in a launch of several problems: those with which the SMs' rounds of tiles take the fewest
+// (three more for a tile's begin and end).
+Plan plan_in_group(const Job* jobs, int count, int i) {
+  int longest = 1;
+  for (int q = 0; q < count; ++q) longest = std::max(longest, steps_of(jobs[q]));
+  long long best = -1;
+  int cap = longest;
+  for (int n = 1; n <= 32 && longest / n >= 4; ++n) {
+    const int steps = (longest + n - 1) / n;
+    long long tiles = 0;
+    for (int q = 0; q < count; ++q) tiles += static_cast<long long>(tiles_of(jobs[q], 64)) * ((steps_of(jobs[q]) + steps - 1) / steps);
+    const long long cost = (tiles + kNumSMs - 1) / kNumSMs * (steps + 3);
+    if (best < 0 || cost < best) { best = cost; cap = steps; }
+  }
+  const int steps = steps_of(jobs[i]), parts = (steps + cap - 1) / cap, per = (steps + parts - 1) / parts;
+  return {64, (steps + per - 1) / per, per * kBK};
 }
 
 }  // namespace
@@ -324,33 +430,44 @@ size_t workspace_bytes(int batch, int M, int N, int K) {
   return pl.splits > 1 ? static_cast<size_t>(pl.splits) * batch * M * N * sizeof(float) : 0;
 }
 
-int run(const Matrix& a, bool a_rows, const Matrix& b, bool b_rows, const void* bias, void* c, long long ldc,
-        long long c_batch_stride, bool accumulate, int batch, int M, int N, int K, void* ws, size_t ws_bytes, int* status,
-        cudaStream_t stream) {
-  if (!a.ptr || !b.ptr || !c) return MXK_ERR_NULL;
-  if (batch <= 0 || M <= 0 || N <= 0 || K <= 0) return MXK_ERR_DIMS;
-  if (!aligned16(a.ptr) || !aligned16(b.ptr) || a.ld % 8 || b.ld % 8 || a.batch_stride % 8 || b.batch_stride % 8) return MXK_ERR_ALIGN;
-  const Plan pl = plan(batch, M, N, K);
-  if (pl.splits > 1 && (!ws || reinterpret_cast<uintptr_t>(ws) % 32 || ws_bytes < workspace_bytes(batch, M, N, K))) return MXK_ERR_WORKSPACE;
-  Params p{};
-  if (!encode(&p.map_a, a, a_rows ? M : K, a_rows ? K : M, batch, a_rows ? kBK : kBM) ||
-      !encode(&p.map_b, b, b_rows ? N : K, b_rows ? K : N, batch, b_rows ? kBK : pl.bn))
-    return MXK_ERR_UNSUPPORTED;
-  p.c = static_cast<__nv_bfloat16*>(c);
-  p.bias = static_cast<const __nv_bfloat16*>(bias);
-  p.partial = static_cast<float*>(ws);
-  p.ldc = ldc;
-  p.c_batch_stride = c_batch_stride;
-  p.batch = batch; p.M = M; p.N = N; p.K = K;
-  p.k_split = pl.k_split; p.splits = pl.splits;
-  p.accumulate = accumulate;
-  const auto rows_on = [&](int elements) { return reinterpret_cast<uintptr_t>(c) % (2 * elements) == 0 && ldc % elements == 0 && c_batch_stride % elements == 0; };
-  p.vec = rows_on(16) ? 16 : rows_on(8) ? 8 : 1;
+int run(const Job& job, bool a_rows, bool b_rows, void* ws, size_t ws_bytes, int* status, cudaStream_t stream) {
+  if (job.batch <= 0 || job.M <= 0 || job.N <= 0 || job.K <= 0) return MXK_ERR_DIMS;
+  const Plan pl = plan(job.batch, job.M, job.N, job.K);
+  if (pl.splits > 1 && (!ws || reinterpret_cast<uintptr_t>(ws) % 32 || ws_bytes < workspace_bytes(job.batch, job.M, job.N, job.K))) return MXK_ERR_WORKSPACE;
+  Params<1> p{};
+  if (const int st = fill(p.problem[0], job, a_rows, b_rows, pl, static_cast<float*>(ws)); st != MXK_OK) return st;
+  p.count = 1;
+  p.tiles = tiles_of(job, pl.bn) * pl.splits;
   p.status = status;
-  const int st = pl.bn == 128 ? launch_bn<128>(p, a_rows, b_rows, stream) : launch_bn<64>(p, a_rows, b_rows, stream);
-  if (st != MXK_OK || pl.splits == 1) return st;
-  if (pl.splits > 8) reduce_splits<8>(p, stream);
-  else reduce_splits<1>(p, stream);
+  if (const int st = pl.bn == 128 ? launch<128>(p, a_rows, b_rows, stream) : launch<64>(p, a_rows, b_rows, stream); st != MXK_OK) return st;
+  reduce_splits(p, stream);
+  return launch_status();
+}
+
+size_t group_workspace_bytes(const Job* jobs, int count) {
+  size_t floats = 0;
+  for (int i = 0; i < count; ++i) floats += partial_floats(jobs[i], plan_in_group(jobs, count, i));
+  return floats * sizeof(float);
+}
+
+int run_group(const Job* jobs, int count, bool a_rows, bool b_rows, void* ws, size_t ws_bytes, int* status, cudaStream_t stream) {
+  if (count < 1 || count > kMaxGroup) return MXK_ERR_DIMS;
+  for (int i = 0; i < count; ++i)
+    if (jobs[i].batch <= 0 || jobs[i].M <= 0 || jobs[i].N <= 0 || jobs[i].K <= 0) return MXK_ERR_DIMS;
+  if (const size_t need = group_workspace_bytes(jobs, count); need && (!ws || reinterpret_cast<uintptr_t>(ws) % 32 || ws_bytes < need)) return MXK_ERR_WORKSPACE;
+  Params<kMaxGroup> p{};
+  float* partial = static_cast<float*>(ws);
+  for (int i = 0; i < count; ++i) {
+    const Plan pl = plan_in_group(jobs, count, i);
+    if (const int st = fill(p.problem[i], jobs[i], a_rows, b_rows, pl, partial); st != MXK_OK) return st;
+    partial += partial_floats(jobs[i], pl);
+    p.problem[i].first_tile = p.tiles;
+    p.tiles += tiles_of(jobs[i], 64) * pl.splits;
+  }
+  p.count = count;
+  p.status = status;
+  if (const int st = launch<64>(p, a_rows, b_rows, stream); st != MXK_OK) return st;
+  reduce_splits(p, stream);
   return launch_status();
 }
 

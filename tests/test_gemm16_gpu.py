@@ -55,3 +55,22 @@ def test_sums_into_rows_at_any_address(n, ld, at, k):
     rest[at:].view(130, ld)[:, :n] = False
     assert torch.equal(held[rest], before[rest])
     ops.check_status()
+
+
+# several products in one launch: of one size and of very different ones, batched and not, split and whole
+@pytest.mark.parametrize("tokens", [5, 700, 6000])
+@pytest.mark.parametrize("by_rows", [False, True])
+def test_products_that_share_a_launch(tokens, by_rows):
+    from memorax_b200 import _C, ops
+    g = torch.Generator("cuda").manual_seed(tokens)
+    mk = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    if by_rows:   # gradients of weights: both contracted over their rows
+        a, b = [mk(tokens, 264).t(), mk(3, tokens, 72).transpose(1, 2), mk(tokens, 8).t(), mk(tokens, 128).t()], [mk(tokens, 136), mk(3, tokens, 40), mk(tokens, 768), mk(tokens, 64)]
+    else:
+        a, b = [mk(4, tokens, 64), mk(4, tokens, 64), mk(tokens, 520)], [mk(4, 128, 64).transpose(1, 2), mk(4, 64, 64).transpose(1, 2), mk(96, 520).t()]
+    c = [torch.empty(*x.shape[:-1], y.shape[-1], device="cuda", dtype=torch.bfloat16) for x, y in zip(a, b)]
+    _C.products_bf16(a, b, c)
+    for x, y, got in zip(a, b, c):
+        want = x.double() @ y.double()
+        assert float((got.double() - want).norm() / want.norm()) <= 4e-3
+    ops.check_status()
