@@ -456,9 +456,9 @@ int reduce_splits(const float* partial, int splits, int M, int N, float* c, long
   return launch_status();
 }
 
-// Products with a weight of more than this many k go to gemm32_f16.cu, half the work of the tensor cores: 131 against 184 us at
+// Products with a weight of more than this many k go to gemm32_f16.cu, half the work of the tensor cores: 121 against 184 us at
 // 65536 x 1024 x 256.  Below, three bf16 planes are the more precise form: errors against float64 at K = 64 / 128 / 256 with normal
-// entries 0.7 / 1.2 / 2.3e-7, of two float16 planes 1.35 / 1.4 / 1.4e-7.
+// entries 0.7 / 1.2 / 2.3e-7, of two float16 planes 1.35 / 1.4 / 1.8e-7.
 constexpr int kShortK = 255;
 __host__ __device__ constexpr bool two_planes(int K) { return K > kShortK; }
 

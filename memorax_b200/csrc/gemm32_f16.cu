@@ -11,10 +11,11 @@
 // times as large: full precision down to 2^-23 of the largest element, and an error of 2^-44 of it below that.
 //
 // Precision: the tensor core truncates when it adds to a float32 accumulator (3e-8 of the sum per addition of 16 k), so the hi*hi
-// accumulator lives for one stage of 64 k, two in contractions from 384 on, and is summed up in float32 registers; the two small
-// products have an accumulator of their own, whose truncations are 2^-11 as large, for the whole tile.  Errors against float64,
-// relative 2-norm (three bf16 planes, drained every 512 k, in brackets; below 256 k they are the more precise form):
-//   4096 x 1024 x 256     normal entries 1.4e-7 (2.3e-7)   lognormal, sigma 3: 1.5e-7 (3.3e-7)
+// accumulator lives for one stage of 64 k, two at a tile's begin (under the stores of the tile before: 129 -> 121 us at 65536 x 1024
+// x 256) and in contractions from 384 on, and is summed up in float32 registers; the two small products have an accumulator of their
+// own, whose truncations are 2^-11 as large, for the whole tile.  Errors against float64, relative 2-norm (three bf16 planes, drained
+// every 512 k, in brackets; below 256 k they are the more precise form):
+//   4096 x 1024 x 256     normal entries 1.8e-7 (2.3e-7)   lognormal, sigma 3: 1.5e-7 (3.3e-7)
 //   4096 x 256 x 512                     2.1e-7 (4.7e-7)                       1.2e-7 (6.1e-7)
 //   4096 x 256 x 1024                    2.1e-7 (4.7e-7)                       1.4e-7 (4.5e-7)
 //
@@ -28,8 +29,8 @@
 //   1 warp     issues the MMAs (12 per stage of 64 k), 1 warp the copies of the weight's image, 1 warp those of A (TMA)
 // Registers are dealt out by setmaxnreg: a thread of the epilogue holds up to 128 sums.  (A loaded straight from global memory
 // into the producers' registers: 142 us at 65536 x 256 x 1024, its loads then wait for room in an L1 of 28 KB.)
-// Measured, without the splitting of the weight (three bf16 planes before): 65536 x 1024 x 256 131 us (184), 65536 x 256 x 1024
-// 102 us (173), 24000 x 1024 x 512 90 us (126), 65536 x 128 x 256 29 us (40).
+// Measured, without the splitting of the weight (three bf16 planes before): 65536 x 1024 x 256 121 us (184), 65536 x 256 x 1024
+// 103 us (173), 24000 x 1024 x 512 89 us (126), 65536 x 128 x 256 28 us (40).
 #include <algorithm>
 
 #include "gemm32_common.cuh"
@@ -43,6 +44,7 @@ namespace {
 using namespace umma;
 
 constexpr int kLongRuns = 384; // from here on the hi*hi accumulator lives for two stages
+constexpr int kFirstRun = 2;   // and always a tile's first: the epilogue is still at the tile before
 
 struct Params {
   CUtensorMap map_a;     // kWide: boxes of 128 rows x 32 k
@@ -57,7 +59,7 @@ struct Params {
   int M, N, K;
   int k_split;           // k per split (a multiple of kBK)
   int splits;            // more than one: c is [splits][M][N]
-  int run;               // stages that the hi*hi accumulator lives for
+  int run;               // stages that the hi*hi accumulator lives for after a tile's first run
   Epilogue ep;           // of a contraction that is not split
   int* status;
 };
@@ -85,6 +87,20 @@ struct Config {
   static constexpr int kThreads = 32 * (kMmaWarp + 4);   // warpgroups deal registers: 640 threads of 96
   static constexpr int kRegsEpilogue = BN == 256 ? 168 : 152, kRegsProducer = BN == 256 ? 56 : 64, kRegsMma = BN == 256 ? 32 : 48;
   static_assert(kEpilogueWarps * kRegsEpilogue + kProducerWarps * kRegsProducer + 4 * kRegsMma == kThreads / 32 * 96, "the launch's registers");
+};
+
+// The tiles of a CTA (pair), one after the other: `n` fastest, then `m`, then the split.  (Taken apart by divisions for every tile, the
+// coordinates cost the epilogue 1 to 3 %.)
+struct Walk {
+  int n, m, sp;
+  int step_n, step_m, step_sp;
+  __device__ __forceinline__ Walk(int first, int step, int nt, int mt)
+      : n(first % nt), m(first / nt % mt), sp(first / nt / mt), step_n(step % nt), step_m(step / nt % mt), step_sp(step / nt / mt) {}
+  __device__ __forceinline__ void next(int nt, int mt) {
+    n += step_n; m += step_m; sp += step_sp;
+    if (n >= nt) { n -= nt; ++m; }
+    if (m >= mt) { m -= mt; ++sp; }
+  }
 };
 
 // kWide: rows of A begin on 16-byte boundaries; where they do not, the producers read them element by element.  kEp: something is
@@ -138,10 +154,7 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
   const uint32_t tmem = *tmem_slot;
   bool timed_out = false;
   const auto wait = [&](uint64_t* bar, uint32_t parity) { mbar_wait_flag(bar, parity, timed_out); };
-  const auto k_length = [&](int tile) {
-    const int sp = tile / (mt * nt);
-    return min(p.K, (sp + 1) * p.k_split) - sp * p.k_split;
-  };
+  const auto k_length = [&](const Walk& at) { return min(p.K - at.sp * p.k_split, p.k_split); };
   // Whether a row of the tile begins a new unit at this stage; the same in both CTAs.  (Read after a barrier that the producers'
   // arrivals of the stage lead to; a slot is written again only when its stage has been drained.)
   const auto event_at = [&](int turn) { return *const_cast<volatile uint32_t*>(events + turn % kSlots) == turn + 1u; };
@@ -153,10 +166,9 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
     const int col0 = (warp >> 2) * (BN / 2), row0 = (warp & 3) * 32 + (lane >> 2);   // this thread: rows row0 + 8 i
     float sum[kChunks][4][8];          // columns 32 c + 8 (lane % 4) + e
     int turn = 0, main_turn = 0, low_turn = 0;   // stages, accumulators
-    for (int tile = first_tile; tile < tiles; tile += tile_step) {
-      const int mn = tile % (mt * nt), sp = tile / (mt * nt);
-      const int n0 = (mn % nt) * BN + col0, m0 = (mn / nt) * kTileM + rank * kBM + row0;
-      const int k_len = k_length(tile);
+    Walk at(first_tile, tile_step, nt, mt);
+    for (int tile = first_tile; tile < tiles; tile += tile_step, at.next(nt, mt)) {
+      const int sp = at.sp, n0 = at.n * BN + col0, m0 = at.m * kTileM + rank * kBM + row0, k_len = k_length(at);
       int unit[4] = {};   // of the rows' sums: 2^unit
       int4 unit_w = make_int4(0, 0, 0, 0);   // of four of W's rows a lane, for the end of the tile
       if (lane < BN / 8) unit_w = __ldg(reinterpret_cast<const int4*>(p.unit_w + n0) + lane);
@@ -208,7 +220,7 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
           ++main_turn;
           drained = false;
           // the run's stages: one where an event began it, fewer than p.run where one ended it
-          const int most = seg > 0 && event_at(turn) ? 1 : p.run;
+          const int most = seg == 0 ? kFirstRun : event_at(turn) ? 1 : p.run;
           int n = 0;
           do {
             ++n;
@@ -307,14 +319,15 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
     int stage = 0, raw = 0, turn = 0;
     uint32_t parity = 1, raw_parity = 0;   // a fresh barrier's previous phase counts as complete
     int unit[2] = {};             // of this lane's rows
-    for (int tile = first_tile; tile < tiles; tile += tile_step) {
-      const int k_len = k_length(tile);
+    Walk at(first_tile, tile_step, nt, mt);
+    for (int tile = first_tile; tile < tiles; tile += tile_step, at.next(nt, mt)) {
+      const int k_len = k_length(at);
 #pragma unroll 1
       for (int seg = 0; seg < k_len; seg += kBK, ++turn) {
         float x[2][2][8];
         if (kWide) wait(&raw_full[raw], raw_parity);
         const uint8_t* const src = smem + L::kRawAt + raw * L::kRaw + r0 * 128;
-        const int m = tile % (mt * nt) / nt * kTileM + rank * kBM + r0, k = tile / (mt * nt) * p.k_split + seg + (lane >> 3) * 8;
+        const int m = at.m * kTileM + rank * kBM + r0, k = at.sp * p.k_split + seg + (lane >> 3) * 8;
 #pragma unroll
         for (int g = 0; g < 2; ++g)
 #pragma unroll
@@ -392,10 +405,11 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
       const auto done = [&](uint64_t* bar) {
         if (leader) (kPair ? commit_pair : commit)(bar);
       };
-      for (int tile = first_tile; tile < tiles; tile += tile_step) {
-        const int k_len = k_length(tile);
+      Walk at(first_tile, tile_step, nt, mt);
+      for (int tile = first_tile; tile < tiles; tile += tile_step, at.next(nt, mt)) {
+        const int k_len = k_length(at);
         bool low_open = false;
-        int run = 0;   // stages in the hi*hi accumulator
+        int run = 0, most = 0;   // stages in the hi*hi accumulator, and how many it takes
         for (int seg = 0; seg < k_len; seg += kBK, ++turn) {
           wait(&full[stage], parity);
           if (kPair && rank != 0) {   // the other CTA issues
@@ -426,12 +440,15 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
           };
           const int set = main_turn % kSets;
           const uint32_t acc = tmem + set * 2 * BN, low = tmem + (low_turn % kSets) * 2 * BN + BN;
-          if (run == 0) wait(&main_empty[set], ((main_turn / kSets) & 1) ^ 1);
+          if (run == 0) {
+            // (a run that an event begins is one stage: the epilogue learns of the event by its end, and until it has drained the
+            // small products' accumulator the next one cannot be begun)
+            most = seg == 0 ? kFirstRun : event ? 1 : p.run;
+            wait(&main_empty[set], ((main_turn / kSets) & 1) ^ 1);
+          }
           fence_after_sync();
           product(acc, a0, b0, run > 0);
-          // (a run that an event begins is one stage: the epilogue learns of the event by its end, and until it has drained the
-          // small products' accumulator the next one cannot be begun)
-          if (++run == p.run || event || seg + kBK >= k_len) {
+          if (++run == most || seg + kBK >= k_len) {
             done(&main_full[set]);
             ++main_turn;
             run = 0;
@@ -459,8 +476,9 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
       const int k_images = (p.K + kBK - 1) / kBK;
       int stage = 0;
       uint32_t parity = 1;
-      for (int tile = first_tile; tile < tiles; tile += tile_step) {
-        const int n0 = (tile % nt) * BN + rank * kRowsB, k0 = tile / (mt * nt) * p.k_split, k_len = k_length(tile);
+      Walk at(first_tile, tile_step, nt, mt);
+      for (int tile = first_tile; tile < tiles; tile += tile_step, at.next(nt, mt)) {
+        const int n0 = at.n * BN + rank * kRowsB, k0 = at.sp * p.k_split, k_len = k_length(at);
         const uint8_t* image = p.image + (static_cast<size_t>(n0 / kRowsB) * k_images + k0 / kBK) * (2 * L::kPlaneB);
         for (int seg = 0; seg < k_len; seg += kBK, image += 2 * L::kPlaneB) {
           wait(&empty[stage], parity);
@@ -473,8 +491,9 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
       // ---------------------------------------------------------- float32 tiles of A
       int raw = 0;
       uint32_t parity = 1;
-      for (int tile = first_tile; tile < tiles; tile += tile_step) {
-        const int m0 = tile % (mt * nt) / nt * kTileM + rank * kBM, k0 = tile / (mt * nt) * p.k_split, k_len = k_length(tile);
+      Walk at(first_tile, tile_step, nt, mt);
+      for (int tile = first_tile; tile < tiles; tile += tile_step, at.next(nt, mt)) {
+        const int m0 = at.m * kTileM + rank * kBM, k0 = at.sp * p.k_split, k_len = k_length(at);
         for (int seg = 0; seg < k_len; seg += kBK) {
           wait(&raw_empty[raw], parity);
           uint8_t* const dst = smem + L::kRawAt + raw * L::kRaw;
