@@ -94,42 +94,64 @@ __global__ void __launch_bounds__(128) lru_step_read_kernel(LruWeights w, const 
 
 constexpr int kSkipBlocks = 4 * kNumSMs;
 
-// HBM-bound: one read of both operands; a block takes every gridDim.x-th group of rows, its threads the columns.  Four blocks
-// an SM with eight rows of both operands in flight per thread are the 64 KiB that HBM wants outstanding (16 KiB: 45 us for
-// 65536 x 256).
-constexpr int kSkipRows = 8;
+// HBM-bound: one read of both operands; a block takes every gridDim.x-th group of rows, its threads the columns, kVec of them each.
+// Four blocks an SM with four rows of both operands as 16-byte vectors under way per thread are 128 KiB, the last rows among them
+// (65536 x 256: 25 us; eight rows of single elements and the remainder one by one: 42).
+template <int kVec>
 __global__ void __launch_bounds__(256) skip_grad_kernel(const float* __restrict__ gy, const float* __restrict__ x,
                                                         float* __restrict__ partial, long long rows, int F) {
   enter_kernel();
-  __shared__ float sums[256];
-  const int per = F < 256 ? 256 / F : 1;   // rows side by side in a block
-  const int width = min(F, 256);
+  constexpr int kRows = kVec == 4 ? 4 : 8;
+  __shared__ float sums[256][kVec];
+  const int vectors = F / kVec, width = min(vectors, 256);
+  const int per = 256 / width;   // rows side by side in a block
   const int ro = threadIdx.x / width, ct = threadIdx.x % width;
-  for (int c0 = 0; c0 < F; c0 += 256) {
-    const int c = c0 + ct;
-    float s[4] = {0.f, 0.f, 0.f, 0.f};
-    if (ro < per && c < F) {
+  const auto load = [](const float* p, float* v) {
+    if constexpr (kVec == 4) {
+      const float4 u = ld_stream(reinterpret_cast<const float4*>(p));
+      v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w;
+    } else {
+      v[0] = ld_stream(p);
+    }
+  };
+  for (int c0 = 0; c0 < vectors; c0 += 256) {
+    const int c = (c0 + ct) * kVec;
+    float s[2][kVec] = {};
+    if (ro < per && c0 + ct < vectors) {
       const long long step = static_cast<long long>(gridDim.x) * per;
       long long r = static_cast<long long>(blockIdx.x) * per + ro;
-      for (; r + (kSkipRows - 1) * step < rows; r += kSkipRows * step) {
-        float a[kSkipRows], b[kSkipRows];
+      const float *pg = gy + r * F + c, *px = x ? x + r * F + c : nullptr;
+      for (; r < rows; r += kRows * step, pg += kRows * step * F) {
+        float a[kRows][kVec], b[kRows][kVec];
 #pragma unroll
-        for (int u = 0; u < kSkipRows; ++u) {
-          a[u] = ld_stream(gy + (r + u * step) * F + c);
-          b[u] = x ? ld_stream(x + (r + u * step) * F + c) : 1.f;
+        for (int u = 0; u < kRows; ++u) {
+          const bool in = r + u * step < rows;
+#pragma unroll
+          for (int e = 0; e < kVec; ++e) {
+            a[u][e] = 0.f;
+            b[u][e] = 1.f;
+          }
+          if (in) load(pg + u * step * F, a[u]);
+          if (in && px) load(px + u * step * F, b[u]);
         }
+        if (px) px += kRows * step * F;
 #pragma unroll
-        for (int u = 0; u < kSkipRows; ++u) s[u & 3] = fmaf(a[u], b[u], s[u & 3]);
+        for (int u = 0; u < kRows; ++u)
+#pragma unroll
+          for (int e = 0; e < kVec; ++e) s[u & 1][e] = fmaf(a[u][e], b[u][e], s[u & 1][e]);
       }
-      for (; r < rows; r += step) s[0] = fmaf(gy[r * F + c], x ? x[r * F + c] : 1.f, s[0]);
     }
     __syncthreads();
-    sums[threadIdx.x] = (s[0] + s[1]) + (s[2] + s[3]);
+#pragma unroll
+    for (int e = 0; e < kVec; ++e) sums[threadIdx.x][e] = s[0][e] + s[1][e];
     __syncthreads();
-    if (ro == 0 && c < F) {
-      float v = 0.f;
-      for (int i = 0; i < per; ++i) v += sums[i * width + ct];
-      partial[static_cast<size_t>(blockIdx.x) * F + c] = v;
+    if (ro == 0 && c0 + ct < vectors) {
+#pragma unroll
+      for (int e = 0; e < kVec; ++e) {
+        float v = 0.f;
+        for (int i = 0; i < per; ++i) v += sums[i * width + ct][e];
+        partial[static_cast<size_t>(blockIdx.x) * F + c + e] = v;
+      }
     }
   }
 }
@@ -425,7 +447,8 @@ int lru_step(const LruWeights& w, const float* x, const float* h0, const float* 
 int skip_grad_blocks(long long rows) { return static_cast<int>(rows < kSkipBlocks ? rows : kSkipBlocks); }
 
 int skip_grad(const float* gy, const float* x, float* partial, long long rows, int F, cudaStream_t stream) {
-  mxk::launch_kernel(skip_grad_kernel, skip_grad_blocks(rows), 256, 0, stream, gy, x, partial, rows, F);
+  const bool vectors = F % 4 == 0 && aligned16(gy) && (!x || aligned16(x));
+  mxk::launch_kernel(vectors ? skip_grad_kernel<4> : skip_grad_kernel<1>, skip_grad_blocks(rows), 256, 0, stream, gy, x, partial, rows, F);
   return launch_status();
 }
 

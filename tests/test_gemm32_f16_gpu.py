@@ -133,3 +133,16 @@ def test_layers_with_long_contractions(cell, feat, width):
     want = torch.autograd.grad(want_y, [xd, *p.values()], gy.double())
     for name, a, b in zip(["y", "x", *p], [y, *grads], [want_y, *want]):
         assert float((a.detach().double() - b).norm() / b.norm()) <= 2e-6, name
+
+
+# the skip weight's gradient: vectors and single columns, more columns than threads, remainders of the rows a block takes
+@pytest.mark.parametrize("tokens,feat", [(1, 4), (700, 3), (3000, 264), (5000, 256), (2500, 1028), (600, 1300)])
+def test_column_sums_of_products(tokens, feat):
+    from memorax_b200.memoroid import LRUCell, Memoroid
+    torch.manual_seed(tokens)
+    cell = LRUCell(feat, 8).cuda()
+    x, gy = torch.randn(1, tokens, feat, device="cuda"), torch.randn(1, tokens, feat, device="cuda")
+    _, y = Memoroid(cell)(x, torch.zeros(1, tokens, device="cuda"), None)
+    got, want = torch.autograd.grad(y, cell.D, gy)[0], (x.double() * gy.double()).sum((0, 1))
+    # (float32 sums in some order: at most 24 additions in a row at these sizes, each to 2^-24 of the terms' sum)
+    assert bool(((got.double() - want).abs() <= 24 * 2.0 ** -24 * (x.double() * gy.double()).abs().sum((0, 1))).all())
