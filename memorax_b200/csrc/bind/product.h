@@ -17,6 +17,10 @@ namespace mxk_host {
 // which costs gemm16 its wide stores); 32768 x 256, 4 heads of 64: 350 | 338 | 336 | 571.  mLSTM, 6016 x 256: 351 | 290 | 291 |
 // 289; 65536 x 512: 2586 | 2994 | 2950 | 3045 (the sums into existing tensors, which the line does not tell apart).
 constexpr double kLibraryFlops = 8e9;
+// The same for the gradient of a weight, whose long contraction the kernel splits over all SMs (GPU time alone, own | library in
+// microseconds): 256 x 256 over 65536 tokens 14 | 25, 768 x 256 over 32768 18 | 20, 512 x 512 over 32768 22 | 27, 1024 x 512 over 16384
+// 22 | 23, 128 x 1024 over 65536 32 | 32; beyond, 768 x 256 over 65536 37 | 32, 1024 x 512 over 32768 46 | 33.
+constexpr double kLibraryFlopsGradient = 1.75e10;
 
 // A product over the last two dimensions as the kernel's job; `fits`: whether it is one for the kernel.
 struct AsJob {
@@ -38,7 +42,7 @@ inline AsJob as_job(const Tensor& a, const Tensor& b, const Tensor& c, const Ten
   const auto fits = [&](const Tensor& t, const g::Matrix& m) {
     return (t.stride(r) == 1 || t.stride(q) == 1) && m.ld % 8 == 0 && m.batch_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(m.ptr) & 15) == 0;
   };
-  j.fits = 2.0 * batch * M * N * K <= kLibraryFlops && fits(a, ma) && fits(b, mb) && c.stride(q) == 1;
+  j.fits = 2.0 * batch * M * N * K <= (j.a_rows && j.b_rows ? kLibraryFlopsGradient : kLibraryFlops) && fits(a, ma) && fits(b, mb) && c.stride(q) == 1;
   j.job = {ma, mb, bias.defined() ? bias.data_ptr() : nullptr, c.data_ptr(), c.stride(r), n == 3 ? c.stride(0) : 0, accumulate,
            static_cast<int>(batch), static_cast<int>(M), static_cast<int>(N), static_cast<int>(K)};
   return j;
