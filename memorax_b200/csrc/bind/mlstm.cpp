@@ -36,11 +36,45 @@ Tensor heads(const Tensor& t, int at, const Shape& s) { return view_of(t, at, {s
 Tensor parts(const Tensor& t, int first, int count, const Shape& s) {
   return view_of(t, first * s.d, {s.H, s.M, count * s.d}, {3 * s.d, t.size(1), 1});
 }
-void* column(const Tensor& t, int c) { return static_cast<uint8_t*>(t.data_ptr()) + 2 * c; }
+// Buffers of one allocation: places in a bf16 tensor, on 512-byte boundaries (a layer of this many short launches waits for the host,
+// where a tensor of its own for each took 1 us to make and as much again to keep for the backward pass).
+struct Places {
+  int64_t used = 0;
+  int64_t take(int64_t elements) {
+    const int64_t at = used;
+    used += (elements + 255) / 256 * 256;
+    return at;
+  }
+  int64_t take_floats(int64_t n) { return take(2 * n); }
+  int64_t take_bytes(int64_t n) { return take((n + 1) / 2); }
+};
+void* column(const Tensor& t, int64_t c) { return static_cast<uint8_t*>(t.data_ptr()) + 2 * c; }
+float* floats(const Tensor& t, int64_t at) { return static_cast<float*>(column(t, at)); }
+
+// What the forward pass leaves for the backward pass.
+struct Kept {
+  int64_t up, u, qkv, qk_w, gates, logits, log_i, log_f, ks, h, g, m_steps, states, size;
+  Kept(const Shape& s, bool keep) {
+    Places at;
+    up = at.take(2ll * s.M * s.hid);
+    u = at.take(1ll * s.M * s.hid);
+    qkv = at.take(3ll * s.M * s.hid);
+    qk_w = at.take(2ll * s.hid * s.d);
+    gates = at.take(6ll * s.H * s.hid + 2 * s.H);
+    logits = at.take(2ll * s.M * s.H);
+    log_i = at.take_floats(1ll * s.M * s.H);
+    log_f = at.take_floats(1ll * s.M * s.H);
+    ks = at.take(1ll * s.M * s.hid);
+    h = at.take(1ll * s.M * s.hid);
+    g = at.take(1ll * s.M * s.hid);
+    m_steps = keep ? at.take_floats(1ll * s.M * s.H) : 0;
+    states = keep ? at.take_bytes(mxk_mlstm_bf16_chunk_states_bytes(s.B, s.T, s.H, s.d)) : 0;
+    size = at.used;
+  }
+};
 
 struct Result {
-  Tensor y, c_last, n_last, m_last, f_last;
-  Tensor up, u, qk_w, qkv, ks, gate_w, logits, log_i, log_f, h, g, m_steps, states;
+  Tensor y, c_last, n_last, m_last, f_last, kept;
 };
 
 Result forward(const Tensor& x, const variable_list& p, const Tensor& c0, const Tensor& n0, const Tensor& m0, const Tensor& f0, const Tensor& done,
@@ -52,37 +86,28 @@ Result forward(const Tensor& x, const variable_list& p, const Tensor& c0, const 
   r.n_last = empty_like_of(x, {s.B, 1, s.H, s.d, 1}, at::kFloat);
   r.m_last = empty_like_of(x, {s.B, 1, s.H, 1, 1}, at::kFloat);
   r.f_last = empty_like_of(x, {s.B, 1, s.H, 1, 1}, at::kFloat);
-  r.up = product(matrix(x, s.M, s.F), transposed(p[kUp]));
-  r.u = empty_like_of(x, {s.M, s.hid}, bf);
-  check("mlstm_conv_fwd", l::mlstm_conv_fwd(r.up.data_ptr(), 2 * s.hid, p[kConvW].data_ptr(), p[kConvB].data_ptr(), r.u.data_ptr(), s.B, s.T, s.hid, st));
-  r.qkv = empty_like_of(x, {s.M, 3 * s.hid}, bf);
+  const Kept at(s, keep);
+  const Tensor& all = r.kept = empty_like_of(x, {at.size}, bf);
+  const Tensor up = matrix(all, s.M, 2 * s.hid, 0, at.up), u = matrix(all, s.M, s.hid, 0, at.u), qkv = matrix(all, s.M, 3 * s.hid, 0, at.qkv),
+               g = matrix(all, s.M, s.hid, 0, at.g), qk_w = piece(all, at.qk_w, {s.H, 2 * s.d, s.d}), logits = matrix(all, s.M, 2 * s.H, 0, at.logits);
   const int64_t gate_w_size = 6ll * s.H * s.hid;
-  const Tensor gates = empty_like_of(x, {gate_w_size + 2 * s.H}, bf);
-  r.qk_w = empty_like_of(x, {s.H, 2 * s.d, s.d}, bf);
-  r.gate_w = piece(gates, 0, {2 * s.H, 3 * s.hid});
-  const Tensor gate_b = piece(gates, gate_w_size, {2 * s.H});
+  const Tensor gate_w = matrix(all, 2 * s.H, 3 * s.hid, 0, at.gates), gate_b = piece(all, at.gates + gate_w_size, {2 * s.H});
+  float *const log_i = floats(all, at.log_i), *const log_f = floats(all, at.log_f);
+  void *const ks = column(all, at.ks), *const h = column(all, at.h);
+  product_into(matrix(x, s.M, s.F), transposed(p[kUp]), up);
+  check("mlstm_conv_fwd", l::mlstm_conv_fwd(up.data_ptr(), 2 * s.hid, p[kConvW].data_ptr(), p[kConvB].data_ptr(), u.data_ptr(), s.B, s.T, s.hid, st));
   check("mlstm_weights", l::mlstm_weights(p[kQ].data_ptr(), p[kK].data_ptr(), p[kIW].data_ptr(), p[kFW].data_ptr(), p[kIB].data_ptr(), p[kFB].data_ptr(),
-                                          r.qk_w.data_ptr(), r.gate_w.data_ptr(), gate_b.data_ptr(), s.H, s.d, st));
-  products_into({{heads(r.u, 0, s), swapped(r.qk_w), parts(r.qkv, 0, 2, s)}, {heads(r.up, 0, s), swapped(p[kV]), parts(r.qkv, 2, 1, s)}});
-  r.logits = product(r.qkv, transposed(r.gate_w), gate_b);
-  r.log_i = empty_like_of(x, {s.M, s.H}, at::kFloat);
-  r.log_f = empty_like_of(x, {s.M, s.H}, at::kFloat);
-  r.ks = empty_like_of(x, {s.M, s.hid}, bf);
-  check("mlstm_gates_fwd", l::mlstm_gates_fwd(r.logits.data_ptr(), column(r.qkv, s.d), 3 * s.hid, 3 * s.d, s.scale(), ptr(r.log_i),
-                                              ptr(r.log_f), r.ks.data_ptr(), s.M, s.H, s.d, st));
-  r.h = empty_like_of(x, {s.M, s.hid}, bf);
-  if (keep) {
-    r.m_steps = empty_like_of(x, {s.M, s.H}, at::kFloat);
-    r.states = scratch(x, mxk_mlstm_bf16_chunk_states_bytes(s.B, s.T, s.H, s.d));
-  }
-  check("mxk_mlstm_bf16_fwd", mxk::mlstm_tc::forward(r.qkv.data_ptr(), r.ks.data_ptr(), column(r.qkv, 2 * s.d), 3 * s.hid, 3 * s.d, ptr(r.log_i), ptr(r.log_f), ptr(c0), ptr(n0),
-                                                     ptr(m0), ptr(f0), bytes(done), r.h.data_ptr(), ptr(r.c_last), ptr(r.n_last), ptr(r.m_last), ptr(r.f_last),
-                                                     ptr(r.m_steps), ptr<void>(r.states), status_ptr(x), s.B, s.T, s.H, s.d, eps, st));
-  r.g = empty_like_of(x, {s.M, s.hid}, bf);
-  check("mlstm_out_fwd", l::mlstm_out_fwd(r.h.data_ptr(), r.u.data_ptr(), column(r.up, s.hid), 2 * s.hid, p[kNorm].data_ptr(), p[kSkip].data_ptr(), r.g.data_ptr(), s.M,
+                                          qk_w.data_ptr(), gate_w.data_ptr(), gate_b.data_ptr(), s.H, s.d, st));
+  products_into({{heads(u, 0, s), swapped(qk_w), parts(qkv, 0, 2, s)}, {heads(up, 0, s), swapped(p[kV]), parts(qkv, 2, 1, s)}});
+  product_into(qkv, transposed(gate_w), logits, gate_b);
+  check("mlstm_gates_fwd", l::mlstm_gates_fwd(logits.data_ptr(), column(qkv, s.d), 3 * s.hid, 3 * s.d, s.scale(), log_i, log_f, ks, s.M, s.H, s.d, st));
+  check("mxk_mlstm_bf16_fwd", mxk::mlstm_tc::forward(qkv.data_ptr(), ks, column(qkv, 2 * s.d), 3 * s.hid, 3 * s.d, log_i, log_f, ptr(c0), ptr(n0),
+                                                     ptr(m0), ptr(f0), bytes(done), h, ptr(r.c_last), ptr(r.n_last), ptr(r.m_last), ptr(r.f_last),
+                                                     keep ? floats(all, at.m_steps) : nullptr, keep ? column(all, at.states) : nullptr, status_ptr(x), s.B, s.T, s.H, s.d, eps, st));
+  check("mlstm_out_fwd", l::mlstm_out_fwd(h, u.data_ptr(), column(up, s.hid), 2 * s.hid, p[kNorm].data_ptr(), p[kSkip].data_ptr(), g.data_ptr(), s.M,
                                           s.H, s.d, st));
   r.y = empty_like_of(x, {s.B, s.T, p[kOut].size(0)}, bf);
-  product_into(r.g, transposed(p[kOut]), matrix(r.y, s.M, p[kOut].size(0)));
+  product_into(g, transposed(p[kOut]), matrix(r.y, s.M, p[kOut].size(0)));
   return r;
 }
 
@@ -97,8 +122,7 @@ struct MlstmLayer : torch::autograd::Function<MlstmLayer> {
     ctx->saved_data["eps"] = eps;
     variable_list saved{x};
     saved.insert(saved.end(), p.begin(), p.end());
-    for (const Tensor& t : {c0, n0, m0, done, r.up, r.u, r.qkv, r.ks, r.gate_w, r.logits, r.log_i, r.log_f, r.h, r.g, r.m_steps, r.states, r.c_last, r.n_last, r.qk_w})
-      saved.push_back(t);
+    for (const Tensor& t : {c0, n0, m0, done, r.kept, r.c_last, r.n_last}) saved.push_back(t);
     ctx->save_for_backward(std::move(saved));
     ctx->mark_non_differentiable({r.f_last});
     return {r.c_last, r.n_last, r.m_last, r.f_last, r.y};
@@ -109,13 +133,18 @@ struct MlstmLayer : torch::autograd::Function<MlstmLayer> {
     const Tensor& x = v[0];
     const variable_list p(v.begin() + 1, v.begin() + 1 + kParams);
     const Tensor *t = &v[1 + kParams];
-    const Tensor &c0 = t[0], &n0 = t[1], &m0 = t[2], &done = t[3], &up = t[4], &u = t[5], &qkv = t[6], &ks = t[7], &gate_w = t[8], &logits = t[9], &log_i = t[10],
-                 &log_f = t[11], &h = t[12], &g = t[13], &m_steps = t[14], &states = t[15], &c_last = t[16], &n_last = t[17], &qk_w = t[18];
+    const Tensor &c0 = t[0], &n0 = t[1], &m0 = t[2], &done = t[3], &all = t[4], &c_last = t[5], &n_last = t[6];
     const c10::cuda::CUDAGuard guard(x.device());
     const Shape s = shape_of(x, p);
     const auto bf = at::kBFloat16;
     const auto st = stream();
     const int64_t out = p[kOut].size(0);
+    const Kept at_kept(s, true);
+    const auto rows = [&](const Tensor& in, int64_t at, int64_t cols) { return matrix(in, s.M, cols, 0, at); };
+    const Tensor up = rows(all, at_kept.up, 2 * s.hid), u = rows(all, at_kept.u, s.hid), qkv = rows(all, at_kept.qkv, 3 * s.hid), g = rows(all, at_kept.g, s.hid),
+                 qk_w = piece(all, at_kept.qk_w, {s.H, 2 * s.d, s.d}), gate_w = matrix(all, 2 * s.H, 3 * s.hid, 0, at_kept.gates);
+    float *const log_i = floats(all, at_kept.log_i), *const log_f = floats(all, at_kept.log_f);
+    void *const ks = column(all, at_kept.ks), *const h = column(all, at_kept.h), *const logits = column(all, at_kept.logits);
     const auto given = [&](int i) { return gout[i].defined() ? dense(gout[i]) : Tensor(); };
     const Tensor gc = given(0), gn = given(1), gm = given(2);
     const Tensor gy = matrix(gout[4].defined() ? dense(gout[4]) : empty_like_of(x, {s.M, out}, bf).zero_(), s.M, out);
@@ -129,23 +158,29 @@ struct MlstmLayer : torch::autograd::Function<MlstmLayer> {
       gn0 = empty_like_of(x, {s.B, 1, s.H, s.d, 1}, at::kFloat);
       gm0 = empty_like_of(x, {s.B, 1, s.H, 1, 1}, at::kFloat);
     }
-    const Tensor gg = product(gy, p[kOut]);
-    const Tensor gh = empty_like_of(x, {s.M, s.hid}, bf), gu = empty_like_of(x, {s.M, s.hid}, bf), gks = empty_like_of(x, {s.M, s.hid}, bf), gx = empty_like_of(x, {s.M, s.hid}, bf);
-    const Tensor gup = empty_like_of(x, {s.M, 2 * s.hid}, bf), gqkv = empty_like_of(x, {s.M, 3 * s.hid}, bf), glogits = empty_like_of(x, {s.M, 2 * s.H}, bf);
-    const Tensor gli = empty_like_of(x, {s.M, s.H}, at::kFloat), glf = empty_like_of(x, {s.M, s.H}, at::kFloat);
     const int out_rows = l::mlstm_out_blocks(s.M, s.hid), gate_rows = l::mlstm_gate_blocks(s.M), conv_rows = l::mlstm_conv_blocks(s.B, s.T, s.hid);
     const int cols[3] = {2 * s.hid, 2 * s.H, 5 * s.hid};
-    const Tensor part = empty_like_of(x, {static_cast<int64_t>(out_rows) * cols[0] + gate_rows * cols[1] + static_cast<int64_t>(conv_rows) * cols[2]}, at::kFloat);
-    float* const part_out = ptr(part);
+    const int64_t wide = static_cast<int64_t>(s.M) * s.hid, heads_all = static_cast<int64_t>(s.M) * s.H;
+    Places place;
+    const int64_t at_gg = place.take(wide), at_gh = place.take(wide), at_gu = place.take(wide), at_gks = place.take(wide), at_gx = place.take(wide), at_gup = place.take(2 * wide),
+                  at_gqkv = place.take(3 * wide), at_glogits = place.take(2 * heads_all), at_gli = place.take_floats(heads_all), at_glf = place.take_floats(heads_all),
+                  at_part = place.take_floats(static_cast<int64_t>(out_rows) * cols[0] + gate_rows * cols[1] + static_cast<int64_t>(conv_rows) * cols[2]);
+    const Tensor temp = empty_like_of(x, {place.used}, bf);
+    const Tensor gg = rows(temp, at_gg, s.hid), gu = rows(temp, at_gu, s.hid), gx = rows(temp, at_gx, s.hid), gup = rows(temp, at_gup, 2 * s.hid),
+                 gqkv = rows(temp, at_gqkv, 3 * s.hid), glogits = rows(temp, at_glogits, 2 * s.H);
+    void *const gh = column(temp, at_gh), *const gks = column(temp, at_gks);
+    float *const gli = floats(temp, at_gli), *const glf = floats(temp, at_glf);
+    float* const part_out = floats(temp, at_part);
     float* const part_gate = part_out + static_cast<size_t>(out_rows) * cols[0];
     float* const part_conv = part_gate + static_cast<size_t>(gate_rows) * cols[1];
-    check("mlstm_out_bwd", l::mlstm_out_bwd(gg.data_ptr(), h.data_ptr(), u.data_ptr(), column(up, s.hid), 2 * s.hid, p[kNorm].data_ptr(), p[kSkip].data_ptr(), gh.data_ptr(),
+    product_into(gy, p[kOut], gg);
+    check("mlstm_out_bwd", l::mlstm_out_bwd(gg.data_ptr(), h, u.data_ptr(), column(up, s.hid), 2 * s.hid, p[kNorm].data_ptr(), p[kSkip].data_ptr(), gh,
                                             column(gup, s.hid), 2 * s.hid, gu.data_ptr(), part_out, s.M, s.H, s.d, st));
-    check("mxk_mlstm_bf16_bwd", mxk::mlstm_tc::backward(qkv.data_ptr(), ks.data_ptr(), column(qkv, 2 * s.d), 3 * s.hid, 3 * s.d, ptr(log_i), ptr(log_f), ptr(c0), ptr(n0), ptr(m0),
-                                                        bytes(done), gh.data_ptr(), ptr(c_last), ptr(n_last), ptr(m_steps), states.data_ptr(), ptr(gc), ptr(gn), ptr(gm),
-                                                        gqkv.data_ptr(), gks.data_ptr(), column(gqkv, 2 * s.d), 3 * s.hid, 3 * s.d, ptr(gli), ptr(glf), ptr(gc0), ptr(gn0), ptr(gm0),
+    check("mxk_mlstm_bf16_bwd", mxk::mlstm_tc::backward(qkv.data_ptr(), ks, column(qkv, 2 * s.d), 3 * s.hid, 3 * s.d, log_i, log_f, ptr(c0), ptr(n0), ptr(m0),
+                                                        bytes(done), gh, ptr(c_last), ptr(n_last), floats(all, at_kept.m_steps), column(all, at_kept.states), ptr(gc), ptr(gn), ptr(gm),
+                                                        gqkv.data_ptr(), gks, column(gqkv, 2 * s.d), 3 * s.hid, 3 * s.d, gli, glf, ptr(gc0), ptr(gn0), ptr(gm0),
                                                         status_ptr(x), s.B, s.T, s.H, s.d, ctx->saved_data["eps"].toDouble(), st));
-    check("mlstm_gates_bwd", l::mlstm_gates_bwd(logits.data_ptr(), ptr(gli), ptr(glf), gks.data_ptr(), s.scale(), column(gqkv, s.d), 3 * s.hid, 3 * s.d,
+    check("mlstm_gates_bwd", l::mlstm_gates_bwd(logits, gli, glf, gks, s.scale(), column(gqkv, s.d), 3 * s.hid, 3 * s.d,
                                                 glogits.data_ptr(), part_gate, s.M, s.H, s.d, st));
     product_into(glogits, gate_w, gqkv, Tensor(), true);
     const Tensor gqk = parts(gqkv, 0, 2, s), gvalue = parts(gqkv, 2, 1, s);
