@@ -8,11 +8,16 @@
 // is so large that exp could leave float32's range (kSafe), the block takes the log form for that stretch of time.
 //
 // Bound: HBM (16 / 24 bytes per element; 30 / 45 us for 12.3 M elements) and about five special-function evaluations
-// per element, which have to overlap: time is split over sixteen warps of a block.  A block owns 32 channels of one
+// per element, which have to overlap: time is split over the warps of a block.  A block owns 32 channels of one
 // sequence; every thread loads its stretch of at most kSteps steps, folds it into one affine map of the incoming value
-// (forward: the state, backward: the carried cotangent; a reset cuts the map's slope), the sixteen maps are chained
+// (forward: the state, backward: the carried cotangent; a reset cuts the map's slope), the maps are chained
 // through shared memory, and the stretch is replayed from the right incoming value.  Longer sequences take several
-// turns.  (One thread per channel walking all of T in log form: 116 / 136 us at 96 x 250 x 512.)
+// turns.  A stretch that a block takes whole, in the linear form and without a reset, runs through loops without their tests
+// (a quarter fewer instructions).  96 x 250 x 512: 59 / 58 us (before, with those tests, one lane alone at a kink and blocks
+// of sixteen warps: 96 / 68; one thread per channel walking all of T in log form: 116 / 136), 256 x 256 x 512: 137 / 147
+// (206 / 176).  Left: the special functions and the dependent steps between two barriers of a turn.
+#include <type_traits>
+
 #include "layers.cuh"
 #include "logspace.cuh"
 #include "mxk_common.cuh"
@@ -22,7 +27,7 @@ namespace mxk {
 namespace layers {
 namespace {
 
-constexpr int kSegs = 16, kSteps = 8;
+constexpr int kSteps = 8;
 // How a block took a turn, and left its states with `forms`.
 constexpr uint8_t kLinear = 0, kLog = 1;
 
@@ -40,6 +45,45 @@ __device__ __noinline__ float dot_in_order(const float* __restrict__ in, const f
   for (int k = 0; k < F; ++k) acc = fmaf(in[k], w[k], acc);
   return acc;
 }
+// The same sum for one element, which is what a stretch mostly has if it has any: the warp brings the rows, every lane adds them up.
+// (A lane alone with its loads held its block for 7 us at 512 terms, and the forward pass of 96 x 250 x 512 for 45 of 97.)
+constexpr int kChunk = 128;
+__device__ __noinline__ float dot_of_warp(const float* __restrict__ in, const float* __restrict__ w, int F, float (*buf)[kChunk], int lane) {
+  float x[kChunk / 32], v[kChunk / 32], acc = 0.f;
+  const auto load = [&](int k0) {
+#pragma unroll
+    for (int u = 0; u < kChunk / 32; ++u) {
+      const int k = k0 + u * 32 + lane;
+      x[u] = k < F ? __ldg(in + k) : 0.f;
+      v[u] = k < F ? __ldg(w + k) : 0.f;
+    }
+  };
+  load(0);
+  for (int k0 = 0; k0 < F; k0 += kChunk) {
+#pragma unroll
+    for (int u = 0; u < kChunk / 32; ++u) {
+      buf[0][u * 32 + lane] = x[u];
+      buf[1][u * 32 + lane] = v[u];
+    }
+    __syncwarp();
+    if (k0 + kChunk < F) load(k0 + kChunk);
+    if (k0 + kChunk <= F) {
+#pragma unroll 8
+      for (int k = 0; k < kChunk; k += 4) {
+        const float4 a = *reinterpret_cast<const float4*>(&buf[0][k]), b = *reinterpret_cast<const float4*>(&buf[1][k]);
+        acc = fmaf(a.x, b.x, acc);
+        acc = fmaf(a.y, b.y, acc);
+        acc = fmaf(a.z, b.z, acc);
+        acc = fmaf(a.w, b.w, acc);
+      }
+    } else {
+      for (int k = 0; k < F - k0; ++k) acc = fmaf(buf[0][k], buf[1][k], acc);
+    }
+    __syncwarp();
+  }
+  return acc;
+}
+constexpr int kFewNear = 4;   // elements of a step up to which the warp takes them one by one
 
 // Two-norms of the rows of a (rows_a, F), then of those of b (rows_b, F); a warp each.  0 where the squares leave float32's
 // range: the gates are saturated there.  HBM-bound: one read of a.
@@ -96,7 +140,9 @@ __device__ __forceinline__ unsigned reset_mask(const uint8_t* drow, int t_begin,
   return __ballot_sync(0xffffffffu, reset);
 }
 
-__global__ void __launch_bounds__(32 * kSegs, 2)
+// kSegs: warps of a block, and parts of a turn's time.
+template <int kSegs>
+__global__ void __launch_bounds__(32 * kSegs, 32 / kSegs)
 mingru_fwd_kernel(const float* __restrict__ z, const float* ht, float* ht_kink, const float* __restrict__ dense_in,
                   const float* __restrict__ dense_w, const float* __restrict__ norms, int F, long long ld,
                   const float* __restrict__ x0, const float* __restrict__ a0, const uint8_t* __restrict__ done,
@@ -105,6 +151,7 @@ mingru_fwd_kernel(const float* __restrict__ z, const float* ht, float* ht_kink, 
   enter_kernel();
   __shared__ float sa[kSegs][32], sq[kSegs][32], sd[kSegs][32];
   __shared__ unsigned sr[kSegs];   // reset bits of a stretch
+  __shared__ __align__(16) float rows[kSegs][2][kChunk];
   __shared__ float carry_x[32], carry_a[32];
   const int lane = threadIdx.x & 31, seg = threadIdx.x >> 5;
   const int groups = (D + 31) / 32;
@@ -117,24 +164,34 @@ mingru_fwd_kernel(const float* __restrict__ z, const float* ht, float* ht_kink, 
     carry_a[lane] = (in && a0) ? a0[static_cast<size_t>(b) * D + d] : 0.f;
   }
   const auto form_at = [&](int turn_no) { return static_cast<size_t>(blockIdx.x) * ((T + turn_len - 1) / turn_len) + turn_no; };
+  const int step = static_cast<int>(ld);
   const float range = (ht_kink && in) ? kNearKink * __ldg(norms + static_cast<long long>(B) * T + d) : 0.f;
   for (int turn = 0; turn < T; turn += turn_len) {
     const int t_begin = turn + seg * len, t_end = min(min(T, turn + turn_len), t_begin + len);
     const int count = t_end - t_begin;   // steps of this warp (may be negative)
+    // (nearly every warp's stretch is whole and without a reset: its loops are kept free of what the others ask step by step)
+    const bool whole = __all_sync(0xffffffffu, in && count == kSteps);
     float lv[kSteps], dv[kSteps];
     {
       const long long token = static_cast<long long>(b) * T + t_begin;
       const float *pz = z + token * ld + d, *ph = ht + token * ld + d;
+      if (whole) {
 #pragma unroll
-      for (int i = 0; i < kSteps; ++i) {
-        const bool on = in && i < count;
-        lv[i] = on ? ld_stream(pz) : 0.f;
-        dv[i] = on ? ld_stream(ph) : 1.f;
-        pz += ld;
-        ph += ld;
+        for (int i = 0; i < kSteps; ++i) {
+          lv[i] = ld_stream(pz + i * step);
+          dv[i] = ld_stream(ph + i * step);
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < kSteps; ++i) {
+          const bool on = in && i < count;
+          lv[i] = on ? ld_stream(pz + i * step) : 0.f;
+          dv[i] = on ? ld_stream(ph + i * step) : 1.f;
+        }
       }
     }
     const unsigned resets = reset_mask(drow, t_begin, count, lane);
+    const bool plain = whole && resets == 0;
     float most = 0.f;
 #pragma unroll
     for (int i = 0; i < kSteps; ++i) most = fmaxf(most, fmaxf(fabsf(lv[i]), fabsf(dv[i])));
@@ -150,11 +207,21 @@ mingru_fwd_kernel(const float* __restrict__ z, const float* ht, float* ht_kink, 
       if (__any_sync(0xffffffffu, near != 0)) {
         if (__reduce_add_sync(0xffffffffu, __popc(near & zero) - __popc(near & ~zero)) > 1) near &= ~zero;
 #pragma unroll
-        for (int i = 0; i < kSteps; ++i)
-          if (near >> i & 1u) {
-            dv[i] = dot_in_order(dense_in + (token0 + i) * F, dense_w + static_cast<long long>(d) * F, F);
-            ht_kink[(token0 + i) * ld + d] = dv[i];
+        for (int i = 0; i < kSteps; ++i) {
+          unsigned lanes = __ballot_sync(0xffffffffu, near >> i & 1u);
+          if (lanes == 0) continue;
+          const float* const row = dense_in + (token0 + i) * F;
+          if (__popc(lanes) <= kFewNear) {
+            for (; lanes; lanes &= lanes - 1) {
+              const int l = __ffs(lanes) - 1;
+              const float v = dot_of_warp(row, dense_w + static_cast<long long>(d - lane + l) * F, F, rows[seg], lane);
+              if (lane == l) dv[i] = v;
+            }
+          } else if (near >> i & 1u) {
+            dv[i] = dot_in_order(row, dense_w + static_cast<long long>(d) * F, F);
           }
+          if (near >> i & 1u) ht_kink[(token0 + i) * ld + d] = dv[i];
+        }
       }
     }
     const bool linear = !__syncthreads_or(!(most <= kSafe) || (seg == 0 && !(carry_x[lane] <= kSafe)));
@@ -170,12 +237,19 @@ mingru_fwd_kernel(const float* __restrict__ z, const float* ht, float* ht_kink, 
         const float sh = rcp(1.f + exp_safe(-hi)), g = hi >= 0.f ? hi + 0.5f : sh;
         lv[i] = (zi >= 0.f ? r : er) * g;
         dv[i] = zi >= 0.f ? er : r;
-        if (i < count) {
-          if (resets >> i & 1u) { A = 0.f; Q = lv[i]; dec = 0.f; prod = dv[i]; }
-          else { A *= dv[i]; Q = fmaf(dv[i], Q, lv[i]); prod *= dv[i]; }
-        }
-        if (i % 4 == 3) { dec += log_safe(prod); prod = 1.f; }   // four decays are at least e^-80
       }
+      const auto fold = [&](auto asked) {   // four decays are at least e^-80
+#pragma unroll
+        for (int i = 0; i < kSteps; ++i) {
+          if (!asked.value || i < count) {
+            if (asked.value && (resets >> i & 1u)) { A = 0.f; Q = lv[i]; dec = 0.f; prod = dv[i]; }
+            else { A *= dv[i]; Q = fmaf(dv[i], Q, lv[i]); prod *= dv[i]; }
+          }
+          if (i % 4 == 3) { dec += log_safe(prod); prod = 1.f; }
+        }
+      };
+      if (plain) fold(std::false_type());
+      else fold(std::true_type());
       sa[seg][lane] = A;
       sq[seg][lane] = Q;
       sd[seg][lane] = dec;
@@ -184,17 +258,24 @@ mingru_fwd_kernel(const float* __restrict__ z, const float* ht, float* ht_kink, 
       __syncthreads();
       // (a stretch with a reset forgets what comes in, finite or not)
       for (int s2 = 0; s2 < seg; ++s2) cur = sr[s2] ? sq[s2][lane] : fmaf(sa[s2][lane], cur, sq[s2][lane]);
-      float *ps = states + out0, *py = y + out0;
+      float *const ps = states + out0, *const py = y + out0;
+      if (plain && states && forms && y) {
 #pragma unroll
-      for (int i = 0; i < kSteps; ++i) {
-        if (i < count) {
-          cur = (resets >> i & 1u) ? lv[i] : fmaf(dv[i], cur, lv[i]);
-          if (in) {
-            if (states) st_stream(ps, forms ? cur : log_safe(cur));
-            if (y) st_stream(py, cur);
+        for (int i = 0; i < kSteps; ++i) {
+          cur = fmaf(dv[i], cur, lv[i]);
+          st_stream(ps + i * D, cur);
+          st_stream(py + i * D, cur);
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < kSteps; ++i) {
+          if (i < count) {
+            cur = (resets >> i & 1u) ? lv[i] : fmaf(dv[i], cur, lv[i]);
+            if (in) {
+              if (states) st_stream(ps + i * D, forms ? cur : log_safe(cur));
+              if (y) st_stream(py + i * D, cur);
+            }
           }
-          ps += D;
-          py += D;
         }
       }
       if (t_begin < t_end && t_end == min(T, turn + turn_len)) {
@@ -253,7 +334,8 @@ mingru_fwd_kernel(const float* __restrict__ z, const float* ht, float* ht_kink, 
 }
 
 // states, forms: as the forward kernel left them (without forms: log states)
-__global__ void __launch_bounds__(32 * kSegs, 2)
+template <int kSegs>
+__global__ void __launch_bounds__(32 * kSegs, 32 / kSegs)
 mingru_bwd_kernel(const float* __restrict__ z, const float* __restrict__ ht, long long ld, const float* __restrict__ states,
                   const uint8_t* __restrict__ forms, const float* __restrict__ x0, const uint8_t* __restrict__ done,
                   const float* __restrict__ gx, const float* __restrict__ gy, const float* __restrict__ gx_last,
@@ -267,6 +349,7 @@ mingru_bwd_kernel(const float* __restrict__ z, const float* __restrict__ ht, lon
   const bool in = d < D;
   const uint8_t* drow = done ? done + static_cast<size_t>(b) * T : nullptr;
   const int len = (turn_len + kSegs - 1) / kSegs;
+  const int step = static_cast<int>(ld);
   if (seg == 0) carry[lane] = (in && gx_last) ? gx_last[static_cast<size_t>(b) * D + d] : 0.f;
   for (int turn = (T - 1) / turn_len * turn_len; turn >= 0; turn -= turn_len) {
     const int t_begin = turn + seg * len, t_end = min(min(T, turn + turn_len), t_begin + len);
@@ -278,23 +361,31 @@ mingru_bwd_kernel(const float* __restrict__ z, const float* __restrict__ ht, lon
     const bool logs = stored(turn / turn_len) == kLog;
     const bool prev_log = t_begin == 0 || (t_begin > turn ? logs : stored(turn / turn_len - 1) == kLog);
     float zv[kSteps], hv[kSteps], sv[kSteps], e[kSteps], w[kSteps], prev = 0.f;
+    const bool whole = __all_sync(0xffffffffu, in && count == kSteps);
     {
-      const float *pz = z + io0, *ph = ht + io0, *ps = states + at0, *pg = gy + at0;
+      const float *const pz = z + io0, *const ph = ht + io0, *const ps = states + at0, *const pg = gy + at0;
       if (in && count > 0) prev = t_begin > 0 ? ps[-D] : (x0 ? x0[static_cast<size_t>(b) * D + d] : -INFINITY);
+      if (whole && gy) {
 #pragma unroll
-      for (int i = 0; i < kSteps; ++i) {
-        const bool on = in && i < count;
-        zv[i] = on ? ld_stream(pz) : 0.f;
-        hv[i] = on ? ld_stream(ph) : 0.f;
-        sv[i] = on ? ld_stream(ps) : (logs ? 0.f : 1.f);
-        e[i] = (on && gy) ? ld_stream(pg) : 0.f;
-        pz += ld;
-        ph += ld;
-        ps += D;
-        pg += D;
+        for (int i = 0; i < kSteps; ++i) {
+          zv[i] = ld_stream(pz + i * step);
+          hv[i] = ld_stream(ph + i * step);
+          sv[i] = ld_stream(ps + i * D);
+          e[i] = ld_stream(pg + i * D);
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < kSteps; ++i) {
+          const bool on = in && i < count;
+          zv[i] = on ? ld_stream(pz + i * step) : 0.f;
+          hv[i] = on ? ld_stream(ph + i * step) : 0.f;
+          sv[i] = on ? ld_stream(ps + i * D) : (logs ? 0.f : 1.f);
+          e[i] = (on && gy) ? ld_stream(pg + i * D) : 0.f;
+        }
       }
     }
     const unsigned resets = reset_mask(drow, t_begin, count, lane);
+    const bool plain = whole && resets == 0;
     bool linear = !logs;
     if (!forms) {
       float most = (t_begin == 0 && x0) ? fmaxf(prev, 0.f) : 0.f;
@@ -317,17 +408,21 @@ mingru_bwd_kernel(const float* __restrict__ z, const float* __restrict__ ht, lon
 #pragma unroll
         for (int i = 0; i < kSteps; ++i) e[i] *= sv[i];
       }
+      const auto fold = [&](auto asked) {
 #pragma unroll
-      for (int i = kSteps - 1; i >= 0; --i) {
-        const float ez = exp_safe(-fabsf(zv[i])), r = rcp(1.f + ez), er = ez * r;
-        const float share = (zv[i] >= 0.f ? er : r) * (i > 0 ? sv[i > 0 ? i - 1 : 0] : prev) * rcp(sv[i]);
-        w[i] = (resets >> i & 1u) ? 0.f : share;
-        zv[i] = zv[i] >= 0.f ? r : er;   // sigmoid(z)
-        if (i < count) {
-          Q = w[i] * (e[i] + Q);
-          P *= w[i];
+        for (int i = kSteps - 1; i >= 0; --i) {
+          const float ez = exp_safe(-fabsf(zv[i])), r = rcp(1.f + ez), er = ez * r;
+          const float share = (zv[i] >= 0.f ? er : r) * (i > 0 ? sv[i > 0 ? i - 1 : 0] : prev) * rcp(sv[i]);
+          w[i] = asked.value && (resets >> i & 1u) ? 0.f : share;
+          zv[i] = zv[i] >= 0.f ? r : er;   // sigmoid(z)
+          if (!asked.value || i < count) {
+            Q = w[i] * (e[i] + Q);
+            P *= w[i];
+          }
         }
-      }
+      };
+      if (plain) fold(std::false_type());
+      else fold(std::true_type());
     } else {
       // log form, from the log states
       if (!prev_log) prev = logf(prev);
@@ -354,31 +449,27 @@ mingru_bwd_kernel(const float* __restrict__ z, const float* __restrict__ ht, lon
     float c = carry[lane];
     for (int s2 = kSegs - 1; s2 > seg; --s2) c = fmaf(sp[s2][lane], c, sq[s2][lane]);
     __syncthreads();   // every segment has read the carry
-    float *oz = gz + io0 + (count - 1) * ld, *oh = gh + io0 + (count - 1) * ld;
+    float *const oz = gz + io0, *const oh = gh + io0;
+    const auto replay = [&](auto asked) {
 #pragma unroll
-    for (int i = kSteps - 1; i >= 0; --i) {
-      if (i < count) {
-        const float g = e[i] + c, g_d = w[i] * g, g_ls = (1.f - w[i]) * g;
-        c = g_d;
-        // d(-softplus(-z))/dz = 1 - sigmoid(z), d(-softplus(z))/dz = -sigmoid(z)
-        const float sh = rcp(1.f + exp_safe(fminf(hv[i], 80.f))), dg = hv[i] >= 0.f ? rcp(hv[i] + 0.5f) : sh;
-        if (in) {
-          st_stream(oz, fmaf(-zv[i], g, g_ls));
-          st_stream(oh, g_ls * dg);
+      for (int i = kSteps - 1; i >= 0; --i) {
+        if (!asked.value || i < count) {
+          const float g = e[i] + c, g_d = w[i] * g, g_ls = (1.f - w[i]) * g;
+          c = g_d;
+          // d(-softplus(-z))/dz = 1 - sigmoid(z), d(-softplus(z))/dz = -sigmoid(z)
+          const float dg = rcp(hv[i] >= 0.f ? hv[i] + 0.5f : 1.f + exp_safe(hv[i]));
+          if (!asked.value || in) {
+            st_stream(oz + i * step, fmaf(-zv[i], g, g_ls));
+            st_stream(oh + i * step, g_ls * dg);
+          }
         }
-        oz -= ld;
-        oh -= ld;
       }
-    }
+    };
+    if (plain) replay(std::false_type());
+    else replay(std::true_type());
     if (seg == 0) carry[lane] = c;
   }
   if (seg == 0 && in && gx0) gx0[static_cast<size_t>(b) * D + d] = carry[lane];
-}
-
-// Steps a block takes per turn: as evenly divided as the stretches allow (T = 250 is two turns of 125, not 128 + 122).
-int turn_length(int T) {
-  const int most = kSegs * kSteps, turns = (T + most - 1) / most;
-  return (T + turns - 1) / turns;
 }
 
 template <int kSplit>
@@ -412,6 +503,16 @@ mingru_step_kernel(const float* __restrict__ in, const float* __restrict__ w_z, 
 }
 
 unsigned blocks_of(int B, int D) { return static_cast<unsigned>(static_cast<long long>(B) * ((D + 31) / 32)); }
+// Warps of a block.  Two blocks of sixteen fit an SM: as long as the grid fits so, they halve the turns (us, forward / backward: 1 x 1000 x 64
+// 29 / 22 with sixteen, 42 / 34 with eight; 8 x 250 x 512 28 / 8 and 35 / 12).  Above, four blocks of eight keep an SM at it while one of
+// them waits at its barriers, and a grid up to twice that size is one wave instead of two (19 x 250 x 512: 32 / 18 and 20 / 16;
+// 96 x 250 x 512 backward: 60 and 55).
+int segments(int B, int D) { return blocks_of(B, D) > 2 * kNumSMs ? 8 : 16; }
+// Steps a block takes per turn: as evenly divided as the stretches allow (T = 250 is two turns of 125, not 128 + 122).
+int turn_length(int B, int T, int D) {
+  const int most = segments(B, D) * kSteps, turns = (T + most - 1) / most;
+  return (T + turns - 1) / turns;
+}
 int check_dims(int B, int T, int D) {
   return (B <= 0 || T <= 0 || D <= 0 || static_cast<long long>(B) * ((D + 31) / 32) > 0x7fffffffLL) ? MXK_ERR_DIMS : MXK_OK;
 }
@@ -428,19 +529,21 @@ int mingru_fwd(const float* z, const float* h_tilde, const NearKink& kink, long 
                const uint8_t* done, float* states, uint8_t* forms, float* y, float* x_last, float* a_last, int B, int T, int D,
                cudaStream_t stream) {
   if (const int st = check_dims(B, T, D)) return st;
-  mxk::launch_kernel(mingru_fwd_kernel, blocks_of(B, D), 32 * kSegs, 0, stream, z, h_tilde, kink.h, kink.in, kink.w, kink.norms, kink.F, ld, x0,
-                     a0, done, states, forms, y, x_last, a_last, B, T, D, turn_length(T));
+  const int segs = segments(B, D);
+  mxk::launch_kernel(segs == 8 ? mingru_fwd_kernel<8> : mingru_fwd_kernel<16>, blocks_of(B, D), 32 * segs, 0, stream, z, h_tilde, kink.h, kink.in, kink.w,
+                     kink.norms, kink.F, ld, x0, a0, done, states, forms, y, x_last, a_last, B, T, D, turn_length(B, T, D));
   return launch_status();
 }
 
-size_t mingru_forms(int B, int T, int D) { return static_cast<size_t>(blocks_of(B, D)) * ((T + turn_length(T) - 1) / turn_length(T)); }
+size_t mingru_forms(int B, int T, int D) { return static_cast<size_t>(blocks_of(B, D)) * ((T + turn_length(B, T, D) - 1) / turn_length(B, T, D)); }
 
 int mingru_bwd(const float* z, const float* h_tilde, long long ld, const float* states, const uint8_t* forms, const float* x0, const uint8_t* done,
                const float* gx, const float* gy, const float* gx_last, float* gz, float* gh, float* gx0, int B, int T, int D,
                cudaStream_t stream) {
   if (const int st = check_dims(B, T, D)) return st;
-  mxk::launch_kernel(mingru_bwd_kernel, blocks_of(B, D), 32 * kSegs, 0, stream, z, h_tilde, ld, states, forms, x0, done, gx, gy, gx_last, gz, gh, gx0,
-                                                                B, T, D, turn_length(T));
+  const int segs = segments(B, D);
+  mxk::launch_kernel(segs == 8 ? mingru_bwd_kernel<8> : mingru_bwd_kernel<16>, blocks_of(B, D), 32 * segs, 0, stream, z, h_tilde, ld, states, forms, x0, done, gx,
+                     gy, gx_last, gz, gh, gx0, B, T, D, turn_length(B, T, D));
   return launch_status();
 }
 

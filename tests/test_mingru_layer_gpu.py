@@ -72,6 +72,36 @@ def test_the_side_of_the_kink_is_that_of_the_sum_in_order(scale, w_scale):
     assert float((slope - want).abs().max()) <= 1e-3
 
 
+# The same with few channels of a warp at the kink, which the warp sums one by one in chunks of 128 terms, and with one more
+# than that; blocks of sixteen warps (one sequence) and of eight (a grid beyond two blocks an SM)
+@pytest.mark.parametrize("feat", [65, 128, 130, 515])
+@pytest.mark.parametrize("near", [(0,), (3, 17, 39), (1, 2, 30, 31), (4, 5, 6, 7, 8)])
+@pytest.mark.parametrize("bsz", [1, 200])
+def test_few_channels_at_the_kink(feat, near, bsz):
+    from memorax_b200.memoroid import MinGRUCell, Memoroid
+    torch.manual_seed(feat)
+    steps, dim, b, t = 11, 40, bsz // 2, 9
+    cell = MinGRUCell(dim, in_features=feat)
+    x = torch.randn(bsz, steps, feat)
+    xt, rows = x[b, t].double(), list(near)
+    acc = torch.zeros(len(rows))
+    with torch.no_grad():
+        w = cell.h.weight[rows].double()
+        cell.h.weight[rows] = (w - (w @ xt)[:, None] * xt / (xt @ xt)).float()
+        cell.z.weight.zero_()
+        terms = cell.h.weight[rows].double() * xt
+        for k in range(feat):
+            acc = (acc.double() + terms[:, k]).float()
+    cell, x = cell.cuda(), x.cuda()
+    gy = torch.zeros(bsz, steps, dim, device="cuda")
+    gy[b, t] = 1
+    _, y = Memoroid(cell)(x, torch.ones(bsz, steps, device="cuda"), None)
+    (gw,) = torch.autograd.grad(y, [cell.h.weight], gy)
+    slope = (gw.cpu().double() @ xt) / (xt @ xt) / 0.5
+    # float32 logarithms of the states at magnitude 1/2: their errors are below 1e-5 of the slopes 1 and 1/4
+    assert float((slope[rows] - torch.where(acc >= 0, 1.0, 0.25).double()).abs().max()) <= 1e-3
+
+
 # elements that are zero or tiny because the inputs or the weights are need no second look, which costs thousands of cycles
 @pytest.mark.parametrize("case", ["zero inputs", "small inputs", "padding", "zero channels", "small channels", "one-hot inputs, pruned weights"])
 def test_no_input_is_slow(case):
