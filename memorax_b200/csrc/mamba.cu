@@ -5,15 +5,17 @@
 // A block owns one (sequence, head) and walks time in stretches of 64 steps: the stretch's 48 channels are convolved into
 // shared memory, its four quarters are scanned by four warps from a zero state, the quarters' end states are chained, and
 // each warp replays its quarter from the right incoming state (a lane owns 8 of the 256 states; a step is 16 multiply-adds
-// for the update and 8 for the read-out).  Bound by issue slots at full size (about 40 instructions per warp and step) and
-// by the chain of stretches when there are few sequences; the materialised form moved 2 KB per token and head and ran
-// about thirty elementwise launches each way.
+// for the update and 8 for the read-out).  Bound by dependent steps and barriers (instructions issue in 40 % of the cycles)
+// and by the chain of stretches when there are few sequences; the materialised form moved 2 KB per token and head and ran
+// about thirty elementwise launches each way.  Outside the scans a thread keeps one channel and slides the taps over its
+// rows (with the channel of every element found from its index, and a load per tap, those passes were 40 % of the
+// instructions).  128 x 64 steps x 8 heads: 28 -> 17 us; 128 x 250 x 8: 94 -> 58; 1 x 2048 x 8: 425 -> 271.
 //
 // The backward pass starts every stretch from its saved state and needs sums that are each cheap in one lane layout only,
 // so three groups of four warps run side by side: C's cotangent from the states (lane = n), x's (lane = p) and B's
 // (lane = n) from the cotangent of the states.  The first group leaves every h_{t-1} in shared memory for the third,
 // which has the decay's cotangent <dh_t, h_{t-1}> as a plain dot product (as a difference of larger sums it lost two
-// digits).
+// digits).  Sums over lanes are taken for four steps together, 9 shuffles instead of 24.  128 x 64 x 8: 81 -> 59 us, 128 x 250 x 8: 321 -> 240, 1 x 2048 x 8: 635 -> 450.
 #include "layers.cuh"
 #include "mxk_common.cuh"
 
@@ -22,7 +24,7 @@ namespace layers {
 namespace {
 
 constexpr int kN = 16, kP = 16, kStates = kN * kP;   // per head
-constexpr int kLen = 64, kQuarter = kLen / 4;        // steps per stretch and per warp
+constexpr int kQuarter = 16;                         // steps per warp
 constexpr int kTaps = 4, kHalo = kTaps - 1;
 constexpr int kCh = 3 * 16;                          // channels of a head: x | B | C
 
@@ -38,27 +40,48 @@ __device__ __forceinline__ int conv_channel(int c, int h, int hid) { return (c >
 // conv_w | conv_b | a_log | dt_bias | d of every head
 __host__ __device__ constexpr int partial_floats(int H) { return 48 * H * (kTaps + 1) + 3 * H; }
 
+template <int kLen>
 struct Stretch {            // of one head
   float raw[kLen + kHalo][kCh];   // projections, three steps of the past in front
   float act[kLen][kCh];     // silu(conv): x | B | C
-  float dt[kLen], decay[kLen];
+  float dt[kLen], decay[kLen], kept[kLen];   // kept: decay, or 0 where a sequence begins
   unsigned char reset[kLen];
 };
 
-__device__ __forceinline__ float convolve(const Stretch& s, const MambaParams& w, int r, int c, int ch) {
-  float v = __ldg(w.conv_b + ch);
+// The taps of one channel.
+struct Taps {
+  float w[kTaps], bias;
+  __device__ __forceinline__ Taps(const MambaParams& p, int chn) : bias(__ldg(p.conv_b + chn)) {
 #pragma unroll
-  for (int k = 0; k < kTaps; ++k) v = fmaf(__ldg(w.conv_w + ch * kTaps + k), s.raw[r + k][c], v);
-  return v;
-}
+    for (int k = 0; k < kTaps; ++k) w[k] = __ldg(p.conv_w + chn * kTaps + k);
+  }
+  // of four rows in a row, the oldest first
+  __device__ __forceinline__ float operator()(const float* v) const {
+    float u = bias;
+#pragma unroll
+    for (int k = 0; k < kTaps; ++k) u = fmaf(w[k], v[k], u);
+    return u;
+  }
+};
 
-// Convolves and activates the stretch at t0.  Ends with a barrier.
-__device__ __forceinline__ void load_stretch(Stretch& s, const MambaParams& w, const float* __restrict__ proj, long long ld,
-                                             const uint8_t* drow, int b, int h, int H, int T, int t0, int tid, int threads) {
+// Convolves and activates the stretch at t0.  A thread has one channel and every row / kGroups of it: its taps and columns are found once, and
+// a window slides over its rows.  Threads beyond kGroups x 48 only help with the steps.  Ends with a barrier.
+template <int kGroups, int kLen>
+__device__ __forceinline__ void load_stretch(Stretch<kLen>& s, const MambaParams& w, const float* __restrict__ proj, long long ld,
+                                             const uint8_t* drow, int b, int h, int H, int T, int t0, int tid, int pc, int pg) {
   const int hid = H * 16;
-  for (int i = tid; i < (kLen + kHalo) * kCh; i += threads) {
-    const int r = i / kCh, c = i % kCh, t = t0 + r - kHalo;
-    s.raw[r][c] = (t >= 0 && t < T) ? __ldg(proj + (static_cast<long long>(b) * T + t) * ld + proj_col(c, h, hid)) : 0.f;
+  constexpr int kRows = kLen / kGroups;
+  if (pg < kGroups) {
+    const float* const col = proj + static_cast<long long>(b) * T * ld + proj_col(pc, h, hid);
+#pragma unroll 8
+    for (int i = 0; i < kRows; ++i) {
+      const int r = i * kGroups + pg, t = t0 + r;
+      s.raw[r + kHalo][pc] = t < T ? __ldg(col + t * ld) : 0.f;
+    }
+    for (int r = pg; r < kHalo; r += kGroups) {
+      const int t = t0 + r - kHalo;
+      s.raw[r][pc] = (t >= 0 && t < T) ? __ldg(col + t * ld) : 0.f;
+    }
   }
   if (tid < kLen) {
     const int t = t0 + tid;
@@ -69,13 +92,25 @@ __device__ __forceinline__ void load_stretch(Stretch& s, const MambaParams& w, c
     }
     s.dt[tid] = dt;        // past the end: nothing enters, nothing decays
     s.decay[tid] = decay;
-    s.reset[tid] = (t < T && drow) ? drow[t] : 0;
+    const unsigned char reset = (t < T && drow) ? drow[t] : 0;
+    s.reset[tid] = reset;
+    s.kept[tid] = reset ? 0.f : decay;
   }
   __syncthreads();
-  for (int i = tid; i < kLen * kCh; i += threads) {
-    const int r = i / kCh, c = i % kCh;
-    const float v = convolve(s, w, r, c, conv_channel(c, h, hid));
-    s.act[r][c] = v * sigmoid(v);
+  if (pg < kGroups) {
+    const Taps taps(w, conv_channel(pc, h, hid));
+    float v[kTaps];
+#pragma unroll
+    for (int k = 0; k < kHalo; ++k) v[k + 1] = s.raw[pg * kRows + k][pc];
+#pragma unroll 8
+    for (int i = 0; i < kRows; ++i) {
+      const int r = pg * kRows + i;
+#pragma unroll
+      for (int k = 0; k < kHalo; ++k) v[k] = v[k + 1];
+      v[kHalo] = s.raw[r + kHalo][pc];
+      const float u = taps(v);
+      s.act[r][pc] = u * sigmoid(u);
+    }
   }
   __syncthreads();
 }
@@ -86,23 +121,27 @@ __device__ __forceinline__ void load8(const float* p, float* v) {   // 16-byte a
   v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
 
+// kParts: warps, and parts of a stretch.
+template <int kParts>
 struct FwdSmem {
-  Stretch s;
-  float end[4][8][32];      // [quarter][state of a lane][lane]
-  float prod[4], dec[4];    // product of the decays (0 with a reset), and since the last reset
-  int had[4];
+  Stretch<kParts * kQuarter> s;
+  float end[kParts][8][32];           // [part][state of a lane][lane]
+  float prod[kParts], dec[kParts];    // product of the decays (0 with a reset), and since the last reset
+  int had[kParts];
   float carry[8][32];
   float carry_a;
 };
 
 // lane = p + 16 * (n >= 8): states n = 8 * (lane / 16) + j
-__global__ void __launch_bounds__(128) mamba_scan_fwd_kernel(MambaParams w, const float* __restrict__ proj, long long ld,
+template <int kParts>
+__global__ void __launch_bounds__(kParts * 32) mamba_scan_fwd_kernel(MambaParams w, const float* __restrict__ proj, long long ld,
                                                              const float* __restrict__ h0, const float* __restrict__ a0,
                                                              const uint8_t* __restrict__ done, float* __restrict__ y_pre,
                                                              float* __restrict__ h_last, float* __restrict__ a_last,
                                                              float* __restrict__ states, int T, int H) {
   enter_kernel();
-  __shared__ __align__(16) FwdSmem sm;
+  constexpr int kLen = kParts * kQuarter;
+  __shared__ __align__(16) FwdSmem<kParts> sm;
   const int tid = threadIdx.x, lane = tid & 31, q = tid >> 5;
   const int b = blockIdx.x / H, h = blockIdx.x % H, hid = H * 16;
   const int p = lane & 15, n0 = (lane >> 4) * 8;
@@ -117,30 +156,33 @@ __global__ void __launch_bounds__(128) mamba_scan_fwd_kernel(MambaParams w, cons
   }
   for (int c = 0; c < stretches; ++c) {
     const int t0 = c * kLen;
-    load_stretch(sm.s, w, proj, ld, drow, b, h, H, T, t0, tid, 128);
+    load_stretch<kParts / 2>(sm.s, w, proj, ld, drow, b, h, H, T, t0, tid, tid % kCh, tid / kCh);
     float st[8], v8[8];
     // ---- from a zero state: where the quarter ends
     {
-      float prod = 1.f, dec = 1.f;
-      int had = 0;
 #pragma unroll
       for (int j = 0; j < 8; ++j) st[j] = 0.f;
 #pragma unroll 4
       for (int i = 0; i < kQuarter; ++i) {
         const int t = q * kQuarter + i;
-        const bool reset = sm.s.reset[t] != 0;
-        const float d = reset ? 0.f : sm.s.decay[t];
+        const float d = sm.s.kept[t];
         const float xd = sm.s.act[t][p] * sm.s.dt[t];
         load8(&sm.s.act[t][16 + n0], v8);
 #pragma unroll
         for (int j = 0; j < 8; ++j) st[j] = fmaf(d, st[j], v8[j] * xd);
-        prod *= d;
-        dec = reset ? sm.s.decay[t] : dec * sm.s.decay[t];
-        had |= reset;
       }
 #pragma unroll
       for (int j = 0; j < 8; ++j) sm.end[q][j][lane] = st[j];
-      if (lane == 0) { sm.prod[q] = prod; sm.dec[q] = dec; sm.had[q] = had; }
+      // the quarter's decays, a lane a step: of all of them, and of those from the last reset on
+      const int t = q * kQuarter + p;
+      const unsigned resets = __ballot_sync(0xffffffffu, sm.s.reset[t] != 0) & 0xffffu;
+      float prod = sm.s.kept[t], dec = p >= 31 - __clz(resets) ? sm.s.decay[t] : 1.f;
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) {
+        prod *= __shfl_xor_sync(0xffffffffu, prod, o);
+        dec *= __shfl_xor_sync(0xffffffffu, dec, o);
+      }
+      if (lane == 0) { sm.prod[q] = prod; sm.dec[q] = dec; sm.had[q] = resets != 0; }
     }
     __syncthreads();
 #pragma unroll
@@ -158,7 +200,7 @@ __global__ void __launch_bounds__(128) mamba_scan_fwd_kernel(MambaParams w, cons
 #pragma unroll 4
     for (int i = 0; i < kQuarter; ++i) {
       const int t = q * kQuarter + i;
-      const float d = sm.s.reset[t] ? 0.f : sm.s.decay[t];
+      const float d = sm.s.kept[t];
       const float x = sm.s.act[t][p], xd = x * sm.s.dt[t];
       load8(&sm.s.act[t][16 + n0], v8);
 #pragma unroll
@@ -171,17 +213,17 @@ __global__ void __launch_bounds__(128) mamba_scan_fwd_kernel(MambaParams w, cons
       if (lane < 16 && t0 + t < T) y_pre[(static_cast<size_t>(b) * T + t0 + t) * hid + h * 16 + p] = fmaf(skip, x, y);
     }
     __syncthreads();   // carry and summaries have been read
-    if (q == 3) {
+    if (q == kParts - 1) {
 #pragma unroll
       for (int j = 0; j < 8; ++j) sm.carry[j][lane] = st[j];
       if (lane == 0) {
         float a = sm.carry_a;
-        for (int s2 = 0; s2 < 4; ++s2) a = sm.had[s2] ? sm.dec[s2] : a * sm.dec[s2];
+        for (int s2 = 0; s2 < kParts; ++s2) a = sm.had[s2] ? sm.dec[s2] : a * sm.dec[s2];
         sm.carry_a = a;
       }
     }
   }
-  if (q == 3) {
+  if (q == kParts - 1) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) h_last[static_cast<size_t>(blockIdx.x) * kStates + (n0 + j) * kP + p] = sm.carry[j][lane];
     if (lane == 0) a_last[blockIdx.x] = sm.carry_a;
@@ -189,23 +231,37 @@ __global__ void __launch_bounds__(128) mamba_scan_fwd_kernel(MambaParams w, cons
 }
 
 // ------------------------------------------------------------------------------------------------------ backward
+// kParts: warps of a group, and parts of a stretch.
+template <int kParts>
 struct BwdSmem {
-  Stretch s;
+  static constexpr int kLen = kParts * kQuarter;
+  Stretch<kLen> s;
   float g[kLen + kHalo][kCh];        // cotangents of the activations, then of the convolution's output; three steps of
                                      // the future behind
   float gy[kLen][16];
   union {
-    float end[3][4][8][32];          // [task][quarter]...: where a quarter ends from nothing
+    float end[3][kParts][8][32];     // [task][part]...: where a part ends from nothing
     float4 prev[kLen][2][32];        // h_{t-1}, eight states per lane
-    float red[384];
+    struct {
+      float of_group[kTaps + 1][kParts * 96], of_warp[3][kParts * 3];
+    } sums;
   };
-  float prod[4];
+  float prod[kParts];
   float carry[2][8][32];             // decay-weighted cotangent of the state entering the stretch from the right
   float e[kLen], u0[kLen];           // <dh_t, h_{t-1}>, <dh_t, B_t x_t>
 };
-static_assert(2 * (sizeof(BwdSmem) + 1024) <= 228 * 1024, "two blocks per SM");
+constexpr int bwd_blocks(int parts) { return parts == 1 ? 7 : 8 / parts; }   // per SM
+template <int kParts> constexpr bool fits = bwd_blocks(kParts) * (sizeof(BwdSmem<kParts>) + 1024) <= 228 * 1024;
+static_assert(fits<1> && fits<2> && fits<4>, "blocks per SM");
 
-__global__ void __launch_bounds__(384, 2) mamba_scan_bwd_kernel(MambaParams w, const float* __restrict__ proj, long long ld,
+// Sums over the two halves of a warp: of a in the lower one, of b in the upper one.
+__device__ __forceinline__ float halves(float a, float b, int lane) {
+  const bool up = lane & 16;
+  return (up ? b : a) + __shfl_xor_sync(0xffffffffu, up ? a : b, 16);
+}
+
+template <int kParts>
+__global__ void __launch_bounds__(kParts * 96, bwd_blocks(kParts)) mamba_scan_bwd_kernel(MambaParams w, const float* __restrict__ proj, long long ld,
                                                                 const uint8_t* __restrict__ done,
                                                                 const float* __restrict__ states,
                                                                 const float* __restrict__ gy_pre,
@@ -213,9 +269,10 @@ __global__ void __launch_bounds__(384, 2) mamba_scan_bwd_kernel(MambaParams w, c
                                                                 float* __restrict__ gh0, float* __restrict__ partial, int T, int H) {
   enter_kernel();
   extern __shared__ __align__(16) uint8_t raw_smem[];
-  BwdSmem& sm = *reinterpret_cast<BwdSmem*>(raw_smem);
+  BwdSmem<kParts>& sm = *reinterpret_cast<BwdSmem<kParts>*>(raw_smem);
+  constexpr int kLen = kParts * kQuarter, kThreads = kParts * 96, kGroups = kThreads / kCh, kRows = kLen / kGroups;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int task = warp >> 2, q = warp & 3;   // task 0: C (lane = n), 1: x (lane = p), 2: B (lane = n)
+  const int task = warp / kParts, q = warp % kParts;   // task 0: C (lane = n), 1: x (lane = p), 2: B (lane = n)
   const int b = blockIdx.x / H, h = blockIdx.x % H, hid = H * 16;
   const int l16 = lane & 15, o8 = (lane >> 4) * 8;   // own index, and the first of the eight contracted ones
   const uint8_t* drow = done ? done + static_cast<size_t>(b) * T : nullptr;
@@ -229,18 +286,18 @@ __global__ void __launch_bounds__(384, 2) mamba_scan_bwd_kernel(MambaParams w, c
 #pragma unroll
     for (int j = 0; j < 8; ++j) sm.carry[task - 1][j][lane] = gh_last ? gh_last[base + state_at(j)] : 0.f;
   }
-  for (int i = tid; i < kHalo * kCh; i += 384) sm.g[kLen + i / kCh][i % kCh] = 0.f;
-  // gradients of the convolution: thread = channel x 8 groups of 8 steps
-  const int pc = tid % kCh, pg = tid / kCh;
+  for (int i = tid; i < kHalo * kCh; i += kThreads) sm.g[kLen + i / kCh][i % kCh] = 0.f;
+  const int pc = tid % kCh, pg = tid / kCh;   // outside the scans: thread = channel x kGroups groups of kRows steps
+  const int chn = conv_channel(pc, h, hid);
   float gw[kTaps] = {0.f, 0.f, 0.f, 0.f}, gbias = 0.f, ga = 0.f, gdtb = 0.f, gd = 0.f;
 
   for (int c = stretches - 1; c >= 0; --c) {
     const int t0 = c * kLen;
-    for (int i = tid; i < kLen * 16; i += 384) {
+    for (int i = tid; i < kLen * 16; i += kThreads) {
       const int r = i >> 4, p = i & 15;
       sm.gy[r][p] = t0 + r < T ? __ldg(gy_pre + (static_cast<size_t>(b) * T + t0 + r) * hid + h * 16 + p) : 0.f;
     }
-    load_stretch(sm.s, w, proj, ld, drow, b, h, H, T, t0, tid, 384);
+    load_stretch<kGroups>(sm.s, w, proj, ld, drow, b, h, H, T, t0, tid, pc, pg);
     float st[8], a8[8];
     // ---- each quarter from nothing: states forward in time (task 0), their cotangents backward (tasks 1, 2)
 #pragma unroll
@@ -249,7 +306,7 @@ __global__ void __launch_bounds__(384, 2) mamba_scan_bwd_kernel(MambaParams w, c
 #pragma unroll 4
     for (int i = 0; i < kQuarter; ++i) {
       const int t = q * kQuarter + (task == 0 ? i : kQuarter - 1 - i);
-      const float d = sm.s.reset[t] ? 0.f : sm.s.decay[t];
+      const float d = sm.s.kept[t];
       if (task == 0) {
         const float bd = sm.s.act[t][16 + l16] * sm.s.dt[t];
         load8(&sm.s.act[t][o8], a8);
@@ -279,7 +336,7 @@ __global__ void __launch_bounds__(384, 2) mamba_scan_bwd_kernel(MambaParams w, c
     } else {
 #pragma unroll
       for (int j = 0; j < 8; ++j) st[j] = sm.carry[task - 1][j][lane];
-      for (int s2 = 3; s2 > q; --s2) {
+      for (int s2 = kParts - 1; s2 > q; --s2) {
         const float d = sm.prod[s2];
 #pragma unroll
         for (int j = 0; j < 8; ++j) st[j] = fmaf(d, st[j], sm.end[task][s2][j][lane]);
@@ -288,53 +345,72 @@ __global__ void __launch_bounds__(384, 2) mamba_scan_bwd_kernel(MambaParams w, c
     __syncthreads();   // summaries and carries have been read; the summaries' memory takes the states
     // ---- replay
     if (task == 0) {
-#pragma unroll 4
-      for (int i = 0; i < kQuarter; ++i) {
-        const int t = q * kQuarter + i;
-        const float d = sm.s.reset[t] ? 0.f : sm.s.decay[t], bd = sm.s.act[t][16 + l16] * sm.s.dt[t];
-        sm.prev[t][0][lane] = make_float4(st[0], st[1], st[2], st[3]);
-        sm.prev[t][1][lane] = make_float4(st[4], st[5], st[6], st[7]);
-        load8(&sm.s.act[t][o8], a8);
+#pragma unroll 2
+      for (int i = 0; i < kQuarter; i += 2) {
+        float v[2];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) st[j] = fmaf(d, st[j], a8[j] * bd);
-        load8(&sm.gy[t][o8], a8);
-        float v = 0.f;
+        for (int u = 0; u < 2; ++u) {
+          const int t = q * kQuarter + i + u;
+          const float d = sm.s.kept[t], bd = sm.s.act[t][16 + l16] * sm.s.dt[t];
+          sm.prev[t][0][lane] = make_float4(st[0], st[1], st[2], st[3]);
+          sm.prev[t][1][lane] = make_float4(st[4], st[5], st[6], st[7]);
+          load8(&sm.s.act[t][o8], a8);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v = fmaf(a8[j], st[j], v);
-        v += __shfl_xor_sync(0xffffffffu, v, 16);
-        if (lane < 16) sm.g[t][32 + l16] = v;
+          for (int j = 0; j < 8; ++j) st[j] = fmaf(d, st[j], a8[j] * bd);
+          load8(&sm.gy[t][o8], a8);
+          v[u] = 0.f;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[u] = fmaf(a8[j], st[j], v[u]);
+        }
+        sm.g[q * kQuarter + i + (lane >> 4)][32 + l16] = halves(v[0], v[1], lane);
       }
       asm volatile("bar.arrive %0, 64;" ::"r"(q + 1) : "memory");   // this quarter's states are there
     } else {
       if (task == 2) asm volatile("bar.sync %0, 64;" ::"r"(q + 1) : "memory");
-#pragma unroll 4
-      for (int i = kQuarter - 1; i >= 0; --i) {
-        const int t = q * kQuarter + i;
-        const float d = sm.s.reset[t] ? 0.f : sm.s.decay[t], dt = sm.s.dt[t];
-        const float own = task == 1 ? sm.gy[t][l16] : sm.s.act[t][32 + l16];
-        load8(task == 1 ? &sm.s.act[t][32 + o8] : &sm.gy[t][o8], a8);
-        float x8[8], v = 0.f, e = 0.f;
-        load8(task == 1 ? &sm.s.act[t][16 + o8] : &sm.s.act[t][o8], x8);
+      for (int i = kQuarter - 4; i >= 0; i -= 4) {
+        float v[4], e[4];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          a8[j] = fmaf(a8[j], own, st[j]);   // dh_t
-          v = fmaf(x8[j], a8[j], v);
-          st[j] = d * a8[j];
+        for (int u = 3; u >= 0; --u) {
+          const int t = q * kQuarter + i + u;
+          const float d = sm.s.kept[t];
+          const float own = task == 1 ? sm.gy[t][l16] : sm.s.act[t][32 + l16];
+          load8(task == 1 ? &sm.s.act[t][32 + o8] : &sm.gy[t][o8], a8);
+          float x8[8];
+          load8(task == 1 ? &sm.s.act[t][16 + o8] : &sm.s.act[t][o8], x8);
+          v[u] = 0.f;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            a8[j] = fmaf(a8[j], own, st[j]);   // dh_t
+            v[u] = fmaf(x8[j], a8[j], v[u]);
+            st[j] = d * a8[j];
+          }
+          if (task == 2) {
+            const float4 p0 = sm.prev[t][0][lane], p1 = sm.prev[t][1][lane];
+            e[u] = a8[0] * p0.x + a8[1] * p0.y + a8[2] * p0.z + a8[3] * p0.w;
+            e[u] += a8[4] * p1.x + a8[5] * p1.y + a8[6] * p1.z + a8[7] * p1.w;
+          }
         }
-        v += __shfl_xor_sync(0xffffffffu, v, 16);
-        if (task == 1) {
-          if (lane < 16) sm.g[t][l16] = fmaf(dt, v, skip * own);
-        } else {
-          const float4 p0 = sm.prev[t][0][lane], p1 = sm.prev[t][1][lane];
-          e = a8[0] * p0.x + a8[1] * p0.y + a8[2] * p0.z + a8[3] * p0.w;
-          e += a8[4] * p1.x + a8[5] * p1.y + a8[6] * p1.z + a8[7] * p1.w;
-          if (lane < 16) sm.g[t][16 + l16] = dt * v;
-          // lower half: <dh, h_{t-1}>, upper half: B . (cotangent of B)
-          e += __shfl_xor_sync(0xffffffffu, e, 16);
-          if (lane >= 16) e = v * sm.s.act[t][16 + l16];
+        float both[4];   // of task 2: e of two steps, and B . (cotangent of B)
 #pragma unroll
-          for (int o = 8; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
-          if (l16 == 0) (lane == 0 ? sm.e : sm.u0)[t] = e;
+        for (int u = 0; u < 4; u += 2) {   // a half of the warp per step
+          const int t = q * kQuarter + i + u + (lane >> 4);
+          const float sum = halves(v[u], v[u + 1], lane);
+          if (task == 1) {
+            sm.g[t][l16] = fmaf(sm.s.dt[t], sum, skip * sm.gy[t][l16]);
+          } else {
+            sm.g[t][16 + l16] = sm.s.dt[t] * sum;
+            both[u] = halves(e[u], e[u + 1], lane);
+            both[u + 1] = sum * sm.s.act[t][16 + l16];
+          }
+        }
+        if (task == 2) {   // four sums over 16 lanes; lane 4 m of a half ends with the one of `both` at m
+          const bool b3 = lane & 8, b2 = lane & 4;
+          const float r0 = (b3 ? both[2] : both[0]) + __shfl_xor_sync(0xffffffffu, b3 ? both[0] : both[2], 8);
+          const float r1 = (b3 ? both[3] : both[1]) + __shfl_xor_sync(0xffffffffu, b3 ? both[1] : both[3], 8);
+          float r = (b2 ? r1 : r0) + __shfl_xor_sync(0xffffffffu, b2 ? r0 : r1, 4);
+          r += __shfl_xor_sync(0xffffffffu, r, 2);
+          r += __shfl_xor_sync(0xffffffffu, r, 1);
+          if ((lane & 3) == 0) (b2 ? sm.u0 : sm.e)[q * kQuarter + i + (b3 ? 2 : 0) + (lane >> 4)] = r;
         }
       }
       if (q == 0) {
@@ -353,35 +429,49 @@ __global__ void __launch_bounds__(384, 2) mamba_scan_bwd_kernel(MambaParams w, c
       gdtb += gdt;
       ga += gl * sm.s.dt[tid] * neg_a;
     }
-    // ---- through SiLU
-    for (int i = tid; i < kLen * kCh; i += 384) {
-      const int r = i / kCh, ch = i % kCh;
-      const float u = convolve(sm.s, w, r, ch, conv_channel(ch, h, hid)), sg = sigmoid(u);
-      if (ch < 16) gd = fmaf(sm.gy[r][ch], u * sg, gd);
-      sm.g[r][ch] = t0 + r < T ? sm.g[r][ch] * sg * (1.f + u * (1.f - sg)) : 0.f;
-    }
-    __syncthreads();
-    // ---- through the convolution: inputs, weights, bias
-    for (int i = tid; i < kLen * kCh; i += 384) {
-      const int r = i / kCh, cc = i % kCh;
-      if (t0 + r < T) {
-        const int chn = conv_channel(cc, h, hid);
-        float v = 0.f;
+    // ---- through SiLU; the convolution's weights and bias
+    {
+      const Taps taps(w, chn);
+      float v[kTaps];
 #pragma unroll
-        for (int k = 0; k < kTaps; ++k) v = fmaf(__ldg(w.conv_w + chn * kTaps + k), sm.g[r + kHalo - k][cc], v);
-        gproj[(static_cast<long long>(b) * T + t0 + r) * ld + proj_col(cc, h, hid)] = v;
+      for (int k = 0; k < kHalo; ++k) v[k + 1] = sm.s.raw[pg * kRows + k][pc];
+#pragma unroll
+      for (int i = 0; i < kRows; ++i) {
+        const int r = pg * kRows + i;
+#pragma unroll
+        for (int k = 0; k < kHalo; ++k) v[k] = v[k + 1];
+        v[kHalo] = sm.s.raw[r + kHalo][pc];
+        const float u = taps(v), sg = sigmoid(u);
+        if (pc < 16) gd = fmaf(sm.gy[r][pc], u * sg, gd);
+        const float g = t0 + r < T ? sm.g[r][pc] * sg * (1.f + u * (1.f - sg)) : 0.f;
+        sm.g[r][pc] = g;
+        gbias += g;
+#pragma unroll
+        for (int k = 0; k < kTaps; ++k) gw[k] = fmaf(g, v[k], gw[k]);
       }
     }
+    __syncthreads();
+    // ---- through the convolution: inputs
+    {
+      const Taps taps(w, chn);
+      float* const to = gproj + (static_cast<long long>(b) * T + t0 + pg * kRows) * ld + proj_col(pc, h, hid);
+      float v[kTaps];   // v[k]: row r + k
 #pragma unroll
-    for (int i = 0; i < kLen / 8; ++i) {
-      const int r = pg * (kLen / 8) + i;
-      const float g = sm.g[r][pc];
-      gbias += g;
+      for (int k = 0; k < kHalo; ++k) v[k + 1] = sm.g[pg * kRows + k][pc];
 #pragma unroll
-      for (int k = 0; k < kTaps; ++k) gw[k] = fmaf(g, sm.s.raw[r + k][pc], gw[k]);
+      for (int i = 0; i < kRows; ++i) {
+        const int r = pg * kRows + i;
+#pragma unroll
+        for (int k = 0; k < kHalo; ++k) v[k] = v[k + 1];
+        v[kHalo] = sm.g[r + kHalo][pc];
+        float u = 0.f;
+#pragma unroll
+        for (int k = 0; k < kTaps; ++k) u = fmaf(taps.w[k], v[kHalo - k], u);
+        if (t0 + r < T) to[i * ld] = u;
+      }
     }
     __syncthreads();
-    for (int i = tid; i < kHalo * kCh; i += 384) sm.g[kLen + i / kCh][i % kCh] = sm.g[i / kCh][i % kCh];
+    for (int i = tid; i < kHalo * kCh; i += kThreads) sm.g[kLen + i / kCh][i % kCh] = sm.g[i / kCh][i % kCh];
     __syncthreads();
   }
   if (gh0 && task == 1 && q == 0) {
@@ -391,43 +481,29 @@ __global__ void __launch_bounds__(384, 2) mamba_scan_bwd_kernel(MambaParams w, c
   // ---- parameter gradients of this (sequence, head)
   float* const row = partial + static_cast<size_t>(b) * partial_floats(H);
   const int channels = 3 * hid;
-  const auto over_groups = [&](float v) {   // sum over the 8 step groups of a channel, at pg == 0
-    __syncthreads();
-    sm.red[tid] = v;
-    __syncthreads();
-    float t = 0.f;
-    if (pg == 0)
 #pragma unroll
-      for (int i = 0; i < 8; ++i) t += sm.red[i * kCh + pc];
-    return t;
-  };
-  const int chn = conv_channel(pc, h, hid);
+  for (int k = 0; k < kTaps; ++k) sm.sums.of_group[k][tid] = gw[k];
+  sm.sums.of_group[kTaps][tid] = gbias;
 #pragma unroll
-  for (int k = 0; k < kTaps; ++k) {
-    const float v = over_groups(gw[k]);
-    if (pg == 0) row[chn * kTaps + k] = v;
+  for (int o = 16; o > 0; o >>= 1) {
+    ga += __shfl_xor_sync(0xffffffffu, ga, o);
+    gdtb += __shfl_xor_sync(0xffffffffu, gdtb, o);
+    gd += __shfl_xor_sync(0xffffffffu, gd, o);
   }
-  {
-    const float v = over_groups(gbias);
-    if (pg == 0) row[channels * kTaps + chn] = v;
+  if (lane == 0) { sm.sums.of_warp[0][warp] = ga; sm.sums.of_warp[1][warp] = gdtb; sm.sums.of_warp[2][warp] = gd; }
+  __syncthreads();
+  for (int i = tid; i < (kTaps + 1) * kCh; i += kThreads) {
+    const int k = i / kCh, ch = i % kCh, to = conv_channel(ch, h, hid);
+    float v = 0.f;
+#pragma unroll
+    for (int j = 0; j < kGroups; ++j) v += sm.sums.of_group[k][j * kCh + ch];
+    row[k < kTaps ? to * kTaps + k : channels * kTaps + to] = v;
   }
-  const auto over_block = [&](float v) {
-    __syncthreads();
+  if (tid < 3) {
+    float v = 0.f;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) sm.red[warp] = v;
-    __syncthreads();
-    float t = 0.f;
-#pragma unroll
-    for (int i = 0; i < 12; ++i) t += sm.red[i];
-    return t;
-  };
-  float* const heads = row + channels * (kTaps + 1);
-  const float s_a = over_block(ga), s_b = over_block(gdtb), s_d = over_block(gd);
-  if (tid == 0) {
-    heads[h] = s_a;
-    heads[H + h] = s_b;
-    heads[2 * H + h] = s_d;
+    for (int i = 0; i < kThreads / 32; ++i) v += sm.sums.of_warp[tid][i];
+    row[channels * (kTaps + 1) + tid * H + h] = v;
   }
 }
 
@@ -495,9 +571,26 @@ __global__ void __launch_bounds__(256) mamba_gate_bwd_kernel(MambaParams w, cons
   }
 }
 
+// Parts of a stretch: a short sequence is one stretch without the steps that it does not have.  (us, forward / backward, with four parts and now:
+// 512 x 20 steps x 8 heads 53 / 204 and 33 / 104; 1024 x 1 x 8 93 / 383 and 53 / 106.  At 64 steps and more two parts, four blocks an SM, were no
+// faster: 128 x 64 x 8 backward 59 and 59.)
+int parts_of(int T) { return T <= kQuarter ? 1 : T <= 2 * kQuarter ? 2 : 4; }
+
+template <int kParts>
+int launch_scan_bwd(const MambaParams& w, const float* proj, long long ld, const uint8_t* done, const float* states, const float* gy_pre,
+                    const float* gh_last, float* gproj, float* gh0, float* partial, int B, int T, int H, cudaStream_t stream) {
+  if (const int st = allow_smem<mamba_scan_bwd_kernel<kParts>, sizeof(BwdSmem<kParts>)>(); st != MXK_OK) return st;
+  mxk::launch_kernel(mamba_scan_bwd_kernel<kParts>, B * H, kParts * 96, sizeof(BwdSmem<kParts>), stream, w, proj, ld, done, states, gy_pre, gh_last,
+                     gproj, gh0, partial, T, H);
+  return launch_status();
+}
+
 }  // namespace
 
-size_t mamba_state_floats(int B, int T, int H) { return static_cast<size_t>(B) * H * ((T + kLen - 1) / kLen) * kStates; }
+size_t mamba_state_floats(int B, int T, int H) {
+  const int len = parts_of(T) * kQuarter;
+  return static_cast<size_t>(B) * H * ((T + len - 1) / len) * kStates;
+}
 int mamba_partial_floats(int H) { return partial_floats(H); }
 int mamba_gate_blocks(long long tokens) {
   const long long need = (tokens + 7) / 8;
@@ -507,7 +600,9 @@ int mamba_gate_blocks(long long tokens) {
 int mamba_scan_fwd(const MambaParams& w, const float* proj, long long ld, const float* h0, const float* a0, const uint8_t* done,
                    float* y_pre, float* h_last, float* a_last, float* states, int B, int T, int H, cudaStream_t stream) {
   if (B <= 0 || T <= 0 || H <= 0) return MXK_ERR_DIMS;
-  mxk::launch_kernel(mamba_scan_fwd_kernel, B * H, 128, 0, stream, w, proj, ld, h0, a0, done, y_pre, h_last, a_last, states, T, H);
+  const bool whole = parts_of(T) == 4;   // one warp has too few threads for the 48 channels
+  mxk::launch_kernel(whole ? mamba_scan_fwd_kernel<4> : mamba_scan_fwd_kernel<2>, B * H, whole ? 128 : 64, 0, stream, w, proj, ld, h0, a0, done, y_pre,
+                     h_last, a_last, states, T, H);
   return launch_status();
 }
 
@@ -515,10 +610,8 @@ int mamba_scan_bwd(const MambaParams& w, const float* proj, long long ld, const 
                    const float* gy_pre, const float* gh_last, float* gproj, float* gh0,
                    float* partial, int B, int T, int H, cudaStream_t stream) {
   if (B <= 0 || T <= 0 || H <= 0) return MXK_ERR_DIMS;
-  if (const int st = allow_smem<mamba_scan_bwd_kernel, sizeof(BwdSmem)>(); st != MXK_OK) return st;
-  mxk::launch_kernel(mamba_scan_bwd_kernel, B * H, 384, sizeof(BwdSmem), stream, w, proj, ld, done, states, gy_pre, gh_last, gproj, gh0, partial,
-                                                                 T, H);
-  return launch_status();
+  const auto launch = parts_of(T) == 1 ? launch_scan_bwd<1> : parts_of(T) == 2 ? launch_scan_bwd<2> : launch_scan_bwd<4>;
+  return launch(w, proj, ld, done, states, gy_pre, gh_last, gproj, gh0, partial, B, T, H, stream);
 }
 
 int mamba_gate_fwd(const MambaParams& w, const float* proj, long long ld, const float* y_pre, float* z, long long tokens, int H,

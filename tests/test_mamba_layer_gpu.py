@@ -50,6 +50,13 @@ def test_mamba_layer_and_its_gradients(shape, with_carry):
         assert err(got, r) <= 1e-4, (name, err(got, r))
 
 
+# one, two and four parts of 16 steps, on both sides of each; the last two have more blocks than fit at a time
+@pytest.mark.parametrize("shape", [(3, 15, 8, 3), (2, 17, 8, 2), (2, 31, 8, 3), (2, 32, 8, 2), (2, 33, 8, 4), (2, 64, 8, 3), (150, 16, 8, 8), (70, 97, 8, 8)])
+@pytest.mark.parametrize("with_carry", [False, True])
+def test_parts_of_a_stretch(shape, with_carry):
+    test_mamba_layer_and_its_gradients(shape, with_carry)
+
+
 # the gate's backward pass keeps 512 bytes of shared memory a head: more of it in a later call than in an earlier one, and
 # on both sides of what an SM has
 def test_head_counts_one_after_another():
