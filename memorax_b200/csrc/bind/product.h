@@ -11,11 +11,10 @@ namespace mxk_host {
 // 2 M N K above which a product is the library's.  On the GPU its two-SM tiles are the faster form at nearly every size
 // (by 1.1 to 1.6, up to 3.4 for weight gradients); below the line a pass waits for the host, which a library call holds up for
 // longer.
-// Passes with gradients, with the line at 1e8 | 4e9 | 8e9 | 2e10, in microseconds: linear attention (4 heads of 64), 4096 x 256:
-// 207 | 166 | 167 | 168; 8192 x 512: 207 | 188 | 164 | 166; 16384 x 512: 210 | 205 | 186 | 181; 65536 x 512: 452 | 450 | 451 |
-// 474.  Delta rule, 8192 x 512, 4 heads of 128: 261 | 253 | 249 | 386 (rows of its joint projection are not 32-byte aligned,
-// which costs gemm16 its wide stores); 32768 x 256, 4 heads of 64: 350 | 338 | 336 | 571.  mLSTM, 6016 x 256: 351 | 290 | 291 |
-// 289; 65536 x 512: 2586 | 2994 | 2950 | 3045 (the sums into existing tensors, which the line does not tell apart).
+// Passes with gradients, with the line at 4e9 | 8e9 | 2e10, in microseconds: linear attention (4 heads of 64), 8192 x 512: 185 | 160 | 159;
+// 16384 x 512: 199 | 185 | 169; 32768 x 512: 266 | 266 | 274; 65536 x 512: 447 | 448 | 470.  Delta rule, 8192 x 512, 4 heads of 128:
+// 252 | 245 | 251; 32768 x 256, 4 heads of 64: 329 | 333 | 343.  mLSTM, 6016 x 256: 237 | 239 | 237; 16384 x 512: 840 | 835 | 840;
+// 65536 x 256: 1338 | 1404 | 1408; 65536 x 512: 2621 | 2613 | 2733.
 constexpr double kLibraryFlops = 8e9;
 // The same for the gradient of a weight, whose long contraction the kernel splits over all SMs (GPU time alone, own | library in
 // microseconds): 256 x 256 over 65536 tokens 14 | 25, 768 x 256 over 32768 18 | 20, 512 x 512 over 32768 22 | 27, 1024 x 512 over 16384

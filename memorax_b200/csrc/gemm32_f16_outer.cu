@@ -8,8 +8,10 @@
 // relative 2-norm, normal entries: 2.1e-7 at 4096 tokens, 2.4e-7 at 24000 (three bf16 planes, drained every 512 tokens: 4.3e-7 and
 // 4.7e-7); lognormal, sigma 3: 1.1e-7 (4.0e-7).
 //
-// Bound: the producers.  A stage of 256 x 128 is 768 cycles of the tensor pipe and 12288 numbers to convert, about 1200 cycles of
-// the issue slots, and takes 2400: the twelve warps wait for the same barriers and are in the same phase of their work.
+// Bound: shared memory and the producers.  A stage of 256 x 128 is 768 cycles of the tensor pipe and 12288 numbers to convert, about
+// 1200 cycles of the issue slots; they cross shared memory five times over (the copy in, the producers' reads, the planes, the pipe's
+// reads of A and of both halves of B: 1920 cycles at 128 bytes), and it takes 2400: the twelve warps wait for the same barriers and
+// are in the same phase of their work.
 // Measured (three bf16 planes before): 1024 x 256 over 65536 tokens 151 us (185), 1024 x 512 over 24000 114 us (137), 520 x 512
 // over 8192 36 us (38).
 //

@@ -15,7 +15,8 @@
 // so three groups of four warps run side by side: C's cotangent from the states (lane = n), x's (lane = p) and B's
 // (lane = n) from the cotangent of the states.  The first group leaves every h_{t-1} in shared memory for the third,
 // which has the decay's cotangent <dh_t, h_{t-1}> as a plain dot product (as a difference of larger sums it lost two
-// digits).  Sums over lanes are taken for four steps together, 9 shuffles instead of 24.  128 x 64 x 8: 81 -> 59 us, 128 x 250 x 8: 321 -> 240, 1 x 2048 x 8: 635 -> 450.
+// digits).  Sums over lanes are taken for four steps together, 9 shuffles instead of 24.  128 x 64 x 8: 81 -> 59 us,
+// 128 x 250 x 8: 321 -> 240, 1 x 2048 x 8: 635 -> 450.
 #include "layers.cuh"
 #include "mxk_common.cuh"
 
