@@ -1,9 +1,11 @@
 // The elementwise work around the mLSTM layer's products and chunk kernels (mlstm.py:129-229), bf16 in and out, float32
 // arithmetic: causal convolution + SiLU, gates and key scaling, head-wise LayerNorm + skip + output gate, and their
-// gradients.  All HBM-bound, one read and one write of each operand; a thread owns eight channels (16 bytes) and walks
+// gradients.  Bound by HBM, one read and one write of each operand; a thread owns eight or four channels and walks
 // tokens, so that the convolution's window and the parameter gradients stay in registers.  (As separate torch calls they
 // were about sixty launches of a layer step.)
 #include <cuda_bf16.h>
+
+#include <algorithm>
 
 #include "layers.cuh"
 #include "mxk_common.cuh"
@@ -14,6 +16,7 @@ namespace layers {
 namespace {
 
 using umma::pack8_bf16;
+using umma::pack_bf16;
 using umma::unpack8_bf16;
 using bf16 = __nv_bfloat16;
 
@@ -24,6 +27,10 @@ __device__ __forceinline__ float softplus(float x) { return x > 20.f ? x : log1p
 // a value that the bf16 layer holds in memory
 __device__ __forceinline__ float held(float x) { return __bfloat162float(__float2bfloat16(x)); }
 __device__ __forceinline__ void load8(const bf16* p, float* x) { unpack8_bf16(*reinterpret_cast<const uint4*>(p), x); }
+__device__ __forceinline__ void unpack4(uint2 v, float2* x) {
+  x[0] = make_float2(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u));
+  x[1] = make_float2(__uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
+}
 __device__ __forceinline__ void store8(bf16* p, const float* x) { *reinterpret_cast<uint4*>(p) = pack8_bf16(x); }
 
 struct Taps {
@@ -90,119 +97,130 @@ __global__ void __launch_bounds__(256) conv_fwd_kernel(const bf16* __restrict__ 
   }
 }
 
-// A thread walks its run and the three steps after it: the convolution's output is recomputed, its cotangent
-// g_t = gu_t silu'(.) meets the four inputs it came from.
+// A thread walks runs of four channels, and the three steps after each: the convolution's output is recomputed, its cotangent
+// g_t = gu_t silu'(.) meets the four inputs it came from.  Inputs and their cotangents are rings of four steps, the loop's unrolling.
+// Bound: the instructions of an element (about 25, in pairs), at two blocks an SM beside HBM (8 bytes an element).  65536 x 512: 145 us;
+// eight channels a thread, one block of 223 registers an SM, windows moved along by copies and loads two steps ahead: 257.  6016 x 256: 14.5 (31.5).
 template <int kRun>
-__global__ void __launch_bounds__(256) conv_bwd_kernel(const bf16* __restrict__ up, long long ld, const bf16* __restrict__ conv_w,
-                                                       const bf16* __restrict__ conv_b, const bf16* __restrict__ gu,
-                                                       const bf16* __restrict__ gx, bf16* __restrict__ gup,
-                                                       float* __restrict__ partial, int B, int T, int hid, int runs, int lanes) {
+__global__ void __launch_bounds__(256, 2) conv_bwd_kernel(const bf16* __restrict__ up, long long ld, const bf16* __restrict__ conv_w,
+                                                          const bf16* __restrict__ conv_b, const bf16* __restrict__ gu,
+                                                          const bf16* __restrict__ gx, bf16* __restrict__ gup,
+                                                          float* __restrict__ partial, int B, int T, int hid, int runs, int lanes) {
   enter_kernel();
   extern __shared__ float red[];   // [channel][taps + bias] sums of the block's runs, one run group at a time
-  const int groups = hid / 8;
-  // a block: `lanes` channel groups (a divisor of both 256 and groups) x 256 / lanes runs
-  const int cg = blockIdx.y * lanes + threadIdx.x % lanes, c = cg * 8;
-  const long long seq_run = static_cast<long long>(blockIdx.x) * (256 / lanes) + threadIdx.x / lanes;
-  const int b = static_cast<int>(seq_run / runs), t0 = static_cast<int>(seq_run % runs) * kRun;
-  float gw[kTaps][8], gb[8];
+  // a block: `lanes` groups of four channels (a divisor of both 256 and of all of them) x 256 / lanes runs
+  const int l = threadIdx.x % lanes, rg = threadIdx.x / lanes, c = (blockIdx.y * lanes + l) * 4;
+  float2 w[kTaps][2], bias[2], gw[kTaps][2], gb[2];
+  {
+    float raw[4 * kTaps];
+    load8(conv_w + c * kTaps, raw);
+    load8(conv_w + c * kTaps + 8, raw + 8);
 #pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    gb[e] = 0.f;
-#pragma unroll
-    for (int k = 0; k < kTaps; ++k) gw[k][e] = 0.f;
+    for (int k = 0; k < kTaps; ++k) {
+      w[k][0] = make_float2(raw[k], raw[kTaps + k]);
+      w[k][1] = make_float2(raw[2 * kTaps + k], raw[3 * kTaps + k]);
+    }
+    unpack4(*reinterpret_cast<const uint2*>(conv_b + c), bias);
   }
-  if (b < B) {
-    const Taps taps(conv_w, conv_b, c);
-    float win[kTaps][8], acc[kTaps][8];   // inputs t-3..t; cotangents of inputs t-3..t
+  const float2 zero = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int k = 0; k < kTaps; ++k)
+  for (int h = 0; h < 2; ++h) {
+    gb[h] = zero;
 #pragma unroll
-      for (int e = 0; e < 8; ++e) win[k][e] = acc[k][e] = 0.f;
+    for (int k = 0; k < kTaps; ++k) gw[k][h] = zero;
+  }
+  const long long all = static_cast<long long>(B) * runs;
+  for (long long run = static_cast<long long>(blockIdx.x) * (256 / lanes) + rg; run < all; run += static_cast<long long>(gridDim.x) * (256 / lanes)) {
+    const int b = static_cast<int>(run / runs), t0 = static_cast<int>(run % runs) * kRun;
+    const long long tok0 = static_cast<long long>(b) * T + t0;
+    const bf16* const pu = up + tok0 * ld + c;
+    const bf16* const pg = gu + tok0 * hid + c;
+    const bf16* const px = gx + tok0 * hid + c;
+    bf16* const po = gup + tok0 * ld + c;
+    const auto at = [](const bf16* from) { return *reinterpret_cast<const uint2*>(from); };
+    uint2 nu[4], ng[4], nx[4];   // four steps, already on their way
 #pragma unroll
-    for (int k = 0; k < kTaps - 1; ++k) {
-      const int t = t0 - (kTaps - 1) + k;
-      if (t >= 0) load8(up + (static_cast<long long>(b) * T + t) * ld + c, win[k]);
-    }
-    const bf16* pu = up + (static_cast<long long>(b) * T + t0) * ld + c;
-    const bf16* pg = gu + (static_cast<long long>(b) * T + t0) * hid + c;
-    const bf16* px = gx + (static_cast<long long>(b) * T + t0) * hid + c;
-    constexpr int kAhead = 2;
-    uint4 nu[kAhead], ng[kAhead], nx[kAhead];   // the steps after this one, already on their way
-#pragma unroll
-    for (int i = 0; i < kAhead; ++i) {
+    for (int i = 0; i < 4; ++i)
       if (t0 + i < T) {
-        nu[i] = *reinterpret_cast<const uint4*>(pu + i * ld);
-        ng[i] = *reinterpret_cast<const uint4*>(pg + i * hid);
-        nx[i] = *reinterpret_cast<const uint4*>(px + i * hid);
+        nu[i] = at(pu + i * ld);
+        ng[i] = at(pg + i * hid);
+        nx[i] = at(px + i * hid);
       }
+    float2 win[4][2], acc[4][2];   // step t0 + i in slot i & 3
+#pragma unroll
+    for (int i = 1; i < 4; ++i) {
+      win[i][0] = win[i][1] = zero;
+      if (t0 + i - 4 >= 0) unpack4(at(pu + (i - 4) * ld), win[i]);
+      acc[i][0] = acc[i][1] = zero;
     }
-#pragma unroll kAhead
-    for (int i = 0; i < kRun + kTaps - 1; ++i) {
-      const int t = t0 + i;
-      const bool own = i < kRun;
-      const uint4 x_done = nx[(i + 1) % kAhead];   // of step t - 3 (the same slot: kAhead divides 4)
-      if (t < T) {
-        float g[8];
-        unpack8_bf16(nu[i % kAhead], win[kTaps - 1]);
-        unpack8_bf16(ng[i % kAhead], g);
-        if (t + kAhead < T && i + kAhead < kRun + kTaps - 1) {
-          nu[i % kAhead] = *reinterpret_cast<const uint4*>(pu + (i + kAhead) * ld);
-          ng[i % kAhead] = *reinterpret_cast<const uint4*>(pg + (i + kAhead) * hid);
-        }
+#pragma unroll 1
+    for (int i0 = 0; i0 < kRun + 4; i0 += 4) {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          float a = taps.b[e];
+      for (int s = 0; s < 4; ++s) {
+        const int i = i0 + s, t = t0 + i;
+        const uint2 x_done = nx[(s + 1) & 3];   // of step t - 3
+        acc[s][0] = acc[s][1] = zero;
+        if (t < T && i < kRun + kTaps - 1) {
+          const bool own = i < kRun;
+          float2 g[2];
+          unpack4(nu[s], win[s]);
+          unpack4(ng[s], g);
+          if (t + 4 < T && i + 4 < kRun + kTaps - 1) {
+            nu[s] = at(pu + (i + 4) * ld);
+            ng[s] = at(pg + (i + 4) * hid);
+          }
 #pragma unroll
-          for (int k = 0; k < kTaps; ++k) a = fmaf(taps.w[k][e], win[k][e], a);
-          a = held(a);
-          const float s = sigmoid(a);
-          g[e] *= s * (1.f + a * (1.f - s));
-          if (own) gb[e] += g[e];
+          for (int h = 0; h < 2; ++h) {
+            float2 a = bias[h];
 #pragma unroll
-          for (int k = 0; k < kTaps; ++k) {
-            acc[k][e] = fmaf(taps.w[k][e], g[e], acc[k][e]);
-            if (own) gw[k][e] = fmaf(g[e], win[k][e], gw[k][e]);
+            for (int k = 0; k < kTaps; ++k) a = __ffma2_rn(w[k][h], win[(s + 1 + k) & 3][h], a);
+            a = make_float2(held(a.x), held(a.y));
+            const float sx = sigmoid(a.x), sy = sigmoid(a.y);
+            g[h].x *= sx * (1.f + a.x * (1.f - sx));
+            g[h].y *= sy * (1.f + a.y * (1.f - sy));
+#pragma unroll
+            for (int k = 0; k < kTaps; ++k) acc[(s + 1 + k) & 3][h] = __ffma2_rn(w[k][h], g[h], acc[(s + 1 + k) & 3][h]);
+            if (own) {
+              gb[h].x += g[h].x;
+              gb[h].y += g[h].y;
+#pragma unroll
+              for (int k = 0; k < kTaps; ++k) gw[k][h] = __ffma2_rn(g[h], win[(s + 1 + k) & 3][h], gw[k][h]);
+            }
           }
         }
-      }
-      // input t - 3 has met every output it reaches
-      const int done = t - (kTaps - 1);
-      if (done >= t0 && done < T) {
-        const long long dt = static_cast<long long>(b) * T + done;
-        float x[8];
-        unpack8_bf16(x_done, x);
-        if (done + kAhead < T && done + kAhead < t0 + kRun)
-          nx[(i + 1) % kAhead] = *reinterpret_cast<const uint4*>(px + (i - (kTaps - 1) + kAhead) * hid);
+        // input t - 3 has met every output it reaches
+        const int done = i - (kTaps - 1);
+        if (done >= 0 && done < kRun && t0 + done < T) {
+          float2 x[2];
+          unpack4(x_done, x);
+          if (done + 4 < kRun && t0 + done + 4 < T) nx[(s + 1) & 3] = at(px + (done + 4) * hid);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) x[e] += acc[0][e];
-        store8(gup + dt * ld + c, x);
-      }
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-#pragma unroll
-        for (int k = 0; k < kTaps - 1; ++k) { win[k][e] = win[k + 1][e]; acc[k][e] = acc[k + 1][e]; }
-        acc[kTaps - 1][e] = 0.f;
+          for (int h = 0; h < 2; ++h) {
+            x[h].x += acc[(s + 1) & 3][h].x;
+            x[h].y += acc[(s + 1) & 3][h].y;
+          }
+          *reinterpret_cast<uint2*>(po + done * ld) = make_uint2(pack_bf16(x[0].x, x[0].y), pack_bf16(x[1].x, x[1].y));
+        }
       }
     }
   }
   // block sums, run groups added in order
-  const int l = threadIdx.x % lanes, rg = threadIdx.x / lanes;
   for (int r = 0; r < 256 / lanes; ++r) {
     __syncthreads();
     if (rg == r) {
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        float* row = red + (l * 8 + e) * (kTaps + 1);
+      for (int e = 0; e < 4; ++e) {
+        float* const row = red + (l * 4 + e) * (kTaps + 1);
 #pragma unroll
-        for (int k = 0; k < kTaps; ++k) row[k] = (r ? row[k] : 0.f) + gw[k][e];
-        row[kTaps] = (r ? row[kTaps] : 0.f) + gb[e];
+        for (int k = 0; k < kTaps; ++k) row[k] = (r ? row[k] : 0.f) + (e & 1 ? gw[k][e >> 1].y : gw[k][e >> 1].x);
+        row[kTaps] = (r ? row[kTaps] : 0.f) + (e & 1 ? gb[e >> 1].y : gb[e >> 1].x);
       }
     }
   }
   __syncthreads();
   float* const out = partial + static_cast<size_t>(blockIdx.x) * hid * (kTaps + 1);
-  for (int i = threadIdx.x; i < lanes * 8 * (kTaps + 1); i += 256) {
-    const int ch = blockIdx.y * lanes * 8 + i / (kTaps + 1), k = i % (kTaps + 1);
+  for (int i = threadIdx.x; i < lanes * 4 * (kTaps + 1); i += 256) {
+    const int ch = blockIdx.y * lanes * 4 + i / (kTaps + 1), k = i % (kTaps + 1);
     out[k < kTaps ? ch * kTaps + k : hid * kTaps + ch] = red[i];
   }
 }
@@ -410,10 +428,10 @@ __global__ void __launch_bounds__(256) out_bwd_kernel(const bf16* __restrict__ g
 // walks them one after the other)
 int run_of(int B, int T, int hid) { return static_cast<long long>(B) * T * (hid / 8) >= 16LL * 512 * kNumSMs ? 16 : 4; }
 int runs_of(int T, int run) { return (T + run - 1) / run; }
-// channel groups side by side in a block of the convolution's backward pass: 16 (128 channels) or what divides
+// groups of four channels side by side in a block of the convolution's backward pass: 32 or what divides
 int conv_lanes(int hid) {
-  int l = 16;
-  while ((hid / 8) % l) l /= 2;
+  int l = 32;
+  while ((hid / 4) % l) l /= 2;
   return l;
 }
 
@@ -430,17 +448,18 @@ int mlstm_conv_fwd(const void* up, long long ld, const void* conv_w, const void*
   return run == 16 ? go(conv_fwd_kernel<16>) : go(conv_fwd_kernel<4>);
 }
 
+// of runs; a wave at most, since every one leaves a row of sums
 int mlstm_conv_blocks(int B, int T, int hid) {
-  const int per = 256 / conv_lanes(hid);
-  return static_cast<int>((static_cast<long long>(B) * runs_of(T, run_of(B, T, hid)) + per - 1) / per);
+  const int lanes = conv_lanes(hid), per = 256 / lanes, most = std::max(1, 2 * kNumSMs / (hid / 4 / lanes));
+  return static_cast<int>(std::min<long long>(most, (static_cast<long long>(B) * runs_of(T, run_of(B, T, hid)) + per - 1) / per));
 }
 
 int mlstm_conv_bwd(const void* up, long long ld, const void* conv_w, const void* conv_b, const void* gu, const void* gx, void* gup,
                    float* partial, int B, int T, int hid, cudaStream_t stream) {
-  const int lanes = conv_lanes(hid), bytes = lanes * 8 * (kTaps + 1) * static_cast<int>(sizeof(float));
+  const int lanes = conv_lanes(hid), bytes = lanes * 4 * (kTaps + 1) * static_cast<int>(sizeof(float));
   const int run = run_of(B, T, hid), runs = runs_of(T, run);
   const auto go = [&](auto kernel) {
-    mxk::launch_kernel(kernel, dim3(mlstm_conv_blocks(B, T, hid), hid / 8 / lanes), 256, bytes, stream, static_cast<const bf16*>(up), ld, static_cast<const bf16*>(conv_w), static_cast<const bf16*>(conv_b), static_cast<const bf16*>(gu),
+    mxk::launch_kernel(kernel, dim3(mlstm_conv_blocks(B, T, hid), hid / 4 / lanes), 256, bytes, stream, static_cast<const bf16*>(up), ld, static_cast<const bf16*>(conv_w), static_cast<const bf16*>(conv_b), static_cast<const bf16*>(gu),
         static_cast<const bf16*>(gx), static_cast<bf16*>(gup), partial, B, T, hid, runs, lanes);
     return launch_status();
   };
