@@ -55,6 +55,17 @@ __device__ __forceinline__ void load_tile(void* dst, const CUtensorMap* map, uin
       "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
       : "memory");
 }
+// Sixteen elements of a row on 32 or on 16 bytes.
+__device__ __forceinline__ void store16(__nv_bfloat16* dst, const uint32_t* w, bool on32) {
+  if (on32) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]),
+                 "r"(w[5]), "r"(w[6]), "r"(w[7])
+                 : "memory");
+  } else {
+    reinterpret_cast<uint4*>(dst)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+    reinterpret_cast<uint4*>(dst)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+  }
+}
 __device__ __forceinline__ void arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
@@ -171,9 +182,52 @@ __global__ void __launch_bounds__(kThreads, 1) gemm16_kernel(const __grid_consta
       const int sp = at.sp, z = at.z, n0 = at.n0, m = at.m0 + sub * 32 + lane;
       const bool in = m < p.M;
       const int buf = turn & 1;
+      const uint32_t src = tmem + buf * BN + (static_cast<uint32_t>(sub * 32) << 16);
+      if (p.accumulate && p.splits == 1 && p.vec >= 8 && !p.bias && n0 + BN <= p.N) {
+        // a whole row of the tile to be added to: all of it is on its way while the product is formed (32 bytes after another
+        // left HBM waiting: 65536 x 1536 x 16 211 us, 16 bytes 143, 102 now)
+        __nv_bfloat16* const dst = p.c + z * p.c_batch_stride + m * p.ldc + n0;
+        uint32_t had[BN / 16][8];
+        if (in) {
+#pragma unroll
+          for (int i = 0; i < BN / 16; ++i) {
+            uint32_t* const h = had[i];
+            if (p.vec == 16) {
+              asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                           : "=r"(h[0]), "=r"(h[1]), "=r"(h[2]), "=r"(h[3]), "=r"(h[4]), "=r"(h[5]), "=r"(h[6]), "=r"(h[7])
+                           : "l"(dst + 16 * i)
+                           : "memory");
+            } else {
+              const uint4 x = reinterpret_cast<const uint4*>(dst)[2 * i], y = reinterpret_cast<const uint4*>(dst)[2 * i + 1];
+              h[0] = x.x; h[1] = x.y; h[2] = x.z; h[3] = x.w;
+              h[4] = y.x; h[5] = y.y; h[6] = y.z; h[7] = y.w;
+            }
+          }
+        }
+        mbar_wait_flag(&acc_full[buf], (turn >> 1) & 1, timed_out);
+        fence_after_sync();
+#pragma unroll
+        for (int i = 0; i < BN / 16; ++i) {
+          float v[16];
+          __syncwarp();
+          tmem_ld8(src + i * 16, v);
+          tmem_ld8(src + i * 16 + 8, v + 8);
+          tmem_ld_wait();
+          if (in) {
+            uint32_t w[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+              w[e] = pack_bf16(v[2 * e] + __uint_as_float(had[i][e] << 16), v[2 * e + 1] + __uint_as_float(had[i][e] & 0xffff0000u));
+            store16(dst + 16 * i, w, p.vec == 16);
+          }
+        }
+        fence_before_sync();
+        __syncwarp();
+        if (lane == 0) arrive(&acc_empty[buf]);
+        continue;
+      }
       mbar_wait_flag(&acc_full[buf], (turn >> 1) & 1, timed_out);
       fence_after_sync();
-      const uint32_t src = tmem + buf * BN + (static_cast<uint32_t>(sub * 32) << 16);
 #pragma unroll 1
       for (int c = 0; c < BN; c += 16) {
         if (n0 + c >= p.N) break;
@@ -214,17 +268,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm16_kernel(const __grid_consta
 #pragma unroll
                 for (int e = 0; e < 16; ++e) v[e] += had[e];
               }
-              if (p.vec == 16) {
-                uint32_t w[8];
+              uint32_t w[8];
 #pragma unroll
-                for (int e = 0; e < 8; ++e) w[e] = pack_bf16(v[2 * e], v[2 * e + 1]);
-                asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]),
-                             "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
-                             : "memory");
-              } else {
-                *reinterpret_cast<uint4*>(dst) = pack8_bf16(v);
-                *reinterpret_cast<uint4*>(dst + 8) = pack8_bf16(v + 8);
-              }
+              for (int e = 0; e < 8; ++e) w[e] = pack_bf16(v[2 * e], v[2 * e + 1]);
+              store16(dst, w, p.vec == 16);
             } else {
 #pragma unroll
               for (int e = 0; e < 16; ++e) {

@@ -57,6 +57,26 @@ def test_sums_into_rows_at_any_address(n, ld, at, k):
     ops.check_status()
 
 
+# sums into whole tiles, whose rows are fetched ahead, beside cut ones; rows on 32 and on 16 bytes, in batches
+@pytest.mark.parametrize("m", [1, 127, 300])
+@pytest.mark.parametrize("n", [56, 64, 128, 200, 320])
+@pytest.mark.parametrize("k", [8, 72])
+@pytest.mark.parametrize("pad", [0, 8])
+def test_sums_into_whole_tiles(m, n, k, pad):
+    from memorax_b200 import _C, ops
+    g = torch.Generator("cuda").manual_seed(m + n + k)
+    mk = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    a, b, held = mk(2, m, k), mk(2, k, n), mk(2, m + 3, n + pad)
+    c, before = held[:, :m, :n], held.clone()
+    want = a.double() @ b.double() + c.double()
+    _C.product_bf16(a, b, None, c)
+    # one rounding to bf16 of a float32 sum
+    assert float(((c.double() - want).abs() / (want.abs() + 1e-3)).max()) <= 2.0 ** -8 + 1e-4
+    held[:, :m, :n] = before[:, :m, :n]
+    assert torch.equal(held, before)
+    ops.check_status()
+
+
 # several products in one launch: of one size and of very different ones, batched and not, split and whole
 @pytest.mark.parametrize("tokens", [5, 700, 6000])
 @pytest.mark.parametrize("by_rows", [False, True])
