@@ -26,6 +26,12 @@ __device__ __forceinline__ float sigmoid(float x) { return 1.f / (1.f + __expf(-
 __device__ __forceinline__ float softplus(float x) { return x > 20.f ? x : log1pf(__expf(x)); }
 // a value that the bf16 layer holds in memory
 __device__ __forceinline__ float held(float x) { return __bfloat162float(__float2bfloat16(x)); }
+// The same for two and for eight: a conversion of a pair costs what one of a single value does, and the gate has eight to an element.
+__device__ __forceinline__ float2 held(float2 x) {
+  const uint32_t p = pack_bf16(x.x, x.y);
+  return make_float2(__uint_as_float(p << 16), __uint_as_float(p & 0xffff0000u));
+}
+__device__ __forceinline__ void hold8(float* x) { unpack8_bf16(pack8_bf16(x), x); }
 __device__ __forceinline__ void load8(const bf16* p, float* x) { unpack8_bf16(*reinterpret_cast<const uint4*>(p), x); }
 __device__ __forceinline__ void unpack4(uint2 v, float2* x) {
   x[0] = make_float2(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u));
@@ -33,68 +39,69 @@ __device__ __forceinline__ void unpack4(uint2 v, float2* x) {
 }
 __device__ __forceinline__ void store8(bf16* p, const float* x) { *reinterpret_cast<uint4*>(p) = pack8_bf16(x); }
 
+// The taps of four channels, in pairs.
 struct Taps {
-  float w[kTaps][8], b[8];
+  float2 w[kTaps][2], b[2];
   __device__ __forceinline__ Taps(const bf16* conv_w, const bf16* conv_b, int c) {
-    float raw[8 * kTaps];
+    float raw[4 * kTaps];
+    load8(conv_w + c * kTaps, raw);
+    load8(conv_w + c * kTaps + 8, raw + 8);
 #pragma unroll
-    for (int i = 0; i < kTaps; ++i) load8(conv_w + c * kTaps + i * 8, raw + i * 8);
-#pragma unroll
-    for (int e = 0; e < 8; ++e)
-#pragma unroll
-      for (int k = 0; k < kTaps; ++k) w[k][e] = raw[e * kTaps + k];
-    load8(conv_b + c, b);
+    for (int k = 0; k < kTaps; ++k) {
+      w[k][0] = make_float2(raw[k], raw[kTaps + k]);
+      w[k][1] = make_float2(raw[2 * kTaps + k], raw[3 * kTaps + k]);
+    }
+    unpack4(*reinterpret_cast<const uint2*>(conv_b + c), b);
   }
 };
 
+// A thread walks a run of four channels; inputs are a ring of four steps, the loop's unrolling, loads as far ahead.  65536 x 512:
+// 49 us (eight channels and moved windows 68); bound by instructions, the sigmoids' divisions among them (HBM 21).
 template <int kRun>   // tokens per thread
 __global__ void __launch_bounds__(256) conv_fwd_kernel(const bf16* __restrict__ up, long long ld, const bf16* __restrict__ conv_w,
                                                        const bf16* __restrict__ conv_b, bf16* __restrict__ u, int B, int T, int hid,
                                                        int runs) {
   enter_kernel();
-  const int groups = hid / 8;
+  const int groups = hid / 4;
   const long long id = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
-  const int c = static_cast<int>(id % groups) * 8;
+  const int c = static_cast<int>(id % groups) * 4;
   const long long seq_run = id / groups;
+  if (seq_run >= static_cast<long long>(B) * runs) return;
   const int b = static_cast<int>(seq_run / runs), t0 = static_cast<int>(seq_run % runs) * kRun;
-  if (b >= B) return;
-  const Taps taps(conv_w, conv_b, c);
-  float win[kTaps][8];
-#pragma unroll
-  for (int k = 0; k < kTaps - 1; ++k) {
-    const int t = t0 - (kTaps - 1) + k;
-    if (t >= 0) load8(up + (static_cast<long long>(b) * T + t) * ld + c, win[k]);
-    else
-#pragma unroll
-      for (int e = 0; e < 8; ++e) win[k][e] = 0.f;
-  }
-  const bf16* src = up + (static_cast<long long>(b) * T + t0) * ld + c;
-  uint4 next[4];   // four steps ahead: the loop waits for no load it has just issued
+  const long long tok0 = static_cast<long long>(b) * T + t0;
+  const bf16* const src = up + tok0 * ld + c;
+  bf16* const dst = u + tok0 * hid + c;
+  const auto at = [](const bf16* from) { return *reinterpret_cast<const uint2*>(from); };
+  uint2 next[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i)
-    if (t0 + i < T) next[i] = *reinterpret_cast<const uint4*>(src + i * ld);
-#pragma unroll 4
-  for (int i = 0; i < kRun; ++i) {
-    const int t = t0 + i;
-    if (t >= T) break;
-    const long long tok = static_cast<long long>(b) * T + t;
-    unpack8_bf16(next[i % 4], win[kTaps - 1]);
-    if (i + 4 < kRun && t + 4 < T) next[i % 4] = *reinterpret_cast<const uint4*>(src + (i + 4) * ld);
-    float v[8];
+    if (t0 + i < T) next[i] = at(src + i * ld);
+  float2 win[kTaps][2];   // step t0 + i in slot i & 3
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      float a = taps.b[e];
-#pragma unroll
-      for (int k = 0; k < kTaps; ++k) a = fmaf(taps.w[k][e], win[k][e], a);
-      a = held(a);
-      v[e] = a * sigmoid(a);
-    }
-    store8(u + tok * hid + c, v);
-#pragma unroll
-    for (int k = 0; k < kTaps - 1; ++k)
-#pragma unroll
-      for (int e = 0; e < 8; ++e) win[k][e] = win[k + 1][e];
+  for (int i = 1; i < 4; ++i) {
+    win[i][0] = win[i][1] = make_float2(0.f, 0.f);
+    if (t0 + i - 4 >= 0) unpack4(at(src + (i - 4) * ld), win[i]);
   }
+  const Taps taps(conv_w, conv_b, c);
+#pragma unroll 1
+  for (int i0 = 0; i0 < kRun; i0 += 4)
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      const int i = i0 + s;
+      if (t0 + i >= T) break;
+      unpack4(next[s], win[s]);
+      if (i + 4 < kRun && t0 + i + 4 < T) next[s] = at(src + (i + 4) * ld);
+      float2 v[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float2 a = taps.b[h];
+#pragma unroll
+        for (int k = 0; k < kTaps; ++k) a = __ffma2_rn(taps.w[k][h], win[(s + 1 + k) & 3][h], a);
+        a = held(a);
+        v[h] = make_float2(a.x * sigmoid(a.x), a.y * sigmoid(a.y));
+      }
+      *reinterpret_cast<uint2*>(dst + i * hid) = make_uint2(pack_bf16(v[0].x, v[0].y), pack_bf16(v[1].x, v[1].y));
+    }
 }
 
 // A thread walks runs of four channels, and the three steps after each: the convolution's output is recomputed, its cotangent
@@ -110,18 +117,8 @@ __global__ void __launch_bounds__(256, 2) conv_bwd_kernel(const bf16* __restrict
   extern __shared__ float red[];   // [channel][taps + bias] sums of the block's runs, one run group at a time
   // a block: `lanes` groups of four channels (a divisor of both 256 and of all of them) x 256 / lanes runs
   const int l = threadIdx.x % lanes, rg = threadIdx.x / lanes, c = (blockIdx.y * lanes + l) * 4;
-  float2 w[kTaps][2], bias[2], gw[kTaps][2], gb[2];
-  {
-    float raw[4 * kTaps];
-    load8(conv_w + c * kTaps, raw);
-    load8(conv_w + c * kTaps + 8, raw + 8);
-#pragma unroll
-    for (int k = 0; k < kTaps; ++k) {
-      w[k][0] = make_float2(raw[k], raw[kTaps + k]);
-      w[k][1] = make_float2(raw[2 * kTaps + k], raw[3 * kTaps + k]);
-    }
-    unpack4(*reinterpret_cast<const uint2*>(conv_b + c), bias);
-  }
+  const Taps taps(conv_w, conv_b, c);
+  float2 gw[kTaps][2], gb[2];
   const float2 zero = make_float2(0.f, 0.f);
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
@@ -171,15 +168,15 @@ __global__ void __launch_bounds__(256, 2) conv_bwd_kernel(const bf16* __restrict
           }
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
-            float2 a = bias[h];
+            float2 a = taps.b[h];
 #pragma unroll
-            for (int k = 0; k < kTaps; ++k) a = __ffma2_rn(w[k][h], win[(s + 1 + k) & 3][h], a);
-            a = make_float2(held(a.x), held(a.y));
+            for (int k = 0; k < kTaps; ++k) a = __ffma2_rn(taps.w[k][h], win[(s + 1 + k) & 3][h], a);
+            a = held(a);
             const float sx = sigmoid(a.x), sy = sigmoid(a.y);
             g[h].x *= sx * (1.f + a.x * (1.f - sx));
             g[h].y *= sy * (1.f + a.y * (1.f - sy));
 #pragma unroll
-            for (int k = 0; k < kTaps; ++k) acc[(s + 1 + k) & 3][h] = __ffma2_rn(w[k][h], g[h], acc[(s + 1 + k) & 3][h]);
+            for (int k = 0; k < kTaps; ++k) acc[(s + 1 + k) & 3][h] = __ffma2_rn(taps.w[k][h], g[h], acc[(s + 1 + k) & 3][h]);
             if (own) {
               gb[h].x += g[h].x;
               gb[h].y += g[h].y;
@@ -319,6 +316,8 @@ __device__ __forceinline__ float head_sum(float v) {
   return v;
 }
 
+// Bound by instructions: about eight roundings to bf16 and a sigmoid an element (HBM 42 us at 65536 x 512).  77 us with all loads before
+// the sums and roundings in pairs; 96 with u's and z's after them and single roundings.
 template <int LPH>
 __global__ void __launch_bounds__(256) out_fwd_kernel(const bf16* __restrict__ h, const bf16* __restrict__ u, const bf16* __restrict__ z,
                                                       long long ld, const bf16* __restrict__ norm_w, const bf16* __restrict__ skip,
@@ -328,8 +327,16 @@ __global__ void __launch_bounds__(256) out_fwd_kernel(const bf16* __restrict__ h
   const long long tok = i / hid8;
   const int c = static_cast<int>(i % hid8) * 8;
   const bool in = tok < tokens;
-  float x[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  if (in) load8(h + tok * hid8 * 8 + c, x);
+  uint4 raw[5] = {};   // all on their way before the sums of a head
+  if (in) {
+    raw[0] = *reinterpret_cast<const uint4*>(h + tok * hid8 * 8 + c);
+    raw[1] = *reinterpret_cast<const uint4*>(u + tok * hid8 * 8 + c);
+    raw[2] = *reinterpret_cast<const uint4*>(z + tok * ld + c);
+    raw[3] = *reinterpret_cast<const uint4*>(norm_w + c);
+    raw[4] = *reinterpret_cast<const uint4*>(skip + c);
+  }
+  float x[8];
+  unpack8_bf16(raw[0], x);
   float s = 0.f, q = 0.f;
 #pragma unroll
   for (int e = 0; e < 8; ++e) s += x[e];
@@ -339,18 +346,36 @@ __global__ void __launch_bounds__(256) out_fwd_kernel(const bf16* __restrict__ h
   const float rstd = rsqrtf(head_sum<LPH>(q) * (1.f / (8 * LPH)) + 1e-5f);
   if (!in) return;
   float w[8], sk[8], uu[8], zz[8];
-  load8(norm_w + c, w);
-  load8(skip + c, sk);
-  load8(u + tok * hid8 * 8 + c, uu);
-  load8(z + tok * ld + c, zz);
+  unpack8_bf16(raw[1], uu);
+  unpack8_bf16(raw[2], zz);
+  unpack8_bf16(raw[3], w);
+  unpack8_bf16(raw[4], sk);
 #pragma unroll
-  for (int e = 0; e < 8; ++e) x[e] = held(held(held((x[e] - mean) * rstd) * held(1.f + w[e])) + held(sk[e] * uu[e])) * held(zz[e] * sigmoid(zz[e]));
+  for (int e = 0; e < 8; ++e) {
+    x[e] = (x[e] - mean) * rstd;
+    w[e] += 1.f;
+    uu[e] *= sk[e];
+    zz[e] *= sigmoid(zz[e]);
+  }
+  hold8(x);
+  hold8(w);
+  hold8(uu);
+  hold8(zz);
+#pragma unroll
+  for (int e = 0; e < 8; ++e) x[e] *= w[e];
+  hold8(x);
+#pragma unroll
+  for (int e = 0; e < 8; ++e) x[e] += uu[e];
+  hold8(x);
+#pragma unroll
+  for (int e = 0; e < 8; ++e) x[e] *= zz[e];
   store8(g + tok * hid8 * 8 + c, x);
 }
 
-// A thread keeps its eight channels over all its tokens (256 / hid8 tokens side by side in a block).
+// A thread keeps its eight channels over all its tokens (256 / hid8 tokens side by side in a block), the next one's rows on their
+// way.  65536 x 512: 104 us (HBM 73); 150 with loads where they are used and single roundings.
 template <int LPH>
-__global__ void __launch_bounds__(256) out_bwd_kernel(const bf16* __restrict__ gg, const bf16* __restrict__ h, const bf16* __restrict__ u,
+__global__ void __launch_bounds__(256, 2) out_bwd_kernel(const bf16* __restrict__ gg, const bf16* __restrict__ h, const bf16* __restrict__ u,
                                                       const bf16* __restrict__ z, long long ld, const bf16* __restrict__ norm_w,
                                                       const bf16* __restrict__ skip, bf16* __restrict__ gh, bf16* __restrict__ gz,
                                                       long long ld_gz, bf16* __restrict__ gu, float* __restrict__ partial,
@@ -363,20 +388,31 @@ __global__ void __launch_bounds__(256) out_bwd_kernel(const bf16* __restrict__ g
   load8(norm_w + c, w);
   load8(skip + c, sk);
 #pragma unroll
-  for (int e = 0; e < 8; ++e) gw[e] = gs[e] = 0.f;
+  for (int e = 0; e < 8; ++e) {
+    gw[e] = gs[e] = 0.f;
+    w[e] += 1.f;
+  }
+  hold8(w);
   const long long step = static_cast<long long>(gridDim.x) * per;
+  uint4 raw[4];
+  const auto fetch = [&](long long tok) {
+    const bool in = tok < tokens;
+    const uint4 none = make_uint4(0, 0, 0, 0);
+    raw[0] = in ? *reinterpret_cast<const uint4*>(h + tok * hid8 * 8 + c) : none;
+    raw[1] = in ? *reinterpret_cast<const uint4*>(gg + tok * hid8 * 8 + c) : none;
+    raw[2] = in ? *reinterpret_cast<const uint4*>(u + tok * hid8 * 8 + c) : none;
+    raw[3] = in ? *reinterpret_cast<const uint4*>(z + tok * ld + c) : none;
+  };
+  fetch(static_cast<long long>(blockIdx.x) * per + ro);
   for (long long t0 = static_cast<long long>(blockIdx.x) * per; t0 < tokens; t0 += step) {   // all lanes stay for the shuffles
     const long long tok = t0 + ro;
     const bool in = tok < tokens;
     float x[8], g[8], uu[8], zz[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) x[e] = g[e] = uu[e] = zz[e] = 0.f;
-    if (in) {
-      load8(h + tok * hid8 * 8 + c, x);
-      load8(gg + tok * hid8 * 8 + c, g);
-      load8(u + tok * hid8 * 8 + c, uu);
-      load8(z + tok * ld + c, zz);
-    }
+    unpack8_bf16(raw[0], x);
+    unpack8_bf16(raw[1], g);
+    unpack8_bf16(raw[2], uu);
+    unpack8_bf16(raw[3], zz);
+    fetch(tok + step);
     float s = 0.f, q = 0.f;
 #pragma unroll
     for (int e = 0; e < 8; ++e) s += x[e];
@@ -385,19 +421,51 @@ __global__ void __launch_bounds__(256) out_bwd_kernel(const bf16* __restrict__ g
     for (int e = 0; e < 8; ++e) q = fmaf(x[e] - mean, x[e] - mean, q);
     const float rstd = rsqrtf(head_sum<LPH>(q) * (1.f / (8 * LPH)) + 1e-5f);
     float s1 = 0.f, s2 = 0.f;
+    // in the order of the layer: normed, scaled, skip and sum before the output gate; then their cotangents
+    float n[8], y[8], t[8], sg[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) n[e] = x[e] = (x[e] - mean) * rstd;
+    hold8(n);
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-      const float sg = sigmoid(zz[e]), silu = held(zz[e] * sg), xh = (x[e] - mean) * rstd;
-      const float y = held(held(held(xh) * held(1.f + w[e])) + held(sk[e] * uu[e]));   // before the output gate
-      zz[e] = held(g[e] * y) * sg * (1.f + zz[e] * (1.f - sg));
-      g[e] = held(g[e] * silu);                               // cotangent of y
-      gw[e] += held(g[e] * held(xh));
-      gs[e] += held(g[e] * uu[e]);
+      y[e] = n[e] * w[e];
+      t[e] = sk[e] * uu[e];
+    }
+    hold8(y);
+    hold8(t);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) y[e] += t[e];
+    hold8(y);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      sg[e] = sigmoid(zz[e]);
+      t[e] = zz[e] * sg[e];
+      y[e] *= g[e];
+    }
+    hold8(t);
+    hold8(y);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      zz[e] = y[e] * sg[e] * (1.f + zz[e] * (1.f - sg[e]));
+      g[e] *= t[e];
+    }
+    hold8(g);   // cotangent of the sum
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      n[e] *= g[e];
+      t[e] = g[e] * uu[e];
       uu[e] = g[e] * sk[e];
-      g[e] = held(g[e] * held(1.f + w[e]));
-      x[e] = xh;
+      g[e] *= w[e];
+    }
+    hold8(n);
+    hold8(t);
+    hold8(g);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      gw[e] += n[e];
+      gs[e] += t[e];
       s1 += g[e];
-      s2 = fmaf(g[e], xh, s2);
+      s2 = fmaf(g[e], x[e], s2);
     }
     s1 = head_sum<LPH>(s1) * (1.f / (8 * LPH));
     s2 = head_sum<LPH>(s2) * (1.f / (8 * LPH));
@@ -440,7 +508,7 @@ int conv_lanes(int hid) {
 int mlstm_conv_fwd(const void* up, long long ld, const void* conv_w, const void* conv_b, void* u, int B, int T, int hid,
                    cudaStream_t stream) {
   const int run = run_of(B, T, hid), runs = runs_of(T, run);
-  const long long threads = static_cast<long long>(B) * runs * (hid / 8);
+  const long long threads = static_cast<long long>(B) * runs * (hid / 4);
   const auto go = [&](auto kernel) {
     mxk::launch_kernel(kernel, static_cast<unsigned>((threads + 255) / 256), 256, 0, stream, static_cast<const bf16*>(up), ld, static_cast<const bf16*>(conv_w), static_cast<const bf16*>(conv_b), static_cast<bf16*>(u), B, T, hid, runs);
     return launch_status();
