@@ -57,6 +57,13 @@ def test_parts_of_a_stretch(shape, with_carry):
     test_mamba_layer_and_its_gradients(shape, with_carry)
 
 
+# rows of the gate in four and in eight registers a lane, cut and whole, and longer ones; several tokens to a warp
+@pytest.mark.parametrize("heads", [1, 3, 8, 9, 16, 17])
+@pytest.mark.parametrize("bsz", [2, 290])
+def test_rows_of_the_gate(heads, bsz):
+    test_mamba_layer_and_its_gradients((bsz, 17, 8, heads), False)
+
+
 # the gate's backward pass keeps 512 bytes of shared memory a head: more of it in a later call than in an earlier one, and
 # on both sides of what an SM has
 def test_head_counts_one_after_another():
