@@ -186,7 +186,9 @@ __device__ __forceinline__ void split8(const float* x, float s, uint4& hi, uint4
 __device__ __forceinline__ int placed(int n) { return 8 * ((n >> 1) & 3) + 2 * (n >> 3) + (n & 1); }
 
 constexpr int kBM = 128;
-constexpr int kSlots = 8;      // stages whose units and events are kept: more than producers are ahead of the epilogue
+// Stages whose units and events are kept.  The epilogue reads those of a run that begins at stage t after it has given its accumulators
+// back: two more runs of two stages may then be formed and three more stages filled, t + 8 the last of them.
+constexpr int kSlots = 16;
 constexpr int kHeadroom = 6;   // powers of two that a row may grow by after its first stage
 
 template <int N> __device__ __forceinline__ void more_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
