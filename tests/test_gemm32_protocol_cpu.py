@@ -145,3 +145,86 @@ def test_products_with_a_weight(stages, sets, run_length):
         play(rng, [producers(), tensor_core(), epilogue()],
              lambda: [b.phase for g in (full, empty, main_full, main_empty, low_full, low_empty) for b in g])
         assert drained == [(t, s) for t in range(tiles) for s in range(per_tile)]
+
+
+# The product of two activations: one accumulator a run, units of the other CTA's columns that arrive when they please.
+@pytest.mark.parametrize("run_length", [1, 2])
+def test_products_of_two_activations(run_length, stages=2, sets=2):
+    for seed in range(300):
+        rng = random.Random(seed)
+        tiles, per_tile, p_event = rng.randrange(1, 6), rng.randrange(1, 17), rng.choice([0, .1, .5, 1])
+        event = [[i > 0 and rng.random() < p_event for i in range(per_tile)] for _ in range(tiles)]
+        full, empty, acc_full, acc_empty, peer = bars(stages), bars(stages), bars(sets), bars(sets), bars(SLOTS)
+        events, units, theirs, acc, sent = [0] * SLOTS, [None] * SLOTS, [None] * SLOTS, [[] for _ in range(sets)], []
+        total = tiles * per_tile
+
+        def producers():
+            for turn in range(total):
+                t, s = divmod(turn, per_tile)
+                while not empty[turn % stages].done(1 ^ (turn // stages & 1)):
+                    yield
+                units[turn % SLOTS] = (t, s)
+                sent.append(turn)
+                if event[t][s]:
+                    events[turn % SLOTS] = turn + 1
+                yield
+                full[turn % stages].arrive()
+
+        def copies():   # of the other CTA's units
+            for turn in range(total):
+                while not sent:
+                    yield
+                for _ in range(rng.choice([0, 0, 30])):
+                    yield
+                theirs[sent.pop(0) % SLOTS] = divmod(turn, per_tile)
+                peer[turn % SLOTS].arrive()
+
+        def tensor_core():
+            turn = runs = 0
+            for t in range(tiles):
+                run = 0
+                for s in range(per_tile):
+                    while not full[turn % stages].done(turn // stages & 1):
+                        yield
+                    if s > 0 and run > 0 and events[turn % SLOTS] == turn + 1:
+                        acc_full[runs % sets].arrive()
+                        run, runs = 0, runs + 1
+                    at = runs % sets
+                    if run == 0:
+                        while not acc_empty[at].done(1 ^ (runs // sets & 1)):
+                            yield
+                        acc[at] = []
+                    acc[at].append((t, s))
+                    empty[turn % stages].arrive()
+                    run += 1
+                    if run == run_length or s + 1 == per_tile:
+                        acc_full[at].arrive()
+                        run, runs = 0, runs + 1
+                    turn += 1
+                    yield
+
+        def epilogue():
+            turn = run = 0
+            for t in range(tiles):
+                s = 0
+                while s < per_tile:
+                    while not acc_full[run % sets].done(run // sets & 1):
+                        yield
+                    slot, first = turn % SLOTS, s
+                    got = list(acc[run % sets])
+                    acc_empty[run % sets].arrive()
+                    yield
+                    n, run = 0, run + 1
+                    while True:
+                        while not peer[turn % SLOTS].done(turn // SLOTS & 1):
+                            yield
+                        n, s, turn = n + 1, s + 1, turn + 1
+                        if not (n < run_length and s < per_tile and events[turn % SLOTS] != turn + 1):
+                            break
+                    assert got == [(t, first + i) for i in range(n)]
+                for _ in range(rng.choice([1, 1, 60])):
+                    yield
+                assert units[slot] == theirs[slot] == (t, first)   # the sums are scaled at the tile's end
+
+        play(rng, [producers(), copies(), tensor_core(), epilogue()], lambda: [b.phase for g in (full, empty, acc_full, acc_empty, peer) for b in g])
+        assert not sent and [b.phase for b in peer] == [len(range(i, total, SLOTS)) for i in range(SLOTS)]
