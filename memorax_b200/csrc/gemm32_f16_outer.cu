@@ -147,30 +147,28 @@ __global__ void __launch_bounds__(Config<kPair>::kThreads, 1) gemm32_f16_outer_k
         const int set = run % kSets;
         wait(&acc_full[set], (run / kSets) & 1);
         fence_after_sync();
-        if (seg == 0 || event_at(turn)) {
-          const int8_t* const next = units + turn % kSlots * 256;
+        const int8_t* const next = units + turn % kSlots * 256;
+        if (seg > 0 && event_at(turn)) {   // the sums are brought to the new units, none of which is smaller
           if (kPair) wait(&peer_units[turn % kSlots], (turn / kSlots) & 1);
-          if (seg > 0) {   // the sums are brought to the new units, none of which is smaller
+#pragma unroll
+          for (int c = 0; c < kChunks; ++c)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const int at = 128 + col0 + c * 32 + (e >> 1) * 8 + (lane & 3) * 2 + (e & 1);
+              const float r = pow2(max(unit[at] - next[at], -126));
+#pragma unroll
+              for (int i = 0; i < 4; ++i) sum[c][i][e] *= r;
+            }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float r = pow2(max(unit[row0 + 8 * i] - next[row0 + 8 * i], -126));
 #pragma unroll
             for (int c = 0; c < kChunks; ++c)
 #pragma unroll
-              for (int e = 0; e < 8; ++e) {
-                const int at = 128 + col0 + c * 32 + (e >> 1) * 8 + (lane & 3) * 2 + (e & 1);
-                const float r = pow2(max(unit[at] - next[at], -126));
-#pragma unroll
-                for (int i = 0; i < 4; ++i) sum[c][i][e] *= r;
-              }
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const float r = pow2(max(unit[row0 + 8 * i] - next[row0 + 8 * i], -126));
-#pragma unroll
-              for (int c = 0; c < kChunks; ++c)
-#pragma unroll
-                for (int e = 0; e < 8; ++e) sum[c][i][e] *= r;
-            }
+              for (int e = 0; e < 8; ++e) sum[c][i][e] *= r;
           }
         }
-        unit = units + turn % kSlots * 256;
+        unit = next;
         const uint32_t src = tmem + set * 2 * BN + col0 + (static_cast<uint32_t>((warp & 3) * 32) << 16);
 #pragma unroll
         for (int c = 0; c < kChunks; ++c)
@@ -193,6 +191,8 @@ __global__ void __launch_bounds__(Config<kPair>::kThreads, 1) gemm32_f16_outer_k
         }
         int n = 0;   // an event ends a run
         do {
+          // The other CTA's units come by themselves: nothing else says that they are there, and none may be on its way when the kernel ends.
+          if (kPair) wait(&peer_units[turn % kSlots], (turn / kSlots) & 1);
           ++n;
           seg += kBK;
           ++turn;
