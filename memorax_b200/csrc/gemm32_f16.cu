@@ -153,7 +153,8 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
   fence_after_sync();
   const uint32_t tmem = *tmem_slot;
   bool timed_out = false;
-  const auto wait = [&](uint64_t* bar, uint32_t parity) { mbar_wait_flag(bar, parity, timed_out); };
+  // (of a pair, either CTA arrives on the other's barriers, and stores what is read behind them)
+  const auto wait = [&](uint64_t* bar, uint32_t parity) { (kPair ? mbar_wait_cluster_flag : mbar_wait_flag)(bar, parity, timed_out); };
   const auto k_length = [&](const Walk& at) { return min(p.K - at.sp * p.k_split, p.k_split); };
   // Whether a row of the tile begins a new unit at this stage; the same in both CTAs.  (Read after a barrier that the producers'
   // arrivals of the stage lead to; a slot is written again only when its stage has been drained.)
@@ -393,12 +394,12 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
             *reinterpret_cast<uint4*>(dst + L::kPlaneA) = lo;
           }
         }
-        if (event) {   // before the arrivals that let the MMAs of this stage begin
+        if (event)   // before the arrivals that let the MMAs of this stage begin
           for (int r = 0; r < (kPair ? 2 : 1); ++r) store_at(events + slot, r, turn + 1u);
-          asm volatile("fence.acq_rel.cluster;" ::: "memory");
-        }
         fence_smem_to_async();
+        const bool told_event = __any_sync(0xffffffffu, event);
         __syncwarp();
+        if (kPair && told_event) asm volatile("fence.acq_rel.cluster;" ::: "memory");   // (by the lane that arrives; its arrival is a release in the CTA)
         if (lane == 0) {
           if (kPair) arrive_written(&full[stage]);
           else arrive(&full[stage]);

@@ -118,7 +118,8 @@ __global__ void __launch_bounds__(Config<kPair>::kThreads, 1) gemm32_f16_outer_k
   fence_after_sync();
   const uint32_t tmem = *tmem_slot;
   bool timed_out = false;
-  const auto wait = [&](uint64_t* bar, uint32_t parity) { mbar_wait_flag(bar, parity, timed_out); };
+  // (of a pair, either CTA arrives on the other's barriers, and stores what is read behind them)
+  const auto wait = [&](uint64_t* bar, uint32_t parity) { (kPair ? mbar_wait_cluster_flag : mbar_wait_flag)(bar, parity, timed_out); };
   const auto k_length = [&](int tile) {
     const int sp = tile / (mt * nt);
     return min(p.K, (sp + 1) * p.k_split) - sp * p.k_split;
@@ -289,12 +290,12 @@ __global__ void __launch_bounds__(Config<kPair>::kThreads, 1) gemm32_f16_outer_k
         // the next stage's values, on their way under what is left of this one
         if (seg + kBK < k_len) load(tile, seg + kBK);
         else if (tile + tile_step < tiles) load(tile + tile_step, 0);
-        if (event) {   // before the arrivals that let the MMAs of this stage begin
+        if (event)   // before the arrivals that let the MMAs of this stage begin
           for (int r = 0; r < (kPair ? 2 : 1); ++r) store_at(events + slot, r, turn + 1u);
-          asm volatile("fence.acq_rel.cluster;" ::: "memory");
-        }
         fence_smem_to_async();
+        const bool told_event = __any_sync(0xffffffffu, event);
         __syncwarp();
+        if (kPair && told_event) asm volatile("fence.acq_rel.cluster;" ::: "memory");   // (by the lane that arrives; its arrival is a release in the CTA)
         if (kPair && is_b && half == 0 && lane < 2) send16(told + 16 * lane, &peer_units[slot], rank ^ 1, *reinterpret_cast<const volatile uint4*>(told + 16 * lane));
         if (lane == 0) {
           if (kPair && pw == 0) tma::expect_bytes(&peer_units[slot], L::kColsB);

@@ -228,3 +228,11 @@ def test_products_of_two_activations(run_length, stages=2, sets=2):
 
         play(rng, [producers(), copies(), tensor_core(), epilogue()], lambda: [b.phase for g in (full, empty, acc_full, acc_empty, peer) for b in g])
         assert not sent and [b.phase for b in peer] == [len(range(i, total, SLOTS)) for i in range(SLOTS)]
+
+
+# Of a pair, either CTA arrives on the other's barriers: a wait of CTA scope would not order what the other one stored before.
+@pytest.mark.parametrize("kernel", ["gemm32_f16.cu", "gemm32_f16_outer.cu"])
+def test_pairs_wait_at_cluster_scope(kernel):
+    source = open(os.path.join(CSRC, kernel)).read()
+    waits = re.findall(r".*mbar_wait\w*.*", source)
+    assert waits and all("kPair ? mbar_wait_cluster_flag : mbar_wait_flag" in line for line in waits)
