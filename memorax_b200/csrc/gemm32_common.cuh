@@ -1,8 +1,6 @@
 // What the two kernels of float32 products share (gemm32.cu: three bf16 planes, gemm32_f16.cu: two scaled float16 planes).
 #pragma once
 
-#include <cfloat>
-
 #include <cuda_fp16.h>
 
 #include "gemm32.cuh"
@@ -134,11 +132,10 @@ struct Plan {
   int bn, splits, k_split;
 };
 Plan plan(int M, int N, int K);
-// Planes of an image: two for every tile of `bn` rows and stage of kBK, to the end of the last of each.  A word for every row follows
-// (its unit's exponent and its faint elements, see below), and the rows themselves, kBK floats for every stage.
+// Planes of an image: two for every tile of `bn` rows and stage of kBK, to the end of the last of each; the exponents of the
+// rows' units follow.
 __host__ __device__ inline size_t planes_bytes(int bn, int N, int K) { return static_cast<size_t>((N + bn - 1) / bn) * ((K + kBK - 1) / kBK) * (2 * bn * kBK * 2); }
-__host__ __device__ inline size_t words_bytes(int bn, int N) { return static_cast<size_t>((N + bn - 1) / bn) * bn * sizeof(int); }
-inline size_t image_bytes(int bn, int N, int K) { return planes_bytes(bn, N, K) + words_bytes(bn, N) + static_cast<size_t>((N + bn - 1) / bn) * bn * ((K + kBK - 1) / kBK) * kBK * sizeof(float); }
+inline size_t image_bytes(int bn, int N, int K) { return planes_bytes(bn, N, K) + static_cast<size_t>((N + bn - 1) / bn) * bn * sizeof(int); }
 // C = A W^T; `partial` (splits x M x N) takes the parts of a split contraction.
 int launch_weights(const Plan& pl, const float* a, long long lda, const void* image, float* c, long long ldc, int M, int N, int K, const Epilogue& ep,
                    float* partial, int* status, cudaStream_t stream);
@@ -157,66 +154,7 @@ __device__ __forceinline__ float scale_by(float x, int e) {
   return x * pow2(h) * pow2(e - h);
 }
 
-// Faint elements.  In its unit, an element of at least kFaint is held to 2^-23 of itself; a smaller one only to 2^-36, and below that it
-// is gone.  Where what is large in its row meets zeros on the other side (padding that holds a sentinel, a feature without a weight), such
-// elements are all that an output has.  So they are counted: of a row of a weight, and by stages of kBK of a row (column) that is
-// converted in the kernel, where a stage that begins a new unit counts as one, too, since the sum before it is scaled down.  Elements of the
-// other side are below 2^15, so the error of an output, in both units, is below 2^-21 for a faint element and 2^-15 for a stage.  An output of at
-// least kFaintElement and kFaintStage times these numbers loses less than 2^-22 of itself; a smaller one is summed again in float32 from the
-// operands (`dots`).  Ordinary outputs are about 2^26: entries that are normal on both sides have less than one such output a product.
-constexpr float kFaint = 1.f / 8192, kFaintElement = 2.f, kFaintStage = 128.f;
-constexpr int kMostFaint = (1 << 22) - 1;   // elements that a row's word counts
-// A row's word: faint elements << 8 | exponent of its unit + kUnitBias.
-constexpr int kUnitBias = 128, kLeastUnit = -126;
-__device__ __forceinline__ bool is_faint(float x, float scale) { return x != 0.f && fabsf(x) * scale < kFaint; }
-// Running minimum of the magnitudes of float16 pairs, and whether it is so small that the elements have to be looked at (zeros among them).
-__device__ __forceinline__ uint32_t least_of(uint32_t pair, uint32_t least) {
-  const __half2 v = __hmin2(__habs2(*reinterpret_cast<const __half2*>(&pair)), *reinterpret_cast<const __half2*>(&least));
-  return *reinterpret_cast<const uint32_t*>(&v);
-}
-__device__ __forceinline__ uint32_t least_of(uint4 pairs, uint32_t least) { return least_of(pairs.x, least_of(pairs.y, least_of(pairs.z, least_of(pairs.w, least)))); }
-__device__ __forceinline__ bool may_be_faint(uint32_t least) { return (least & 0xffffu) < 0x0800u || (least >> 16) < 0x0800u; }
-constexpr uint32_t kNoneFaint = 0x7bff7bffu;
-// Faint stages as a byte: counted in 1 << shift of them, so that all of a contraction's fit.
-inline int faint_shift(int k_split) {
-  int shift = 0;
-  while ((k_split / kBK + 1) >> shift > 254) ++shift;
-  return shift;
-}
-__device__ __forceinline__ uint8_t faint_byte(int stages, int shift) { return static_cast<uint8_t>(min((stages + (1 << shift) - 1) >> shift, 255)); }
-// Tiles whose counts are kept.  They are written with a tile's last stage and read at its end; a tile has four stages or more, and at most one
-// of a CTA's tiles is a shorter rest of a contraction, so that 13 stages at least lie between two counts in one place (kSlots).
-constexpr int kFaintTiles = 4;
-
-// sum[i][e] = the sum over k of a(k)[i] b(k)[e], in float32, by a warp: a lane has every 32nd k.  (Infinity counts as the largest number,
-// as in the planes.)
-template <typename A, typename B>
-__device__ __forceinline__ void dots(int k_len, int lane, float (&sum)[4][2], A&& a, B&& b) {
-#pragma unroll
-  for (int i = 0; i < 4; ++i) sum[i][0] = sum[i][1] = 0.f;
-#pragma unroll 2
-  for (int k = lane; k < k_len; k += 32) {
-    float x[4], y[2];
-    a(k, x);
-    b(k, y);
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      y[e] = fminf(fmaxf(y[e], -FLT_MAX), FLT_MAX);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) sum[i][e] = fmaf(fminf(fmaxf(x[i], -FLT_MAX), FLT_MAX), y[e], sum[i][e]);
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum[i >> 1][i & 1] += __shfl_xor_sync(0xffffffffu, sum[i >> 1][i & 1], o);
-}
-// Whether a sum is taken again: below `row` + `col`.  `*_small`: the unit is the smallest one, where no bits are lost and all may be zero.
-__device__ __forceinline__ bool too_faint(float sum, float row, float col, bool row_small, bool col_small) {
-  return fabsf(sum) < row + col && (sum != 0.f || !(row_small || col_small));
-}
-
-// Exponent of the unit in which a stretch with this largest magnitude is kept: [kLeastUnit, 113].  (Infinity counts as the largest number.)
+// Exponent of the unit in which a stretch with this largest magnitude is kept: [-126, 113].  (Infinity counts as the largest number.)
 __device__ __forceinline__ int unit_of(float most) {
   const int e = static_cast<int>(__float_as_uint(most) >> 23);
   return min(max(e, 1 + kTargetExp), 254) - 127 - kTargetExp;
@@ -251,7 +189,7 @@ constexpr int kBM = 128;
 // Stages whose units and events are kept.  The epilogue reads those of a run that begins at stage t after it has given its accumulators
 // back: two more runs of two stages may then be formed and three more stages filled, t + 8 the last of them.
 constexpr int kSlots = 16;
-constexpr int kHeadroom = 4;   // powers of two that a row may grow by after its first stage (six leave four bits less to what is faint)
+constexpr int kHeadroom = 6;   // powers of two that a row may grow by after its first stage
 
 template <int N> __device__ __forceinline__ void more_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void fewer_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
@@ -307,7 +245,6 @@ __device__ __forceinline__ void load_box(void* dst, const CUtensorMap* map, uint
 __device__ __forceinline__ void split_rows(const WeightJob& jb, int block) {
   constexpr int kParts = 256 / kSplitRows, kHeld = 2;
   __shared__ float most_of[kParts][kSplitRows];
-  __shared__ int faint_of[kSplitRows];
   const int kb = (jb.K + kBK - 1) / kBK, groups = kb * (kBK / 8);
   const int row_in = threadIdx.x % kSplitRows, part = threadIdx.x / kSplitRows, n = block * kSplitRows + row_in;
   float x[kHeld][8], most = 0.f;
@@ -321,7 +258,6 @@ __device__ __forceinline__ void split_rows(const WeightJob& jb, int block) {
     for (int i = 0; i < kHeld * 8; ++i) most = fmaxf(most, fabsf(x[i >> 3][i & 7]));
   }
   most_of[part][row_in] = most;
-  if (part == 0) faint_of[row_in] = 0;
   __syncthreads();
 #pragma unroll 8
   for (int i = 0; i < kParts; ++i) most = fmaxf(most, most_of[i][row_in]);
@@ -330,9 +266,6 @@ __device__ __forceinline__ void split_rows(const WeightJob& jb, int block) {
   // a tile of 256 or 128 columns is cut into the halves that its two CTAs hold
   const int cut = jb.bn == 64 ? 64 : jb.bn / 2, tile_row = n % cut;
   uint4* const dst = static_cast<uint4*>(jb.image) + static_cast<size_t>(n / cut) * kb * (2 * cut * (kBK / 8)) + (tile_row & ~31) + placed(tile_row & 31);
-  int* const words = reinterpret_cast<int*>(static_cast<uint8_t*>(jb.image) + planes_bytes(jb.bn, jb.N, jb.K));
-  float* const row = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(words) + words_bytes(jb.bn, jb.N)) + static_cast<size_t>(n) * groups * 8;
-  int faint = 0;
   for (int g0 = part; g0 < groups; g0 += kHeld * kParts) {
     if (groups > kHeld * kParts) load(g0);
 #pragma unroll
@@ -344,16 +277,9 @@ __device__ __forceinline__ void split_rows(const WeightJob& jb, int block) {
       uint4* const d = dst + static_cast<size_t>(g / (kBK / 8)) * (2 * cut * (kBK / 8)) + (g % (kBK / 8)) * cut;
       d[0] = hi;
       d[cut * (kBK / 8)] = lo;
-      reinterpret_cast<float4*>(row + g * 8)[0] = make_float4(x[i][0], x[i][1], x[i][2], x[i][3]);
-      reinterpret_cast<float4*>(row + g * 8)[1] = make_float4(x[i][4], x[i][5], x[i][6], x[i][7]);
-      if (may_be_faint(least_of(hi, kNoneFaint)))
-#pragma unroll
-        for (int e = 0; e < 8; ++e) faint += is_faint(x[i][e], scale);
     }
   }
-  if (faint) atomicAdd(&faint_of[row_in], faint);
-  __syncthreads();
-  if (part == 0) words[n] = min(faint_of[row_in], kMostFaint) << 8 | (unit + kUnitBias);
+  if (part == 0) reinterpret_cast<int*>(static_cast<uint8_t*>(jb.image) + planes_bytes(jb.bn, jb.N, jb.K))[n] = unit;
 }
 
 }  // namespace f16

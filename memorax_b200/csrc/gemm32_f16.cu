@@ -8,8 +8,7 @@
 // Scales.  A row of the weight is scaled so that its largest element is in [2^14, 2^15).  A row of A takes the scale of its first
 // kBK elements, with room for elements 2^kHeadroom larger; where one later does not fit, the producers begin a new scale at that
 // stage (`event`), the accumulator of the small products is drained and the row's sum brought to the new unit.  lo is kept 2^11
-// times as large: full precision down to 2^-23 of the largest element.  What is smaller is faint (gemm32_common.cuh): the epilogue sums
-// those outputs again in float32 that faint elements could be a larger part of.
+// times as large: full precision down to 2^-23 of the largest element, and an error of 2^-44 of it below that.
 //
 // Precision: the tensor core truncates when it adds to a float32 accumulator (3e-8 of the sum per addition of 16 k), so the hi*hi
 // accumulator lives for one stage of 64 k, two at a tile's begin (under the stores of the tile before: 129 -> 121 us at 65536 x 1024
@@ -52,9 +51,7 @@ struct Params {
   const float* a;
   long long lda;
   const uint8_t* image;
-  const int* word_w;     // of W's rows, to the end of the last tile: units and faint elements
-  const float* w;        // W's rows
-  long long ldw;
+  const int* unit_w;     // exponents of the units of W's rows, to the end of the last tile
   float* c;
   long long ldc;
   int c_vec;             // floats per aligned access to a row
@@ -63,7 +60,6 @@ struct Params {
   int k_split;           // k per split (a multiple of kBK)
   int splits;            // more than one: c is [splits][M][N]
   int run;               // stages that the hi*hi accumulator lives for after a tile's first run
-  int faint_shift;
   Epilogue ep;           // of a contraction that is not split
   int* status;
 };
@@ -83,8 +79,7 @@ struct Config {
   static constexpr uint32_t kTmem = kSets * 2 * BN;
   static constexpr int kRawAt = kStages * kStage;
   static constexpr int kUnits = kRawAt + kRaws * kRaw;      // int8 [kSlots][128], units of the rows of A
-  static constexpr int kFaints = kUnits + kSlots * 128;     // uint8 [kFaintTiles][128], faint stages of the rows of A
-  static constexpr int kEvents = kFaints + kFaintTiles * 128;   // [kSlots]
+  static constexpr int kEvents = kUnits + kSlots * 128;     // [kSlots]
   static constexpr int kBarriers = kEvents + kSlots * 4;
   static constexpr int kBytes = kBarriers + (3 * kStages + 2 * kRaws + 4 * kSets + 2) * 8;
   static constexpr int kEpilogueWarps = 8, kProducerWarps = 8;
@@ -135,7 +130,6 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
   uint64_t* const raw_empty = raw_full + L::kRaws;
   uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(raw_empty + L::kRaws);
   int8_t* const units = reinterpret_cast<int8_t*>(smem + L::kUnits);
-  uint8_t* const faints = smem + L::kFaints;
   uint32_t* const events = reinterpret_cast<uint32_t*>(smem + L::kEvents);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
@@ -172,13 +166,13 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
     constexpr int kChunks = BN / 64;   // of 32 columns
     const int col0 = (warp >> 2) * (BN / 2), row0 = (warp & 3) * 32 + (lane >> 2);   // this thread: rows row0 + 8 i
     float sum[kChunks][4][8];          // columns 32 c + 8 (lane % 4) + e
-    int turn = 0, main_turn = 0, low_turn = 0, own = 0;   // stages, accumulators, tiles
+    int turn = 0, main_turn = 0, low_turn = 0;   // stages, accumulators
     Walk at(first_tile, tile_step, nt, mt);
-    for (int tile = first_tile; tile < tiles; tile += tile_step, at.next(nt, mt), ++own) {
+    for (int tile = first_tile; tile < tiles; tile += tile_step, at.next(nt, mt)) {
       const int sp = at.sp, n0 = at.n * BN + col0, m0 = at.m * kTileM + rank * kBM + row0, k_len = k_length(at);
       int unit[4] = {};   // of the rows' sums: 2^unit
-      int4 word_w = make_int4(0, 0, 0, 0);   // of four of W's rows a lane, for the end of the tile
-      if (lane < BN / 8) word_w = __ldg(reinterpret_cast<const int4*>(p.word_w + n0) + lane);
+      int4 unit_w = make_int4(0, 0, 0, 0);   // of four of W's rows a lane, for the end of the tile
+      if (lane < BN / 8) unit_w = __ldg(reinterpret_cast<const int4*>(p.unit_w + n0) + lane);
 #pragma unroll
       for (int c = 0; c < kChunks; ++c)
 #pragma unroll
@@ -251,12 +245,11 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
         }
       }
       float* const dst = p.c + (p.splits > 1 ? static_cast<size_t>(sp) * p.M * p.N : 0);
-      // units whose powers are factors that leave room for the sums (a row of zeros has the smallest), nothing faint, and a whole tile
-      const uint8_t* const faint = faints + own % kFaintTiles * 128 + row0;
+      // units whose powers are factors that leave room for the sums (a row of zeros has the smallest), and a whole tile
       bool plain = true;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) plain &= unit[i] <= 60 && faint[8 * i] == 0;
-      plain &= max(max(word_w.x, word_w.y), max(word_w.z, word_w.w)) <= 60 + kUnitBias;
+      for (int i = 0; i < 4; ++i) plain &= unit[i] <= 60;
+      plain &= max(max(unit_w.x, unit_w.y), max(unit_w.z, unit_w.w)) <= 60;
       if (p.vectors && __all_sync(0xffffffffu, plain) && m0 - row0 + kBM <= p.M && n0 + BN / 2 <= p.N) {
         float fr[4];
 #pragma unroll
@@ -270,8 +263,8 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
             float fc[4], bias[4], scale[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-              const int mine = e == 0 ? word_w.x : e == 1 ? word_w.y : e == 2 ? word_w.z : word_w.w;
-              fc[e] = pow2(__shfl_sync(0xffffffffu, mine, c * 8 + (lane & 3) * 2 + h) - kUnitBias);
+              const int mine = e == 0 ? unit_w.x : e == 1 ? unit_w.y : e == 2 ? unit_w.z : unit_w.w;
+              fc[e] = pow2(__shfl_sync(0xffffffffu, mine, c * 8 + (lane & 3) * 2 + h));
               if (kEp) {
                 bias[e] = p.ep.bias ? __ldg(p.ep.bias + n + e) : 0.f;
                 scale[e] = p.ep.add_scale ? __ldg(p.ep.add_scale + n + e) : 1.f;
@@ -297,23 +290,19 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
       } else {
         float copy[kChunks * 32];
         int copy_unit[4];
-        float limit[4];
 #pragma unroll
         for (int i = 0; i < kChunks * 32; ++i) copy[i] = sum[i >> 5][i >> 3 & 3][i & 7];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          copy_unit[i] = unit[i];
-          limit[i] = kFaintStage * static_cast<float>(faint[8 * i] << p.faint_shift);
-        }
+        for (int i = 0; i < 4; ++i) copy_unit[i] = unit[i];
 #pragma unroll 1
         for (int c = 0; c < kChunks; ++c) {   // a vector of eight columns of four rows, all that is read for it on its way at once (one element
           // after element: 2023 x 16 x 256 with 16 columns added held the launch for 4 us more)
           const int n = n0 + c * 32 + (lane & 3) * 8, left = p.N - n;
-          int word_col[8];
+          int unit_col[8];
           float bias[8], scale[8], add[4][8];
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
-            word_col[e] = __ldg(p.word_w + n + e);
+            unit_col[e] = __ldg(p.unit_w + n + e);
             if (kEp) {
               bias[e] = p.ep.bias && e < left ? __ldg(p.ep.bias + n + e) : 0.f;
               scale[e] = p.ep.add_scale && e < left ? __ldg(p.ep.add_scale + n + e) : 1.f;
@@ -321,50 +310,12 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
               for (int i = 0; i < 4; ++i) add[i][e] = p.ep.add && e < left && m0 + 8 * i < p.M ? __ldg(p.ep.add + (m0 + 8 * i) * p.ep.ld_add + n + e) : 0.f;
             }
           }
-          uint32_t again = 0;   // sums that faint elements may have spoilt
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            const float limit_col = kFaintElement * static_cast<float>(word_col[e] >> 8);
-            word_col[e] = (word_col[e] & 255) - kUnitBias;
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-              if (e < left && m0 + 8 * i < p.M &&
-                  too_faint(copy[c * 32 + 8 * i + e], limit[i], limit_col, copy_unit[i] <= kLeastUnit + kHeadroom, word_col[e] == kLeastUnit))
-                again |= 1u << (8 * i + e);
-          }
-#pragma unroll 1
-          for (unsigned lanes = __ballot_sync(0xffffffffu, again != 0); lanes; lanes &= lanes - 1) {
-            const int from = __ffs(lanes) - 1, m = m0 - (lane >> 2) + (from >> 2), k0 = sp * p.k_split;
-            const uint32_t which = __shfl_sync(0xffffffffu, again, from);
-#pragma unroll 1
-            for (int e0 = 0; e0 < 8; e0 += 2) {   // two columns of the four rows
-              const uint32_t bits = which >> e0;
-              if (!(bits & 0x03030303u)) continue;
-              const float* const w = p.w + (n0 + c * 32 + (from & 3) * 8 + e0) * p.ldw + k0;
-              float r[4][2];
-              dots(k_len, lane, r,
-                   [&](int k, float* v) {
-#pragma unroll
-                     for (int i = 0; i < 4; ++i) v[i] = __ldg(p.a + min(m + 8 * i, p.M - 1) * p.lda + k0 + k);
-                   },
-                   [&](int k, float* v) {
-                     v[0] = __ldg(w + k);
-                     v[1] = __ldg(w + p.ldw + k);
-                   });
-              if (lane == from) {
-#pragma unroll
-                for (int i = 0; i < 8; ++i)
-                  if (bits >> (8 * (i >> 1) + (i & 1)) & 1u) copy[c * 32 + 8 * (i >> 1) + e0 + (i & 1)] = r[i >> 1][i & 1];
-              }
-            }
-          }
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             float x[8];
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
-              x[e] = copy[c * 32 + 8 * i + e];
-              if (!(again >> (8 * i + e) & 1u)) x[e] = scale_by(x[e], copy_unit[i] + word_col[e]);
+              x[e] = scale_by(copy[(c * 4 + i) * 8 + e], copy_unit[i] + unit_col[e]);
               if (kEp) x[e] = fmaf(add[i][e], scale[e], x[e] + bias[e]);
             }
             store8(dst + (m0 + 8 * i) * p.ldc + n, m0 + 8 * i < p.M ? left : 0, p.c_vec, x);
@@ -378,13 +329,12 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
     // A warp converts 16 rows, in blocks of 8 rows x 32 k; a lane owns 8 consecutive k of a row, eight consecutive lanes eight rows
     // (no bank conflicts on either side: the float32 tile is swizzled).
     const int pw = warp - kEpilogueWarps, r0 = pw * 16 + (lane & 7);
-    int stage = 0, raw = 0, turn = 0, own = 0;
+    int stage = 0, raw = 0, turn = 0;
     uint32_t parity = 1, raw_parity = 0;   // a fresh barrier's previous phase counts as complete
     int unit[2] = {};             // of this lane's rows
     Walk at(first_tile, tile_step, nt, mt);
-    for (int tile = first_tile; tile < tiles; tile += tile_step, at.next(nt, mt), ++own) {
+    for (int tile = first_tile; tile < tiles; tile += tile_step, at.next(nt, mt)) {
       const int k_len = k_length(at);
-      uint32_t faint = 0;         // stages of the two rows, sixteen bits each
 #pragma unroll 1
       for (int seg = 0; seg < k_len; seg += kBK, ++turn) {
         float x[2][2][8];
@@ -425,17 +375,13 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
         for (int g = 0; g < 2; ++g) {
           const int u = unit_of(most[g]);
           if (seg == 0 || u > unit[g]) {
-            if (seg > 0) {
-              event = true;
-              faint += 1u << (16 * g);
-            }
+            event |= seg > 0;
             unit[g] = u + kHeadroom;
           }
           s[g] = scale_of(unit[g]);
         }
         wait(&empty[stage], parity);
         uint8_t* const base = smem + stage * L::kStage + ((lane >> 3) * kBM + r0) * 16;
-        uint32_t least = kNoneFaint;
 #pragma unroll
         for (int g = 0; g < 2; ++g) {
           if (lane < 8) units[slot * 128 + r0 + g * 8] = static_cast<int8_t>(unit[g]);
@@ -446,21 +392,7 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
             uint8_t* const dst = base + (b * 4 * kBM + g * 8) * 16;
             *reinterpret_cast<uint4*>(dst) = hi;
             *reinterpret_cast<uint4*>(dst + L::kPlaneA) = lo;
-            least = least_of(hi, least);
           }
-        }
-        if (__any_sync(0xffffffffu, may_be_faint(least))) {   // (zeros, mostly)
-#pragma unroll
-          for (int g = 0; g < 2; ++g) {
-            bool any = false;
-#pragma unroll
-            for (int e = 0; e < 16; ++e) any |= is_faint(x[g][e >> 3][e & 7], s[g]);
-            if (__ballot_sync(0xffffffffu, any) >> (lane & 7) & 0x01010101u) faint += 1u << (16 * g);
-          }
-        }
-        if (seg + kBK >= k_len && lane < 8) {
-#pragma unroll
-          for (int g = 0; g < 2; ++g) faints[own % kFaintTiles * 128 + r0 + 8 * g] = faint_byte(faint >> (16 * g) & 0xffffu, p.faint_shift);
         }
         if (event)   // before the arrivals that let the MMAs of this stage begin
           for (int r = 0; r < (kPair ? 2 : 1); ++r) store_at(events + slot, r, turn + 1u);
@@ -640,15 +572,12 @@ int launch_weights(const Plan& pl, const float* a, long long lda, const void* im
   Params p{};
   p.a = a; p.lda = lda;
   p.image = static_cast<const uint8_t*>(image);
-  p.word_w = reinterpret_cast<const int*>(p.image + planes_bytes(pl.bn, N, K));
-  p.w = reinterpret_cast<const float*>(p.image + planes_bytes(pl.bn, N, K) + words_bytes(pl.bn, N));
-  p.ldw = static_cast<long long>((K + kBK - 1) / kBK) * kBK;
+  p.unit_w = reinterpret_cast<const int*>(p.image + planes_bytes(pl.bn, N, K));
   p.c = pl.splits > 1 ? partial : c;
   p.ldc = pl.splits > 1 ? N : ldc;
   p.M = M; p.N = N; p.K = K;
   p.k_split = pl.k_split; p.splits = pl.splits;
   p.run = K < kLongRuns ? 1 : 2;
-  p.faint_shift = faint_shift(pl.k_split);
   if (pl.splits == 1) p.ep = ep;
   p.status = status;
   p.c_vec = vec_of(p.c, p.ldc);

@@ -43,7 +43,6 @@ struct Params {
   int k_split;           // tokens per split (a multiple of kBK)
   int splits;            // more than one: c is [splits][M][N]
   int run;               // stages that the accumulators live for
-  int faint_shift;
   int* status;
 };
 
@@ -58,8 +57,7 @@ struct Config {
   static constexpr uint32_t kTmem = kSets * 2 * kBN;
   static constexpr int kRawAt = kStages * kStage;
   static constexpr int kUnits = kRawAt + kRaws * kRaw;             // int8 [kSlots][128 + 128], units of the columns of A and B
-  static constexpr int kFaints = kUnits + kSlots * 256;            // uint8 [kFaintTiles][2][128 + 128], faint stages of A's and B's columns, of the halves of a stage
-  static constexpr int kMax = kFaints + kFaintTiles * 512;         // float [2][6][2][32], maxima of the halves
+  static constexpr int kMax = kUnits + kSlots * 256;               // float [2][6][2][32], maxima of the halves of a stage
   static constexpr int kEvents = kMax + 2 * 6 * 2 * 32 * 4;        // [kSlots]
   static constexpr int kBarriers = kEvents + kSlots * 4;
   static constexpr int kBytes = kBarriers + (2 * kStages + 2 * kRaws + 2 * kSets + kSlots + 2) * 8;
@@ -99,7 +97,6 @@ __global__ void __launch_bounds__(Config<kPair>::kThreads, 1) gemm32_f16_outer_k
   uint64_t* const raw_empty = raw_full + L::kRaws;
   uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(raw_empty + L::kRaws);
   int8_t* const units = reinterpret_cast<int8_t*>(smem + L::kUnits);
-  uint8_t* const faints = smem + L::kFaints;
   uint32_t* const events = reinterpret_cast<uint32_t*>(smem + L::kEvents);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
@@ -136,8 +133,8 @@ __global__ void __launch_bounds__(Config<kPair>::kThreads, 1) gemm32_f16_outer_k
     constexpr int kChunks = BN / 64;   // of 32 columns
     const int col0 = (warp >> 2) * (BN / 2), row0 = (warp & 3) * 32 + (lane >> 2);   // this thread: rows row0 + 8 i
     float sum[kChunks][4][8];          // [2 j + e]: column 32 c + 8 j + 2 (lane % 4) + e
-    int turn = 0, run = 0, own = 0;
-    for (int tile = first_tile; tile < tiles; tile += tile_step, ++own) {
+    int turn = 0, run = 0;
+    for (int tile = first_tile; tile < tiles; tile += tile_step) {
       const int mn = tile % (mt * nt), sp = tile / (mt * nt);
       const int n0 = (mn % nt) * BN + col0, m0 = (mn / nt) * kTileM + rank * kBM + row0;
       const int k_len = k_length(tile);
@@ -206,92 +203,26 @@ __global__ void __launch_bounds__(Config<kPair>::kThreads, 1) gemm32_f16_outer_k
       int unit_row[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) unit_row[i] = unit[row0 + 8 * i];
-      const auto store2 = [&](int m, int n, float2 v) {
-        if (m >= p.M || n >= p.N) return;
-        float* const out = dst + m * p.ldc + n;
-        if (p.c_vec >= 4 && n + 1 < p.N) {
-          *reinterpret_cast<float2*>(out) = v;
-        } else {
-          out[0] = v.x;
-          if (n + 1 < p.N) out[1] = v.y;
-        }
-      };
-      const uint8_t* const faint = faints + own % kFaintTiles * 512;
-      const auto stages_at = [&](int i) { return static_cast<int>(faint[i]) + faint[256 + i]; };
-      int any = stages_at((warp & 3) * 32 + lane);
 #pragma unroll
-      for (int c = 0; c < kChunks; ++c) any |= stages_at(128 + col0 + c * 32 + lane);
-      if (!__any_sync(0xffffffffu, any != 0)) {
+      for (int c = 0; c < kChunks; ++c)
 #pragma unroll
-        for (int c = 0; c < kChunks; ++c)
+        for (int j = 0; j < 4; ++j) {
+          const int nc = c * 32 + j * 8 + (lane & 3) * 2, n = n0 + nc;
+          const char2 unit_col = *reinterpret_cast<const char2*>(unit + 128 + col0 + nc);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int nc = c * 32 + j * 8 + (lane & 3) * 2;
-            const char2 unit_col = *reinterpret_cast<const char2*>(unit + 128 + col0 + nc);
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-              store2(m0 + 8 * i, n0 + nc, make_float2(scale_by(sum[c][i][2 * j], unit_row[i] + unit_col.x), scale_by(sum[c][i][2 * j + 1], unit_row[i] + unit_col.y)));
-          }
-        continue;
-      }
-      // (a rolled loop over a copy in local memory, as in gemm32_f16.cu)
-      float copy[kChunks * 32];
-#pragma unroll
-      for (int i = 0; i < kChunks * 32; ++i) copy[i] = sum[i >> 5][i >> 3 & 3][i & 7];
-      const float a_stage = kFaintStage * static_cast<float>(1 << p.faint_shift);
-#pragma unroll 1
-      for (int c = 0; c < kChunks; ++c) {
-        const auto column = [](int e, int of) { return (e >> 1) * 8 + (of & 3) * 2 + (e & 1); };   // of lane `of`, in the chunk
-        uint32_t again = 0;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const int nc = c * 32 + column(e, lane), at = 128 + col0 + nc;
-          const float limit_col = a_stage * stages_at(at);
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-            if (m0 + 8 * i < p.M && n0 + nc < p.N &&
-                too_faint(copy[c * 32 + 8 * i + e], a_stage * stages_at(row0 + 8 * i), limit_col, unit_row[i] <= kLeastUnit + kHeadroom, unit[at] <= kLeastUnit + kHeadroom))
-              again |= 1u << (8 * i + e);
-        }
-#pragma unroll 1
-        for (unsigned lanes = __ballot_sync(0xffffffffu, again != 0); lanes; lanes &= lanes - 1) {
-          const int from = __ffs(lanes) - 1, m = m0 - (lane >> 2) + (from >> 2);
-          const long long k0 = static_cast<long long>(sp) * p.k_split;
-          const uint32_t which = __shfl_sync(0xffffffffu, again, from);
-#pragma unroll 1
-          for (int e0 = 0; e0 < 8; e0 += 2) {   // two columns of the four rows
-            const uint32_t bits = which >> e0;
-            if (!(bits & 0x03030303u)) continue;
-            const int n = n0 + c * 32 + column(e0, from);
-            float r[4][2];
-            dots(k_len, lane, r,
-                 [&](int k, float* v) {
-#pragma unroll
-                   for (int i = 0; i < 4; ++i) v[i] = __ldg(p.a + (k0 + k) * p.lda + min(m + 8 * i, p.M - 1));
-                 },
-                 [&](int k, float* v) {
-                   v[0] = __ldg(p.b + (k0 + k) * p.ldb + min(n, p.N - 1));
-                   v[1] = __ldg(p.b + (k0 + k) * p.ldb + min(n + 1, p.N - 1));
-                 });
-            if (lane == from) {
-#pragma unroll
-              for (int i = 0; i < 8; ++i)
-                if (bits >> (8 * (i >> 1) + (i & 1)) & 1u) copy[c * 32 + 8 * (i >> 1) + e0 + (i & 1)] = r[i >> 1][i & 1];
+          for (int i = 0; i < 4; ++i) {
+            const int m = m0 + 8 * i;
+            const float2 v = make_float2(scale_by(sum[c][i][2 * j], unit_row[i] + unit_col.x), scale_by(sum[c][i][2 * j + 1], unit_row[i] + unit_col.y));
+            if (m >= p.M || n >= p.N) continue;
+            float* const out = dst + m * p.ldc + n;
+            if (p.c_vec >= 4 && n + 1 < p.N) {
+              *reinterpret_cast<float2*>(out) = v;
+            } else {
+              out[0] = v.x;
+              if (n + 1 < p.N) out[1] = v.y;
             }
           }
         }
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int nc = c * 32 + column(2 * j, lane);
-            const char2 unit_col = *reinterpret_cast<const char2*>(unit + 128 + col0 + nc);
-            float2 v = make_float2(copy[c * 32 + 8 * i + 2 * j], copy[c * 32 + 8 * i + 2 * j + 1]);
-            if (!(again >> (8 * i + 2 * j) & 1u)) v.x = scale_by(v.x, unit_row[i] + unit_col.x);
-            if (!(again >> (8 * i + 2 * j + 1) & 1u)) v.y = scale_by(v.y, unit_row[i] + unit_col.y);
-            store2(m0 + 8 * i, n0 + nc, v);
-          }
-      }
     }
   } else if (warp < kMmaWarp) {
     // ------------------------------------------------------------ producers
@@ -304,7 +235,7 @@ __global__ void __launch_bounds__(Config<kPair>::kThreads, 1) gemm32_f16_outer_k
     const int col = block * 32 + lane, rows = is_b ? L::kColsB : kBM, plane = is_b ? L::kPlaneB : L::kPlaneA;
     const int unit_at = is_b ? 128 + rank * L::kColsB + block * 32 : block * 32;   // of this warp's first column in a slot's units
     float* const maxima = reinterpret_cast<float*>(smem + L::kMax) + partners * 64;
-    int stage = 0, raw = 0, turn = 0, own = 0;
+    int stage = 0, raw = 0, turn = 0;
     uint32_t parity = 1, raw_parity = 0;
     int unit = 0;   // of this lane's column
     float x[32];
@@ -324,13 +255,10 @@ __global__ void __launch_bounds__(Config<kPair>::kThreads, 1) gemm32_f16_outer_k
       }
     };
     if (first_tile < tiles) load(first_tile, 0);
-    for (int tile = first_tile; tile < tiles; tile += tile_step, ++own) {
+    for (int tile = first_tile; tile < tiles; tile += tile_step) {
       const int k_len = k_length(tile);
-      int faint = 0;   // stages
-      uint8_t* const told_faint = faints + own % kFaintTiles * 512 + half * 256 + unit_at;
 #pragma unroll 1
       for (int seg = 0; seg < k_len; seg += kBK, ++turn) {
-        const bool last = seg + kBK >= k_len;
         float m[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) m[i] = fmaxf(fmaxf(fabsf(x[i]), fabsf(x[i + 8])), fmaxf(fabsf(x[i + 16]), fabsf(x[i + 24])));
@@ -352,25 +280,15 @@ __global__ void __launch_bounds__(Config<kPair>::kThreads, 1) gemm32_f16_outer_k
         int8_t* const told = units + slot * 256 + unit_at;
         if (half == 0) told[lane] = static_cast<int8_t>(unit);
         uint8_t* const dst = smem + stage * L::kStage + (is_b ? 2 * L::kPlaneA : 0) + (half * 4 * rows + col) * 16;
-        uint32_t least = kNoneFaint;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           uint4 hi, lo;
           split8(x + 8 * j, scale, hi, lo);
           *reinterpret_cast<uint4*>(dst + j * rows * 16) = hi;
           *reinterpret_cast<uint4*>(dst + j * rows * 16 + plane) = lo;
-          least = least_of(hi, least);
         }
-        if (may_be_faint(least)) {   // (zeros, mostly)
-          bool any = false;
-#pragma unroll
-          for (int i = 0; i < 32; ++i) any |= is_faint(x[i], scale);
-          faint += any;
-        }
-        faint += event;
-        if (last) told_faint[lane] = faint_byte(faint, p.faint_shift);
         // the next stage's values, on their way under what is left of this one
-        if (!last) load(tile, seg + kBK);
+        if (seg + kBK < k_len) load(tile, seg + kBK);
         else if (tile + tile_step < tiles) load(tile + tile_step, 0);
         if (event)   // before the arrivals that let the MMAs of this stage begin
           for (int r = 0; r < (kPair ? 2 : 1); ++r) store_at(events + slot, r, turn + 1u);
@@ -378,12 +296,9 @@ __global__ void __launch_bounds__(Config<kPair>::kThreads, 1) gemm32_f16_outer_k
         const bool told_event = __any_sync(0xffffffffu, event);
         __syncwarp();
         if (kPair && told_event) asm volatile("fence.acq_rel.cluster;" ::: "memory");   // (by the lane that arrives; its arrival is a release in the CTA)
-        if (kPair && is_b && lane < 2) {
-          if (half == 0) send16(told + 16 * lane, &peer_units[slot], rank ^ 1, *reinterpret_cast<const volatile uint4*>(told + 16 * lane));
-          if (last) send16(told_faint + 16 * lane, &peer_units[slot], rank ^ 1, *reinterpret_cast<const volatile uint4*>(told_faint + 16 * lane));
-        }
+        if (kPair && is_b && half == 0 && lane < 2) send16(told + 16 * lane, &peer_units[slot], rank ^ 1, *reinterpret_cast<const volatile uint4*>(told + 16 * lane));
         if (lane == 0) {
-          if (kPair && pw == 0) tma::expect_bytes(&peer_units[slot], (last ? 3 : 1) * L::kColsB);
+          if (kPair && pw == 0) tma::expect_bytes(&peer_units[slot], L::kColsB);
           if (kPair) arrive_written(&full[stage]);
           else arrive(&full[stage]);
         }
@@ -523,7 +438,6 @@ int launch_outer(const Plan& pl, const float* a, long long lda, const float* b, 
   p.M = M; p.N = N; p.K = K;
   p.k_split = pl.k_split; p.splits = pl.splits;
   p.run = K < kLongRuns ? 1 : 2;
-  p.faint_shift = faint_shift(pl.k_split);
   p.status = status;
   const bool wide = vec_of(a, lda) >= 4 && vec_of(b, ldb) >= 4;
   if (wide) {
