@@ -1,5 +1,5 @@
 // float32 matrix products on the tensor cores (tcgen05): contractions of at most 255 elements, and the host side of all of them.
-// (Longer ones: gemm32_f16.cu, gemm32_f16_outer.cu.)
+// (Longer ones: gemm32_long.cu, gemm32_long_outer.cu.)
 //
 // A float32 number is the exact sum of three bf16 numbers (8 + 8 + 8 mantissa bits: hi + mid + lo), so a product
 // of float32 matrices is a sum of bf16 products accumulated in float32.  The six largest of the nine are kept;
@@ -66,33 +66,6 @@ struct Layout {
   static constexpr int kAccs = BN == 256 ? 1 : 2;
   static constexpr uint32_t kTmem = kAccs * 2 * BN;
 };
-
-// Two floats to bf16, to the nearest; what lies beyond bf16's largest number, the largest floats and infinity, becomes that
-// number (an infinite plane times a zero one would be NaN).
-__device__ __forceinline__ uint32_t pack_finite(float lo, float hi) {
-  uint32_t v;
-  asm("cvt.rn.satfinite.bf16x2.f32 %0, %1, %2;" : "=r"(v) : "f"(hi), "f"(lo));
-  return v;
-}
-
-// hi / mid / lo bf16 planes of eight floats
-__device__ __forceinline__ void split8(const float* x, uint4& hi, uint4& mid, uint4& lo) {
-  uint32_t h[4], m[4], l[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    float a = x[2 * i], b = x[2 * i + 1];
-    h[i] = pack_finite(a, b);
-    a -= __uint_as_float(h[i] << 16);
-    b -= __uint_as_float(h[i] & 0xFFFF0000u);
-    m[i] = pack_finite(a, b);
-    a -= __uint_as_float(m[i] << 16);
-    b -= __uint_as_float(m[i] & 0xFFFF0000u);
-    l[i] = pack_finite(a, b);
-  }
-  hi = make_uint4(h[0], h[1], h[2], h[3]);
-  mid = make_uint4(m[0], m[1], m[2], m[3]);
-  lo = make_uint4(l[0], l[1], l[2], l[3]);
-}
 
 // One operand tile of a stage: `ROWS` contracted over its rows ([kBK][EXT]) or its columns ([EXT][kBK]); split into
 // blocks of 8 rows x 32 columns, one block per warp and turn: a lane owns 8 consecutive columns of a row, eight
@@ -456,12 +429,6 @@ int reduce_splits(const float* partial, int splits, int M, int N, float* c, long
   return launch_status();
 }
 
-// Products with a weight of more than this many k go to gemm32_f16.cu, half the work of the tensor cores: 121 against 184 us at
-// 65536 x 1024 x 256.  Below, three bf16 planes are the more precise form: errors against float64 at K = 64 / 128 / 256 with normal
-// entries 0.7 / 1.2 / 2.3e-7, of two float16 planes 1.35 / 1.4 / 1.8e-7.
-constexpr int kShortK = 255;
-__host__ __device__ constexpr bool two_planes(int K) { return K > kShortK; }
-
 // Width of a tile: 256 columns halve the shared-memory traffic per product, but only where enough tiles are left to give every SM
 // one.  Narrower tiles are the only way to occupy more SMs.
 int tile_columns(int M, int N) {
@@ -515,36 +482,37 @@ __global__ void __launch_bounds__(256) split_weights_kernel(const __grid_constan
     return;
   }
   const WeightJob& jb = sp.job[j];
-  if (two_planes(jb.K)) return f16::split_rows(jb, blockIdx.x - sp.first_block[j]);
-  const int bn = jb.bn, kb = (jb.K + kBK - 1) / kBK;
+  const bool of_long = jb.K > kShortK;
+  const int bn = jb.bn, bk = of_long ? longk::kBK : kBK, kb = (jb.K + bk - 1) / bk, groups = bk / 8;
   const long long id = static_cast<long long>(blockIdx.x - sp.first_block[j]) * 256 + threadIdx.x;
-  // id = ((n_tile * kb + k_block) * 4 + k_group) * bn + n: consecutive threads write consecutive vectors
+  // id = ((n_tile * kb + k_block) * groups + k_group) * bn + n: consecutive threads write (nearly) consecutive vectors
   const int n_in = static_cast<int>(id % bn);
   const long long rest = id / bn;
-  const int kg = static_cast<int>(rest & 3), k_block = static_cast<int>((rest >> 2) % kb);
-  const int n_tile = static_cast<int>((rest >> 2) / kb);
+  const int kg = static_cast<int>(rest % groups), k_block = static_cast<int>(rest / groups % kb);
+  const int n_tile = static_cast<int>(rest / groups / kb);
   if (n_tile * bn >= jb.N) return;
   float x[8];
-  weight_vector(jb, n_tile * bn + n_in, k_block * 4 + kg, x);
+  weight_vector(jb, n_tile * bn + n_in, k_block * groups + kg, x);
   uint4 hi, mid, lo;
   split8(x, hi, mid, lo);
-  // a tile of 256 columns is cut into the halves that its two CTAs hold
-  const int cut = bn == 256 ? 128 : bn, part = n_tile * (bn / cut) + n_in / cut;
-  uint4* const dst = static_cast<uint4*>(jb.image) + (static_cast<size_t>(part) * kb + k_block) * (3 * cut * 4) + kg * cut + n_in % cut;
+  // a tile of a pair of CTAs is cut into the halves that the two hold
+  const int cut = of_long ? longk::rows_of(bn) : bn == 256 ? 128 : bn, part = n_tile * (bn / cut) + n_in / cut, row = n_in % cut;
+  uint4* const dst = static_cast<uint4*>(jb.image) + (static_cast<size_t>(part) * kb + k_block) * (3 * cut * groups) + kg * cut +
+                     (of_long ? (row & ~31) + longk::placed(row & 31) : row);
   dst[0] = hi;
-  dst[cut * 4] = mid;
-  dst[2 * cut * 4] = lo;
+  dst[cut * groups] = mid;
+  dst[2 * cut * groups] = lo;
 }
 
 }  // namespace
 
-int tile_width(int M, int N, int K) { return two_planes(K) ? f16::plan(M, N, K).bn : tile_columns(M, N); }
+int tile_width(int M, int N, int K) { return K > kShortK ? longk::plan(M, N, K).bn : tile_columns(M, N); }
 
 size_t image_bytes(int M, int N, int K) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   const int bn = tile_width(M, N, K);
-  if (two_planes(K)) return f16::image_bytes(bn, N, K);
-  return static_cast<size_t>((N + bn - 1) / bn) * ((K + kBK - 1) / kBK) * (3 * bn * kBK * 2);
+  const int bk = K > kShortK ? longk::kBK : kBK;
+  return static_cast<size_t>((N + bn - 1) / bn) * ((K + bk - 1) / bk) * (3 * bn * bk * 2);
 }
 
 int split_weights(const WeightJob* jobs, int count, const LambdaJob& lambda, cudaStream_t stream) {
@@ -555,8 +523,9 @@ int split_weights(const WeightJob* jobs, int count, const LambdaJob& lambda, cud
     if (!jb.image || jb.w.count < 1) return MXK_ERR_NULL;
     if (!aligned16(jb.image)) return MXK_ERR_ALIGN;
     sp.job[j] = jb;
-    const long long vectors = static_cast<long long>((jb.N + jb.bn - 1) / jb.bn) * jb.bn * ((jb.K + kBK - 1) / kBK) * 4;
-    sp.first_block[j + 1] = sp.first_block[j] + (two_planes(jb.K) ? (jb.N + jb.bn - 1) / jb.bn * (jb.bn / f16::kSplitRows) : static_cast<int>((vectors + 255) / 256));
+    const int bk = jb.K > kShortK ? longk::kBK : kBK;
+    const long long vectors = static_cast<long long>((jb.N + jb.bn - 1) / jb.bn) * jb.bn * ((jb.K + bk - 1) / bk) * (bk / 8);
+    sp.first_block[j + 1] = sp.first_block[j] + static_cast<int>((vectors + 255) / 256);
   }
   for (int j = count; j < 4; ++j) sp.first_block[j + 1] = sp.first_block[count];
   const int blocks = sp.first_block[4] + (lambda.N + 255) / 256;
@@ -570,7 +539,7 @@ int split_weights(const WeightJob* jobs, int count, const LambdaJob& lambda, cud
 size_t workspace_bytes(int M, int N, int K) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   // (of a weight's product or of two activations')
-  const int splits = two_planes(K) ? std::max(f16::plan(M, N, K).splits, f16::plan_outer(M, N, K).splits) : 1;
+  const int splits = K > kShortK ? std::max(longk::plan(M, N, K).splits, longk::plan_outer(M, N, K).splits) : 1;
   return splits > 1 ? static_cast<size_t>(splits) * M * N * sizeof(float) : 0;
 }
 
@@ -579,10 +548,10 @@ int run_weights(const float* a, long long lda, const void* image, float* c, long
   if (!a || !image || !c) return MXK_ERR_NULL;
   if (M <= 0 || N <= 0 || K <= 0) return MXK_ERR_DIMS;
   if (!aligned16(image)) return MXK_ERR_ALIGN;
-  if (two_planes(K)) {
-    const f16::Plan pl = f16::plan(M, N, K);
+  if (K > kShortK) {
+    const longk::Plan pl = longk::plan(M, N, K);
     if (pl.splits > 1 && (!ws || ws_bytes < static_cast<size_t>(pl.splits) * M * N * sizeof(float))) return MXK_ERR_WORKSPACE;
-    const int st = f16::launch_weights(pl, a, lda, image, c, ldc, M, N, K, ep, ws, status, stream);
+    const int st = longk::launch_weights(pl, a, lda, image, c, ldc, M, N, K, ep, ws, status, stream);
     return st != MXK_OK || pl.splits == 1 ? st : reduce_splits(ws, pl.splits, M, N, c, ldc, ep, stream);
   }
   Params p{};
@@ -599,10 +568,10 @@ int run_outer(const float* a, long long lda, const float* b, long long ldb, floa
               float* ws, size_t ws_bytes, int* partials, int* status, cudaStream_t stream) {
   if (!a || !b || !c) return MXK_ERR_NULL;
   if (M <= 0 || N <= 0 || K <= 0) return MXK_ERR_DIMS;
-  if (two_planes(K)) {
-    const f16::Plan pl = f16::plan_outer(M, N, K);
+  if (K > kShortK) {
+    const longk::Plan pl = longk::plan_outer(M, N, K);
     if (pl.splits > 1 && (!ws || ws_bytes < static_cast<size_t>(pl.splits) * M * N * sizeof(float))) return MXK_ERR_WORKSPACE;
-    const int st = f16::launch_outer(pl, a, lda, b, ldb, c, ldc, M, N, K, ws, status, stream);
+    const int st = longk::launch_outer(pl, a, lda, b, ldb, c, ldc, M, N, K, ws, status, stream);
     if (partials) *partials = pl.splits;
     return st != MXK_OK || pl.splits == 1 || partials ? st : reduce_splits(ws, pl.splits, M, N, c, ldc, {}, stream);
   }

@@ -1,4 +1,4 @@
-// float32 matrix products on the tensor cores: host-side interface (gemm32.cu).
+// float32 matrix products on the tensor cores: host-side interface.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -10,6 +10,9 @@ namespace mxk {
 namespace gemm32 {
 
 constexpr int kMaxSegs = 6;
+// Contractions of at most this many elements: gemm32.cu.  Longer ones: gemm32_long.cu, gemm32_long_outer.cu, which are the more precise form
+// and, with a weight, the faster one (142 against 187 us at 65536 x 1024 x 256); three stages of theirs or fewer have not been measured.
+constexpr int kShortK = 255;
 
 // A row-major weight matrix.  kStacked: rows of up to kMaxSegs arrays on top of each other (the Dense layers that read
 // the same input), array s holding rows [row_end[s-1], row_end[s]).  The two others are the complex-diagonal cells'
@@ -44,7 +47,7 @@ struct Epilogue {
 };
 
 // Weights in the form the kernel multiplies with: W [N][K] (or its transpose stored [K][N], `transposed`) as hi / mid /
-// lo bf16 planes cut into the tiles of the product C[M][N] = A[M][K] W^T, `image_bytes` long.
+// lo bf16 planes cut into the tiles and stages of the product C[M][N] = A[M][K] W^T, `image_bytes` long.
 struct WeightJob {
   Weight w;
   bool transposed = false;

@@ -1,7 +1,5 @@
-// What the two kernels of float32 products share (gemm32.cu: three bf16 planes, gemm32_f16.cu: two scaled float16 planes).
+// What the kernels of float32 products share (gemm32.cu, gemm32_long.cu, gemm32_long_outer.cu).
 #pragma once
-
-#include <cuda_fp16.h>
 
 #include "gemm32.cuh"
 #include "mxk_common.cuh"
@@ -50,6 +48,33 @@ inline int vec_of(const void* p, long long ld) {
   if (a % 32 == 0 && ld % 8 == 0) return 8;
   if (a % 16 == 0 && ld % 4 == 0) return 4;
   return 1;
+}
+
+// Two floats to bf16, to the nearest; what lies beyond bf16's largest number, the largest floats and infinity, becomes that
+// number (an infinite plane times a zero one would be NaN).
+__device__ __forceinline__ uint32_t pack_finite(float lo, float hi) {
+  uint32_t v;
+  asm("cvt.rn.satfinite.bf16x2.f32 %0, %1, %2;" : "=r"(v) : "f"(hi), "f"(lo));
+  return v;
+}
+
+// hi / mid / lo bf16 planes of eight floats
+__device__ __forceinline__ void split8(const float* x, uint4& hi, uint4& mid, uint4& lo) {
+  uint32_t h[4], m[4], l[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float a = x[2 * i], b = x[2 * i + 1];
+    h[i] = pack_finite(a, b);
+    a -= __uint_as_float(h[i] << 16);
+    b -= __uint_as_float(h[i] & 0xFFFF0000u);
+    m[i] = pack_finite(a, b);
+    a -= __uint_as_float(m[i] << 16);
+    b -= __uint_as_float(m[i] & 0xFFFF0000u);
+    l[i] = pack_finite(a, b);
+  }
+  hi = make_uint4(h[0], h[1], h[2], h[3]);
+  mid = make_uint4(m[0], m[1], m[2], m[3]);
+  lo = make_uint4(l[0], l[1], l[2], l[3]);
 }
 
 // Eight elements along k from k = 8 g on of W's row n, zero past the matrix.  (What kind of weight it is, is asked once, so that
@@ -122,75 +147,30 @@ __device__ __forceinline__ void weight_vector(const WeightJob& jb, int n, int g,
   }
 }
 
-// ---- two float16 planes (gemm32_f16.cu) ----
-namespace f16 {
+// ---- contractions of more than kShortK (gemm32_long.cu) ----
+namespace longk {
 
-constexpr int kSplitRows = 4;   // rows of a weight that a block of split_rows splits, with 64 threads each
 constexpr int kBK = 64;
 
 struct Plan {
   int bn, splits, k_split;
 };
 Plan plan(int M, int N, int K);
-// Planes of an image: two for every tile of `bn` rows and stage of kBK, to the end of the last of each; the exponents of the
-// rows' units follow.
-__host__ __device__ inline size_t planes_bytes(int bn, int N, int K) { return static_cast<size_t>((N + bn - 1) / bn) * ((K + kBK - 1) / kBK) * (2 * bn * kBK * 2); }
-inline size_t image_bytes(int bn, int N, int K) { return planes_bytes(bn, N, K) + static_cast<size_t>((N + bn - 1) / bn) * bn * sizeof(int); }
+// Rows of a weight that one CTA of a tile's holds.
+__host__ __device__ constexpr int rows_of(int bn) { return bn == 64 ? 64 : bn / 2; }
 // C = A W^T; `partial` (splits x M x N) takes the parts of a split contraction.
 int launch_weights(const Plan& pl, const float* a, long long lda, const void* image, float* c, long long ldc, int M, int N, int K, const Epilogue& ep,
                    float* partial, int* status, cudaStream_t stream);
-// C = A^T B, both stored [K][..] (gemm32_f16_outer.cu).
+// C = A^T B, both stored [K][..] (gemm32_long_outer.cu).
 Plan plan_outer(int M, int N, int K);
 int launch_outer(const Plan& pl, const float* a, long long lda, const float* b, long long ldb, float* c, long long ldc, int M, int N, int K, float* partial,
                  int* status, cudaStream_t stream);
-
-constexpr float kLo = 2048.f;     // lo planes are this much larger than what they stand for
-constexpr int kTargetExp = 14;    // the largest element of a row is scaled to [2^14, 2^15)
-
-__device__ __forceinline__ float pow2(int e) { return __uint_as_float(static_cast<uint32_t>(e + 127) << 23); }   // e in [-126, 127]
-// x 2^e for |e| <= 252, rounded once where the result is a normal number
-__device__ __forceinline__ float scale_by(float x, int e) {
-  const int h = e >> 1;
-  return x * pow2(h) * pow2(e - h);
-}
-
-// Exponent of the unit in which a stretch with this largest magnitude is kept: [-126, 113].  (Infinity counts as the largest number.)
-__device__ __forceinline__ int unit_of(float most) {
-  const int e = static_cast<int>(__float_as_uint(most) >> 23);
-  return min(max(e, 1 + kTargetExp), 254) - 127 - kTargetExp;
-}
-__device__ __forceinline__ float scale_of(int unit) { return pow2(-unit); }
-// Two floats to float16, to the nearest; what does not fit, infinity alone, becomes the largest number (an infinite plane times a
-// zero one would be NaN).
-__device__ __forceinline__ uint32_t pack_half(float lo, float hi) {
-  uint32_t v;
-  asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(v) : "f"(hi), "f"(lo));
-  return v;
-}
-
-// hi and lo planes of two scaled floats
-__device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo) {
-  hi = pack_half(a, b);
-  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hi));
-  lo = pack_half((a - f.x) * kLo, (b - f.y) * kLo);
-}
-__device__ __forceinline__ void split8(const float* x, float s, uint4& hi, uint4& lo) {
-  split2(x[0] * s, x[1] * s, hi.x, lo.x);
-  split2(x[2] * s, x[3] * s, hi.y, lo.y);
-  split2(x[4] * s, x[5] * s, hi.z, lo.z);
-  split2(x[6] * s, x[7] * s, hi.w, lo.w);
-}
 
 // Column of a 32-column block in which W's row `n` of the block is placed, so that the eight values that a thread reads from a
 // lane with tmem_ld_16x32 are consecutive columns of C and its stores fill whole lines.
 __device__ __forceinline__ int placed(int n) { return 8 * ((n >> 1) & 3) + 2 * (n >> 3) + (n & 1); }
 
 constexpr int kBM = 128;
-// Stages whose units and events are kept.  The epilogue reads those of a run that begins at stage t after it has given its accumulators
-// back: two more runs of two stages may then be formed and three more stages filled, t + 8 the last of them.
-constexpr int kSlots = 16;
-constexpr int kHeadroom = 6;   // powers of two that a row may grow by after its first stage
-
 template <int N> __device__ __forceinline__ void more_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void fewer_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
@@ -209,11 +189,6 @@ __device__ __forceinline__ void arrive_written(uint64_t* bar) {
       "mbarrier.arrive.shared::cluster.b64 _, [ra];\n\t}\n" ::"r"(umma::smem_u32(bar))
       : "memory");
 }
-// Stores to CTA `rank` of the cluster.
-__device__ __forceinline__ void store_at(uint32_t* p, int rank, uint32_t v) {
-  asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, %1;\n\tst.shared::cluster.u32 [ra], %2;\n\t}\n" ::"r"(umma::smem_u32(p)), "r"(rank), "r"(v) : "memory");
-}
-
 // 16 TMEM lanes x 32 columns: r[4 j + 2 h + e] is lane (lane / 4) + 8 h, column 8 j + 2 (lane % 4) + e.
 __device__ __forceinline__ void tmem_ld_16x32(uint32_t taddr, uint32_t* r) {
   asm volatile(
@@ -240,48 +215,6 @@ __device__ __forceinline__ void load_box(void* dst, const CUtensorMap* map, uint
       : "memory");
 }
 
-// A block splits four rows of a weight: 64 threads a row look for its largest element, then each writes the planes of every 64th
-// vector of eight k.  Bound: the latency of its loads, all of them under way together up to 1024 k (1024 x 256: 4.6 us).
-__device__ __forceinline__ void split_rows(const WeightJob& jb, int block) {
-  constexpr int kParts = 256 / kSplitRows, kHeld = 2;
-  __shared__ float most_of[kParts][kSplitRows];
-  const int kb = (jb.K + kBK - 1) / kBK, groups = kb * (kBK / 8);
-  const int row_in = threadIdx.x % kSplitRows, part = threadIdx.x / kSplitRows, n = block * kSplitRows + row_in;
-  float x[kHeld][8], most = 0.f;
-  const auto load = [&](int g0) {
-#pragma unroll
-    for (int i = 0; i < kHeld; ++i) weight_vector(jb, n, g0 + i * kParts, x[i]);   // (zero past the matrix)
-  };
-  for (int g0 = part; g0 < groups; g0 += kHeld * kParts) {
-    load(g0);
-#pragma unroll
-    for (int i = 0; i < kHeld * 8; ++i) most = fmaxf(most, fabsf(x[i >> 3][i & 7]));
-  }
-  most_of[part][row_in] = most;
-  __syncthreads();
-#pragma unroll 8
-  for (int i = 0; i < kParts; ++i) most = fmaxf(most, most_of[i][row_in]);
-  const int unit = unit_of(most);
-  const float scale = scale_of(unit);
-  // a tile of 256 or 128 columns is cut into the halves that its two CTAs hold
-  const int cut = jb.bn == 64 ? 64 : jb.bn / 2, tile_row = n % cut;
-  uint4* const dst = static_cast<uint4*>(jb.image) + static_cast<size_t>(n / cut) * kb * (2 * cut * (kBK / 8)) + (tile_row & ~31) + placed(tile_row & 31);
-  for (int g0 = part; g0 < groups; g0 += kHeld * kParts) {
-    if (groups > kHeld * kParts) load(g0);
-#pragma unroll
-    for (int i = 0; i < kHeld; ++i) {
-      const int g = g0 + i * kParts;
-      if (g >= groups) break;
-      uint4 hi, lo;
-      split8(x[i], scale, hi, lo);
-      uint4* const d = dst + static_cast<size_t>(g / (kBK / 8)) * (2 * cut * (kBK / 8)) + (g % (kBK / 8)) * cut;
-      d[0] = hi;
-      d[cut * (kBK / 8)] = lo;
-    }
-  }
-  if (part == 0) reinterpret_cast<int*>(static_cast<uint8_t*>(jb.image) + planes_bytes(jb.bn, jb.N, jb.K))[n] = unit;
-}
-
-}  // namespace f16
+}  // namespace longk
 }  // namespace gemm32
 }  // namespace mxk

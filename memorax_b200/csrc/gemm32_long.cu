@@ -1,36 +1,27 @@
-// float32 products with a weight on the tensor cores (tcgen05), contractions of 256 elements and more.
+// float32 products with a weight on the tensor cores (tcgen05), contractions of more than kShortK elements.
 //
-// A float32 number, scaled by a power of two, is the sum of two float16 numbers (hi + lo, 11 + 11 mantissa bits and lo's sign) to
-// within 2^-23 of itself, so a product of float32 matrices is three float16 products, hi*hi + hi*lo + lo*hi, accumulated in
-// float32; lo*lo is below 2^-22 of |a||b|, and mostly below 2^-24.  (The sum of three bf16 numbers, which needs no scales, takes
-// six: gemm32.cu.)
-//
-// Scales.  A row of the weight is scaled so that its largest element is in [2^14, 2^15).  A row of A takes the scale of its first
-// kBK elements, with room for elements 2^kHeadroom larger; where one later does not fit, the producers begin a new scale at that
-// stage (`event`), the accumulator of the small products is drained and the row's sum brought to the new unit.  lo is kept 2^11
-// times as large: full precision down to 2^-23 of the largest element, and an error of 2^-44 of it below that.
+// A float32 number is the exact sum of three bf16 numbers, and the six largest of the nine products are formed, as in gemm32.cu.  (Two
+// scaled float16 numbers take three products, 124 and 106 us at the sizes below, but an element 2^25 below the largest of its row is then
+// lost, and with it an output where the large one meets a zero: padding that holds a sentinel, a feature without a weight.)
 //
 // Precision: the tensor core truncates when it adds to a float32 accumulator (3e-8 of the sum per addition of 16 k), so the hi*hi
-// accumulator lives for one stage of 64 k, two at a tile's begin (under the stores of the tile before: 129 -> 121 us at 65536 x 1024
-// x 256) and in contractions from 384 on, and is summed up in float32 registers; the two small products have an accumulator of their
-// own, whose truncations are 2^-11 as large, for the whole tile.  Errors against float64, relative 2-norm (three bf16 planes, drained
-// every 512 k, in brackets; below 256 k they are the more precise form):
-//   4096 x 1024 x 256     normal entries 1.8e-7 (2.3e-7)   lognormal, sigma 3: 1.5e-7 (3.3e-7)
-//   4096 x 256 x 512                     2.1e-7 (4.7e-7)                       1.2e-7 (6.1e-7)
-//   4096 x 256 x 1024                    2.1e-7 (4.7e-7)                       1.4e-7 (4.5e-7)
+// accumulator lives for one stage of 64 k, two at a tile's begin (under the stores of the tile before) and in contractions from 384 on, and is
+// summed up in float32 registers; the five small products have an accumulator of their own, whose truncations are 2^-8 as large, for at
+// most kLowRun stages.  Errors against float64, relative 2-norm (drained every 512 k, in brackets):
+//   65536 x 1024 x 256    normal entries 1.05e-7 (2.3e-7)
+//   65536 x 256 x 1024                   1.34e-7 (4.7e-7)    lognormal, sigma 3: 1.3e-7 (4.3e-7)
+//   24000 x 1024 x 512                   1.27e-7 (4.7e-7)                        1.2e-7 (3.7e-7)
 //
-// Bound: the tensor pipe at three float16 products per float32 product (1.66 PFLOP/s / 3 = 554 TFLOP/s; 463 with the waves of
-// 65536 x 256 x 1024 and all but the products left out), and C's way to memory.  Beside it shared memory: a stage of 256 columns
-// is 96 KB read by the pipe in 1536 cycles, 64 KB of tiles and 32 KB of planes written and 32 KB of float32 read.
+// Bound: the tensor pipe at six products (24 MMAs, 3072 cycles a stage of 256 columns) and, beside it, shared memory: 192 KB read by the
+// pipe, 80 KB of tiles and 48 KB of planes written and 32 KB of float32 read, 2750 cycles at 128 bytes.
+// Measured with the splitting of the weight (the form of gemm32.cu, whose producers read global memory): 65536 x 1024 x 256 142 us (187),
+// 65536 x 256 x 1024 145 us (183), 24000 x 1024 x 512 118 us (133), 65536 x 128 x 256 37.5 us (50), 8192 x 520 x 512 52 us (52).
 //
 // One persistent CTA per SM, warp-specialised:
 //   8 warps    epilogue: accumulators (TMEM) -> sums in registers -> global, whole lines
-//   8 warps    producers: float32 tiles, two or three stages ahead in shared memory -> scaled float16 planes
-//   1 warp     issues the MMAs (12 per stage of 64 k), 1 warp the copies of the weight's image, 1 warp those of A (TMA)
-// Registers are dealt out by setmaxnreg: a thread of the epilogue holds up to 128 sums.  (A loaded straight from global memory
-// into the producers' registers: 142 us at 65536 x 256 x 1024, its loads then wait for room in an L1 of 28 KB.)
-// Measured, without the splitting of the weight (three bf16 planes before): 65536 x 1024 x 256 121 us (184), 65536 x 256 x 1024
-// 103 us (173), 24000 x 1024 x 512 89 us (126), 65536 x 128 x 256 28 us (40).
+//   8 warps    producers: float32 tiles, one or two stages ahead in shared memory -> bf16 planes
+//   1 warp     issues the MMAs (24 per stage of 64 k), 1 warp the copies of the weight's image, 1 warp those of A (TMA)
+// Registers are dealt out by setmaxnreg: a thread of the epilogue holds up to 128 sums.
 #include <algorithm>
 
 #include "gemm32_common.cuh"
@@ -38,20 +29,20 @@
 
 namespace mxk {
 namespace gemm32 {
-namespace f16 {
+namespace longk {
 namespace {
 
 using namespace umma;
 
 constexpr int kLongRuns = 384; // from here on the hi*hi accumulator lives for two stages
 constexpr int kFirstRun = 2;   // and always a tile's first: the epilogue is still at the tile before
+constexpr int kLowRun = 8;     // stages that the accumulator of the small products lives for
 
 struct Params {
   CUtensorMap map_a;     // kWide: boxes of 128 rows x 32 k
   const float* a;
   long long lda;
   const uint8_t* image;
-  const int* unit_w;     // exponents of the units of W's rows, to the end of the last tile
   float* c;
   long long ldc;
   int c_vec;             // floats per aligned access to a row
@@ -60,6 +51,7 @@ struct Params {
   int k_split;           // k per split (a multiple of kBK)
   int splits;            // more than one: c is [splits][M][N]
   int run;               // stages that the hi*hi accumulator lives for after a tile's first run
+  int zero;              // 0
   Epilogue ep;           // of a contraction that is not split
   int* status;
 };
@@ -69,18 +61,15 @@ template <int BN>
 struct Config {
   static constexpr bool kPair = BN != 64;
   static constexpr int kTileM = kPair ? 2 * kBM : kBM;
-  static constexpr int kRowsB = kPair ? BN / 2 : BN;   // rows of W in this CTA
+  static constexpr int kRowsB = rows_of(BN);   // rows of W in this CTA
   static constexpr int kPlaneA = kBM * kBK * 2, kPlaneB = kRowsB * kBK * 2;   // bytes
-  static constexpr int kStage = 2 * (kPlaneA + kPlaneB);
-  static constexpr int kStages = kRowsB == 128 ? 2 : 3;
-  static constexpr int kRaw = kBM * kBK * 4, kRaws = kRowsB == 128 ? 3 : 2;   // float32 tiles of A: two halves of 32 k, rows of 128 bytes
+  static constexpr int kStage = 3 * (kPlaneA + kPlaneB), kStages = 2;
+  static constexpr int kRaw = kBM * kBK * 4, kRaws = kRowsB == 128 ? 1 : 2;   // float32 tiles of A: two halves of 32 k, rows of 128 bytes
   // accumulators: BN columns for hi*hi and BN for the small products, twice where TMEM has room
   static constexpr int kSets = BN == 256 ? 1 : 2;
   static constexpr uint32_t kTmem = kSets * 2 * BN;
   static constexpr int kRawAt = kStages * kStage;
-  static constexpr int kUnits = kRawAt + kRaws * kRaw;      // int8 [kSlots][128], units of the rows of A
-  static constexpr int kEvents = kUnits + kSlots * 128;     // [kSlots]
-  static constexpr int kBarriers = kEvents + kSlots * 4;
+  static constexpr int kBarriers = kRawAt + kRaws * kRaw;
   static constexpr int kBytes = kBarriers + (3 * kStages + 2 * kRaws + 4 * kSets + 2) * 8;
   static constexpr int kEpilogueWarps = 8, kProducerWarps = 8;
   static constexpr int kMmaWarp = kEpilogueWarps + kProducerWarps, kImageWarp = kMmaWarp + 1, kRawWarp = kMmaWarp + 2;
@@ -108,7 +97,7 @@ struct Walk {
 // (The instruction cache is small beside this much unrolled code: what is rare is a rolled loop over a copy of the sums in
 // local memory, or another instantiation.)
 template <int BN, bool kWide, bool kEp>
-__global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(const __grid_constant__ Params p) {
+__global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_long_kernel(const __grid_constant__ Params p) {
   using L = Config<BN>;
   constexpr bool kPair = L::kPair;
   constexpr int kStages = L::kStages, kSets = L::kSets, kTileM = L::kTileM, kRowsB = L::kRowsB;
@@ -129,8 +118,6 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
   uint64_t* const raw_full = low_empty + kSets;    // copies -> producers, a float32 tile
   uint64_t* const raw_empty = raw_full + L::kRaws;
   uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(raw_empty + L::kRaws);
-  int8_t* const units = reinterpret_cast<int8_t*>(smem + L::kUnits);
-  uint32_t* const events = reinterpret_cast<uint32_t*>(smem + L::kEvents);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (tid == 0) {
@@ -142,7 +129,6 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
     for (int s = 0; s < L::kRaws; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], kProducerWarps); }
     mbar_init_fence();
   }
-  if (tid < kSlots) events[tid] = 0;
   if (warp == kMmaWarp) {
     if (kPair) tmem_alloc_pair(tmem_slot, L::kTmem);
     else tmem_alloc(tmem_slot, L::kTmem);
@@ -153,42 +139,28 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
   fence_after_sync();
   const uint32_t tmem = *tmem_slot;
   bool timed_out = false;
-  // (of a pair, either CTA arrives on the other's barriers, and stores what is read behind them)
+  // (of a pair, either CTA arrives on the other's barriers)
   const auto wait = [&](uint64_t* bar, uint32_t parity) { (kPair ? mbar_wait_cluster_flag : mbar_wait_flag)(bar, parity, timed_out); };
   const auto k_length = [&](const Walk& at) { return min(p.K - at.sp * p.k_split, p.k_split); };
-  // Whether a row of the tile begins a new unit at this stage; the same in both CTAs.  (Read after a barrier that the producers'
-  // arrivals of the stage lead to; a slot is written again only when its stage has been drained.)
-  const auto event_at = [&](int turn) { return *const_cast<volatile uint32_t*>(events + turn % kSlots) == turn + 1u; };
-
   if (warp < kEpilogueWarps) {
     // ------------------------------------------------------------ epilogue
     more_registers<L::kRegsEpilogue>();
     constexpr int kChunks = BN / 64;   // of 32 columns
     const int col0 = (warp >> 2) * (BN / 2), row0 = (warp & 3) * 32 + (lane >> 2);   // this thread: rows row0 + 8 i
     float sum[kChunks][4][8];          // columns 32 c + 8 (lane % 4) + e
-    int turn = 0, main_turn = 0, low_turn = 0;   // stages, accumulators
+    int main_turn = 0, low_turn = 0;   // accumulators
     Walk at(first_tile, tile_step, nt, mt);
     for (int tile = first_tile; tile < tiles; tile += tile_step, at.next(nt, mt)) {
-      const int sp = at.sp, n0 = at.n * BN + col0, m0 = at.m * kTileM + rank * kBM + row0, k_len = k_length(at);
-      int unit[4] = {};   // of the rows' sums: 2^unit
-      int4 unit_w = make_int4(0, 0, 0, 0);   // of four of W's rows a lane, for the end of the tile
-      if (lane < BN / 8) unit_w = __ldg(reinterpret_cast<const int4*>(p.unit_w + n0) + lane);
+      const int sp = at.sp, n0 = at.n * BN + col0, m0 = at.m * kTileM + rank * kBM + row0, stages = (k_length(at) + kBK - 1) / kBK;
 #pragma unroll
       for (int c = 0; c < kChunks; ++c)
 #pragma unroll
         for (int i = 0; i < 32; ++i) sum[c][i >> 3][i & 7] = 0.f;
-      bool drained = false;   // the small products that an event ended
+      bool low = false;
 #pragma unroll 1
-      for (int seg = 0;;) {   // one accumulator a turn: hi*hi of a run of stages, the small products before an event and at the end
-        const int slot = turn % kSlots;
-        bool low = seg >= k_len;
-        if (!low) {
-          wait(&main_full[main_turn % kSets], (main_turn / kSets) & 1);
-          low = seg > 0 && !drained && event_at(turn);
-        }
-        const int set = (low ? low_turn : main_turn) % kSets;
-        const float f = low ? 1.f / kLo : 1.f;
-        if (low) wait(&low_full[set], (low_turn / kSets) & 1);
+      for (int stage = 0;;) {   // one accumulator a turn: hi*hi of a run of stages, the small products of kLowRun of them
+        const int turn = low ? low_turn : main_turn, set = turn % kSets;
+        wait((low ? low_full : main_full) + set, (turn / kSets) & 1);
         fence_after_sync();
         const uint32_t src = tmem + set * 2 * BN + (low ? BN : 0) + col0 + (static_cast<uint32_t>((warp & 3) * 32) << 16);
 #pragma unroll
@@ -201,87 +173,47 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
 #pragma unroll
             for (int j = 0; j < 4; ++j)
 #pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                float& x = sum[c][2 * h + (i >> 1)][2 * j + (i & 1)];
-                x = fmaf(__uint_as_float(r[4 * j + i]), f, x);
-              }
+              for (int i = 0; i < 4; ++i) sum[c][2 * h + (i >> 1)][2 * j + (i & 1)] += __uint_as_float(r[4 * j + i]);
           }
         fence_before_sync();
         __syncwarp();
         if (lane == 0) {
-          uint64_t* const bar = low ? &low_empty[set] : &main_empty[set];
+          uint64_t* const bar = (low ? low_empty : main_empty) + set;
           if (kPair) arrive_read(bar);
           else arrive(bar);
         }
-        if (!low) {
-          if (seg == 0) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) unit[i] = units[slot * 128 + row0 + 8 * i];
-          }
+        if (low) {
+          ++low_turn;
+          low = false;
+          if (stage == stages) break;
+        } else {
           ++main_turn;
-          drained = false;
-          // the run's stages: one where an event began it, fewer than p.run where one ended it
-          const int most = seg == 0 ? kFirstRun : event_at(turn) ? 1 : p.run;
-          int n = 0;
-          do {
-            ++n;
-            seg += kBK;
-            ++turn;
-          } while (n < most && seg < k_len && !event_at(turn));
-          continue;
-        }
-        ++low_turn;
-        if (seg >= k_len) break;
-        drained = true;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int u = units[slot * 128 + row0 + 8 * i];   // no smaller than before
-          const float r = pow2(max(unit[i] - u, -126));
-          unit[i] = u;
-#pragma unroll
-          for (int c = 0; c < kChunks; ++c)
-#pragma unroll
-            for (int e = 0; e < 8; ++e) sum[c][i][e] *= r;
+          stage = min(stage + (stage == 0 ? kFirstRun : p.run), stages);
+          low = stage % kLowRun == 0 || stage == stages;
         }
       }
       float* const dst = p.c + (p.splits > 1 ? static_cast<size_t>(sp) * p.M * p.N : 0);
-      // units whose powers are factors that leave room for the sums (a row of zeros has the smallest), and a whole tile
-      bool plain = true;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) plain &= unit[i] <= 60;
-      plain &= max(max(unit_w.x, unit_w.y), max(unit_w.z, unit_w.w)) <= 60;
-      if (p.vectors && __all_sync(0xffffffffu, plain) && m0 - row0 + kBM <= p.M && n0 + BN / 2 <= p.N) {
-        float fr[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) fr[i] = pow2(unit[i]);
+      if (p.vectors && m0 - row0 + kBM <= p.M && n0 + BN / 2 <= p.N) {   // a whole tile
         float* out = dst + m0 * p.ldc + n0 + (lane & 3) * 8;
 #pragma unroll
         for (int c = 0; c < kChunks; ++c, out += 32) {
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {   // four columns
+          for (int h = 0; h < 2 && kEp; ++h) {   // four columns
             const int n = n0 + c * 32 + (lane & 3) * 8 + 4 * h;
-            float fc[4], bias[4], scale[4];
+            float bias[4], scale[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-              const int mine = e == 0 ? unit_w.x : e == 1 ? unit_w.y : e == 2 ? unit_w.z : unit_w.w;
-              fc[e] = pow2(__shfl_sync(0xffffffffu, mine, c * 8 + (lane & 3) * 2 + h));
-              if (kEp) {
-                bias[e] = p.ep.bias ? __ldg(p.ep.bias + n + e) : 0.f;
-                scale[e] = p.ep.add_scale ? __ldg(p.ep.add_scale + n + e) : 1.f;
-              }
+              bias[e] = p.ep.bias ? __ldg(p.ep.bias + n + e) : 0.f;
+              scale[e] = p.ep.add_scale ? __ldg(p.ep.add_scale + n + e) : 1.f;
             }
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
               float* const x = sum[c][i] + 4 * h;
-#pragma unroll
-              for (int e = 0; e < 4; ++e) x[e] = x[e] * fr[i] * fc[e];
-              if (kEp) {
-                const float4 ad = p.ep.add ? __ldg(reinterpret_cast<const float4*>(p.ep.add + (m0 + 8 * i) * p.ep.ld_add + n)) : make_float4(0.f, 0.f, 0.f, 0.f);
-                x[0] = fmaf(ad.x, scale[0], x[0] + bias[0]);
-                x[1] = fmaf(ad.y, scale[1], x[1] + bias[1]);
-                x[2] = fmaf(ad.z, scale[2], x[2] + bias[2]);
-                x[3] = fmaf(ad.w, scale[3], x[3] + bias[3]);
-              }
+              const float4 ad = p.ep.add ? __ldg(reinterpret_cast<const float4*>(p.ep.add + (m0 + 8 * i) * p.ep.ld_add + n)) : make_float4(0.f, 0.f, 0.f, 0.f);
+              x[0] = fmaf(ad.x, scale[0], x[0] + bias[0]);
+              x[1] = fmaf(ad.y, scale[1], x[1] + bias[1]);
+              x[2] = fmaf(ad.z, scale[2], x[2] + bias[2]);
+              x[3] = fmaf(ad.w, scale[3], x[3] + bias[3]);
             }
           }
 #pragma unroll
@@ -289,33 +221,26 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
         }
       } else {
         float copy[kChunks * 32];
-        int copy_unit[4];
 #pragma unroll
         for (int i = 0; i < kChunks * 32; ++i) copy[i] = sum[i >> 5][i >> 3 & 3][i & 7];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) copy_unit[i] = unit[i];
 #pragma unroll 1
         for (int c = 0; c < kChunks; ++c) {   // a vector of eight columns of four rows, all that is read for it on its way at once (one element
           // after element: 2023 x 16 x 256 with 16 columns added held the launch for 4 us more)
           const int n = n0 + c * 32 + (lane & 3) * 8, left = p.N - n;
-          int unit_col[8];
           float bias[8], scale[8], add[4][8];
 #pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            unit_col[e] = __ldg(p.unit_w + n + e);
-            if (kEp) {
-              bias[e] = p.ep.bias && e < left ? __ldg(p.ep.bias + n + e) : 0.f;
-              scale[e] = p.ep.add_scale && e < left ? __ldg(p.ep.add_scale + n + e) : 1.f;
+          for (int e = 0; e < 8 && kEp; ++e) {
+            bias[e] = p.ep.bias && e < left ? __ldg(p.ep.bias + n + e) : 0.f;
+            scale[e] = p.ep.add_scale && e < left ? __ldg(p.ep.add_scale + n + e) : 1.f;
 #pragma unroll
-              for (int i = 0; i < 4; ++i) add[i][e] = p.ep.add && e < left && m0 + 8 * i < p.M ? __ldg(p.ep.add + (m0 + 8 * i) * p.ep.ld_add + n + e) : 0.f;
-            }
+            for (int i = 0; i < 4; ++i) add[i][e] = p.ep.add && e < left && m0 + 8 * i < p.M ? __ldg(p.ep.add + (m0 + 8 * i) * p.ep.ld_add + n + e) : 0.f;
           }
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             float x[8];
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
-              x[e] = scale_by(copy[(c * 4 + i) * 8 + e], copy_unit[i] + unit_col[e]);
+              x[e] = copy[(c * 4 + i) * 8 + e];
               if (kEp) x[e] = fmaf(add[i][e], scale[e], x[e] + bias[e]);
             }
             store8(dst + (m0 + 8 * i) * p.ldc + n, m0 + 8 * i < p.M ? left : 0, p.c_vec, x);
@@ -329,22 +254,22 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
     // A warp converts 16 rows, in blocks of 8 rows x 32 k; a lane owns 8 consecutive k of a row, eight consecutive lanes eight rows
     // (no bank conflicts on either side: the float32 tile is swizzled).
     const int pw = warp - kEpilogueWarps, r0 = pw * 16 + (lane & 7);
-    int stage = 0, raw = 0, turn = 0;
+    int stage = 0, raw = 0;
     uint32_t parity = 1, raw_parity = 0;   // a fresh barrier's previous phase counts as complete
-    int unit[2] = {};             // of this lane's rows
     Walk at(first_tile, tile_step, nt, mt);
     for (int tile = first_tile; tile < tiles; tile += tile_step, at.next(nt, mt)) {
       const int k_len = k_length(at);
 #pragma unroll 1
-      for (int seg = 0; seg < k_len; seg += kBK, ++turn) {
+      for (int seg = 0; seg < k_len; seg += kBK) {
         float x[2][2][8];
         if (kWide) wait(&raw_full[raw], raw_parity);
         const uint8_t* const src = smem + L::kRawAt + raw * L::kRaw + r0 * 128;
         const int m = at.m * kTileM + rank * kBM + r0, k = at.sp * p.k_split + seg + (lane >> 3) * 8;
+        uint32_t seen = 0;
 #pragma unroll
         for (int g = 0; g < 2; ++g)
 #pragma unroll
-          for (int b = 0; b < 2; ++b)
+          for (int b = 0; b < 2; ++b) {
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
               if (!kWide) {
@@ -355,51 +280,29 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
               }
               read_once(src + b * (L::kRaw / 2) + g * 1024 + (((lane >> 3) * 2 + h) ^ (lane & 7)) * 16, x[g][b] + 4 * h);
             }
-        float most[2];
 #pragma unroll
-        for (int g = 0; g < 2; ++g) {
-          float m[8];
-#pragma unroll
-          for (int e = 0; e < 8; ++e) m[e] = fmaxf(fabsf(x[g][0][e]), fabsf(x[g][1][e]));
-          most[g] = fmaxf(fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3])), fmaxf(fmaxf(m[4], m[5]), fmaxf(m[6], m[7])));
-          most[g] = fmaxf(most[g], __shfl_xor_sync(0xffffffffu, most[g], 8));
-          most[g] = fmaxf(most[g], __shfl_xor_sync(0xffffffffu, most[g], 16));
-        }
-        // The tile may be overwritten once every lane has its values: the vote takes the maxima, and those take all of them.
-        if (kWide && !__any_sync(0xffffffffu, most[0] < 0.f || most[1] < 0.f) && lane == 0) arrive(&raw_empty[raw]);
-        if (++raw == L::kRaws) { raw = 0; raw_parity ^= 1; }
-        const int slot = turn % kSlots;
-        bool event = false;
-        float s[2];
-#pragma unroll
-        for (int g = 0; g < 2; ++g) {
-          const int u = unit_of(most[g]);
-          if (seg == 0 || u > unit[g]) {
-            event |= seg > 0;
-            unit[g] = u + kHeadroom;
+            for (int e = 0; e < 8; ++e) seen |= __float_as_uint(x[g][b][e]);
           }
-          s[g] = scale_of(unit[g]);
+        if (kWide) {   // the tile may be overwritten once every lane has its values: the vote takes all of them, and the arrival the vote
+          const int off = __any_sync(0xffffffffu, seen == 1u) ? p.zero : 0;
+          if (lane == 0) arrive(&raw_empty[raw] + off);
+          if (++raw == L::kRaws) { raw = 0; raw_parity ^= 1; }
         }
         wait(&empty[stage], parity);
         uint8_t* const base = smem + stage * L::kStage + ((lane >> 3) * kBM + r0) * 16;
 #pragma unroll
-        for (int g = 0; g < 2; ++g) {
-          if (lane < 8) units[slot * 128 + r0 + g * 8] = static_cast<int8_t>(unit[g]);
+        for (int g = 0; g < 2; ++g)
 #pragma unroll
           for (int b = 0; b < 2; ++b) {
-            uint4 hi, lo;
-            split8(x[g][b], s[g], hi, lo);
+            uint4 hi, mid, lo;
+            split8(x[g][b], hi, mid, lo);
             uint8_t* const dst = base + (b * 4 * kBM + g * 8) * 16;
             *reinterpret_cast<uint4*>(dst) = hi;
-            *reinterpret_cast<uint4*>(dst + L::kPlaneA) = lo;
+            *reinterpret_cast<uint4*>(dst + L::kPlaneA) = mid;
+            *reinterpret_cast<uint4*>(dst + 2 * L::kPlaneA) = lo;
           }
-        }
-        if (event)   // before the arrivals that let the MMAs of this stage begin
-          for (int r = 0; r < (kPair ? 2 : 1); ++r) store_at(events + slot, r, turn + 1u);
         fence_smem_to_async();
-        const bool told_event = __any_sync(0xffffffffu, event);
         __syncwarp();
-        if (kPair && told_event) asm volatile("fence.acq_rel.cluster;" ::: "memory");   // (by the lane that arrives; its arrival is a release in the CTA)
         if (lane == 0) {
           if (kPair) arrive_written(&full[stage]);
           else arrive(&full[stage]);
@@ -412,77 +315,70 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
     if (warp == kMmaWarp) {
       // ---------------------------------------------------------- tensor core
       const bool leader = elect_one();
-      const uint32_t idesc = idesc_f16(kTileM, BN, false, false);
-      int stage = 0, turn = 0, main_turn = 0, low_turn = 0;
+      const uint32_t idesc = idesc_bf16(kTileM, BN, false, false);
+      int slot = 0, main_turn = 0, low_turn = 0;
       uint32_t parity = 0;
       const auto done = [&](uint64_t* bar) {
         if (leader) (kPair ? commit_pair : commit)(bar);
       };
       Walk at(first_tile, tile_step, nt, mt);
       for (int tile = first_tile; tile < tiles; tile += tile_step, at.next(nt, mt)) {
-        const int k_len = k_length(at);
-        bool low_open = false;
-        int run = 0, most = 0;   // stages in the hi*hi accumulator, and how many it takes
-        for (int seg = 0; seg < k_len; seg += kBK, ++turn) {
-          wait(&full[stage], parity);
+        const int k_len = k_length(at), stages = (k_len + kBK - 1) / kBK;
+        int run = 0;   // stages in the hi*hi accumulator
+        for (int stage = 0; stage < stages; ++stage) {
+          wait(&full[slot], parity);
           if (kPair && rank != 0) {   // the other CTA issues
-            if (leader) arrive_written(&peer_full[stage]);
+            if (leader) arrive_written(&peer_full[slot]);
             __syncwarp();
-            if (++stage == kStages) { stage = 0; parity ^= 1; }
+            if (++slot == kStages) { slot = 0; parity ^= 1; }
             continue;
           }
-          if (kPair) wait(&peer_full[stage], parity);
-          const bool event = seg > 0 && event_at(turn);
-          if (event) {
-            if (run > 0) done(&main_full[main_turn++ % kSets]);
-            run = 0;
-            done(&low_full[low_turn % kSets]);
-            ++low_turn;
-            low_open = false;
-          }
-          const uint32_t sa = smem_u32(smem + stage * L::kStage), sb = sa + 2 * L::kPlaneA;
-          const Operand a0{sa, kBM, false}, a1{sa + L::kPlaneA, kBM, false}, b0{sb, kRowsB, false}, b1{sb + L::kPlaneB, kRowsB, false};
-          const int steps = min(kBK, k_len - seg + 15) / 16;   // of 16 k
-          const auto product = [&](uint32_t d, const Operand& a, const Operand& b, bool accumulate) {
-            const uint64_t da = a.desc(0), db = b.desc(0);
+          if (kPair) wait(&peer_full[slot], parity);
+          const uint32_t sa = smem_u32(smem + slot * L::kStage), sb = sa + 3 * L::kPlaneA;
+          const auto a = [&](int i) { return Operand{sa + i * L::kPlaneA, kBM, false}; };   // hi, mid, lo
+          const auto b = [&](int i) { return Operand{sb + i * L::kPlaneB, kRowsB, false}; };
+          const int steps = min(kBK, k_len - stage * kBK + 15) / 16;   // of 16 k
+          const auto product = [&](uint32_t d, const Operand& x, const Operand& y, bool accumulate) {
+            const uint64_t dx = x.desc(0), dy = y.desc(0);
 #pragma unroll
             for (int k = 0; k < kBK / 16; ++k)
               if (leader && k < steps)
-                (kPair ? mma_bf16_pair : mma_bf16)(d, da + static_cast<uint64_t>(k * a.advance()), db + static_cast<uint64_t>(k * b.advance()), idesc,
+                (kPair ? mma_bf16_pair : mma_bf16)(d, dx + static_cast<uint64_t>(k * x.advance()), dy + static_cast<uint64_t>(k * y.advance()), idesc,
                                                   (accumulate || k > 0) ? 1u : 0u);
           };
-          const int set = main_turn % kSets;
-          const uint32_t acc = tmem + set * 2 * BN, low = tmem + (low_turn % kSets) * 2 * BN + BN;
-          if (run == 0) {
-            // (a run that an event begins is one stage: the epilogue learns of the event by its end, and until it has drained the
-            // small products' accumulator the next one cannot be begun)
-            most = seg == 0 ? kFirstRun : event ? 1 : p.run;
-            wait(&main_empty[set], ((main_turn / kSets) & 1) ^ 1);
-          }
+          const int set = main_turn % kSets, low_set = low_turn % kSets;
+          const uint32_t acc = tmem + set * 2 * BN, low = tmem + low_set * 2 * BN + BN;
+          if (run == 0) wait(&main_empty[set], ((main_turn / kSets) & 1) ^ 1);
           fence_after_sync();
-          product(acc, a0, b0, run > 0);
-          if (++run == most || seg + kBK >= k_len) {
+          product(acc, a(0), b(0), run > 0);
+          const bool last = stage + 1 == stages;
+          if (++run == (stage < kFirstRun ? kFirstRun : p.run) || last) {
             done(&main_full[set]);
             ++main_turn;
             run = 0;
           }
-          if (!low_open) {
-            wait(&low_empty[low_turn % kSets], ((low_turn / kSets) & 1) ^ 1);
+          const bool fresh = stage % kLowRun == 0;
+          if (fresh) {
+            wait(&low_empty[low_set], ((low_turn / kSets) & 1) ^ 1);
             fence_after_sync();
           }
-          product(low, a0, b1, low_open);
-          product(low, a1, b0, true);
-          low_open = true;
-          done(&empty[stage]);
-          if (++stage == kStages) { stage = 0; parity ^= 1; }
+          product(low, a(2), b(0), !fresh);
+          product(low, a(0), b(2), true);
+          product(low, a(1), b(1), true);
+          product(low, a(1), b(0), true);
+          product(low, a(0), b(1), true);
+          done(&empty[slot]);
+          if ((stage + 1) % kLowRun == 0 || last) {
+            done(&low_full[low_set]);
+            ++low_turn;
+          }
+          if (++slot == kStages) { slot = 0; parity ^= 1; }
         }
-        if (rank == 0) done(&low_full[low_turn % kSets]);
-        ++low_turn;
       }
       // the last commits may still be on their way to barriers in this CTA's shared memory
       for (int s = 0; s < kStages; ++s) {
-        wait(&empty[stage], parity ^ 1);
-        if (++stage == kStages) { stage = 0; parity ^= 1; }
+        wait(&empty[slot], parity ^ 1);
+        if (++slot == kStages) { slot = 0; parity ^= 1; }
       }
     } else if (warp == L::kImageWarp && lane == 0) {
       // ---------------------------------------------------------- the weight's image
@@ -492,11 +388,11 @@ __global__ void __launch_bounds__(Config<BN>::kThreads, 1) gemm32_f16_kernel(con
       Walk at(first_tile, tile_step, nt, mt);
       for (int tile = first_tile; tile < tiles; tile += tile_step, at.next(nt, mt)) {
         const int n0 = at.n * BN + rank * kRowsB, k0 = at.sp * p.k_split, k_len = k_length(at);
-        const uint8_t* image = p.image + (static_cast<size_t>(n0 / kRowsB) * k_images + k0 / kBK) * (2 * L::kPlaneB);
-        for (int seg = 0; seg < k_len; seg += kBK, image += 2 * L::kPlaneB) {
+        const uint8_t* image = p.image + (static_cast<size_t>(n0 / kRowsB) * k_images + k0 / kBK) * (3 * L::kPlaneB);
+        for (int seg = 0; seg < k_len; seg += kBK, image += 3 * L::kPlaneB) {
           wait(&empty[stage], parity);
-          tma::expect_bytes(&full[stage], 2 * L::kPlaneB);
-          tma::load_bulk(smem + stage * L::kStage + 2 * L::kPlaneA, image, 2 * L::kPlaneB, &full[stage]);
+          tma::expect_bytes(&full[stage], 3 * L::kPlaneB);
+          tma::load_bulk(smem + stage * L::kStage + 3 * L::kPlaneA, image, 3 * L::kPlaneB, &full[stage]);
           if (++stage == kStages) { stage = 0; parity ^= 1; }
         }
       }
@@ -536,8 +432,8 @@ int tile_ctas(int bn) { return bn == 64 ? 1 : 2; }
 template <int BN, bool kWide, bool kEp>
 int launch(const Params& p, long long ctas, cudaStream_t stream) {
   using L = Config<BN>;
-  if (const int st = allow_smem<gemm32_f16_kernel<BN, kWide, kEp>, L::kBytes>(); st != MXK_OK) return st;
-  mxk::launch_kernel_clusters(gemm32_f16_kernel<BN, kWide, kEp>, L::kPair ? 2 : 1, static_cast<unsigned>(std::min(ctas, static_cast<long long>(kNumSMs))),
+  if (const int st = allow_smem<gemm32_long_kernel<BN, kWide, kEp>, L::kBytes>(); st != MXK_OK) return st;
+  mxk::launch_kernel_clusters(gemm32_long_kernel<BN, kWide, kEp>, L::kPair ? 2 : 1, static_cast<unsigned>(std::min(ctas, static_cast<long long>(kNumSMs))),
                               L::kThreads, L::kBytes, stream, p);
   return launch_status();
 }
@@ -572,7 +468,6 @@ int launch_weights(const Plan& pl, const float* a, long long lda, const void* im
   Params p{};
   p.a = a; p.lda = lda;
   p.image = static_cast<const uint8_t*>(image);
-  p.unit_w = reinterpret_cast<const int*>(p.image + planes_bytes(pl.bn, N, K));
   p.c = pl.splits > 1 ? partial : c;
   p.ldc = pl.splits > 1 ? N : ldc;
   p.M = M; p.N = N; p.K = K;
@@ -595,6 +490,6 @@ int launch_weights(const Plan& pl, const float* a, long long lda, const void* im
   return pl.bn == 256 ? launch<256>(p, wide, ctas, stream) : pl.bn == 128 ? launch<128>(p, wide, ctas, stream) : launch<64>(p, wide, ctas, stream);
 }
 
-}  // namespace f16
+}  // namespace longk
 }  // namespace gemm32
 }  // namespace mxk

@@ -1,31 +1,26 @@
-// float32 products of two activations, C = A^T B (the gradient of a weight), contractions of 256 tokens and more, on the tensor
-// cores: scaled float16 planes as in gemm32_f16.cu.
+// float32 products of two activations, C = A^T B (the gradient of a weight), contractions of more than kShortK tokens, on the tensor cores:
+// three bf16 planes and six products as in gemm32_long.cu.
 //
-// Both operands are contracted over their rows and converted here.  Scales are per column: that of its first kBK tokens in a tile,
-// with room for elements 2^kHeadroom larger; where one later does not fit, a new unit begins at that stage (`event`) and the
-// accumulators are closed before it.  They live for one stage, two in contractions from 512 on, in any case (eight truncating
-// additions), and are then added to float32 sums in registers, which are kept in the columns' units.  Errors against float64,
-// relative 2-norm, normal entries: 2.1e-7 at 4096 tokens, 2.4e-7 at 24000 (three bf16 planes, drained every 512 tokens: 4.3e-7 and
-// 4.7e-7); lognormal, sigma 3: 1.1e-7 (4.0e-7).
+// Both operands are contracted over their rows and converted here.  The accumulators live for one stage, two in contractions from 512 on
+// (eight truncating additions), and are then added to float32 sums in registers.  Errors against float64, relative 2-norm, normal entries: 1.4e-7 at
+// 8192 tokens, 1.9e-7 at 65536 (drained every 512 tokens: 4.2e-7 and 4.75e-7).
 //
-// Bound: shared memory and the producers.  A stage of 256 x 128 is 768 cycles of the tensor pipe and 12288 numbers to convert, about
-// 1200 cycles of the issue slots; they cross shared memory five times over (the copy in, the producers' reads, the planes, the pipe's
-// reads of A and of both halves of B: 1920 cycles at 128 bytes), and it takes 2400: the twelve warps wait for the same barriers and
-// are in the same phase of their work.
-// Measured (three bf16 planes before): 1024 x 256 over 65536 tokens 151 us (185), 1024 x 512 over 24000 114 us (137), 520 x 512
-// over 8192 36 us (38).
+// Bound: shared memory.  A stage of 256 x 128 is 1536 cycles of the tensor pipe, but 48 KB copied in and read by the producers, 72 KB of planes
+// written and 192 KB read by the pipe (A and both halves of B for six products): 2800 cycles at 128 bytes.
+// Measured with the sum of the splits (the form of gemm32.cu): 1024 x 256 over 65536 tokens 202 us (204), 1024 x 512 over 24000 153 us (148),
+// 520 x 512 over 8192 53 us (50).
 //
 // One persistent CTA per SM, pairs on tiles of 256 x 128, or alone on 128 x 64:
 //   8 warps    epilogue: accumulators (TMEM) -> sums in registers -> global
 //   12 warps   producers: 32 columns x 32 tokens of a stage each, eight warps for A and four for B
-//   1 warp     issues the MMAs (12 per stage of 64 tokens), 1 warp the copies of both float32 tiles (TMA)
+//   1 warp     issues the MMAs (24 per stage of 64 tokens), 1 warp the copies of both float32 tiles (TMA)
 #include <algorithm>
 
 #include "gemm32_common.cuh"
 
 namespace mxk {
 namespace gemm32 {
-namespace f16 {
+namespace longk {
 namespace {
 
 using namespace umma;
@@ -43,6 +38,7 @@ struct Params {
   int k_split;           // tokens per split (a multiple of kBK)
   int splits;            // more than one: c is [splits][M][N]
   int run;               // stages that the accumulators live for
+  int zero;              // 0
   int* status;
 };
 
@@ -51,16 +47,13 @@ template <bool kPair>
 struct Config {
   static constexpr int kTileM = kPair ? 2 * kBM : kBM, kBN = kPair ? 128 : 64, kColsB = 64;   // columns of B in this CTA
   static constexpr int kPlaneA = kBM * kBK * 2, kPlaneB = kColsB * kBK * 2;   // bytes
-  static constexpr int kStage = 2 * (kPlaneA + kPlaneB), kStages = 2;
-  static constexpr int kBox = 32 * kBK * 4, kRaw = (kBM + kColsB) / 32 * kBox, kRaws = 2;   // float32 tiles: boxes of 32 columns, rows of 128 bytes
+  static constexpr int kStage = 3 * (kPlaneA + kPlaneB), kStages = 2;
+  static constexpr int kBox = 32 * kBK * 4, kRaw = (kBM + kColsB) / 32 * kBox, kRaws = 1;   // float32 tiles: boxes of 32 columns, rows of 128 bytes
   static constexpr int kSets = 2;   // accumulators: kBN columns for hi*hi and kBN for the small products, twice
   static constexpr uint32_t kTmem = kSets * 2 * kBN;
   static constexpr int kRawAt = kStages * kStage;
-  static constexpr int kUnits = kRawAt + kRaws * kRaw;             // int8 [kSlots][128 + 128], units of the columns of A and B
-  static constexpr int kMax = kUnits + kSlots * 256;               // float [2][6][2][32], maxima of the halves of a stage
-  static constexpr int kEvents = kMax + 2 * 6 * 2 * 32 * 4;        // [kSlots]
-  static constexpr int kBarriers = kEvents + kSlots * 4;
-  static constexpr int kBytes = kBarriers + (2 * kStages + 2 * kRaws + 2 * kSets + kSlots + 2) * 8;
+  static constexpr int kBarriers = kRawAt + kRaws * kRaw;
+  static constexpr int kBytes = kBarriers + (2 * kStages + 2 * kRaws + 2 * kSets + 2) * 8;
   static constexpr int kEpilogueWarps = 8, kProducerWarps = 12, kWarpsA = 8;
   static constexpr int kMmaWarp = kEpilogueWarps + kProducerWarps, kRawWarp = kMmaWarp + 1;
   static constexpr int kThreads = 32 * (kMmaWarp + 4);   // warpgroups deal registers: 768 threads of 80
@@ -68,17 +61,8 @@ struct Config {
   static_assert(kEpilogueWarps * kRegsEpilogue + kProducerWarps * kRegsProducer + 4 * kRegsMma == kThreads / 32 * 80, "the launch's registers");
 };
 
-// Sixteen bytes to the other CTA of the pair, counted by the barrier of this offset there.
-__device__ __forceinline__ void send16(void* p, uint64_t* bar, int rank, uint4 v) {
-  asm volatile(
-      "{\n\t.reg .b32 ra, rb;\n\tmapa.shared::cluster.u32 ra, %0, %2;\n\tmapa.shared::cluster.u32 rb, %1, %2;\n\t"
-      "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [ra], {%3, %4, %5, %6}, [rb];\n\t}\n" ::"r"(smem_u32(p)),
-      "r"(smem_u32(bar)), "r"(rank), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
-      : "memory");
-}
-
 template <bool kPair, bool kWide>
-__global__ void __launch_bounds__(Config<kPair>::kThreads, 1) gemm32_f16_outer_kernel(const __grid_constant__ Params p) {
+__global__ void __launch_bounds__(Config<kPair>::kThreads, 1) gemm32_long_outer_kernel(const __grid_constant__ Params p) {
   using L = Config<kPair>;
   constexpr int kStages = L::kStages, kSets = L::kSets, kTileM = L::kTileM, BN = L::kBN;
   constexpr int kEpilogueWarps = L::kEpilogueWarps, kProducerWarps = L::kProducerWarps, kMmaWarp = L::kMmaWarp;
@@ -92,22 +76,17 @@ __global__ void __launch_bounds__(Config<kPair>::kThreads, 1) gemm32_f16_outer_k
   uint64_t* const empty = full + kStages;        // MMA -> producers
   uint64_t* const acc_full = empty + kStages;    // MMA -> epilogue
   uint64_t* const acc_empty = acc_full + kSets;  // epilogue -> MMA
-  uint64_t* const peer_units = acc_empty + kSets;   // the other CTA's units of B's columns
-  uint64_t* const raw_full = peer_units + kSlots;   // copies -> producers, the float32 tiles
+  uint64_t* const raw_full = acc_empty + kSets;  // copies -> producers, the float32 tiles
   uint64_t* const raw_empty = raw_full + L::kRaws;
   uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(raw_empty + L::kRaws);
-  int8_t* const units = reinterpret_cast<int8_t*>(smem + L::kUnits);
-  uint32_t* const events = reinterpret_cast<uint32_t*>(smem + L::kEvents);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (tid == 0) {
     for (int s = 0; s < kStages; ++s) { mbar_init(&full[s], kProducerWarps * (kPair ? 2 : 1)); mbar_init(&empty[s], 1); }
     for (int s = 0; s < kSets; ++s) { mbar_init(&acc_full[s], 1); mbar_init(&acc_empty[s], kEpilogueWarps * (kPair ? 2 : 1)); }
-    for (int s = 0; s < kSlots; ++s) mbar_init(&peer_units[s], 1);
     for (int s = 0; s < L::kRaws; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], kProducerWarps); }
     mbar_init_fence();
   }
-  if (tid < kSlots) events[tid] = 0;
   if (warp == kMmaWarp) {
     if (kPair) tmem_alloc_pair(tmem_slot, L::kTmem);
     else tmem_alloc(tmem_slot, L::kTmem);
@@ -118,58 +97,32 @@ __global__ void __launch_bounds__(Config<kPair>::kThreads, 1) gemm32_f16_outer_k
   fence_after_sync();
   const uint32_t tmem = *tmem_slot;
   bool timed_out = false;
-  // (of a pair, either CTA arrives on the other's barriers, and stores what is read behind them)
+  // (of a pair, either CTA arrives on the other's barriers)
   const auto wait = [&](uint64_t* bar, uint32_t parity) { (kPair ? mbar_wait_cluster_flag : mbar_wait_flag)(bar, parity, timed_out); };
   const auto k_length = [&](int tile) {
     const int sp = tile / (mt * nt);
     return min(p.K, (sp + 1) * p.k_split) - sp * p.k_split;
   };
-  // Whether a column of the tile begins a new unit at this stage; the same in both CTAs.
-  const auto event_at = [&](int turn) { return *const_cast<volatile uint32_t*>(events + turn % kSlots) == turn + 1u; };
-
   if (warp < kEpilogueWarps) {
     // ------------------------------------------------------------ epilogue
     more_registers<L::kRegsEpilogue>();
     constexpr int kChunks = BN / 64;   // of 32 columns
     const int col0 = (warp >> 2) * (BN / 2), row0 = (warp & 3) * 32 + (lane >> 2);   // this thread: rows row0 + 8 i
     float sum[kChunks][4][8];          // [2 j + e]: column 32 c + 8 j + 2 (lane % 4) + e
-    int turn = 0, run = 0;
+    int turn = 0;   // accumulators
     for (int tile = first_tile; tile < tiles; tile += tile_step) {
       const int mn = tile % (mt * nt), sp = tile / (mt * nt);
       const int n0 = (mn % nt) * BN + col0, m0 = (mn / nt) * kTileM + rank * kBM + row0;
-      const int k_len = k_length(tile);
+      const int stages = (k_length(tile) + kBK - 1) / kBK;
 #pragma unroll
       for (int c = 0; c < kChunks; ++c)
 #pragma unroll
         for (int i = 0; i < 32; ++i) sum[c][i >> 3][i & 7] = 0.f;
-      const int8_t* unit = nullptr;   // of the sums: a slot, whose units are those of the stages after it up to the next event
 #pragma unroll 1
-      for (int seg = 0; seg < k_len; ++run) {
-        const int set = run % kSets;
-        wait(&acc_full[set], (run / kSets) & 1);
+      for (int stage = 0; stage < stages; stage += p.run, ++turn) {
+        const int set = turn % kSets;
+        wait(&acc_full[set], (turn / kSets) & 1);
         fence_after_sync();
-        const int8_t* const next = units + turn % kSlots * 256;
-        if (seg > 0 && event_at(turn)) {   // the sums are brought to the new units, none of which is smaller
-          if (kPair) wait(&peer_units[turn % kSlots], (turn / kSlots) & 1);
-#pragma unroll
-          for (int c = 0; c < kChunks; ++c)
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              const int at = 128 + col0 + c * 32 + (e >> 1) * 8 + (lane & 3) * 2 + (e & 1);
-              const float r = pow2(max(unit[at] - next[at], -126));
-#pragma unroll
-              for (int i = 0; i < 4; ++i) sum[c][i][e] *= r;
-            }
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float r = pow2(max(unit[row0 + 8 * i] - next[row0 + 8 * i], -126));
-#pragma unroll
-            for (int c = 0; c < kChunks; ++c)
-#pragma unroll
-              for (int e = 0; e < 8; ++e) sum[c][i][e] *= r;
-          }
-        }
-        unit = next;
         const uint32_t src = tmem + set * 2 * BN + col0 + (static_cast<uint32_t>((warp & 3) * 32) << 16);
 #pragma unroll
         for (int c = 0; c < kChunks; ++c)
@@ -182,7 +135,7 @@ __global__ void __launch_bounds__(Config<kPair>::kThreads, 1) gemm32_f16_outer_k
 #pragma unroll
             for (int j = 0; j < 4; ++j)
 #pragma unroll
-              for (int i = 0; i < 4; ++i) sum[c][2 * h + (i >> 1)][2 * j + (i & 1)] += fmaf(__uint_as_float(q[4 * j + i]), 1.f / kLo, __uint_as_float(r[4 * j + i]));
+              for (int i = 0; i < 4; ++i) sum[c][2 * h + (i >> 1)][2 * j + (i & 1)] += __uint_as_float(r[4 * j + i]) + __uint_as_float(q[4 * j + i]);
           }
         fence_before_sync();
         __syncwarp();
@@ -190,36 +143,23 @@ __global__ void __launch_bounds__(Config<kPair>::kThreads, 1) gemm32_f16_outer_k
           if (kPair) arrive_read(&acc_empty[set]);
           else arrive(&acc_empty[set]);
         }
-        int n = 0;   // an event ends a run
-        do {
-          // The other CTA's units come by themselves: nothing else says that they are there, and none may be on its way when the kernel ends.
-          if (kPair) wait(&peer_units[turn % kSlots], (turn / kSlots) & 1);
-          ++n;
-          seg += kBK;
-          ++turn;
-        } while (n < p.run && seg < k_len && !event_at(turn));
       }
       float* const dst = p.c + (p.splits > 1 ? static_cast<size_t>(sp) * p.M * p.N : 0);
-      int unit_row[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) unit_row[i] = unit[row0 + 8 * i];
 #pragma unroll
       for (int c = 0; c < kChunks; ++c)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const int nc = c * 32 + j * 8 + (lane & 3) * 2, n = n0 + nc;
-          const char2 unit_col = *reinterpret_cast<const char2*>(unit + 128 + col0 + nc);
+          const int n = n0 + c * 32 + j * 8 + (lane & 3) * 2;
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const int m = m0 + 8 * i;
-            const float2 v = make_float2(scale_by(sum[c][i][2 * j], unit_row[i] + unit_col.x), scale_by(sum[c][i][2 * j + 1], unit_row[i] + unit_col.y));
             if (m >= p.M || n >= p.N) continue;
             float* const out = dst + m * p.ldc + n;
             if (p.c_vec >= 4 && n + 1 < p.N) {
-              *reinterpret_cast<float2*>(out) = v;
+              *reinterpret_cast<float2*>(out) = make_float2(sum[c][i][2 * j], sum[c][i][2 * j + 1]);
             } else {
-              out[0] = v.x;
-              if (n + 1 < p.N) out[1] = v.y;
+              out[0] = sum[c][i][2 * j];
+              if (n + 1 < p.N) out[1] = sum[c][i][2 * j + 1];
             }
           }
         }
@@ -228,16 +168,13 @@ __global__ void __launch_bounds__(Config<kPair>::kThreads, 1) gemm32_f16_outer_k
     // ------------------------------------------------------------ producers
     fewer_registers<L::kRegsProducer>();
     // A warp converts 32 columns x 32 tokens, a column a lane, and leaves vectors of eight tokens: what was contracted over rows
-    // becomes K-major on the way, with a scale a lane.  Another warp has the stage's other 32 tokens; the two exchange their maxima.
+    // becomes K-major on the way.
     const int pw = warp - kEpilogueWarps;
     const bool is_b = pw >= L::kWarpsA;
-    const int block = is_b ? pw & 1 : pw & 3, half = is_b ? (pw - L::kWarpsA) >> 1 : pw >> 2, partners = is_b ? 4 + block : block;
+    const int block = is_b ? pw & 1 : pw & 3, half = is_b ? (pw - L::kWarpsA) >> 1 : pw >> 2;
     const int col = block * 32 + lane, rows = is_b ? L::kColsB : kBM, plane = is_b ? L::kPlaneB : L::kPlaneA;
-    const int unit_at = is_b ? 128 + rank * L::kColsB + block * 32 : block * 32;   // of this warp's first column in a slot's units
-    float* const maxima = reinterpret_cast<float*>(smem + L::kMax) + partners * 64;
-    int stage = 0, raw = 0, turn = 0;
+    int stage = 0, raw = 0;
     uint32_t parity = 1, raw_parity = 0;
-    int unit = 0;   // of this lane's column
     float x[32];
     const auto load = [&](int tile, int seg) {
       if (kWide) {
@@ -245,6 +182,13 @@ __global__ void __launch_bounds__(Config<kPair>::kThreads, 1) gemm32_f16_outer_k
         const uint8_t* const src = smem + L::kRawAt + raw * L::kRaw + ((is_b ? kBM / 32 : 0) + block) * L::kBox + half * 4096 + (lane & 3) * 4;
 #pragma unroll
         for (int i = 0; i < 32; ++i) x[i] = read_once(src + i * 128 + ((lane >> 2) ^ (i & 7)) * 16);
+        // the tiles may be overwritten once every lane has its values: the vote takes all of them, and the arrival the vote
+        uint32_t seen = 0;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) seen |= __float_as_uint(x[i]);
+        const int off = __any_sync(0xffffffffu, seen == 1u) ? p.zero : 0;
+        if (lane == 0) arrive(&raw_empty[raw] + off);
+        if (++raw == L::kRaws) { raw = 0; raw_parity ^= 1; }
       } else {
         const int mn = tile % (mt * nt), k = tile / (mt * nt) * p.k_split + half * 32 + seg;
         const int c = (is_b ? (mn % nt) * BN + rank * L::kColsB : (mn / nt) * kTileM + rank * kBM) + col, end = is_b ? p.N : p.M;
@@ -258,47 +202,23 @@ __global__ void __launch_bounds__(Config<kPair>::kThreads, 1) gemm32_f16_outer_k
     for (int tile = first_tile; tile < tiles; tile += tile_step) {
       const int k_len = k_length(tile);
 #pragma unroll 1
-      for (int seg = 0; seg < k_len; seg += kBK, ++turn) {
-        float m[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) m[i] = fmaxf(fmaxf(fabsf(x[i]), fabsf(x[i + 8])), fmaxf(fabsf(x[i + 16]), fabsf(x[i + 24])));
-        const float own = fmaxf(fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3])), fmaxf(fmaxf(m[4], m[5]), fmaxf(m[6], m[7])));
-        float* const now = maxima + (turn & 1) * (6 * 64);
-        now[half * 32 + lane] = own;
-        asm volatile("bar.sync %0, 64;" ::"r"(1 + partners) : "memory");
-        // (every lane has all of its values, or its maximum would not be there)
-        if (kWide && lane == 0) arrive(&raw_empty[raw]);
-        if (++raw == L::kRaws) { raw = 0; raw_parity ^= 1; }
-        const int slot = turn % kSlots, u = unit_of(fmaxf(own, now[(half ^ 1) * 32 + lane]));
-        bool event = false;
-        if (seg == 0 || u > unit) {
-          event = seg > 0;
-          unit = u + kHeadroom;
-        }
-        const float scale = scale_of(unit);
+      for (int seg = 0; seg < k_len; seg += kBK) {
         wait(&empty[stage], parity);
-        int8_t* const told = units + slot * 256 + unit_at;
-        if (half == 0) told[lane] = static_cast<int8_t>(unit);
-        uint8_t* const dst = smem + stage * L::kStage + (is_b ? 2 * L::kPlaneA : 0) + (half * 4 * rows + col) * 16;
+        uint8_t* const dst = smem + stage * L::kStage + (is_b ? 3 * L::kPlaneA : 0) + (half * 4 * rows + col) * 16;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          uint4 hi, lo;
-          split8(x + 8 * j, scale, hi, lo);
+          uint4 hi, mid, lo;
+          split8(x + 8 * j, hi, mid, lo);
           *reinterpret_cast<uint4*>(dst + j * rows * 16) = hi;
-          *reinterpret_cast<uint4*>(dst + j * rows * 16 + plane) = lo;
+          *reinterpret_cast<uint4*>(dst + j * rows * 16 + plane) = mid;
+          *reinterpret_cast<uint4*>(dst + j * rows * 16 + 2 * plane) = lo;
         }
         // the next stage's values, on their way under what is left of this one
         if (seg + kBK < k_len) load(tile, seg + kBK);
         else if (tile + tile_step < tiles) load(tile + tile_step, 0);
-        if (event)   // before the arrivals that let the MMAs of this stage begin
-          for (int r = 0; r < (kPair ? 2 : 1); ++r) store_at(events + slot, r, turn + 1u);
         fence_smem_to_async();
-        const bool told_event = __any_sync(0xffffffffu, event);
         __syncwarp();
-        if (kPair && told_event) asm volatile("fence.acq_rel.cluster;" ::: "memory");   // (by the lane that arrives; its arrival is a release in the CTA)
-        if (kPair && is_b && half == 0 && lane < 2) send16(told + 16 * lane, &peer_units[slot], rank ^ 1, *reinterpret_cast<const volatile uint4*>(told + 16 * lane));
         if (lane == 0) {
-          if (kPair && pw == 0) tma::expect_bytes(&peer_units[slot], L::kColsB);
           if (kPair) arrive_written(&full[stage]);
           else arrive(&full[stage]);
         }
@@ -310,57 +230,57 @@ __global__ void __launch_bounds__(Config<kPair>::kThreads, 1) gemm32_f16_outer_k
     if (warp == kMmaWarp) {
       // ---------------------------------------------------------- tensor core
       const bool leader = elect_one();
-      const uint32_t idesc = idesc_f16(kTileM, BN, false, false);
-      int stage = 0, turn = 0, runs = 0;
+      const uint32_t idesc = idesc_bf16(kTileM, BN, false, false);
+      int slot = 0, turn = 0;
       uint32_t parity = 0;
       const auto done = [&](uint64_t* bar) {
         if (leader) (kPair ? commit_pair : commit)(bar);
       };
-        for (int tile = first_tile; tile < tiles; tile += tile_step) {
-          const int k_len = k_length(tile);
-          int run = 0;   // stages in the accumulators
-          for (int seg = 0; seg < k_len; seg += kBK, ++turn) {
-            if (rank != 0) {   // the other CTA issues; its commits reach this one's barriers
-              wait(&empty[stage], parity);
-              if (++stage == kStages) { stage = 0; parity ^= 1; }
-              continue;
-            }
-            wait(&full[stage], parity);
-            if (seg > 0 && run > 0 && event_at(turn)) {
-              done(&acc_full[runs++ % kSets]);
-              run = 0;
-            }
-            const int set = runs % kSets;
-            if (run == 0) wait(&acc_empty[set], ((runs / kSets) & 1) ^ 1);
-            fence_after_sync();
-            const uint32_t sa = smem_u32(smem + stage * L::kStage), sb = sa + 2 * L::kPlaneA, acc = tmem + set * 2 * BN;
-            const Operand a0{sa, kBM, false}, a1{sa + L::kPlaneA, kBM, false}, b0{sb, L::kColsB, false}, b1{sb + L::kPlaneB, L::kColsB, false};
-            const int steps = min(kBK, k_len - seg + 15) / 16;   // of 16 tokens
-            const auto product = [&](uint32_t d, const Operand& a, const Operand& b, bool accumulate) {
-              const uint64_t da = a.desc(0), db = b.desc(0);
-#pragma unroll
-              for (int k = 0; k < kBK / 16; ++k)
-                if (leader && k < steps)
-                  (kPair ? mma_bf16_pair : mma_bf16)(d, da + static_cast<uint64_t>(k * a.advance()), db + static_cast<uint64_t>(k * b.advance()), idesc,
-                                                    (accumulate || k > 0) ? 1u : 0u);
-            };
-            product(acc, a0, b0, run > 0);
-            product(acc + BN, a0, b1, run > 0);
-            product(acc + BN, a1, b0, true);
-            done(&empty[stage]);
-            if (++run == p.run || seg + kBK >= k_len) {
-              done(&acc_full[set]);
-              ++runs;
-              run = 0;
-            }
-            if (++stage == kStages) { stage = 0; parity ^= 1; }
+      for (int tile = first_tile; tile < tiles; tile += tile_step) {
+        const int k_len = k_length(tile);
+        int run = 0;   // stages in the accumulators
+        for (int seg = 0; seg < k_len; seg += kBK) {
+          if (rank != 0) {   // the other CTA issues; its commits reach this one's barriers
+            wait(&empty[slot], parity);
+            if (++slot == kStages) { slot = 0; parity ^= 1; }
+            continue;
           }
+          wait(&full[slot], parity);
+          const int set = turn % kSets;
+          if (run == 0) wait(&acc_empty[set], ((turn / kSets) & 1) ^ 1);
+          fence_after_sync();
+          const uint32_t sa = smem_u32(smem + slot * L::kStage), sb = sa + 3 * L::kPlaneA, acc = tmem + set * 2 * BN, low = acc + BN;
+          const auto a = [&](int i) { return Operand{sa + i * L::kPlaneA, kBM, false}; };   // hi, mid, lo
+          const auto b = [&](int i) { return Operand{sb + i * L::kPlaneB, L::kColsB, false}; };
+          const int steps = min(kBK, k_len - seg + 15) / 16;   // of 16 tokens
+          const auto product = [&](uint32_t d, const Operand& x, const Operand& y, bool accumulate) {
+            const uint64_t dx = x.desc(0), dy = y.desc(0);
+#pragma unroll
+            for (int k = 0; k < kBK / 16; ++k)
+              if (leader && k < steps)
+                (kPair ? mma_bf16_pair : mma_bf16)(d, dx + static_cast<uint64_t>(k * x.advance()), dy + static_cast<uint64_t>(k * y.advance()), idesc,
+                                                  (accumulate || k > 0) ? 1u : 0u);
+          };
+          product(low, a(2), b(0), run > 0);
+          product(low, a(0), b(2), true);
+          product(low, a(1), b(1), true);
+          product(low, a(1), b(0), true);
+          product(low, a(0), b(1), true);
+          product(acc, a(0), b(0), run > 0);
+          done(&empty[slot]);
+          if (++run == p.run || seg + kBK >= k_len) {
+            done(&acc_full[set]);
+            ++turn;
+            run = 0;
+          }
+          if (++slot == kStages) { slot = 0; parity ^= 1; }
         }
-        // the last commits may still be on their way to barriers in this CTA's shared memory
-        for (int s = 0; rank == 0 && s < kStages; ++s) {
-          wait(&empty[stage], parity ^ 1);
-          if (++stage == kStages) { stage = 0; parity ^= 1; }
-        }
+      }
+      // the last commits may still be on their way to barriers in this CTA's shared memory
+      for (int s = 0; rank == 0 && s < kStages; ++s) {
+        wait(&empty[slot], parity ^ 1);
+        if (++slot == kStages) { slot = 0; parity ^= 1; }
+      }
     } else if (kWide && warp == L::kRawWarp && lane == 0) {
       // ---------------------------------------------------------- float32 tiles
       int raw = 0;
@@ -397,8 +317,8 @@ int tile_ctas(int bn) { return bn == 64 ? 1 : 2; }
 template <bool kPair, bool kWide>
 int launch(const Params& p, long long ctas, cudaStream_t stream) {
   using L = Config<kPair>;
-  if (const int st = allow_smem<gemm32_f16_outer_kernel<kPair, kWide>, L::kBytes>(); st != MXK_OK) return st;
-  mxk::launch_kernel_clusters(gemm32_f16_outer_kernel<kPair, kWide>, kPair ? 2 : 1, static_cast<unsigned>(std::min(ctas, static_cast<long long>(kNumSMs))),
+  if (const int st = allow_smem<gemm32_long_outer_kernel<kPair, kWide>, L::kBytes>(); st != MXK_OK) return st;
+  mxk::launch_kernel_clusters(gemm32_long_outer_kernel<kPair, kWide>, kPair ? 2 : 1, static_cast<unsigned>(std::min(ctas, static_cast<long long>(kNumSMs))),
                               L::kThreads, L::kBytes, stream, p);
   return launch_status();
 }
@@ -455,6 +375,6 @@ int launch_outer(const Plan& pl, const float* a, long long lda, const float* b, 
   return wide ? launch<false, true>(p, ctas, stream) : launch<false, false>(p, ctas, stream);
 }
 
-}  // namespace f16
+}  // namespace longk
 }  // namespace gemm32
 }  // namespace mxk

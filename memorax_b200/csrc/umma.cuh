@@ -47,11 +47,6 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N, bool a_mn_major,
          (static_cast<uint32_t>(M >> 4) << 24);
 }
 
-// The same with float16 operands.
-__host__ __device__ constexpr uint32_t idesc_f16(int M, int N, bool a_mn_major, bool b_mn_major) {
-  return idesc_bf16(M, N, a_mn_major, b_mn_major) & ~((1u << 7) | (1u << 10));
-}
-
 // 128-byte-swizzled row-major tiles ("SW tiles"): rows of 64 two-byte elements, one 128-byte line per
 // row, the 16-byte chunk j of row r stored at chunk position j ^ (r & 7); tile base 1024-byte aligned.
 // This is what a tiled TMA load with CU_TENSOR_MAP_SWIZZLE_128B writes (128-byte pieces instead of the

@@ -102,6 +102,31 @@ def test_few_channels_at_the_kink(feat, near, bsz):
     assert float((slope[rows] - torch.where(acc >= 0, 1.0, 0.25).double()).abs().max()) <= 1e-3
 
 
+# Two large terms that nearly cancel, for many tokens and channels, in short and in long products.  A channel's own feature is zero in
+# every input and its weight is 2^-10, so that the inputs' gradients there are those of the pre-activations, 1/2 g'.
+@pytest.mark.parametrize("feat", [130, 256, 515])
+def test_cancelling_terms_at_the_kink(feat):
+    from memorax_b200.memoroid import MinGRUCell, Memoroid
+    torch.manual_seed(feat)
+    bsz, steps, dim = 64, 128, 64
+    cell = MinGRUCell(dim, in_features=feat)
+    x = torch.zeros(bsz, steps, feat)
+    x[..., 2] = 1 + torch.rand(bsz, steps)
+    x[..., feat - 1] = -x[..., 2] * (1 + 2.0 ** -20 * torch.randn(bsz, steps))
+    with torch.no_grad():
+        cell.z.weight.zero_()
+        w = cell.h.weight.zero_()
+        w[:, 2] = 1 + torch.rand(dim)
+        w[:, feat - 1] = w[:, 2] * (1 + 2.0 ** -20 * torch.randn(dim))
+        w[torch.arange(dim), 3 + torch.arange(dim)] = 2.0 ** -10
+        first = (x[..., 2].double()[..., None] * w[:, 2].double()).float()              # the sum in order: one rounding,
+        side = first.double() + x[..., feat - 1].double()[..., None] * w[:, feat - 1].double() >= 0   # then its sign
+    cell, x = cell.cuda(), x.cuda().requires_grad_()
+    _, y = Memoroid(cell)(x, torch.ones(bsz, steps, device="cuda"), None)
+    slope = torch.autograd.grad(y, x, torch.ones_like(y))[0][..., 3:3 + dim].cpu() * 2 ** 11
+    assert float((slope - torch.where(side, 1.0, 0.25)).abs().max()) <= 1e-3, int(((slope > 0.6) != side).sum())
+
+
 # elements that are zero or tiny because the inputs or the weights are need no second look, which costs thousands of cycles
 @pytest.mark.parametrize("case", ["zero inputs", "small inputs", "padding", "zero channels", "small channels", "one-hot inputs, pruned weights"])
 def test_no_input_is_slow(case):
