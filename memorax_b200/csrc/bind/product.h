@@ -20,11 +20,18 @@ constexpr double kLibraryFlops = 8e9;
 // microseconds): 256 x 256 over 65536 tokens 14 | 25, 768 x 256 over 32768 18 | 20, 512 x 512 over 32768 22 | 27, 1024 x 512 over 16384
 // 22 | 23, 128 x 1024 over 65536 32 | 32; beyond, 768 x 256 over 65536 37 | 32, 1024 x 512 over 32768 46 | 33.
 constexpr double kLibraryFlopsGradient = 1.75e10;
+// 2 M N K above which a product that is no gradient has a launch of its own: the tiles of a joint one are 64 columns wide, which costs more
+// than a launch from here on (together | apart in microseconds, two products into the rows of the mLSTM layer's heads, forward and backward, with
+// the larger one's operations: 4e8 8.7 | 10.4 and 7.4 | 9.4, 8e8 14.7 | 13.1 and 11.9 | 11.2, 1e9 19.3 | 15.6 and 13.5 | 13.2, 4.3e9 68 | 45 and
+// 47 | 37).  Gradients of weights are split over the SMs anyway: together at all sizes that are the kernel's (the layer's five, 6000 tokens of
+// 256 features 16 | 41, 16384 of 512 77 | 87, 65536 of 256 110 | 119).
+constexpr double kGroupFlops = 6e8;
 
 // A product over the last two dimensions as the kernel's job; `fits`: whether it is one for the kernel.
 struct AsJob {
   mxk::gemm16::Job job;
   bool a_rows, b_rows, fits;
+  double flops;
 };
 inline AsJob as_job(const Tensor& a, const Tensor& b, const Tensor& c, const Tensor& bias, bool accumulate) {
   namespace g = mxk::gemm16;
@@ -41,7 +48,8 @@ inline AsJob as_job(const Tensor& a, const Tensor& b, const Tensor& c, const Ten
   const auto fits = [&](const Tensor& t, const g::Matrix& m) {
     return (t.stride(r) == 1 || t.stride(q) == 1) && m.ld % 8 == 0 && m.batch_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(m.ptr) & 15) == 0;
   };
-  j.fits = 2.0 * batch * M * N * K <= (j.a_rows && j.b_rows ? kLibraryFlopsGradient : kLibraryFlops) && fits(a, ma) && fits(b, mb) && c.stride(q) == 1;
+  j.flops = 2.0 * batch * M * N * K;
+  j.fits = j.flops <= (j.a_rows && j.b_rows ? kLibraryFlopsGradient : kLibraryFlops) && fits(a, ma) && fits(b, mb) && c.stride(q) == 1;
   j.job = {ma, mb, bias.defined() ? bias.data_ptr() : nullptr, c.data_ptr(), c.stride(r), n == 3 ? c.stride(0) : 0, accumulate,
            static_cast<int>(batch), static_cast<int>(M), static_cast<int>(N), static_cast<int>(K)};
   return j;
@@ -70,7 +78,7 @@ inline void product_into(const Tensor& a, const Tensor& b, const Tensor& c, cons
     at::mm_out(out, a, b);
   }
 }
-// Products that do not depend on one another: one launch where all of them are the kernel's and stored alike.
+// Products that do not depend on one another: one launch where all of them are the kernel's, stored alike, and short or gradients.
 struct Product {
   Tensor a, b, c;
   bool accumulate = false;
@@ -83,7 +91,7 @@ inline void products_into(const std::vector<Product>& products) {
   for (const Product& p : products) {
     if (!together) break;
     const AsJob j = as_job(p.a, p.b, p.c, Tensor(), p.accumulate);
-    together = j.fits && (count == 0 || (j.a_rows == a_rows && j.b_rows == b_rows));
+    together = j.fits && (j.flops <= kGroupFlops || (j.a_rows && j.b_rows)) && (count == 0 || (j.a_rows == a_rows && j.b_rows == b_rows));
     a_rows = j.a_rows;
     b_rows = j.b_rows;
     jobs[count++] = j.job;

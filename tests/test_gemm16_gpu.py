@@ -77,8 +77,9 @@ def test_sums_into_whole_tiles(m, n, k, pad):
     ops.check_status()
 
 
-# several products in one launch: of one size and of very different ones, batched and not, split and whole
-@pytest.mark.parametrize("tokens", [5, 700, 6000])
+# several products in one launch: of one size and of very different ones, batched and not, split and whole; in launches of their own (the
+# last size, where they are no gradients)
+@pytest.mark.parametrize("tokens", [5, 700, 6000, 20000])
 @pytest.mark.parametrize("by_rows", [False, True])
 def test_products_that_share_a_launch(tokens, by_rows):
     from memorax_b200 import _C, ops
