@@ -51,7 +51,7 @@ struct Params {
   int k_split;           // k per split (a multiple of kBK)
   int splits;            // more than one: c is [splits][M][N]
   int run;               // stages that the hi*hi accumulator lives for after a tile's first run
-  int zero;              // 0
+  int zero;              // 0, which the compiler does not know
   Epilogue ep;           // of a contraction that is not split
   int* status;
 };

@@ -7,7 +7,7 @@
 //
 // Bound: shared memory.  A stage of 256 x 128 is 1536 cycles of the tensor pipe, but 48 KB copied in and read by the producers, 72 KB of planes
 // written and 192 KB read by the pipe (A and both halves of B for six products): 2800 cycles at 128 bytes.
-// Measured with the sum of the splits (the form of gemm32.cu): 1024 x 256 over 65536 tokens 202 us (204), 1024 x 512 over 24000 153 us (148),
+// Measured with the sum of the splits (the form of gemm32.cu): 1024 x 256 over 65536 tokens 203 us (204), 1024 x 512 over 24000 153 us (148),
 // 520 x 512 over 8192 53 us (50).
 //
 // One persistent CTA per SM, pairs on tiles of 256 x 128, or alone on 128 x 64:
@@ -38,7 +38,7 @@ struct Params {
   int k_split;           // tokens per split (a multiple of kBK)
   int splits;            // more than one: c is [splits][M][N]
   int run;               // stages that the accumulators live for
-  int zero;              // 0
+  int zero;              // 0, which the compiler does not know
   int* status;
 };
 
@@ -213,15 +213,15 @@ __global__ void __launch_bounds__(Config<kPair>::kThreads, 1) gemm32_long_outer_
           *reinterpret_cast<uint4*>(dst + j * rows * 16 + plane) = mid;
           *reinterpret_cast<uint4*>(dst + j * rows * 16 + 2 * plane) = lo;
         }
-        // the next stage's values, on their way under what is left of this one
-        if (seg + kBK < k_len) load(tile, seg + kBK);
-        else if (tile + tile_step < tiles) load(tile + tile_step, 0);
         fence_smem_to_async();
         __syncwarp();
         if (lane == 0) {
           if (kPair) arrive_written(&full[stage]);
           else arrive(&full[stage]);
         }
+        // (not before the arrival: there is one float32 tile, and the next may not have come yet; 65536 tokens of 1024 x 256 206 -> 203 us)
+        if (seg + kBK < k_len) load(tile, seg + kBK);
+        else if (tile + tile_step < tiles) load(tile + tile_step, 0);
         if (++stage == kStages) { stage = 0; parity ^= 1; }
       }
     }
